@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "gemm.cuh"
+#include "gemm_wide.cuh"
 #include "qgemm.cuh"
 #include "pre6.cuh"
 #include "sample.cuh"
@@ -381,7 +382,9 @@ enum KClass { KC_GEMM = 0, KC_WKV = 1, KC_LN = 2, KC_OTHER = 3 };
 struct GemmLaunch {
     GemmParams p;
     int grid = 0;
-    int grid_wide = 0;         // grid of steps with >= 64 tokens: whole tiles per CTA (see make_launch)
+    int grid_wide = 0;         // grid of steps with more than 64 tokens (see make_launch)
+    bool by_tile = false;      // that grid's CTAs own whole tiles
+    int max_contrib = 1, max_contrib_wide = 1;      // CTAs that can share a tile, per grid
     int total_tiles = 0;
     size_t weight_bytes = 0;   // algorithmic (unpadded) weight bytes streamed (f16, or codes + block parameters)
     int qtype = QT_NONE;       // weight format of every segment of the launch (qgemm.cuh)
@@ -825,22 +828,31 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
             for (int cand = num_sms; cand * 4 >= num_sms * 3; --cand)
                 if (tile % cand == 0) { g.grid = cand; break; }
     }
-    // Steps of 64 / 128 tokens: a partial accumulator tile is 32 / 64 KB per contributor, and the last arriver of a cut tile
-    // spends tens of microseconds summing them (measured: 3B K+R at 128 tokens, last MMA at 9-15 us, slowest CTA exits at
-    // 82 us; profiles/r02_steptrace_prefill128_3b.log).  Those steps run whole tiles per CTA, even if that leaves SMs idle.
-    g.grid_wide = g.grid;
-    if (force_grid <= 0) {
-        if (tile <= num_sms) g.grid_wide = tile;
-        else
-            for (int cand = num_sms; cand * 2 >= num_sms; --cand)        // several whole tiles per CTA; else keep stream-K
-                if (tile % cand == 0) { g.grid_wide = cand; break; }
+    // Steps of more than 64 tokens (gemm_wide.cuh): a partial accumulator tile is 64 / 128 KB, so launches that put at least half
+    // of the SMs to work give every CTA whole tiles, in rounds of equal length; the low-rank launches (2-20 tiles of a long k)
+    // cut their block sequence over the SMs, at least four blocks per CTA (3 CTAs and 68 us for 320 x 4096 at 128 tokens before).
+    if (qtype == QT_NONE) {
+        g.by_tile = tile * 2 >= num_sms;
+        g.grid_wide = g.by_tile ? cdiv(tile, cdiv(tile, num_sms)) : std::min(blk, std::max(tile, std::min(num_sms, cdiv(blk, 4))));
+        if (g.grid_wide == tile) g.by_tile = true;
+    } else {
+        g.grid_wide = g.grid;
+        if (force_grid <= 0) {
+            if (tile <= num_sms) g.grid_wide = tile;
+            else
+                for (int cand = num_sms; cand * 2 >= num_sms; --cand)        // several whole tiles per CTA; else keep stream-K
+                    if (tile % cand == 0) { g.grid_wide = cand; break; }
+        }
     }
-    const int per_cta = std::max(1, blk / g.grid);
-    g.p.max_contrib = cdiv(kbmax, per_cta) + 1;
+    g.max_contrib = cdiv(kbmax, std::max(1, blk / g.grid)) + 1;
+    g.max_contrib_wide = g.by_tile ? 1 : cdiv(kbmax, std::max(1, blk / g.grid_wide)) + 1;
+    g.p.max_contrib = g.max_contrib;
     g.p.counters = (unsigned*)dalloc((size_t)tile * 4, true);
     g.p.nrows = d_meta;   // T by default
     g.p.w_lbo = GEMM_W_LBO; g.p.w_sbo = GEMM_W_SBO; g.p.a_lbo = GEMM_A_LBO; g.p.a_sbo = GEMM_A_SBO;
-    gemm_ws_floats = std::max(gemm_ws_floats, (size_t)tile * g.p.max_contrib * (size_t)maxT * GEMM_BN);
+    const size_t part = (size_t)tile * GEMM_BN;
+    gemm_ws_floats = std::max({gemm_ws_floats, part * g.max_contrib * std::min(maxT, 64), g.by_tile ? 0 : part * g.max_contrib_wide * maxT});
+    if (qtype != QT_NONE) gemm_ws_floats = std::max(gemm_ws_floats, part * g.max_contrib * maxT);
     weight_bytes_total += g.weight_bytes;
     return g;
 }
@@ -901,15 +913,21 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
 #undef QLAUNCH
         return;
     }
+    auto launch_wide = [&](void (*kern)(GemmParams, int, int), size_t smem, bool wide) {
+        GemmParams p = g.p;
+        p.max_contrib = wide ? g.max_contrib_wide : g.max_contrib;
+        launch_k(kern, dim3(wide ? g.grid_wide : g.grid), dim3(WIDE_THREADS), smem, p, KC_GEMM, s, prof, (int)(wide && g.by_tile), g.total_tiles);
+    };
     // RING 2 = one stage less than fits, so the small kernels around a projection can share its SMs (findings r1 §7)
     switch (MT) {
         case 1:
             if (split) launch_k(gemm_kernel<2, 2, true>, dim3(g.grid), dim3(GEMM_THREADS), GemmCfg<2, 2>::SMEM_BYTES, g.p, KC_GEMM, s, prof);
             else launch_k(gemm_kernel<1, 2>, dim3(g.grid), dim3(GEMM_THREADS), GemmCfg<1, 2>::SMEM_BYTES, g.p, KC_GEMM, s, prof);
             break;
-        case 2: launch_k(gemm_kernel<2>, dim3(g.grid), dim3(GEMM_THREADS), GemmCfg<2>::SMEM_BYTES, g.p, KC_GEMM, s, prof); break;
-        case 4: launch_k(gemm_kernel<4>, dim3(g.grid_wide), dim3(GEMM_THREADS), GemmCfg<4>::SMEM_BYTES, g.p, KC_GEMM, s, prof); break;
-        default: launch_k(gemm_kernel<8>, dim3(g.grid_wide), dim3(GEMM_THREADS), GemmCfg<8>::SMEM_BYTES, g.p, KC_GEMM, s, prof); break;
+        case 2: launch_wide(gemm_wide_kernel<2>, WideCfg<2>::SMEM_BYTES, false); break;
+        case 4: launch_wide(gemm_wide_kernel<4>, WideCfg<4>::SMEM_BYTES, false); break;
+        case 8: launch_wide(gemm_wide_kernel<8>, WideCfg<8>::SMEM_BYTES, true); break;
+        default: launch_wide(gemm_wide_kernel<16>, WideCfg<16>::SMEM_BYTES, true); break;
     }
 }
 
@@ -946,9 +964,10 @@ void b200rwkv_engine::build(const StFile& st) {
     CK(cudaStreamCreateWithFlags(&sm_stream, cudaStreamNonBlocking));
     CK(cudaFuncSetAttribute(gemm_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<1, 2>::SMEM_BYTES));
     CK(cudaFuncSetAttribute(gemm_kernel<2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<2, 2>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<2>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(gemm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<4>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(gemm_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<8>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_wide_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<2>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_wide_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<4>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<8>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<16>::SMEM_BYTES));
     if (quant_layers > 0 && quant_type != QT_NONE) {
         REQUIRE(quant_type == QT_INT8 || quant_type == QT_NF4, B200RWKV_ERR_UNSUPPORTED, "quant_type must be Int8 or NF4 (SF4 is not implemented)");
         REQUIRE(world == 1, B200RWKV_ERR_UNSUPPORTED, "quantised layers are single-GPU in this version");
@@ -1458,7 +1477,7 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             ++seq_pos;
             g2.p.next_W = nx.qtype == QT_NONE ? nx.p.W : nullptr;     // the L2 prefetch walks 32 KB f16 blocks
             g2.p.next_blocks = nx.p.total_blocks;
-            g2.p.next_grid = mt >= 4 ? nx.grid_wide : nx.grid;
+            g2.p.next_grid = mt >= 8 ? nx.grid_wide : nx.grid;
             g2.p.prefetch_blocks = prefetch_blocks;
         }
         for (int i = 0; i < g2.p.nseg; ++i)
@@ -1561,7 +1580,7 @@ void b200rwkv_engine::run_step(int MT, int MTR) {
         launch_total += launches_last_step;
         return;
     }
-    const int key = MT * 8 + MTR;
+    const int key = MT * 32 + MTR;
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;
