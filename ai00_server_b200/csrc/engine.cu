@@ -31,6 +31,7 @@
 #include "streamtest.cuh"
 #endif
 #include "wkv.cuh"
+#include "wkv_scan.cuh"
 #include "linear.cuh"
 #include "rmsnorm.cuh"
 #include "latent_attn.cuh"
@@ -613,8 +614,8 @@ struct b200rwkv_engine {
         return d_step_trace + (size_t)STEP_TRACE_ROW * launches_last_step;
     }
     void launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, Profiler* prof, bool split = false);
-    void enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof);
-    void run_step(int MT, int MTR);
+    void enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof, bool runs = false);   // runs: some sequence holds more than WKV_STAGE_TOK tokens
+    void run_step(int MT, int MTR, bool runs = false);
     int fill_meta(int* m, const std::vector<int>& slots, const std::vector<int>& counts, const std::vector<const uint32_t*>& toks,
                   const std::vector<int>& outmode /*0 none,1 last,2 full*/, int* R_out);
     void infer(int nslot, const int32_t* slot, const int32_t* ntok, const uint32_t* tokens, const int32_t* option,
@@ -1439,15 +1440,18 @@ void b200rwkv_engine::finalize_tp() {
 // -----------------------------------------------------------------------------------------
 // one forward step over the tokens described by d_meta
 // -----------------------------------------------------------------------------------------
-void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof) {
+void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof, bool runs) {
     launches_last_step = 0;
     const int rows = MT * 16;
     // token rows of this step's A16 operands (common.cuh): every producer and consumer of the step uses the same value
     const int th = (split_on && MT == 1) ? 32 : 16 * MT;
     const int th_rows = (split_on && MT == 1) ? 32 : 16 * MTR;        // the head's operand holds output rows
     last_th = th;
+    // sequences of more than WKV_STAGE_TOK tokens: the scan kernel, with the decays of its own launch (split operands stay with the
+    // decode kernel, whose steps hold 16 tokens at most)
+    const bool scan = runs && !split_on;
     auto pre_skipped = [&](const Layer& ly, int gi) {
-        if (fold_wd2 && gi == ly.wd2_index) return true;                 // the WKV kernel evaluates the decay LoRA stage 2
+        if (fold_wd2 && !scan && gi == ly.wd2_index) return true;        // the WKV kernel evaluates the decay LoRA stage 2
         return fused_pre_ok && MT == 1 && ly.w1_raw && gi < 2;           // the front-half kernel holds both ddlerp LoRA stages
     };
     // projection launches of this step in stream order: each one prefetches the head of the next into L2 (the last one
@@ -1533,6 +1537,12 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             wp.trace = tr_next(2);
             wp.kq_tile = th; wp.d1_kq = th;
             const bool sp = split_on && MT == 1;
+            if (scan) {
+                const dim3 grid(Hl, wkv_slots), block(WKS_THREADS);
+                if (info.version == 5) launch_k(wkv_scan_kernel<5>, grid, block, WksCfg<5>::SMEM_BYTES, wp, KC_WKV, s, prof);
+                else if (info.version == 6) launch_k(wkv_scan_kernel<6>, grid, block, WksCfg<6>::SMEM_BYTES, wp, KC_WKV, s, prof);
+                else launch_k(wkv_scan_kernel<7>, grid, block, WksCfg<7>::SMEM_BYTES, wp, KC_WKV, s, prof);
+            } else {
             const size_t sm_b = wkv_smem_bytes(info.version, fold_wd2, info.time_decay_adapter, rows, sp);
             switch (info.version * 2 + (sp ? 1 : 0)) {
                 case 10: launch_k(wkv_kernel<5>, dim3(Hl, wkv_slots), dim3(WKV_SA_THREADS), sm_b, wp, KC_WKV, s, prof, rows); break;
@@ -1541,6 +1551,7 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
                 case 13: launch_k(wkv_kernel<6, true>, dim3(Hl, wkv_slots), dim3(WKV_SA_THREADS), sm_b, wp, KC_WKV, s, prof, rows); break;
                 case 14: launch_k(wkv_kernel<7>, dim3(Hl, wkv_slots), dim3(WKV_SA_THREADS), sm_b, wp, KC_WKV, s, prof, rows); break;
                 default: launch_k(wkv_kernel<7, true>, dim3(Hl, wkv_slots), dim3(WKV_SA_THREADS), sm_b, wp, KC_WKV, s, prof, rows); break;
+            }
             }
         }
         gemm(ly.o);
@@ -1573,20 +1584,20 @@ void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MTR) {
     launch_k(keep_rows_kernel, dim3(MTR * 16, KEEP_CHUNKS), dim3(KEEP_THREADS), 0, kp, KC_OTHER, s, nullptr);
 }
 
-void b200rwkv_engine::run_step(int MT, int MTR) {
+void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
     if (!use_graph) {
-        enqueue_step(stream, MT, MTR, nullptr);
+        enqueue_step(stream, MT, MTR, nullptr, runs);
         enqueue_keep(stream, MTR);
         launch_total += launches_last_step;
         return;
     }
-    const int key = MT * 32 + MTR;
+    const int key = (MT * 32 + MTR) * 2 + (runs ? 1 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_step(stream, MT, MTR, nullptr);
+            enqueue_step(stream, MT, MTR, nullptr, runs);
             enqueue_keep(stream, MTR);
         } catch (...) {
             cudaStreamEndCapture(stream, &g);
@@ -1726,7 +1737,7 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
         CK(cudaMemcpyAsync(d_meta, hm, meta_ints * 4, cudaMemcpyHostToDevice, stream));
         CK(cudaEventRecord(meta_ev[mb], stream));
         if (kx) kx_run_step(T, R, kx_decode, kx_split);
-        else run_step(mt_bucket(T), R > 0 ? mt_bucket(R) : 0);
+        else run_step(mt_bucket(T), R > 0 ? mt_bucket(R) : 0, *std::max_element(s_counts.begin(), s_counts.end()) > WKV_STAGE_TOK);
         if (hidden_keep) {       // hidden rows of every token of this call (b200rwkv_last_hidden), in entry order
             int t0 = 0;
             for (size_t j = 0; j < s_entry.size(); ++j) {
@@ -2748,9 +2759,18 @@ int32_t b200rwkv_op_wkv(int32_t device, int32_t version, int32_t T, int32_t H, c
     CK(cudaMemset(p.out, 0, halves * 2));
     const size_t smem = wkv_smem_bytes(version, false, 0, maxT);
     switch (version) {
-        case 5: wkv_kernel<5><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT); break;
-        case 6: wkv_kernel<6><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT); break;
-        default: wkv_kernel<7><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT); break;
+        case 5:
+            if (T > WKV_STAGE_TOK) wkv_scan_kernel<5><<<dim3(H, 1), WKS_THREADS, WksCfg<5>::SMEM_BYTES>>>(p);
+            else wkv_kernel<5><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT);
+            break;
+        case 6:
+            if (T > WKV_STAGE_TOK) wkv_scan_kernel<6><<<dim3(H, 1), WKS_THREADS, WksCfg<6>::SMEM_BYTES>>>(p);
+            else wkv_kernel<6><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT);
+            break;
+        default:
+            if (T > WKV_STAGE_TOK) wkv_scan_kernel<7><<<dim3(H, 1), WKS_THREADS, WksCfg<7>::SMEM_BYTES>>>(p);
+            else wkv_kernel<7><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT);
+            break;
     }
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());

@@ -14,8 +14,8 @@
 //     four warps holding the whole accumulator in registers the epilogue was longer than the main loop;
 //   * partial tiles of a split k range lie in the workspace as [token group][4-token quad][row] float4, so that a warp writes and
 //     reads 512 contiguous bytes (one row per lane with the tokens side by side was 32 sectors per request);
-//     Measured (7B widths, 100 tokens, ncu): low-rank stage 1 68 -> 19 us, R/K/V/G 75 -> 45, channel mix 67 / 36 -> 46 / 29;
-//     32 prompts of 512 tokens through four layers of 3B widths 144.7 -> 88.7 ms;
+//     Measured (100 tokens, 7B widths, ncu): low-rank stages 68 -> 27 and 43 -> 27 us, R/K/V/G 75 -> 42, output 25 -> 18, channel
+//     mix 67 -> 45 and 36 -> 32;
 //   * launches with at least half as many tiles as SMs give every CTA whole tiles (WIDE_BY_TILE), the others (low-rank stages)
 //     cut their block sequence over the SMs and the last arriver of a tile sums the parts in fixed order.
 #pragma once
