@@ -42,13 +42,13 @@ __device__ __forceinline__ void rot_cos_sin(int pos, double freq, float& cs, flo
 // 128-wide k block of ALL tokens of the step -- is ONE contiguous run (one bulk TMA copy) and (b) that run IS the UMMA
 // canonical K-major / no-swizzle operand of `th` token rows, which ONE tcgen05.mma with N = th consumes:
 //   [k block (128 k)][k8 chunk 16][th token rows][8 halves]      (8 rows x 16 B = one 128-byte core matrix)
-// th = 16 x (token tiles of the step) = 16 / 32 / 64 / 128; a step's producers and consumers agree on it (the engine passes
+// th = 16 x (token tiles of the step) = 16 / 32 / 64 / 128 / 256; a step's producers and consumers agree on it (the engine passes
 // it to every launch).  Measured (profiles/r02_findings.md §8): a tcgen05.mma with N = 16 costs ~80 cycles whatever N is, so
 // eight N = 16 MMAs per k step (128-token steps) made the projections MMA-bound; one N = 128 MMA does not.
 // Split operands (precision 1): th = 32, rows 0-15 hold the hi halves of the 16 tokens, rows 16-31 the lo halves.
-// Every buffer reserves 128 token rows per k block and K padded to whole k blocks (padding k is multiplied by zero weights).
+// Every buffer reserves 256 token rows per k block and K padded to whole k blocks (padding k is multiplied by zero weights).
 // ---------------------------------------------------------------------------------------
-constexpr int A16_MAX_ROWS = 128;                      // token rows per k block: steps of up to 128 tokens
+constexpr int A16_MAX_ROWS = 256;                      // token rows per k block: steps of up to 256 tokens
 constexpr int A16_KB_HALVES = A16_MAX_ROWS * 128;      // halves per k block of a buffer
 __host__ __device__ inline size_t a16_index(int m, int k, int th) {
     return (size_t)(k >> 7) * A16_KB_HALVES + ((size_t)((k >> 3) & 15) * th + m) * 8 + (k & 7);

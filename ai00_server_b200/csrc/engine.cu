@@ -384,6 +384,7 @@ struct GemmLaunch {
     GemmParams p;
     int grid = 0;
     int grid_wide = 0;         // grid of steps with more than 64 tokens (see make_launch)
+    bool short_k = false;      // every tile is one block long: gemm_wide.cuh's SHORT form
     bool by_tile = false;      // that grid's CTAs own whole tiles
     int max_contrib = 1, max_contrib_wide = 1;      // CTAs that can share a tile, per grid
     int total_tiles = 0;
@@ -502,6 +503,7 @@ struct b200rwkv_engine {
     // step plumbing
     static constexpr int META_RING = 4;
     cudaEvent_t meta_ev[META_RING] = {nullptr, nullptr, nullptr, nullptr};
+    std::vector<std::pair<int, int>> last_runs;     // token runs (first, count) of the last portion in the last step's rows
     bool hidden_keep = false;          // b200rwkv_keep_hidden: accumulate the hidden rows of every token of an infer call
     float* d_hidden_all = nullptr;
     size_t hidden_cap_rows = 0;
@@ -835,7 +837,9 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
     if (qtype == QT_NONE) {
         g.by_tile = tile * 2 >= num_sms;
         g.grid_wide = g.by_tile ? cdiv(tile, cdiv(tile, num_sms)) : std::min(blk, std::max(tile, std::min(num_sms, cdiv(blk, 4))));
-        if (g.grid_wide == tile) g.by_tile = true;
+        g.short_k = kbmax == 1;
+        if (g.short_k) g.grid_wide = std::min(tile, 2 * num_sms);
+        if (g.grid_wide == tile || g.short_k) g.by_tile = true;
     } else {
         g.grid_wide = g.grid;
         if (force_grid <= 0) {
@@ -927,8 +931,14 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
             break;
         case 2: launch_wide(gemm_wide_kernel<2>, WideCfg<2>::SMEM_BYTES, false); break;
         case 4: launch_wide(gemm_wide_kernel<4>, WideCfg<4>::SMEM_BYTES, false); break;
-        case 8: launch_wide(gemm_wide_kernel<8>, WideCfg<8>::SMEM_BYTES, true); break;
-        default: launch_wide(gemm_wide_kernel<16>, WideCfg<16>::SMEM_BYTES, true); break;
+        case 8:
+            if (g.short_k) launch_wide(gemm_wide_kernel<8, true>, WideCfg<8, true>::SMEM_BYTES, true);
+            else launch_wide(gemm_wide_kernel<8>, WideCfg<8>::SMEM_BYTES, true);
+            break;
+        default:
+            if (g.short_k) launch_wide(gemm_wide_kernel<16, true>, WideCfg<16, true>::SMEM_BYTES, true);
+            else launch_wide(gemm_wide_kernel<16>, WideCfg<16>::SMEM_BYTES, true);
+            break;
     }
 }
 
@@ -968,6 +978,8 @@ void b200rwkv_engine::build(const StFile& st) {
     CK(cudaFuncSetAttribute(gemm_wide_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<2>::SMEM_BYTES));
     CK(cudaFuncSetAttribute(gemm_wide_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<4>::SMEM_BYTES));
     CK(cudaFuncSetAttribute(gemm_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<8>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_wide_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<8, true>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_wide_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<16, true>::SMEM_BYTES));
     CK(cudaFuncSetAttribute(gemm_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<16>::SMEM_BYTES));
     if (quant_layers > 0 && quant_type != QT_NONE) {
         REQUIRE(quant_type == QT_INT8 || quant_type == QT_NF4, B200RWKV_ERR_UNSUPPORTED, "quant_type must be Int8 or NF4 (SF4 is not implemented)");
@@ -994,6 +1006,10 @@ void b200rwkv_engine::build(const StFile& st) {
     if (const char* v = dbg_env("B200RWKV_PREFETCH_BLOCKS")) prefetch_blocks = std::max(0, atoi(v));
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;
     if (const char* v = dbg_env("B200RWKV_LN_CLUSTER")) ln_cluster = atoi(v) != 0;
+
+    // 256-token steps: single-GPU f16 models (quantised launches stop at 128 token rows, split operands at 16 tokens, and a
+    // tensor-parallel rank would double the block it shares with its peers)
+    maxT = (world == 1 && precision == 0 && quant_layers == 0) ? A16_MAX_ROWS : 128;
 
     // ---- step metadata ----
     meta_ints = MetaView::ints(maxT, S);
@@ -1570,7 +1586,7 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
     if (world > 1) launch_k(tp_barrier_kernel, dim3(1), dim3(32), 0, tpbar, KC_OTHER, s, prof);
 }
 
-static inline int mt_bucket(int rows) { return rows <= 16 ? 1 : (rows <= 32 ? 2 : (rows <= 64 ? 4 : 8)); }
+static inline int mt_bucket(int rows) { return rows <= 16 ? 1 : (rows <= 32 ? 2 : (rows <= 64 ? 4 : (rows <= 128 ? 8 : 16))); }
 
 // last logits row of every slot of this step -> keep[slot] (rank 0 gathers the vocabulary shards); see sample.cuh
 void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MTR) {
@@ -1674,7 +1690,10 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
     // logits_out == NULL: the rows stay in HBM (b200rwkv_sample_topk reads the last row of every slot from there)
     const bool copy_logits = want_logits && logits_out != nullptr;
     // f32-activation mode runs every step decode-shaped (<= 16 tokens): the split-operand kernels are the 16-token ones
-    const int step_cap = std::min(chunk, split_on ? 16 : maxT);
+    const int step_cap = std::min(chunk, split_on ? 16 : (kx ? maxT : std::min(maxT, 128)));
+    // RWKV steps of full portions hold two of them (gemm_wide.cuh: one pass over the weights for 256 tokens; 128-token steps are bound by
+    // the weight stream): the portions, and with them the rows b200rwkv_last_hidden answers, are those of 128-token steps
+    const int substeps = !kx && step_cap == 128 && maxT >= 256 ? 2 : 1;
     // Step packing: every step shares its token budget evenly over the entries that still have tokens (web-rwkv shares the
     // chunk "fairly across slots"; results do not depend on the cut).  Many slots with one token each keep
     // the WKV kernels wide (one CTA per head and slot) where a single slot with 64 tokens would run them 40 CTAs wide.
@@ -1699,23 +1718,34 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
         if (n_active == 0) break;
         std::vector<int> s_entry, s_slots, s_counts, s_out;
         std::vector<const uint32_t*> s_toks;
-        // at least WKV_STAGE_TOK tokens per slot and step while prompts are long: a WKV CTA then loads and stores its 16 KB
-        // of state once per four tokens (staged path) and a step touches a quarter of the slots' states
-        const int quota = std::max(WKV_STAGE_TOK, step_cap / n_active);
-        int used = 0;
-        for (int i = 0; i < nslot && used < step_cap; ++i) {
-            const int remain = ntok[i] - pos[i];
-            if (remain <= 0) continue;
-            const int take = std::min({remain, quota, step_cap - used});
-            s_entry.push_back(i);
-            s_counts.push_back(take);
-            used += take;
+        std::vector<int> step(nslot, 0), part(nslot, 0);
+        for (int sub = 0; sub < substeps; ++sub) {
+            // at least WKV_STAGE_TOK tokens per slot and portion while prompts are long: a WKV CTA then loads and stores its 16 KB
+            // of state once per four tokens or more, and a portion touches a quarter of the slots' states
+            n_active = 0;
+            for (int i = 0; i < nslot; ++i) n_active += (pos[i] + step[i] < ntok[i]);
+            if (n_active == 0) break;
+            const int quota = std::max(WKV_STAGE_TOK, step_cap / n_active);
+            int used = 0;
+            for (int i = 0; i < nslot; ++i) {
+                part[i] = std::max(0, std::min({ntok[i] - pos[i] - step[i], quota, step_cap - used}));
+                used += part[i];
+            }
+            for (int i = 0; i < nslot && used < step_cap; ++i) {      // left-over budget, in entry order
+                if (part[i] == 0) continue;
+                const int extra = std::min(ntok[i] - pos[i] - step[i] - part[i], step_cap - used);
+                part[i] += extra;
+                used += extra;
+            }
+            for (int i = 0; i < nslot; ++i) step[i] += part[i];
         }
-        for (size_t j = 0; j < s_entry.size() && used < step_cap; ++j) {      // left-over budget, in entry order
-            const int i = s_entry[j];
-            const int extra = std::min(ntok[i] - pos[i] - s_counts[j], step_cap - used);
-            s_counts[j] += extra;
-            used += extra;
+        last_runs.clear();
+        for (int i = 0, t = 0; i < nslot; ++i) {
+            if (step[i] == 0) continue;
+            s_entry.push_back(i);
+            s_counts.push_back(step[i]);
+            t += step[i];
+            if (part[i] > 0) last_runs.push_back({t - part[i], part[i]});
         }
         for (size_t j = 0; j < s_entry.size(); ++j) {
             const int i = s_entry[j];
@@ -2809,10 +2839,20 @@ int32_t b200rwkv_last_hidden(b200rwkv_engine* e, float* out, size_t cap) {
         CK(cudaSetDevice(e->dev));
         CK(cudaStreamSynchronize(e->stream));
         const bool all = e->hidden_keep && e->d_hidden_all;
-        rows = all ? e->hidden_rows : e->last_T;
+        rows = 0;
+        if (all) rows = e->hidden_rows;
+        else
+            for (const auto& r : e->last_runs) rows += r.second;
         const size_t n = (size_t)rows * e->C;
         REQUIRE(n <= cap, B200RWKV_ERR_INVALID, "hidden buffer too small");
-        if (n) CK(cudaMemcpy(out, all ? e->d_hidden_all : e->d_hidden, n * 4, cudaMemcpyDeviceToHost));
+        if (n && all) CK(cudaMemcpy(out, e->d_hidden_all, n * 4, cudaMemcpyDeviceToHost));
+        if (n && !all) {
+            size_t at = 0;
+            for (const auto& r : e->last_runs) {
+                CK(cudaMemcpy(out + at, e->d_hidden + (size_t)r.first * e->C, (size_t)r.second * e->C * 4, cudaMemcpyDeviceToHost));
+                at += (size_t)r.second * e->C;
+            }
+        }
         API_END
     }();
     return st < 0 ? st : rows;

@@ -28,19 +28,22 @@ constexpr int WIDE_THREADS = WIDE_EPI_THREADS + 64;         // + MMA warp + TMA 
 constexpr int WIDE_KS = 64;                                 // k per stage
 constexpr int WIDE_STAGE_BUDGET = 204800;
 
-template <int MT>
+// SHORT: launches whose tiles are one block long (second low-rank stages) are all epilogue: a ring of one block and a single
+// accumulator, so that two CTAs share an SM and one tile's operand loads hide behind the other's
+template <int MT, bool SHORT = false>
 struct WideCfg {
     static constexpr int W_BYTES = GEMM_BN * WIDE_KS * 2;   // 16 KB
     static constexpr int A_BYTES = MT * 16 * WIDE_KS * 2;   // 2 KB per 16 tokens
     static constexpr int STAGE_BYTES = W_BYTES + A_BYTES;
-    static constexpr int NSTAGE = WIDE_STAGE_BUDGET / STAGE_BYTES;
-    static constexpr int PAIR = MT >= 4 ? 2 : 1;            // 16-token groups an epilogue warp handles at a time
+    static constexpr int NSTAGE = SHORT ? 2 : WIDE_STAGE_BUDGET / STAGE_BYTES;
+    static constexpr int NACC = SHORT ? 1 : 2;              // accumulators
+    static constexpr int PAIR = MT >= 4 && !SHORT ? 2 : 1;  // 16-token groups an epilogue warp handles at a time (SHORT: half the registers)
     static constexpr int OUT_HALVES = GEMM_BN * GEMM_STAGE_PITCH;            // transpose buffer of one group (6 KB)
     static constexpr int OUT_BYTES = 2 * PAIR * OUT_HALVES * 2;
     static constexpr int BAR_OFF = NSTAGE * STAGE_BYTES + OUT_BYTES;
     static constexpr int SMEM_BYTES = BAR_OFF + (2 * NSTAGE + 4) * 8 + 16;
-    static constexpr int TMEM_COLS = 2 * 16 * MT;           // double-buffered accumulator: 64 .. 512 columns
-    static_assert(SMEM_BYTES <= 227 * 1024 - 1024, "one CTA per SM");
+    static constexpr int TMEM_COLS = NACC * 16 * MT < 32 ? 32 : NACC * 16 * MT;     // 32 .. 512 columns
+    static_assert(SMEM_BYTES <= 227 * 1024 - 1024, "one CTA per SM, two if SHORT");
 };
 
 // block range of a CTA: whole tiles, or an equal share of the block sequence
@@ -50,9 +53,9 @@ __device__ __forceinline__ int wide_tile_block(const GemmParams& p, int t) {
     return p.seg[s].blk_begin + (t - p.seg[s].tile_begin) * p.seg[s].KB;
 }
 
-template <int MT>
-__global__ void __launch_bounds__(WIDE_THREADS, 1) gemm_wide_kernel(const __grid_constant__ GemmParams p, const int by_tile, const int total_tiles) {
-    using Cfg = WideCfg<MT>;
+template <int MT, bool SHORT = false>
+__global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(const __grid_constant__ GemmParams p, const int by_tile, const int total_tiles) {
+    using Cfg = WideCfg<MT, SHORT>;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int s_last;
     __half* const s_out = reinterpret_cast<__half*>(smem + Cfg::NSTAGE * Cfg::STAGE_BYTES);
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) gemm_wide_kernel(const __grid
             SegWalk w;
             for (w.init(p, b0, b1); !w.done(); w.next(), ++segcount) {
                 const int nst = 2 * w.nblk();
-                const unsigned acc = segcount & 1u, use = segcount >> 1;
+                const unsigned acc = segcount % Cfg::NACC, use = segcount / Cfg::NACC;
                 if (use > 0) mbar_wait(tempty_bar + acc * 8, (use - 1) & 1u, 11);
                 tc_fence_after();
                 const uint32_t d0 = tmem_base + acc * (16 * MT);
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) gemm_wide_kernel(const __grid
         SegWalk w;
         for (w.init(p, b0, b1); !w.done(); w.next(), ++segcount) {
             const GemmSeg& sg = p.seg[w.seg];
-            const unsigned acc = segcount & 1u, use = segcount >> 1;
+            const unsigned acc = segcount % Cfg::NACC, use = segcount / Cfg::NACC;
             mbar_wait(tfull_bar + acc * 8, use & 1u, 13);
             tc_fence_after();
             const uint32_t tm = tmem_base + lane_base + acc * (16 * MT);
@@ -236,13 +239,19 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) gemm_wide_kernel(const __grid
                 if (ncontrib == 1) { tc_ld16(tm + mt * 16, v); return; }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = 0.f;
-                for (int s = 0; s < ncontrib; ++s) {
-                    const float* src = ws0 + (size_t)s * (GEMM_BN * 16 * MT) + (size_t)(mt * 4) * (GEMM_BN * 4);
+                for (int s0 = 0; s0 < ncontrib; s0 += 4) {              // fixed order; four contributors' loads in flight
+                    float4 q[4][4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float4 q = __ldcg(reinterpret_cast<const float4*>(src + (size_t)j * (GEMM_BN * 4)));
-                        v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
+                    for (int u = 0; u < 4; ++u) {
+                        const float* src = ws0 + (size_t)(s0 + u) * (GEMM_BN * 16 * MT) + (size_t)(mt * 4) * (GEMM_BN * 4);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            q[u][j] = s0 + u < ncontrib ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)j * (GEMM_BN * 4))) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) { v[4 * j] += q[u][j].x; v[4 * j + 1] += q[u][j].y; v[4 * j + 2] += q[u][j].z; v[4 * j + 3] += q[u][j].w; }
                 }
             };
             auto body = [&](auto act_c) {

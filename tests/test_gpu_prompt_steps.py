@@ -45,3 +45,23 @@ def test_step_sizes(preset, n):
 @pytest.mark.parametrize("preset", ["tiny5", "tiny6", "tiny7"])
 def test_full_rows_of_ragged_batches(preset, lens):
     _check(preset, lens, full=True)
+
+
+@pytest.mark.parametrize("lens, rows", [([200], [(0, 128, 200)]), ([130, 140, 5], [(1, 121, 140)])])
+def test_last_hidden_answers_the_last_portion(lens, rows):
+    """Without keep_hidden the hidden rows are those of the call's last portion of at most 128 tokens, whatever a step holds."""
+    st = synth.make_st("tiny6", 3)
+    orc = O.Oracle(O.parse_st(st), "f16")
+    rng = np.random.default_rng(9)
+    toks = [rng.integers(1, 500, n).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=128)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        m.infer_raw(list(range(len(lens))), lens, sum(toks, []), [capi.OPTION_NONE] * len(lens))
+        got = m.last_hidden(max_rows=128)
+        want = np.concatenate([orc.hidden(toks[s], orc.state_init())[0][a:b] for s, a, b in rows])
+        assert got.shape == want.shape
+        assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+    finally:
+        m.close()
