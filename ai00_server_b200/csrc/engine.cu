@@ -33,6 +33,7 @@
 #include "wkv.cuh"
 #include "wkv_scan.cuh"
 #include "linear.cuh"
+#include "linear_umma.cuh"
 #include "rmsnorm.cuh"
 #include "latent_attn.cuh"
 #include "gla.cuh"
@@ -463,9 +464,10 @@ struct b200rwkv_engine {
     std::unique_ptr<Group> group;             // set on rank 0 of an in-process tensor-parallel engine
     b200rwkv_info info;
     int dev = 0, rank = 0, world = 1, num_sms = 148;
-    int S = 0, chunk = 0, maxT = A16_MAX_ROWS, precision = 0;      // steps of up to 128 tokens
+    int S = 0, chunk = 0, maxT = A16_MAX_ROWS, precision = 0;      // token rows of a step
     int L = 0, C = 0, F = 0, V = 0, H = 0, N = 64, Cl = 0, Hl = 0, Fl = 0, Vl = 0;
     bool use_graph = true, use_pdl = true;
+    bool planning = false;             // a walk over the launches of a step that launches nothing (workspace sizes)
     int split_att = 1, split_ffn = 1;
     // tensor parallel: one symmetric comm block per rank (partials, gate block, logits shard, flags)
     uint8_t* comm_base = nullptr;
@@ -556,6 +558,7 @@ struct b200rwkv_engine {
     void ff_enqueue_layers(cudaStream_t s, int rows, int nslot_grid, bool decode, int nsplit, Profiler* prof);
     __nv_bfloat16* kx_up16(const std::vector<uint16_t>& v);
     float* kx_up32(const std::vector<float>& v);
+    bool kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int rows, int groups);
     void kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int rows, int groups, bool force_exact = false);
     void kx_short_conv(cudaStream_t s, Profiler* prof, const ShortConvParams& cp, int rows, int nslot_grid, bool decode);
     void kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, int H_, int dk, int dv, const float* q, const float* k, const float* v,
@@ -865,6 +868,7 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
 template <typename P, typename... X>
 void b200rwkv_engine::launch_k(void (*kern)(P, X...), dim3 grid, dim3 block, size_t smem, const P& params, int cls, cudaStream_t s,
                                Profiler* prof, X... extra) {
+    if (planning) { launch_cluster = 0; return; }
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;

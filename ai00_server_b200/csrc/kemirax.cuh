@@ -395,6 +395,10 @@ struct SeqModel {
     float* lin_ws = nullptr; size_t lin_ws_floats = 0;
     __nv_bfloat16* pairs = nullptr;               // [buckets + 1][W] embedding rows of token pairs
     float* last_tok = nullptr;                    // [S] last token of every sequence (families with pair embeddings)
+    // bf16 operand rows of one projection launch (linear_umma.cuh) per stream, sized by a walk over the largest step; tile counters
+    __nv_bfloat16 *lin_x16 = nullptr, *lin_x16_side = nullptr; size_t lin_x16_bytes = 0;
+    unsigned *lin_counters = nullptr, *lin_counters_side = nullptr;
+    int max_top = 1;                             // experts a token may choose (rows of the routed launches)
     bool side_lin = false; float* lin_ws_side = nullptr;      // projections also run on the side stream: split-k sums of their own
     float* dbg_layers = nullptr;                  // [L][maxT][W] residual after every layer (bring-up aid; nullptr: off)
     int max_split = 16;

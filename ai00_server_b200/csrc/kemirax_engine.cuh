@@ -286,13 +286,82 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
     CK(cudaFuncSetAttribute(lin_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_TC_SMEM));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<32>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<64>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<128>::SMEM_BYTES));
+    if (!m.exact) {
+        m.max_top = std::max(1, (int)z.max_top);
+        m.lin_counters = (unsigned*)dalloc(LU_MAX_COUNTERS * 4, true);
+        if (m.side_lin) m.lin_counters_side = (unsigned*)dalloc(LU_MAX_COUNTERS * 4, true);
+        planning = true;
+        kx_enqueue_step(stream, maxT, maxT, false, 1, nullptr);
+        planning = false;
+        if (m.lin_x16_bytes) {
+            m.lin_x16 = (__nv_bfloat16*)dalloc(m.lin_x16_bytes, false);
+            if (m.side_lin) m.lin_x16_side = (__nv_bfloat16*)dalloc(m.lin_x16_bytes, false);
+        }
+    }
     CK(cudaDeviceSynchronize());
+}
+
+static void lu_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+    static PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        CK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q));
+        REQUIRE(f && q == cudaDriverEntryPointSuccess, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+        return (PFN_cuTensorMapEncodeTiled_v12000)f;
+    }();
+    const cuuint64_t dim[2] = {K, rows}, stride[1] = {K * 2};
+    const cuuint32_t box[2] = {LU_KS, box_rows}, es[2] = {1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dim, stride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    REQUIRE(r == CUDA_SUCCESS, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+}
+
+// the tcgen05 form of a grouped linear: rows of 16-byte chunks (K % 8, aligned weights: what a TMA box row needs), groups whose
+// weights follow one another.  Row tiles of 128 (the MMA rate's knee, 64 cycles), less for steps of few rows; routed launches see
+// a fraction of the step's rows per group and take the next smaller tile.
+bool b200rwkv_engine::kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int rows, int groups) {
+    SeqModel& m = *kx;
+    if (p.K % 8 != 0 || (reinterpret_cast<uintptr_t>(p.W) & 15) != 0 || (groups > 1 && p.w_gstride != (long long)p.N * p.K)) return false;
+    const bool pairs = p.epi == LE_GLU_CLAMP || p.epi == LE_GLU_SILU || p.epi == LE_SPLIT_GLU_RELU;
+    if (pairs && (p.N % 2 != 0 || (p.epi == LE_SPLIT_GLU_RELU && p.split % 2 != 0))) return false;
+    const size_t total = p.off ? (size_t)rows * m.max_top : (size_t)groups * rows;
+    if (planning) { m.lin_x16_bytes = std::max(m.lin_x16_bytes, total * p.K * 2); return true; }
+    const bool side = m.side_lin && s == m.side_stream;
+    __nv_bfloat16* const x16 = side ? m.lin_x16_side : m.lin_x16;
+    const int tn = p.off ? (rows <= 64 ? 32 : (rows <= 128 ? 64 : 128)) : (rows <= 32 ? 32 : (rows <= 64 ? 64 : 128));
+    const int mtiles = cdiv(p.N, LU_BM), ttiles = cdiv(rows, tn), slabs = cdiv(p.K, LU_KS);
+    int ks = 1;
+    if (groups == 1 && !p.off && !p.xlist && mtiles * ttiles <= LU_MAX_COUNTERS) {
+        // k parts until the SMs are busy, at least six slabs (a ring full) each
+        ks = std::max(1, std::min({num_sms / (mtiles * ttiles), 8, slabs / 6}));
+        while (ks > 1 && (size_t)mtiles * ttiles * ks * LU_BM * tn > m.lin_ws_floats) --ks;
+        ks = cdiv(slabs, cdiv(slabs, ks));
+    }
+    launch_k(lin_pack_kernel, dim3(std::min(cdiv(rows * (p.K / 8), 256), 4 * num_sms), groups), dim3(256), 0, p, KC_GEMM, s, prof, x16);
+    LinUmmaParams u;
+    memset(&u, 0, sizeof(u));
+    lu_map(&u.tw, p.W, (uint64_t)groups * p.N, p.K, LU_BM);
+    lu_map(&u.tx, x16, total, p.K, tn);
+    u.l = p; u.groups = groups; u.ksplit = ks;
+    u.l.ws = side ? m.lin_ws_side : m.lin_ws;
+    u.counters = side ? m.lin_counters_side : m.lin_counters;
+    // list launches: the rows of all groups together are at most rows * top, plus a partial tile per group
+    const int tiles = p.off ? cdiv((int)total, tn) + groups : groups * ttiles;
+    const dim3 grid(std::min(num_sms, mtiles * tiles * ks));
+    if (tn == 32) launch_k(lin_umma_kernel<32>, grid, dim3(LU_THREADS), LuCfg<32>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    else if (tn == 64) launch_k(lin_umma_kernel<64>, grid, dim3(LU_THREADS), LuCfg<64>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    else launch_k(lin_umma_kernel<128>, grid, dim3(LU_THREADS), LuCfg<128>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    return true;
 }
 
 // one grouped linear launch; `rows` bounds the row count of any group (the step's bucket)
 void b200rwkv_engine::kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int rows, int groups, bool force_exact) {
     p.max_rows = rows;
     const bool exact = kx->exact || force_exact;
+    if (!exact && rows > 16 && kx_umma(s, prof, p, rows, groups)) return;
     if (!exact && rows <= 16) {
         launch_k(lin_mma16_kernel, dim3(cdiv(p.N, LIN_M16_BN), 1, groups), dim3(LIN_M16_WARPS * 32), 0, p, KC_GEMM, s, prof);
     } else if (rows <= LIN_SK_ROWS || (exact && rows <= 16)) {

@@ -4,8 +4,9 @@
 // offsets into X / Y), or the experts of a routed feed-forward (row lists built on the device).  Row counts come from device
 // memory (the step metadata, the router's per-expert counts), so a captured step graph never changes.
 //
-//   lin_tile_kernel<EXACT>   steps of many rows.  EXACT = false: bf16 operands on the tensor cores (mma.sync m16n8k16, f32
-//                            accumulate) behind a two-stage cp.async pipeline, activations rounded to bf16 when the fragments
+//   lin_umma_kernel          (linear_umma.cuh) serving precision, steps of more than 16 rows: tcgen05
+//   lin_tile_kernel<EXACT>   steps of many rows.  EXACT = false: the same problem where K or the weights' address do not allow 16-byte
+//                            boxes (K % 8 != 0): bf16 operands on the tensor cores (mma.sync m16n8k16, f32 accumulate) behind a two-stage cp.async pipeline, activations rounded to bf16 when the fragments
 //                            are built; EXACT = true: plain f32 FMA on the f32 activations (bf16 weights widen exactly), no
 //                            reduced-precision product anywhere.
 //   lin_mma16_kernel         serving precision, steps of up to 16 rows (decode): the same tensor-core product with the k range

@@ -1,9 +1,12 @@
 """Prompt steps of the RWKV path at the edges of their shapes: token counts around every tile size of the projection kernel,
 row counts of the head, sequences of unequal length, against the CPU oracle in the same operand precision."""
+import json
+
 import numpy as np
 import pytest
 
 from ai00_server_b200 import capi, runtime, synth
+from oracle import kemirax_numpy, panupel_numpy
 from oracle import rwkv_numpy as O
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +68,38 @@ def test_last_hidden_answers_the_last_portion(lens, rows):
         assert np.abs(got - want).max() <= TOL * np.abs(want).max()
     finally:
         m.close()
+
+
+# serving precision of the config.json families: bf16 operands (2^-9 each), f32 sums.  A row of a few layers is off by a few of those
+# roundings, a few percent where a norm divides by a small read-out; a wrong tile, edge or row list is off by its own size
+BF16_TOL = 5e-2
+
+
+def _check_family(make, layers, module, n, **kw):
+    cfg, st, w = make(layers, seed=4, **kw)
+    toks = np.random.default_rng(n).integers(1, 90, n).tolist()
+    m = runtime.Model(st, max_batch=1, token_chunk_size=512, config=cfg, kv_tokens=n + 64, kv_page=16)
+    try:
+        m.state.reset(0)
+        got = m.infer_raw([0], [n], toks, [capi.OPTION_FULL])[0]
+        want = module.run(json.loads(cfg), w, toks)
+        err = np.sqrt(((got - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean())
+        assert np.median(err) <= BF16_TOL and (err <= 4 * BF16_TOL).mean() >= 0.98, (n, float(np.median(err)), float(err.max()))
+    finally:
+        m.close()
+
+
+@pytest.mark.parametrize("n", [17, 32, 33, 64, 65, 127, 128, 129, 300])
+def test_projections_of_a_step_of_n_rows(n):
+    """Row tiles of 32 / 64 / 128 and their remainders, outputs and k ranges that are no multiple of a tile."""
+    L = synth.panupel_layer
+    _check_family(synth.make_panupel, [L("delta", heads=3, dim=24, ff=200), L("parallel", heads=2, dim=40, mm_heads=1, mm_dim=24, ff=72)], panupel_numpy, n,
+                  width=136)
+
+
+@pytest.mark.parametrize("n", [20, 70, 130])
+@pytest.mark.parametrize("experts, top", [(3, 1), (8, 4)])
+def test_routed_projections_of_a_step_of_n_rows(n, experts, top):
+    """Row lists of experts: groups of very unequal size, empty ones among them."""
+    layer = synth.kemirax_layer("gla", heads=2, dim=16, vdim=24, experts=experts, identity=1, top=top, ff=88, shared_ff=40)
+    _check_family(synth.make_kemirax, [layer], kemirax_numpy, n, width=72)
