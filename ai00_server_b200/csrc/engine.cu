@@ -528,11 +528,11 @@ struct b200rwkv_engine {
     std::vector<char> keep_valid;            // slot has a logits row (guarded by keep_mu)
     std::mutex keep_mu;
     cudaEvent_t step_done = nullptr;         // recorded on `stream` after every step: the sampling stream waits on it
-    float* tk_cand_x = nullptr; unsigned* tk_cand_id = nullptr; float2* tk_stats = nullptr;
-    unsigned* tk_out_id = nullptr; float* tk_out_p = nullptr;
+    uint8_t* tk_out = nullptr;         // pinned: [S][TOPK_MAX] ids, [S][TOPK_MAX] probabilities (null: vocabulary too large)
     uint8_t *tk_dev = nullptr, *tk_host = nullptr;
     size_t tk_cap = 0;
     void enqueue_keep(cudaStream_t s, int MTR);
+    void topk_setup();
     void sample_topk(int nrows, const int32_t* slots, const int32_t* pen_off, const uint32_t* pen_tok, const float* pen_val,
                      const uint32_t* allow_bits, const int32_t* bias_off, const uint32_t* bias_tok, const float* bias_val,
                      int top_k, uint32_t* ids_out, float* probs_out);
@@ -640,6 +640,7 @@ b200rwkv_engine::~b200rwkv_engine() {
     if (sm_in) cudaFree(sm_in);
     if (sm_out) cudaFree(sm_out);
     if (h_meta) cudaFreeHost(h_meta);
+    if (tk_out) cudaFreeHost(tk_out);
     if (tk_dev) cudaFree(tk_dev);
     if (tk_host) cudaFreeHost(tk_host);
     if (step_done) cudaEventDestroy(step_done);
@@ -1070,14 +1071,7 @@ void b200rwkv_engine::build(const StFile& st) {
     keep_valid.assign(S, 0);
     if (rank == 0) {
         d_keep = (float*)dalloc((size_t)S * V * 4);
-        const int nseg = cdiv(V, TOPK_SEG);
-        if (nseg <= TOPK_MAX_SEGS) {       // larger vocabularies: b200rwkv_sample_topk answers UNSUPPORTED
-            tk_cand_x = (float*)dalloc((size_t)S * nseg * TOPK_MAX * 4);
-            tk_cand_id = (unsigned*)dalloc((size_t)S * nseg * TOPK_MAX * 4);
-            tk_stats = (float2*)dalloc((size_t)S * nseg * 8);
-            tk_out_id = (unsigned*)dalloc((size_t)S * TOPK_MAX * 4);
-            tk_out_p = (float*)dalloc((size_t)S * TOPK_MAX * 4);
-        }
+        topk_setup();
     }
     for (int i = 0; i < 6; ++i) a_x[i] = a16_alloc(C);
     a_out = a16_alloc(Cl);
@@ -1828,6 +1822,12 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
     if (hidden_keep) hidden_rows = (int)total_tok;
 }
 
+void b200rwkv_engine::topk_setup() {
+    if (V > TOPK_MAX_V) return;        // larger vocabularies: b200rwkv_sample_topk answers UNSUPPORTED
+    CK(cudaMallocHost(&tk_out, (size_t)S * TOPK_MAX * 8));
+    CK(cudaFuncSetAttribute(topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TOPK_SMEM));
+}
+
 // GPU sampling front half (sample.cuh).  Runs on the softmax stream under the softmax mutex: the reference samples from the
 // task that owns softmax (run.rs:1237), concurrently with the infer task; the per-slot rows it reads are only rewritten by a
 // step that contains the slot, which the host cannot submit before this call returned the slot's token.
@@ -1835,7 +1835,7 @@ void b200rwkv_engine::sample_topk(int nrows, const int32_t* slots, const int32_t
                                   const uint32_t* allow_bits, const int32_t* bias_off, const uint32_t* bias_tok, const float* bias_val,
                                   int top_k, uint32_t* ids_out, float* probs_out) {
     REQUIRE(rank == 0, B200RWKV_ERR_INVALID, "sample_topk: only rank 0 holds the gathered logits");
-    REQUIRE(tk_cand_x, B200RWKV_ERR_UNSUPPORTED, "sample_topk: num_vocab > 65536 is not supported");
+    REQUIRE(tk_out, B200RWKV_ERR_UNSUPPORTED, "sample_topk: num_vocab > 65536 is not supported");
     REQUIRE(nrows >= 1 && nrows <= S && slots && ids_out && probs_out, B200RWKV_ERR_INVALID, "sample_topk: bad argument");
     REQUIRE(top_k >= 1 && top_k <= TOPK_MAX, B200RWKV_ERR_INVALID, "sample_topk: top_k must be in [1, 128]");
     {
@@ -1855,47 +1855,56 @@ void b200rwkv_engine::sample_topk(int nrows, const int32_t* slots, const int32_t
         REQUIRE(!pen_off || (pen_off[i] >= 0 && pen_off[i] <= pen_off[i + 1]), B200RWKV_ERR_INVALID, "sample_topk: penalty offsets must ascend");
         REQUIRE(!bias_off || (bias_off[i] >= 0 && bias_off[i] <= bias_off[i + 1]), B200RWKV_ERR_INVALID, "sample_topk: bias offsets must ascend");
     }
-    const size_t words = (size_t)(V + 31) / 32;
-    auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
-    // one staging blob: slot[n] | pen_off[n+1] | bias_off[n+1] | pen_tok | pen_val | bias_tok | bias_val | allow
-    const size_t o_slot = 0, o_po = al(o_slot + (size_t)nrows * 4), o_bo = al(o_po + (size_t)(nrows + 1) * 4),
-                 o_pt = al(o_bo + (size_t)(nrows + 1) * 4), o_pv = al(o_pt + (size_t)npen * 4), o_bt = al(o_pv + (size_t)npen * 4),
-                 o_bv = al(o_bt + (size_t)nbias * 4), o_al = al(o_bv + (size_t)nbias * 4),
-                 total = al(o_al + (allow_bits ? (size_t)nrows * words * 4 : 0));
-    if (total > tk_cap) {
-        if (tk_dev) { CK(cudaFree(tk_dev)); tk_dev = nullptr; }
-        if (tk_host) { CK(cudaFreeHost(tk_host)); tk_host = nullptr; }
-        tk_cap = 0;
-        const size_t want = std::max<size_t>(total * 2, 1 << 20);
-        CK(cudaMalloc(&tk_dev, want));
-        CK(cudaMallocHost(&tk_host, want));
-        tk_cap = want;
-    }
-    std::vector<int32_t> zeros(nrows + 1, 0);
-    memcpy(tk_host + o_slot, slots, (size_t)nrows * 4);
-    memcpy(tk_host + o_po, pen_off ? pen_off : zeros.data(), (size_t)(nrows + 1) * 4);
-    memcpy(tk_host + o_bo, bias_off ? bias_off : zeros.data(), (size_t)(nrows + 1) * 4);
-    if (npen) { memcpy(tk_host + o_pt, pen_tok, (size_t)npen * 4); memcpy(tk_host + o_pv, pen_val, (size_t)npen * 4); }
-    if (nbias) { memcpy(tk_host + o_bt, bias_tok, (size_t)nbias * 4); memcpy(tk_host + o_bv, bias_val, (size_t)nbias * 4); }
-    if (allow_bits) memcpy(tk_host + o_al, allow_bits, (size_t)nrows * words * 4);
-    CK(cudaStreamWaitEvent(sm_stream, step_done, 0));
-    CK(cudaMemcpyAsync(tk_dev, tk_host, total, cudaMemcpyHostToDevice, sm_stream));
     TopkParams tp;
     memset(&tp, 0, sizeof(tp));
-    tp.keep = d_keep; tp.V = V; tp.nseg = cdiv(V, TOPK_SEG);
-    tp.slot = (const int*)(tk_dev + o_slot);
-    tp.pen_off = (const int*)(tk_dev + o_po); tp.pen_tok = (const unsigned*)(tk_dev + o_pt); tp.pen_val = (const float*)(tk_dev + o_pv);
-    tp.bias_off = (const int*)(tk_dev + o_bo); tp.bias_tok = (const unsigned*)(tk_dev + o_bt); tp.bias_val = (const float*)(tk_dev + o_bv);
-    tp.allow = allow_bits ? (const unsigned*)(tk_dev + o_al) : nullptr;
-    tp.cand_x = tk_cand_x; tp.cand_id = tk_cand_id; tp.stats = tk_stats;
-    tp.top_k = top_k; tp.out_id = tk_out_id; tp.out_p = tk_out_p;
-    topk_segment_kernel<<<dim3(tp.nseg, nrows), TOPK_SEG_THREADS, 0, sm_stream>>>(tp);
+    tp.keep = d_keep; tp.V = V;
+    tp.top_k = top_k;
+    tp.out_id = (unsigned*)tk_out; tp.out_p = (float*)(tk_out + (size_t)nrows * top_k * 4);
+    CK(cudaStreamWaitEvent(sm_stream, step_done, 0));
+    if (npen == 0 && nbias == 0 && !allow_bits && nrows <= TOPK_INLINE) {
+        std::copy(slots, slots + nrows, tp.slot_inline);       // nothing to upload
+    } else {
+        const size_t words = (size_t)(V + 31) / 32;
+        auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
+        // one staging blob: slot[n] | pen_off[n+1] | bias_off[n+1] | pen_tok | pen_val | bias_tok | bias_val | allow
+        const size_t o_slot = 0, o_po = al(o_slot + (size_t)nrows * 4), o_bo = al(o_po + (size_t)(nrows + 1) * 4),
+                     o_pt = al(o_bo + (size_t)(nrows + 1) * 4), o_pv = al(o_pt + (size_t)npen * 4), o_bt = al(o_pv + (size_t)npen * 4),
+                     o_bv = al(o_bt + (size_t)nbias * 4), o_al = al(o_bv + (size_t)nbias * 4),
+                     total = al(o_al + (allow_bits ? (size_t)nrows * words * 4 : 0));
+        if (total > tk_cap) {
+            if (tk_dev) { CK(cudaFree(tk_dev)); tk_dev = nullptr; }
+            if (tk_host) { CK(cudaFreeHost(tk_host)); tk_host = nullptr; }
+            tk_cap = 0;
+            const size_t want = std::max<size_t>(total * 2, 1 << 20);
+            CK(cudaMalloc(&tk_dev, want));
+            CK(cudaMallocHost(&tk_host, want));
+            tk_cap = want;
+        }
+        memcpy(tk_host + o_slot, slots, (size_t)nrows * 4);
+        if (npen) {
+            memcpy(tk_host + o_po, pen_off, (size_t)(nrows + 1) * 4);
+            memcpy(tk_host + o_pt, pen_tok, (size_t)npen * 4);
+            memcpy(tk_host + o_pv, pen_val, (size_t)npen * 4);
+            tp.pen_off = (const int*)(tk_dev + o_po); tp.pen_tok = (const unsigned*)(tk_dev + o_pt); tp.pen_val = (const float*)(tk_dev + o_pv);
+        }
+        if (nbias) {
+            memcpy(tk_host + o_bo, bias_off, (size_t)(nrows + 1) * 4);
+            memcpy(tk_host + o_bt, bias_tok, (size_t)nbias * 4);
+            memcpy(tk_host + o_bv, bias_val, (size_t)nbias * 4);
+            tp.bias_off = (const int*)(tk_dev + o_bo); tp.bias_tok = (const unsigned*)(tk_dev + o_bt); tp.bias_val = (const float*)(tk_dev + o_bv);
+        }
+        if (allow_bits) {
+            memcpy(tk_host + o_al, allow_bits, (size_t)nrows * words * 4);
+            tp.allow = (const unsigned*)(tk_dev + o_al);
+        }
+        tp.slot = (const int*)(tk_dev + o_slot);
+        CK(cudaMemcpyAsync(tk_dev, tk_host, total, cudaMemcpyHostToDevice, sm_stream));
+    }
+    topk_kernel<<<dim3(TOPK_CTAS, nrows), TOPK_THREADS, TOPK_SMEM, sm_stream>>>(tp);
     CK(cudaGetLastError());
-    topk_merge_kernel<<<nrows, TOPK_MERGE_THREADS, 0, sm_stream>>>(tp);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(ids_out, tk_out_id, (size_t)nrows * top_k * 4, cudaMemcpyDeviceToHost, sm_stream));
-    CK(cudaMemcpyAsync(probs_out, tk_out_p, (size_t)nrows * top_k * 4, cudaMemcpyDeviceToHost, sm_stream));
     CK(cudaStreamSynchronize(sm_stream));
+    memcpy(ids_out, tp.out_id, (size_t)nrows * top_k * 4);
+    memcpy(probs_out, tp.out_p, (size_t)nrows * top_k * 4);
 }
 
 // API layout <-> device layout for a live slot (snap == nullptr) or a snapshot record [L][C | Hl*N*N | C]

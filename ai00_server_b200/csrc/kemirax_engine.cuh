@@ -258,16 +258,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     // ---- logits rows kept for sampling (sample.cuh) ----
     keep_valid.assign(S, 0);
     d_keep = (float*)dalloc((size_t)S * V * 4);
-    {
-        const int nseg = cdiv(V, TOPK_SEG);
-        if (nseg <= TOPK_MAX_SEGS) {
-            tk_cand_x = (float*)dalloc((size_t)S * nseg * TOPK_MAX * 4);
-            tk_cand_id = (unsigned*)dalloc((size_t)S * nseg * TOPK_MAX * 4);
-            tk_stats = (float2*)dalloc((size_t)S * nseg * 8);
-            tk_out_id = (unsigned*)dalloc((size_t)S * TOPK_MAX * 4);
-            tk_out_p = (float*)dalloc((size_t)S * TOPK_MAX * 4);
-        }
-    }
+    topk_setup();
     comm_base = (uint8_t*)d_logits; off_logits = 0;       // the keep-rows gather reads the (single) logits shard from here
     peer_base[0] = comm_base;
     connected = true;

@@ -14,28 +14,38 @@
 // reproducible.  (The reference sorts probabilities with an unstable radix sort: any order of equal probabilities is a
 // valid outcome there; this is one of them, because the probability is a non-decreasing function of the logit.)
 //
-// Shape: the vocabulary row (65536 f32 = 256 KB, L2 resident) is cut into 2048-element segments.
-//   kernel 1 (grid = segments x rows): load, apply the two sparse lists and the mask, segment max / sum-exp, bitonic sort in
-//            shared memory, keep the segment's best 128;
-//   kernel 2 (grid = rows): combine the segment statistics into the softmax denominator (fixed order), merge the 32 sorted
-//            lists pairwise -- the 128 best of two descending lists are first(a[i], b[127-i]), a bitonic sequence that seven
-//            compare-exchange stages sort -- five rounds, then probabilities of the survivors.
-// Nothing here is bandwidth: 16 rows x 256 KB from L2; two short launches.
+// Shape: one launch, a cluster of eight CTAs per row, an eighth of the row each, in registers (32 elements a thread).  Nothing here is
+// bandwidth (16 rows x 256 KB from L2); sorting every element was the cost (35-65 us for the segments' bitonic sorts, 13 us to merge).
+//   * an element and its place in the total order are one 64-bit key (ordered logit, inverted id);
+//   * the best key of every thread gives two lower bounds of the row's top_k-th key: the smallest over the CTAs of the (top_k / 8)-th best
+//     thread, and the largest over the CTAs of the top_k-th best thread.  Elements at or above the larger bound are candidates: about
+//     1.7 top_k of them for a smooth row, at most 32 top_k per CTA for any row (then the CTA keeps its own best top_k);
+//   * every CTA ranks its own candidates against all of the cluster's, read through distributed shared memory: a rank below top_k IS the
+//     output position.  Softmax statistics are combined in CTA order.
+// Results go straight to pinned host memory.  Measured at 16 rows of 65536: see the figures at topk_kernel.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace b200 {
 
 constexpr int TOPK_MAX = 128;
-constexpr int TOPK_SEG = 2048;            // elements per segment
-constexpr int TOPK_SEG_THREADS = 256;
-constexpr int TOPK_MAX_SEGS = 32;         // => num_vocab <= 65536
-constexpr int TOPK_MERGE_THREADS = 1024;
+constexpr int TOPK_CTAS = 8, TOPK_THREADS = 256;                // CTAs of a row (one cluster), threads of a CTA
+constexpr int TOPK_PER_THREAD = 32;                             // elements
+constexpr int TOPK_SLICE = TOPK_THREADS * TOPK_PER_THREAD;      // elements of a CTA: 8192
+constexpr int TOPK_MAX_V = TOPK_CTAS * TOPK_SLICE;              // 65536
+constexpr int TOPK_LIST = 4096;                                 // candidates of a CTA before it cuts them (127 threads x 32 at most)
+constexpr int TOPK_SHARE = 512;                                 // candidates a CTA may share
+constexpr int TOPK_INLINE = 64;                                 // rows whose slots travel as kernel parameters
+constexpr size_t TOPK_SMEM = (size_t)TOPK_LIST * 8 + (size_t)TOPK_CTAS * TOPK_SHARE * 8;
 
 struct TopkParams {
     const float* keep;          // [S][V] last logits row of every slot
-    int V, nseg;
-    const int* slot;            // [nrows]
+    int V;
+    const int* slot;            // [nrows] (null: slot_inline)
+    int slot_inline[TOPK_INLINE];
+    // adjustments (all null: none)
     const int* pen_off;         // [nrows + 1]
     const unsigned* pen_tok;    // logits[tok] -= val   (entries of one row have distinct tokens)
     const float* pen_val;
@@ -43,139 +53,180 @@ struct TopkParams {
     const unsigned* bias_tok;   // logits[tok] += val   (distinct tokens within a row)
     const float* bias_val;
     const unsigned* allow;      // optional [nrows][ceil(V / 32)]: bit = 1 -> token allowed; disallowed -> -inf
-    float* cand_x;              // [nrows][nseg][128]
-    unsigned* cand_id;          // [nrows][nseg][128]
-    float2* stats;              // [nrows][nseg] (max, sum exp(x - max))
     int top_k;
-    unsigned* out_id;           // [nrows][top_k]
+    unsigned* out_id;           // [nrows][top_k], pinned host memory
     float* out_p;               // [nrows][top_k]
 };
 
-// strict total order: larger logit first, then smaller id
-__device__ __forceinline__ bool cand_before(const float xa, const unsigned ia, const float xb, const unsigned ib) {
-    return xa > xb || (xa == xb && ia < ib);
+// strict total order as one number: larger logit first, then smaller id (-0 and +0 are one value); 0 is below every element
+__device__ __forceinline__ unsigned long long topk_key(float x, unsigned id) {
+    const unsigned b = __float_as_uint(x == 0.f ? 0.f : x);
+    const unsigned o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    return ((unsigned long long)o << 32) | (unsigned)~id;
+}
+__device__ __forceinline__ float topk_logit(unsigned long long key) {
+    const unsigned o = (unsigned)(key >> 32);
+    return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
 }
 
-__global__ void __launch_bounds__(TOPK_SEG_THREADS) topk_segment_kernel(const __grid_constant__ TopkParams p) {
-    __shared__ float sx[TOPK_SEG];
-    __shared__ unsigned sid[TOPK_SEG];
+// 16 rows of 65536 logits, top_k = 128 (ncu): 65 + 13 us for the two kernels before, 26 us now
+__global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS) topk_kernel(const __grid_constant__ TopkParams p) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char topk_smem[];
+    unsigned long long* const list = reinterpret_cast<unsigned long long*>(topk_smem);      // [TOPK_LIST], shared: the first TOPK_SHARE
+    unsigned long long* const all = list + TOPK_LIST;                                       // [TOPK_CTAS * TOPK_SHARE]
+    float* const sx = reinterpret_cast<float*>(topk_smem);                                  // [TOPK_SLICE] while lists are applied
+    __shared__ unsigned long long s_best[TOPK_THREADS];
+    __shared__ unsigned long long s_few, s_full;            // the (top_k / 8)-th and the top_k-th best thread
+    __shared__ float2 s_stat;                               // (max, sum exp(x - max)) of the slice
     __shared__ float red[32];
-    const int seg = blockIdx.x, row = blockIdx.y, tid = threadIdx.x;
-    const int seg0 = seg * TOPK_SEG;
-    const float* src = p.keep + (size_t)p.slot[row] * p.V;
-    const unsigned* allow = p.allow ? p.allow + (size_t)row * ((p.V + 31) / 32) : nullptr;
+    __shared__ int s_n;
+    const int cta = blockIdx.x, row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int slice = ((p.V + TOPK_CTAS - 1) / TOPK_CTAS + 3) & ~3;
+    const int lo = min(cta * slice, p.V), cnt = min(lo + slice, p.V) - lo;
+    const float* const src = p.keep + (size_t)(p.slot ? p.slot[row] : p.slot_inline[row]) * p.V + lo;
+    const bool vec = (p.V & 3) == 0;                        // rows and slices start on 16-byte boundaries
+    float x[TOPK_PER_THREAD];
 #pragma unroll
-    for (int j = 0; j < TOPK_SEG / TOPK_SEG_THREADS; ++j) {
-        const int li = tid + TOPK_SEG_THREADS * j, i = seg0 + li;
-        sx[li] = (i < p.V) ? src[i] : -INFINITY;
-        sid[li] = (i < p.V) ? (unsigned)i : 0xFFFFFFFFu;
-    }
-    __syncthreads();
-    // Sampler::transform: penalties (distinct tokens: race free)
-    for (int e = p.pen_off[row] + tid; e < p.pen_off[row + 1]; e += TOPK_SEG_THREADS) {
-        const unsigned t = p.pen_tok[e];
-        if (t >= (unsigned)seg0 && t < (unsigned)(seg0 + TOPK_SEG) && t < (unsigned)p.V) sx[t - seg0] -= p.pen_val[e];
-    }
-    __syncthreads();
-    // Formatter::transform: tokens the grammar does not allow
-    if (allow) {
+    for (int q = 0; q < TOPK_PER_THREAD / 4; ++q) {
+        const int i = (q * TOPK_THREADS + tid) * 4;
+        if (vec && i + 3 < cnt) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + i));
+            x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < TOPK_SEG / TOPK_SEG_THREADS; ++j) {
-            const int li = tid + TOPK_SEG_THREADS * j, i = seg0 + li;
-            if (i < p.V && !((allow[i >> 5] >> (i & 31)) & 1u)) sx[li] = -INFINITY;
+            for (int e = 0; e < 4; ++e) x[4 * q + e] = i + e < cnt ? __ldcg(src + i + e) : -INFINITY;
+        }
+    }
+    auto index = [&](int j) { return ((j >> 2) * TOPK_THREADS + tid) * 4 + (j & 3); };      // place of x[j] in the slice
+    if (p.pen_off || p.bias_off || p.allow) {
+#pragma unroll
+        for (int j = 0; j < TOPK_PER_THREAD; ++j) sx[index(j)] = x[j];
+        __syncthreads();
+        auto apply = [&](const int* off, const unsigned* tok, const float* val, const float sign) {
+            for (int e = off[row] + tid; e < off[row + 1]; e += TOPK_THREADS) {
+                const int i = (int)tok[e] - lo;
+                if (tok[e] < (unsigned)p.V && i >= 0 && i < cnt) sx[i] = fmaf(sign, val[e], sx[i]);
+            }
+        };
+        // Sampler::transform (penalties), Formatter::transform (tokens the grammar does not allow), bias: in this order
+        if (p.pen_off) apply(p.pen_off, p.pen_tok, p.pen_val, -1.f);
+        __syncthreads();
+        if (p.allow) {
+            const unsigned* allow = p.allow + (size_t)row * ((p.V + 31) / 32);
+            for (int i = tid; i < cnt; i += TOPK_THREADS)
+                if (!((allow[(lo + i) >> 5] >> ((lo + i) & 31)) & 1u)) sx[i] = -INFINITY;
         }
         __syncthreads();
-    }
-    // bias
-    for (int e = p.bias_off[row] + tid; e < p.bias_off[row + 1]; e += TOPK_SEG_THREADS) {
-        const unsigned t = p.bias_tok[e];
-        if (t >= (unsigned)seg0 && t < (unsigned)(seg0 + TOPK_SEG) && t < (unsigned)p.V) sx[t - seg0] += p.bias_val[e];
-    }
-    __syncthreads();
-    // segment statistics of the softmax
-    float mx = -INFINITY;
+        if (p.bias_off) apply(p.bias_off, p.bias_tok, p.bias_val, 1.f);
+        __syncthreads();
 #pragma unroll
-    for (int j = 0; j < TOPK_SEG / TOPK_SEG_THREADS; ++j) mx = fmaxf(mx, sx[tid + TOPK_SEG_THREADS * j]);
+        for (int j = 0; j < TOPK_PER_THREAD; ++j) x[j] = sx[index(j)];
+    }
+    // softmax statistics of the slice, best key of the thread
+    float mx = -INFINITY;
+    unsigned long long best = 0;
+#pragma unroll
+    for (int j = 0; j < TOPK_PER_THREAD; ++j) {
+        const int i = index(j);
+        if (i < cnt) {
+            mx = fmaxf(mx, x[j]);
+            best = max(best, topk_key(x[j], (unsigned)(lo + i)));
+        }
+    }
+    s_best[tid] = best;
+    if (tid == 0) { s_few = 0; s_full = 0; s_n = 0; }
     mx = block_max_any(mx, red);
-    float s = 0.f;
+    float sum = 0.f;
     if (mx > -INFINITY) {
 #pragma unroll
-        for (int j = 0; j < TOPK_SEG / TOPK_SEG_THREADS; ++j) s += expf(sx[tid + TOPK_SEG_THREADS * j] - mx);
+        for (int j = 0; j < TOPK_PER_THREAD; ++j)
+            if (index(j) < cnt) sum += expf(x[j] - mx);
     }
-    s = block_sum_any(s, red);
-    if (tid == 0) p.stats[(size_t)row * p.nseg + seg] = make_float2(mx, s);
-    // bitonic sort, best first
-    for (int k = 2; k <= TOPK_SEG; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            __syncthreads();
+    sum = block_sum_any(sum, red);                          // (its barriers also publish s_best)
+    if (tid == 0) s_stat = make_float2(mx, sum);
+    int above = 0;
+    for (int i = 0; i < TOPK_THREADS; ++i) above += s_best[i] > best;
+    if (best && above == (p.top_k + TOPK_CTAS - 1) / TOPK_CTAS - 1) s_few = best;
+    if (best && above == p.top_k - 1) s_full = best;
+    cluster.sync();
+    unsigned long long few = ~0ull, full = 0;
+    float M = -INFINITY;
+    for (int c = 0; c < TOPK_CTAS; ++c) {
+        few = min(few, *cluster.map_shared_rank(&s_few, c));
+        full = max(full, *cluster.map_shared_rank(&s_full, c));
+        M = fmaxf(M, cluster.map_shared_rank(&s_stat, c)->x);
+    }
+    const unsigned long long bound = max(max(few, full), 1ull);
+    // candidates of the slice -> list, in any order
+    int mine = 0;
 #pragma unroll
-            for (int q = 0; q < TOPK_SEG / 2 / TOPK_SEG_THREADS; ++q) {
-                const int t = tid + TOPK_SEG_THREADS * q;            // compare-exchange index 0 .. 1023
-                const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)); // lower element of the pair
-                const int l = i | j;
-                const bool up = (i & k) == 0;                         // this block sorts best-first
-                const float xa = sx[i], xb = sx[l];
-                const unsigned ia = sid[i], ib = sid[l];
-                const bool a_first = cand_before(xa, ia, xb, ib);
-                if (a_first != up) { sx[i] = xb; sx[l] = xa; sid[i] = ib; sid[l] = ia; }
-            }
+    for (int j = 0; j < TOPK_PER_THREAD; ++j) mine += index(j) < cnt && topk_key(x[j], (unsigned)(lo + index(j))) >= bound;
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+    }
+    int wbase = 0;
+    if (lane == 31 && at) wbase = atomicAdd(&s_n, at);
+    at += __shfl_sync(0xffffffffu, wbase, 31) - mine;
+    if (mine) {
+#pragma unroll
+        for (int j = 0; j < TOPK_PER_THREAD; ++j) {
+            const unsigned long long key = topk_key(x[j], (unsigned)(lo + index(j)));
+            if (index(j) < cnt && key >= bound) list[at++] = key;
         }
     }
     __syncthreads();
-    if (tid < TOPK_MAX) {
-        const size_t o = ((size_t)row * p.nseg + seg) * TOPK_MAX + tid;
-        p.cand_x[o] = sx[tid];
-        p.cand_id[o] = sid[tid];
-    }
-}
-
-__global__ void __launch_bounds__(TOPK_MERGE_THREADS) topk_merge_kernel(const __grid_constant__ TopkParams p) {
-    __shared__ float sx[TOPK_MAX_SEGS * TOPK_MAX];
-    __shared__ unsigned sid[TOPK_MAX_SEGS * TOPK_MAX];
-    __shared__ float s_m, s_inv;
-    const int row = blockIdx.x, tid = threadIdx.x;
-    for (int i = tid; i < TOPK_MAX_SEGS * TOPK_MAX; i += TOPK_MERGE_THREADS) {
-        const int sg = i / TOPK_MAX;
-        const bool ok = sg < p.nseg;
-        const size_t o = ((size_t)row * p.nseg + sg) * TOPK_MAX + (i % TOPK_MAX);
-        sx[i] = ok ? p.cand_x[o] : -INFINITY;
-        sid[i] = ok ? p.cand_id[o] : 0xFFFFFFFFu;
-    }
-    if (tid < 32) {
-        // softmax denominator from the segment statistics, fixed order (lane = segment, xor tree)
-        const float2 st = (tid < p.nseg) ? p.stats[(size_t)row * p.nseg + tid] : make_float2(-INFINITY, 0.f);
-        const float M = warp_max(st.x);
-        float sc = (st.x > -INFINITY) ? st.y * expf(st.x - M) : 0.f;
-        sc = warp_sum(sc);
-        if (tid == 0) { s_m = M; s_inv = 1.0f / sc; }
-    }
-    // five merge rounds: lists a = 2 p s, b = (2 p + 1) s -> a
-    for (int s = 1; s < TOPK_MAX_SEGS; s <<= 1) {
-        const int npair = TOPK_MAX_SEGS / (2 * s);
+    int n = s_n;
+    if (n > TOPK_SHARE) {                                   // a row whose best elements sit in few threads: the CTA's own best top_k
+        unsigned long long key[TOPK_LIST / TOPK_THREADS];
+        int rank[TOPK_LIST / TOPK_THREADS];
+        for (int u = 0; u < TOPK_LIST / TOPK_THREADS; ++u) {
+            const int i = tid + u * TOPK_THREADS;
+            key[u] = i < n ? list[i] : 0;
+            rank[u] = 0;
+            for (int k = 0; k < n && i < n; ++k) rank[u] += list[k] > key[u];
+        }
         __syncthreads();
-        for (int t = tid; t < npair * TOPK_MAX; t += TOPK_MERGE_THREADS) {
-            const int pr = t / TOPK_MAX, i = t % TOPK_MAX;
-            const int a = (2 * pr) * s * TOPK_MAX + i, b = (2 * pr + 1) * s * TOPK_MAX + (TOPK_MAX - 1 - i);
-            if (!cand_before(sx[a], sid[a], sx[b], sid[b])) { sx[a] = sx[b]; sid[a] = sid[b]; }
-        }
-        for (int j = TOPK_MAX / 2; j > 0; j >>= 1) {
-            __syncthreads();
-            for (int t = tid; t < npair * (TOPK_MAX / 2); t += TOPK_MERGE_THREADS) {
-                const int pr = t / (TOPK_MAX / 2), u = t % (TOPK_MAX / 2);
-                const int i = (2 * pr) * s * TOPK_MAX + (((u & ~(j - 1)) << 1) | (u & (j - 1)));
-                const int l = i + j;
-                const float xa = sx[i], xb = sx[l];
-                const unsigned ia = sid[i], ib = sid[l];
-                if (!cand_before(xa, ia, xb, ib)) { sx[i] = xb; sx[l] = xa; sid[i] = ib; sid[l] = ia; }
-            }
+        for (int u = 0; u < TOPK_LIST / TOPK_THREADS; ++u)
+            if (tid + u * TOPK_THREADS < n && rank[u] < p.top_k) list[rank[u]] = key[u];
+        n = p.top_k;
+        __syncthreads();
+        if (tid == 0) s_n = n;
+    }
+    cluster.sync();
+    int total = 0;
+    float denom = 0.f;
+    for (int c = 0; c < TOPK_CTAS; ++c) {
+        const int nc = *cluster.map_shared_rank(&s_n, c);
+        const unsigned long long* from = cluster.map_shared_rank(list, c);
+        for (int i = tid; i < nc; i += TOPK_THREADS) all[total + i] = from[i];
+        total += nc;
+        const float2 st = *cluster.map_shared_rank(&s_stat, c);
+        if (st.x > -INFINITY) denom += st.y * expf(st.x - M);
+    }
+    cluster.sync();                                         // every CTA has read the others: they may leave
+    const float inv = 1.0f / denom;
+    for (int i = warp; i < n; i += TOPK_THREADS / 32) {
+        const unsigned long long key = list[i];
+        int rank = 0;
+        for (int k = lane; k < total; k += 32) rank += all[k] > key;
+        rank = __reduce_add_sync(0xffffffffu, rank);
+        if (lane == 0 && rank < p.top_k) {
+            // same expression as softmax_kernel (misc.cuh): exp(x - max) * (1 / sum)
+            const float v = topk_logit(key);
+            p.out_id[(size_t)row * p.top_k + rank] = ~(unsigned)key;
+            p.out_p[(size_t)row * p.top_k + rank] = v > -INFINITY ? expf(v - M) * inv : 0.f;
         }
     }
-    __syncthreads();
-    if (tid < p.top_k) {
-        // same expression as softmax_kernel (misc.cuh): exp(x - max) * (1 / sum)
-        p.out_id[(size_t)row * p.top_k + tid] = sid[tid];
-        p.out_p[(size_t)row * p.top_k + tid] = (sx[tid] > -INFINITY) ? expf(sx[tid] - s_m) * s_inv : 0.f;
-    }
+    if (cta == 0)
+        for (int i = p.V + tid; i < p.top_k; i += TOPK_THREADS) {       // a vocabulary smaller than top_k
+            p.out_id[(size_t)row * p.top_k + i] = 0xFFFFFFFFu;
+            p.out_p[(size_t)row * p.top_k + i] = 0.f;
+        }
 }
 
 // ---------------------------------------------------------------------------------------
