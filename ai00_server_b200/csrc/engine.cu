@@ -625,6 +625,7 @@ struct b200rwkv_engine {
                   const std::vector<int>& outmode /*0 none,1 last,2 full*/, int* R_out);
     void infer(int nslot, const int32_t* slot, const int32_t* ntok, const uint32_t* tokens, const int32_t* option,
                float* logits_out, size_t cap, int32_t* rows_out);
+    void slot_xfer(const std::vector<SlotSeg>& segs, float* rec, int mode, const int* table = nullptr, int page = 1);
     void state_xform(int slot, bool import, float* snap = nullptr);
 };
 
@@ -1907,6 +1908,25 @@ void b200rwkv_engine::sample_topk(int nrows, const int32_t* slots, const int32_t
     memcpy(probs_out, tp.out_p, (size_t)nrows * top_k * 4);
 }
 
+// runs of a slot's memory <-> record (or zero), SLOT_SEGS runs to a launch
+void b200rwkv_engine::slot_xfer(const std::vector<SlotSeg>& segs, float* rec, int mode, const int* table, int page) {
+    for (size_t i = 0; i < segs.size(); i += SLOT_SEGS) {
+        const size_t n = std::min<size_t>(SLOT_SEGS, segs.size() - i);
+        SlotXfer x;
+        memset(&x, 0, sizeof(x));
+        x.rec = rec; x.mode = mode; x.table = table; x.page = page;
+        long long most = 0;
+        for (size_t j = 0; j < n; ++j) {
+            x.seg[j] = segs[i + j];
+            most = std::max(most, (long long)segs[i + j].cnt * segs[i + j].nl);
+        }
+        // four 16-byte accesses a thread, at most two CTAs per SM and run
+        const int grid = (int)std::max<long long>(1, std::min<long long>((most + 4095) / 4096, 2 * num_sms));
+        slot_xfer_kernel<<<dim3(grid, (unsigned)n), SLOT_THREADS, 0, stream>>>(x);
+        CK(cudaGetLastError());
+    }
+}
+
 // API layout <-> device layout for a live slot (snap == nullptr) or a snapshot record [L][C | Hl*N*N | C]
 void b200rwkv_engine::state_xform(int slot, bool import, float* snap) {
     StateXform x;
@@ -2281,17 +2301,13 @@ static int32_t rank_state_back(b200rwkv_engine* e, int32_t slot, float* out) {
 }
 
 // device-side snapshot: [L][C | Hl*N*N | C]
+static std::vector<SlotSeg> rwkv_slot_segs(const b200rwkv_engine* e, int slot) {
+    const long long C = e->C, W = (long long)e->Hl * e->N * e->N, S = e->S, rec = 2 * C + W;
+    return {{e->att_shift + slot * C, S * C, 0, rec, (int)C, e->L}, {e->wkv_state + slot * W, S * W, C, rec, (int)W, e->L},
+            {e->ffn_shift + slot * C, S * C, C + W, rec, (int)C, e->L}};
+}
 static void snapshot_copy(b200rwkv_engine* e, int slot, float* buf, bool to_snapshot) {
-    const size_t C = e->C, W = (size_t)e->Hl * e->N * e->N, S = e->S, L = e->L;
-    const size_t rec = 2 * C + W;
-    struct Part { float* dev; size_t width; size_t off; };
-    Part parts[3] = {{e->att_shift + (size_t)slot * C, C, 0}, {e->wkv_state + (size_t)slot * W, W, C}, {e->ffn_shift + (size_t)slot * C, C, C + W}};
-    for (auto& p : parts) {
-        if (to_snapshot)
-            CK(cudaMemcpy2DAsync(buf + p.off, rec * 4, p.dev, S * p.width * 4, p.width * 4, L, cudaMemcpyDeviceToDevice, e->stream));
-        else
-            CK(cudaMemcpy2DAsync(p.dev, S * p.width * 4, buf + p.off, rec * 4, p.width * 4, L, cudaMemcpyDeviceToDevice, e->stream));
-    }
+    e->slot_xfer(rwkv_slot_segs(e, slot), buf, to_snapshot ? SLOT_EXPORT : SLOT_IMPORT);
 }
 
 // allocate a snapshot record (+ a logits row when this rank keeps them)
@@ -2351,8 +2367,9 @@ static int32_t rank_state_write(b200rwkv_engine* e, int32_t slot, uint64_t snaps
     else snapshot_copy(e, slot, it->second.buf, false);
     if (e->d_keep && it->second.logits)
         CK(cudaMemcpyAsync(e->d_keep + (size_t)slot * e->V, it->second.logits, (size_t)e->V * 4, cudaMemcpyDeviceToDevice, e->stream));
+    // nothing of the caller's is in flight: later steps follow on the stream, samplers wait for the event, and the record's memory is
+    // given back by cudaFree, which waits for the device
     CK(cudaEventRecord(e->step_done, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
     {
         std::lock_guard<std::mutex> lk2(e->keep_mu);
         e->keep_valid[slot] = (e->d_keep && it->second.logits) ? 1 : 0;
@@ -3151,15 +3168,14 @@ static int32_t rank_state_reset(b200rwkv_engine* e, int32_t slot) {
     API_BEGIN(e)
     REQUIRE(e, B200RWKV_ERR_INVALID, "null engine");
     REQUIRE(slot >= 0 && slot < e->S, B200RWKV_ERR_STATE, "slot out of range");
-    if (!e->kx) {
-        std::vector<float> init(e->api_state_floats(), 0.f);
-        if (!e->init_state.empty()) init = e->init_state;
-        return rank_state_load(e, slot, init.data());
-    }
+    if (!e->kx && !e->init_state.empty()) return rank_state_load(e, slot, e->init_state.data());
     std::lock_guard<std::mutex> lk(e->mu);
     CK(cudaSetDevice(e->dev));
+    if (!e->kx) {
+        e->slot_xfer(rwkv_slot_segs(e, slot), nullptr, SLOT_ZERO);
+        return B200RWKV_OK;
+    }
     e->kx_reset(slot);
-    CK(cudaStreamSynchronize(e->stream));
     std::lock_guard<std::mutex> lk2(e->keep_mu);
     e->keep_valid[slot] = 0;
     API_END

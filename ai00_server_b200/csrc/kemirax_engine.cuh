@@ -642,19 +642,6 @@ void b200rwkv_engine::kx_release(int slot) {
     m.pos[slot] = 0;
 }
 
-struct KxRowsParams { float* flat; float* cache; const int* table; int page, D, n; bool to_cache; };
-
-__global__ void kx_cache_rows_kernel(const KxRowsParams p) {
-    const int j = blockIdx.x;
-    if (j >= p.n) return;
-    float* c = p.cache + ((size_t)p.table[j / p.page] * p.page + j % p.page) * p.D;
-    float* f = p.flat + (size_t)j * p.D;
-    for (int d = threadIdx.x; d < p.D; d += blockDim.x) {
-        if (p.to_cache) c[d] = f[d];
-        else f[d] = c[d];
-    }
-}
-
 // export (import = false): slot -> record with `ctx_rows` cache rows per layer; import: record holding `n` tokens -> slot
 void b200rwkv_engine::kx_xfer(int slot, float* rec, int ctx_rows, bool import, int n) {
     SeqModel& m = *kx;
@@ -664,30 +651,32 @@ void b200rwkv_engine::kx_xfer(int slot, float* rec, int ctx_rows, bool import, i
         const int want = cdiv(n, m.page);
         REQUIRE((size_t)want <= m.free_pages.size(), B200RWKV_ERR_STATE, "attention cache is full");
         for (int i = 0; i < want; ++i) { m.pages[slot].push_back(m.free_pages.back()); m.free_pages.pop_back(); }
-        if (want > 0) CK(cudaMemcpyAsync(m.d_table + (size_t)slot * m.npages, m.pages[slot].data(), (size_t)want * 4, cudaMemcpyHostToDevice, stream));
-        CK(cudaStreamSynchronize(stream));                  // the pageable source above is read by now
+        for (int i = 0; i < want; i += SLOT_PAGES) {            // page numbers travel as kernel parameters
+            SlotPages sp;
+            sp.dst = m.d_table + (size_t)slot * m.npages + i;
+            sp.n = std::min(SLOT_PAGES, want - i);
+            std::copy_n(m.pages[slot].data() + i, sp.n, sp.page);
+            slot_pages_kernel<<<1, SLOT_PAGES, 0, stream>>>(sp);
+            CK(cudaGetLastError());
+        }
         m.pos[slot] = n;
     } else {
         n = m.pos[slot];
         REQUIRE(n <= ctx_rows, B200RWKV_ERR_STATE, "sequence is longer than the state tensor's cache rows");
     }
-    size_t o = 4;
-    auto copy = [&](float* dev, size_t cnt) {
-        if (import) CK(cudaMemcpyAsync(dev, rec + o, cnt * 4, cudaMemcpyDeviceToDevice, stream));
-        else CK(cudaMemcpyAsync(rec + o, dev, cnt * 4, cudaMemcpyDeviceToDevice, stream));
-        o += cnt;
-    };
+    std::vector<SlotSeg> segs;
+    long long o = 4;
     for (KxLayer& l : m.layers) {
-        for (const KxLayer::Block& b : l.fixed) copy(b.base + (size_t)slot * b.per_slot, b.per_slot);
+        for (const KxLayer::Block& b : l.fixed) {
+            if (b.per_slot) segs.push_back({b.base + (size_t)slot * b.per_slot, (long long)b.per_slot, o, (long long)b.per_slot, (int)b.per_slot, 1});
+            o += (long long)b.per_slot;
+        }
         if (l.cache_D > 0) {
-            if (n > 0) {
-                KxRowsParams rp{rec + o, l.cache, m.d_table + (size_t)slot * m.npages, m.page, l.cache_D, n, import};
-                kx_cache_rows_kernel<<<n, 128, 0, stream>>>(rp);
-                CK(cudaGetLastError());
-            }
-            o += (size_t)ctx_rows * l.cache_D;
+            if (n > 0) segs.push_back({l.cache, 0, o, l.cache_D, (int)l.cache_D, n});
+            o += (long long)ctx_rows * l.cache_D;
         }
     }
+    slot_xfer(segs, rec, import ? SLOT_IMPORT : SLOT_EXPORT, m.d_table + (size_t)slot * m.npages, m.page);
     if (import && m.cfg.family == KX_FAMILY_PASOPEL) ps_repool(slot, n);      // block means are derived from the cache rows
 }
 
@@ -708,7 +697,9 @@ static void kx_relayout(const SeqModel& m, const float* src, int src_rows, float
 void b200rwkv_engine::kx_reset(int slot) {
     SeqModel& m = *kx;
     kx_release(slot);
+    std::vector<SlotSeg> segs;
     for (KxLayer& l : m.layers)
         for (const KxLayer::Block& b : l.fixed)
-            if (b.per_slot) CK(cudaMemsetAsync(b.base + (size_t)slot * b.per_slot, 0, b.per_slot * 4, stream));
+            if (b.per_slot) segs.push_back({b.base + (size_t)slot * b.per_slot, (long long)b.per_slot, 0, (long long)b.per_slot, (int)b.per_slot, 1});
+    slot_xfer(segs, nullptr, SLOT_ZERO);
 }

@@ -23,6 +23,55 @@ __global__ void __launch_bounds__(1024) softmax_kernel(const float* __restrict__
 }
 
 // ---------------------------------------------------------------------------------------
+// Sequence memory of one slot <-> a flat record on the device, or zero, in one launch: up to SLOT_SEGS runs of floats, each `nl` pieces of
+// `cnt` floats (layers of a state array, or rows of an attention cache behind the slot's page-table row).
+// A prefix-cache hit is this launch and nothing else; it was three strided copies (RWKV) or a copy per block and layer and a host
+// synchronisation (30-78 us per slot), and an empty sequence was a zero state tensor uploaded from the host (0.5 ms per slot).
+// ---------------------------------------------------------------------------------------
+struct SlotSeg {
+    float* dev;
+    long long dev_ls;        // floats between pieces on the device side (0: cache rows, placed by the page table)
+    long long off, rec_ls;   // first float in the record, floats between pieces there
+    int cnt, nl;
+};
+constexpr int SLOT_SEGS = 24, SLOT_THREADS = 256;
+enum SlotMode { SLOT_EXPORT, SLOT_IMPORT, SLOT_ZERO };
+struct SlotXfer {
+    float* rec;
+    int mode, page;
+    const int* table;        // page-table row of the slot
+    SlotSeg seg[SLOT_SEGS];
+};
+
+__global__ void __launch_bounds__(SLOT_THREADS) slot_xfer_kernel(const __grid_constant__ SlotXfer p) {
+    const SlotSeg& s = p.seg[blockIdx.y];
+    auto move = [&](auto vec_t) {
+        using T = decltype(vec_t);
+        constexpr int V = sizeof(T) / 4;
+        const int per = s.cnt / V, total = per * s.nl;
+        for (int i = blockIdx.x * SLOT_THREADS + threadIdx.x; i < total; i += gridDim.x * SLOT_THREADS) {
+            const int l = i / per, e = i - l * per;
+            const size_t at = s.dev_ls ? (size_t)l * s.dev_ls : ((size_t)p.table[l / p.page] * p.page + l % p.page) * s.cnt;
+            T* const d = reinterpret_cast<T*>(s.dev + at) + e;
+            if (p.mode == SLOT_ZERO) { *d = T{}; continue; }
+            T* const r = reinterpret_cast<T*>(p.rec + s.off + (size_t)l * s.rec_ls) + e;
+            if (p.mode == SLOT_IMPORT) *d = *r;
+            else *r = *d;
+        }
+    };
+    const bool vec = (s.cnt & 3) == 0 && (s.dev_ls & 3) == 0 && (s.off & 3) == 0 && (s.rec_ls & 3) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(s.dev) | reinterpret_cast<uintptr_t>(p.rec)) & 15) == 0;
+    if (vec) move(float4{});
+    else move(float{});
+}
+
+constexpr int SLOT_PAGES = 128;
+struct SlotPages { int* dst; int n; int page[SLOT_PAGES]; };
+__global__ void slot_pages_kernel(const __grid_constant__ SlotPages p) {
+    if (threadIdx.x < p.n) p.dst[threadIdx.x] = p.page[threadIdx.x];
+}
+
+// ---------------------------------------------------------------------------------------
 // State import / export between the API layout and the device layout.
 // API (web-rwkv shape [C, N+2, L, 1], x fastest; reference run.rs:987, lib.rs:267-272;
 // SURVEY.md App. C) per slot: api[l][row][c], row 0 = time-mix shift, rows 1..N = WKV with
