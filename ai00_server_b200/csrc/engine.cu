@@ -385,7 +385,8 @@ struct GemmLaunch {
     GemmParams p;
     int grid = 0;
     int grid_wide = 0;         // grid of steps with more than 64 tokens (see make_launch)
-    bool short_k = false;      // every tile is one block long: gemm_wide.cuh's SHORT form
+    bool short_k = false;      // every tile is one block long: gemm_wide.cuh's SHORT form,
+    int short_parts = 1;       // with this many CTAs to a tile
     bool by_tile = false;      // that grid's CTAs own whole tiles
     int max_contrib = 1, max_contrib_wide = 1;      // CTAs that can share a tile, per grid
     int total_tiles = 0;
@@ -838,12 +839,16 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
     }
     // Steps of more than 64 tokens (gemm_wide.cuh): a partial accumulator tile is 64 / 128 KB, so launches that put at least half
     // of the SMs to work give every CTA whole tiles, in rounds of equal length; the low-rank launches (2-20 tiles of a long k)
-    // cut their block sequence over the SMs, at least four blocks per CTA (3 CTAs and 68 us for 320 x 4096 at 128 tokens before).
+    // cut their block sequence over the SMs, at least ten blocks per CTA (adding a contributor's 64 / 128 KB costs about five blocks;
+    // 3 CTAs and 68 us for 320 x 4096 at 128 tokens in the decode kernel's whole-tile grid).
     if (qtype == QT_NONE) {
         g.by_tile = tile * 2 >= num_sms;
-        g.grid_wide = g.by_tile ? cdiv(tile, cdiv(tile, num_sms)) : std::min(blk, std::max(tile, std::min(num_sms, cdiv(blk, 4))));
+        g.grid_wide = g.by_tile ? cdiv(tile, cdiv(tile, num_sms)) : std::min(blk, std::max(tile, std::min(num_sms, cdiv(blk, 10))));
         g.short_k = kbmax == 1;
-        if (g.short_k) g.grid_wide = std::min(tile, 2 * num_sms);
+        if (g.short_k) {
+            g.short_parts = tile <= num_sms / 2 ? 4 : (tile <= num_sms ? 2 : 1);
+            g.grid_wide = std::min(tile, 2 * num_sms / g.short_parts);
+        }
         if (g.grid_wide == tile || g.short_k) g.by_tile = true;
     } else {
         g.grid_wide = g.grid;
@@ -927,7 +932,7 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
     auto launch_wide = [&](void (*kern)(GemmParams, int, int), size_t smem, bool wide) {
         GemmParams p = g.p;
         p.max_contrib = wide ? g.max_contrib_wide : g.max_contrib;
-        launch_k(kern, dim3(wide ? g.grid_wide : g.grid), dim3(WIDE_THREADS), smem, p, KC_GEMM, s, prof, (int)(wide && g.by_tile), g.total_tiles);
+        launch_k(kern, dim3(wide ? g.grid_wide : g.grid, wide && g.short_k ? g.short_parts : 1), dim3(WIDE_THREADS), smem, p, KC_GEMM, s, prof, (int)(wide && g.by_tile), g.total_tiles);
     };
     // RING 2 = one stage less than fits, so the small kernels around a projection can share its SMs (findings r1 §7)
     switch (MT) {
@@ -1008,6 +1013,7 @@ void b200rwkv_engine::build(const StFile& st) {
         CK(cudaFuncSetAttribute(wkv_kernel<6, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
         CK(cudaFuncSetAttribute(wkv_kernel<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
     }
+    CK(cudaFuncSetAttribute(ln_mix_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (LN_ROWS + 1) * C * 4));
     if (precision == 1) split_act = true;         // f32-activation mode (web-rwkv `Bundle::<f32>`): no activation is rounded to f16
     if (const char* v = dbg_env("B200RWKV_PREFETCH_BLOCKS")) prefetch_blocks = std::max(0, atoi(v));
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;
@@ -1513,6 +1519,8 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             launch_cluster = PRE_CLUSTER;
             if (split_on) launch_k(ln_mix_cluster_kernel<true>, dim3(PRE_GRID), dim3(PRE_THREADS), 0, lp, KC_LN, s, prof);
             else launch_k(ln_mix_cluster_kernel<false>, dim3(PRE_GRID), dim3(PRE_THREADS), 0, lp, KC_LN, s, prof);
+        } else if (MT >= 2) {
+            launch_k(ln_mix_rows_kernel, dim3(rows / LN_ROWS), dim3(LN_ROWS_THREADS), (size_t)(LN_ROWS + 1) * C * 4, lp, KC_LN, s, prof);
         } else {
             launch_k(ln_mix_kernel, dim3(rows), dim3(LN_THREADS), 0, lp, KC_LN, s, prof);
         }

@@ -29,7 +29,7 @@ constexpr int WIDE_KS = 64;                                 // k per stage
 constexpr int WIDE_STAGE_BUDGET = 204800;
 
 // SHORT: launches whose tiles are one block long (second low-rank stages) are all epilogue: a ring of one block and a single
-// accumulator, so that two CTAs share an SM and one tile's operand loads hide behind the other's
+// accumulator, so that two CTAs share an SM, and up to four CTAs share the token groups of a tile
 template <int MT, bool SHORT = false>
 struct WideCfg {
     static constexpr int W_BYTES = GEMM_BN * WIDE_KS * 2;   // 16 KB
@@ -183,7 +183,9 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
         const int nrows = *p.nrows;
         const int grp = warp >> 2, row = tid & (GEMM_BN - 1);
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        constexpr int P = Cfg::PAIR, NG = MT / 2;               // groups of this warp: mt = grp + 2 i, i < NG
+        constexpr int P = Cfg::PAIR;                            // 16-token groups of this warp: mt = grp + 2 i, i in [i0, i1)
+        // gridDim.y CTAs share a tile of a SHORT launch: each multiplies all tokens and finishes its share of them
+        const int i0 = blockIdx.y * (MT / 2) / gridDim.y, i1 = (blockIdx.y + 1) * (MT / 2) / gridDim.y;
         unsigned segcount = 0;
         SegWalk w;
         for (w.init(p, b0, b1); !w.done(); w.next(), ++segcount) {
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
             if (ncontrib > 1) {
                 float* const mine = ws0 + (size_t)(cta - c_first) * (GEMM_BN * 16 * MT);
 #pragma unroll 1
-                for (int i = 0; i < NG; ++i) {
+                for (int i = i0; i < i1; ++i) {
                     const int mt = grp + 2 * i;
                     float v[16];
                     tc_ld16(tm + mt * 16, v);
@@ -234,34 +236,45 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
             const float bias = (row_ok && sg.bias) ? sg.bias[n] : 0.f;
             const float mu = (lerp && row_ok) ? sg.aux2[n] : 0.f;
             const int mmax = min(nrows, MT * 16);
-            // one pair of 16-token groups: accumulators (TMEM, or the parts in contributor order)
-            auto load = [&](const int mt, float (&v)[16]) {
-                if (ncontrib == 1) { tc_ld16(tm + mt * 16, v); return; }
+            // the 16-token groups i .. i + P - 1: accumulators (TMEM, or the parts in contributor order, all loads of two contributors in flight)
+            auto load = [&](const int i, float (&v)[P][16]) {
+                if (SHORT || ncontrib == 1) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = 0.f;
-                for (int s0 = 0; s0 < ncontrib; s0 += 4) {              // fixed order; four contributors' loads in flight
-                    float4 q[4][4];
+                    for (int q = 0; q < P; ++q) tc_ld16(tm + (grp + 2 * (i + q)) * 16, v[q]);
+                    return;
+                }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float* src = ws0 + (size_t)(s0 + u) * (GEMM_BN * 16 * MT) + (size_t)(mt * 4) * (GEMM_BN * 4);
+                for (int q = 0; q < P; ++q)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            q[u][j] = s0 + u < ncontrib ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)j * (GEMM_BN * 4))) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
+                    for (int j = 0; j < 16; ++j) v[q][j] = 0.f;
+                for (int s0 = 0; s0 < ncontrib; s0 += 2) {
+                    float4 x[2][P][4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < 2; ++u)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) { v[4 * j] += q[u][j].x; v[4 * j + 1] += q[u][j].y; v[4 * j + 2] += q[u][j].z; v[4 * j + 3] += q[u][j].w; }
+                        for (int q = 0; q < P; ++q) {
+                            const float* src = ws0 + (size_t)(s0 + u) * (GEMM_BN * 16 * MT) + (size_t)((grp + 2 * (i + q)) * 4) * (GEMM_BN * 4);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                x[u][q][j] = s0 + u < ncontrib ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)j * (GEMM_BN * 4))) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int q = 0; q < P; ++q)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                v[q][4 * j] += x[u][q][j].x; v[q][4 * j + 1] += x[u][q][j].y; v[q][4 * j + 2] += x[u][q][j].z; v[q][4 * j + 3] += x[u][q][j].w;
+                            }
                 }
             };
             auto body = [&](auto act_c) {
                 constexpr int ACT_C = decltype(act_c)::value;
 #pragma unroll 1
-                for (int i = 0; i < NG; i += P) {
+                for (int i = i0; i < i1; i += P) {
                     float v[P][16];
-#pragma unroll
-                    for (int q = 0; q < P; ++q) load(grp + 2 * (i + q), v[q]);
-                    if (ncontrib == 1 && i + P >= NG) drained();
+                    load(i, v);
+                    if (ncontrib == 1 && i + P >= i1) drained();
                     if (out_mode == OUT_F32) {
                         if (row_ok) {
                             float* o = reinterpret_cast<float*>(sg.out) + n;

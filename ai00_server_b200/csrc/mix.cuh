@@ -238,6 +238,111 @@ __global__ void __launch_bounds__(LN_THREADS) ln_mix_kernel(const __grid_constan
     trace_stamp(p.trace, 7);
 }
 
+// Steps of more than 16 tokens: LN_ROWS neighbouring tokens to a CTA, a group of LN_THREADS threads per row and one for the row before
+// them.  A token's shift partner is the normed row of the token before it: ln_mix_kernel computes it a second time, after its own row, so a
+// launch was two dependent chains of loads and reductions and read every partial sum twice (18-23 us for 256 rows of 2560 with 5-7
+// partial sums); here the rows' chains run side by side and the partner is in shared memory.  Same sums in the same order.
+constexpr int LN_ROWS = 2, LN_ROWS_THREADS = (LN_ROWS + 1) * LN_THREADS;
+
+template <int NV>
+__device__ __forceinline__ void ln_mix_rows_nv(const LnMixParams& p, const int t0, float* rows, float* red) {
+    const int C = p.C, T = p.meta.T(), g = threadIdx.x / LN_THREADS, tid = threadIdx.x % LN_THREADS, lane = tid & 31, warp = tid >> 5;
+    const int t = t0 - 1 + g;                                  // group 0: the row before
+    const bool live = t >= 0 && t < T && (g > 0 || (t0 < T && p.meta.tok_prev()[t0] >= 0));
+    auto group_sum = [&](float v) {                            // block_sum of the group's LN_THREADS threads
+        v = warp_sum(v);
+        named_bar_sync(1 + g, LN_THREADS);
+        if (lane == 0) red[g * 8 + warp] = v;
+        named_bar_sync(1 + g, LN_THREADS);
+        return warp_sum(lane < LN_THREADS / 32 ? red[g * 8 + lane] : 0.f);
+    };
+    float4 a[NV];
+    if (live) {
+        const size_t base = (size_t)t * C;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = 4 * (tid + LN_THREADS * j);
+            a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c >= C) continue;
+            a[j] = ld4(p.x_in + base + c);
+            if (p.n_parts == 0) continue;
+            float4 v[8], s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = q < p.n_parts ? ld4(p.parts[q] + base + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) add4(s, v[q]);         // fixed order, identical on all ranks
+            if (p.n_gate > 0) {
+                const int gb = c / p.gate_cl;
+                const float4 gt = ld4(p.gates[gb] + (size_t)t * p.gate_cl + (c - gb * p.gate_cl));
+                s.x *= gt.x; s.y *= gt.y; s.z *= gt.z; s.w *= gt.w;
+            }
+            add4(a[j], s);
+        }
+        if (g > 0 && (p.x_out != p.x_in || p.n_parts > 0)) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                const int c = 4 * (tid + LN_THREADS * j);
+                if (c < C) *reinterpret_cast<float4*>(p.x_out + base + c) = a[j];
+            }
+        }
+        float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) s1 += (a[j].x + a[j].y) + (a[j].z + a[j].w);
+        const float mean = group_sum(s1) / (float)C;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            if (4 * (tid + LN_THREADS * j) >= C) continue;
+            const float dx = a[j].x - mean, dy = a[j].y - mean, dz = a[j].z - mean, dw = a[j].w - mean;
+            s2 += (dx * dx + dy * dy) + (dz * dz + dw * dw);
+        }
+        const float rstd = 1.0f / sqrtf(group_sum(s2) / (float)C + LN_EPS);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = 4 * (tid + LN_THREADS * j);
+            if (c >= C) continue;
+            a[j] = ln_apply(a[j], mean, rstd, ld4(p.ln_w + c), ld4(p.ln_b + c));
+            *reinterpret_cast<float4*>(rows + (size_t)g * C + c) = a[j];
+        }
+    }
+    __syncthreads();
+    if (!live || g == 0) return;
+    const int slot = p.meta.tok_slot()[t];
+    const bool shared = p.meta.tok_prev()[t] >= 0, commit = p.meta.tok_last()[t] != 0 && p.commit_dst;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int c = 4 * (tid + LN_THREADS * j);
+        if (c >= C) continue;
+        const float4 pv = shared ? *reinterpret_cast<const float4*>(rows + (size_t)(g - 1) * C + c) : ld4(p.shift_state + (size_t)slot * C + c);
+        const float4 sx = make_float4(pv.x - a[j].x, pv.y - a[j].y, pv.z - a[j].z, pv.w - a[j].w);
+        *reinterpret_cast<float4*>(p.xx_out + (size_t)t * C + c) = a[j];
+        if (p.sx_out) *reinterpret_cast<float4*>(p.sx_out + (size_t)t * C + c) = sx;
+        if (commit) *reinterpret_cast<float4*>(p.commit_dst + (size_t)slot * C + c) = ld4(p.commit_src + (size_t)t * C + c);
+#pragma unroll 2
+        for (int m = 0; m < p.n_mix; ++m) {
+            const float4 mu = ld4(p.mu[m] + c);
+            *reinterpret_cast<uint2*>(p.mix_out[m] + a16_index(t, c, p.kq_tile)) =
+                make_uint2(pack_h2(a[j].x + sx.x * mu.x, a[j].y + sx.y * mu.y), pack_h2(a[j].z + sx.z * mu.z, a[j].w + sx.w * mu.w));
+        }
+    }
+}
+
+__global__ void __launch_bounds__(LN_ROWS_THREADS) ln_mix_rows_kernel(const __grid_constant__ LnMixParams p) {
+    extern __shared__ __align__(16) float ln_rows[];
+    __shared__ float red[(LN_ROWS + 1) * 8];
+    trace_stamp(p.trace, 0);
+    pdl_launch_dependents();
+    pdl_wait();
+    trace_stamp(p.trace, 1);
+    const int t0 = blockIdx.x * LN_ROWS, nv = (p.C + 4 * LN_THREADS - 1) / (4 * LN_THREADS);
+    if (t0 >= p.meta.T()) return;
+    if (nv <= 1) ln_mix_rows_nv<1>(p, t0, ln_rows, red);
+    else if (nv == 2) ln_mix_rows_nv<2>(p, t0, ln_rows, red);
+    else if (nv <= 3) ln_mix_rows_nv<3>(p, t0, ln_rows, red);
+    else if (nv <= 4) ln_mix_rows_nv<4>(p, t0, ln_rows, red);
+    else ln_mix_rows_nv<8>(p, t0, ln_rows, red);
+    trace_stamp(p.trace, 7);
+}
+
 // ---------------------------------------------------------------------------------------
 // Embedding gather + LN0 (reference: web-rwkv embeds on the CPU and runs ln0 on the device,
 // SURVEY.md §2.2 K1; here the f16 table lives in HBM and both are one kernel).

@@ -4,13 +4,12 @@
 // What bounds it: the chain of tokens of one (head, sequence), 64-odd CTAs for one prompt.  The decode kernel spends four barriers, a
 // round trip to memory and the norm of one warp on every token (2.6 us a token at 7B widths, the decay LoRA evaluated in place); here
 // the loop over tokens has NO barrier and no memory latency:
-//   * the vectors of the next TC tokens are requested while TC tokens run, and everything that does not depend on the state (v6: the
-//     scalar sum r u k that the current token contributes; v7: unit key, removal / write vectors, value residual, bonus) is worked
-//     out per group of tokens, a warp per token;
-//   * a thread holds 4 values x 8 keys of the state; its keys are {4 j .. 4 j + 3} and {32 + 4 j ..}, so that the eight lanes of a
-//     value row read 128 contiguous bytes of shared memory per vector and the other three rows of the warp share them;
+//   * the vectors of the next TC tokens are requested while TC tokens run, and what does not depend on the state (v7: unit key, removal /
+//     write vectors, value residual, bonus) is worked out per group of tokens, a warp per token;
+//   * a thread holds 4 values x 8 neighbouring keys of the state; key-indexed vectors lie in shared memory with each run of eight split into
+//     two half rows, so that the eight lanes of a value row read 128 contiguous bytes and the other three rows of the warp share them;
 //   * the four read-outs of a thread are summed over the eight lanes by halving (4 shuffles instead of 12); norms and outputs
-//     follow per group, a warp per token.
+//     follow per group, a warp per token.  All sums run in wkv.cuh's order: a cut of a prompt over both kernels does not show.
 // Decays come from the decay projection's own launch in these steps (17 us beside the scan's own time below).
 // Measured (one prompt of 100 tokens, 64 heads, ncu): 263 -> 33 us per layer.
 #pragma once
@@ -25,13 +24,15 @@ template <int VER> struct WksCfg {
     static constexpr int BUF = NA * TC * WKV_N;             // floats of one group
     static constexpr int SMEM_BYTES = (2 * BUF + 2 * TC + TC * WKV_N) * 4;
 };
+// place of key c in a staged vector: keys 8 j .. 8 j + 3 at 4 j, 8 j + 4 .. 8 j + 7 at 32 + 4 j
+__device__ __forceinline__ int wks_place(int c) { return (c >> 3) * 4 + (c & 3) + ((c >> 2) & 1) * 32; }
 
 template <int VER>
-__global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_constant__ WkvParams p) {
+__global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_constant__ WkvParams p) {
     using Cfg = WksCfg<VER>;
     constexpr int TC = Cfg::TC, TW = TC / 4;                // tokens per warp in the per-group phases
     extern __shared__ __align__(16) float wks[];
-    float* const sc = wks + 2 * Cfg::BUF;                   // [2][TC] scalar of the token (v5 / v6: sum r u k; v7: bonus)
+    float* const sc = wks + 2 * Cfg::BUF;                   // [2][TC] v7: bonus of the token
     float* const so = sc + 2 * TC;                          // [TC][64] read-outs
     pdl_launch_dependents();
     const int h = blockIdx.x, si = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -44,16 +45,20 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
     for (int e = 0; e < 4; ++e)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const float4 v4 = __ldcs(reinterpret_cast<const float4*>(M + (ig * 4 + e) * WKV_N + 32 * q + 4 * j));
+            const float4 v4 = __ldcs(reinterpret_cast<const float4*>(M + (ig * 4 + e) * WKV_N + 8 * j + 4 * q));
             m[e][4 * q] = v4.x; m[e][4 * q + 1] = v4.y; m[e][4 * q + 2] = v4.z; m[e][4 * q + 3] = v4.w;
         }
-    const int c2 = ch + 2 * lane;                           // the per-group phases give a lane two neighbouring channels
-    auto ld2 = [](const float* q) { return *reinterpret_cast<const float2*>(q); };
+    const int c2 = ch + lane;                               // the per-group phases give a lane the channels lane and lane + 32
+    auto ld2 = [](const float* q) { return make_float2(q[0], q[32]); };
     const float2 lw = ld2(p.lnx_w + c2), lb = ld2(p.lnx_b + c2);
-    float2 u = make_float2(0.f, 0.f), kk_ = u, ka_ = u, rk_ = u, ws = u;
+    float2 kk_ = make_float2(0.f, 0.f), ka_ = kk_, rk_ = kk_, ws = kk_;
     if (VER == 7) { kk_ = ld2(p.k_k + c2); ka_ = ld2(p.k_a + c2); rk_ = ld2(p.r_k + c2); }
-    else u = ld2(p.u + c2);
     if (VER == 5) ws = ld2(p.w_static + c2);
+    float u[8];
+    if (VER != 7) {
+#pragma unroll
+        for (int f = 0; f < 8; ++f) u[f] = p.u[ch + 8 * j + f];
+    }
     pdl_wait();
 
     struct Row { float2 r, k, v, w, a, nu, vf; };
@@ -74,7 +79,12 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
     };
     auto prepare = [&](const int g0, const int b) {         // registers -> shared memory, with all that the state does not enter
         float* const buf = wks + b * Cfg::BUF;
-        auto st2 = [&](const int arr, const int tt, const float2 x) { *reinterpret_cast<float2*>(buf + (arr * TC + tt) * WKV_N + 2 * lane) = x; };
+        auto st2 = [&](const int arr, const int tt, const float2 x) {      // by key
+            float* const d = buf + (arr * TC + tt) * WKV_N;
+            d[wks_place(lane)] = x.x;
+            d[wks_place(lane + 32)] = x.y;
+        };
+        auto sum2 = [&](const float2 x) { return warp_sum(x.x) + warp_sum(x.y); };
 #pragma unroll
         for (int i = 0; i < TW; ++i) {
             const int tt = warp + 4 * i, t = g0 + tt;
@@ -84,20 +94,21 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
             if (VER == 7) {
                 const float2 a = row[i].a;
                 float2 kk = make_float2(k.x * kk_.x, k.y * kk_.y);
-                const float norm = fmaxf(sqrtf(warp_sum(kk.x * kk.x + kk.y * kk.y)), 1e-12f);
+                const float norm = fmaxf(sqrtf(sum2(make_float2(kk.x * kk.x, kk.y * kk.y))), 1e-12f);
                 kk.x /= norm; kk.y /= norm;
                 k.x *= 1.f + (a.x - 1.f) * ka_.x; k.y *= 1.f + (a.y - 1.f) * ka_.y;
-                if (p.layer0) *reinterpret_cast<float2*>(p.v_first + (size_t)(t0 + t) * p.ld + c2) = v;
-                else { v.x += (row[i].vf.x - v.x) * row[i].nu.x; v.y += (row[i].vf.y - v.y) * row[i].nu.y; }
-                const float bonus = warp_sum(r.x * k.x * rk_.x + r.y * k.y * rk_.y);
+                if (p.layer0) {
+                    float* const d = p.v_first + (size_t)(t0 + t) * p.ld + c2;
+                    d[0] = v.x; d[32] = v.y;
+                } else { v.x += (row[i].vf.x - v.x) * row[i].nu.x; v.y += (row[i].vf.y - v.y) * row[i].nu.y; }
+                const float bonus = sum2(make_float2(r.x * k.x * rk_.x, r.y * k.y * rk_.y));
                 if (lane == 0) sc[b * TC + tt] = bonus;
                 st2(4, tt, make_float2(-kk.x, -kk.y));
                 st2(5, tt, make_float2(kk.x * a.x, kk.y * a.y));
-            } else {
-                const float s = warp_sum(r.x * u.x * k.x + r.y * u.y * k.y);
-                if (lane == 0) sc[b * TC + tt] = s;
             }
-            st2(0, tt, r); st2(1, tt, k); st2(2, tt, v);
+            st2(0, tt, r); st2(1, tt, k);
+            buf[(2 * TC + tt) * WKV_N + lane] = v.x;        // by value
+            buf[(2 * TC + tt) * WKV_N + lane + 32] = v.y;
             st2(3, tt, VER == 5 ? ws : row[i].w);
         }
     };
@@ -128,25 +139,24 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
             if (VER != 7) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float s0 = 0.f, s1 = 0.f;
+                    float acc = 0.f;
 #pragma unroll
-                    for (int f = 0; f < 8; f += 2) {
-                        s0 = fmaf(r[f], m[e][f], s0);
-                        s1 = fmaf(r[f + 1], m[e][f + 1], s1);
-                        m[e][f] = fmaf(w[f], m[e][f], k[f] * v[e]);
-                        m[e][f + 1] = fmaf(w[f + 1], m[e][f + 1], k[f + 1] * v[e]);
+                    for (int f = 0; f < 8; ++f) {
+                        const float kv = k[f] * v[e];
+                        acc += r[f] * (u[f] * kv + m[e][f]);
+                        m[e][f] = kv + w[f] * m[e][f];
                     }
-                    o[e] = s0 + s1;
+                    o[e] = acc;
                 }
             } else {
                 float nk[8], ka[8], sa[4];
                 ld8(4, nk); ld8(5, ka);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float s0 = 0.f, s1 = 0.f;
+                    float s = 0.f;
 #pragma unroll
-                    for (int f = 0; f < 8; f += 2) { s0 = fmaf(nk[f], m[e][f], s0); s1 = fmaf(nk[f + 1], m[e][f + 1], s1); }
-                    sa[e] = s0 + s1;
+                    for (int f = 0; f < 8; f += 4) s += (m[e][f] * nk[f] + m[e][f + 1] * nk[f + 1]) + (m[e][f + 2] * nk[f + 2] + m[e][f + 3] * nk[f + 3]);
+                    sa[e] = s;
                 }
 #pragma unroll
                 for (int off = 4; off > 0; off >>= 1)
@@ -154,15 +164,13 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
                     for (int e = 0; e < 4; ++e) sa[e] += __shfl_xor_sync(0xffffffffu, sa[e], off);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float s0 = 0.f, s1 = 0.f;
+                    float acc = 0.f;
 #pragma unroll
-                    for (int f = 0; f < 8; f += 2) {
-                        m[e][f] = fmaf(m[e][f], w[f], fmaf(sa[e], ka[f], v[e] * k[f]));
-                        m[e][f + 1] = fmaf(m[e][f + 1], w[f + 1], fmaf(sa[e], ka[f + 1], v[e] * k[f + 1]));
-                        s0 = fmaf(m[e][f], r[f], s0);
-                        s1 = fmaf(m[e][f + 1], r[f + 1], s1);
+                    for (int f = 0; f < 8; ++f) {
+                        m[e][f] = m[e][f] * w[f] + sa[e] * ka[f] + v[e] * k[f];
+                        acc += m[e][f] * r[f];
                     }
-                    o[e] = s0 + s1;
+                    o[e] = acc;
                 }
             }
             // sum over the eight lanes of a row group, halving the values: lane j ends with value (j >> 1) of its four
@@ -180,16 +188,19 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
         for (int i = 0; i < TW; ++i) {
             const int tt = warp + 4 * i;
             if (tt >= n) continue;
-            const float s = sc[b * TC + tt];
-            const float2 v = ld2(buf + (2 * TC + tt) * WKV_N + 2 * lane);
-            float2 x = ld2(so + tt * WKV_N + 2 * lane);
-            if (VER != 7) { x.x = fmaf(s, v.x, x.x); x.y = fmaf(s, v.y, x.y); }
+            const float2 x = ld2(so + tt * WKV_N + lane);
             const float mean = warp_sum(x.x + x.y) * (1.f / WKV_N);
             const float d0 = x.x - mean, d1 = x.y - mean;
             const float rstd = 1.0f / sqrtf(warp_sum(d0 * d0 + d1 * d1) * (1.f / WKV_N) + GN_EPS);
             float y0 = d0 * rstd * lw.x + lb.x, y1 = d1 * rstd * lw.y + lb.y;
-            if (VER == 7) { y0 += s * v.x; y1 += s * v.y; }
-            *reinterpret_cast<uint32_t*>(p.out + a16_index(t0 + g0 + tt, c2, p.kq_tile)) = pack_h2(y0 * gate[i].x, y1 * gate[i].y);
+            if (VER == 7) {
+                const float s = sc[b * TC + tt];
+                const float2 v = ld2(buf + (2 * TC + tt) * WKV_N + lane);
+                y0 += s * v.x; y1 += s * v.y;
+            }
+            y0 *= gate[i].x; y1 *= gate[i].y;
+            p.out[a16_index(t0 + g0 + tt, c2, p.kq_tile)] = f2h_sat(y0);
+            p.out[a16_index(t0 + g0 + tt, c2 + 32, p.kq_tile)] = f2h_sat(y1);
         }
         __syncthreads();                                    // the group's buffers are refilled next
     }
@@ -197,7 +208,7 @@ __global__ void __launch_bounds__(WKS_THREADS, 4) wkv_scan_kernel(const __grid_c
     for (int e = 0; e < 4; ++e)
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-            __stcs(reinterpret_cast<float4*>(M + (ig * 4 + e) * WKV_N + 32 * q + 4 * j), make_float4(m[e][4 * q], m[e][4 * q + 1], m[e][4 * q + 2], m[e][4 * q + 3]));
+            __stcs(reinterpret_cast<float4*>(M + (ig * 4 + e) * WKV_N + 8 * j + 4 * q), make_float4(m[e][4 * q], m[e][4 * q + 1], m[e][4 * q + 2], m[e][4 * q + 3]));
 }
 
 }  // namespace b200
