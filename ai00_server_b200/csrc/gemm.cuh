@@ -87,14 +87,12 @@ struct GemmParams {
     float* ws;              // [total_tiles][max_contrib][128][MT*16] partial tiles
     unsigned* counters;     // [total_tiles], zero between launches
     const int* nrows;       // device: valid token rows
-    uint32_t w_lbo, w_sbo, a_lbo, a_sbo;   // UMMA descriptor strides (bytes)
     unsigned long long* trace;             // profiling aid: 8 globaltimer stamps of CTA 0 (null in production)
     // L2 prefetch of the NEXT projection launch of the step (set per launch by the engine): when this CTA's producer
     // has requested its last block it asks L2 for the first `prefetch_blocks` blocks the same CTA index will stream in
     // that launch, so HBM keeps working through this launch's tail, the launch boundary and any small kernel between
     const uint8_t* next_W;
     int next_blocks, next_grid, prefetch_blocks;
-    int qvar;               // qgemm.cuh: hand-off variant / diagnostic switches (bit 0 set in production)
     GemmSeg seg[GEMM_MAX_SEG];
 };
 
@@ -166,7 +164,7 @@ __device__ __forceinline__ void gemm_mma_role(const GemmParams& p, const int b0,
                                               const uint32_t full_bar, const uint32_t empty_bar, const uint32_t tfull_bar,
                                               const uint32_t tempty_bar, const uint32_t tmem_base, RingPos& rp, unsigned& segcount) {
     constexpr uint32_t IDESC = umma_idesc_f16(GEMM_BN, 16 * MT);
-    const uint32_t w_lbo = p.w_lbo, w_sbo = p.w_sbo, a_sbo = p.a_sbo;
+    // every descriptor field is a constant: with run-time strides the issue of one MMA cost ~146 cycles, three times the instruction itself
     constexpr uint32_t a_lbo = 16 * MT * 16;          // bytes between the k8 chunks of the token operand: 16 MT rows x 16 B
     SegWalk w;
     w.init(p, b0, b1);
@@ -176,6 +174,7 @@ __device__ __forceinline__ void gemm_mma_role(const GemmParams& p, const int b0,
         if (use > 0) mbar_wait(tempty_bar + acc * 8, (use - 1) & 1u, 11);     // epilogue drained this buffer
         tc_fence_after();
         const uint32_t d0 = tmem_base + acc * (16 * MT);
+        uint32_t accumulate = 0;
         for (int i = 0; i < nblk; ++i) {
             mbar_wait(full_bar + rp.stage * 8, rp.phase, 12);
             tc_fence_after();
@@ -184,9 +183,10 @@ __device__ __forceinline__ void gemm_mma_role(const GemmParams& p, const int b0,
             // canonical tile [k8 chunk][16 MT rows][16 B] (common.cuh), chunk stride = 16 MT x 16 bytes
 #pragma unroll
             for (int k16 = 0; k16 < GEMM_BK / 16; ++k16) {
-                const uint64_t adesc = umma_desc(st + k16 * 2 * w_lbo, w_lbo, w_sbo);
-                const uint64_t bdesc = umma_desc(st + GEMM_WBYTES + k16 * 2 * a_lbo, a_lbo, a_sbo);
-                tc_mma_f16(d0, adesc, bdesc, IDESC, (i > 0 || k16 > 0) ? 1u : 0u);
+                const uint64_t adesc = umma_desc(st + k16 * 2 * GEMM_W_LBO, GEMM_W_LBO, GEMM_W_SBO);
+                const uint64_t bdesc = umma_desc(st + GEMM_WBYTES + k16 * 2 * a_lbo, a_lbo, GEMM_A_SBO);
+                tc_mma_f16(d0, adesc, bdesc, IDESC, accumulate);
+                accumulate = 1;
             }
             tc_commit(empty_bar + rp.stage * 8);          // slot is free once these MMAs have read it
             rp.advance<NSTAGE>(1);
