@@ -263,17 +263,15 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_kernel(const LatentAtt
 
 // ------------------------------------------------------------------------------------------------------------------
 // Tensor-core variant for the serving precision: the same CTA shape (16 (token, head) rows, 32-key tiles, online softmax in
-// f32) with both products on mma.sync m16n8k8 TF32 (operands rounded to TF32 with cvt.rna, f32 accumulation):
+// f32) with both products on mma.sync m16n8k8 TF32 (operands rounded to TF32, f32 accumulation):
 //   scores  S[16 x 32]  = Q[16 x D] . K^T      warp w owns keys 8w .. 8w+7, D / 8 k-steps
 //   output  O[16 x rk] += P[16 x 32] . C       warp w owns a quarter of the latent channels, 4 k-steps per 8 channels
 // Scores go through shared memory between the two so that the softmax keeps the row-per-warp form of the f32 kernel.
 // Row strides are = 4 (mod 32) floats: fragment loads of the score phase are bank-conflict free.
 // ------------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t to_tf32(float v) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(r) : "f"(v));
-    return r;
-}
+// nearest TF32 value, ties away from zero (what cvt.rna does), in integer operations: every operand of every product is rounded, and the
+// conversion's issue rate was what the two products waited for.  A NaN stays one (the addition would carry it into another value).
+__device__ __forceinline__ uint32_t to_tf32(float v) { return v != v ? 0x7FFFE000u : (__float_as_uint(v) + 0x1000u) & 0xFFFFE000u; }
 __device__ __forceinline__ void mma_tf32_1688(float c[4], const uint32_t a[4], const uint32_t b[2]) {
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -312,7 +310,7 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
     for (int e = threadIdx.x; e < 16 * DS; e += LA_THREADS) {
         const int r = e / DS, d = e % DS;
         const int qi = r / HG, h = h0 + r % HG;
-        sq[e] = (d < D && qi < nt && h < p.H) ? p.q[(size_t)(t0 + qi) * p.H * D + (size_t)h * D + d] : 0.f;
+        sq[e] = (d < D && qi < nt && h < p.H) ? __uint_as_float(to_tf32(p.q[(size_t)(t0 + qi) * p.H * D + (size_t)h * D + d])) : 0.f;
     }
     for (int e = threadIdx.x; e < LA_KT * (DS - D); e += LA_THREADS) {       // pad columns of the key tile stay zero
         const int j = e / (DS - D), d = D + e % (DS - D);
@@ -362,7 +360,7 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
 #pragma unroll 4
             for (int ks = 0; ks < Dp; ks += 8) {
                 uint32_t a[4], b[2];
-                a[0] = to_tf32(qa0[ks]); a[1] = to_tf32(qa1[ks]); a[2] = to_tf32(qa0[ks + 4]); a[3] = to_tf32(qa1[ks + 4]);
+                a[0] = __float_as_uint(qa0[ks]); a[1] = __float_as_uint(qa1[ks]); a[2] = __float_as_uint(qa0[ks + 4]); a[3] = __float_as_uint(qa1[ks + 4]);
                 b[0] = to_tf32(kb0[ks]); b[1] = to_tf32(kb0[ks + 4]);
                 mma_tf32_1688(acc, a, b);
             }
@@ -390,7 +388,7 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
             for (int of = 16; of > 0; of >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, of);
             l[i] = l[i] * corr + ps;
             m[i] = mn;
-            ss[r * 36 + lane] = pj;
+            ss[r * 36 + lane] = __uint_as_float(to_tf32(pj));
             if (lane == 0) scorr[r] = corr;
         }
         __syncthreads();
@@ -398,8 +396,8 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
             uint32_t a[4][4];
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
-                a[ks][0] = to_tf32(ss[gq * 36 + ks * 8 + tq]); a[ks][1] = to_tf32(ss[(gq + 8) * 36 + ks * 8 + tq]);
-                a[ks][2] = to_tf32(ss[gq * 36 + ks * 8 + tq + 4]); a[ks][3] = to_tf32(ss[(gq + 8) * 36 + ks * 8 + tq + 4]);
+                a[ks][0] = __float_as_uint(ss[gq * 36 + ks * 8 + tq]); a[ks][1] = __float_as_uint(ss[(gq + 8) * 36 + ks * 8 + tq]);
+                a[ks][2] = __float_as_uint(ss[gq * 36 + ks * 8 + tq + 4]); a[ks][3] = __float_as_uint(ss[(gq + 8) * 36 + ks * 8 + tq + 4]);
             }
             const float c0 = scorr[gq], c1 = scorr[gq + 8];
 #pragma unroll

@@ -103,3 +103,20 @@ def test_routed_projections_of_a_step_of_n_rows(n, experts, top):
     """Row lists of experts: groups of very unequal size, empty ones among them."""
     layer = synth.kemirax_layer("gla", heads=2, dim=16, vdim=24, experts=experts, identity=1, top=top, ff=88, shared_ff=40)
     _check_family(synth.make_kemirax, [layer], kemirax_numpy, n, width=72)
+
+
+def test_a_nan_stays_one_in_latent_attention():
+    """A key that is not a number makes every later row so (rounding to TF32 by integer arithmetic must not turn it into a number)."""
+    cfg, st, _ = synth.make_kemirax([synth.kemirax_layer("latent_attention", mlp=False)], seed=4)
+    st = st.copy()
+    head = int(st[:8].view("<u8")[0])
+    e = json.loads(bytes(st[8:8 + head]))["embed"]
+    rows = st[8 + head + e["data_offsets"][0]:8 + head + e["data_offsets"][1]].reshape(e["shape"][0], -1)
+    rows[7] = np.full(rows.shape[1] // 2, 0x7fc0, "<u2").view(np.uint8)
+    m = runtime.Model(st, max_batch=1, token_chunk_size=32, config=cfg, kv_tokens=64, kv_page=16)
+    try:
+        m.state.reset(0)
+        got = m.infer_raw([0], [24], [1, 2, 7] + list(range(10, 31)), [capi.OPTION_FULL])[0]
+        assert np.isnan(got[2:]).all()
+    finally:
+        m.close()
