@@ -47,6 +47,8 @@ struct BiasAttnPrepParams {
 };
 
 __global__ void __launch_bounds__(128) bias_attn_prep_kernel(const BiasAttnPrepParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -131,6 +133,8 @@ __device__ __forceinline__ void ba_load_tiles(const float* cache, const int* tbl
 
 template <int RBT>
 __global__ void __launch_bounds__(BA_THREADS) bias_attn_kernel(const BiasAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = p.cl, rank = blockIdx.x % CL, ch = blockIdx.x / CL;
@@ -319,6 +323,8 @@ __host__ __device__ inline size_t bias_attn_reg_smem(int qb, int H, int G, int d
 
 template <int RB>
 __global__ void __launch_bounds__(BAR_THREADS, 2) bias_attn_reg_kernel(const BiasAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = p.cl, rank = blockIdx.x % CL, ch = blockIdx.x / CL;

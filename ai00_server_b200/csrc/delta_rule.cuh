@@ -33,6 +33,8 @@ struct ShortConvParams {
 };
 
 __global__ void __launch_bounds__(256) short_conv_kernel(const ShortConvParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int slot = p.meta.tok_slot()[t];
@@ -57,6 +59,8 @@ __global__ void __launch_bounds__(256) short_conv_kernel(const ShortConvParams p
 }
 
 __global__ void __launch_bounds__(256) conv_commit_kernel(const ShortConvParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int i = blockIdx.x;
     if (i >= p.meta.nslots()) return;
     const int slot = p.meta.slot_id()[i], t0 = p.meta.slot_start()[i], nt = p.meta.slot_count()[i];
@@ -74,6 +78,8 @@ __global__ void __launch_bounds__(256) conv_commit_kernel(const ShortConvParams 
 
 // steps of one token per sequence: convolution and new tail in one pass (the thread that reads a channel's tail also moves it on)
 __global__ void __launch_bounds__(256) short_conv_step_kernel(const ShortConvParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int keep = p.taps - 1;
@@ -106,6 +112,8 @@ struct DeltaScanParams {
 
 template <bool CHANNEL, bool STEP>
 __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) delta_scan_kernel(const DeltaScanParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const ScanShape& sh = p.s;
     const int h = blockIdx.x / sh.ncta, cb = blockIdx.x % sh.ncta, si = blockIdx.y;
     const MetaView& meta = p.norm.meta;

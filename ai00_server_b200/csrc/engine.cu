@@ -468,6 +468,9 @@ struct b200rwkv_engine {
     int S = 0, chunk = 0, maxT = A16_MAX_ROWS, precision = 0;      // token rows of a step
     int L = 0, C = 0, F = 0, V = 0, H = 0, N = 64, Cl = 0, Hl = 0, Fl = 0, Vl = 0;
     bool use_graph = true, use_pdl = true;
+    // config.json families: every kernel triggers its dependents and waits for the kernel in front of it at its start, so that a launch
+    // right behind another on the same stream overlaps that kernel's tail (a join has more than one kernel in front: full dependency)
+    cudaStream_t pdl_prev = nullptr;   // stream of the last launch, null behind a join
     bool planning = false;             // a walk over the launches of a step that launches nothing (workspace sizes)
     int split_att = 1, split_ffn = 1;
     // tensor parallel: one symmetric comm block per rank (partials, gate block, logits shard, flags)
@@ -826,7 +829,8 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
     g.grid = std::min(g.grid, blk);
     if (force_grid > 0) g.grid = std::min(force_grid, blk);
     else {
-        // Whole tiles per CTA whenever that keeps >= 3/4 of the SMs streaming: no cross-CTA fix-up in the tail, and
+        // Whole tiles per CTA whenever that keeps >= 3/4 of the SMs streaming (one SM draws ~48 B/ns from HBM, so 81 whole tiles of a 3B
+        // layer take 17-19 us where 148 CTAs with cut tiles take 15.5): no cross-CTA fix-up in the tail, and
         // (measured, profiles/r01_findings.md §7) grids of <= 16 CTAs per GPC finish together while 144-148 CTAs skew
         // by 25 % because the 18/20-SM GPCs share the same GPC bandwidth as the 16-SM ones.
         if (tile <= num_sms && tile * 4 >= num_sms * 3) g.grid = tile;
@@ -888,7 +892,7 @@ void b200rwkv_engine::launch_k(void (*kern)(P, X...), dim3 grid, dim3 block, siz
         ++na;
         launch_cluster = 0;
     }
-    if (use_pdl && !prof) {
+    if ((use_pdl || (kx && pdl_prev == s)) && !prof) {
         at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[na].val.programmaticStreamSerializationAllowed = 1;
         ++na;
@@ -901,6 +905,7 @@ void b200rwkv_engine::launch_k(void (*kern)(P, X...), dim3 grid, dim3 block, siz
         CK(cudaEventCreate(&eb));
         CK(cudaEventRecord(ea, s));
     }
+    pdl_prev = s;
     CK(cudaLaunchKernelEx(&cfg, kern, params, extra...));
     if (prof) {
         CK(cudaEventRecord(eb, s));

@@ -213,7 +213,7 @@ void b200rwkv_engine::ff_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
         } else {                                   // attention and feed-forward in one product, straight into the residual
             kx_lin(s, prof, lin(m.vout, KO, l.o, m.x, W, W, KO, LE_ADD), rows, 1);
         }
-        if (fork) { CK(cudaEventRecord(m.side_join, s2)); CK(cudaStreamWaitEvent(s, m.side_join, 0)); }
+        if (fork) { CK(cudaEventRecord(m.side_join, s2)); CK(cudaStreamWaitEvent(s, m.side_join, 0)); pdl_prev = nullptr; }
         if (m.dbg_layers && !use_graph)            // bring-up aid: the residual as this layer leaves it
             boundary(m.dbg_layers + li * (size_t)maxT * W, nullptr, nullptr, 0, nullptr);
     }

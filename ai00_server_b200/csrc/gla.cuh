@@ -25,6 +25,8 @@ struct GlaParams {
 
 template <bool STEP>
 __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) gla_scan_kernel(const GlaParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const ScanShape& sh = p.s;
     const int h = blockIdx.x / sh.ncta, cb = blockIdx.x % sh.ncta, si = blockIdx.y;
     const MetaView& meta = p.norm.meta;

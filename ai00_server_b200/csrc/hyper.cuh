@@ -48,6 +48,8 @@ constexpr int HC_THREADS_FEW_ROWS = 1024;       // block size for steps of few t
 
 template <int THREADS, int SMAX>
 __global__ void __launch_bounds__(THREADS) hc_step_kernel(const HcStepParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     __shared__ float s_mix[SMAX * SMAX], s_out[SMAX], s_in[SMAX];
     extern __shared__ __align__(16) float hc_u[];      // [W] the read row
@@ -127,6 +129,8 @@ __global__ void __launch_bounds__(THREADS) hc_step_kernel(const HcStepParams p) 
 struct HcSumParams { const float* x; float* out; int S, W; MetaView meta; };
 
 __global__ void __launch_bounds__(NORM_THREADS) hc_sum_kernel(const HcSumParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     for (int c = threadIdx.x; c < p.W; c += blockDim.x) {

@@ -200,7 +200,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     L = nl; C = W; V = m.V; Vl = V; Cl = C; H = Hl = 0; N = 0; F = Fl = 0;
     REQUIRE(world == 1, B200RWKV_ERR_UNSUPPORTED, "models that come with a config.json run on one GPU in this version");
     REQUIRE(quant_layers == 0 && loras.empty(), B200RWKV_ERR_UNSUPPORTED, "models that come with a config.json take no LoRA / quantised layers");
-    use_pdl = false;                                       // these kernels carry no programmatic-dependency waits
+    use_pdl = false;                                       // per launch instead (launch_k): side streams join here
     // steps of up to 512 tokens when the caller's token_chunk_size asks for them (prompts then stream the weights once per 512
     // tokens and fill the experts' row tiles); 128 otherwise, like the other families
     maxT = chunk > 256 ? 512 : (chunk > 128 ? 256 : 128);
@@ -354,7 +354,11 @@ void b200rwkv_engine::kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int ro
     const bool exact = kx->exact || force_exact;
     if (!exact && rows > 16 && kx_umma(s, prof, p, rows, groups)) return;
     if (!exact && rows <= 16) {
-        launch_k(lin_mma16_kernel, dim3(cdiv(p.N, LIN_M16_BN), 1, groups), dim3(LIN_M16_WARPS * 32), 0, p, KC_GEMM, s, prof);
+        // 32 outputs per CTA halve the activation traffic, while that fills the chip twice; else 16 outputs and twice the warps, so that an SM
+        // that gets one CTA still has 64 KB of weights in flight
+        const int live = p.off ? std::min(groups, rows * kx->max_top) : groups;
+        if (cdiv(p.N, 32) * live >= 2 * num_sms) launch_k(lin_mma16_kernel<8, 4, 2>, dim3(cdiv(p.N, 32), 1, groups), dim3(256), 0, p, KC_GEMM, s, prof);
+        else launch_k(lin_mma16_kernel<16, 2, 4>, dim3(cdiv(p.N, 16), 1, groups), dim3(512), 0, p, KC_GEMM, s, prof);
     } else if (rows <= LIN_SK_ROWS || (exact && rows <= 16)) {
         launch_k(lin_skinny_kernel, dim3(cdiv(p.N, 2 * LIN_SK_WARPS), 1, groups), dim3(LIN_SK_WARPS * 32), 0, p, KC_GEMM, s, prof);
     } else if (exact) {

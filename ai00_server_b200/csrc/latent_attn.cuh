@@ -41,6 +41,8 @@ struct SeqMeta {
 struct PageUpdateParams { SeqMeta sm; int* table; int stride; };
 
 __global__ void page_update_kernel(const PageUpdateParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int n = p.sm.n_upd();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int* u = p.sm.upd() + 3 * i;
@@ -67,6 +69,8 @@ __device__ __forceinline__ float rot_pair_entry(const float* s, int i, int pos, 
 }
 
 __global__ void __launch_bounds__(128) rope_rows_kernel(const RopeParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const float pos = (float)p.sm.tok_pos()[t];
@@ -97,6 +101,8 @@ struct KvWriteParams {
 };
 
 __global__ void __launch_bounds__(128) kv_write_kernel(const KvWriteParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
@@ -152,6 +158,8 @@ __host__ __device__ constexpr size_t latent_attn_smem(int D) {
 
 template <int QB, int HG>
 __global__ void __launch_bounds__(LA_THREADS) latent_attn_kernel(const LatentAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int R = QB * HG;                     // (token, head) rows of this CTA
     constexpr int RPW = R / 4;                     // rows per warp
     static_assert(R % 4 == 0, "rows must split over four warps");
@@ -286,6 +294,8 @@ constexpr int LA_TC_MAX_NT = 16;                   // 8-channel tiles per warp: 
 
 template <int QB, int HG>
 __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const LatentAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     static_assert(QB * HG == 16, "one m16 tile of (token, head) rows");
     const int ci = blockIdx.x;
     if (ci >= p.sm.n_chunks()) return;
@@ -446,6 +456,8 @@ struct LatentMergeParams {
 };
 
 __global__ void __launch_bounds__(128) latent_merge_kernel(const LatentMergeParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y;
     if (t >= p.meta.T()) return;
     const float* src = p.part + ((size_t)t * p.H + h) * p.nsplit * (p.rk + 2);

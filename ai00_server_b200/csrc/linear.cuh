@@ -24,6 +24,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace b200 {
 
 enum LinEpi {
@@ -129,6 +131,8 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float2 v) {
 
 template <bool EXACT>
 __global__ void __launch_bounds__(LIN_THREADS) lin_tile_kernel(const LinParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int g = blockIdx.z;
     const int rows = p.cnt[(size_t)g * p.cnt_gstride];
     const int r0 = blockIdx.y * LIN_BM;
@@ -310,6 +314,8 @@ __global__ void __launch_bounds__(LIN_THREADS) lin_tile_kernel(const LinParams p
 
 // sums the split-k partials in split order and runs the epilogue (one group, rows in place)
 __global__ void __launch_bounds__(256) lin_splitk_finish_kernel(const LinParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.y;
     if (r >= p.cnt[0]) return;
     const int n = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
@@ -330,6 +336,8 @@ __global__ void __launch_bounds__(256) lin_splitk_finish_kernel(const LinParams 
 constexpr int LIN_SK_ROWS = 8, LIN_SK_WARPS = 8;
 
 __global__ void __launch_bounds__(LIN_SK_WARPS * 32) lin_skinny_kernel(const LinParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int g = blockIdx.z;
     const int rows = p.cnt[(size_t)g * p.cnt_gstride];
     if (rows <= 0) return;
@@ -405,16 +413,20 @@ __global__ void __launch_bounds__(LIN_SK_WARPS * 32) lin_skinny_kernel(const Lin
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// steps of up to 16 rows on the tensor cores: 16 outputs per CTA, the k range split over 8 warps.  A lane streams 16 bytes of
+// steps of up to 16 rows on the tensor cores: 8 NT outputs per CTA, the k range split over the warps.  A lane streams 16 bytes of
 // one weight row (8 consecutive k) and the matching 8 activations of rows g and g + 8 straight from global memory; those 8 k
 // feed two m16n8k16 products (any fixed pairing of k between the A and B fragments is a valid sum order), so no operand
 // passes through shared memory and every weight byte is read once, in full 32-byte sectors.
+// The launch is a short stream (8-134 MB) behind a small kernel: what bounds it is how much of it is in flight, and, with f32
+// activations of 16 rows twice the bytes of 16 bf16 weight rows, what the SM takes in from L2.  A lane asks for U k blocks at a time (eight
+// 16-byte loads) one batch ahead of the products, and for the first batch BEFORE griddepcontrol.wait, since weights are no kernel's output.
+// Measured (16 rows, panupel w2048, ncu: cold and one at a time, so without the early request): 36 launches 695 us with four loads in flight
+// behind the wait -> 632; a decode step of that stack 0.70 -> 0.58 ms, of the kemirax one 0.53 -> 0.50, with the programmatic edges
+// (1.066x and 1.026x of it, same binary with and without).
 // ------------------------------------------------------------------------------------------------------------------
-constexpr int LIN_M16_WARPS = 8;
-
 __device__ __forceinline__ void lin_ld8(const float* p, bool vec, int valid, float v[8]) {
     if (vec && valid >= 8) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     } else {
 #pragma unroll
@@ -422,101 +434,114 @@ __device__ __forceinline__ void lin_ld8(const float* p, bool vec, int valid, flo
     }
 }
 
-constexpr int LIN_M16_BN = 16;                     // outputs per CTA: two n8 tiles share every activation fragment
-
-__global__ void __launch_bounds__(LIN_M16_WARPS * 32, 3) lin_mma16_kernel(const LinParams p) {
+template <int WARPS, int NT, int U>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) lin_mma16_kernel(const LinParams p) {
+    constexpr int BN = NT * 8, STEP = WARPS * 32;
     const int g = blockIdx.z;
-    const int rows = p.cnt[(size_t)g * p.cnt_gstride];
-    if (rows <= 0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
-    const int n0 = blockIdx.x * LIN_M16_BN;
-    const int base = p.off ? p.off[g] : 0;
-    const float* X = p.X + g * p.x_gstride;
+    const int n0 = blockIdx.x * BN;
     const int K = p.K;
     const __nv_bfloat16* Wg = p.W + g * p.w_gstride;
-    const __nv_bfloat16* wrow[2];
-    bool nvalid[2];
+    const __nv_bfloat16* wrow[NT];
+    bool nvalid[NT];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < NT; ++j) {
         const int n = n0 + j * 8 + gq;
         nvalid[j] = n < p.N;
         wrow[j] = Wg + (size_t)min(n, p.N - 1) * K;
     }
     const bool vecW = (K % 8 == 0) && ((reinterpret_cast<uintptr_t>(Wg) & 15) == 0);
-    const bool vecX = (p.ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
-    __shared__ float red[LIN_M16_WARPS][16][LIN_M16_BN];
-    for (int rb = 0; rb < rows; rb += 16) {
-        const int rlo = rb + gq, rhi = rb + gq + 8;
-        const float* xlo = rlo < rows ? X + (size_t)(p.xlist ? p.xlist[base + rlo] : base + rlo) * p.ldx : nullptr;
-        const float* xhi = rhi < rows ? X + (size_t)(p.xlist ? p.xlist[base + rhi] : base + rhi) * p.ldx : nullptr;
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        constexpr int U = 2;                       // k blocks per batch: 4 weight loads in flight per lane
-        for (int kb0 = warp * 32; kb0 < K; kb0 += LIN_M16_WARPS * 32 * U) {
-            uint4 wq[U][2];
+    auto weights = [&](const int kb, uint4 (&wq)[U][NT]) {          // blocks kb, kb + STEP, ... of this warp
 #pragma unroll
-            for (int u = 0; u < U; ++u) {          // all weight loads of the batch first: they are the HBM stream
-                const int k = kb0 + u * LIN_M16_WARPS * 32 + tq * 8;
-                const int valid = max(0, min(8, K - k));
+        for (int u = 0; u < U; ++u) {
+            const int k = kb + u * STEP + tq * 8;
+            const int valid = max(0, min(8, K - k));
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    wq[u][j] = make_uint4(0, 0, 0, 0);
-                    if (nvalid[j] && valid > 0) {
-                        if (vecW) {
-                            wq[u][j] = __ldg(reinterpret_cast<const uint4*>(wrow[j] + k));
-                        } else {
-                            __align__(16) __nv_bfloat16 t[8];
+            for (int j = 0; j < NT; ++j) {
+                wq[u][j] = make_uint4(0, 0, 0, 0);
+                if (nvalid[j] && valid > 0) {
+                    if (vecW) {
+                        wq[u][j] = __ldg(reinterpret_cast<const uint4*>(wrow[j] + k));
+                    } else {
+                        __align__(16) __nv_bfloat16 t[8];
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) t[e] = e < valid ? wrow[j][k + e] : __float2bfloat16(0.f);
-                            wq[u][j] = *reinterpret_cast<const uint4*>(t);
-                        }
+                        for (int e = 0; e < 8; ++e) t[e] = e < valid ? wrow[j][k + e] : __float2bfloat16(0.f);
+                        wq[u][j] = *reinterpret_cast<const uint4*>(t);
                     }
                 }
             }
+        }
+    };
+    pdl_launch_dependents();
+    uint4 cur[U][NT], nxt[U][NT];
+    if (p.off) {                                   // routed: an expert without rows is not read
+        pdl_wait();
+        if (p.cnt[(size_t)g * p.cnt_gstride] <= 0) return;
+        weights(warp * 32, cur);
+    } else {
+        weights(warp * 32, cur);
+        pdl_wait();
+    }
+    const int rows = min(p.cnt[(size_t)g * p.cnt_gstride], 16);
+    if (rows <= 0) return;
+    const int base = p.off ? p.off[g] : 0;
+    const float* X = p.X + g * p.x_gstride;
+    const bool vecX = (p.ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) & 15) == 0);
+    const float* xlo = gq < rows ? X + (size_t)(p.xlist ? p.xlist[base + gq] : base + gq) * p.ldx : nullptr;
+    const float* xhi = gq + 8 < rows ? X + (size_t)(p.xlist ? p.xlist[base + gq + 8] : base + gq + 8) * p.ldx : nullptr;
+    float acc[NT][4];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = kb0 + u * LIN_M16_WARPS * 32 + tq * 8;
-                const int valid = max(0, min(8, K - k));
-                if (kb0 + u * LIN_M16_WARPS * 32 >= K) break;          // warp-uniform
-                float lo[8], hi[8];
-                if (xlo && valid > 0) lin_ld8(xlo + k, vecX, valid, lo);
-                else {
+    for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    for (int kb0 = warp * 32; kb0 < K; kb0 += STEP * U) {
+        if (kb0 + STEP * U < K) weights(kb0 + STEP * U, nxt);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) lo[e] = 0.f;
-                }
-                if (xhi && valid > 0) lin_ld8(xhi + k, vecX, valid, hi);
-                else {
+        for (int u = 0; u < U; ++u) {
+            const int k = kb0 + u * STEP + tq * 8;
+            const int valid = max(0, min(8, K - k));
+            if (kb0 + u * STEP >= K) break;        // warp-uniform
+            float lo[8], hi[8];
+            if (xlo && valid > 0) lin_ld8(xlo + k, vecX, valid, lo);
+            else {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) hi[e] = 0.f;
-                }
-                uint32_t a0[4], a1[4];
-                a0[0] = pack_bf16x2(make_float2(lo[0], lo[1])); a0[1] = pack_bf16x2(make_float2(hi[0], hi[1]));
-                a0[2] = pack_bf16x2(make_float2(lo[2], lo[3])); a0[3] = pack_bf16x2(make_float2(hi[2], hi[3]));
-                a1[0] = pack_bf16x2(make_float2(lo[4], lo[5])); a1[1] = pack_bf16x2(make_float2(hi[4], hi[5]));
-                a1[2] = pack_bf16x2(make_float2(lo[6], lo[7])); a1[3] = pack_bf16x2(make_float2(hi[6], hi[7]));
+                for (int e = 0; e < 8; ++e) lo[e] = 0.f;
+            }
+            if (xhi && valid > 0) lin_ld8(xhi + k, vecX, valid, hi);
+            else {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    uint32_t b[2];
-                    b[0] = wq[u][j].x; b[1] = wq[u][j].y;
-                    mma_bf16_16816(acc[j], a0, b);
-                    b[0] = wq[u][j].z; b[1] = wq[u][j].w;
-                    mma_bf16_16816(acc[j], a1, b);
-                }
+                for (int e = 0; e < 8; ++e) hi[e] = 0.f;
+            }
+            uint32_t a0[4], a1[4];
+            a0[0] = pack_bf16x2(make_float2(lo[0], lo[1])); a0[1] = pack_bf16x2(make_float2(hi[0], hi[1]));
+            a0[2] = pack_bf16x2(make_float2(lo[2], lo[3])); a0[3] = pack_bf16x2(make_float2(hi[2], hi[3]));
+            a1[0] = pack_bf16x2(make_float2(lo[4], lo[5])); a1[1] = pack_bf16x2(make_float2(hi[4], hi[5]));
+            a1[2] = pack_bf16x2(make_float2(lo[6], lo[7])); a1[3] = pack_bf16x2(make_float2(hi[6], hi[7]));
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                uint32_t b[2];
+                b[0] = cur[u][j].x; b[1] = cur[u][j].y;
+                mma_bf16_16816(acc[j], a0, b);
+                b[0] = cur[u][j].z; b[1] = cur[u][j].w;
+                mma_bf16_16816(acc[j], a1, b);
             }
         }
-        __syncthreads();                           // red of the previous row block has been read
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            red[warp][gq][j * 8 + tq * 2] = acc[j][0]; red[warp][gq][j * 8 + tq * 2 + 1] = acc[j][1];
-            red[warp][gq + 8][j * 8 + tq * 2] = acc[j][2]; red[warp][gq + 8][j * 8 + tq * 2 + 1] = acc[j][3];
-        }
-        __syncthreads();
-        if (threadIdx.x < 128) {
-            const int r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 2;
-            float s0 = 0.f, s1 = 0.f;
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int w = 0; w < LIN_M16_WARPS; ++w) { s0 += red[w][r][c]; s1 += red[w][r][c + 1]; }
-            if (rb + r < rows && n0 + c < p.N) lin_store(p, g, base + rb + r, n0 + c, s0, s1, n0 + c + 1 < p.N);
-        }
+            for (int j = 0; j < NT; ++j) cur[u][j] = nxt[u][j];
+    }
+    __shared__ float red[WARPS][16][BN];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        red[warp][gq][j * 8 + tq * 2] = acc[j][0]; red[warp][gq][j * 8 + tq * 2 + 1] = acc[j][1];
+        red[warp][gq + 8][j * 8 + tq * 2] = acc[j][2]; red[warp][gq + 8][j * 8 + tq * 2 + 1] = acc[j][3];
+    }
+    __syncthreads();
+    if (threadIdx.x < 16 * BN / 2) {               // whole warps, at most the CTA
+        const int r = threadIdx.x / (BN / 2), c = (threadIdx.x % (BN / 2)) * 2;
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) { s0 += red[w][r][c]; s1 += red[w][r][c + 1]; }
+        if (r < rows && n0 + c < p.N) lin_store(p, g, base + r, n0 + c, s0, s1, n0 + c + 1 < p.N);
     }
 }
 

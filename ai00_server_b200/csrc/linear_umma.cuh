@@ -59,6 +59,8 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 }
 
 __global__ void __launch_bounds__(256) lin_pack_kernel(const LinParams p, __nv_bfloat16* out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int g = blockIdx.y;
     const int rows = p.cnt[(size_t)g * p.cnt_gstride], K8 = p.K >> 3;
     const int base = p.off ? p.off[g] : 0;
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
     const uint32_t full_bar = ring + Cfg::BAR_OFF, empty_bar = full_bar + Cfg::NSTAGE * 8;
     const uint32_t tfull_bar = empty_bar + Cfg::NSTAGE * 8, tempty_bar = tfull_bar + 16, tmem_slot = tempty_bar + 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < Cfg::NSTAGE; ++s) { mbar_init(full_bar + s * 8, 1); mbar_init(empty_bar + s * 8, 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(tfull_bar + s * 8, 1); mbar_init(tempty_bar + s * 8, LU_EPI_WARPS); }
@@ -132,6 +135,7 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+    pdl_wait();
     LuWalk<TN> w;
     w.init(p);
 

@@ -37,6 +37,8 @@ constexpr int MM_MAX_N = SCAN_MAX_DK / SCAN_THREADS_PROMPT;      // normaliser e
 
 template <bool STEP>
 __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) matrix_memory_kernel(const MatrixMemoryParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const ScanShape& sh = p.s;
     const int h = blockIdx.x / sh.ncta, cb = blockIdx.x % sh.ncta, si = blockIdx.y;
     const MetaView& meta = p.norm.meta;

@@ -66,6 +66,8 @@ __device__ __forceinline__ int moe_warp_take_max(float* a, int n, float& val) {
 // One CTA per token: router logits in f32 on the f32 row (every warp takes outputs warp, warp + 8, ...), then warp 0 turns them
 // into the choice: softmax, + selection bias, `top` largest, weights = the unbiased probabilities.
 __global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(const MoeRouteParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float moe_route_sm[];
     float* sh = moe_route_sm;                 // [K]
     float* z = sh + p.K;                      // [NE]
@@ -204,6 +206,8 @@ struct MoeGroupParams {
 };
 
 __global__ void __launch_bounds__(256) moe_group_kernel(const MoeGroupParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ int moe_smem[];         // [E] counts, [E] offsets, [T * top] choices
     int* s_cnt = moe_smem;
     int* s_off = s_cnt + p.E;
@@ -256,6 +260,8 @@ struct MoeCombineParams {
 };
 
 __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombineParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;

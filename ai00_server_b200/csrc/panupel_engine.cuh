@@ -210,7 +210,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             sp.meta = mv; sp.sm = m.sm;
             launch_cluster = nsplit;
             launch_k(plan.kern, dim3(chunks_grid * sp.nsub * nsplit, cdiv(H_, plan.hb)), dim3(plan.threads), plan.smem, sp, KC_WKV, s, prof);
-            if (fork) { CK(cudaEventRecord(m.side_join, s2)); CK(cudaStreamWaitEvent(s, m.side_join, 0)); }
+            if (fork) { CK(cudaEventRecord(m.side_join, s2)); CK(cudaStreamWaitEvent(s, m.side_join, 0)); pdl_prev = nullptr; }
         } else {
             const PnDeltaRow r(c);
             const int C_ = l.conv_C, ldc = rup(C_, 4);

@@ -28,6 +28,8 @@ struct RetentionParams {
 __host__ __device__ inline size_t retention_smem_bytes(int dk, int dv) { return ((size_t)dk * dv + 2 * (size_t)dk + 32) * sizeof(float); }
 
 __global__ void retention_kernel(const RetentionParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int h = blockIdx.x, si = blockIdx.y;
     if (si >= p.meta.nslots()) return;
     const int slot = p.meta.slot_id()[si], t0 = p.meta.slot_start()[si], nt = p.meta.slot_count()[si];
@@ -98,6 +100,8 @@ constexpr int RET_REG_MAX_DK = 128, RET_REG_MAX_DV = 256;
 
 template <int DKC>
 __global__ void __launch_bounds__(RET_REG_MAX_DV) retention_reg_kernel(const RetentionParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int h = blockIdx.x, si = blockIdx.y;
     if (si >= p.meta.nslots()) return;
     const int slot = p.meta.slot_id()[si], t0 = p.meta.slot_start()[si], nt = p.meta.slot_count()[si];

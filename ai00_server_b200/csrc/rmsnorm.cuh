@@ -51,6 +51,8 @@ struct EmbedRowsParams {
 };
 
 __global__ void __launch_bounds__(NORM_THREADS) embed_rows_kernel(const EmbedRowsParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int tok = p.meta.tok()[t];
@@ -80,6 +82,8 @@ __global__ void __launch_bounds__(NORM_THREADS) embed_rows_kernel(const EmbedRow
 
 // own launch after embed_rows_kernel: a first token of the step may still be reading the old one
 __global__ void __launch_bounds__(128) last_token_commit_kernel(const EmbedRowsParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.meta.nslots()) return;
     p.last_tok[p.meta.slot_id()[i]] = (float)p.meta.tok()[p.meta.slot_start()[i] + p.meta.slot_count()[i] - 1];
@@ -97,6 +101,8 @@ struct NormShiftParams {
 };
 
 __global__ void __launch_bounds__(NORM_THREADS) norm_shift_kernel(const NormShiftParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
@@ -127,6 +133,8 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_shift_kernel(const NormShif
 // shift-state commit, run after norm_shift_kernel of the same layer (a first token of the sequence may still be reading the
 // old row while the last token's CTA would overwrite it, so the commit is its own launch)
 __global__ void __launch_bounds__(NORM_THREADS) shift_commit_kernel(const NormShiftParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int i = blockIdx.x;
     if (i >= p.meta.nslots()) return;
     const int t = p.meta.slot_start()[i] + p.meta.slot_count()[i] - 1;
@@ -144,6 +152,8 @@ struct RmsRowsParams {
 };
 
 __global__ void __launch_bounds__(128) rms_rows_kernel(const RmsRowsParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     const int r = blockIdx.x, c = blockIdx.y;
     if (r >= *p.nrows) return;
@@ -167,6 +177,8 @@ struct FinalNormParams {
 };
 
 __global__ void __launch_bounds__(NORM_THREADS) final_norm_kernel(const FinalNormParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
@@ -201,6 +213,8 @@ struct NormAddParams {
 constexpr int NORM_ADD_MAX_TOP = 8;
 
 __global__ void __launch_bounds__(NORM_THREADS) norm_add_kernel(const NormAddParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     extern __shared__ __align__(16) float norm_add_row[];      // [W] the combined row (expert form only)
     const int t = blockIdx.x;
@@ -270,6 +284,8 @@ constexpr int PRE_NORM_THREADS_FEW_ROWS = 1024;    // block size for steps of fe
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) pre_norm_kernel(const PreNormParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     extern __shared__ __align__(16) float pre_norm_row[];      // [W]
     const int t = blockIdx.x;

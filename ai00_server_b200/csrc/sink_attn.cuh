@@ -66,6 +66,8 @@ __device__ __forceinline__ void sa_pool_block(const PoolWriteParams& p, const in
 }
 
 __global__ void __launch_bounds__(128) pool_write_kernel(const PoolWriteParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int ipos = p.sm.tok_pos()[t];
@@ -74,6 +76,8 @@ __global__ void __launch_bounds__(128) pool_write_kernel(const PoolWriteParams p
 }
 
 __global__ void __launch_bounds__(128) pool_rebuild_kernel(const PoolWriteParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     if ((int)blockIdx.x < p.nblocks) sa_pool_block(p, p.table + (size_t)p.slot * p.stride, blockIdx.x);
 }
 
@@ -98,6 +102,8 @@ struct RotPrepParams {
 constexpr int ROT_PREP_THREADS = 256;
 
 __global__ void __launch_bounds__(ROT_PREP_THREADS) rot_prep_kernel(const RotPrepParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     extern __shared__ __align__(16) float rot_cs[];              // [dims / 2] cosines, [dims / 2] sines
     const int t = blockIdx.x;
@@ -205,6 +211,8 @@ __host__ __device__ inline size_t sink_attn_smem(int qb, int HB, int dk, int dv,
 
 template <int RBT>
 __global__ void __launch_bounds__(SA_THREADS) sink_attn_kernel(const SinkAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = p.cl, rank = blockIdx.x % CL;
@@ -476,6 +484,8 @@ __host__ __device__ inline size_t sink_attn_reg_smem(int qb, int HB, int rep, in
 
 template <int RB, int NC, int NB>
 __global__ void __launch_bounds__(SAR_THREADS, NC == 1 ? 2 : 1) sink_attn_reg_kernel(const SinkAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int KT = 8 * NB;                     // keys per tile
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();

@@ -154,6 +154,8 @@ __device__ __forceinline__ float head_norm_value(const HeadNormParams& p, float 
 }
 
 __global__ void __launch_bounds__(128) head_norm_kernel(const HeadNormParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     for (int h = blockIdx.y * 4 + (threadIdx.x >> 5); h < p.H; h += gridDim.y * 4) head_norm_row(p, t, h, threadIdx.x & 31);

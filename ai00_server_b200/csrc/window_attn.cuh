@@ -43,6 +43,8 @@ struct AttnPrepParams {
 };
 
 __global__ void __launch_bounds__(128) attn_prep_kernel(const AttnPrepParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -140,6 +142,8 @@ __device__ __forceinline__ void wa_tile(int ti, int n0, const int* lo, const int
 }
 
 __global__ void __launch_bounds__(WA_THREADS) window_attn_kernel(const WindowAttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = p.cl, rank = blockIdx.x % CL, ch = blockIdx.x / CL;

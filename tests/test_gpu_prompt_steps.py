@@ -105,6 +105,13 @@ def test_routed_projections_of_a_step_of_n_rows(n, experts, top):
     _check_family(synth.make_kemirax, [layer], kemirax_numpy, n, width=72)
 
 
+@pytest.mark.parametrize("n", [1, 9, 16])
+@pytest.mark.parametrize("ff", [4740, 4744, 600])
+def test_projections_of_a_step_of_few_rows(n, ff):
+    """Steps of up to 16 rows: 32 outputs a CTA (2 ff from 9472 on) and 16, ragged last CTAs, k ranges that are no multiple of a lane's 8."""
+    _check_family(synth.make_panupel, [synth.panupel_layer("delta", heads=3, dim=24, ff=ff)], panupel_numpy, n, width=136)
+
+
 def test_a_nan_stays_one_in_latent_attention():
     """A key that is not a number makes every later row so (rounding to TF32 by integer arithmetic must not turn it into a number)."""
     cfg, st, _ = synth.make_kemirax([synth.kemirax_layer("latent_attention", mlp=False)], seed=4)
