@@ -562,6 +562,7 @@ struct b200rwkv_engine {
     void ff_enqueue_layers(cudaStream_t s, int rows, int nslot_grid, bool decode, int nsplit, Profiler* prof);
     __nv_bfloat16* kx_up16(const std::vector<uint16_t>& v);
     float* kx_up32(const std::vector<float>& v);
+    void kx_pre_norm(cudaStream_t s, Profiler* prof, const PreNormParams& pn, int rows);
     bool kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int rows, int groups);
     void kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int rows, int groups, bool force_exact = false);
     void kx_short_conv(cudaStream_t s, Profiler* prof, const ShortConvParams& cp, int rows, int nslot_grid, bool decode);

@@ -156,9 +156,7 @@ void b200rwkv_engine::ff_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
     auto boundary = [&](float* snap, const float* weight, float* h, int compact, float* hidden) {
         PreNormParams pn{m.x, nullptr, nullptr, nullptr, 0, nullptr, snap, nullptr, nullptr, weight, eps, h, compact, hidden, W, mv};
         if (halves) { pn.y = m.y; pn.post_w = halves->norm1b_w; pn.y2 = m.hs; pn.post2_w = halves->norm2b_w; pn.post_mul = 0.5f * mul; }
-        const size_t sm_b = (size_t)W * (halves ? 8 : 4);
-        if (rows <= 32) launch_k(pre_norm_kernel<PRE_NORM_THREADS_FEW_ROWS>, dim3(rows), dim3(PRE_NORM_THREADS_FEW_ROWS), sm_b, pn, KC_LN, s, prof);
-        else launch_k(pre_norm_kernel<NORM_THREADS>, dim3(rows), dim3(NORM_THREADS), sm_b, pn, KC_LN, s, prof);
+        kx_pre_norm(s, prof, pn, rows);
         halves = nullptr;
     };
     const int chunks_grid = decode ? rows : cdiv(rows, m.qb_prompt) + nslot_grid;

@@ -250,6 +250,8 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     if (m.side_lin) m.lin_ws_side = fa(m.lin_ws_floats);
     m.sel = (int*)dalloc(T_ * z.max_top * 4); m.row_of = (int*)dalloc(T_ * z.max_top * 4); m.list = (int*)dalloc(T_ * z.max_top * 4);
     m.cnt = (int*)dalloc((size_t)z.max_E * 4); m.off = (int*)dalloc((size_t)z.max_E * 4);
+    if (!m.exact && W % 8 == 0) m.h16 = (__nv_bfloat16*)dalloc(T_ * W * 2, true);
+    if (!m.exact && z.n_ys % 8 == 0 && z.n_ys) m.ys16 = (__nv_bfloat16*)dalloc(T_ * z.n_ys * 2, true);
     d_hidden = fa(T_ * W);
     d_logits = fa(T_ * V);
     d_api = fa(m.flat_floats(m.state_ctx));
@@ -331,11 +333,11 @@ bool b200rwkv_engine::kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int 
         while (ks > 1 && (size_t)mtiles * ttiles * ks * LU_BM * tn > m.lin_ws_floats) --ks;
         ks = cdiv(slabs, cdiv(slabs, ks));
     }
-    launch_k(lin_pack_kernel, dim3(std::min(cdiv(rows * (p.K / 8), 256), 4 * num_sms), groups), dim3(256), 0, p, KC_GEMM, s, prof, x16);
+    if (!p.X16) launch_k(lin_pack_kernel, dim3(std::min(cdiv(rows * (p.K / 8), 256), 4 * num_sms), groups), dim3(256), 0, p, KC_GEMM, s, prof, x16);
     LinUmmaParams u;
     memset(&u, 0, sizeof(u));
     lu_map(&u.tw, p.W, (uint64_t)groups * p.N, p.K, LU_BM);
-    lu_map(&u.tx, x16, total, p.K, tn);
+    lu_map(&u.tx, p.X16 ? p.X16 : x16, total, p.K, tn);
     u.l = p; u.groups = groups; u.ksplit = ks;
     u.l.ws = side ? m.lin_ws_side : m.lin_ws;
     u.counters = side ? m.lin_counters_side : m.lin_counters;
@@ -348,11 +350,28 @@ bool b200rwkv_engine::kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int 
     return true;
 }
 
+// the boundary of a pre-norm sublayer (rmsnorm.cuh): in registers where the row is whole float4 and nothing routed is pending
+void b200rwkv_engine::kx_pre_norm(cudaStream_t s, Profiler* prof, const PreNormParams& pn, int rows) {
+    const int W = pn.W, nv = cdiv(W, 4 * PRE_NORM_VEC_THREADS);
+    if (!pn.rows && !pn.shared && W % 4 == 0 && nv <= PRE_NORM_VEC_MAX) {
+        auto go = [&](void (*kern)(PreNormParams)) { launch_k(kern, dim3(rows), dim3(PRE_NORM_VEC_THREADS), 0, pn, KC_LN, s, prof); };
+        if (nv == 1) go(pre_norm_vec_kernel<1>);
+        else if (nv == 2) go(pre_norm_vec_kernel<2>);
+        else if (nv <= 4) go(pre_norm_vec_kernel<4>);
+        else go(pre_norm_vec_kernel<8>);
+        return;
+    }
+    const size_t smem = (size_t)W * 4 * (pn.y2 ? 2 : 1);
+    if (rows <= 32) launch_k(pre_norm_kernel<PRE_NORM_THREADS_FEW_ROWS>, dim3(rows), dim3(PRE_NORM_THREADS_FEW_ROWS), smem, pn, KC_LN, s, prof);
+    else launch_k(pre_norm_kernel<NORM_THREADS>, dim3(rows), dim3(NORM_THREADS), smem, pn, KC_LN, s, prof);
+}
+
 // one grouped linear launch; `rows` bounds the row count of any group (the step's bucket)
 void b200rwkv_engine::kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int rows, int groups, bool force_exact) {
     p.max_rows = rows;
     const bool exact = kx->exact || force_exact;
     if (!exact && rows > 16 && kx_umma(s, prof, p, rows, groups)) return;
+    REQUIRE(!p.X16 && !p.Y16, B200RWKV_ERR_UNSUPPORTED, "bf16 operands need the tcgen05 projection");   // sized by the caller for it
     if (!exact && rows <= 16) {
         // 32 outputs per CTA halve the activation traffic, while that fills the chip twice; else 16 outputs and twice the warps, so that an SM
         // that gets one CTA still has 64 KB of weights in flight

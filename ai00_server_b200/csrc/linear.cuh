@@ -46,6 +46,10 @@ struct LinParams {
     const float* X; int ldx; long long x_gstride;      // X + g * x_gstride, row stride ldx (floats)
     const __nv_bfloat16* W; long long w_gstride;       // W + g * w_gstride, row n at n * K
     float* Y; int ldy; long long y_gstride;
+    // linear_umma.cuh: the activations as bf16 rows [row][K] a kernel in front has written (one group, rows in place; X is not read then),
+    // and gated units written as bf16 [row][ldy] for the next projection instead of Y
+    const __nv_bfloat16* X16;
+    __nv_bfloat16* Y16;
     int N, K;
     const int* cnt; int cnt_gstride;                   // rows of group g = cnt[g * cnt_gstride]
     const int* off;                                    // first compact row of group g (nullptr: 0)

@@ -263,7 +263,9 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
                                 if (in && n < l.split) yr[n] = v[j] + bias;
                                 else if (in && (lane & 1) == 0) l.Y2[(size_t)(yrow0 + c + j) * l.ldy2 + ((n - l.split) >> 1)] = fmaxf(v[j], 0.f) * up;
                             } else if (in && (lane & 1) == 0) {
-                                yr[n >> 1] = EPI == LE_GLU_CLAMP ? lin_glu(v[j], up, l.limit) : v[j] * lin_sigmoid(v[j]) * up;
+                                const float y = EPI == LE_GLU_CLAMP ? lin_glu(v[j], up, l.limit) : v[j] * lin_sigmoid(v[j]) * up;
+                                if (l.Y16) l.Y16[(size_t)(yrow0 + c + j) * l.ldy + (n >> 1)] = __float2bfloat16(y);
+                                else yr[n >> 1] = y;
                             }
                         } else if (in) {
                             const float a = v[j] + bias;

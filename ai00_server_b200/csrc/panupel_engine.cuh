@@ -159,12 +159,18 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
         p.X = X; p.ldx = ldx; p.W = Wt; p.Y = Y; p.ldy = ldy; p.N = N_; p.K = K_; p.cnt = cntT; p.epi = epi; p.bias = bias;
         return p;
     };
+    // prompt steps: the norm and the gated units leave their projections' bf16 operands
+    const bool x16 = rows > 16 && m.h16 && W % 4 == 0 && cdiv(W, 4 * PRE_NORM_VEC_THREADS) <= PRE_NORM_VEC_MAX;
+    auto from_h = [&](LinParams p) {
+        if (x16) p.X16 = m.h16;
+        return p;
+    };
     const float* post_w = nullptr;                 // norm weight of a finished sublayer whose output waits in m.y
     auto boundary = [&](float* snap, float* cat, const float* weight, float* h, int compact, float* hidden) {
         PreNormParams pn{m.x, nullptr, nullptr, nullptr, 0, nullptr, snap, cat ? m.embed : nullptr, nullptr, weight, eps, h, compact, hidden, W, mv,
                          post_w ? m.y : nullptr, post_w, m.cfg.residual_mul, cat};
-        if (rows <= 32) launch_k(pre_norm_kernel<PRE_NORM_THREADS_FEW_ROWS>, dim3(rows), dim3(PRE_NORM_THREADS_FEW_ROWS), (size_t)W * 4, pn, KC_LN, s, prof);
-        else launch_k(pre_norm_kernel<NORM_THREADS>, dim3(rows), dim3(NORM_THREADS), (size_t)W * 4, pn, KC_LN, s, prof);
+        if (x16 && h == m.h) { pn.h = nullptr; pn.h16 = m.h16; }
+        kx_pre_norm(s, prof, pn, rows);
         post_w = nullptr;
     };
     const int chunks_grid = decode ? rows : cdiv(rows, m.qb_prompt) + nslot_grid;
@@ -177,7 +183,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             kx_lin(s, prof, lin(m.G, 2 * W, m.pass_in, m.x, W, W, 2 * W), rows, 1);
         }
         boundary(nullptr, nullptr, l.norm1_w, m.h, 0, nullptr);
-        kx_lin(s, prof, lin(m.h, W, l.proj, m.pr, PN, l.proj_n, W, LE_STORE, l.proj_b), rows, 1);
+        kx_lin(s, prof, from_h(lin(m.h, W, l.proj, m.pr, PN, l.proj_n, W, LE_STORE, l.proj_b)), rows, 1);
         int KO = H_ * dv;                          // heads' outputs side by side, the input of the output projection
         if (c.mixer == KX_PARALLEL) {
             const PnParallelRow r(c);
@@ -226,8 +232,10 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
         post_w = l.norm1b_w;
         if (c.has_mlp) {
             boundary(nullptr, nullptr, l.norm2_w, m.h, 0, nullptr);
-            kx_lin(s, prof, lin(m.h, W, l.sh_gu, m.ys, c.ff, 2 * c.ff, W, LE_GLU_SILU), rows, 1);
-            kx_lin(s, prof, lin(m.ys, c.ff, l.sh_down, m.y, W, W, c.ff), rows, 1);
+            LinParams gu = from_h(lin(m.h, W, l.sh_gu, m.ys, c.ff, 2 * c.ff, W, LE_GLU_SILU)), down = lin(m.ys, c.ff, l.sh_down, m.y, W, W, c.ff);
+            if (x16 && m.ys16 && c.ff % 8 == 0) { gu.Y16 = m.ys16; down.X16 = m.ys16; }
+            kx_lin(s, prof, gu, rows, 1);
+            kx_lin(s, prof, down, rows, 1);
             post_w = l.norm2b_w;
         }
         if (m.dbg_layers && !use_graph)            // bring-up aid: the residual as this run leaves it

@@ -166,8 +166,7 @@ void b200rwkv_engine::ps_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
     Pending pend;
     auto boundary = [&](float* snap, const __nv_bfloat16* table, const float* vec, const float* weight, float* h, int compact, float* hidden) {
         PreNormParams pn{m.x, pend.rows, m.row_of, m.wgt, pend.top, pend.shared, snap, table, vec, weight, m.cfg.eps, h, compact, hidden, W, mv};
-        if (rows <= 32) launch_k(pre_norm_kernel<PRE_NORM_THREADS_FEW_ROWS>, dim3(rows), dim3(PRE_NORM_THREADS_FEW_ROWS), (size_t)W * 4, pn, KC_LN, s, prof);
-        else launch_k(pre_norm_kernel<NORM_THREADS>, dim3(rows), dim3(NORM_THREADS), (size_t)W * 4, pn, KC_LN, s, prof);
+        kx_pre_norm(s, prof, pn, rows);
         pend = Pending();
     };
     const int chunks_grid = decode ? rows : cdiv(rows, m.qb_prompt) + nslot_grid;

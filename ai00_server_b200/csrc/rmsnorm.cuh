@@ -278,6 +278,7 @@ struct PreNormParams {
     float* cat = nullptr;             // [T, 2 W] (nullptr: none)
     const float* y2 = nullptr;        // [T, W] a second output (nullptr: none; only beside y)
     const float* post2_w = nullptr;   // [W]
+    __nv_bfloat16* h16 = nullptr;     // [T, W] the normed row as the next projection's bf16 operand (nullptr: none; h may be null then)
 };
 
 constexpr int PRE_NORM_THREADS_FEW_ROWS = 1024;    // block size for steps of few tokens (decode): a thread then owns one or two columns
@@ -352,6 +353,87 @@ __global__ void __launch_bounds__(THREADS) pre_norm_kernel(const PreNormParams p
     ss = rms_block_sum(ss, red);
     const float r = 1.f / sqrtf(ss / (float)W + p.eps);
     for (int c = threadIdx.x; c < W; c += blockDim.x) p.h[(size_t)row * W + c] = pre_norm_row[c] * r * p.weight[c];
+}
+
+// The same boundary without routed rows, for widths of whole float4: a thread keeps its columns in registers, every load of the row is
+// requested before the first sum.  (The scalar form walked the row three times through shared memory.  Measured at width 2048, ncu: 14 ->
+// 7.9 us for 512 rows, 7.5 -> 4.8 for 16.)
+constexpr int PRE_NORM_VEC_THREADS = 256, PRE_NORM_VEC_MAX = 8;
+
+template <int NV>
+__global__ void __launch_bounds__(PRE_NORM_VEC_THREADS) pre_norm_vec_kernel(const PreNormParams p) {
+    __shared__ float red[32];
+    pdl_launch_dependents();
+    const int W = p.W, t = blockIdx.x;
+    float4 w[NV], pw[NV], pw2[NV];                      // weights are no kernel's output: requested before the wait
+    auto each = [&](auto&& f) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int c = 4 * (threadIdx.x + PRE_NORM_VEC_THREADS * j);
+            if (c < W) f(j, c);
+        }
+    };
+    auto ld = [](const float* q) { return *reinterpret_cast<const float4*>(q); };
+    each([&](int j, int c) {
+        if (p.weight) w[j] = ld(p.weight + c);
+        if (p.y) pw[j] = ld(p.post_w + c);
+        if (p.y2) pw2[j] = ld(p.post2_w + c);
+    });
+    pdl_wait();
+    if (t >= p.meta.T()) return;
+    const size_t at = (size_t)t * W;
+    const __nv_bfloat16* er = p.table ? p.table + (size_t)p.meta.tok()[t] * W : nullptr;
+    float4 x[NV], y[NV], y2[NV], em[NV];
+    each([&](int j, int c) {
+        x[j] = ld(p.x + at + c);
+        if (p.y) y[j] = ld(p.y + at + c);
+        if (p.y2) y2[j] = ld(p.y2 + at + c);
+        em[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (er) {
+            const uint2 q = *reinterpret_cast<const uint2*>(er + c);
+            const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+            em[j] = make_float4(a.x, a.y, b.x, b.y);
+        }
+    });
+    auto sq = [](const float4 v) { return (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); };
+    auto madd = [](float4& a, const float4 v, const float r, const float4 g) { a.x += v.x * r * g.x; a.y += v.y * r * g.y; a.z += v.z * r * g.z; a.w += v.w * r * g.w; };
+    auto add = [](float4& a, const float4 v) { a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w; };
+    auto apply = [&](const float4 (&v)[NV], const float4 (&g)[NV]) {
+        float ss = 0.f;
+        each([&](int j, int) { ss += sq(v[j]); });
+        const float r = p.post_mul / sqrtf(rms_block_sum(ss, red) / (float)W + p.eps);
+        each([&](int j, int) { madd(x[j], v[j], r, g[j]); });
+    };
+    if (p.y) apply(y, pw);
+    if (p.y2) apply(y2, pw2);
+    const bool writes = p.y || (er && !p.cat) || p.vec;
+    float ss = 0.f;
+    each([&](int j, int c) {
+        auto st = [&](float* q, const float4 v) { *reinterpret_cast<float4*>(q) = v; };
+        if (p.snap) st(p.snap + at + c, x[j]);
+        if (p.cat) {
+            st(p.cat + 2 * at + c, x[j]);
+            st(p.cat + 2 * at + W + c, em[j]);
+        } else if (er) {
+            add(x[j], em[j]);
+        }
+        if (p.vec) add(x[j], ld(p.vec + c));
+        if (writes) st(p.x + at + c, x[j]);
+        if (p.hidden) st(p.hidden + at + c, x[j]);
+        ss += sq(x[j]);
+    });
+    if (!p.weight) return;
+    const int row = p.compact ? p.meta.tok_outrow()[t] : t;
+    if (row < 0) return;
+    const float r = 1.f / sqrtf(rms_block_sum(ss, red) / (float)W + p.eps);
+    each([&](int j, int c) {
+        const float4 h = make_float4(x[j].x * r * w[j].x, x[j].y * r * w[j].y, x[j].z * r * w[j].z, x[j].w * r * w[j].w);
+        if (p.h) *reinterpret_cast<float4*>(p.h + (size_t)row * W + c) = h;
+        if (p.h16) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(h.x, h.y), hi = __floats2bfloat162_rn(h.z, h.w);
+            *reinterpret_cast<uint2*>(p.h16 + (size_t)row * W + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+    });
 }
 
 }  // namespace b200

@@ -112,6 +112,13 @@ def test_projections_of_a_step_of_few_rows(n, ff):
     _check_family(synth.make_panupel, [synth.panupel_layer("delta", heads=3, dim=24, ff=ff)], panupel_numpy, n, width=136)
 
 
+@pytest.mark.parametrize("n", [5, 40])
+@pytest.mark.parametrize("width", [138, 1020, 1028, 2056, 4104])
+def test_boundaries_of_a_row_of_n_columns(width, n):
+    """Rows of 1 .. 8 float4 a thread, of whole float4 without whole bf16 operands (1020), and of neither (138)."""
+    _check_family(synth.make_panupel, [synth.panupel_layer("delta", heads=2, dim=24, ff=48)], panupel_numpy, n, width=width)
+
+
 def test_a_nan_stays_one_in_latent_attention():
     """A key that is not a number makes every later row so (rounding to TF32 by integer arithmetic must not turn it into a number)."""
     cfg, st, _ = synth.make_kemirax([synth.kemirax_layer("latent_attention", mlp=False)], seed=4)
