@@ -379,6 +379,17 @@ static bool state_from_st(const StFile& st, int L, int H, int N, int C, std::vec
 static inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 static inline int rup(int a, int b) { return cdiv(a, b) * b; }
 
+// dynamic shared memory a kernel may be launched with.  The limit belongs to the process, not to an engine: it is only ever raised, so that a
+// narrower model loaded later leaves the launches of a wider one valid
+template <typename K>
+static void allow_smem(K* kern, size_t bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes a;
+    CK(cudaFuncGetAttributes(&a, kern));
+    if ((size_t)a.maxDynamicSharedSizeBytes < bytes) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 enum KClass { KC_GEMM = 0, KC_WKV = 1, KC_LN = 2, KC_OTHER = 3 };
 
 struct GemmLaunch {
@@ -1009,7 +1020,7 @@ void b200rwkv_engine::build(const StFile& st) {
         CK(cudaFuncSetAttribute(wkv_kernel<6, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
         CK(cudaFuncSetAttribute(wkv_kernel<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
     }
-    CK(cudaFuncSetAttribute(ln_mix_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (LN_ROWS + 1) * C * 4));
+    allow_smem(ln_mix_rows_kernel, (size_t)(LN_ROWS + 1) * C * 4);
     if (precision == 1) split_act = true;         // f32-activation mode (web-rwkv `Bundle::<f32>`): no activation is rounded to f16
     if (const char* v = dbg_env("B200RWKV_PREFETCH_BLOCKS")) prefetch_blocks = std::max(0, atoi(v));
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;

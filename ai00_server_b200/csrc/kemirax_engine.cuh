@@ -266,14 +266,13 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     connected = true;
 
     if (m.max_D > 0) {
-        const int smem = (int)latent_attn_smem<1, 16>(m.max_D);
-        CK(cudaFuncSetAttribute(latent_attn_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        CK(cudaFuncSetAttribute(latent_attn_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        CK(cudaFuncSetAttribute(latent_attn_kernel<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        const int smem_tc = (int)latent_attn_tc_smem(m.max_D);
-        CK(cudaFuncSetAttribute(latent_attn_tc_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_tc));
-        CK(cudaFuncSetAttribute(latent_attn_tc_kernel<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_tc));
-        CK(cudaFuncSetAttribute(latent_attn_tc_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_tc));
+        const size_t smem = latent_attn_smem<1, 16>(m.max_D), smem_tc = latent_attn_tc_smem(m.max_D);
+        allow_smem(latent_attn_kernel<4, 4>, smem);
+        allow_smem(latent_attn_kernel<1, 16>, smem);
+        allow_smem(latent_attn_kernel<1, 8>, smem);
+        allow_smem(latent_attn_tc_kernel<4, 4>, smem_tc);
+        allow_smem(latent_attn_tc_kernel<1, 16>, smem_tc);
+        allow_smem(latent_attn_tc_kernel<2, 8>, smem_tc);
     }
     CK(cudaFuncSetAttribute(gla_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
