@@ -1604,7 +1604,7 @@ static inline int mt_bucket(int rows) { return rows <= 16 ? 1 : (rows <= 32 ? 2 
 
 // last logits row of every slot of this step -> keep[slot] (rank 0 gathers the vocabulary shards); see sample.cuh
 void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MTR) {
-    if (MTR <= 0 || rank != 0 || !d_keep || Vl % 4 != 0) return;
+    if (MTR <= 0 || rank != 0 || !d_keep) return;
     KeepParams kp;
     memset(&kp, 0, sizeof(kp));
     for (int q = 0; q < world; ++q) kp.shard[q] = (const float*)(peer_base[q] + off_logits);

@@ -254,12 +254,17 @@ __global__ void __launch_bounds__(KEEP_THREADS) keep_rows_kernel(const __grid_co
     pdl_wait();
     if (!live) return;
     float* dst = p.keep + (size_t)slot * p.V;
-    const int n4 = p.Vl >> 2;       // Vl % 4 == 0 is checked by the host
-    for (int q = 0; q < p.world; ++q) {
-        const float4* src = reinterpret_cast<const float4*>(p.shard[q] + (size_t)r * p.Vl);
-        float4* d4 = reinterpret_cast<float4*>(dst + (size_t)q * p.Vl);
-        for (int i = blockIdx.y * KEEP_THREADS + threadIdx.x; i < n4; i += KEEP_CHUNKS * KEEP_THREADS) d4[i] = __ldcg(src + i);
-    }
+    auto copy = [&](auto vec_t) {                           // whole float4 where every row begins on a 16-byte boundary
+        using T = decltype(vec_t);
+        const int n = p.Vl / (int)(sizeof(T) / 4);
+        for (int q = 0; q < p.world; ++q) {
+            const T* src = reinterpret_cast<const T*>(p.shard[q] + (size_t)r * p.Vl);
+            T* d = reinterpret_cast<T*>(dst + (size_t)q * p.Vl);
+            for (int i = blockIdx.y * KEEP_THREADS + threadIdx.x; i < n; i += KEEP_CHUNKS * KEEP_THREADS) d[i] = __ldcg(src + i);
+        }
+    };
+    if ((p.Vl & 3) == 0) copy(float4{});
+    else copy(0.f);
 }
 
 }  // namespace b200
