@@ -312,6 +312,13 @@ __device__ __forceinline__ void trace_stamp(unsigned long long* tr, const int i)
         tr[i] = t;
     }
 }
+// behind the eight stamps of a trace row: {SM id, two times} of every CTA.  CTAs beyond the row's places share one, which keeps the latest time
+constexpr int TRACE_ROW = 512, TRACE_CTAS = (TRACE_ROW - 8) / 3;
+__device__ __forceinline__ void trace_cta(unsigned long long* tr, const int i, const unsigned long long v) {
+    unsigned long long* const at = tr + 8 + 3 * ((blockIdx.x + gridDim.x * blockIdx.y) % TRACE_CTAS) + i;
+    if (i == 0) *at = v;
+    else atomicMax(at, v);
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -624,7 +624,7 @@ struct b200rwkv_engine {
     unsigned long long* d_step_trace = nullptr;
     std::vector<int> step_trace_types;
     static constexpr int STEP_TRACE_MAX = 1024;
-    static constexpr int STEP_TRACE_ROW = 512;     // 8 stamps of CTA 0 + {SM id, last MMA, exit} of every projection CTA
+    static constexpr int STEP_TRACE_ROW = TRACE_ROW;     // 8 stamps of CTA 0 + {SM id, last MMA, exit} of every projection CTA
     bool trace_capture = false;                    // stamps are wired into the launches being enqueued / captured right now
     std::vector<long long> step_trace_bytes;       // algorithmic weight bytes of each traced projection launch
     unsigned long long* tr_next(int label) {
@@ -2708,7 +2708,7 @@ static int32_t rank_profile_insitu(b200rwkv_engine* e, int32_t nslot, const int3
             const bool gemm = e->step_trace_types[i] >= 1000000;
             unsigned long long st = gemm ? q[2] : q[1], en = q[7];
             if (gemm)
-                for (int c = 0; c < e->num_sms && 8 + 3 * c + 2 < (int)row; ++c) en = std::max(en, q[8 + 3 * c + 2]);
+                for (int c = 0; c < TRACE_CTAS; ++c) en = std::max(en, q[8 + 3 * c + 2]);
             if (!st || !en) continue;
             s_acc[i] += (double)(st - t0) * 1e-3;
             e_acc[i] += (double)(en - t0) * 1e-3;

@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, RING == 1 ? 2 : 1) gemm_kernel(c
             if (p.trace) {       // every CTA: SM id and the time its last MMA was issued (skew across the grid)
                 unsigned smid;
                 asm volatile("mov.u32 %0, %smid;" : "=r"(smid));
-                p.trace[8 + 3 * cta] = smid;
-                p.trace[8 + 3 * cta + 1] = globaltimer_ns();
+                trace_cta(p.trace, 0, smid);
+                trace_cta(p.trace, 1, globaltimer_ns());
             }
         }
     } else {
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, RING == 1 ? 2 : 1) gemm_kernel(c
     tc_fence_before();
     __syncthreads();
     if (tid == 0) stamp(7);
-    if (tid == 0 && p.trace) p.trace[8 + 3 * cta + 2] = globaltimer_ns();
+    if (tid == 0 && p.trace) trace_cta(p.trace, 2, globaltimer_ns());
     if (warp == GEMM_EPI_WARPS) tc_dealloc(tmem_base, Cfg::TMEM_COLS);
 }
 

@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
             if (p.trace) {
                 unsigned smid;
                 asm volatile("mov.u32 %0, %smid;" : "=r"(smid));
-                p.trace[8 + 3 * cta] = smid;
-                p.trace[8 + 3 * cta + 1] = globaltimer_ns();
+                trace_cta(p.trace, 0, smid);
+                trace_cta(p.trace, 1, globaltimer_ns());
             }
         }
     } else {
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
     __syncthreads();
     if (tid == 0) {
         trace_stamp(p.trace, 7);
-        if (p.trace) p.trace[8 + 3 * cta + 2] = globaltimer_ns();
+        if (p.trace) trace_cta(p.trace, 2, globaltimer_ns());
     }
     if (warp == WIDE_EPI_WARPS) tc_dealloc(tmem_base, Cfg::TMEM_COLS);
 }

@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(QGEMM_THREADS, 1) qgemm_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     if (tid == 0 && tr) tr[7] = globaltimer_ns();
-    if (tid == 0 && p.trace) p.trace[8 + 3 * cta + 2] = globaltimer_ns();
+    if (tid == 0 && p.trace) trace_cta(p.trace, 2, globaltimer_ns());
     if (warp == GEMM_EPI_WARPS) tc_dealloc(tmem_base, Cfg::TMEM_COLS);
 }
 
