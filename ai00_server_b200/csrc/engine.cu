@@ -2999,7 +2999,7 @@ int32_t b200rwkv_debug_trace(b200rwkv_engine* e, uint64_t* out, size_t cap, int3
 // every launch streams cold weights.  which: 0.. = index into the pre-WKV launches, 10 = output
 // projection, 20/21 = channel-mix launches, 30 = head.  Returns ms per launch and weight bytes.
 int32_t b200rwkv_debug_gemm_time(b200rwkv_engine* e, int32_t which, int32_t reps, float* ms_out, int64_t* bytes_out,
-                                 uint64_t* trace_out /* [L][8] stamps of CTA 0 for the last round, or null */) {
+                                 uint64_t* trace_out /* [L][16] first words of the stamp rows of the last round, or null */) {
     API_BEGIN(e)
     REQUIRE(e && ms_out && bytes_out && reps >= 1, B200RWKV_ERR_INVALID, "bad argument");
     std::lock_guard<std::mutex> lk(e->mu);
@@ -3021,17 +3021,18 @@ int32_t b200rwkv_debug_gemm_time(b200rwkv_engine* e, int32_t which, int32_t reps
     CK(cudaEventCreate(&b));
     const int n = reps * e->L;
     unsigned long long* d_tr = nullptr;
-    if (trace_out) { CK(cudaMalloc(&d_tr, (size_t)e->L * 16 * 8)); CK(cudaMemset(d_tr, 0, (size_t)e->L * 16 * 8)); }
+    DevTmp tr_rows(trace_out ? (size_t)e->L * TRACE_ROW * 8 : 8);
+    if (trace_out) { d_tr = (unsigned long long*)tr_rows.p; CK(cudaMemset(d_tr, 0, (size_t)e->L * TRACE_ROW * 8)); }
     for (int i = 0; i < e->L; ++i) e->launch_gemm(pick(i), 1, e->stream, nullptr);
     CK(cudaEventRecord(a, e->stream));
     for (int i = 0; i < n; ++i) {
         GemmLaunch g = pick(i);
-        if (d_tr && i >= n - e->L) g.p.trace = d_tr + (size_t)(i % e->L) * 16;
+        if (d_tr && i >= n - e->L) g.p.trace = d_tr + (size_t)(i % e->L) * TRACE_ROW;
         e->launch_gemm(g, 1, e->stream, nullptr);
     }
     CK(cudaEventRecord(b, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    if (d_tr) { CK(cudaMemcpy(trace_out, d_tr, (size_t)e->L * 16 * 8, cudaMemcpyDeviceToHost)); CK(cudaFree(d_tr)); }
+    if (d_tr) CK(cudaMemcpy2D(trace_out, 16 * 8, d_tr, TRACE_ROW * 8, 16 * 8, e->L, cudaMemcpyDeviceToHost));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, a, b));
     *ms_out = ms / n;

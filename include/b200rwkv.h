@@ -292,7 +292,8 @@ int32_t b200rwkv_debug_read(b200rwkv_engine*, const char* name, float* out, size
  * front-half kernel); types[i] = 0 LN, 2 WKV, 6 front half, 1000000 + weight MiB for a projection launch. */
 int32_t b200rwkv_debug_trace(b200rwkv_engine*, uint64_t* out, size_t cap, int32_t* types, int32_t* nphase);
 
-/* Profiling aid: one projection launch class timed in isolation over all layers. */
+/* Profiling aid: one projection launch class timed in isolation over all layers; trace_out (optional, [num_layer][16]) receives the first
+ * words of every launch's stamp row. */
 int32_t b200rwkv_debug_gemm_time(b200rwkv_engine*, int32_t which, int32_t reps, float* ms_out, int64_t* bytes_out,
                                  uint64_t* trace_out);
 

@@ -33,3 +33,17 @@ def test_rows_of_launches_with_many_ctas():
         assert (times[:, 1] >= times[:, 0]).all() and np.ptp(times) < 1e9
     finally:
         m.close()
+
+
+def test_stamps_of_one_launch_class():
+    """Every layer's launch has a whole row on the device, of which the first 16 words come back."""
+    shape = dataclasses.replace(synth.PRESETS["tiny6"], L=5)
+    m = runtime.Model(synth.make_st(shape, 1), max_batch=4, token_chunk_size=32)
+    try:
+        ms, nb, tr = C.c_float(0), C.c_int64(0), np.zeros((5, 16), np.uint64)
+        capi.check(capi.lib().b200rwkv_debug_gemm_time(m._h, 10, 2, C.byref(ms), C.byref(nb), capi.ptr(tr)), m._h)
+        entry, leave = tr[:, 0].astype(np.int64), tr[:, 7].astype(np.int64)
+        assert ms.value > 0 and nb.value > 0
+        assert (entry > 0).all() and (leave >= entry).all() and (np.diff(entry) > 0).all()
+    finally:
+        m.close()
