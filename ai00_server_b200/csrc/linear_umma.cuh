@@ -43,7 +43,7 @@ struct LuCfg {
     static constexpr int NSTAGE = 196608 / STAGE_BYTES > 8 ? 8 : 196608 / STAGE_BYTES;
     static constexpr int BAR_OFF = NSTAGE * STAGE_BYTES;
     static constexpr int SMEM_BYTES = BAR_OFF + (2 * NSTAGE + 4) * 8 + 16 + 1024;       // + alignment of the ring
-    static constexpr int TMEM_COLS = 2 * TN;                                            // 64 .. 512: double-buffered accumulator
+    static constexpr int TMEM_COLS = 2 * TN;                                            // 64 .. 256: double-buffered accumulator
 };
 
 // K-major operand in the 128-byte swizzle: 8-row atoms of 1024 bytes; a k16 step is 32 bytes further
@@ -123,7 +123,6 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
     const uint32_t full_bar = ring + Cfg::BAR_OFF, empty_bar = full_bar + Cfg::NSTAGE * 8;
     const uint32_t tfull_bar = empty_bar + Cfg::NSTAGE * 8, tempty_bar = tfull_bar + 16, tmem_slot = tempty_bar + 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    pdl_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < Cfg::NSTAGE; ++s) { mbar_init(full_bar + s * 8, 1); mbar_init(empty_bar + s * 8, 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(tfull_bar + s * 8, 1); mbar_init(tempty_bar + s * 8, LU_EPI_WARPS); }
@@ -135,6 +134,8 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+    // only now: a dependent CTA that took its tensor memory first would wait for this grid while this grid waited for columns
+    pdl_launch_dependents();
     pdl_wait();
     LuWalk<TN> w;
     w.init(p);
