@@ -2382,8 +2382,8 @@ static int32_t rank_state_write(b200rwkv_engine* e, int32_t slot, uint64_t snaps
     else snapshot_copy(e, slot, it->second.buf, false);
     if (e->d_keep && it->second.logits)
         CK(cudaMemcpyAsync(e->d_keep + (size_t)slot * e->V, it->second.logits, (size_t)e->V * 4, cudaMemcpyDeviceToDevice, e->stream));
-    // nothing of the caller's is in flight: later steps follow on the stream, samplers wait for the event, and the record's memory is
-    // given back by cudaFree, which waits for the device
+    // nothing of the caller's is in flight: later steps follow on the stream, samplers wait for the event, and whoever gives the record's
+    // memory back waits for the stream first (rank_state_free)
     CK(cudaEventRecord(e->step_done, e->stream));
     {
         std::lock_guard<std::mutex> lk2(e->keep_mu);
@@ -2399,6 +2399,7 @@ static int32_t rank_state_free(b200rwkv_engine* e, uint64_t snapshot_id) {
     auto it = e->snaps.find(snapshot_id);
     REQUIRE(it != e->snaps.end(), B200RWKV_ERR_STATE, "unknown snapshot id");
     CK(cudaSetDevice(e->dev));
+    CK(cudaStreamSynchronize(e->stream));      // a copy out of the record may still be in flight (rank_state_write)
     CK(cudaFree(it->second.buf));
     if (it->second.logits) CK(cudaFree(it->second.logits));
     e->snaps.erase(it);
