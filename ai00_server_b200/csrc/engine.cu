@@ -640,7 +640,7 @@ struct b200rwkv_engine {
                   const std::vector<int>& outmode /*0 none,1 last,2 full*/, int* R_out);
     void infer(int nslot, const int32_t* slot, const int32_t* ntok, const uint32_t* tokens, const int32_t* option,
                float* logits_out, size_t cap, int32_t* rows_out);
-    void slot_xfer(const std::vector<SlotSeg>& segs, float* rec, int mode, const int* table = nullptr, int page = 1);
+    void slot_xfer(const std::vector<SlotSeg>& whole, float* rec, int mode, const int* table = nullptr, int page = 1);
     void state_xform(int slot, bool import, float* snap = nullptr);
 };
 
@@ -1924,7 +1924,16 @@ void b200rwkv_engine::sample_topk(int nrows, const int32_t* slots, const int32_t
 }
 
 // runs of a slot's memory <-> record (or zero), SLOT_SEGS runs to a launch
-void b200rwkv_engine::slot_xfer(const std::vector<SlotSeg>& segs, float* rec, int mode, const int* table, int page) {
+void b200rwkv_engine::slot_xfer(const std::vector<SlotSeg>& whole, float* rec, int mode, const int* table, int page) {
+    std::vector<SlotSeg> segs;
+    for (SlotSeg s : whole) {
+        const int nl = s.nl, most = std::max(1, SLOT_RUN / std::max(1, s.cnt));
+        for (int l = 0; l < nl; l += most, s.dev += most * s.dev_ls, s.off += most * s.rec_ls) {
+            s.nl = std::min(most, nl - l);
+            s.l0 = l;
+            segs.push_back(s);
+        }
+    }
     for (size_t i = 0; i < segs.size(); i += SLOT_SEGS) {
         const size_t n = std::min<size_t>(SLOT_SEGS, segs.size() - i);
         SlotXfer x;

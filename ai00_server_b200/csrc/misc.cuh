@@ -33,8 +33,10 @@ struct SlotSeg {
     long long dev_ls;        // floats between pieces on the device side (0: cache rows, placed by the page table)
     long long off, rec_ls;   // first float in the record, floats between pieces there
     int cnt, nl;
+    int l0;                  // first piece, counted in rows of the cache
 };
 constexpr int SLOT_SEGS = 24, SLOT_THREADS = 256;
+constexpr int SLOT_RUN = 1 << 22;        // floats of a run (more than one piece): the host cuts longer ones, so that 32-bit indices hold
 enum SlotMode { SLOT_EXPORT, SLOT_IMPORT, SLOT_ZERO };
 struct SlotXfer {
     float* rec;
@@ -51,7 +53,7 @@ __global__ void __launch_bounds__(SLOT_THREADS) slot_xfer_kernel(const __grid_co
         const int per = s.cnt / V, total = per * s.nl;
         for (int i = blockIdx.x * SLOT_THREADS + threadIdx.x; i < total; i += gridDim.x * SLOT_THREADS) {
             const int l = i / per, e = i - l * per;
-            const size_t at = s.dev_ls ? (size_t)l * s.dev_ls : ((size_t)p.table[l / p.page] * p.page + l % p.page) * s.cnt;
+            const size_t at = s.dev_ls ? (size_t)l * s.dev_ls : ((size_t)p.table[(s.l0 + l) / p.page] * p.page + (s.l0 + l) % p.page) * s.cnt;
             T* const d = reinterpret_cast<T*>(s.dev + at) + e;
             if (p.mode == SLOT_ZERO) { *d = T{}; continue; }
             T* const r = reinterpret_cast<T*>(p.rec + s.off + (size_t)l * s.rec_ls) + e;

@@ -24,3 +24,25 @@ def test_a_record_freed_right_behind_its_write():
             b.free()
     finally:
         m.close()
+
+
+@pytest.mark.parametrize("rank", [512, 510])
+def test_a_long_sequence_of_cache_rows(rank):
+    """A run of cache rows longer than one run of the transfer kernel (2^22 floats), of whole float4 and of single floats."""
+    cfg, st, _ = synth.make_kemirax([synth.kemirax_layer("latent_attention", heads=1, kv_rank=rank, mlp=False)], seed=4)
+    n = 8120
+    m = runtime.Model(st, max_batch=2, token_chunk_size=512, config=cfg, kv_tokens=2 * n + 64, kv_page=32)
+    try:
+        toks = np.random.default_rng(1).integers(1, 90, n).tolist()
+        m.state.reset(0)
+        m.state.reset(1)
+        m.infer_raw([0], [n], toks, [capi.OPTION_LAST])
+        assert n * (rank + 8) > 1 << 22
+        snap = m.state.read(0)
+        m.state.write(snap, 1)
+        assert np.array_equal(m.state.back(1), m.state.back(0))
+        a, b = m.infer_raw([0, 1], [1, 1], [5, 5], [capi.OPTION_LAST] * 2)
+        assert np.array_equal(a, b)
+        snap.free()
+    finally:
+        m.close()
