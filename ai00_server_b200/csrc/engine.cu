@@ -481,6 +481,8 @@ struct b200rwkv_engine {
     bool use_graph = true, use_pdl = true;
     // config.json families: every kernel triggers its dependents and waits for the kernel in front of it at its start, so that a launch
     // right behind another on the same stream overlaps that kernel's tail (a join has more than one kernel in front: full dependency)
+    // Not in f32-exact models: their prompt projections are a few long CTAs of plain FMA, and CTAs placed beside waiting ones share SMs while
+    // others idle (width 1024, steps of 64 rows: 5.3 -> 6.5 ms of two Panupel layers, 4.0 -> 4.6 Kemirax, 2.9 -> 3.9 Zufulix with the edges)
     cudaStream_t pdl_prev = nullptr;   // stream of the last launch, null behind a join
     bool planning = false;             // a walk over the launches of a step that launches nothing (workspace sizes)
     int split_att = 1, split_ffn = 1;
@@ -904,7 +906,7 @@ void b200rwkv_engine::launch_k(void (*kern)(P, X...), dim3 grid, dim3 block, siz
         ++na;
         launch_cluster = 0;
     }
-    if ((use_pdl || (kx && pdl_prev == s)) && !prof) {
+    if ((use_pdl || (kx && !kx->exact && pdl_prev == s)) && !prof) {
         at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[na].val.programmaticStreamSerializationAllowed = 1;
         ++na;
