@@ -1843,7 +1843,7 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
 void b200rwkv_engine::topk_setup() {
     if (V > TOPK_MAX_V) return;        // larger vocabularies: b200rwkv_sample_topk answers UNSUPPORTED
     CK(cudaMallocHost(&tk_out, (size_t)S * TOPK_MAX * 8));
-    CK(cudaFuncSetAttribute(topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TOPK_SMEM));
+    CK(cudaFuncSetAttribute(topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)topk_smem(TOPK_MAX_V)));
 }
 
 // GPU sampling front half (sample.cuh).  Runs on the softmax stream under the softmax mutex: the reference samples from the
@@ -1918,7 +1918,7 @@ void b200rwkv_engine::sample_topk(int nrows, const int32_t* slots, const int32_t
         tp.slot = (const int*)(tk_dev + o_slot);
         CK(cudaMemcpyAsync(tk_dev, tk_host, total, cudaMemcpyHostToDevice, sm_stream));
     }
-    topk_kernel<<<dim3(TOPK_CTAS, nrows), TOPK_THREADS, TOPK_SMEM, sm_stream>>>(tp);
+    topk_kernel<<<dim3(TOPK_CTAS, nrows), TOPK_THREADS, topk_smem(V), sm_stream>>>(tp);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(sm_stream));
     memcpy(ids_out, tp.out_id, (size_t)nrows * top_k * 4);

@@ -38,7 +38,10 @@ constexpr int TOPK_MAX_V = TOPK_CTAS * TOPK_SLICE;              // 65536
 constexpr int TOPK_LIST = 4096;                                 // candidates of a CTA before it cuts them (127 threads x 32 at most)
 constexpr int TOPK_SHARE = 512;                                 // candidates a CTA may share
 constexpr int TOPK_INLINE = 64;                                 // rows whose slots travel as kernel parameters
-constexpr size_t TOPK_SMEM = (size_t)TOPK_LIST * 8 + (size_t)TOPK_CTAS * TOPK_SHARE * 8;
+__host__ __device__ constexpr int topk_slice(int V) { return ((V + TOPK_CTAS - 1) / TOPK_CTAS + 3) & ~3; }      // elements of a CTA
+// entries of its list, and bytes of shared memory (a small vocabulary cannot fill either: more CTAs to an SM)
+__host__ __device__ constexpr int topk_list(int V) { return topk_slice(V) < TOPK_LIST ? topk_slice(V) : TOPK_LIST; }
+__host__ __device__ constexpr size_t topk_smem(int V) { return ((size_t)topk_list(V) + (size_t)TOPK_CTAS * (topk_slice(V) < TOPK_SHARE ? topk_slice(V) : TOPK_SHARE)) * 8; }
 
 struct TopkParams {
     const float* keep;          // [S][V] last logits row of every slot
@@ -74,35 +77,37 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char topk_smem[];
-    unsigned long long* const list = reinterpret_cast<unsigned long long*>(topk_smem);      // [TOPK_LIST], shared: the first TOPK_SHARE
-    unsigned long long* const all = list + TOPK_LIST;                                       // [TOPK_CTAS * TOPK_SHARE]
-    float* const sx = reinterpret_cast<float*>(topk_smem);                                  // [TOPK_SLICE] while lists are applied
+    unsigned long long* const list = reinterpret_cast<unsigned long long*>(topk_smem);      // [topk_list(V)], shared: the first TOPK_SHARE
+    unsigned long long* const all = list + topk_list(p.V);                                  // [TOPK_CTAS * TOPK_SHARE]
+    float* const sx = reinterpret_cast<float*>(topk_smem);                                  // [cnt] while lists are applied
     __shared__ unsigned long long s_best[TOPK_THREADS];
     __shared__ unsigned long long s_few, s_full;            // the (top_k / 8)-th and the top_k-th best thread
     __shared__ float2 s_stat;                               // (max, sum exp(x - max)) of the slice
     __shared__ float red[32];
     __shared__ int s_n;
     const int cta = blockIdx.x, row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int slice = ((p.V + TOPK_CTAS - 1) / TOPK_CTAS + 3) & ~3;
+    const int slice = topk_slice(p.V);
     const int lo = min(cta * slice, p.V), cnt = min(lo + slice, p.V) - lo;
     const float* const src = p.keep + (size_t)(p.slot ? p.slot[row] : p.slot_inline[row]) * p.V + lo;
-    const bool vec = (p.V & 3) == 0;                        // rows and slices start on 16-byte boundaries
+    // slices below four elements a thread are dealt out one by one: with whole float4 too few threads would hold any for the bounds below
+    const bool quads = slice >= 4 * TOPK_THREADS, vec = quads && (p.V & 3) == 0;        // (rows and slices start on 16-byte boundaries)
+    auto index = [&](int j) { return quads ? ((j >> 2) * TOPK_THREADS + tid) * 4 + (j & 3) : j * TOPK_THREADS + tid; };     // place of x[j] in the slice
     float x[TOPK_PER_THREAD];
 #pragma unroll
     for (int q = 0; q < TOPK_PER_THREAD / 4; ++q) {
-        const int i = (q * TOPK_THREADS + tid) * 4;
+        const int i = index(4 * q);
         if (vec && i + 3 < cnt) {
             const float4 v = __ldcg(reinterpret_cast<const float4*>(src + i));
             x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
         } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) x[4 * q + e] = i + e < cnt ? __ldcg(src + i + e) : -INFINITY;
+            for (int e = 0; e < 4; ++e) x[4 * q + e] = index(4 * q + e) < cnt ? __ldcg(src + index(4 * q + e)) : -INFINITY;
         }
     }
-    auto index = [&](int j) { return ((j >> 2) * TOPK_THREADS + tid) * 4 + (j & 3); };      // place of x[j] in the slice
     if (p.pen_off || p.bias_off || p.allow) {
 #pragma unroll
-        for (int j = 0; j < TOPK_PER_THREAD; ++j) sx[index(j)] = x[j];
+        for (int j = 0; j < TOPK_PER_THREAD; ++j)
+            if (index(j) < cnt) sx[index(j)] = x[j];
         __syncthreads();
         auto apply = [&](const int* off, const unsigned* tok, const float* val, const float sign) {
             for (int e = off[row] + tid; e < off[row + 1]; e += TOPK_THREADS) {
@@ -122,7 +127,8 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
         if (p.bias_off) apply(p.bias_off, p.bias_tok, p.bias_val, 1.f);
         __syncthreads();
 #pragma unroll
-        for (int j = 0; j < TOPK_PER_THREAD; ++j) x[j] = sx[index(j)];
+        for (int j = 0; j < TOPK_PER_THREAD; ++j)
+            if (index(j) < cnt) x[j] = sx[index(j)];
     }
     // softmax statistics of the slice, best key of the thread
     float mx = -INFINITY;
