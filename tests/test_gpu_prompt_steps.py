@@ -73,6 +73,9 @@ def test_last_hidden_answers_the_last_portion(lens, rows):
 # serving precision of the config.json families: bf16 operands (2^-9 each), f32 sums.  A row of a few layers is off by a few of those
 # roundings, a few percent where a norm divides by a small read-out; a wrong tile, edge or row list is off by its own size
 BF16_TOL = 5e-2
+# every single row, the last of a tile among them: a row that was not computed (zeros) is off by its own size, 1, one that holds another row's
+# or stale sums by about 1.4
+ROW_TOL = 0.5
 
 
 def _check_family(make, layers, module, n, **kw):
@@ -84,7 +87,7 @@ def _check_family(make, layers, module, n, **kw):
         got = m.infer_raw([0], [n], toks, [capi.OPTION_FULL])[0]
         want = module.run(json.loads(cfg), w, toks)
         err = np.sqrt(((got - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean())
-        assert np.median(err) <= BF16_TOL and (err <= 4 * BF16_TOL).mean() >= 0.98, (n, float(np.median(err)), float(err.max()))
+        assert np.median(err) <= BF16_TOL and err.max() <= ROW_TOL, (n, float(np.median(err)), int(err.argmax()), float(err.max()))
     finally:
         m.close()
 
