@@ -62,6 +62,8 @@ struct QGemmCfg {
     static constexpr int TMEM_COLS = NEED_COLS <= 32 ? 32 : (NEED_COLS <= 64 ? 64 : (NEED_COLS <= 128 ? 128 : (NEED_COLS <= 256 ? 256 : 512)));
     static_assert(NEED_COLS <= 512, "tensor memory has 512 columns");
     static_assert(NSTAGE >= 2, "ring needs two stages");
+    // a group sees only every second use of a stage of an odd ring; the buffer it waits for (used NBUF blocks ago) tells that the use between has landed
+    static_assert(NSTAGE % Q_DQ_GROUPS == 0 || NSTAGE >= NBUF + Q_DQ_GROUPS, "an expansion group could take an older phase of a stage for the one it waits for");
     static_assert(RAW_W % 128 == 0 && STAGE_BYTES % 128 == 0, "stage blocks stay 128-byte aligned");
 };
 
