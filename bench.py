@@ -168,8 +168,9 @@ def prefill_main(args):
     steps, warm = max(1, min(args.steps, 4)), max(3, args.warmup if args.warmup < 8 else 3)
     metric = f"prefill tokens/s {MODEL_NAMES.get(preset, preset)} fp16 {B}x{Tn}-token inputs (embeddings route)"
     st = synth.make_st(shape, 0)
-    PASS = 128                                              # tokens per weight pass (the engine's largest step)
-    model = runtime.Model(st, max_batch=B, token_chunk_size=PASS, device=0)
+    CHUNK, QUOTA = 128, 4                                   # a portion's tokens; what a sequence gets of one while many prompts wait
+    PASS = 2 * CHUNK                                        # tokens per weight pass: an f16 model on one GPU packs two full portions to a step
+    model = runtime.Model(st, max_batch=B, token_chunk_size=CHUNK, device=0)
     slots = list(range(B))
     rng = np.random.default_rng(1234)
     toks = rng.integers(1, min(shape.V, 65530), size=(B, Tn), dtype=np.int64)
@@ -232,7 +233,8 @@ def prefill_main(args):
     for j in range(nt):
         model.infer_raw(slots[:nb], [1] * nb, toks[:nb, j].tolist(), [capi.OPTION_NONE] * nb)
     dec_vs_pre = [float(np.abs(model.state.back(i) - got[i]).max() / np.abs(got[i]).max()) for i in range(nb)]
-    # where a pass goes: in-situ windows of one 128-slot x 1-token step (the shape every prefill pass has here)
+    # the launches of a pass, as far as a replay of one token per slot shows them: the projections are those of the measured passes (as many
+    # token rows), the recurrence is not (one token a slot runs the decode kernel, the measured passes the scan kernel)
     breakdown = None
     try:
         wins, step_us = model.profile_insitu(slots[:PASS], toks[:PASS, 0].astype(np.uint32), reps=3)
@@ -242,13 +244,14 @@ def prefill_main(args):
             name = "gemm" if ty >= 1000000 else {0: "ln_mix", 2: "wkv", 6: "front_half"}.get(ty, "ln_mix")
             a = agg.setdefault(name, [0.0, 0])
             a[0] += wdw["end_us"] - wdw["start_us"]; a[1] += 1
-        breakdown = {"step_us": step_us, "class_us": {k: v[0] for k, v in agg.items()}, "class_launches": {k: v[1] for k, v in agg.items()}}
+        breakdown = {"shape": f"{len(slots[:PASS])} slots x 1 token (decode recurrence, not the measured scan)", "step_us": step_us, "class_us": {k: v[0] for k, v in agg.items()}, "class_launches": {k: v[1] for k, v in agg.items()}}
     except Exception as ex:                                  # profiling is evidence, not the measurement
         breakdown = {"error": str(ex)}
     peaks, peak_src = read_peaks()
     n_pass = -(-ntok // PASS)
+    pass_seqs = min(B, max(1, CHUNK // max(QUOTA, CHUNK // B)))             # sequences whose state a pass reads and writes
     wbytes = 2 * (synth.num_params(shape) - shape.V * shape.C)              # every pass streams all weights but the embedding
-    pass_bytes = wbytes + PASS * 2 * shape.L * (shape.H * 64 * 64 + 2 * shape.C) * 4
+    pass_bytes = wbytes + pass_seqs * 2 * shape.L * (shape.H * 64 * 64 + 2 * shape.C) * 4
     flops = 2.0 * (synth.num_params(shape) - 2 * shape.V * shape.C) * ntok  # no head: the route needs no logits
     line = {"metric": metric, "value": ntok / dt, "unit": "tokens/s", "n_gpus": 1, "steps": steps, "warmup": warm,
             "ms_per_step": dt * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f16", "data": "synthetic",
@@ -256,18 +259,18 @@ def prefill_main(args):
                        "preset": preset, "seqs": B, "seq_len": Tn, "tokens_per_pass": PASS,
                        "l2": f"inputs larger than L2 (5.9 GB of weights streamed per {PASS}-token pass), no flush"},
             "clocks": clocks,
-            "e2e": {"value": ntok / de, "unit": "tokens/s", "ms_per_step": de * 1e3, "h2d_bytes_per_step": int(ntok * 4 + n_pass * 1800),
+            "e2e": {"value": ntok / de, "unit": "tokens/s", "ms_per_step": de * 1e3, "h2d_bytes_per_step": int(n_pass * 4 * (8 + 6 * PASS + 3 * B)),       # step metadata, token ids included
                     "d2h_bytes_per_step": int(state_buf.nbytes),
                     "api": "b200rwkv_infer (host token ids, OPTION_NONE) + b200rwkv_state_back of every slot (the embedding, run.rs:984-989)"},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "hbm", "kernel": f"gemm_kernel<8> ({PASS}-token passes: every pass streams all projection weights once)",
+            "roofline": {"bound": "hbm", "kernel": f"gemm_wide_kernel<16> ({PASS}-token passes: every pass streams all projection weights once)",
                          "achieved": n_pass * pass_bytes / dt / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": n_pass * pass_bytes / dt / 1e9 / peaks["hbm_gbs"], "traffic": None,
                          "peak_source": f"MEASURED_PEAKS.json ({peak_src})", "passes": n_pass, "bytes_per_pass": int(pass_bytes),
                          "tensor_tflops_achieved": flops / dt / 1e12, "tensor_tflops_peak_sustained": peaks.get("bf16_tflops_sustained"),
-                         "note": f"the route turns tensor-bound at >= 280 FLOP/B = ~300 tokens per weight pass; at {PASS} tokens per pass "
-                                 "(shared memory: 32 KB weights + 32 KB tokens per stage, TMEM: 256 of 512 columns) it is still bound by "
-                                 "streaming the weights, which is what `achieved` measures"},
+                         "note": f"the route turns tensor-bound at >= 280 FLOP/B = ~300 tokens per weight pass; at {PASS} tokens a stage is 16 KB of "
+                                 "weights and 32 KB of tokens and the accumulators take all 512 TMEM columns; `achieved` is the weight "
+                                 "(and state) stream, tensor_tflops_achieved the arithmetic"},
             "cpu_baseline": {"value": nb * nt / cdt, "unit": "tokens/s", "cores": rc.num_threads(), "kind": "port",
                              "sample": f"first {nt} tokens of the first {nb} sequences, C/OpenMP oracle (token by token)"},
             "pass_breakdown": breakdown,
