@@ -43,8 +43,8 @@ __device__ __forceinline__ void rot_cos_sin(int pos, double freq, float& cs, flo
 // canonical K-major / no-swizzle operand of `th` token rows, which ONE tcgen05.mma with N = th consumes:
 //   [k block (128 k)][k8 chunk 16][th token rows][8 halves]      (8 rows x 16 B = one 128-byte core matrix)
 // th = 16 x (token tiles of the step) = 16 / 32 / 64 / 128 / 256; a step's producers and consumers agree on it (the engine passes
-// it to every launch).  Measured (profiles/r02_findings.md §8): a tcgen05.mma with N = 16 costs ~80 cycles whatever N is, so
-// eight N = 16 MMAs per k step (128-token steps) made the projections MMA-bound; one N = 128 MMA does not.
+// it to every launch).  One MMA of N = th takes the tensor core's time (16 tokens 39 cycles, 64 48, 128 64, 256 128, with compile-time
+// descriptors), eight of N = 16 five times that.
 // Split operands (precision 1): th = 32, rows 0-15 hold the hi halves of the 16 tokens, rows 16-31 the lo halves.
 // Every buffer reserves 256 token rows per k block and K padded to whole k blocks (padding k is multiplied by zero weights).
 // ---------------------------------------------------------------------------------------
@@ -58,7 +58,7 @@ __device__ __forceinline__ __half f2h_sat(float v) {
     v = fminf(fmaxf(v, -65504.f), 65504.f);
     return __float2half_rn(v);
 }
-// Split operand (precision 1 = f32 activations, DESIGN.md §2): a projection input v travels as two f16 numbers hi + lo = v
+// Split operand (precision 1 = f32 activations): a projection input v travels as two f16 numbers hi + lo = v
 // (to ~2^-22 relative); hi sits at token row t, lo at row t + 16 of the same A16 buffer (the second 16-token tile), the
 // projection multiplies both tiles and its epilogue adds the two accumulator tiles.
 __device__ __forceinline__ void split_h(const float v, __half& hi, __half& lo) {

@@ -845,7 +845,7 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
     else {
         // Whole tiles per CTA whenever that keeps >= 3/4 of the SMs streaming (one SM draws ~48 B/ns from HBM, so 81 whole tiles of a 3B
         // layer take 17-19 us where 148 CTAs with cut tiles take 15.5): no cross-CTA fix-up in the tail, and
-        // (measured, profiles/r01_findings.md §7) grids of <= 16 CTAs per GPC finish together while 144-148 CTAs skew
+        // (measured) grids of <= 16 CTAs per GPC finish together while 144-148 CTAs skew
         // by 25 % because the 18/20-SM GPCs share the same GPC bandwidth as the 16-SM ones.
         if (tile <= num_sms && tile * 4 >= num_sms * 3) g.grid = tile;
         else if (tile > num_sms)
@@ -946,7 +946,7 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
         p.max_contrib = wide ? g.max_contrib_wide : g.max_contrib;
         launch_k(kern, dim3(wide ? g.grid_wide : g.grid, wide && g.short_k ? g.short_parts : 1), dim3(WIDE_THREADS), smem, p, KC_GEMM, s, prof, (int)(wide && g.by_tile), g.total_tiles);
     };
-    // RING 2 = one stage less than fits, so the small kernels around a projection can share its SMs (findings r1 §7)
+    // RING 2 = one stage less than fits, so the small kernels around a projection can share its SMs
     switch (MT) {
         case 1:
             if (split) launch_k(gemm_kernel<2, 2, true>, dim3(g.grid), dim3(GEMM_THREADS), GemmCfg<2, 2>::SMEM_BYTES, g.p, KC_GEMM, s, prof);
@@ -966,7 +966,7 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
 }
 
 // static split-K factor of a row-parallel projection: the S <= 8 / world (partial buffers the LN stages sum) that cuts K
-// into whole 128-wide blocks, gives every CTA whole tiles and puts the most SMs to work.  (Measured, round 2: with the
+// into whole 128-wide blocks, gives every CTA whole tiles and puts the most SMs to work.  (Measured: with the
 // old cap of 4 the 3B channel-mix value projection ran on 40 CTAs, 22 us for 43 MB; 7 slices -> 140 CTAs.)
 int b200rwkv_engine::pick_split(int K, int tiles) const {
     if (dbg_env("B200RWKV_NOSPLIT")) return 1;
@@ -1188,7 +1188,7 @@ void b200rwkv_engine::build(const StFile& st) {
                 sv.push_back(d);
                 ly.pre.push_back(make_launch(sv));
             }
-            // W2: [5, C, Dm]; order w,k,v,r,g (SURVEY.md App. A)
+            // W2: [5, C, Dm]; order w,k,v,r,g
             {
                 static const char* names[5] = {"time_mix_w", "time_mix_k", "time_mix_v", "time_mix_r", "time_mix_g"};
                 std::vector<SegDesc> sv;
@@ -1711,7 +1711,7 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
     // the weight stream): the portions, and with them the rows b200rwkv_last_hidden answers, are those of 128-token steps
     const int substeps = !kx && step_cap == 128 && maxT >= 256 ? 2 : 1;
     // Step packing: every step shares its token budget evenly over the entries that still have tokens (web-rwkv shares the
-    // chunk "fairly across slots", SURVEY.md A4; results do not depend on the cut).  Many slots with one token each keep
+    // chunk "fairly across slots"; results do not depend on the cut).  Many slots with one token each keep
     // the WKV kernels wide (one CTA per head and slot) where a single slot with 64 tokens would run them 40 CTAs wide.
     std::vector<size_t> base(nslot + 1, 0), row_base(nslot + 1, 0);
     std::vector<int> pos(nslot, 0), rows_done(nslot, 0);
@@ -2210,7 +2210,7 @@ int32_t b200rwkv_tp_connect(b200rwkv_engine* e, const uint8_t* handles) {
 }
 
 // In-process variant (all ranks live in this process, e.g. tests with several ranks on one GPU, or a
-// host that owns every GPU of the box as in SURVEY.md §8b): exchange the comm-block pointers directly.
+// host that owns every GPU of the box): exchange the comm-block pointers directly.
 int32_t b200rwkv_tp_connect_local(b200rwkv_engine** engines, int32_t n) {
     API_BEGIN((b200rwkv_engine*)nullptr)
     REQUIRE(engines && n >= 1 && n <= 8, B200RWKV_ERR_INVALID, "bad argument");
@@ -2417,7 +2417,7 @@ static int32_t rank_state_free(b200rwkv_engine* e, uint64_t snapshot_id) {
     API_END
 }
 
-// ---- device-resident state cache (SURVEY.md §8f-4): snapshots <-> host tensors, without passing through a slot ----
+// ---- device-resident state cache: snapshots <-> host tensors, without passing through a slot ----
 static int32_t rank_snapshot_back(b200rwkv_engine* e, uint64_t snapshot_id, float* state_out, float* logits_out) {
     API_BEGIN(e)
     REQUIRE(e && (state_out || logits_out), B200RWKV_ERR_INVALID, "null argument");
@@ -3292,7 +3292,7 @@ int32_t b200rwkv_profile_insitu(b200rwkv_engine* e, int32_t nslot, const int32_t
 #undef RANKS
 
 // Replaces `ModelBuilder...build_vN()` + `Bundle::new` + `TokioRuntime::new` (lib.rs:484-497) with everything the reference's
-// ReloadRequest carries for this path: devices (one engine object owning all tensor-parallel ranks, SURVEY.md §8b), LoRA files
+// ReloadRequest carries for this path: devices (one engine object owning all tensor-parallel ranks), LoRA files
 // (lib.rs:466-485), precision (lib.rs:493).
 int32_t b200rwkv_create_ex(const uint8_t* st, size_t len, const b200rwkv_options* opt, b200rwkv_engine** out) {
     if (!out || !opt) { g_err = "null argument"; return B200RWKV_ERR_INVALID; }

@@ -2,13 +2,13 @@
 //
 // Replaces web-rwkv's WGSL `matmul_vec_fp16` / `matmul_mat_fp16` dispatches that the reference
 // reaches through `Runtime::infer` (reference crates/ai00-core/src/run.rs:1143): the R/K/V/G/O,
-// channel-mix, LoRA and head projections (SURVEY.md §2.2 K3-K5, K8-K10).
+// channel-mix, LoRA and head projections.
 //
 // HBM-bound by construction (T <= 64 rows per pass, each weight byte is used once per step), so
 // the design is about keeping ~200 KB of weight bytes in flight per SM and never stalling the
 // stream.  At batch 16 the math is 16 FLOP per weight byte = ~100 TFLOP/s at HBM rate: measured
 // on B200 the legacy mma.sync path tops out near 140 TFLOP/s (HMMA.16816 issues once per 32
-// cycles per sub-partition; profiles/r01_gemm_mma_sync.md), so the tensor work is on tcgen05:
+// cycles per sub-partition), so the tensor work is on tcgen05:
 //   * swap-AB: the WEIGHT tile is the 128-row M operand, the token tile is the N=16 operand, the
 //     f32 accumulator (128 lanes x 16 columns) lives in TMEM; one elected thread issues
 //     tcgen05.mma.cta_group::1.kind::f16, eight k16 steps per 32 KB stage;
@@ -347,7 +347,7 @@ __device__ __forceinline__ void gemm_epilogue_role(const GemmParams& p, const in
                 // A16 outputs (operand of a following projection).  Thread t holds output row n = one k index of that operand
                 // for 16 tokens; the layout wants, per token, 8 consecutive k in one 16-byte chunk.  Written straight from the
                 // registers that is one 2-byte store per token and row, four 32-byte sectors per warp instruction -- measured
-                // 33 us per 128-token tile (r02_findings.md §8).  So the tile is transposed through 6 KB of shared memory:
+                // 33 us per 128-token tile.  So the tile is transposed through 6 KB of shared memory:
                 // every thread stages its 16 tokens, then writes two (token, chunk) pairs as 16-byte stores, 16 lanes = 256
                 // contiguous bytes.  All 128 epilogue threads take part (rows past the segment stage zeros).
                 const bool lerp = (out_mode == OUT_LERP_A16);

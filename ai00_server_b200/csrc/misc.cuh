@@ -75,8 +75,8 @@ __global__ void slot_pages_kernel(const __grid_constant__ SlotPages p) {
 
 // ---------------------------------------------------------------------------------------
 // State import / export between the API layout and the device layout.
-// API (web-rwkv shape [C, N+2, L, 1], x fastest; reference run.rs:987, lib.rs:267-272;
-// SURVEY.md App. C) per slot: api[l][row][c], row 0 = time-mix shift, rows 1..N = WKV with
+// API (web-rwkv shape [C, N+2, L, 1], x fastest; reference run.rs:987, lib.rs:267-272)
+// per slot: api[l][row][c], row 0 = time-mix shift, rows 1..N = WKV with
 // row 1+i, col h*N+j <-> S[l,h][i][j], row N+1 = channel-mix shift.
 // Device: att_shift[l][slot][c], ffn_shift[l][slot][c], wkv[l][slot][h][value][key].
 // v5/v6: S[i=key][j=value]  -> M[value=j][key=i]   (transpose)

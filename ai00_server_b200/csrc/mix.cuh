@@ -1,7 +1,7 @@
 // Residual update + LayerNorm + token shift + static lerps, one 256-thread group per token.
 //
 // Replaces web-rwkv's `layer_norm`, `token_shift` and `add` WGSL dispatches on the path
-// `Runtime::infer` (reference run.rs:1143; SURVEY.md §2.2 K1-K3, App. A/B).  Fused so the
+// `Runtime::infer` (reference run.rs:1143).  Fused so the
 // residual stream makes one HBM/L2 round trip per half-layer:
 //     x_out = x_in + gate (.) sum_p part[p]            (projection results of the previous
 //                                                       half-layer, one partial per TP rank)
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(LN_ROWS_THREADS) ln_mix_rows_kernel(const __gr
 
 // ---------------------------------------------------------------------------------------
 // Embedding gather + LN0 (reference: web-rwkv embeds on the CPU and runs ln0 on the device,
-// SURVEY.md §2.2 K1; here the f16 table lives in HBM and both are one kernel).
+// here the f16 table lives in HBM and both are one kernel).
 // ---------------------------------------------------------------------------------------
 struct EmbedParams {
     const __half* emb;     // [V, C]

@@ -1,9 +1,9 @@
 // Decode-shaped (<= 16 tokens) front half of a time-mix / channel-mix block as ONE launch of 16 clusters x 8 CTAs.
 //
-// Replaces, on the path `Runtime::infer` (reference run.rs:1143; SURVEY.md §2.2 K1-K3, App. A), web-rwkv's
+// Replaces, on the path `Runtime::infer` (reference run.rs:1143), web-rwkv's
 // `layer_norm` + `token_shift` (+ for RWKV-6 the two LoRA matmuls of the data-dependent token shift) dispatches.
 //
-// Why: measured on B200 (profiles/r01_findings.md §3) the per-op chain spends 10 us in the one-CTA-per-token LN launch and
+// Why: measured on B200, the per-op chain spends 10 us in the one-CTA-per-token LN launch and
 // 15.5 + 19 us in the two 2.6 MB LoRA GEMM launches of every RWKV-6 layer -- 45 us in which HBM idles, against 66 us of
 // weight streaming per layer.  Nothing here is bandwidth: it is a chain of L2 round trips, so the shape is chosen for
 // the shortest chain:

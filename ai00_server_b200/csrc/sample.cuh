@@ -2,7 +2,7 @@
 // head projection left in HBM.  Only <= 128 (token id, probability) pairs per slot cross PCIe.
 //
 // Replaces, for samplers that need only the head of the sorted distribution (Nucleus with top_k <= 128, greedy), what the
-// reference does per generated token per slot (SURVEY.md §8f-1):
+// reference does per generated token per slot:
 //   crates/ai00-core/src/run.rs:664-697   output.to_vec() (num_vocab f32 = 256 KiB D2H), Sampler::transform (penalties,
 //                                         sampler/nucleus.rs:61-67), Formatter::transform (BNF mask, sampler/bnf.rs:37-40),
 //                                         bias add (run.rs:679-681), softmax round trip (2 x 256 KiB, run.rs:1164-1190)

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128) prefetch_probe_kernel(const uint8_t* src,
 // lane issues `n` kind::f16 MMAs back to back (A from shared memory or from tensor memory, eight distinct k16 slices of a
 // zeroed operand tile in rotation, like the projection's main loop), commits, waits.  Answers what a [M x 16] x [16 x N]
 // instruction costs when nothing else is in the way -- the projection GEMMs are bound by this, not by HBM, once the weight
-// bytes per block shrink (r02_findings.md §11).
+// bytes per block shrink.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128, 1) mma_rate_kernel(int M, int N, int a_in_tmem, int n, long long* cycles_out) {
     extern __shared__ __align__(1024) uint8_t smem[];       // A tile: 128 rows x 128 k (32 KB) | B tile: 256 rows x 128 k (64 KB) | barrier

@@ -2,8 +2,7 @@
 // GroupNorm (eps 64e-5), the v7 bonus term and the output gate.
 //
 // Replaces web-rwkv's `time_mix_v5` / `time_mix_v6` / `time_mix_v7` + `group_norm` WGSL
-// dispatches under `Runtime::infer` (reference run.rs:1143; SURVEY.md §2.2 K6/K6'/K7, math in
-// App. A / App. B).
+// dispatches under `Runtime::infer` (reference run.rs:1143).
 //
 // One 256-thread group per (head, slot).  The 64x64 f32 head state (16 KB) lives in HBM as
 // M[value][key] for every version (v6's S[key][value] is stored transposed; the API layout is
@@ -359,7 +358,7 @@ __global__ void __launch_bounds__(WKV_SA_THREADS, 7) wkv_kernel(const __grid_con
             }
     }
 
-    // w[t][c] = exp(-exp(time_decay[c] + sum_k Wd2[c][k] * tanh(Wd1 xw)[t][k]))   (SURVEY.md App. A), for the token whose
+    // w[t][c] = exp(-exp(time_decay[c] + sum_k Wd2[c][k] * tanh(Wd1 xw)[t][k])), for the token whose
     // decay-LoRA input sits at `dt` (hi) / `dt + WKV_STAGE_TOK * Dd` (lo halves of split operands), into wl[slot_tok][64]
     auto fold_token = [&](const __half* dt, const int slot_tok) {
         const int c = tid & (WKV_N - 1), qk = tid >> 6;

@@ -1,8 +1,8 @@
 """Deterministic synthetic RWKV weights in the reference's on-disk `.st` layout.
 
-No RWKV checkpoints exist offline (SURVEY.md §0.4), so tests and bench.py use
+No RWKV checkpoints exist offline, so tests and bench.py use
 random-init weights of the named architectures.  The file image written here
-follows /root/reference/assets/scripts/convert_safetensors.py:22-101 exactly:
+follows assets/scripts/convert_safetensors.py:22-101 exactly:
 safetensors container, metadata {"format": "pt"}, every tensor float16, lower-case
 keys after the `time_maa->time_mix` / `time_faaaa->time_first` renames, LoRA
 matrices already transposed to [out, in].
@@ -54,7 +54,7 @@ PRESETS = {
     "small6": Shape(6, 4, 512, 1792, V=2048, Dm=32, Dd=64),
     "small5": Shape(5, 3, 512, 1792, V=2048),                                   # 8 heads: shards over 8 GPUs
     "small7": Shape(7, 3, 512, 2048, V=2048, Dd=32, Da=32, Dv=16, Dg=64),
-    # BASELINE.json shapes (last row)
+    # the benchmarked shapes
     "v6-1b6": Shape(6, 24, 2048, 7168, Dm=32, Dd=64),
     "v6-3b": Shape(6, 32, 2560, 8960, Dm=32, Dd=64),
     "v6-7b": Shape(6, 32, 4096, 14336, Dm=64, Dd=128),
@@ -115,7 +115,7 @@ def tensor_spec(s: Shape) -> list[tuple[str, tuple[int, ...], float, float]]:
             add(a + "g1", (s.Dg, C), -1.0 * _sq(C), 1.0 * _sq(C))
             # gate LoRA / output gains sized so that the synthetic model is as well conditioned as the RWKV-6 presets: with
             # gain 2 / 0.5 here the random RWKV-7 stack is chaotic (two f32 implementations that differ only in summation
-            # order are 3e-3 apart after one token at 32 layers, f16 vs f32 operands 0.3: profiles/r02_findings.md), which
+            # order are 3e-3 apart after one token at 32 layers, f16 vs f32 operands 0.3), which
             # says nothing about an engine; trained RWKV-7 checkpoints initialise both near zero.
             add(a + "g2", (C, s.Dg), -1.0 * _sq(s.Dg), 1.0 * _sq(s.Dg))
             add(a + "k_k", (1, 1, C), 0.5, 1.2)
@@ -259,7 +259,7 @@ def num_params(shape: Shape | str) -> int:
 
 
 def algorithmic_bytes_per_step(s: Shape | str, batch: int) -> int:
-    """SURVEY.md §8(d) / BASELINE.md §3 figure: f16 weights streamed once per decode step,
+    """f16 weights streamed once per decode step,
     f32 state read + written once, embedding rows in, f32 logits out."""
     if isinstance(s, str):
         s = PRESETS[s]

@@ -16,7 +16,7 @@ from . import capi
 
 
 def shard_plan(info: dict, world: int, rank: int) -> dict:
-    """Which slice of the model a rank owns (mirrors b200rwkv_engine::build; SURVEY.md §8e):
+    """Which slice of the model a rank owns (mirrors b200rwkv_engine::build):
     heads / R,K,V,G rows / ffn.key rows / head rows are column-parallel, att.output and ffn.value
     are row-parallel (partials summed by the next LN stage), everything small is replicated."""
     H, N, C, F, V = info["num_head"], info["head_size"], info["num_emb"], info["num_hidden"], info["num_vocab"]

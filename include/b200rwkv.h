@@ -77,7 +77,7 @@ int32_t b200rwkv_create(const uint8_t* st, size_t len, int32_t device, int32_t m
 
 /* Everything the reference's ReloadRequest carries for this path (crates/ai00-core/src/lib.rs:196-240, 484-497), one call:
  *   - devices: `num_devices` in {1, 2, 4, 8} CUDA ordinals of this box.  With more than one, the returned handle is ONE engine
- *     that owns every tensor-parallel rank (head / column parallel, SURVEY.md §8e) and one worker thread per rank: every call
+ *     that owns every tensor-parallel rank (head / column parallel) and one worker thread per rank: every call
  *     below is made once, by the same two tasks as before, and drives all GPUs -- the reference's single `Runtime` object
  *     (run.rs:1230-1234).  State tensors are merged / scattered by head inside state_back / state_load.
  *   - LoRA files blended into the projection matrices while they are uploaded (lib.rs:466-485, `LoraBlend::full(alpha)`):
@@ -130,7 +130,7 @@ typedef struct {
                                       /* Quant::SF4 is not implemented: create_ex answers B200RWKV_ERR_UNSUPPORTED */
 int32_t b200rwkv_create_ex(const uint8_t* st, size_t len, const b200rwkv_options* opt, b200rwkv_engine** out);
 
-/* Tensor-parallel construction, one process per GPU (head / column parallel, SURVEY.md §8e).
+/* Tensor-parallel construction, one process per GPU (head / column parallel).
  * (The in-process alternative -- one handle, all ranks inside -- is b200rwkv_create_ex above.)
  * Every rank calls create_tp with the same model, then exchanges the opaque handle blobs
  * (b200rwkv_tp_export on each rank, all-gathered by the host over any side channel) and
@@ -184,7 +184,7 @@ int32_t b200rwkv_state_free(b200rwkv_engine*, uint64_t snapshot_id);            
  * rows (min(pool, 8192) rows per caching layer, the first [0] of them valid); snapshots hold only the valid rows. */
 int32_t b200rwkv_state_reset(b200rwkv_engine*, int32_t slot);
 
-/* Device-resident state cache (SURVEY.md §8f-4).  The reference's cache holds `CachedItem { state: TensorCpu, output:
+/* Device-resident state cache.  The reference's cache holds `CachedItem { state: TensorCpu, output:
  * TensorCpu }` (crates/ai00-core/src/run.rs:199-205): every check-out / check-in is a State::load / State::back PCIe copy of
  * the whole state (34.6 MB per slot at 7B; run.rs:838, 996, 561).  Here a cached item is a snapshot id: state_read /
  * state_write are device-to-device copies, and the snapshot carries the slot's last logits row with it, so a cache hit can
@@ -205,7 +205,7 @@ int32_t b200rwkv_read_state(const b200rwkv_info* info, const uint8_t* st, size_t
  * crates/ai00-core/src/run.rs:1179.  in/out: [rows, num_vocab] f32. */
 int32_t b200rwkv_softmax(b200rwkv_engine*, int32_t rows, const float* in, float* out);
 
-/* GPU front half of token sampling (SURVEY.md §8f-1).  Replaces, for samplers that only need the head of the sorted
+/* GPU front half of token sampling.  Replaces, for samplers that only need the head of the sorted
  * distribution (Nucleus with top_k <= 128 -- the reference default, sampler/nucleus.rs:16-17 -- and greedy), the per-token
  * per-slot sequence of crates/ai00-core/src/run.rs:664-697: `output.to_vec()` (num_vocab f32 D2H), `Sampler::transform`
  * (penalties, sampler/nucleus.rs:61-67), `Formatter::transform` (BNF mask, sampler/bnf.rs:37-40), the bias add

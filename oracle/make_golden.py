@@ -16,7 +16,7 @@ Two kinds of fixture:
    checksum).  They pin the oracle against accidental edits and give the C restatement
    (oracle/rwkv_ref.c) and the CUDA engine a fixture that does not need the oracle at
    run time.  They are NOT an independent check of the math — the reference holds no
-   golden vectors for this path (SURVEY.md §8c: parity unpinned).
+   golden vectors for this path (parity unpinned).
 """
 from __future__ import annotations
 

@@ -14,7 +14,7 @@ runs unmodified on the CPU:
 The weight mapping is the one of fla's `utils/convert_from_rwkv6.py` applied to the `.st` names (reference
 assets/scripts/convert_safetensors.py:22-101): BlinkDL orders the five lerp branches (w, k, v, r, g), fla (r, w, k, v, g).
 `norm_eps = 64e-5` is passed explicitly to the RWKV-6 layer (fla's default 1e-5 is not the official head_size_divisor = 8 value), so
-that fixture does not pin the RWKV-6 GroupNorm epsilon (SURVEY.md §9 A1); everything else in the two sub-layers it does.
+that fixture does not pin the RWKV-6 GroupNorm epsilon; everything else in the two sub-layers it does.
 RWKV-7 (`fuse_norm=False`: torch GroupNorm and `F.normalize`, no Triton): `fused_addcmul_rwkv7`, `fused_k_rwkv7`,
 `gate_output_correction` -> fla's own `torch_addcmul_rwkv7`, `k_update_ref`, `gate_output_correction_ref`; the recurrence -> fla's
 pure-torch `dplr_recurrence` with a = -kk, b = kk * a exactly as the layer's chunk branch calls it (already pinned by

@@ -6,16 +6,16 @@ bench.py's cpu_baseline leg use it, and only as the checker.
 
 PARITY UNPINNED: the arithmetic of this path lives in the third-party crate
 `web-rwkv = 0.10.18` (reference Cargo.toml:34-38, Cargo.lock:5530-5533), whose
-source is not under /root/reference, and the reference ships no tests, golden
-vectors or fixtures for it (SURVEY.md §0.3, §8c).  This file restates the
+source is not in the reference tree, and the reference ships no tests, golden
+vectors or fixtures for it.  This file restates the
 published RWKV algorithm that crate implements and is anchored on the
 reference's own call sites and on-disk contract:
 
 * weights: the `.st` layout written by
-  /root/reference/assets/scripts/convert_safetensors.py:22-101 (lower-cased
+  assets/scripts/convert_safetensors.py:22-101 (lower-cased
   keys, f16, `time_maa->time_mix`, `time_faaaa->time_first`, last-two-dims
   transposes of the LoRA matrices so every matrix is [out, in]) and
-  /root/reference/crates/converter/src/main.rs:8-22;
+  crates/converter/src/main.rs:8-22;
 * forward contract: one f32 logits row of length `num_vocab` per requested token
   (reference crates/ai00-core/src/run.rs:675,694,730), `RnnOption::Last` vs
   `Full` (run.rs:812-822, 710-724);
@@ -32,7 +32,7 @@ reference's own call sites and on-disk contract:
 
 Math follows BlinkDL's published inference code (rwkv pip `model.py`
 att_one_v5_2/att_one_v6_0/ffn_one_v6 and RWKV-LM `rwkv_v7_demo_rnn.py`), as
-restated in SURVEY.md App. A / App. B.
+restated here.
 
 `act` selects the activation precision contract:
   "f32": every intermediate stays f32 (weights are f16 values up-converted).

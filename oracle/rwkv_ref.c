@@ -3,12 +3,12 @@
  * TEST INFRASTRUCTURE ONLY: used by tests/ (cross-checked against oracle/rwkv_numpy.py and the
  * committed goldens) and as bench.py's `cpu_baseline` / `--impl reference` arm, where it stands
  * in for the reference's own CPU path (web-rwkv on lavapipe), which cannot be built in this image
- * (no Rust toolchain, no Vulkan loader; SURVEY.md §0.4, §8c).  PARITY UNPINNED: the reference
+ * (no Rust toolchain, no Vulkan loader).  PARITY UNPINNED: the reference
  * holds no golden vectors for this path; see oracle/rwkv_numpy.py for what anchors the math.
  *
- * Math: SURVEY.md App. A (BlinkDL rwkv pip model.py att_one_v6_0 / ffn_one_v6, att_one_v5_2) and App. B (RWKV-LM
+ * Math: RWKV-5.2 / 6 (BlinkDL rwkv pip model.py att_one_v6_0 / ffn_one_v6, att_one_v5_2) and RWKV-7 (RWKV-LM
  * rwkv_v7_demo_rnn.py: delta-rule state update, kk normalisation, value residual, bonus term),
- * weights in the `.st` layout of /root/reference/assets/scripts/convert_safetensors.py:22-101
+ * weights in the `.st` layout of assets/scripts/convert_safetensors.py:22-101
  * (all f16, matrices [out, in]).  State per slot: (L, N+2, C) f32 == web-rwkv [C, N+2, L, 1]
  * (reference crates/ai00-core/src/run.rs:987).
  *
@@ -119,7 +119,7 @@ static void lora2(const h16* W1, const h16* W2, int D, int C, const float* x, in
     gemm(W2, C, D, mid, B, out);
 }
 
-/* RWKV-7 decode step (SURVEY.md App. B; oracle/rwkv_numpy.py::_att_v7 / _ffn_v7 is the NumPy twin).
+/* RWKV-7 decode step (oracle/rwkv_numpy.py::_att_v7 / _ffn_v7 is the NumPy twin).
  * State rows 1..N of a layer hold S[h][i (value)][j (key)] at row 1+i, column h*N+j. */
 static int ref_decode_step_v7(const RefModel* m, int B, const int32_t* tokens, float* state, float* logits) {
     const int C = m->C, F = m->F, V = m->V, H = m->H, N = m->N, L = m->L, q = m->act_f16;

@@ -13,7 +13,7 @@ Follows, line by line:
 All arithmetic in f32 like the Rust code.  Ties: the reference sorts with voracious_sort (unstable), so the order of equal
 probabilities is unspecified there; this restatement orders by (adjusted logit descending, token id ascending), which is one
 of the reference's possible outcomes (the probability is a non-decreasing function of the logit) and is what the GPU front
-half (csrc/sample.cuh) defines.  Pinning: the reference has no tests or vectors for this path (SURVEY.md §4), so this file is
+half (csrc/sample.cuh) defines.  Pinning: the reference has no tests or vectors for this path, so this file is
 pinned only by construction -- parity unpinned, like the model oracle.
 """
 from __future__ import annotations

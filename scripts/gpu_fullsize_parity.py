@@ -1,8 +1,8 @@
-"""Engine vs the C/OpenMP oracle at a BASELINE shape (default v6-3b, B=2; use v6-7b on a box with >= 64 host cores):
+"""Engine vs the C/OpenMP oracle at a full-size shape (default v6-3b, B=2; use v6-7b on a box with >= 64 host cores):
 relative logits error against BOTH oracle contracts, argmax agreement, and the oracle-vs-oracle noise floor beside it
-(profiles/r01_noise_floor.txt).  Not run in round 1 (GPU budget); first item of round 2.
+(the distance of the two operand contracts from each other).
 
-    gpurun -- 'python scripts/gpu_fullsize_parity.py v6-3b 2 4'
+    python scripts/gpu_fullsize_parity.py v6-3b 2 4
 """
 import os
 import sys

@@ -1,4 +1,4 @@
-"""`bench.py --impl reference` (the CPU arm the driver runs next to the B200 arm) prints one contract-shaped JSON line.
+"""`bench.py --impl reference` (the CPU arm beside the B200 arm) prints one contract-shaped JSON line.
 Runs the C/OpenMP oracle on a CI-sized preset; nothing here touches a GPU."""
 import json
 import os
@@ -9,7 +9,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_reference_arm_prints_the_contract_line():
-    # OMP_NUM_THREADS=1 is what torchrun exports to its workers: the arm must size its own team (VERDICT r1)
+    # OMP_NUM_THREADS=1 is what torchrun exports to its workers: the arm must size its own team
     env = dict(os.environ, OMP_NUM_THREADS="1", B200RWKV_CPU_THREADS="2")
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "2", "--warmup", "1",
                           "--preset", "small6", "--batch", "4"],

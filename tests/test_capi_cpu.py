@@ -96,7 +96,7 @@ def _edit_header(st: np.ndarray, fn) -> np.ndarray:
 
 def test_st_tensor_sizes_are_validated():
     """A tensor whose byte range does not equal dtype x shape, a wrong rank, or an absurd shape must be a clean
-    B200RWKV_ERR_INVALID from the host-only parser (the loader trusted shape-derived sizes)."""
+    B200RWKV_ERR_INVALID from the host-only parser (the loader once trusted shape-derived sizes)."""
     st = synth.make_st("tiny6", 0)
     assert capi.info_from_st(st)["version"] == 6
 

@@ -39,7 +39,7 @@ def test_wkv6_kernel_reproduces_the_fla_fixture(golden_dir, split):
 
 def test_wkv5_kernel_with_static_decay(golden_dir):
     """RWKV-5 is the same recurrence with a per-channel static decay: the fixture's first-token decay for all tokens, checked
-    against a float64 evaluation of the recurrence (SURVEY.md App. A)."""
+    against a float64 evaluation of the recurrence."""
     g = np.load(os.path.join(golden_dir, "wkv6_fla.npz"))
     w = np.exp(-np.exp(g["wraw"][0].astype(np.float64)))             # [H, N]
     r, k, v, u = (g[n].astype(np.float64) for n in ("r", "k", "v", "u"))

@@ -2,7 +2,7 @@
 ctypes mirror of the reference's Runtime/State interface), against the CPU oracle on the same
 seeded synthetic `.st` weights and against the committed golden fixtures.
 
-Tolerance (BASELINE.json north_star): logits within 1e-3 relative, argmax token ids exact.
+Tolerance: logits within 1e-3 relative, argmax token ids exact.
 "relative" is measured against the logits range: max|d| / max|logits|.  The engine and the
 oracle's "f16" contract round the same operands to f16, so the observed error is ~1e-5; the
 "f32" contract (no activation rounding at all) must also stay inside 1e-3.
@@ -120,7 +120,7 @@ def test_decode_matches_prefill_and_chunking(models, preset):
 
 
 def test_batching_invariance_and_ragged_batch(models):
-    """Logits of slot i are independent of what the other slots do (SURVEY.md §4 (4))."""
+    """Logits of slot i are independent of what the other slots do."""
     m, orc, _ = models("tiny6")
     rng = np.random.default_rng(11)
     runs = [rng.integers(1, 500, size=n).tolist() for n in (1, 6, 3, 9)]
@@ -286,7 +286,7 @@ def test_short_ragged_steps_use_the_cluster_kernels(models, preset):
 def test_f32_activation_mode_tracks_the_f32_oracle(models, preset):
     """precision 1 (web-rwkv `Bundle::<f32>`): every projection input travels as a hi + lo f16 pair, no activation is rounded
     to f16 any more, so decode must sit within f32 summation noise of the pure-f32 oracle -- an order of magnitude inside the
-    1e-3 budget and independent of depth (DESIGN.md §2)."""
+    1e-3 budget and independent of depth."""
     m, _, st = models(preset, exact=True)
     orc = O.Oracle(O.parse_st(st), "f32")
     rng = np.random.default_rng(8)
@@ -332,7 +332,7 @@ def test_v7_with_the_2b9_lora_ranks(models, exact, dims):
 
 
 def test_device_resident_state_cache(models):
-    """CachedItem {state, output} as device snapshots (SURVEY.md 8f-4): read / write are D2D and carry the slot's last logits
+    """CachedItem {state, output} as device snapshots: read / write are D2D and carry the slot's last logits
     row; snapshot_back / snapshot_load move a cached item to / from host tensors without occupying a slot."""
     m, orc, _ = models("tiny6")
     m.state.load(m.state.init(), 0)

@@ -143,7 +143,7 @@ def test_unsupported_quant_requests_fail_loudly():
 @pytest.mark.parametrize("qtype", [capi.QUANT_INT8, capi.QUANT_NF4])
 def test_quantised_projections_at_the_7b_layer_shape(qtype):
     """One layer with the 7B dimensions (C = 4096, F = 14336, LoRA ranks 64 / 128): the tile counts, stream-K cuts and split-K
-    slices of the BASELINE shape, batch 16, against the oracle on the dequantised weights."""
+    slices of the 7B shape, batch 16, against the oracle on the dequantised weights."""
     import dataclasses
     shp = dataclasses.replace(synth.PRESETS["v6-7b"], L=1, V=4096)
     st = synth.make_st(shp, 0)

@@ -1,14 +1,14 @@
-"""BASELINE.json's shapes on the GPU at the batch sizes the configs name: RWKV-6 7B / batch 16 (the bench workload),
+"""The benchmarked shapes on the GPU at the batch sizes they are quoted at: RWKV-6 7B / batch 16 (the bench workload),
 RWKV-6 3B / batch 1, RWKV-7 2.9B / batch 8.  Engine (through the C ABI) vs the C/OpenMP oracle on the same seeded
 synthetic `.st`, both activation contracts, with the oracle-vs-oracle distance of the same step beside it.
 
-What is asserted (north_star: logits within 1e-3 relative, argmax exact):
+What is asserted (logits within 1e-3 relative, argmax exact):
   * default engine path (projection inputs rounded to f16, the web-rwkv fp16 contract): two correct implementations of
-    that contract are 2e-3..5e-3 apart at 24-32 layers (profiles/r01_noise_floor.txt), so the bound is the measured
+    that contract are 2e-3..5e-3 apart at 24-32 layers, so the bound is the measured
     floor of the same step (C oracle f16-contract vs f32-contract), not a constant: engine-vs-oracle <= 2 x floor, and
     the argmax equals the oracle's unless the oracle's own top-2 gap is inside that noise;
   * exact path (split hi+lo f16 operands, no activation rounding): <= 1e-3 against the pure-f32 oracle and argmax exact.
-Measured distances are appended to gpurun_out/parity_fullsize.jsonl (copied to profiles/ by the builder).
+Measured distances are appended to parity_fullsize.jsonl in the output folder.
 Size-independent properties (determinism, batching invariance, state round trip) run at the 7B shape.
 """
 import dataclasses

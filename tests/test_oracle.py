@@ -96,7 +96,7 @@ def test_st_image_readable_by_safetensors():
 
 
 def test_info_and_algorithmic_bytes_match_baseline_table():
-    # BASELINE.md §3 / SURVEY.md §8(d)
+    # the published shapes
     assert abs(synth.num_params("v6-7b") / 1e9 - 7.636) < 1e-3
     assert abs(synth.algorithmic_bytes_per_step("v6-7b", 16) / 1e9 - 15.846) < 1e-3
     assert abs(synth.algorithmic_bytes_per_step("v6-1b6", 1) / 1e9 - 2.958) < 1e-3
