@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
                 bulk_g2s_hint(smem_base + i * Cfg::STAGE_BYTES, W + (size_t)i * Cfg::W_BYTES, Cfg::W_BYTES, full_bar + i * 8, pol_w);
             }
             pdl_wait();
-            trace_stamp(p.trace, 2);
+            if (p.trace && cta == 0 && blockIdx.y == 0) p.trace[2] = globaltimer_ns();      // (trace_stamp is thread 0's)
             int seg = gemm_find_seg(p, b0);
             int kb = (b0 - p.seg[seg].blk_begin) % p.seg[seg].KB, KB = p.seg[seg].KB;
             int left = p.seg[seg].blk_begin + p.seg[seg].tiles * KB - b0;

@@ -35,6 +35,20 @@ def test_rows_of_launches_with_many_ctas():
         m.close()
 
 
+@pytest.mark.parametrize("slots", [1, 16, 17, 40, 72, 130])
+def test_windows_of_every_projection(slots):
+    """The profiling replay answers a window for every projection launch, whatever kernel the step's size takes."""
+    m = runtime.Model(synth.make_st("tiny6", 1), max_batch=slots, token_chunk_size=128)
+    try:
+        win, step_us = m.profile_insitu(list(range(slots)), np.arange(1, slots + 1, dtype=np.uint32), reps=2)
+        proj = [w for w in win if w["type"] >= 1000000]
+        # per layer at least R/K/V/G, output and two channel-mix launches, and the head
+        assert len(proj) >= 2 * 4 + 1
+        assert all(0 <= w["start_us"] < w["end_us"] <= step_us + 1e-3 for w in proj) and sum(w["bytes"] for w in proj) > 0
+    finally:
+        m.close()
+
+
 def test_stamps_of_one_launch_class():
     """Every layer's launch has a whole row on the device, of which the first 16 words come back."""
     shape = dataclasses.replace(synth.PRESETS["tiny6"], L=5)
