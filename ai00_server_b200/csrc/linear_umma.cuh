@@ -14,7 +14,7 @@
 // What bounds it: 16 KB of weights and TN x 128 B of rows per 64 k against 4 MMAs of 64 cycles (TN = 128), i.e. the bytes an SM
 // pulls from L2; lin_tile_kernel (mma.sync on 64 x 64 tiles, f32 activations through shared memory) ran at 5-9 % of the tensor pipe.
 // Measured: the 17 projections of a 512-token step (four layers of width 2048, ncu) 2970 -> 549 us, packing 78 us beside them; 16 prompts of
-// 1024 tokens 151 -> 50 ms, eight documents through latent attention and routed experts 17.7 -> 7.7 ms.
+// 1024 tokens 124 -> 48 ms, eight documents through latent attention and routed experts 15.3 -> 7.7 ms.
 #pragma once
 #include <cuda.h>
 #include <cudaTypedefs.h>

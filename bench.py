@@ -912,7 +912,7 @@ def main():
         per = (lambda n, k: n * k + n * k // 128 * 4) if args.quant == "int8" else (lambda n, k: n * k // 2 + n * k // 64 * 2)
         alg_bytes += qlayers * sum(per(n, k) - 2 * n * k for n, k in mats)
     traffic = None       # DRAM bytes of the same launches from the committed ncu capture (N = 1 capture of this workload)
-    tpath = os.path.join(ROOT, "profiles", "r01_gemm_traffic.json")
+    tpath = os.path.join(ROOT, "profiles", "gemm_traffic.json")
     if world == 1 and PRESET == "v6-7b" and BATCH == 16 and args.quant == "none" and os.path.exists(tpath):
         tj = json.load(open(tpath))
         traffic = tj["layers"] * sum(x["dram_bytes"] for x in tj["per_layer_gemm_launches"]) + tj["head"]["algorithmic_weight_bytes"]
@@ -921,7 +921,7 @@ def main():
                 "achieved": gemm_gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gemm_gbs / peaks["hbm_gbs"],
                 "peak_source": f"MEASURED_PEAKS.json ({peak_src})", "traffic": traffic,
                 "traffic_note": "per step, summed over the same projection launches as `achieved`: ncu dram read+write bytes of one "
-                                "captured layer x 32 + the head's algorithmic bytes (profiles/r01_gemm_traffic.json)",
+                                "captured layer x 32 + the head's algorithmic bytes (profiles/gemm_traffic.json)",
                 "how": "in situ: algorithmic weight bytes of the step's projection launches / sum of their windows [griddepcontrol.wait "
                        "released, last CTA exit] inside a graph-replayed step (globaltimer stamps, mean of 5 replays)",
                 "algorithmic_bytes_per_step_gemm": int(gemm_bytes), "gemm_us_per_step": gemm_us, "gemm_launches_per_step": int(gemm_n),
@@ -950,7 +950,7 @@ def main():
         ms2, _ = m2.bench_decode(slots, dec, args.warmup, args.steps)
         exact_rec = {"ms_per_step": ms2 / args.steps, "value": BATCH * args.steps / (ms2 * 1e-3), "unit": "tokens/s",
                      "what": "b200rwkv_create(precision = 1): split f16 hi+lo operands, no activation rounded; logits within 1.6e-4 of the "
-                             "f32 oracle at the 7B shape (tests/test_gpu_zfullsize.py, profiles/r02_parity_fullsize.jsonl)"}
+                             "f32 oracle at the 7B shape (tests/test_gpu_zfullsize.py, profiles/parity_fullsize.jsonl)"}
         m2.close()
 
     # ---- cpu baseline (rank 0, N=1 only) ----
