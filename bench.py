@@ -1,9 +1,9 @@
 #!/usr/bin/env python
-"""bench.py — decode tokens/s of the RWKV hot path on B200 (BASELINE.json metric).
+"""bench.py — decode tokens/s of the RWKV hot path on B200.
 
 A "step" is one decode step of the whole model for every slot of the batch (one token per
 slot): the per-layer WKV recurrence + token shift + GroupNorm, all projections and the head.
-Workload at N=1: configs[2] of BASELINE.json, RWKV-6-World-7B shape, fp16 weights, batch 16,
+Workload at N=1: RWKV-6-World-7B shape, fp16 weights, batch 16,
 slots primed with a 128-token synthetic prompt (random-init weights of that architecture,
 there are no checkpoints offline).
 
@@ -32,7 +32,7 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# the headline metric is quoted on configs[2] (7B, batch 16); configs[1] and [3] are the secondary lines
+# the headline metric is quoted on 7B at batch 16; 3B at batch 1 and RWKV-7 2.9B at batch 8 are the secondary lines
 MODEL_NAMES = {"v6-7b": "RWKV-6-World-7B", "v6-3b": "RWKV-6-World-3B", "v6-1b6": "RWKV-6-World-1.6B", "v7-2b9": "RWKV-7-World-2.9B"}
 PRESET = os.environ.get("B200RWKV_BENCH_PRESET", "v6-7b")
 BATCH = int(os.environ.get("B200RWKV_BENCH_BATCH", "16"))
@@ -102,7 +102,7 @@ class ClockSampler:
 
 
 def make_tokens(n_steps: int, batch: int, vocab: int):
-    rng = np.random.default_rng(1234)                      # SURVEY.md §8(d)
+    rng = np.random.default_rng(1234)
     return rng.integers(1, min(vocab, 65530), size=(batch, n_steps), dtype=np.int64)
 
 
@@ -156,7 +156,7 @@ def cpu_arm(weights, batch: int, steps: int, warmup: int, toks_bt: np.ndarray, b
 
 
 def prefill_main(args):
-    """cfg 5: `seqs` prompts of `seq_len` tokens through the embeddings route's path -- prefill with
+    """`seqs` prompts of `seq_len` tokens through the embeddings route's path -- prefill with
     no logits, then State::back of every slot (run.rs:984-989 returns the backed state as the embedding).  A "step" is one
     pass over all seqs x seq_len tokens."""
     import torch
@@ -702,11 +702,11 @@ def main():
     ap.add_argument("--warmup", type=int, default=8)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--cpu-steps", type=int, default=int(os.environ.get("B200RWKV_BENCH_CPU_STEPS", "6")))
-    ap.add_argument("--preset", default=PRESET, help="model shape: v6-7b (headline), v6-3b, v7-2b9, v6-1b6 (BASELINE.json configs)")
+    ap.add_argument("--preset", default=PRESET, help="model shape: v6-7b (headline), v6-3b, v7-2b9, v6-1b6")
     ap.add_argument("--batch", type=int, default=BATCH, help="concurrent slots, one token per slot per step")
     ap.add_argument("--exact", action="store_true", help="precision 1: f32-exact activations (split hi+lo operands)")
     ap.add_argument("--mode", default="decode", choices=["decode", "prefill"],
-                    help="prefill = BASELINE.json configs[4]: the embeddings route's workload (prompts in, final states out)")
+                    help="prefill = the embeddings route's workload (prompts in, final states out)")
     ap.add_argument("--quant", default="none", choices=["none", "int8", "nf4"],
                     help="weight-only quantised projection matrices (the reference's quant_type); not the headline configuration")
     ap.add_argument("--quant-layers", type=int, default=-1, help="the reference's `quant`: first N layers (default: all)")

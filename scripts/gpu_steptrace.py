@@ -61,5 +61,5 @@ for layer in (8, 9, 10, 11):
         order = np.argsort(ex)
         slow = np.where(ok)[0][order[-6:]]
         print(f"  L{layer} {name(types[i]):10s} ctas {ok.sum():3d} lastMMA min/med/max {mma.min():6.2f} {np.median(mma):6.2f} {mma.max():6.2f} | exit min/med/max {ex.min():6.2f} {np.median(ex):6.2f} {ex.max():6.2f} | slowest ctas {slow.tolist()} on SMs {c[slow, 0].tolist()}")
-np.save(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out", "steptrace_full.npy"), full[:, :8 + 3 * G])
+np.save("steptrace_full.npy", full[:, :8 + 3 * G])
 m.close()
