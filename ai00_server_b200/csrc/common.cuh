@@ -42,16 +42,19 @@ __device__ __forceinline__ void rot_cos_sin(int pos, double freq, float& cs, flo
 // 128-wide k block of ALL tokens of the step -- is ONE contiguous run (one bulk TMA copy) and (b) that run IS the UMMA
 // canonical K-major / no-swizzle operand of `th` token rows, which ONE tcgen05.mma with N = th consumes:
 //   [k block (128 k)][k8 chunk 16][th token rows][8 halves]      (8 rows x 16 B = one 128-byte core matrix)
-// th = 16 x (token tiles of the step) = 16 / 32 / 64 / 128 / 256; a step's producers and consumers agree on it (the engine passes
+// th = 16 x (token tiles of the step) = 16 / 32 / 64 / 128; a step's producers and consumers agree on it (the engine passes
 // it to every launch).  One MMA of N = th takes the tensor core's time (16 tokens 39 cycles, 64 48, 128 64, 256 128, with compile-time
 // descriptors), eight of N = 16 five times that.
 // Split operands (precision 1): th = 32, rows 0-15 hold the hi halves of the 16 tokens, rows 16-31 the lo halves.
 // Every buffer reserves 256 token rows per k block and K padded to whole k blocks (padding k is multiplied by zero weights).
+// Steps of more than 128 tokens are cut into tiles of 128 (th = 128): two neighbouring tiles fill the 256 rows of a k block, pairs of tiles
+// follow one another at the buffer's own distance.  A launch is told both as th | (k blocks between pairs of tiles) << 16.
 // ---------------------------------------------------------------------------------------
-constexpr int A16_MAX_ROWS = 256;                      // token rows per k block: steps of up to 256 tokens
-constexpr int A16_KB_HALVES = A16_MAX_ROWS * 128;      // halves per k block of a buffer
+constexpr int A16_KB_ROWS = 256;                       // token rows reserved per k block
+constexpr int A16_KB_HALVES = A16_KB_ROWS * 128;       // halves per k block of a buffer
 __host__ __device__ inline size_t a16_index(int m, int k, int th) {
-    return (size_t)(k >> 7) * A16_KB_HALVES + ((size_t)((k >> 3) & 15) * th + m) * 8 + (k & 7);
+    return (size_t)((m >> 8) * (th >> 16) + (k >> 7)) * A16_KB_HALVES + (size_t)((m >> 7) & 1) * (A16_KB_HALVES / 2) +
+           (size_t)(((k >> 3) & 15) * (th & 0xFFFF) + (m & 127)) * 8 + (k & 7);
 }
 
 __device__ __forceinline__ __half f2h_sat(float v) {

@@ -22,6 +22,7 @@
 
 #include "gemm.cuh"
 #include "gemm_wide.cuh"
+#include "gemm_pair.cuh"
 #include "qgemm.cuh"
 #include "pre6.cuh"
 #include "sample.cuh"
@@ -394,6 +395,8 @@ enum KClass { KC_GEMM = 0, KC_WKV = 1, KC_LN = 2, KC_OTHER = 3 };
 
 struct GemmLaunch {
     GemmParams p;
+    CUtensorMap tw;            // the weight blocks as rows of 1 KB (steps of more than 128 tokens)
+    bool chain = false;        // the segments are slices of one k range: longer steps choose their own number of partial sums
     int grid = 0;
     int grid_wide = 0;         // grid of steps with more than 64 tokens (see make_launch)
     bool short_k = false;      // every tile is one block long: gemm_wide.cuh's SHORT form,
@@ -416,6 +419,7 @@ struct SegDesc {
 struct A16Buf {
     __half* p = nullptr;
     int kq = 0;                // k32 blocks per m-tile (padded K / 32)
+    int tile_kb = 0;           // k blocks between 256-token tiles: all matrices of the buffer
     size_t halves_per_matrix = 0;
 };
 
@@ -478,7 +482,7 @@ struct b200rwkv_engine {
     std::unique_ptr<Group> group;             // set on rank 0 of an in-process tensor-parallel engine
     b200rwkv_info info;
     int dev = 0, rank = 0, world = 1, num_sms = 148;
-    int S = 0, chunk = 0, maxT = A16_MAX_ROWS, precision = 0;      // token rows of a step
+    int S = 0, chunk = 0, maxT = 0, precision = 0;      // maxT: token rows of a step
     int L = 0, C = 0, F = 0, V = 0, H = 0, N = 64, Cl = 0, Hl = 0, Fl = 0, Vl = 0;
     bool use_graph = true, use_pdl = true;
     // config.json families: every kernel triggers its dependents and waits for the kernel in front of it at its start, so that a launch
@@ -518,6 +522,17 @@ struct b200rwkv_engine {
     float *f_r = nullptr, *f_k = nullptr, *f_v = nullptr, *f_g = nullptr, *f_w = nullptr, *f_a = nullptr, *f_nu = nullptr,
           *f_vfirst = nullptr, *f_rr = nullptr, *part_att = nullptr, *part_ffn = nullptr, *d_logits = nullptr, *d_hidden = nullptr;
     A16Buf a_x[6], a_lora[5], a_out, a_kk, a_head;
+    // steps of more than 128 tokens (gemm_pair.cuh): every A16 buffer lies in one arena that two tensor maps cover
+    __half* a16_arena = nullptr;
+    size_t a16_arena_halves = 0, a16_used = 0;
+    CUtensorMap ta256, ta128;
+    int step_tokens = 128;             // tokens of a full step
+    int maxR = 0;                      // logits rows of a step
+    int part_stride(bool tiled) const { return tiled ? maxT : std::min(maxT, 128); }      // token rows between partial sums
+    MetaView meta_view(int* base, int T) const { return MetaView{base, T > 128 || kx ? maxT : std::min(maxT, 128), S}; }
+    size_t step_meta_ints(int T) const { return kx ? meta_ints : MetaView::ints(T > 128 ? maxT : std::min(maxT, 128), S); }
+    double pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const;
+    void launch_pair(const GemmLaunch& g, const GemmParams& gp, int rows, int parts, cudaStream_t s, Profiler* prof);
     float* gemm_ws = nullptr;
     size_t gemm_ws_floats = 0;
 
@@ -550,7 +565,7 @@ struct b200rwkv_engine {
     uint8_t* tk_out = nullptr;         // pinned: [S][TOPK_MAX] ids, [S][TOPK_MAX] probabilities (null: vocabulary too large)
     uint8_t *tk_dev = nullptr, *tk_host = nullptr;
     size_t tk_cap = 0;
-    void enqueue_keep(cudaStream_t s, int MTR);
+    void enqueue_keep(cudaStream_t s, int MT, int MTR);
     void topk_setup();
     void sample_topk(int nrows, const int32_t* slots, const int32_t* pen_off, const uint32_t* pen_tok, const float* pen_val,
                      const uint32_t* allow_bits, const int32_t* bias_off, const uint32_t* bias_tok, const float* bias_val,
@@ -607,6 +622,7 @@ struct b200rwkv_engine {
     void build(const StFile& st);
     const __half* upload_tmp(const StTensor& t);
     float* vec_f32(const StFile& st, const std::string& name, size_t off, size_t count, float scale = 1.f, float bias = 0.f);
+    void a16_reserve(size_t kblocks);
     A16Buf a16_alloc(int K, int nmat = 1);
     GemmLaunch make_launch(std::vector<SegDesc>& segs, int force_grid = 0, int qtype = QT_NONE);
     int quant_layers = 0, quant_type = QT_NONE;     // the first `quant_layers` layers hold Int8 / NF4 projection matrices
@@ -767,9 +783,47 @@ A16Buf b200rwkv_engine::a16_alloc(int K, int nmat) {
     A16Buf b;
     const int Kp = rup(K, GEMM_BK);          // whole 128-wide k blocks, zero padded
     b.kq = Kp / 32;
+    b.tile_kb = Kp / GEMM_BK * nmat;
     b.halves_per_matrix = (size_t)(Kp / GEMM_BK) * A16_KB_HALVES;
-    b.p = (__half*)dalloc(b.halves_per_matrix * 2 * nmat, true);
+    const size_t want = b.halves_per_matrix * nmat * cdiv(maxT, A16_KB_ROWS);
+    REQUIRE(a16_used + want <= a16_arena_halves, B200RWKV_ERR_INVALID, "internal: token operand arena too small");
+    b.p = a16_arena + a16_used;
+    a16_used += want;
     return b;
+}
+
+// tiled tensor maps without swizzle: the operands already lie in the order the tensor core reads
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        CK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q));
+        REQUIRE(f && q == cudaDriverEntryPointSuccess, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+        return (PFN_cuTensorMapEncodeTiled_v12000)f;
+    }();
+    return enc;
+}
+static void pair_map_w(CUtensorMap* map, const void* base, size_t bytes) {
+    const cuuint64_t dim[2] = {256, bytes / 1024}, stride[1] = {1024};
+    const cuuint32_t box[2] = {256, 16}, es[2] = {1, 1};
+    const CUresult r = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dim, stride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    REQUIRE(r == CUDA_SUCCESS, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled failed (weights)");
+}
+static void pair_map_a(CUtensorMap* map, const void* base, size_t bytes, int halves) {
+    const cuuint64_t dim[3] = {256, 2, bytes / 2048}, stride[2] = {1024, 2048};
+    const cuuint32_t box[3] = {256, (cuuint32_t)halves, 8}, es[3] = {1, 1, 1};
+    const CUresult r = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dim, stride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    REQUIRE(r == CUDA_SUCCESS, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled failed (token operands)");
+}
+
+void b200rwkv_engine::a16_reserve(size_t kblocks) {
+    a16_arena_halves = kblocks * A16_KB_HALVES * cdiv(maxT, A16_KB_ROWS);
+    a16_arena = (__half*)dalloc(a16_arena_halves * 2, true);
+    if (maxT <= 128) return;
+    pair_map_a(&ta256, a16_arena, a16_arena_halves * 2, 2);
+    pair_map_a(&ta128, a16_arena, a16_arena_halves * 2, 1);
 }
 
 GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_grid, int qtype) {
@@ -808,6 +862,7 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
     g.total_tiles = tile;
     uint8_t* W = (uint8_t*)dalloc((size_t)blk * blk_bytes, false);
     g.p.W = W;
+    if (maxT > 128 && qtype == QT_NONE) pair_map_w(&g.tw, W, (size_t)blk * blk_bytes);
     for (size_t i = 0; i < segs.size(); ++i) {
         SegDesc& d = segs[i];
         const GemmSeg& sg = g.p.seg[i];
@@ -882,8 +937,9 @@ GemmLaunch b200rwkv_engine::make_launch(std::vector<SegDesc>& segs, int force_gr
     g.p.counters = (unsigned*)dalloc((size_t)tile * 4, true);
     g.p.nrows = d_meta;   // T by default
     const size_t part = (size_t)tile * GEMM_BN;
-    gemm_ws_floats = std::max({gemm_ws_floats, part * g.max_contrib * std::min(maxT, 64), g.by_tile ? 0 : part * g.max_contrib_wide * maxT});
-    if (qtype != QT_NONE) gemm_ws_floats = std::max(gemm_ws_floats, part * g.max_contrib * maxT);
+    const size_t most = std::min(maxT, 128);               // tokens of a launch that cuts tiles (longer steps give clusters whole ones)
+    gemm_ws_floats = std::max({gemm_ws_floats, part * g.max_contrib * std::min<size_t>(most, 64), g.by_tile ? 0 : part * g.max_contrib_wide * most});
+    if (qtype != QT_NONE) gemm_ws_floats = std::max(gemm_ws_floats, part * g.max_contrib * most);
     weight_bytes_total += g.weight_bytes;
     return g;
 }
@@ -956,15 +1012,59 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
             break;
         case 2: launch_wide(gemm_wide_kernel<2>, WideCfg<2>::SMEM_BYTES, false); break;
         case 4: launch_wide(gemm_wide_kernel<4>, WideCfg<4>::SMEM_BYTES, false); break;
-        case 8:
+        default:
             if (g.short_k) launch_wide(gemm_wide_kernel<8, true>, WideCfg<8, true>::SMEM_BYTES, true);
             else launch_wide(gemm_wide_kernel<8>, WideCfg<8>::SMEM_BYTES, true);
             break;
-        default:
-            if (g.short_k) launch_wide(gemm_wide_kernel<16, true>, WideCfg<16, true>::SMEM_BYTES, true);
-            else launch_wide(gemm_wide_kernel<16>, WideCfg<16>::SMEM_BYTES, true);
-            break;
     }
+}
+
+// A step of more than 128 tokens: time of a launch in us as the waves of its units take it (a stage of 64 k: 0.30 us of tensor core with 256
+// tokens, 0.21 us of L2 reads with 128), the narrower token tile or more partial sums where they fill the last wave better.  A partial sum costs
+// a write and a read of its rows.
+double b200rwkv_engine::pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const {
+    double best = 1e30;
+    const int clusters = num_sms / 2;
+    for (int P = 1; P <= (g.chain ? std::min(4, g.p.nseg) : 1); ++P)
+        for (int nt = 256; nt >= 128; nt -= 128) {
+            long long units = 0, stages = 0;
+            for (int i = 0; i < g.p.nseg; ++i) {
+                if (!g.chain || i == 0) units += (long long)cdiv(g.p.seg[i].tiles, 2) * (g.chain ? P : 1) * cdiv(rows, nt);
+                stages = g.chain ? stages + 2 * g.p.seg[i].KB : std::max<long long>(stages, 2 * g.p.seg[i].KB);
+            }
+            if (g.chain) stages = (long long)cdiv(g.p.nseg, P) * 2 * g.p.seg[0].KB;
+            const double t = (double)((units + clusters - 1) / clusters) * (stages * (nt == 256 ? 0.30 : 0.21) + 0.8) + (g.chain ? P * (double)rows * C * 8 / 4e6 : 0.0);
+            if (t < best) { best = t; *ntok = nt; *parts = P; }
+        }
+    return best;
+}
+
+void b200rwkv_engine::launch_pair(const GemmLaunch& g, const GemmParams& gp, int rows, int parts, cudaStream_t s, Profiler* prof) {
+    int ntok = 256, best_parts = 1;
+    pair_plan(g, rows, &ntok, &best_parts);
+    if (parts == 0) parts = best_parts;
+    PairParams p;
+    memset(&p, 0, sizeof(p));
+    p.tw = g.tw;
+    p.ta = ntok == 256 ? ta256 : ta128;
+    p.g = gp;
+    for (int i = 0; i < gp.nseg; ++i) {
+        p.a_row[i] = (int)((gp.seg[i].A - a16_arena) / 1024);
+        p.a_tile[i] = gp.seg[i].a_tile;
+    }
+    p.nchain = g.chain ? parts : gp.nseg;
+    for (int c = 0; c < p.nchain; ++c) {
+        p.first[c] = g.chain ? c * gp.nseg / parts : c;
+        p.pair_begin[c + 1] = p.pair_begin[c] + cdiv(gp.seg[p.first[c]].tiles, 2);
+        if (g.chain) p.g.seg[p.first[c]].out = (float*)gp.seg[0].out + (size_t)c * part_stride(true) * C;
+    }
+    p.first[p.nchain] = gp.nseg;
+    p.ttiles = cdiv(rows, ntok);
+    const int units = p.pair_begin[p.nchain] * p.ttiles;
+    launch_cluster = 2;
+    const dim3 grid(2 * std::min(units, num_sms / 2));
+    if (ntok == 256) launch_k(gemm_pair_kernel<256>, grid, dim3(PAIR_THREADS), PairCfg<256>::SMEM_BYTES, p, KC_GEMM, s, prof);
+    else launch_k(gemm_pair_kernel<128>, grid, dim3(PAIR_THREADS), PairCfg<128>::SMEM_BYTES, p, KC_GEMM, s, prof);
 }
 
 // static split-K factor of a row-parallel projection: the S <= 8 / world (partial buffers the LN stages sum) that cuts K
@@ -1004,8 +1104,8 @@ void b200rwkv_engine::build(const StFile& st) {
     CK(cudaFuncSetAttribute(gemm_wide_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<4>::SMEM_BYTES));
     CK(cudaFuncSetAttribute(gemm_wide_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<8>::SMEM_BYTES));
     CK(cudaFuncSetAttribute(gemm_wide_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<8, true>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(gemm_wide_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<16, true>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(gemm_wide_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<16>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_pair_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<256>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(gemm_pair_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<128>::SMEM_BYTES));
     if (quant_layers > 0 && quant_type != QT_NONE) {
         REQUIRE(quant_type == QT_INT8 || quant_type == QT_NF4, B200RWKV_ERR_UNSUPPORTED, "quant_type must be Int8 or NF4 (SF4 is not implemented)");
         REQUIRE(world == 1, B200RWKV_ERR_UNSUPPORTED, "quantised layers are single-GPU in this version");
@@ -1030,9 +1130,11 @@ void b200rwkv_engine::build(const StFile& st) {
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;
     if (const char* v = dbg_env("B200RWKV_LN_CLUSTER")) ln_cluster = atoi(v) != 0;
 
-    // 256-token steps: single-GPU f16 models (quantised launches stop at 128 token rows, split operands at 16 tokens, and a
-    // tensor-parallel rank would double the block it shares with its peers)
-    maxT = (world == 1 && precision == 0 && quant_layers == 0) ? A16_MAX_ROWS : 128;
+    // Steps of more than 128 tokens: single-GPU f16 models (quantised launches stop at 128 token rows, split operands at 16 tokens, and a
+    // tensor-parallel rank would multiply the block it shares with its peers).  Sixteen portions of the caller's chunk size, 2048 tokens at most: weights are
+    // then read once per 2048 tokens and the launches of a layer fill the SMs several times over
+    maxT = (world == 1 && precision == 0 && quant_layers == 0) ? std::max(256, rup((int)std::min<long long>(16ll * chunk, 2048), 256)) : 128;
+    maxR = std::min(maxT, 512);
 
     // ---- step metadata ----
     meta_ints = MetaView::ints(maxT, S);
@@ -1040,7 +1142,7 @@ void b200rwkv_engine::build(const StFile& st) {
     CK(cudaMallocHost(&h_meta, meta_ints * 4 * META_RING));
     memset(h_meta, 0, meta_ints * 4 * META_RING);
     for (auto& ev : meta_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, 1);
 
     // ---- temp upload buffer: largest tensor ----
     for (auto& kv : st.tensors) d_tmp_bytes = std::max(d_tmp_bytes, kv.second.nbytes);
@@ -1054,7 +1156,7 @@ void b200rwkv_engine::build(const StFile& st) {
     state_from_st(st, L, H, N, C, init_state);      // State::init() with a state-tuned model; empty otherwise
 
     // ---- activations ----
-    const size_t TC = (size_t)maxT * C, TCl = (size_t)maxT * Cl;
+    const size_t TC = (size_t)maxT * C, TCl = (size_t)maxT * Cl, PC = (size_t)part_stride(false) * C;
     x_a = (float*)dalloc(TC * 4); x_b = (float*)dalloc(TC * 4);
     xx1 = (float*)dalloc(TC * 4); sx1 = (float*)dalloc(TC * 4); xx2 = (float*)dalloc(TC * 4);
     f_r = (float*)dalloc(TCl * 4); f_k = (float*)dalloc(TCl * 4); f_v = (float*)dalloc(TCl * 4); f_g = (float*)dalloc(TCl * 4);
@@ -1062,10 +1164,11 @@ void b200rwkv_engine::build(const StFile& st) {
     {
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
         off_part_att = 0;
-        off_part_ffn = al(off_part_att + TC * 4 * 8);       // up to 8 split-K slices each
-        off_rr = al(off_part_ffn + TC * 4 * 8);
+        const size_t parts = std::max(PC * 8, maxT > 128 ? TC * 4 : 0) * 4;      // up to 8 split-K slices each, 4 in steps of more than 128 tokens
+        off_part_ffn = al(off_part_att + parts);
+        off_rr = al(off_part_ffn + parts);
         off_logits = al(off_rr + TCl * 4);
-        off_flags = al(off_logits + (size_t)maxT * Vl * 4);
+        off_flags = al(off_logits + (size_t)maxR * Vl * 4);
         comm_bytes = al(off_flags + 256);
         comm_base = (uint8_t*)dalloc(comm_bytes, true);
         part_att = (float*)(comm_base + off_part_att);
@@ -1090,6 +1193,17 @@ void b200rwkv_engine::build(const StFile& st) {
     if (rank == 0) {
         d_keep = (float*)dalloc((size_t)S * V * 4);
         topk_setup();
+    }
+    {
+        const auto kb = [](int K) { return (size_t)cdiv(K, GEMM_BK); };
+        size_t n = 7 * kb(C) + kb(Cl) + kb(Fl);
+        if (ver == 6) n += 5 * kb(info.time_mix_adapter) + kb(info.time_decay_adapter);
+        if (ver == 7)
+            for (const char* t : {"w1", "a1", "v1", "g1"}) {
+                const std::string b = "blocks.0.att.", b1 = "blocks.1.att.";
+                n += kb(std::max({32, st.find(b + t) ? (int)st.dim(b + t, 0, 2) : 0, st.find(b1 + t) ? (int)st.dim(b1 + t, 0, 2) : 0}));
+            }
+        a16_reserve(n);
     }
     for (int i = 0; i < 6; ++i) a_x[i] = a16_alloc(C);
     a_out = a16_alloc(Cl);
@@ -1116,7 +1230,7 @@ void b200rwkv_engine::build(const StFile& st) {
         SegDesc d;
         d.t = &t; d.n0 = n0; d.N = Nn; d.k0 = k0; d.K = K;
         REQUIRE(a_koff % GEMM_BK == 0, B200RWKV_ERR_INVALID, "internal: split-K slices start on k-block boundaries");
-        d.proto.A = ab.p + (size_t)a_mat * ab.halves_per_matrix + (size_t)(a_koff / GEMM_BK) * A16_KB_HALVES; d.proto.a_k8 = ab.kq * 4;
+        d.proto.A = ab.p + (size_t)a_mat * ab.halves_per_matrix + (size_t)(a_koff / GEMM_BK) * A16_KB_HALVES; d.proto.a_tile = ab.tile_kb;
         d.proto.out_mode = OUT_F32; d.proto.act = act; d.proto.bias = bias; d.proto.out = out; d.proto.ldo = ldo;
         return d;
     };
@@ -1124,8 +1238,8 @@ void b200rwkv_engine::build(const StFile& st) {
                        const float* bias) {
         SegDesc d;
         d.t = &t; d.n0 = n0; d.N = Nn; d.k0 = k0; d.K = K;
-        d.proto.A = ab.p; d.proto.a_k8 = ab.kq * 4;
-        d.proto.out_mode = OUT_A16; d.proto.act = act; d.proto.bias = bias; d.proto.out = dst.p; d.proto.ldo = dst.kq;
+        d.proto.A = ab.p; d.proto.a_tile = ab.tile_kb;
+        d.proto.out_mode = OUT_A16; d.proto.act = act; d.proto.bias = bias; d.proto.out = dst.p; d.proto.out_tile = dst.tile_kb;
         return d;
     };
 
@@ -1147,7 +1261,7 @@ void b200rwkv_engine::build(const StFile& st) {
         n1.x_out = x_a;
         if (l > 0) {
             n1.n_parts = S_ffn;
-            for (int sp = 0; sp < S_ffn; ++sp) n1.parts[sp] = part_ffn + (size_t)sp * TC;
+            for (int sp = 0; sp < S_ffn; ++sp) n1.parts[sp] = part_ffn + (size_t)sp * PC;
             if (ver != 7) { n1.n_gate = 1; n1.gate_cl = Cl; n1.gates[0] = f_rr; }
             n1.commit_dst = ffn_shift + (size_t)(l - 1) * S * C;
             n1.commit_src = xx2;
@@ -1198,9 +1312,9 @@ void b200rwkv_engine::build(const StFile& st) {
                     SegDesc d;
                     d.t = &st.get(a + "time_mix_w2"); d.slice = i; d.n0 = 0; d.N = C; d.k0 = 0; d.K = Dm;
                     d.proto.A = a_lora[0].p + (size_t)i * a_lora[0].halves_per_matrix;
-                    d.proto.a_k8 = a_lora[0].kq * 4;
+                    d.proto.a_tile = a_lora[0].tile_kb;
                     d.proto.out_mode = OUT_LERP_A16; d.proto.act = ACT_NONE;
-                    d.proto.out = a_x[i].p; d.proto.ldo = a_x[i].kq;
+                    d.proto.out = a_x[i].p; d.proto.out_tile = a_x[i].tile_kb;
                     d.proto.aux0 = xx1; d.proto.aux1 = sx1; d.proto.aux2 = vec_f32(st, a + names[i], 0, C); d.proto.ld_aux = C;
                     sv.push_back(d);
                 }
@@ -1347,9 +1461,10 @@ void b200rwkv_engine::build(const StFile& st) {
             // next LN stage in fixed order); with tiles * S CTAs every CTA owns whole tiles: no fix-up
             std::vector<SegDesc> sv;
             for (int sp = 0; sp < S_att; ++sp)
-                sv.push_back(f32_seg(Wo, 0, C, c0 + sp * (Cl / S_att), Cl / S_att, a_out, part_att + (size_t)sp * TC, C, ACT_NONE,
+                sv.push_back(f32_seg(Wo, 0, C, c0 + sp * (Cl / S_att), Cl / S_att, a_out, part_att + (size_t)sp * PC, C, ACT_NONE,
                                      nullptr, sp * (Cl / S_att)));
             ly.o = make_launch(sv, S_att > 1 ? cdiv(C, GEMM_BN) * S_att : 0, lq);
+            ly.o.chain = true;
         }
 
         // ---------------- LN2 ----------------
@@ -1357,7 +1472,7 @@ void b200rwkv_engine::build(const StFile& st) {
         base_ln(n2);
         n2.x_in = x_a; n2.x_out = x_b;
         n2.n_parts = S_att;
-        for (int sp = 0; sp < S_att; ++sp) n2.parts[sp] = part_att + (size_t)sp * TC;
+        for (int sp = 0; sp < S_att; ++sp) n2.parts[sp] = part_att + (size_t)sp * PC;
         n2.ln_w = vec_f32(st, b + "ln2.weight", 0, C);
         n2.ln_b = vec_f32(st, b + "ln2.bias", 0, C);
         n2.shift_state = ffn_sh;
@@ -1391,9 +1506,10 @@ void b200rwkv_engine::build(const StFile& st) {
         {
             std::vector<SegDesc> sv;
             for (int sp = 0; sp < S_ffn; ++sp)
-                sv.push_back(f32_seg(Fv, 0, C, f0 + sp * (Fl / S_ffn), Fl / S_ffn, a_kk, part_ffn + (size_t)sp * TC, C, ACT_NONE,
+                sv.push_back(f32_seg(Fv, 0, C, f0 + sp * (Fl / S_ffn), Fl / S_ffn, a_kk, part_ffn + (size_t)sp * PC, C, ACT_NONE,
                                      nullptr, sp * (Fl / S_ffn)));
             ly.ffn.push_back(make_launch(sv, S_ffn > 1 ? cdiv(C, GEMM_BN) * S_ffn : 0, lq));
+            ly.ffn.back().chain = true;
         }
     }
 
@@ -1401,7 +1517,7 @@ void b200rwkv_engine::build(const StFile& st) {
     memset(&lnout, 0, sizeof(lnout));
     lnout.x_in = x_b; lnout.C = C; lnout.meta = mv;
     lnout.n_parts = S_ffn;
-    for (int sp = 0; sp < S_ffn; ++sp) lnout.parts[sp] = part_ffn + (size_t)sp * TC;
+    for (int sp = 0; sp < S_ffn; ++sp) lnout.parts[sp] = part_ffn + (size_t)sp * PC;
     if (ver != 7) { lnout.n_gate = 1; lnout.gate_cl = Cl; lnout.gates[0] = f_rr; }
     lnout.ln_w = vec_f32(st, "ln_out.weight", 0, C);
     lnout.ln_b = vec_f32(st, "ln_out.bias", 0, C);
@@ -1416,6 +1532,18 @@ void b200rwkv_engine::build(const StFile& st) {
         head.p.nrows = d_meta + 2;    // R
     }
 
+    if (maxT > 128) {
+        // tokens of a full step: the count of 256-token tiles whose waves cost least per token over a layer's projections
+        double best = 1e30;
+        for (int t = cdiv(maxT, 512); t <= maxT / 256; ++t) {
+            const Layer& ly = layers.back();
+            int nt, P;
+            double us = pair_plan(ly.o, t * 256, &nt, &P);
+            for (auto& g : ly.pre) if (!g.short_k) us += pair_plan(g, t * 256, &nt, &P);
+            for (auto& g : ly.ffn) us += pair_plan(g, t * 256, &nt, &P);
+            if (us / t < best) { best = us / t; step_tokens = t * 256; }
+        }
+    }
     gemm_ws = (float*)dalloc(gemm_ws_floats * 4, false);
     for (auto& ly : layers) {
         for (auto& g : ly.pre) g.p.ws = gemm_ws;
@@ -1440,7 +1568,7 @@ void b200rwkv_engine::build(const StFile& st) {
 // gate block-wise from the rank that owns those columns.
 // -----------------------------------------------------------------------------------------
 void b200rwkv_engine::finalize_tp() {
-    const size_t TC = (size_t)maxT * C;
+    const size_t TC = (size_t)part_stride(false) * C;
     const int ver = info.version;
     auto parts_of = [&](size_t off, int S, const float** dst) {
         int n = 0;
@@ -1475,10 +1603,25 @@ void b200rwkv_engine::finalize_tp() {
 void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof, bool runs) {
     launches_last_step = 0;
     const int rows = MT * 16;
+    const bool tiled = MT > 8;                 // more than 128 tokens: operands in 128-token tiles, projections on pairs of SMs
+    const MetaView mv = meta_view(d_meta, rows);
     // token rows of this step's A16 operands (common.cuh): every producer and consumer of the step uses the same value
-    const int th = (split_on && MT == 1) ? 32 : 16 * MT;
-    const int th_rows = (split_on && MT == 1) ? 32 : 16 * MTR;        // the head's operand holds output rows
+    const int th = (split_on && MT == 1) ? 32 : (tiled ? 128 : 16 * MT);
+    const int th_rows = (split_on && MT == 1) ? 32 : std::min(128, 16 * MTR);        // the head's operand holds output rows
+    auto th_of = [&](int tile_kb) { return tiled ? th | tile_kb << 16 : th; };
     last_th = th;
+    // longer steps choose how many partial sums the row-parallel projections leave
+    int parts_o = 0, parts_v = 0;
+    if (tiled) {
+        int nt;
+        pair_plan(layers[0].o, rows, &nt, &parts_o);
+        pair_plan(layers[0].ffn.back(), rows, &nt, &parts_v);
+    }
+    auto take_parts = [&](auto& q, float* base, int n) {
+        if (!tiled || q.n_parts == 0) return;
+        q.n_parts = n;
+        for (int i = 0; i < n; ++i) q.parts[i] = base + (size_t)i * part_stride(true) * C;
+    };
     // sequences of more than WKV_STAGE_TOK tokens: the scan kernel, with the decays of its own launch (split operands stay with the
     // decode kernel, whose steps hold 16 tokens at most)
     const bool scan = runs && !split_on;
@@ -1517,15 +1660,28 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             g2.p.prefetch_blocks = prefetch_blocks;
         }
         for (int i = 0; i < g2.p.nseg; ++i)
-            if (g2.p.seg[i].out_mode != OUT_F32) g2.p.seg[i].ldo = th;      // A16 outputs feed a projection of this step
-        launch_gemm(g2, mt, s, prof, split_on && MT == 1);      // split operands only when the whole step is decode-shaped
+            if (g2.p.seg[i].out_mode != OUT_F32) g2.p.seg[i].ldo = th_of(g2.p.seg[i].out_tile);      // A16 outputs feed a projection of this step
+        if (mt > 8 && g.short_k && !g.chain) {
+            // one-block tiles, a CTA per weight tile and 128 tokens
+            launch_k(gemm_wide_kernel<8, true>, dim3(std::min(g.total_tiles, 2 * num_sms), 1, mt / 8), dim3(WIDE_THREADS), WideCfg<8, true>::SMEM_BYTES, g2.p, KC_GEMM, s,
+                     prof, 1, g.total_tiles);
+        } else if (mt > 8) {
+            launch_pair(g, g2.p, mt * 16, g.chain ? (g.p.seg[0].out == (void*)part_att ? parts_o : parts_v) : 0, s, prof);
+        } else {
+            launch_gemm(g2, mt, s, prof, split_on && MT == 1);      // split operands only when the whole step is decode-shaped
+        }
     };
     auto gemm = [&](const GemmLaunch& g) { launch_gemm_chained(g, MT); };
-    launch_k(embed_ln0_kernel, dim3(rows), dim3(LN_THREADS), 0, embed, KC_LN, s, prof);
+    {
+        EmbedParams ep = embed;
+        ep.meta = mv;
+        launch_k(embed_ln0_kernel, dim3(rows), dim3(LN_THREADS), 0, ep, KC_LN, s, prof);
+    }
     auto launch_ln = [&](const LnMixParams& lp0) {
         LnMixParams lp = lp0;
         lp.trace = tr_next(0);
-        lp.kq_tile = th;
+        lp.kq_tile = th_of(a_x[0].tile_kb);
+        lp.meta = mv;
         if (ln_cluster_ok && MT == 1) {
             launch_cluster = PRE_CLUSTER;
             if (split_on) launch_k(ln_mix_cluster_kernel<true>, dim3(PRE_GRID), dim3(PRE_THREADS), 0, lp, KC_LN, s, prof);
@@ -1561,7 +1717,9 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
                 else launch_k(pre6_kernel<4, false>, dim3(PRE_GRID), dim3(PRE_THREADS), 0, q, KC_LN, s, prof);
             }
         } else {
-            launch_ln(ly.ln1);
+            LnMixParams n1 = ly.ln1;
+            take_parts(n1, part_ffn, parts_v);
+            launch_ln(n1);
         }
         for (int gi = 0; gi < (int)ly.pre.size(); ++gi)
             if (!pre_skipped(ly, gi)) gemm(ly.pre[gi]);
@@ -1569,7 +1727,8 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             // decays / staged rows are sized by the step shape: a slot cannot hold more tokens than the step
             WkvParams wp = ly.wkv;
             wp.trace = tr_next(2);
-            wp.kq_tile = th; wp.d1_kq = th;
+            wp.kq_tile = th_of(a_out.tile_kb); wp.d1_kq = th_of(a_lora[1].tile_kb);
+            wp.meta = mv;
             const bool sp = split_on && MT == 1;
             if (scan) {
                 const dim3 grid(Hl, wkv_slots), block(WKS_THREADS);
@@ -1590,13 +1749,19 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
         }
         gemm(ly.o);
         if (world > 1) launch_k(tp_barrier_kernel, dim3(1), dim3(32), 0, tpbar, KC_OTHER, s, prof);
-        launch_ln(ly.ln2);
+        {
+            LnMixParams n2 = ly.ln2;
+            take_parts(n2, part_att, parts_o);
+            launch_ln(n2);
+        }
         for (auto& g : ly.ffn) gemm(g);
         if (world > 1) launch_k(tp_barrier_kernel, dim3(1), dim3(32), 0, tpbar, KC_OTHER, s, prof);
     }
     {
         LnOutParams lo = lnout;
-        lo.kq_tile = th_rows;
+        lo.kq_tile = MTR > 8 ? th_rows | a_head.tile_kb << 16 : th_rows;
+        lo.meta = mv;
+        take_parts(lo, part_ffn, parts_v);
         if (split_on && MT == 1) launch_k(ln_out_kernel<true>, dim3(rows), dim3(LN_THREADS), 0, lo, KC_LN, s, prof);
         else launch_k(ln_out_kernel<false>, dim3(rows), dim3(LN_THREADS), 0, lo, KC_LN, s, prof);
     }
@@ -1604,35 +1769,37 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
     if (world > 1) launch_k(tp_barrier_kernel, dim3(1), dim3(32), 0, tpbar, KC_OTHER, s, prof);
 }
 
-static inline int mt_bucket(int rows) { return rows <= 16 ? 1 : (rows <= 32 ? 2 : (rows <= 64 ? 4 : (rows <= 128 ? 8 : 16))); }
+// 16-token tiles of a step's launches: powers of two up to 128 tokens, whole tiles of 128 beyond
+static inline int mt_bucket(int rows) { return rows <= 16 ? 1 : (rows <= 32 ? 2 : (rows <= 64 ? 4 : cdiv(rows, 128) * 8)); }
 
 // last logits row of every slot of this step -> keep[slot] (rank 0 gathers the vocabulary shards); see sample.cuh
-void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MTR) {
+void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MT, int MTR) {
     if (MTR <= 0 || rank != 0 || !d_keep) return;
     KeepParams kp;
     memset(&kp, 0, sizeof(kp));
     for (int q = 0; q < world; ++q) kp.shard[q] = (const float*)(peer_base[q] + off_logits);
     kp.world = world; kp.Vl = Vl; kp.V = V;
-    kp.meta = MetaView{d_meta, maxT, S};
+    kp.meta = meta_view(d_meta, MT * 16);
     kp.keep = d_keep;
     launch_k(keep_rows_kernel, dim3(MTR * 16, KEEP_CHUNKS), dim3(KEEP_THREADS), 0, kp, KC_OTHER, s, nullptr);
 }
 
 void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
-    if (!use_graph) {
+    // steps of more than 128 tokens go out launch by launch: their kernels outlast their launches, and a graph per length would be built for each
+    if (!use_graph || MT > 8) {
         enqueue_step(stream, MT, MTR, nullptr, runs);
-        enqueue_keep(stream, MTR);
+        enqueue_keep(stream, MT, MTR);
         launch_total += launches_last_step;
         return;
     }
-    const int key = (MT * 32 + MTR) * 2 + (runs ? 1 : 0);
+    const int key = (MT * 256 + MTR) * 2 + (runs ? 1 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
             enqueue_step(stream, MT, MTR, nullptr, runs);
-            enqueue_keep(stream, MTR);
+            enqueue_keep(stream, MT, MTR);
         } catch (...) {
             cudaStreamEndCapture(stream, &g);
             if (g) cudaGraphDestroy(g);
@@ -1652,7 +1819,9 @@ void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
 // fills one step's metadata; returns T
 int b200rwkv_engine::fill_meta(int* m, const std::vector<int>& slots, const std::vector<int>& counts,
                                const std::vector<const uint32_t*>& toks, const std::vector<int>& outmode, int* R_out) {
-    MetaView mv{m, maxT, S};
+    int total = 0;
+    for (int c : counts) total += c;
+    const MetaView mv = meta_view(m, total);
     int* tok = const_cast<int*>(mv.tok());
     int* tslot = const_cast<int*>(mv.tok_slot());
     int* tprev = const_cast<int*>(mv.tok_prev());
@@ -1709,9 +1878,9 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
     const bool copy_logits = want_logits && logits_out != nullptr;
     // f32-activation mode runs every step decode-shaped (<= 16 tokens): the split-operand kernels are the 16-token ones
     const int step_cap = std::min(chunk, split_on ? 16 : (kx ? maxT : std::min(maxT, 128)));
-    // RWKV steps of full portions hold two of them (gemm_wide.cuh: one pass over the weights for 256 tokens; 128-token steps are bound by
-    // the weight stream): the portions, and with them the rows b200rwkv_last_hidden answers, are those of 128-token steps
-    const int substeps = !kx && step_cap == 128 && maxT >= 256 ? 2 : 1;
+    // RWKV steps hold up to sixteen portions (gemm_pair.cuh: one pass over the weights for all their tokens): the portions, and with them the
+    // rows b200rwkv_last_hidden answers, are those of 128-token steps
+    const int substeps = !kx && maxT > 128 ? std::max(1, (int)std::min<long long>(step_tokens, 16ll * chunk) / step_cap) : 1;
     // Step packing: every step shares its token budget evenly over the entries that still have tokens (web-rwkv shares the
     // chunk "fairly across slots"; results do not depend on the cut).  Many slots with one token each keep
     // the WKV kernels wide (one CTA per head and slot) where a single slot with 64 tokens would run them 40 CTAs wide.
@@ -1738,6 +1907,11 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
         std::vector<const uint32_t*> s_toks;
         std::vector<int> step(nslot, 0), part(nslot, 0);
         for (int sub = 0; sub < substeps; ++sub) {
+            if (!kx && sub > 0) {          // room for the logits rows of another portion
+                int rows = 0;
+                for (int i = 0; i < nslot; ++i) rows += option[i] == B200RWKV_OPTION_FULL ? step[i] : (option[i] == B200RWKV_OPTION_LAST && step[i] > 0 ? 1 : 0);
+                if (rows + step_cap > maxR) break;
+            }
             // at least WKV_STAGE_TOK tokens per slot and portion while prompts are long: a WKV CTA then loads and stores its 16 KB
             // of state once per four tokens or more, and a portion touches a quarter of the slots' states
             n_active = 0;
@@ -1782,7 +1956,7 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
         bool kx_decode = false;
         int kx_split = 1;
         if (kx) kx_fill_step(hm, s_slots, s_counts, &kx_decode, &kx_split);
-        CK(cudaMemcpyAsync(d_meta, hm, meta_ints * 4, cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(d_meta, hm, step_meta_ints(T) * 4, cudaMemcpyHostToDevice, stream));
         CK(cudaEventRecord(meta_ev[mb], stream));
         if (kx) kx_run_step(T, R, kx_decode, kx_split);
         else run_step(mt_bucket(T), R > 0 ? mt_bucket(R) : 0, *std::max_element(s_counts.begin(), s_counts.end()) > WKV_STAGE_TOK);
@@ -2605,7 +2779,7 @@ static int32_t rank_bench_decode(b200rwkv_engine* e, int32_t nslot, const int32_
             launches_before = e->launch_total;
         }
         if (flush) CK(cudaMemsetAsync(flush, st & 0xff, flush_bytes, e->stream));
-        CK(cudaMemcpyAsync(e->d_meta, d_all + (size_t)st * e->meta_ints, e->meta_ints * 4, cudaMemcpyDeviceToDevice, e->stream));
+        CK(cudaMemcpyAsync(e->d_meta, d_all + (size_t)st * e->meta_ints, e->step_meta_ints(nslot) * 4, cudaMemcpyDeviceToDevice, e->stream));
         if (e->kx) e->kx_run_step(nslot, nslot, true, splits[st]);
         else e->run_step(MT, MT);
         if (step_ms_out && st >= warmup) CK(cudaEventRecord(marks[st - warmup], e->stream));
@@ -2950,7 +3124,7 @@ int32_t b200rwkv_debug_read(b200rwkv_engine* e, const char* name, float* out, si
                 const int nsum = (n == "part_att") ? e->split_att : (n == "part_ffn" ? e->split_ffn : 1);
                 std::vector<float> tmp((size_t)T * f.cols);
                 for (int sp = 1; sp < nsum; ++sp) {       // split-K partials: sum the slices
-                    CK(cudaMemcpy(tmp.data(), f.p + (size_t)sp * e->maxT * e->C, tmp.size() * 4, cudaMemcpyDeviceToHost));
+                    CK(cudaMemcpy(tmp.data(), f.p + (size_t)sp * e->part_stride(false) * e->C, tmp.size() * 4, cudaMemcpyDeviceToHost));
                     for (size_t i = 0; i < tmp.size(); ++i) out[i] += tmp[i];
                 }
                 return f.cols;
@@ -2966,10 +3140,12 @@ int32_t b200rwkv_debug_read(b200rwkv_engine* e, const char* name, float* out, si
         for (const A& a : as)
             if (n == a.n && a.b->p) {
                 REQUIRE((size_t)T * a.cols <= cap, B200RWKV_ERR_INVALID, "debug buffer too small");
-                std::vector<__half> h(a.b->halves_per_matrix);
-                CK(cudaMemcpy(h.data(), a.b->p + (size_t)a.mat * a.b->halves_per_matrix, h.size() * 2, cudaMemcpyDeviceToHost));
+                const size_t at0 = (size_t)a.mat * a.b->halves_per_matrix;
+                std::vector<__half> h((size_t)a.b->tile_kb * A16_KB_HALVES * cdiv(e->maxT, A16_KB_ROWS) - at0);
+                CK(cudaMemcpy(h.data(), a.b->p + at0, h.size() * 2, cudaMemcpyDeviceToHost));
+                const int th = T > 128 ? e->last_th | a.b->tile_kb << 16 : e->last_th;
                 for (int t = 0; t < T; ++t)
-                    for (int c = 0; c < a.cols; ++c) out[(size_t)t * a.cols + c] = __half2float(h[a16_index(t, c, e->last_th)]);
+                    for (int c = 0; c < a.cols; ++c) out[(size_t)t * a.cols + c] = __half2float(h[a16_index(t, c, th)]);
                 return a.cols;
             }
         throw Error(B200RWKV_ERR_INVALID, "unknown debug buffer: " + n);

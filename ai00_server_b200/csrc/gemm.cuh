@@ -60,7 +60,7 @@ enum OutMode : int {
 
 struct GemmSeg {
     const __half* A;      // A16 activations for this segment (already offset to the segment's first k block)
-    int a_k8;             // (unused)
+    int a_tile;           // k blocks between 256-token tiles of A (steps of more than 128 tokens)
     int KB;               // 128-wide k blocks (K padded up)
     int tiles;            // 128-row output tiles (N padded up)
     int N;                // valid output columns
@@ -70,7 +70,8 @@ struct GemmSeg {
     int act;
     const float* bias;    // optional [N], added before the activation
     void* out;
-    int ldo;              // OUT_F32: row stride (floats); A16 modes: k32 blocks per m-tile of the destination
+    int ldo;              // OUT_F32: row stride (floats); A16 modes: token rows and tile distance of the destination (common.cuh)
+    int out_tile;         // A16 modes: k blocks between 256-token tiles of the destination
     int grp;              // OUT_A16: columns per destination matrix (0 = single matrix)
     int grp_stride;       // OUT_A16: halves between destination matrices
     const float* aux0;    // OUT_LERP_A16: xx [T, ld_aux]

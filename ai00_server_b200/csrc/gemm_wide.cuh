@@ -1,13 +1,11 @@
-// Projection GEMM of prompt steps (17 .. 256 tokens):  Y[T, N] = X[T, K] (f16) * W[N, K]^T (f16), f32 accumulate.
+// Projection GEMM of prompt steps (17 .. 128 tokens; longer steps: gemm_pair.cuh, which leaves the one-block tiles to the SHORT form here):  Y[T, N] = X[T, K] (f16) * W[N, K]^T (f16), f32 accumulate.
 //
 // Same operands, segments, epilogues and stream-K fix-up as gemm.cuh (its decode kernel reads the same weight blocks); replaces
 // the projection dispatches of `Runtime::infer` (reference crates/ai00-core/src/run.rs:1143) in steps that hold a prompt.
 //
-// What bounds it: up to 128 tokens the weight stream (a 128 x 64 weight half block is 16 KB and meets 16 KB of tokens), at 256
-// tokens the bytes an SM can pull from L2 (16 KB + 32 KB per 4 MMAs of 128 cycles).  So a tile takes ALL tokens of the step: a
-// weight byte is read once per step.
-//   * stages hold 64 k (half a weight block, contiguous in both operands' layouts): at 256 tokens four 48 KB stages fit, where
-//     whole blocks would leave two;
+// What bounds it: the weight stream (a 128 x 64 weight half block is 16 KB and meets 16 KB of tokens).  So a tile takes ALL tokens of
+// the step: a weight byte is read once per step.
+//   * stages hold 64 k (half a weight block, contiguous in both operands' layouts);
 //   * one MMA of N = 16 MT per k16 step; all descriptor fields are compile-time constants.  An MMA of N = 128 takes 64 cycles
 //     then (8192 FMA per cycle, the tensor core's rate), N = 256 128;
 //   * EIGHT epilogue warps, two per TMEM lane quarter, each draining every second group of 16 tokens straight from TMEM: with
@@ -113,7 +111,12 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
             int seg = gemm_find_seg(p, b0);
             int kb = (b0 - p.seg[seg].blk_begin) % p.seg[seg].KB, KB = p.seg[seg].KB;
             int left = p.seg[seg].blk_begin + p.seg[seg].tiles * KB - b0;
-            const uint8_t* A0 = reinterpret_cast<const uint8_t*>(p.seg[seg].A);
+            // SHORT: blockIdx.z = 128-token tile of a longer step
+            auto operand = [&]() {
+                const uint8_t* a = reinterpret_cast<const uint8_t*>(p.seg[seg].A);
+                return SHORT ? a + ((size_t)(blockIdx.z >> 1) * p.seg[seg].a_tile * A16_KB_HALVES + (size_t)(blockIdx.z & 1) * (A16_KB_HALVES / 2)) * 2 : a;
+            };
+            const uint8_t* A0 = operand();
             int stage = 0;
             uint32_t ephase = 1;
             for (int i = 0; i < nst; ++i) {
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
                         kb = 0;
                         KB = p.seg[seg].KB;
                         left = p.seg[seg].tiles * KB;
-                        A0 = reinterpret_cast<const uint8_t*>(p.seg[seg].A);
+                        A0 = operand();
                     }
                 }
             }
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
         constexpr int P = Cfg::PAIR;                            // 16-token groups of this warp: mt = grp + 2 i, i in [i0, i1)
         // gridDim.y CTAs share a tile of a SHORT launch: each multiplies all tokens and finishes its share of them
         const int i0 = blockIdx.y * (MT / 2) / gridDim.y, i1 = (blockIdx.y + 1) * (MT / 2) / gridDim.y;
+        const int m0 = SHORT ? (int)blockIdx.z * (16 * MT) : 0;     // first token of this CTA's tile
         unsigned segcount = 0;
         SegWalk w;
         for (w.init(p, b0, b1); !w.done(); w.next(), ++segcount) {
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
             const bool row_ok = n < segN, lerp = (out_mode == OUT_LERP_A16);
             const float bias = (row_ok && sg.bias) ? sg.bias[n] : 0.f;
             const float mu = (lerp && row_ok) ? sg.aux2[n] : 0.f;
-            const int mmax = min(nrows, MT * 16);
+            const int mmax = min(nrows - m0, MT * 16);         // tokens of the tile
             // the 16-token groups i .. i + P - 1: accumulators (TMEM, or the parts in contributor order, all loads of two contributors in flight)
             auto load = [&](const int i, float (&v)[P][16]) {
                 if (SHORT || ncontrib == 1) {
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
                     if (ncontrib == 1 && i + P >= i1) drained();
                     if (out_mode == OUT_F32) {
                         if (row_ok) {
-                            float* o = reinterpret_cast<float*>(sg.out) + n;
+                            float* o = reinterpret_cast<float*>(sg.out) + (size_t)m0 * ldo + n;
 #pragma unroll
                             for (int q = 0; q < P; ++q)
 #pragma unroll
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
                             for (int j = 0; j < 16; ++j) {
                                 const int m = (grp + 2 * (i + q)) * 16 + j;
                                 const bool ok = row_ok && m < mmax;
-                                const size_t a_ = (size_t)m * sg.ld_aux + n;
+                                const size_t a_ = (size_t)(m0 + m) * sg.ld_aux + n;
                                 x0[q][j] = ok ? sg.aux0[a_] : 0.f;
                                 x1[q][j] = ok ? sg.aux1[a_] : 0.f;
                             }
@@ -341,7 +345,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, SHORT ? 2 : 1) gemm_wide_kernel(
                                 base += (size_t)gi * sg.grp_stride;
                                 nn = nc - gi * sg.grp;
                             }
-                            *reinterpret_cast<uint4*>(base + a16_index(mt * 16 + m, nn, ldo)) = make_uint4(r[0], r[1], r[2], r[3]);
+                            *reinterpret_cast<uint4*>(base + a16_index(m0 + mt * 16 + m, nn, ldo)) = make_uint4(r[0], r[1], r[2], r[3]);
                         }
                     }
                     named_bar_sync(2 + grp, GEMM_BN);

@@ -297,16 +297,9 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
 }
 
 static void lu_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K, uint32_t box_rows) {
-    static PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        CK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q));
-        REQUIRE(f && q == cudaDriverEntryPointSuccess, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-        return (PFN_cuTensorMapEncodeTiled_v12000)f;
-    }();
     const cuuint64_t dim[2] = {K, rows}, stride[1] = {K * 2};
     const cuuint32_t box[2] = {LU_KS, box_rows}, es[2] = {1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dim, stride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dim, stride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     REQUIRE(r == CUDA_SUCCESS, B200RWKV_ERR_CUDA, "cuTensorMapEncodeTiled failed");
 }
@@ -626,7 +619,7 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     const int rows = kx_bucket(T), rrows = R > 0 ? kx_bucket(R) : 0;
     if (!use_graph) {
         kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
-        enqueue_keep(stream, rrows / 16 + (rrows % 16 ? 1 : 0));
+        enqueue_keep(stream, 1, rrows / 16 + (rrows % 16 ? 1 : 0));
         launch_total += launches_last_step;
         return;
     }
@@ -639,7 +632,7 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
             kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
-            enqueue_keep(stream, rrows / 16 + (rrows % 16 ? 1 : 0));
+            enqueue_keep(stream, 1, rrows / 16 + (rrows % 16 ? 1 : 0));
         } catch (...) {
             cudaStreamEndCapture(stream, &g);
             if (g) cudaGraphDestroy(g);

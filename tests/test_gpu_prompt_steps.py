@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-3
 
 
-def _check(preset, lens, full, chunk=512):
+def _check(preset, lens, full, chunk=512, state_norm=np.inf):
     st = synth.make_st(preset, 3)
     orc = O.Oracle(O.parse_st(st), "f16")
     V = orc.info.num_vocab
@@ -33,7 +33,7 @@ def _check(preset, lens, full, chunk=512):
             err = np.abs(rows[s] - want).max() / np.abs(want).max()
             assert err <= TOL, (preset, lens, s, err)
             got = m.state.back(s)
-            assert np.abs(got - state).max() <= TOL * np.abs(state).max()
+            assert np.linalg.norm((got - state).ravel(), state_norm) <= TOL * np.linalg.norm(state.ravel(), state_norm)
     finally:
         m.close()
 
@@ -48,6 +48,38 @@ def test_step_sizes(preset, n):
 @pytest.mark.parametrize("preset", ["tiny5", "tiny6", "tiny7"])
 def test_full_rows_of_ragged_batches(preset, lens):
     _check(preset, lens, full=True)
+
+
+# steps of more than 128 tokens: 128- and 256-token tiles of the two-SM projections and their remainders, more tokens than a step holds (2048),
+# a model whose row-parallel projections keep one part (384 / 3 k blocks) and one with odd numbers of 128-row weight tiles
+@pytest.mark.parametrize("n", [383, 385, 513, 1100, 2300])
+@pytest.mark.parametrize("shape", ["tiny6", "tiny7", "odd6"])
+def test_steps_of_many_tiles(shape, n):
+    st = synth.Shape(6, 2, 320, 1160, V=512, Dm=32, Dd=64) if shape == "odd6" else shape
+    _check(st, [n], full=False)
+
+
+@pytest.mark.parametrize("lens", [[300, 250, 1, 700], [90] * 9])
+@pytest.mark.parametrize("preset", ["tiny5", "tiny6", "tiny7"])
+def test_rows_of_long_steps(preset, lens):
+    """More logits rows than a step keeps (512), more than the bucketed head holds (128), sequences of unequal length."""
+    _check(preset, lens, full=True)
+
+
+@pytest.mark.parametrize("preset", ["tiny5", "tiny6", "tiny7"])
+@pytest.mark.parametrize("each", [1, 3])
+def test_many_sequences_of_few_tokens(preset, each):
+    """Long steps whose sequences hold a few tokens each: the decode recurrence reads and writes tiled operands.
+
+    States by their 2-norm: among 150 x 50 000 entries the largest single one is an entry whose key and value both moved to the neighbouring
+    f16 operand, 2 x 2^-11 of it; all entries of a state at once do not, and a wrong row is off by its own size."""
+    _check(preset, [each] * 150, full=False, state_norm=2)
+
+
+@pytest.mark.parametrize("chunk", [1, 9, 33, 100])
+def test_long_steps_of_small_chunks(chunk):
+    """A step holds sixteen portions of the caller's chunk size, whatever they divide."""
+    _check("tiny6", [700, 31], full=False, chunk=chunk)
 
 
 @pytest.mark.parametrize("lens, rows", [([200], [(0, 128, 200)]), ([130, 140, 5], [(1, 121, 140)])])
