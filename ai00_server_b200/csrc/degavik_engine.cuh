@@ -207,7 +207,7 @@ void b200rwkv_engine::dg_load(const StFile& st, KxSizes& z) {
 void b200rwkv_engine::dg_enqueue_layer(cudaStream_t s, KxLayer& l, int rows, int nslot_grid, bool decode, int nsplit, Profiler* prof) {
     SeqModel& m = *kx;
     const int W = m.W;
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, step_rows);
     const int* cntT = d_meta;
     const KxLayerCfg& c = l.c;
     const int H_ = c.heads, G_ = c.kv_heads, dk = c.dim, dv = c.vdim;
@@ -269,7 +269,7 @@ void b200rwkv_engine::dg_enqueue_layer(cudaStream_t s, KxLayer& l, int rows, int
     MoeRouteParams rp{m.x, W, l.router, W, l.corr, E, c.top, m.sel, m.wgt, mv, MOE_TOP_LOGITS};
     launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, E), rp, KC_OTHER, s, prof);
     MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
-    launch_k(moe_group_kernel, dim3(1), dim3(256), ((size_t)E * 2 + (size_t)maxT * c.top) * 4, gp, KC_OTHER, s, prof);
+    launch_k(moe_group_kernel, dim3(1), dim3(rows > 128 ? MOE_GROUP_THREADS : 256), ((size_t)E * 2 + (size_t)rows * c.top) * 4, gp, KC_OTHER, s, prof);
     LinParams p1 = lin(m.x, W, l.gu, m.yc, ff, 2 * ff, W, LE_GLU_SILU);
     p1.w_gstride = (long long)2 * ff * W; p1.cnt = m.cnt; p1.cnt_gstride = 1; p1.off = m.off; p1.xlist = m.list;
     kx_lin(s, prof, p1, rows, E);

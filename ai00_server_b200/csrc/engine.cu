@@ -529,8 +529,13 @@ struct b200rwkv_engine {
     int step_tokens = 128;             // tokens of a full step
     int maxR = 0;                      // logits rows of a step
     int part_stride(bool tiled) const { return tiled ? maxT : std::min(maxT, 128); }      // token rows between partial sums
-    MetaView meta_view(int* base, int T) const { return MetaView{base, T > 128 || kx ? maxT : std::min(maxT, 128), S}; }
-    size_t step_meta_ints(int T) const { return kx ? meta_ints : MetaView::ints(T > 128 ? maxT : std::min(maxT, 128), S); }
+    // step metadata: steps of up to 128 tokens use arrays of that length, so that a decode step uploads a few KB
+    int meta_rows(int T) const { return T > 128 ? maxT : std::min(maxT, 128); }
+    MetaView meta_view(int* base, int T) const { return MetaView{base, meta_rows(T), S}; }
+    SeqMeta seq_meta(int* base, int T) const { return SeqMeta{base + MetaView::ints(meta_rows(T), S), meta_rows(T)}; }
+    size_t step_meta_ints(int T) const { return MetaView::ints(meta_rows(T), S) + (kx ? SeqMeta::ints(meta_rows(T)) : 0); }
+    int step_rows = 0;                 // config.json families: rows of the step being enqueued
+    int dbg_T = 0;                     // rows a layer has in the debug copy of the residual stream
     double pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const;
     void launch_pair(const GemmLaunch& g, const GemmParams& gp, int rows, int parts, cudaStream_t s, Profiler* prof);
     float* gemm_ws = nullptr;
@@ -1877,10 +1882,11 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
     // logits_out == NULL: the rows stay in HBM (b200rwkv_sample_topk reads the last row of every slot from there)
     const bool copy_logits = want_logits && logits_out != nullptr;
     // f32-activation mode runs every step decode-shaped (<= 16 tokens): the split-operand kernels are the 16-token ones
-    const int step_cap = std::min(chunk, split_on ? 16 : (kx ? maxT : std::min(maxT, 128)));
+    const int step_cap = std::min(chunk, split_on ? 16 : (kx ? (kx->dbg_layers ? dbg_T : kx->portion) : std::min(maxT, 128)));
     // RWKV steps hold up to sixteen portions (gemm_pair.cuh: one pass over the weights for all their tokens): the portions, and with them the
     // rows b200rwkv_last_hidden answers, are those of 128-token steps
-    const int substeps = !kx && maxT > 128 ? std::max(1, (int)std::min<long long>(step_tokens, 16ll * chunk) / step_cap) : 1;
+    // (config.json families: portions of up to 512, steps as in kx_build)
+    const int substeps = kx ? (kx->dbg_layers ? 1 : std::max(1, maxT / step_cap)) : (maxT > 128 ? std::max(1, (int)std::min<long long>(step_tokens, 16ll * chunk) / step_cap) : 1);
     // Step packing: every step shares its token budget evenly over the entries that still have tokens (web-rwkv shares the
     // chunk "fairly across slots"; results do not depend on the cut).  Many slots with one token each keep
     // the WKV kernels wide (one CTA per head and slot) where a single slot with 64 tokens would run them 40 CTAs wide.
@@ -1907,10 +1913,15 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
         std::vector<const uint32_t*> s_toks;
         std::vector<int> step(nslot, 0), part(nslot, 0);
         for (int sub = 0; sub < substeps; ++sub) {
-            if (!kx && sub > 0) {          // room for the logits rows of another portion
-                int rows = 0;
-                for (int i = 0; i < nslot; ++i) rows += option[i] == B200RWKV_OPTION_FULL ? step[i] : (option[i] == B200RWKV_OPTION_LAST && step[i] > 0 ? 1 : 0);
-                if (rows + step_cap > maxR) break;
+            if (sub > 0) {                 // room for the logits rows that another portion may add
+                int rows = 0, ends = 0;
+                bool full = false;
+                for (int i = 0; i < nslot; ++i) {
+                    const bool more = pos[i] + step[i] < ntok[i];
+                    if (option[i] == B200RWKV_OPTION_FULL) { rows += step[i]; full = full || more; }
+                    else if (option[i] == B200RWKV_OPTION_LAST) { rows += step[i] > 0; ends += step[i] == 0 && more; }
+                }
+                if (rows + (full ? step_cap : std::min(step_cap, ends)) > maxR) break;
             }
             // at least WKV_STAGE_TOK tokens per slot and portion while prompts are long: a WKV CTA then loads and stores its 16 KB
             // of state once per four tokens or more, and a portion touches a quarter of the slots' states
@@ -3103,13 +3114,13 @@ int32_t b200rwkv_debug_read(b200rwkv_engine* e, const char* name, float* out, si
             // [num_layer][128 token rows][num_emb]
             SeqModel& m = *e->kx;
             if (n == "layers_on") {
-                if (!m.dbg_layers) m.dbg_layers = (float*)e->dalloc((size_t)e->L * e->maxT * m.W * 4);
+                if (!m.dbg_layers) m.dbg_layers = (float*)e->dalloc((size_t)e->L * e->dbg_T * m.W * 4);
                 e->use_graph = false;
                 return m.W;
             }
             REQUIRE(n == "layers" && m.dbg_layers, B200RWKV_ERR_INVALID, "unknown debug buffer: " + n);
-            REQUIRE((size_t)e->L * e->maxT * m.W <= cap, B200RWKV_ERR_INVALID, "debug buffer too small");
-            CK(cudaMemcpy(out, m.dbg_layers, (size_t)e->L * e->maxT * m.W * 4, cudaMemcpyDeviceToHost));
+            REQUIRE((size_t)e->L * e->dbg_T * m.W <= cap, B200RWKV_ERR_INVALID, "debug buffer too small");
+            CK(cudaMemcpy(out, m.dbg_layers, (size_t)e->L * e->dbg_T * m.W * 4, cudaMemcpyDeviceToHost));
             return m.W;
         }
         struct F { const char* n; float* p; int cols; };

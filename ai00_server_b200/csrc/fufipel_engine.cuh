@@ -143,7 +143,7 @@ void b200rwkv_engine::ff_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
     SeqModel& m = *kx;
     const int W = m.W;
     const float eps = m.cfg.eps, mul = m.cfg.residual_mul;
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, step_rows);
     const int* cntT = d_meta;
     auto lin = [&](const float* X, int ldx, const __nv_bfloat16* Wt, float* Y, int ldy, int N_, int K_, int epi = LE_STORE, const float* bias = nullptr) {
         LinParams p;
@@ -213,7 +213,7 @@ void b200rwkv_engine::ff_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
         }
         if (fork) { CK(cudaEventRecord(m.side_join, s2)); CK(cudaStreamWaitEvent(s, m.side_join, 0)); pdl_prev = nullptr; }
         if (m.dbg_layers && !use_graph)            // bring-up aid: the residual as this layer leaves it
-            boundary(m.dbg_layers + li * (size_t)maxT * W, nullptr, nullptr, 0, nullptr);
+            boundary(m.dbg_layers + li * (size_t)dbg_T * W, nullptr, nullptr, 0, nullptr);
     }
     boundary(nullptr, m.final_w, m.hn, 1, d_hidden);
 }

@@ -401,7 +401,8 @@ struct SeqModel {
     unsigned *lin_counters = nullptr, *lin_counters_side = nullptr;
     int max_top = 1;                             // experts a token may choose (rows of the routed launches)
     bool side_lin = false; float* lin_ws_side = nullptr;      // projections also run on the side stream: split-k sums of their own
-    float* dbg_layers = nullptr;                  // [L][maxT][W] residual after every layer (bring-up aid; nullptr: off)
+    int portion = 128;                            // tokens of a portion (a step holds several)
+    float* dbg_layers = nullptr;                  // [L][dbg_T][W] residual after every layer (bring-up aid; nullptr: off)
     int max_split = 16;
     int sa_ygroups = 1, sa_ygroups_decode = 1;    // head groups (grid rows) of the smallest windowed-attention launch of the model (prompt / decode shape)
     SeqMeta sm{nullptr, 0};

@@ -201,21 +201,25 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     REQUIRE(world == 1, B200RWKV_ERR_UNSUPPORTED, "models that come with a config.json run on one GPU in this version");
     REQUIRE(quant_layers == 0 && loras.empty(), B200RWKV_ERR_UNSUPPORTED, "models that come with a config.json take no LoRA / quantised layers");
     use_pdl = false;                                       // per launch instead (launch_k): side streams join here
-    // steps of up to 512 tokens when the caller's token_chunk_size asks for them (prompts then stream the weights once per 512
-    // tokens and fill the experts' row tiles); 128 otherwise, like the other families
-    maxT = chunk > 256 ? 512 : (chunk > 128 ? 256 : 128);
+    // Portions of up to 512 tokens when the caller's token_chunk_size asks for them, 128 otherwise.  A serving-precision step holds sixteen
+    // chunks, 2048 tokens at most: prompts then stream the weights once per 2048 tokens, fill the experts' row tiles and the two-SM projections.
+    // f32-exact steps hold one portion (plain FMA tiles, which a longer step does not fill better)
+    m.portion = chunk > 256 ? 512 : (chunk > 128 ? 256 : 128);
+    maxT = m.exact ? m.portion : std::max(m.portion, rup((int)std::min<long long>(16ll * chunk, 2048), 128));
+    maxR = std::min(maxT, 512);
+    dbg_T = m.portion;
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&sm_stream, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&step_done, cudaEventDisableTiming));
     for (auto& ev : meta_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
 
     // ---- step metadata: the common block, then positions / attention chunks / page-table updates ----
-    const size_t mv_ints = MetaView::ints(maxT, S);
-    meta_ints = mv_ints + SeqMeta::ints(maxT);
+    meta_ints = MetaView::ints(maxT, S) + SeqMeta::ints(maxT);
     d_meta = (int*)dalloc(meta_ints * 4);
     CK(cudaMallocHost(&h_meta, meta_ints * 4 * META_RING));
     memset(h_meta, 0, meta_ints * 4 * META_RING);
-    m.sm = SeqMeta{d_meta + mv_ints, maxT};
+    step_rows = maxT;
+    m.sm = seq_meta(d_meta, step_rows);
 
     // ---- pages ----
     m.page = kv_page > 0 ? kv_page : 64;
@@ -240,7 +244,11 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     const size_t T_ = (size_t)maxT;
     auto fa = [&](size_t n) { return (float*)dalloc(n * 4); };
     m.x = fa(T_ * W * z.n_streams); m.h = fa(T_ * W); m.hs = fa(T_ * W); m.G = fa(T_ * 2 * W); m.hn = fa(T_ * W);
-    m.cq = fa(T_ * z.n_cq); m.q = fa(T_ * z.n_q); m.qa = fa(T_ * z.n_qa); m.kv = fa(T_ * z.n_kv); m.part = fa(T_ * z.n_part);
+    m.cq = fa(T_ * z.n_cq); m.q = fa(T_ * z.n_q); m.qa = fa(T_ * z.n_qa); m.kv = fa(T_ * z.n_kv);
+    // partial attention results: the context is split over at most max_split CTAs and only while the launch has fewer CTAs than two waves, 4 tokens
+    // to a CTA (kx_fill_step): long steps keep one part a token
+    m.part = fa(std::max(std::min(T_, (size_t)16 * num_sms) * z.n_part, T_ * (z.n_part / std::max(1, m.max_split))));
+
     m.olat = fa(T_ * z.n_olat); m.vout = fa(T_ * z.n_vout); m.pr = fa(T_ * z.n_pr); m.z = fa(T_ * z.n_z);
     m.rl = fa(T_ * z.n_rl); m.wgt = fa(T_ * z.max_top); m.yc = fa(T_ * z.max_top * z.n_yc); m.dn = fa(T_ * z.max_top * W);
     m.ys = fa(T_ * z.n_ys); m.ds = fa(T_ * W);
@@ -253,7 +261,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     if (!m.exact && W % 8 == 0) m.h16 = (__nv_bfloat16*)dalloc(T_ * W * 2, true);
     if (!m.exact && z.n_ys % 8 == 0 && z.n_ys) m.ys16 = (__nv_bfloat16*)dalloc(T_ * z.n_ys * 2, true);
     d_hidden = fa(T_ * W);
-    d_logits = fa(T_ * V);
+    d_logits = fa((size_t)maxR * V);
     d_api = fa(m.flat_floats(m.state_ctx));
     x_a = m.x;
 
@@ -278,15 +286,18 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
     CK(cudaFuncSetAttribute(lin_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_TC_SMEM));
-    CK(cudaFuncSetAttribute(lin_umma_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<32>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(lin_umma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<64>::SMEM_BYTES));
-    CK(cudaFuncSetAttribute(lin_umma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<128>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<32>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<64>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<128>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<128, true>::SMEM_BYTES));
+    CK(cudaFuncSetAttribute(lin_umma_kernel<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<256, true>::SMEM_BYTES));
+    allow_smem(moe_group_kernel, (2048 * (size_t)MOE_MAX_TOP + 4096) * 4);
     if (!m.exact) {
         m.max_top = std::max(1, (int)z.max_top);
         m.lin_counters = (unsigned*)dalloc(LU_MAX_COUNTERS * 4, true);
         if (m.side_lin) m.lin_counters_side = (unsigned*)dalloc(LU_MAX_COUNTERS * 4, true);
         planning = true;
-        kx_enqueue_step(stream, maxT, maxT, false, 1, nullptr);
+        for (int r = maxT; r > 16; r = r > 512 ? r - 256 : r / 2) kx_enqueue_step(stream, r, std::min(r, maxR), false, 1, nullptr);
         planning = false;
         if (m.lin_x16_bytes) {
             m.lin_x16 = (__nv_bfloat16*)dalloc(m.lin_x16_bytes, false);
@@ -306,7 +317,10 @@ static void lu_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t K
 
 // the tcgen05 form of a grouped linear: rows of 16-byte chunks (K % 8, aligned weights: what a TMA box row needs), groups whose
 // weights follow one another.  Row tiles of 128 (the MMA rate's knee, 64 cycles), less for steps of few rows; routed launches see
-// a fraction of the step's rows per group and take the next smaller tile.
+// a fraction of the step's rows per group and take the next smaller tile.  Steps of more than 128 rows run on pairs of SMs, with the row tile (256
+// or 128) and the k parts whose waves take least: a stage of 64 k costs about 0.42 us with 256 rows (tensor cores under power) and 0.27 with 128
+// (bytes from L2), a unit 1.5 us of ramp and epilogue, parts a trip through the workspace.  Launches of at most 128 outputs a group (value
+// up-projections of the latent form) would leave the second SM without outputs.
 bool b200rwkv_engine::kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int rows, int groups) {
     SeqModel& m = *kx;
     if (p.K % 8 != 0 || (reinterpret_cast<uintptr_t>(p.W) & 15) != 0 || (groups > 1 && p.w_gstride != (long long)p.N * p.K)) return false;
@@ -316,10 +330,23 @@ bool b200rwkv_engine::kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int 
     if (planning) { m.lin_x16_bytes = std::max(m.lin_x16_bytes, total * p.K * 2); return true; }
     const bool side = m.side_lin && s == m.side_stream;
     __nv_bfloat16* const x16 = side ? m.lin_x16_side : m.lin_x16;
-    const int tn = p.off ? (rows <= 64 ? 32 : (rows <= 128 ? 64 : 128)) : (rows <= 32 ? 32 : (rows <= 64 ? 64 : 128));
-    const int mtiles = cdiv(p.N, LU_BM), ttiles = cdiv(rows, tn), slabs = cdiv(p.K, LU_KS);
+    int tn = p.off ? (rows <= 64 ? 32 : (rows <= 128 ? 64 : 128)) : (rows <= 32 ? 32 : (rows <= 64 ? 64 : 128));
+    const int slabs = cdiv(p.K, LU_KS), each = p.off ? cdiv((int)total, groups) : rows;      // rows of a group
+    const bool pair = rows > 128 && p.N > LU_BM && each > 64, may_split = groups == 1 && !p.off && !p.xlist;
+    const int mtiles = pair ? 2 * cdiv(p.N, 2 * LU_BM) : cdiv(p.N, LU_BM);                   // tiles of 128 outputs, whole pairs of them
     int ks = 1;
-    if (groups == 1 && !p.off && !p.xlist && mtiles * ttiles <= LU_MAX_COUNTERS) {
+    if (pair) {
+        double best = 1e30;
+        for (int nt = 256; nt >= 128; nt -= 128)
+            for (int k = 1; k <= (may_split ? std::min(8, std::max(1, slabs / 6)) : 1); ++k) {
+                const long long tiles = (long long)mtiles * cdiv(each, nt) * groups, units = tiles / 2 * k;
+                if (k > 1 && (tiles > LU_MAX_COUNTERS || (size_t)tiles * k * LU_BM * nt > m.lin_ws_floats || cdiv(slabs, cdiv(slabs, k)) != k)) continue;
+                const double t = (double)((units + num_sms / 2 - 1) / (num_sms / 2)) * (cdiv(slabs, k) * (nt == 256 ? 0.42 : 0.27) + 1.5) + (k > 1 ? 2.5 + 0.5 * k : 0.0);
+                if (t < best) { best = t; tn = nt; ks = k; }
+            }
+    }
+    const int ttiles = cdiv(rows, tn);
+    if (!pair && may_split && mtiles * ttiles <= LU_MAX_COUNTERS) {
         // k parts until the SMs are busy, at least six slabs (a ring full) each
         ks = std::max(1, std::min({num_sms / (mtiles * ttiles), 8, slabs / 6}));
         while (ks > 1 && (size_t)mtiles * ttiles * ks * LU_BM * tn > m.lin_ws_floats) --ks;
@@ -329,16 +356,20 @@ bool b200rwkv_engine::kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int 
     LinUmmaParams u;
     memset(&u, 0, sizeof(u));
     lu_map(&u.tw, p.W, (uint64_t)groups * p.N, p.K, LU_BM);
-    lu_map(&u.tx, p.X16 ? p.X16 : x16, total, p.K, tn);
+    lu_map(&u.tx, p.X16 ? p.X16 : x16, total, p.K, pair ? tn / 2 : tn);
     u.l = p; u.groups = groups; u.ksplit = ks;
     u.l.ws = side ? m.lin_ws_side : m.lin_ws;
     u.counters = side ? m.lin_counters_side : m.lin_counters;
     // list launches: the rows of all groups together are at most rows * top, plus a partial tile per group
     const int tiles = p.off ? cdiv((int)total, tn) + groups : groups * ttiles;
-    const dim3 grid(std::min(num_sms, mtiles * tiles * ks));
-    if (tn == 32) launch_k(lin_umma_kernel<32>, grid, dim3(LU_THREADS), LuCfg<32>::SMEM_BYTES, u, KC_GEMM, s, prof);
-    else if (tn == 64) launch_k(lin_umma_kernel<64>, grid, dim3(LU_THREADS), LuCfg<64>::SMEM_BYTES, u, KC_GEMM, s, prof);
-    else launch_k(lin_umma_kernel<128>, grid, dim3(LU_THREADS), LuCfg<128>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    const dim3 grid(pair ? 2 * std::min(num_sms / 2, mtiles / 2 * tiles * ks) : std::min(num_sms, mtiles * tiles * ks));
+    if (pair) {
+        launch_cluster = 2;
+        if (tn == 256) launch_k(lin_umma_kernel<256, true>, grid, dim3(LU_THREADS), LuCfg<256, true>::SMEM_BYTES, u, KC_GEMM, s, prof);
+        else launch_k(lin_umma_kernel<128, true>, grid, dim3(LU_THREADS), LuCfg<128, true>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    } else if (tn == 32) launch_k(lin_umma_kernel<32, false>, grid, dim3(LU_THREADS), LuCfg<32>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    else if (tn == 64) launch_k(lin_umma_kernel<64, false>, grid, dim3(LU_THREADS), LuCfg<64>::SMEM_BYTES, u, KC_GEMM, s, prof);
+    else launch_k(lin_umma_kernel<128, false>, grid, dim3(LU_THREADS), LuCfg<128>::SMEM_BYTES, u, KC_GEMM, s, prof);
     return true;
 }
 
@@ -402,7 +433,7 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
     SeqModel& m = *kx;
     const ScanShape sh = scan_shape(dk, dv, 3, decode);
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
-                 {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, MetaView{d_meta, maxT, S}}};
+                 {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
     launch_k(decode ? gla_scan_kernel<true> : gla_scan_kernel<false>, dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), sh.smem_floats() * 4, gp, KC_WKV, s, prof);
     if (sh.ncta > 1) launch_k(head_norm_kernel, dim3(rows, cdiv(H_, 4)), dim3(128), 0, gp.norm, KC_LN, s, prof);
 }
@@ -410,8 +441,10 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
 void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool decode, int nsplit, Profiler* prof) {
     launches_last_step = 0;
     SeqModel& m = *kx;
+    step_rows = rows;
+    m.sm = seq_meta(d_meta, rows);
     const int W = m.W;
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, step_rows);
     const int* cntT = d_meta;            // T
     const int* cntR = d_meta + 2;        // R
     auto lin = [&](const float* X, int ldx, const __nv_bfloat16* Wt, float* Y, int ldy, int N_, int K_, int epi = LE_STORE,
@@ -443,7 +476,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
         if (m.cfg.family == KX_FAMILY_DEGAVIK) {
             dg_enqueue_layer(s, l, rows, nslot_grid, decode, nsplit, prof);
             if (m.dbg_layers && !use_graph)
-                CK(cudaMemcpyAsync(m.dbg_layers + li * (size_t)maxT * W, m.x, (size_t)maxT * W * 4, cudaMemcpyDeviceToDevice, s));
+                CK(cudaMemcpyAsync(m.dbg_layers + li * (size_t)dbg_T * W, m.x, (size_t)dbg_T * W * 4, cudaMemcpyDeviceToDevice, s));
             continue;
         }
         NormShiftParams ns{m.x, m.h, m.hs, l.mu, l.shift_state, l.gain, m.cfg.eps, W, mv};
@@ -508,7 +541,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             MoeRouteParams rp{m.h, W, l.router, W, l.corr, NE, c.top, m.sel, m.wgt, mv};
             launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, NE), rp, KC_OTHER, s, prof);
             MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
-            launch_k(moe_group_kernel, dim3(1), dim3(256), ((size_t)std::max(E, 1) * 2 + (size_t)maxT * c.top) * 4, gp, KC_OTHER, s, prof);
+            launch_k(moe_group_kernel, dim3(1), dim3(rows > 128 ? MOE_GROUP_THREADS : 256), ((size_t)std::max(E, 1) * 2 + (size_t)rows * c.top) * 4, gp, KC_OTHER, s, prof);
             if (E > 0) {
                 LinParams p1 = lin(m.h, W, l.gu, m.yc, ff, 2 * ff, W, LE_GLU_CLAMP);
                 p1.w_gstride = (long long)2 * ff * W; p1.cnt = m.cnt; p1.cnt_gstride = 1; p1.off = m.off; p1.xlist = m.list; p1.limit = c.limit;
@@ -527,7 +560,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             launch_k(moe_combine_kernel, dim3(rows), dim3(256), 0, cp, KC_OTHER, s, prof);
         }
         if (m.dbg_layers && !use_graph)
-            CK(cudaMemcpyAsync(m.dbg_layers + li * (size_t)maxT * W, m.x, (size_t)maxT * W * 4, cudaMemcpyDeviceToDevice, s));
+            CK(cudaMemcpyAsync(m.dbg_layers + li * (size_t)dbg_T * W, m.x, (size_t)dbg_T * W * 4, cudaMemcpyDeviceToDevice, s));
     }
     if (!own_stack) {
         FinalNormParams fn{m.x, m.hn, d_hidden, m.final_gain, m.cfg.eps, W, mv, m.final_w};
@@ -541,20 +574,24 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
     }
 }
 
+// rows of a step's launches: powers of two up to 512 (one graph each), whole tiles of 256 beyond
 static inline int kx_bucket(int n) {
-    for (int b = 8; b < 512; b *= 2)
+    for (int b = 8; b <= 512; b *= 2)
         if (n <= b) return b;
-    return 512;
+    return rup(n, 256);
 }
 
 // positions, attention chunks and page-table updates of one step; hands out pages
 void b200rwkv_engine::kx_fill_step(int* hm, const std::vector<int>& slots, const std::vector<int>& counts, bool* decode, int* nsplit) {
     SeqModel& m = *kx;
-    int* base = hm + MetaView::ints(maxT, S);
+    int total = 0;
+    for (int c : counts) total += c;
+    const int mt = meta_rows(total);
+    int* base = hm + MetaView::ints(mt, S);
     int* tok_pos = base + 8;
-    int* ch_start = base + 8 + maxT;
-    int* ch_count = base + 8 + 2 * maxT;
-    int* upd = base + 8 + 3 * maxT;
+    int* ch_start = base + 8 + mt;
+    int* ch_count = base + 8 + 2 * mt;
+    int* upd = base + 8 + 3 * mt;
     int T = 0, nch = 0, nupd = 0, ctx_max = 1;
     bool dec = true;
     for (int c : counts) dec = dec && c == 1;
@@ -617,9 +654,9 @@ void b200rwkv_engine::kx_fill_step(int* hm, const std::vector<int>& slots, const
 
 void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     const int rows = kx_bucket(T), rrows = R > 0 ? kx_bucket(R) : 0;
-    if (!use_graph) {
+    if (!use_graph || rows > 512) {        // (launch by launch: the kernels of a long step outlast their launches)
         kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
-        enqueue_keep(stream, 1, rrows / 16 + (rrows % 16 ? 1 : 0));
+        enqueue_keep(stream, cdiv(rows, 16), rrows / 16 + (rrows % 16 ? 1 : 0));
         launch_total += launches_last_step;
         return;
     }
@@ -632,7 +669,7 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
             kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
-            enqueue_keep(stream, 1, rrows / 16 + (rrows % 16 ? 1 : 0));
+            enqueue_keep(stream, cdiv(rows, 16), rrows / 16 + (rrows % 16 ? 1 : 0));
         } catch (...) {
             cudaStreamEndCapture(stream, &g);
             if (g) cudaGraphDestroy(g);

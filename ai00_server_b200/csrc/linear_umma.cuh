@@ -2,7 +2,7 @@
 // groups, device-side row counts and row lists, epilogues), same operand rounding (f32 activations rounded to bf16 once), f32 sums.
 //
 //   lin_pack_kernel   f32 activations of every group -> bf16 rows [row][K] in a workspace (gathered through the row list)
-//   lin_umma_kernel   one persistent CTA per SM walks the units (group, 128 outputs, TN rows, k range):
+//   lin_umma_kernel   one persistent CTA per SM (PAIR: two, see below) walks the units (group, 128 outputs, TN rows, k range):
 //     * the WEIGHT tile is the 128-row operand, TN rows of activations the other: an output row is a TMEM lane, so that a warp stores
 //       32 neighbouring outputs of one row, bias and (gate, up) pairs sit in neighbouring lanes, and weights stay as stored
 //       (row-major bf16) -- both operands arrive as 64-wide k boxes in the 128-byte swizzle, edges of N, K and the rows zero filled;
@@ -10,16 +10,21 @@
 //     * units of empty groups do not exist: the walk is over the row counts the step (or the router) left on the device;
 //     * launches with fewer units than SMs cut k: every part leaves its raw sums in the workspace and the last arriver adds the parts in
 //       order and runs the epilogue.
+//   PAIR              clusters of two CTAs share a unit of 256 outputs and TN rows (tcgen05 cta_group::2, gemm_pair.cuh): each holds its 128 weight
+//                     rows, half of the activation rows and the accumulators of its outputs, and takes in half the bytes for the same work.
 //
 // What bounds it: 16 KB of weights and TN x 128 B of rows per 64 k against 4 MMAs of 64 cycles (TN = 128), i.e. the bytes an SM
 // pulls from L2; lin_tile_kernel (mma.sync on 64 x 64 tiles, f32 activations through shared memory) ran at 5-9 % of the tensor pipe.
-// Measured: the 17 projections of a 512-token step (four layers of width 2048, ncu) 2970 -> 549 us, packing 78 us beside them; 16 prompts of
+// Measured with PAIR (width 2048, ncu): the 17 projections of four steps of 512 tokens 2295 us, of one step of 2048 now about 1000; 16 prompts of 1024 tokens
+// 47.8 -> 32.5 ms, eight documents 7.7 -> 5.1 ms.
+// Measured before that: the 17 projections of a 512-token step (four layers of width 2048, ncu) 2970 -> 549 us, packing 78 us beside them; 16 prompts of
 // 1024 tokens 124 -> 48 ms, eight documents through latent attention and routed experts 15.3 -> 7.7 ms.
 #pragma once
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
 #include "common.cuh"
+#include "gemm_pair.cuh"
 #include "linear.cuh"
 
 namespace b200 {
@@ -36,14 +41,14 @@ struct alignas(64) LinUmmaParams {
     unsigned* counters;        // [tiles], zero between launches (ksplit > 1)
 };
 
-template <int TN>
+template <int TN, bool PAIR = false>
 struct LuCfg {
-    static constexpr int W_BYTES = LU_BM * LU_KS * 2, X_BYTES = TN * LU_KS * 2;
+    static constexpr int W_BYTES = LU_BM * LU_KS * 2, X_BYTES = (PAIR ? TN / 2 : TN) * LU_KS * 2;
     static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
     static constexpr int NSTAGE = 196608 / STAGE_BYTES > 8 ? 8 : 196608 / STAGE_BYTES;
     static constexpr int BAR_OFF = NSTAGE * STAGE_BYTES;
     static constexpr int SMEM_BYTES = BAR_OFF + (2 * NSTAGE + 4) * 8 + 16 + 1024;       // + alignment of the ring
-    static constexpr int TMEM_COLS = 2 * TN;                                            // 64 .. 256: double-buffered accumulator
+    static constexpr int TMEM_COLS = 2 * TN;                                            // 64 .. 512: double-buffered accumulator
 };
 
 // K-major operand in the 128-byte swizzle: 8-row atoms of 1024 bytes; a k16 step is 32 bytes further
@@ -54,6 +59,13 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) { return um
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+
+// PAIR: counted on the barrier at a cluster address (the leader's)
+__device__ __forceinline__ void tma2_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(map), "r"(x), "r"(y), "r"(bar)
                  : "memory");
 }
@@ -80,7 +92,7 @@ __global__ void __launch_bounds__(256) lin_pack_kernel(const LinParams p, __nv_b
 
 // walks the units of a CTA: unit = ((group's tiles before it) ...) -> (group, output tile, row tile, k part), row tiles fastest so that
 // CTAs that run side by side share a weight tile
-template <int TN>
+template <int TN, bool PAIR>
 struct LuWalk {
     const LinUmmaParams* p;
     int u, step, g, ubase, rows, ttiles, mtiles, per;
@@ -90,8 +102,8 @@ struct LuWalk {
         per = ttiles * mtiles * p->ksplit;
     }
     __device__ __forceinline__ void init(const LinUmmaParams& p_) {
-        p = &p_; u = blockIdx.x; step = gridDim.x; g = 0; ubase = 0;
-        mtiles = (p_.l.N + LU_BM - 1) / LU_BM;
+        p = &p_; u = PAIR ? (int)cluster_id_x() : (int)blockIdx.x; step = PAIR ? (int)ncluster_x() : (int)gridDim.x; g = 0; ubase = 0;
+        mtiles = (p_.l.N + (PAIR ? 2 : 1) * LU_BM - 1) / ((PAIR ? 2 : 1) * LU_BM);
         load_group();
         settle();
     }
@@ -114,53 +126,71 @@ struct LuWalk {
     }
 };
 
-template <int TN>
+template <int TN, bool PAIR>
 __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_constant__ LinUmmaParams p) {
-    using Cfg = LuCfg<TN>;
+    using Cfg = LuCfg<TN, PAIR>;
     extern __shared__ uint8_t lu_smem[];
     __shared__ int s_last;
     const uint32_t ring = (smem_u32(lu_smem) + 1023u) & ~1023u;
     const uint32_t full_bar = ring + Cfg::BAR_OFF, empty_bar = full_bar + Cfg::NSTAGE * 8;
     const uint32_t tfull_bar = empty_bar + Cfg::NSTAGE * 8, tempty_bar = tfull_bar + 16, tmem_slot = tempty_bar + 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = PAIR ? (int)cluster_rank() : 0;         // 0: the leader, which issues the MMAs of both
     if (tid == 0) {
         for (int s = 0; s < Cfg::NSTAGE; ++s) { mbar_init(full_bar + s * 8, 1); mbar_init(empty_bar + s * 8, 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(tfull_bar + s * 8, 1); mbar_init(tempty_bar + s * 8, LU_EPI_WARPS); }
+        for (int s = 0; s < 2; ++s) { mbar_init(tfull_bar + s * 8, 1); mbar_init(tempty_bar + s * 8, (PAIR ? 2 : 1) * LU_EPI_WARPS); }
         mbar_fence_init();
     }
-    if (warp == LU_EPI_WARPS) tc_alloc(tmem_slot, Cfg::TMEM_COLS);
+    if (warp == LU_EPI_WARPS) {
+        if constexpr (PAIR) tc_alloc2(tmem_slot, Cfg::TMEM_COLS);
+        else tc_alloc(tmem_slot, Cfg::TMEM_COLS);
+    }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();                  // the peer's barriers exist before anything arrives there
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
     // only now: a dependent CTA that took its tensor memory first would wait for this grid while this grid waited for columns
     pdl_launch_dependents();
     pdl_wait();
-    LuWalk<TN> w;
+    LuWalk<TN, PAIR> w;
     w.init(p);
+    auto out_tile = [&]() { return PAIR ? 2 * w.mt() + rank : w.mt(); };      // 128 outputs of this CTA
 
     if (warp == LU_EPI_WARPS + 1) {
         if (lane == 0) {
-            int stage = 0;
+            int stage = 0, done = 0;
             uint32_t ephase = 1;
+            const uint32_t lead_full = PAIR ? mapa_u32(full_bar, 0) : 0;
             for (; !w.done(); w.next()) {
                 int s0, n;
                 w.slabs(s0, n);
-                const int wrow = w.g * p.l.N + w.mt() * LU_BM, xrow = (p.l.off ? p.l.off[w.g] : w.g * p.l.max_rows) + w.tt() * TN;
-                for (int i = 0; i < n; ++i) {
+                const int wrow = w.g * p.l.N + out_tile() * LU_BM, xrow = (p.l.off ? p.l.off[w.g] : w.g * p.l.max_rows) + w.tt() * TN + rank * (TN / 2);
+                for (int i = 0; i < n; ++i, ++done) {
                     mbar_wait(empty_bar + stage * 8, ephase, 21);
                     const uint32_t st = ring + stage * Cfg::STAGE_BYTES, fb = full_bar + stage * 8;
-                    mbar_expect_tx(fb, Cfg::STAGE_BYTES);
-                    tma_load_2d(st, &p.tw, (s0 + i) * LU_KS, wrow, fb);
-                    tma_load_2d(st + Cfg::W_BYTES, &p.tx, (s0 + i) * LU_KS, xrow, fb);
+                    if constexpr (PAIR) {
+                        if (rank == 0) mbar_expect_tx(fb, 2 * Cfg::STAGE_BYTES);
+                        tma2_load_2d(st, &p.tw, (s0 + i) * LU_KS, wrow, lead_full + stage * 8);
+                        tma2_load_2d(st + Cfg::W_BYTES, &p.tx, (s0 + i) * LU_KS, xrow, lead_full + stage * 8);
+                    } else {
+                        mbar_expect_tx(fb, Cfg::STAGE_BYTES);
+                        tma_load_2d(st, &p.tw, (s0 + i) * LU_KS, wrow, fb);
+                        tma_load_2d(st + Cfg::W_BYTES, &p.tx, (s0 + i) * LU_KS, xrow, fb);
+                    }
                     if (++stage == Cfg::NSTAGE) { stage = 0; ephase ^= 1; }
                 }
             }
+            // PAIR: every stage in use is released before this CTA may end: the leader's last commits arrive here
+            for (int i = 0, n = PAIR ? min(done, Cfg::NSTAGE) : 0; i < n; ++i) {
+                const int last = done - 1 - i;
+                mbar_wait(empty_bar + (last % Cfg::NSTAGE) * 8, (uint32_t)(last / Cfg::NSTAGE) & 1u, 25);
+            }
         }
     } else if (warp == LU_EPI_WARPS) {
-        if (lane == 0) {
-            constexpr uint32_t IDESC = umma_idesc_bf16(LU_BM, TN);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t IDESC = umma_idesc_bf16((PAIR ? 2 : 1) * LU_BM, TN);
             int stage = 0;
             uint32_t phase = 0;
             unsigned cnt = 0;
@@ -168,40 +198,56 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
                 int s0, n;
                 w.slabs(s0, n);
                 const unsigned acc = cnt & 1u, use = cnt >> 1;
-                if (use > 0) mbar_wait(tempty_bar + acc * 8, (use - 1) & 1u, 22);
+                if (use > 0) {
+                    if constexpr (PAIR) mbar_wait_cluster(tempty_bar + acc * 8, (use - 1) & 1u, 22);
+                    else mbar_wait(tempty_bar + acc * 8, (use - 1) & 1u, 22);
+                }
                 tc_fence_after();
                 const uint32_t d = tmem_base + acc * TN;
                 uint32_t accumulate = 0;
                 for (int i = 0; i < n; ++i) {
-                    mbar_wait(full_bar + stage * 8, phase, 23);
+                    if constexpr (PAIR) mbar_wait_cluster(full_bar + stage * 8, phase, 23);
+                    else mbar_wait(full_bar + stage * 8, phase, 23);
                     tc_fence_after();
                     const uint32_t st = ring + stage * Cfg::STAGE_BYTES;
 #pragma unroll
                     for (int k = 0; k < LU_KS / 16; ++k) {
-                        tc_mma_f16(d, umma_desc_sw128(st + k * 32), umma_desc_sw128(st + Cfg::W_BYTES + k * 32), IDESC, accumulate);
+                        if constexpr (PAIR) tc_mma2_f16(d, umma_desc_sw128(st + k * 32), umma_desc_sw128(st + Cfg::W_BYTES + k * 32), IDESC, accumulate);
+                        else tc_mma_f16(d, umma_desc_sw128(st + k * 32), umma_desc_sw128(st + Cfg::W_BYTES + k * 32), IDESC, accumulate);
                         accumulate = 1;
                     }
-                    tc_commit(empty_bar + stage * 8);
+                    if constexpr (PAIR) tc_commit2(empty_bar + stage * 8);
+                    else tc_commit(empty_bar + stage * 8);
                     if (++stage == Cfg::NSTAGE) { stage = 0; phase ^= 1; }
                 }
-                tc_commit(tfull_bar + acc * 8);
+                if constexpr (PAIR) tc_commit2(tfull_bar + acc * 8);
+                else tc_commit(tfull_bar + acc * 8);
             }
         }
     } else {
         const LinParams& l = p.l;
         const int grp = warp >> 2, row = tid & (LU_BM - 1);
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+        const uint32_t lead_tempty = PAIR ? mapa_u32(tempty_bar, 0) : 0;
+        auto drained = [&](const unsigned acc) {                // this warp has read its part of the accumulator
+            tc_fence_before();
+            __syncwarp();
+            if (lane != 0) return;
+            if constexpr (PAIR) mbar_arrive_cluster(lead_tempty + acc * 8);
+            else mbar_arrive(tempty_bar + acc * 8);
+        };
         unsigned cnt = 0;
         for (; !w.done(); w.next(), ++cnt) {
             const unsigned acc = cnt & 1u, use = cnt >> 1;
-            const int g = w.g, n = w.mt() * LU_BM + row, r0 = w.tt() * TN, nr = min(TN, w.rows - r0);
+            const int g = w.g, n = out_tile() * LU_BM + row, r0 = w.tt() * TN, nr = min(TN, w.rows - r0);
             const int yrow0 = (l.off ? l.off[g] : 0) + r0;
             const bool ok = n < l.N;
             const float bias = ok && l.bias && l.epi != LE_GLU_CLAMP && l.epi != LE_GLU_SILU ? l.bias[(size_t)g * l.N + n] : 0.f;
-            mbar_wait(tfull_bar + acc * 8, use & 1u, 24);
+            if constexpr (PAIR) mbar_wait_cluster(tfull_bar + acc * 8, use & 1u, 24);
+            else mbar_wait(tfull_bar + acc * 8, use & 1u, 24);
             tc_fence_after();
             const uint32_t tm = tmem_base + lane_base + acc * TN;
-            const int tile = w.mt() * w.ttiles + w.tt();
+            const int tile = out_tile() * w.ttiles + w.tt();
             float* const ws = l.ws + (size_t)tile * p.ksplit * (LU_BM * TN) + row * 4;
             if (p.ksplit > 1) {
                 float* const mine = ws + (size_t)w.part() * (LU_BM * TN);
@@ -213,9 +259,7 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
                     for (int j = 0; j < 4; ++j)
                         *reinterpret_cast<float4*>(mine + (size_t)(c / 4 + j) * (LU_BM * 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty_bar + acc * 8);
+                drained(acc);
                 named_bar_sync(1, LU_EPI_THREADS);      // every thread's stores before thread 0's release
                 if (tid == 0) {
                     const unsigned old = atom_add_acq_rel_gpu(p.counters + tile, 1u);
@@ -254,21 +298,39 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
                     } else {
                         tc_ld16(tm + c, v);
                     }
+                    if constexpr (PAIRS) {
+                        // lanes (2 i, 2 i + 1) = (gate, up); N and split are even.  Of two neighbouring rows the even lane finishes the first, the odd lane
+                        // the second: one exchange and one gated unit a lane for two rows (a gated unit of every row in the even lanes alone took
+                        // 28 us a unit of 256 outputs x 256 rows where its MMAs take 13)
+                        const int odd = lane & 1;
+                        const bool glu = EPI != LE_SPLIT_GLU_RELU || n >= l.split;
+#pragma unroll
+                        for (int j = 0; j < 16; j += 2) {
+                            const float x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+                            const float ga_ = odd ? x : v[j], up = odd ? v[j + 1] : x;
+                            if (EPI == LE_SPLIT_GLU_RELU && !glu) {
+#pragma unroll
+                                for (int q = 0; q < 2; ++q)
+                                    if (ok && c + j + q < nr) Y[(size_t)(yrow0 + c + j + q) * l.ldy + n] = v[j + q] + bias;
+                                continue;
+                            }
+                            const int r = c + j + odd;
+                            if (!ok || r >= nr) continue;
+                            if constexpr (EPI == LE_SPLIT_GLU_RELU) {
+                                l.Y2[(size_t)(yrow0 + r) * l.ldy2 + ((n - l.split) >> 1)] = fmaxf(ga_, 0.f) * up;
+                            } else {
+                                const float y = EPI == LE_GLU_CLAMP ? lin_glu(ga_, up, l.limit) : ga_ * lin_sigmoid(ga_) * up;
+                                if (l.Y16) l.Y16[(size_t)(yrow0 + r) * l.ldy + (n >> 1)] = __float2bfloat16(y);
+                                else Y[(size_t)(yrow0 + r) * l.ldy + (n >> 1)] = y;
+                            }
+                        }
+                        continue;
+                    }
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const bool in = ok && c + j < nr;
                         float* const yr = Y + (size_t)(yrow0 + c + j) * l.ldy;
-                        if constexpr (PAIRS) {              // lanes (2 i, 2 i + 1) = (gate, up); N is even
-                            const float up = __shfl_xor_sync(0xffffffffu, v[j], 1);
-                            if constexpr (EPI == LE_SPLIT_GLU_RELU) {
-                                if (in && n < l.split) yr[n] = v[j] + bias;
-                                else if (in && (lane & 1) == 0) l.Y2[(size_t)(yrow0 + c + j) * l.ldy2 + ((n - l.split) >> 1)] = fmaxf(v[j], 0.f) * up;
-                            } else if (in && (lane & 1) == 0) {
-                                const float y = EPI == LE_GLU_CLAMP ? lin_glu(v[j], up, l.limit) : v[j] * lin_sigmoid(v[j]) * up;
-                                if (l.Y16) l.Y16[(size_t)(yrow0 + c + j) * l.ldy + (n >> 1)] = __float2bfloat16(y);
-                                else yr[n >> 1] = y;
-                            }
-                        } else if (in) {
+                        if (in) {
                             const float a = v[j] + bias;
                             float y = a;
                             if constexpr (EPI == LE_SIGMOID) y = lin_sigmoid(a);
@@ -296,16 +358,18 @@ __global__ void __launch_bounds__(LU_THREADS, 1) lin_umma_kernel(const __grid_co
                 case LE_SPLIT_GLU_RELU: body(std::integral_constant<int, LE_SPLIT_GLU_RELU>{}); break;
                 default: body(std::integral_constant<int, LE_STORE>{}); break;
             }
-            if (p.ksplit == 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty_bar + acc * 8);
-            }
+            if (p.ksplit == 1) drained(acc);
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == LU_EPI_WARPS) tc_dealloc(tmem_base, Cfg::TMEM_COLS);
+    if constexpr (PAIR) {
+        cluster_sync_all();                                  // no CTA leaves while its peer's MMAs read its shared memory or arrive on its barriers
+        tc_fence_after();
+        if (warp == LU_EPI_WARPS) tc_dealloc2(tmem_base, Cfg::TMEM_COLS);
+    } else if (warp == LU_EPI_WARPS) {
+        tc_dealloc(tmem_base, Cfg::TMEM_COLS);
+    }
 }
 
 }  // namespace b200

@@ -205,7 +205,8 @@ struct MoeGroupParams {
     MetaView meta;
 };
 
-__global__ void __launch_bounds__(256) moe_group_kernel(const MoeGroupParams p) {
+constexpr int MOE_GROUP_THREADS = 1024;    // a warp per expert in long steps
+__global__ void __launch_bounds__(MOE_GROUP_THREADS) moe_group_kernel(const MoeGroupParams p) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ int moe_smem[];         // [E] counts, [E] offsets, [T * top] choices

@@ -151,7 +151,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
     SeqModel& m = *kx;
     const int W = m.W;
     const float eps = m.cfg.eps;
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, step_rows);
     const int* cntT = d_meta;
     auto lin = [&](const float* X, int ldx, const __nv_bfloat16* Wt, float* Y, int ldy, int N_, int K_, int epi = LE_STORE, const float* bias = nullptr) {
         LinParams p;
@@ -239,7 +239,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             post_w = l.norm2b_w;
         }
         if (m.dbg_layers && !use_graph)            // bring-up aid: the residual as this run leaves it
-            boundary(m.dbg_layers + li * (size_t)maxT * W, nullptr, nullptr, nullptr, 0, nullptr);
+            boundary(m.dbg_layers + li * (size_t)dbg_T * W, nullptr, nullptr, nullptr, 0, nullptr);
     }
     boundary(nullptr, nullptr, m.final_w, m.hn, 1, d_hidden);
 }

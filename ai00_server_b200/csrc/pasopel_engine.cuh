@@ -142,7 +142,7 @@ void b200rwkv_engine::ps_repool(int slot, int n) {
     SeqModel& m = *kx;
     for (KxLayer& l : m.layers) {
         if (!l.pcache || n / l.c.pool == 0) continue;
-        PoolWriteParams pw{l.cache, l.pcache, m.d_table, m.npages, m.page, l.cache_D, l.c.pool, l.prow, slot, n / l.c.pool, MetaView{d_meta, maxT, S}, m.sm};
+        PoolWriteParams pw{l.cache, l.pcache, m.d_table, m.npages, m.page, l.cache_D, l.c.pool, l.prow, slot, n / l.c.pool, meta_view(d_meta, step_rows), m.sm};
         pool_rebuild_kernel<<<n / l.c.pool, 128, 0, stream>>>(pw);
         CK(cudaGetLastError());
     }
@@ -153,7 +153,7 @@ void b200rwkv_engine::ps_repool(int slot, int n) {
 void b200rwkv_engine::ps_enqueue_layers(cudaStream_t s, int rows, int nslot_grid, bool decode, int nsplit, Profiler* prof) {
     SeqModel& m = *kx;
     const int W = m.W;
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, step_rows);
     const int* cntT = d_meta;
     auto lin = [&](const float* X, int ldx, const __nv_bfloat16* Wt, float* Y, int ldy, int N_, int K_, int epi = LE_STORE, const float* bias = nullptr) {
         LinParams p;
@@ -239,7 +239,7 @@ void b200rwkv_engine::ps_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 MoeRouteParams rp{m.h, W, l.router, W, l.corr, E, c.top, m.sel, m.wgt, mv, MOE_TOP_LOGITS};
                 launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, E), rp, KC_OTHER, s, prof);
                 MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
-                launch_k(moe_group_kernel, dim3(1), dim3(256), ((size_t)E * 2 + (size_t)maxT * c.top) * 4, gp, KC_OTHER, s, prof);
+                launch_k(moe_group_kernel, dim3(1), dim3(rows > 128 ? MOE_GROUP_THREADS : 256), ((size_t)E * 2 + (size_t)rows * c.top) * 4, gp, KC_OTHER, s, prof);
                 LinParams p1 = lin(m.h, W, l.gu, m.yc, ff, 2 * ff, W, LE_GLU_SILU);
                 p1.w_gstride = (long long)2 * ff * W; p1.cnt = m.cnt; p1.cnt_gstride = 1; p1.off = m.off; p1.xlist = m.list;
                 kx_lin(s, prof, p1, rows, E);
@@ -254,9 +254,9 @@ void b200rwkv_engine::ps_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             }
         }
         if (m.dbg_layers && !use_graph) {          // bring-up aid: the residual as this run leaves it
-            float* dst = m.dbg_layers + li * (size_t)maxT * W;
+            float* dst = m.dbg_layers + li * (size_t)dbg_T * W;
             if (pend.rows) boundary(dst, nullptr, nullptr, nullptr, nullptr, 0, nullptr);
-            else CK(cudaMemcpyAsync(dst, m.x, (size_t)maxT * W * 4, cudaMemcpyDeviceToDevice, s));
+            else CK(cudaMemcpyAsync(dst, m.x, (size_t)dbg_T * W * 4, cudaMemcpyDeviceToDevice, s));
         }
     }
     boundary(nullptr, nullptr, nullptr, m.final_w, m.hn, 1, d_hidden);

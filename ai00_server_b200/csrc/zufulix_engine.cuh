@@ -202,7 +202,7 @@ void b200rwkv_engine::zf_load(const StFile& st, KxSizes& z) {
 void b200rwkv_engine::zf_enqueue_layers(cudaStream_t s, int rows, int nslot_grid, bool decode, int nsplit, Profiler* prof) {
     SeqModel& m = *kx;
     const int W = m.W, NS = m.streams;
-    MetaView mv{d_meta, maxT, S};
+    const MetaView mv = meta_view(d_meta, step_rows);
     const int* cntT = d_meta;
     auto lin = [&](const float* X, int ldx, const __nv_bfloat16* Wt, float* Y, int ldy, int N_, int K_, int epi = LE_STORE, const float* bias = nullptr) {
         LinParams p;
@@ -247,7 +247,7 @@ void b200rwkv_engine::zf_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 MoeRouteParams rp{m.h, W, l.router, W, nullptr, E, c.top, m.sel, m.wgt, mv, MOE_SIGMOID_GROUPS, c.groups, c.groups_keep};
                 launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, E), rp, KC_OTHER, s, prof);
                 MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
-                launch_k(moe_group_kernel, dim3(1), dim3(256), ((size_t)E * 2 + (size_t)maxT * c.top) * 4, gp, KC_OTHER, s, prof);
+                launch_k(moe_group_kernel, dim3(1), dim3(rows > 128 ? MOE_GROUP_THREADS : 256), ((size_t)E * 2 + (size_t)rows * c.top) * 4, gp, KC_OTHER, s, prof);
                 LinParams p1 = lin(m.h, W, l.gu, m.yc, ff, ff, W, LE_RELU_SQ);
                 p1.w_gstride = (long long)ff * W; p1.cnt = m.cnt; p1.cnt_gstride = 1; p1.off = m.off; p1.xlist = m.list;
                 kx_lin(s, prof, p1, rows, E);
@@ -259,7 +259,7 @@ void b200rwkv_engine::zf_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
         }
         if (m.dbg_layers && !use_graph) {          // bring-up aid: the layer's output lands in the streams now, their sum is kept
             boundary(HC_READ_NONE, nullptr, nullptr, nullptr, nullptr, 0, nullptr);
-            HcSumParams sp{m.x, m.dbg_layers + li * (size_t)maxT * W, NS, W, mv};
+            HcSumParams sp{m.x, m.dbg_layers + li * (size_t)dbg_T * W, NS, W, mv};
             launch_k(hc_sum_kernel, dim3(rows), dim3(NORM_THREADS), 0, sp, KC_LN, s, prof);
         }
     }

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from ai00_server_b200 import capi, runtime, synth
-from oracle import kemirax_numpy, panupel_numpy
+from oracle import kemirax_numpy, panupel_numpy, sampling_numpy
 from oracle import rwkv_numpy as O
 
 pytestmark = pytest.mark.gpu
@@ -124,15 +124,42 @@ def _check_family(make, layers, module, n, **kw):
         m.close()
 
 
-@pytest.mark.parametrize("n", [17, 32, 33, 64, 65, 127, 128, 129, 300])
+@pytest.mark.parametrize("family", ["rwkv", "panupel", "kemirax"])
+def test_kept_rows_of_long_steps(family):
+    """The row a slot keeps for sampling, found through the metadata of a step of more than 128 and of more than 512 tokens."""
+    lens = [130, 700, 5]
+    rng = np.random.default_rng(5)
+    toks = [rng.integers(1, 90, n).tolist() for n in lens]
+    kw = {"max_batch": 3, "token_chunk_size": 512}
+    if family == "rwkv":
+        st = synth.make_st("tiny6", 3)
+    else:
+        layer = synth.panupel_layer("delta", heads=3, dim=24, ff=200) if family == "panupel" else synth.kemirax_layer("latent_attention", mlp=False)
+        cfg, st, _ = (synth.make_panupel if family == "panupel" else synth.make_kemirax)([layer], seed=4)
+        kw.update(config=cfg, kv_tokens=1024, kv_page=16)
+    m = runtime.Model(st, **kw)
+    try:
+        for s in range(3):
+            m.state.reset(s)
+        for call in ([0, 2], [1, 2]):                # 135 tokens in the first step; 705 in the second call's
+            rows = m.infer_raw(call, [lens[s] for s in call], sum((toks[s] for s in call), []), [capi.OPTION_LAST] * 2)
+            ids, _ = m.sample_topk(call, top_k=20)
+            for i in range(2):
+                assert np.array_equal(ids[i], sampling_numpy.sorted_candidates(rows[i][0], top_k=20)[0])
+    finally:
+        m.close()
+
+
+@pytest.mark.parametrize("n", [17, 32, 33, 64, 65, 127, 128, 129, 300, 513, 1100, 2100])
 def test_projections_of_a_step_of_n_rows(n):
-    """Row tiles of 32 / 64 / 128 and their remainders, outputs and k ranges that are no multiple of a tile."""
+    """Row tiles of 32 / 64 / 128, of 128 / 256 on pairs of SMs, and their remainders, outputs and k ranges that are no multiple of a tile; more rows
+    than a step holds (2048)."""
     L = synth.panupel_layer
     _check_family(synth.make_panupel, [L("delta", heads=3, dim=24, ff=200), L("parallel", heads=2, dim=40, mm_heads=1, mm_dim=24, ff=72)], panupel_numpy, n,
                   width=136)
 
 
-@pytest.mark.parametrize("n", [20, 70, 130])
+@pytest.mark.parametrize("n", [20, 70, 130, 700])
 @pytest.mark.parametrize("experts, top", [(3, 1), (8, 4)])
 def test_routed_projections_of_a_step_of_n_rows(n, experts, top):
     """Row lists of experts: groups of very unequal size, empty ones among them."""
