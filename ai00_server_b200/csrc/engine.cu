@@ -33,6 +33,7 @@
 #endif
 #include "wkv.cuh"
 #include "wkv_scan.cuh"
+#include "lora2.cuh"
 #include "linear.cuh"
 #include "linear_umma.cuh"
 #include "rmsnorm.cuh"
@@ -433,6 +434,7 @@ struct Layer {
     // v6 decode front half as one launch (pre6.cuh): row-major copies of the ddlerp LoRA weights
     const __half* w1_raw = nullptr;
     const __half* w2_raw = nullptr;
+    const __half* wd2_raw = nullptr;    // prompt steps (lora2.cuh): row-major time_decay_w2
     const float* mu5[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 };
 
@@ -1334,12 +1336,13 @@ void b200rwkv_engine::build(const StFile& st) {
                         "time_mix_w2 must be [5, C, Dm]");
                 REQUIRE(d2.shape.size() == 2 && d2.shape[0] == C && d2.shape[1] == Dd, B200RWKV_ERR_INVALID, "time_decay_w2 must be [C, Dd]");
             }
+            auto upload_raw = [&](const StTensor& t) {
+                __half* d = (__half*)dalloc(t.nbytes, false);
+                CK(cudaMemcpy(d, t.data, t.nbytes, cudaMemcpyHostToDevice));
+                return d;
+            };
+            if (world == 1 && C % LORA2_COLS == 0 && (Dd == 32 || Dd == 64 || Dd == 128)) ly.wd2_raw = upload_raw(st.get(a + "time_decay_w2"));
             if (fused_pre && (Dm == 32 || Dm == 64) && C % 128 == 0 && C <= PRE_MAX_C) {
-                auto upload_raw = [&](const StTensor& t) {
-                    __half* d = (__half*)dalloc(t.nbytes, false);
-                    CK(cudaMemcpy(d, t.data, t.nbytes, cudaMemcpyHostToDevice));
-                    return d;
-                };
                 ly.w1_raw = upload_raw(st.get(a + "time_mix_w1"));
                 ly.w2_raw = upload_raw(st.get(a + "time_mix_w2"));
                 for (int i = 0; i < 5; ++i) ly.mu5[i] = ly.pre[1].p.seg[i].aux2;
@@ -1608,7 +1611,7 @@ void b200rwkv_engine::finalize_tp() {
 void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof, bool runs) {
     launches_last_step = 0;
     const int rows = MT * 16;
-    const bool tiled = MT > 8;                 // more than 128 tokens: operands in 128-token tiles, projections on pairs of SMs
+    const bool tiled = MT >= 8 && maxT > 128;  // more than 64 tokens: operands in 128-token tiles, projections on pairs of SMs
     const MetaView mv = meta_view(d_meta, rows);
     // token rows of this step's A16 operands (common.cuh): every producer and consumer of the step uses the same value
     const int th = (split_on && MT == 1) ? 32 : (tiled ? 128 : 16 * MT);
@@ -1630,8 +1633,11 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
     // sequences of more than WKV_STAGE_TOK tokens: the scan kernel, with the decays of its own launch (split operands stay with the
     // decode kernel, whose steps hold 16 tokens at most)
     const bool scan = runs && !split_on;
+    auto lora2_w2 = [&](const Layer& ly, int gi) { return MT >= 2 && world == 1 && ly.w2_raw && gi == 1; };
+    auto lora2_wd2 = [&](const Layer& ly, int gi) { return MT >= 2 && scan && ly.wd2_raw && gi == ly.wd2_index; };
     auto pre_skipped = [&](const Layer& ly, int gi) {
         if (fold_wd2 && !scan && gi == ly.wd2_index) return true;        // the WKV kernel evaluates the decay LoRA stage 2
+        if (lora2_w2(ly, gi) || lora2_wd2(ly, gi)) return true;          // lora2.cuh
         return fused_pre_ok && MT == 1 && ly.w1_raw && gi < 2;           // the front-half kernel holds both ddlerp LoRA stages
     };
     // projection launches of this step in stream order: each one prefetches the head of the next into L2 (the last one
@@ -1666,11 +1672,12 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
         }
         for (int i = 0; i < g2.p.nseg; ++i)
             if (g2.p.seg[i].out_mode != OUT_F32) g2.p.seg[i].ldo = th_of(g2.p.seg[i].out_tile);      // A16 outputs feed a projection of this step
-        if (mt > 8 && g.short_k && !g.chain) {
+        const bool pairs = mt >= 8 && maxT > 128;
+        if (pairs && g.short_k && !g.chain && mt > 8) {
             // one-block tiles, a CTA per weight tile and 128 tokens
             launch_k(gemm_wide_kernel<8, true>, dim3(std::min(g.total_tiles, 2 * num_sms), 1, mt / 8), dim3(WIDE_THREADS), WideCfg<8, true>::SMEM_BYTES, g2.p, KC_GEMM, s,
                      prof, 1, g.total_tiles);
-        } else if (mt > 8) {
+        } else if (pairs && !(g.short_k && !g.chain) && (mt > 8 || g.by_tile || g.chain)) {      // (few tiles of a long k and one tile of tokens: k cut over the SMs)
             launch_pair(g, g2.p, mt * 16, g.chain ? (g.p.seg[0].out == (void*)part_att ? parts_o : parts_v) : 0, s, prof);
         } else {
             launch_gemm(g2, mt, s, prof, split_on && MT == 1);      // split operands only when the whole step is decode-shaped
@@ -1726,8 +1733,34 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             take_parts(n1, part_ffn, parts_v);
             launch_ln(n1);
         }
-        for (int gi = 0; gi < (int)ly.pre.size(); ++gi)
-            if (!pre_skipped(ly, gi)) gemm(ly.pre[gi]);
+        for (int gi = 0; gi < (int)ly.pre.size(); ++gi) {
+            if (!pre_skipped(ly, gi)) { gemm(ly.pre[gi]); continue; }
+            if (!lora2_w2(ly, gi) && !lora2_wd2(ly, gi)) continue;
+            Lora2Params q;
+            memset(&q, 0, sizeof(q));
+            q.C = C; q.meta = mv;
+            const bool few = rows <= LORA2_TOK;
+            const dim3 grid(C / (few ? LORA2_FEW_COLS : LORA2_COLS), cdiv(rows, LORA2_TOK));
+            auto go = [&](auto k16, auto groups) {
+                constexpr int K16 = decltype(k16)::value, G = decltype(groups)::value;
+                if (few) launch_k(lora2_kernel<K16, G, LORA2_FEW_COLS>, grid, dim3(LORA2_THREADS), lora2_smem<K16, G, LORA2_FEW_COLS>(), q, KC_GEMM, s, prof);
+                else launch_k(lora2_kernel<K16, G, LORA2_COLS>, grid, dim3(LORA2_THREADS), lora2_smem<K16, G, LORA2_COLS>(), q, KC_GEMM, s, prof);
+            };
+            using std::integral_constant;
+            if (lora2_w2(ly, gi)) {
+                q.w = ly.w2_raw; q.low = a_lora[0].p; q.low_stride = (int)a_lora[0].halves_per_matrix; q.low_th = th_of(a_lora[0].tile_kb);
+                q.xx = xx1; q.sx = sx1; q.out_th = th_of(a_x[0].tile_kb);
+                for (int j = 0; j < 5; ++j) { q.mu[j] = ly.mu5[j]; q.out[j] = a_x[j].p; }
+                if (info.time_mix_adapter == 32) go(integral_constant<int, 2>{}, integral_constant<int, 5>{});
+                else go(integral_constant<int, 4>{}, integral_constant<int, 5>{});
+            } else {
+                q.w = ly.wd2_raw; q.low = a_lora[1].p; q.low_th = th_of(a_lora[1].tile_kb);
+                q.bias = ly.pre[gi].p.seg[0].bias; q.decay = f_w;
+                if (info.time_decay_adapter == 32) go(integral_constant<int, 2>{}, integral_constant<int, 1>{});
+                else if (info.time_decay_adapter == 64) go(integral_constant<int, 4>{}, integral_constant<int, 1>{});
+                else go(integral_constant<int, 8>{}, integral_constant<int, 1>{});
+            }
+        }
         {
             // decays / staged rows are sized by the step shape: a slot cannot hold more tokens than the step
             WkvParams wp = ly.wkv;
