@@ -298,29 +298,23 @@ class Model:
 
     # ---- raw call: one b200rwkv_infer ----
     def infer_raw(self, slots, ntok, tokens, options, out: np.ndarray | None = None, keep_on_device: bool = False):
-        V = self.info["num_vocab"]          # rank 0 receives the gathered full-vocabulary rows
+        # a call per generated token: addresses as plain numbers, no list comprehensions over arrays
         n = len(slots)
-        total = sum(nt if o == capi.OPTION_FULL else (1 if (o == capi.OPTION_LAST and nt > 0) else 0)
-                    for nt, o in zip(ntok, options))
-        if keep_on_device:                  # logits_out = NULL: rows stay in HBM for sample_topk
-            a_slot, a_ntok = np.asarray(slots, np.int32), np.asarray(ntok, np.int32)
-            a_tok, a_opt = np.asarray(tokens, np.uint32), np.asarray(options, np.int32)
-            a_rows = np.zeros(max(n, 1), np.int32)
-            capi.check(capi.lib().b200rwkv_infer(self._h, n, capi.ptr(a_slot), capi.ptr(a_ntok), capi.ptr(a_tok),
-                                                 capi.ptr(a_opt), None, 0, capi.ptr(a_rows)), self._h)
-            return [int(r) for r in a_rows[:n]]
-        if out is None:
-            out = np.empty((max(total, 1), V), np.float32)
-        a_slot = np.asarray(slots, np.int32)
-        a_ntok = np.asarray(ntok, np.int32)
-        a_tok = np.asarray(tokens, np.uint32)
-        a_opt = np.asarray(options, np.int32)
+        a_slot, a_ntok = np.asarray(slots, np.int32), np.asarray(ntok, np.int32)
+        a_tok, a_opt = np.asarray(tokens, np.uint32), np.asarray(options, np.int32)
         a_rows = np.zeros(max(n, 1), np.int32)
-        capi.check(capi.lib().b200rwkv_infer(self._h, n, capi.ptr(a_slot), capi.ptr(a_ntok), capi.ptr(a_tok),
-                                             capi.ptr(a_opt), capi.ptr(out), out.size, capi.ptr(a_rows)), self._h)
+        if keep_on_device:                  # logits_out = NULL: rows stay in HBM for sample_topk
+            capi.check(capi.lib().b200rwkv_infer(self._h, n, a_slot.ctypes.data, a_ntok.ctypes.data, a_tok.ctypes.data, a_opt.ctypes.data, None, 0,
+                                                 a_rows.ctypes.data), self._h)
+            return a_rows[:n].tolist()
+        if out is None:
+            V = self.info["num_vocab"]          # rank 0 receives the gathered full-vocabulary rows
+            total = sum(nt if o == capi.OPTION_FULL else (1 if (o == capi.OPTION_LAST and nt > 0) else 0) for nt, o in zip(ntok, options))
+            out = np.empty((max(total, 1), V), np.float32)
+        capi.check(capi.lib().b200rwkv_infer(self._h, n, a_slot.ctypes.data, a_ntok.ctypes.data, a_tok.ctypes.data, a_opt.ctypes.data, out.ctypes.data, out.size,
+                                             a_rows.ctypes.data), self._h)
         res, off = [], 0
-        for i in range(n):
-            r = int(a_rows[i])
+        for r in a_rows[:n].tolist():
             res.append(out[off:off + r])
             off += r
         return res
@@ -340,13 +334,14 @@ class Model:
         penalties, bias: per-slot dict token -> value (the reference's HashMaps, nucleus.rs:29, run.rs:679);
         allow: optional [n, V] bool array (tokens the formatter allows)."""
         n = len(slots)
-        V = self.info["num_vocab"]
 
-        def pack(maps):
+        def pack(maps):                     # (offsets, tokens, values) of the slots' dicts; no lists at all without any
+            if maps is None:
+                return None, None, None
             off = np.zeros(n + 1, np.int32)
             toks, vals = [], []
             for i in range(n):
-                m = (maps[i] if maps is not None else None) or {}
+                m = maps[i] or {}
                 toks.extend(int(t) for t in m.keys())
                 vals.extend(float(v) for v in m.values())
                 off[i + 1] = len(toks)
@@ -356,6 +351,7 @@ class Model:
         bo, bt, bv = pack(bias)
         bits = None
         if allow is not None:
+            V = self.info["num_vocab"]
             a = np.asarray(allow, bool).reshape(n, V)
             words = (V + 31) // 32
             padded = np.zeros((n, words * 32), bool)
@@ -364,9 +360,8 @@ class Model:
         ids = np.empty((n, top_k), np.uint32)
         probs = np.empty((n, top_k), np.float32)
         a_slot = np.asarray(slots, np.int32)
-        capi.check(capi.lib().b200rwkv_sample_topk(self._h, n, capi.ptr(a_slot), capi.ptr(po), capi.ptr(pt), capi.ptr(pv),
-                                                   capi.ptr(bits) if bits is not None else None, capi.ptr(bo), capi.ptr(bt),
-                                                   capi.ptr(bv), top_k, capi.ptr(ids), capi.ptr(probs)), self._h)
+        at = lambda x: None if x is None else x.ctypes.data  # noqa: E731
+        capi.check(capi.lib().b200rwkv_sample_topk(self._h, n, at(a_slot), at(po), at(pt), at(pv), at(bits), at(bo), at(bt), at(bv), top_k, at(ids), at(probs)), self._h)
         return ids, probs
 
     def launch_count(self) -> int:
