@@ -48,6 +48,7 @@
 #include "bias_attn.cuh"
 #include "hyper.cuh"
 #include "sink_attn.cuh"
+#include "prompt_attn.cuh"
 
 namespace b200 {
 
@@ -480,6 +481,8 @@ struct Group {
     int32_t spmd(const std::function<int32_t(int)>& fn);
 };
 
+typedef void (*SinkAttnKernel)(const SinkAttnParams);
+
 struct b200rwkv_engine {
     std::unique_ptr<Group> group;             // set on rank 0 of an in-process tensor-parallel engine
     b200rwkv_info info;
@@ -608,6 +611,8 @@ struct b200rwkv_engine {
     void kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool decode, int nsplit, Profiler* prof);
     void kx_fill_step(int* hm, const std::vector<int>& slots, const std::vector<int>& counts, bool* decode, int* nsplit);
     void kx_run_step(int T, int R, bool decode, int nsplit);
+    void kx_sink_attn(cudaStream_t s, Profiler* prof, const KxLayer& l, const SinkAttnParams& sp, SinkAttnKernel kern, int threads, size_t smem, int rows, int nslot_grid,
+                      int chunks_grid, bool decode, int nsplit);
     void kx_release(int slot);
     void kx_reset(int slot);
     void kx_xfer(int slot, float* rec, int ctx_rows, bool import, int n);
@@ -1132,6 +1137,9 @@ void b200rwkv_engine::build(const StFile& st) {
         CK(cudaFuncSetAttribute(wkv_kernel<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
     }
     allow_smem(ln_mix_rows_kernel, (size_t)(LN_ROWS + 1) * C * 4);
+    allow_smem(wkv_scan_kernel<5>, WksCfg<5>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<6>, WksCfg<6>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<7>, WksCfg<7>::SMEM_BYTES);
     if (precision == 1) split_act = true;         // f32-activation mode (web-rwkv `Bundle::<f32>`): no activation is rounded to f16
     if (const char* v = dbg_env("B200RWKV_PREFETCH_BLOCKS")) prefetch_blocks = std::max(0, atoi(v));
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;
@@ -3060,6 +3068,9 @@ int32_t b200rwkv_op_wkv(int32_t device, int32_t version, int32_t T, int32_t H, c
     p.kq_tile = 64;                       // token rows of the A16 output: any value >= T the reader below agrees on
     CK(cudaMemset(p.out, 0, halves * 2));
     const size_t smem = wkv_smem_bytes(version, false, 0, maxT);
+    allow_smem(wkv_scan_kernel<5>, WksCfg<5>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<6>, WksCfg<6>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<7>, WksCfg<7>::SMEM_BYTES);
     switch (version) {
         case 5:
             if (T > WKV_STAGE_TOK) wkv_scan_kernel<5><<<dim3(H, 1), WKS_THREADS, WksCfg<5>::SMEM_BYTES>>>(p);

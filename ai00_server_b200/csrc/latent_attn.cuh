@@ -38,6 +38,30 @@ struct SeqMeta {
     __host__ __device__ static size_t ints(int maxT) { return 8 + 6 * (size_t)maxT; }
 };
 
+// The run-th run of at most qt tokens of one sequence, counted through the step's sequences, found by one warp: out = (sequence of the step or -1, run within it)
+__device__ __forceinline__ void step_token_run(const MetaView& meta, const int qt, const int run, int* out) {
+    const int lane = threadIdx.x & 31, nslots = meta.nslots();
+    int left = run, found = -1;
+    for (int s0 = 0; s0 < nslots && found < 0; s0 += 32) {
+        const int s = s0 + lane, n = s < nslots ? (meta.slot_count()[s] + qt - 1) / qt : 0;
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, left < upto);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            left -= __shfl_sync(0xffffffffu, upto - n, l);
+            found = s0 + l;
+        } else {
+            left -= __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
+    if (lane == 0) { out[0] = found; out[1] = left; }
+}
+
 struct PageUpdateParams { SeqMeta sm; int* table; int stride; };
 
 __global__ void page_update_kernel(const PageUpdateParams p) {

@@ -214,8 +214,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             sp.qb = plan.qb; sp.gt = plan.gt; sp.cl = nsplit; sp.nbuf = plan.nbuf; sp.ks = plan.ks;
             sp.nsub = decode ? 1 : m.qb_prompt / plan.qb;
             sp.meta = mv; sp.sm = m.sm;
-            launch_cluster = nsplit;
-            launch_k(plan.kern, dim3(chunks_grid * sp.nsub * nsplit, cdiv(H_, plan.hb)), dim3(plan.threads), plan.smem, sp, KC_WKV, s, prof);
+            kx_sink_attn(s, prof, l, sp, plan.kern, plan.threads, plan.smem, rows, nslot_grid, chunks_grid, decode, nsplit);
             if (fork) { CK(cudaEventRecord(m.side_join, s2)); CK(cudaStreamWaitEvent(s, m.side_join, 0)); pdl_prev = nullptr; }
         } else {
             const PnDeltaRow r(c);

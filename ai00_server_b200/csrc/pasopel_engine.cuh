@@ -201,8 +201,7 @@ void b200rwkv_engine::ps_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             }
             sp.q = m.q; sp.ldq = H_ * dk; sp.pcache = l.pcache; sp.koff = 0; sp.voff = G_ * dk; sp.out = m.vout; sp.ldo = H_ * dv;
             sp.gate = m.pr + C_; sp.ldg = PN; sp.scale = 1.f; sp.pool = c.pool; sp.prow = l.prow;
-            launch_cluster = nsplit;
-            launch_k(plan.kern, attn_grid, dim3(plan.threads), plan.smem, sp, KC_WKV, s, prof);
+            kx_sink_attn(s, prof, l, sp, plan.kern, plan.threads, plan.smem, rows, nslot_grid, chunks_grid, decode, nsplit);
         } else {
             const int dn = c.dim, dr = c.rot_dim, rk = c.kv_rank, D = rk + dr, QW = H_ * (dn + dr);
             RmsRowsParams rr{m.pr, PN, m.cq, c.q_rank, l.dq_norm, c.q_rank, 1, m.cfg.eps, cntT};

@@ -5,7 +5,6 @@
 
 using namespace b200;
 
-typedef void (*SinkAttnKernel)(const SinkAttnParams);
 static inline SinkAttnKernel sa_tile_kernel(int rb) {
     return rb >= 4 ? sink_attn_kernel<4> : (rb == 2 ? sink_attn_kernel<2> : sink_attn_kernel<1>);
 }
@@ -124,6 +123,7 @@ static void sa_plan_model(SeqModel& m) {
         CK(cudaFuncSetAttribute(sa_tile_kernel(rb), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         for (bool decode : {false, true}) CK(cudaFuncSetAttribute(sa_reg_kernel(rb, decode), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
+    allow_smem(prompt_attn_kernel, prompt_attn_smem(PA_DMAX, PA_DMAX));
     // the largest cluster the attention launch may ask for: what the device can co-schedule at this layer's shared memory
     for (const KxLayer& l : m.layers) {
         if (!sa_layer(l.c)) continue;
@@ -158,4 +158,18 @@ static void sa_plan_model(SeqModel& m) {
         m.wa_ctas_prompt = std::max(1, std::min(m.wa_ctas_prompt, np));
         m.wa_ctas_decode = std::max(1, std::min(m.wa_ctas_decode, nd));
     }
+}
+
+// One attention launch.  Prompt steps whose chunks fill the chip without splitting the keys (kx_fill_step's rule) take the kernel that stages a key tile for 64
+// (token, head) rows, where its 16-byte rows and sizes allow; block means and longer rows stay with the forms above.
+void b200rwkv_engine::kx_sink_attn(cudaStream_t s, Profiler* prof, const KxLayer& l, const SinkAttnParams& sp, SinkAttnKernel kern, int threads, size_t smem, int rows,
+                                   int nslot_grid, int chunks_grid, bool decode, int nsplit) {
+    const int rep = sp.H / sp.G;
+    if (!decode && nsplit == 1 && l.sa_reg && sp.pool == 0 && rep <= PA_ROWS && sp.koff % 4 == 0 && sp.voff % 4 == 0 && sp.D % 4 == 0 && sp.ldq % 4 == 0) {
+        PromptAttnParams pa{sp, PA_ROWS / rep};
+        launch_k(prompt_attn_kernel, dim3(cdiv(rows, pa.qt) + nslot_grid, sp.G), dim3(PA_THREADS), prompt_attn_smem(sp.dk, sp.dv), pa, KC_WKV, s, prof);
+        return;
+    }
+    launch_cluster = nsplit;
+    launch_k(kern, dim3(chunks_grid * sp.nsub * nsplit, cdiv(sp.H, sp.HB)), dim3(threads), smem, sp, KC_WKV, s, prof);
 }
