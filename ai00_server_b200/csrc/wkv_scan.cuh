@@ -8,12 +8,16 @@
 //     write vectors, value residual, bonus) is worked out per group of tokens, a warp per token;
 //   * a thread holds 4 values x 8 neighbouring keys of the state; key-indexed vectors lie in shared memory with each run of eight split into
 //     two half rows, so that the eight lanes of a value row read 128 contiguous bytes and the other three rows of the warp share them;
-//   * the four read-outs of a thread are summed over the eight lanes by halving (4 shuffles instead of 12); norms and outputs
-//     follow per group, a warp per token.  The sums of the recurrence, the norm and the bonus run in wkv.cuh's order.
+//   * products run as packed pairs of neighbouring keys (half the instructions of a loop that is bound by them); RWKV-5 / 6: the bonus of the current
+//     token, (sum_c r u k) v, is one number a token, worked out with the group and added behind the sums;
+//   * the loop over tokens leaves the four read-outs of a thread as they are; the eight lanes' parts are summed with the norms and outputs, per group, a
+//     warp per token (exchanges between lanes in the loop were a chain of four, some 25 cycles each, on every token).  Sums over keys run even and odd
+//     keys apart: results agree with wkv.cuh's to f32 rounding.
 // Decays come from the decay projection's own launch in these steps (17 us beside the scan's own time below).  Where the decode kernel
 // evaluates that low-rank stage itself (RWKV-6), its sums run in another order: decays, and with them states, agree to f32 rounding and not to the bit.
 // Measured (one prompt of 100 tokens, 64 heads, ncu): 263 -> 33 us per layer.
 #pragma once
+#include "f32x2.cuh"
 #include "wkv.cuh"
 
 namespace b200 {
@@ -23,7 +27,8 @@ template <int VER> struct WksCfg {
     static constexpr int TC = VER == 7 ? 8 : 16;            // tokens per group
     static constexpr int NA = VER == 7 ? 6 : 4;             // staged vectors: r, k, v, w (, -kk, kk a)
     static constexpr int BUF = NA * TC * WKV_N;             // floats of one group
-    static constexpr int SMEM_BYTES = (2 * BUF + 2 * TC + TC * WKV_N) * 4;
+    static constexpr int OUT_ROW = WKV_N + 4, OUT = 8 * OUT_ROW;      // a token's read-outs: eight partial sums of every value (padded: conflict-free)
+    static constexpr int SMEM_BYTES = (2 * BUF + 2 * TC + TC * OUT) * 4;
 };
 // place of key c in a staged vector: keys 8 j .. 8 j + 3 at 4 j, 8 j + 4 .. 8 j + 7 at 32 + 4 j
 __device__ __forceinline__ int wks_place(int c) { return (c >> 3) * 4 + (c & 3) + ((c >> 2) & 1) * 32; }
@@ -33,21 +38,21 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
     using Cfg = WksCfg<VER>;
     constexpr int TC = Cfg::TC, TW = TC / 4;                // tokens per warp in the per-group phases
     extern __shared__ __align__(16) float wks[];
-    float* const sc = wks + 2 * Cfg::BUF;                   // [2][TC] v7: bonus of the token
-    float* const so = sc + 2 * TC;                          // [TC][64] read-outs
+    float* const sc = wks + 2 * Cfg::BUF;                   // [2][TC] bonus of the token
+    float* const so = sc + 2 * TC;                          // [TC][8][64] partial read-outs
     pdl_launch_dependents();
     const int h = blockIdx.x, si = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ig = tid >> 3, j = tid & 7, ch = h * WKV_N;
     if (si >= p.meta.nslots()) return;
     const int slot = p.meta.slot_id()[si], t0 = p.meta.slot_start()[si], nt = p.meta.slot_count()[si];
     float* const M = p.state + ((size_t)slot * p.H + h) * (WKV_N * WKV_N);
-    float m[4][8];
+    f32x2 m[4][4];                                          // pairs of keys
 #pragma unroll
     for (int e = 0; e < 4; ++e)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const float4 v4 = __ldcs(reinterpret_cast<const float4*>(M + (ig * 4 + e) * WKV_N + 8 * j + 4 * q));
-            m[e][4 * q] = v4.x; m[e][4 * q + 1] = v4.y; m[e][4 * q + 2] = v4.z; m[e][4 * q + 3] = v4.w;
+            m[e][2 * q] = pack2(v4.x, v4.y); m[e][2 * q + 1] = pack2(v4.z, v4.w);
         }
     const int c2 = ch + lane;                               // the per-group phases give a lane the channels lane and lane + 32
     auto ld2 = [](const float* q) { return make_float2(q[0], q[32]); };
@@ -55,11 +60,7 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
     float2 kk_ = make_float2(0.f, 0.f), ka_ = kk_, rk_ = kk_, ws = kk_;
     if (VER == 7) { kk_ = ld2(p.k_k + c2); ka_ = ld2(p.k_a + c2); rk_ = ld2(p.r_k + c2); }
     if (VER == 5) ws = ld2(p.w_static + c2);
-    float u[8];
-    if (VER != 7) {
-#pragma unroll
-        for (int f = 0; f < 8; ++f) u[f] = p.u[ch + 8 * j + f];
-    }
+    const float2 u2 = VER != 7 ? ld2(p.u + c2) : make_float2(0.f, 0.f);
     pdl_wait();
 
     struct Row { float2 r, k, v, w, a, nu, vf; };
@@ -107,6 +108,10 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
                 st2(4, tt, make_float2(-kk.x, -kk.y));
                 st2(5, tt, make_float2(kk.x * a.x, kk.y * a.y));
             }
+            if (VER != 7) {
+                const float bonus = sum2(make_float2(r.x * (u2.x * k.x), r.y * (u2.y * k.y)));
+                if (lane == 0) sc[b * TC + tt] = bonus;
+            }
             st2(0, tt, r); st2(1, tt, k);
             buf[(2 * TC + tt) * WKV_N + lane] = v.x;        // by value
             buf[(2 * TC + tt) * WKV_N + lane + 32] = v.y;
@@ -128,36 +133,39 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
         const float* const buf = wks + b * Cfg::BUF;
 #pragma unroll 2
         for (int tt = 0; tt < n; ++tt) {
-            auto ld8 = [&](const int arr, float (&x)[8]) {
-                const float4 lo = *reinterpret_cast<const float4*>(buf + (arr * TC + tt) * WKV_N + 4 * j);
-                const float4 hi = *reinterpret_cast<const float4*>(buf + (arr * TC + tt) * WKV_N + 32 + 4 * j);
-                x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+            auto ld8 = [&](const int arr, f32x2 (&x)[4]) {
+                const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(buf + (arr * TC + tt) * WKV_N + 4 * j);
+                const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(buf + (arr * TC + tt) * WKV_N + 32 + 4 * j);
+                x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
             };
-            float r[8], k[8], w[8], o[4];
+            f32x2 r[4], k[4], w[4];
+            float o[4];
             ld8(0, r); ld8(1, k); ld8(3, w);
             const float4 v4 = *reinterpret_cast<const float4*>(buf + (2 * TC + tt) * WKV_N + 4 * ig);
-            const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+            const f32x2 v[4] = {pack2(v4.x, v4.x), pack2(v4.y, v4.y), pack2(v4.z, v4.z), pack2(v4.w, v4.w)};
             if (VER != 7) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float acc = 0.f;
+                    f32x2 acc = 0ull;
 #pragma unroll
-                    for (int f = 0; f < 8; ++f) {
-                        const float kv = k[f] * v[e];
-                        acc += r[f] * (u[f] * kv + m[e][f]);
-                        m[e][f] = kv + w[f] * m[e][f];
+                    for (int f = 0; f < 4; ++f) {
+                        fma2(acc, r[f], m[e][f]);
+                        m[e][f] = fmadd2(w[f], m[e][f], prod2(k[f], v[e]));
                     }
-                    o[e] = acc;
+                    const float2 a2 = unpack2(acc);
+                    o[e] = a2.x + a2.y;
                 }
             } else {
-                float nk[8], ka[8], sa[4];
+                f32x2 nk[4], ka[4];
+                float sa[4];
                 ld8(4, nk); ld8(5, ka);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float s = 0.f;
+                    f32x2 s = prod2(m[e][0], nk[0]);
 #pragma unroll
-                    for (int f = 0; f < 8; f += 4) s += (m[e][f] * nk[f] + m[e][f + 1] * nk[f + 1]) + (m[e][f + 2] * nk[f + 2] + m[e][f + 3] * nk[f + 3]);
-                    sa[e] = s;
+                    for (int f = 1; f < 4; ++f) fma2(s, m[e][f], nk[f]);
+                    const float2 a2 = unpack2(s);
+                    sa[e] = a2.x + a2.y;
                 }
 #pragma unroll
                 for (int off = 4; off > 0; off >>= 1)
@@ -165,22 +173,18 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
                     for (int e = 0; e < 4; ++e) sa[e] += __shfl_xor_sync(0xffffffffu, sa[e], off);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float acc = 0.f;
+                    const f32x2 s2 = pack2(sa[e], sa[e]);
+                    f32x2 acc = 0ull;
 #pragma unroll
-                    for (int f = 0; f < 8; ++f) {
-                        m[e][f] = m[e][f] * w[f] + sa[e] * ka[f] + v[e] * k[f];
-                        acc += m[e][f] * r[f];
+                    for (int f = 0; f < 4; ++f) {
+                        m[e][f] = fmadd2(v[e], k[f], fmadd2(s2, ka[f], prod2(m[e][f], w[f])));
+                        fma2(acc, m[e][f], r[f]);
                     }
-                    o[e] = acc;
+                    const float2 a2 = unpack2(acc);
+                    o[e] = a2.x + a2.y;
                 }
             }
-            // sum over the eight lanes of a row group, halving the values: lane j ends with value (j >> 1) of its four
-            const float a0 = (j & 4) ? o[0] : o[2], a1 = (j & 4) ? o[1] : o[3];
-            const float k0 = ((j & 4) ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, a0, 4);
-            const float k1 = ((j & 4) ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, a1, 4);
-            float y = ((j & 2) ? k1 : k0) + __shfl_xor_sync(0xffffffffu, (j & 2) ? k0 : k1, 2);
-            y += __shfl_xor_sync(0xffffffffu, y, 1);
-            if ((j & 1) == 0) so[tt * WKV_N + ig * 4 + (j >> 1)] = y;
+            *reinterpret_cast<float4*>(so + tt * Cfg::OUT + j * Cfg::OUT_ROW + ig * 4) = make_float4(o[0], o[1], o[2], o[3]);
         }
         prepare(g0 + TC, b ^ 1);
         __syncthreads();
@@ -189,14 +193,20 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
         for (int i = 0; i < TW; ++i) {
             const int tt = warp + 4 * i;
             if (tt >= n) continue;
-            const float2 x = ld2(so + tt * WKV_N + lane);
+            float2 x = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const float2 y = ld2(so + tt * Cfg::OUT + q * Cfg::OUT_ROW + lane);
+                x.x += y.x; x.y += y.y;
+            }
+            const float s = sc[b * TC + tt];
+            const float2 v = ld2(buf + (2 * TC + tt) * WKV_N + lane);
+            if (VER != 7) { x.x = fmaf(s, v.x, x.x); x.y = fmaf(s, v.y, x.y); }
             const float mean = warp_sum(x.x + x.y) * (1.f / WKV_N);
             const float d0 = x.x - mean, d1 = x.y - mean;
             const float rstd = 1.0f / sqrtf(warp_sum(d0 * d0 + d1 * d1) * (1.f / WKV_N) + GN_EPS);
             float y0 = d0 * rstd * lw.x + lb.x, y1 = d1 * rstd * lw.y + lb.y;
             if (VER == 7) {
-                const float s = sc[b * TC + tt];
-                const float2 v = ld2(buf + (2 * TC + tt) * WKV_N + lane);
                 y0 += s * v.x; y1 += s * v.y;
             }
             y0 *= gate[i].x; y1 *= gate[i].y;
@@ -209,7 +219,10 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
     for (int e = 0; e < 4; ++e)
 #pragma unroll
         for (int q = 0; q < 2; ++q)
-            __stcs(reinterpret_cast<float4*>(M + (ig * 4 + e) * WKV_N + 8 * j + 4 * q), make_float4(m[e][4 * q], m[e][4 * q + 1], m[e][4 * q + 2], m[e][4 * q + 3]));
+        {
+            const float2 lo = unpack2(m[e][2 * q]), hi = unpack2(m[e][2 * q + 1]);
+            __stcs(reinterpret_cast<float4*>(M + (ig * 4 + e) * WKV_N + 8 * j + 4 * q), make_float4(lo.x, lo.y, hi.x, hi.y));
+        }
 }
 
 }  // namespace b200
