@@ -80,7 +80,7 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
     unsigned long long* const list = reinterpret_cast<unsigned long long*>(topk_smem);      // [topk_list(V)], shared: the first TOPK_SHARE
     unsigned long long* const all = list + topk_list(p.V);                                  // [TOPK_CTAS * TOPK_SHARE]
     float* const sx = reinterpret_cast<float*>(topk_smem);                                  // [cnt] while lists are applied
-    __shared__ unsigned long long s_best[TOPK_THREADS];
+    __shared__ __align__(16) unsigned long long s_best[TOPK_THREADS];
     __shared__ unsigned long long s_few, s_full;            // the (top_k / 8)-th and the top_k-th best thread
     __shared__ float2 s_stat;                               // (max, sum exp(x - max)) of the slice
     __shared__ float red[32];
@@ -153,16 +153,28 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
     sum = block_sum_any(sum, red);                          // (its barriers also publish s_best)
     if (tid == 0) s_stat = make_float2(mx, sum);
     int above = 0;
-    for (int i = 0; i < TOPK_THREADS; ++i) above += s_best[i] > best;
+#pragma unroll 16
+    for (int i = 0; i < TOPK_THREADS; i += 2) {
+        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2*>(s_best + i);
+        above += (b2.x > best) + (b2.y > best);
+    }
     if (best && above == (p.top_k + TOPK_CTAS - 1) / TOPK_CTAS - 1) s_few = best;
     if (best && above == p.top_k - 1) s_full = best;
     cluster.sync();
+    // all remote reads of a phase are requested before the first is used: one trip through the cluster instead of eight
     unsigned long long few = ~0ull, full = 0;
     float M = -INFINITY;
-    for (int c = 0; c < TOPK_CTAS; ++c) {
-        few = min(few, *cluster.map_shared_rank(&s_few, c));
-        full = max(full, *cluster.map_shared_rank(&s_full, c));
-        M = fmaxf(M, cluster.map_shared_rank(&s_stat, c)->x);
+    float2 stat[TOPK_CTAS];
+    {
+        unsigned long long fw[TOPK_CTAS], fl[TOPK_CTAS];
+#pragma unroll
+        for (int c = 0; c < TOPK_CTAS; ++c) {
+            fw[c] = *cluster.map_shared_rank(&s_few, c);
+            fl[c] = *cluster.map_shared_rank(&s_full, c);
+            stat[c] = *cluster.map_shared_rank(&s_stat, c);
+        }
+#pragma unroll
+        for (int c = 0; c < TOPK_CTAS; ++c) { few = min(few, fw[c]); full = max(full, fl[c]); M = fmaxf(M, stat[c].x); }
     }
     const unsigned long long bound = max(max(few, full), 1ull);
     // candidates of the slice -> list, in any order
@@ -204,17 +216,28 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
         if (tid == 0) s_n = n;
     }
     cluster.sync();
-    int total = 0;
+    int total = 0, from[TOPK_CTAS];                         // candidates of the CTAs in front
     float denom = 0.f;
-    for (int c = 0; c < TOPK_CTAS; ++c) {
-        const int nc = *cluster.map_shared_rank(&s_n, c);
-        const unsigned long long* from = cluster.map_shared_rank(list, c);
-        for (int i = tid; i < nc; i += TOPK_THREADS) all[total + i] = from[i];
-        total += nc;
-        const float2 st = *cluster.map_shared_rank(&s_stat, c);
-        if (st.x > -INFINITY) denom += st.y * expf(st.x - M);
+    {
+        int nc[TOPK_CTAS];
+#pragma unroll
+        for (int c = 0; c < TOPK_CTAS; ++c) nc[c] = *cluster.map_shared_rank(&s_n, c);
+#pragma unroll
+        for (int c = 0; c < TOPK_CTAS; ++c) {
+            from[c] = total;
+            total += nc[c];
+            if (stat[c].x > -INFINITY) denom += stat[c].y * expf(stat[c].x - M);
+        }
     }
-    cluster.sync();                                         // every CTA has read the others: they may leave
+    for (int i = tid; i < total; i += TOPK_THREADS) {
+        int c = 0, at0 = 0;
+#pragma unroll
+        for (int q = 1; q < TOPK_CTAS; ++q)
+            if (i >= from[q]) { c = q; at0 = from[q]; }
+        all[i] = cluster.map_shared_rank(list, c)[i - at0];
+    }
+    __syncthreads();
+    cluster.barrier_arrive();                               // this CTA has read the others: they may leave (the wait is at the end)
     const float inv = 1.0f / denom;
     for (int i = warp; i < n; i += TOPK_THREADS / 32) {
         const unsigned long long key = list[i];
@@ -233,6 +256,8 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
             p.out_id[(size_t)row * p.top_k + i] = 0xFFFFFFFFu;
             p.out_p[(size_t)row * p.top_k + i] = 0.f;
         }
+    __syncwarp();
+    cluster.barrier_wait();
 }
 
 // ---------------------------------------------------------------------------------------
