@@ -38,6 +38,7 @@
 #include "linear_umma.cuh"
 #include "rmsnorm.cuh"
 #include "latent_attn.cuh"
+#include "latent_prompt.cuh"
 #include "gla.cuh"
 #include "moe.cuh"
 #include "retention.cuh"

@@ -282,6 +282,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
         allow_smem(latent_attn_tc_kernel<1, 16>, smem_tc);
         allow_smem(latent_attn_tc_kernel<2, 8>, smem_tc);
     }
+        allow_smem(latent_prompt_kernel, LATENT_PROMPT_SMEM);
     CK(cudaFuncSetAttribute(gla_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
@@ -503,7 +504,11 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 launch_k(kv_write_kernel, dim3(rows), dim3(128), 0, kw, KC_OTHER, s, prof);
             }
             LatentAttnParams ap{m.qa, l.cache, m.d_table, m.npages, m.page, m.part, H_, rk, dr, nsplit, c.scale, mv, m.sm};
-            if (!m.exact) {         // serving precision: both products on the tensor cores (TF32 operands, f32 accumulation and softmax)
+            if (whole) {
+                LatentPromptParams lp{ap, m.olat, std::min(H_, 16), 0};
+                lp.qt = LP_ROWS / lp.hg;
+                launch_k(latent_prompt_kernel, dim3(cdiv(rows, lp.qt) + nslot_grid, cdiv(H_, lp.hg)), dim3(LP_THREADS), latent_prompt_smem(D), lp, KC_WKV, s, prof);
+            } else if (!m.exact) {         // serving precision: both products on the tensor cores (TF32 operands, f32 accumulation and softmax)
                 const size_t sm_b = latent_attn_tc_smem(D);
                 if (!decode) launch_k(latent_attn_tc_kernel<4, 4>, dim3(cdiv(rows, 4) + nslot_grid, cdiv(H_, 4), nsplit), dim3(LA_THREADS), sm_b, ap, KC_WKV, s, prof);
                 else if (H_ > 8) launch_k(latent_attn_tc_kernel<1, 16>, dim3(rows, cdiv(H_, 16), nsplit), dim3(LA_THREADS), sm_b, ap, KC_WKV, s, prof);
@@ -517,10 +522,11 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 launch_k(latent_attn_kernel<1, 8>, dim3(rows, cdiv(H_, 8), nsplit), dim3(LA_THREADS), latent_attn_smem<1, 8>(D), ap, KC_WKV, s, prof);
             }
             LatentMergeParams mp{m.part, m.olat, H_, rk, nsplit, mv};
-            launch_k(latent_merge_kernel, dim3(rows, H_), dim3(128), 0, mp, KC_WKV, s, prof);
+            if (!whole) launch_k(latent_merge_kernel, dim3(rows, H_), dim3(128), 0, mp, KC_WKV, s, prof);
             {
                 LinParams p = lin(m.olat, H_ * rk, l.uv, m.vout, H_ * dv, dv, rk);
                 p.x_gstride = rk; p.w_gstride = (long long)dv * rk; p.y_gstride = dv;
+            const bool whole = !m.exact && !decode && nsplit == 1 && D % 4 == 0 && rk <= 64 * LP_MAX_NT && latent_prompt_smem(D) <= LATENT_PROMPT_SMEM;      // latent_prompt.cuh
                 kx_lin(s, prof, p, rows, H_);
             }
             LinParams po = lin(m.vout, H_ * dv, l.o, m.x, W, W, H_ * dv, LE_GATED_ADD);
