@@ -541,6 +541,10 @@ struct b200rwkv_engine {
     SeqMeta seq_meta(int* base, int T) const { return SeqMeta{base + MetaView::ints(meta_rows(T), S), meta_rows(T)}; }
     size_t step_meta_ints(int T) const { return MetaView::ints(meta_rows(T), S) + (kx ? SeqMeta::ints(meta_rows(T)) : 0); }
     int step_rows = 0;                 // config.json families: rows of the step being enqueued
+    int step_seqs = 0;                 // sequences of the step
+    // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
+    // column a thread, and a chain of tokens takes longer with two)
+    bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }
     int dbg_T = 0;                     // rows a layer has in the debug copy of the residual stream
     double pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const;
     void launch_pair(const GemmLaunch& g, const GemmParams& gp, int rows, int parts, cudaStream_t s, Profiler* prof);
@@ -2011,6 +2015,7 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
         if (kx) kx_fill_step(hm, s_slots, s_counts, &kx_decode, &kx_split);
         CK(cudaMemcpyAsync(d_meta, hm, step_meta_ints(T) * 4, cudaMemcpyHostToDevice, stream));
         CK(cudaEventRecord(meta_ev[mb], stream));
+        step_seqs = (int)s_slots.size();
         if (kx) kx_run_step(T, R, kx_decode, kx_split);
         else run_step(mt_bucket(T), R > 0 ? mt_bucket(R) : 0, *std::max_element(s_counts.begin(), s_counts.end()) > WKV_STAGE_TOK);
         if (hidden_keep) {       // hidden rows of every token of this call (b200rwkv_last_hidden), in entry order

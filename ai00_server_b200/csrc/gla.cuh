@@ -23,8 +23,9 @@ struct GlaParams {
     HeadNormParams norm;                          // norm.x: raw read-outs, normed and gated in place
 };
 
-template <bool STEP>
-__global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) gla_scan_kernel(const GlaParams p) {
+// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread
+template <int NCOL>
+__global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT, NCOL == 0 ? 2 : (NCOL == 1 ? 5 : 4)) gla_scan_kernel(const GlaParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const ScanShape& sh = p.s;
@@ -41,8 +42,17 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) gla_scan_kernel(co
     float* rec = p.state + ((size_t)slot * p.H + h) * ((size_t)ks * sh.rt * dv);
     __shared__ float red[SCAN_THREADS / 32];
     const bool mine = part == 0 && col < ncol;    // this thread writes the column's read-outs
-    float s[SCAN_R];
-    scan_load_state(sh, rec, dv, j, part, s);
+    constexpr bool STEP = NCOL == 0;
+    constexpr int NC = STEP ? 1 : NCOL;           // columns of this thread: j, j + cstep
+    const int cstep = blockDim.x >> sh.lks;
+    float s[STEP ? SCAN_R : 1];
+    f32x2 s2[NC][STEP ? 1 : SCAN_R / 2];
+    if constexpr (STEP) {
+        scan_load_state(sh, rec, dv, j, part, s);
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) scan_load_state2(sh, rec, dv, j + c * cstep, part, s2[c]);
+    }
     float g_j = 0.f, w_j = 0.f, o_last = 0.f;     // STEP: gate and weight of the column, asked for early
     if (STEP && mine && sh.ncta == 1) {
         g_j = p.norm.gate[(size_t)t0 * p.norm.ldg + (size_t)h * dv + j];
@@ -82,6 +92,34 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) gla_scan_kernel(co
         float* orow = p.norm.x + (size_t)(t0 + c * sh.tc) * p.norm.ldx + (size_t)h * dv + j;
         for (int t = 0; t < n; ++t) {
             const float* kr = buf + (size_t)t * tokf + part * SCAN_ROW;
+            if constexpr (!STEP) {
+                f32x2 v2[NC], oa[NC], ob[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) { const float v = buf[(size_t)t * tokf + 3 * krow + col + c * cstep]; v2[c] = pack2(v, v); oa[c] = ob[c] = 0ull; }
+#pragma unroll
+                for (int r = 0; r < SCAN_R; r += 4) {
+                    const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(kr + r), q2 = *reinterpret_cast<const ulonglong2*>(kr + krow + r);
+                    const ulonglong2 a2 = *reinterpret_cast<const ulonglong2*>(kr + 2 * krow + r);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        s2[c][r / 2] = fmadd2(k2.x, v2[c], prod2(s2[c][r / 2], a2.x));
+                        s2[c][r / 2 + 1] = fmadd2(k2.y, v2[c], prod2(s2[c][r / 2 + 1], a2.y));
+                        fma2(oa[c], s2[c][r / 2], q2.x); fma2(ob[c], s2[c][r / 2 + 1], q2.y);
+                    }
+                }
+                float o[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float2 a2 = unpack2(oa[c]), b2 = unpack2(ob[c]);
+                    o[c] = (a2.x + a2.y) + (b2.x + b2.y);
+                }
+                for (int o_ = 1; o_ < ks; o_ <<= 1)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) o[c] += __shfl_xor_sync(0xffffffffu, o[c], o_);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (part == 0 && col + c * cstep < ncol) orow[(size_t)t * p.norm.ldx + c * cstep] = o[c] * p.q_scale;
+            } else {
             const float vj = buf[(size_t)t * tokf + 3 * krow + col];
             float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
 #pragma unroll
@@ -93,12 +131,18 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) gla_scan_kernel(co
                 o0 = fmaf(s[r], q4.x, o0); o1 = fmaf(s[r + 1], q4.y, o1); o2 = fmaf(s[r + 2], q4.z, o2); o3 = fmaf(s[r + 3], q4.w, o3);
             }
             const float o = scan_part_sum((o0 + o1) + (o2 + o3), ks) * p.q_scale;
-            if (STEP && sh.ncta == 1) o_last = o;
+            if (sh.ncta == 1) o_last = o;
             else if (mine) orow[(size_t)t * p.norm.ldx] = o;
+            }
         }
         if (!STEP) __syncthreads();
     }
-    scan_store_state(sh, rec, dv, j, part, s);
+    if constexpr (STEP) {
+        scan_store_state(sh, rec, dv, j, part, s);
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) scan_store_state2(sh, rec, dv, j + c * cstep, part, s2[c]);
+    }
     if constexpr (STEP) {
         if (sh.ncta == 1) {                        // the CTA holds the head: norm and gate from registers
             float ss = mine ? o_last * o_last : 0.f;

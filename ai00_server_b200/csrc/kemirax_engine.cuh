@@ -281,9 +281,10 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
         allow_smem(latent_attn_tc_kernel<4, 4>, smem_tc);
         allow_smem(latent_attn_tc_kernel<1, 16>, smem_tc);
         allow_smem(latent_attn_tc_kernel<2, 8>, smem_tc);
-    }
         allow_smem(latent_prompt_kernel, LATENT_PROMPT_SMEM);
-    CK(cudaFuncSetAttribute(gla_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
+    }
+    CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
+    CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
     CK(cudaFuncSetAttribute(lin_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_TC_SMEM));
@@ -424,7 +425,11 @@ void b200rwkv_engine::kx_short_conv(cudaStream_t s, Profiler* prof, const ShortC
         launch_k(short_conv_step_kernel, dim3(rows, cb), dim3(256), 0, cp, KC_OTHER, s, prof);
         return;
     }
-    launch_k(short_conv_kernel, dim3(rows, cb), dim3(256), 0, cp, KC_OTHER, s, prof);
+    auto whole4 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    if (cp.taps == 4 && cp.C % 4 == 0 && cp.ldx % 4 == 0 && cp.ldy % 4 == 0 && whole4(cp.x) && whole4(cp.y) && whole4(cp.w) && whole4(cp.tail))
+        launch_k(short_conv4_kernel, dim3(cdiv(rows, SC4_TOK), cdiv(cp.C, 4 * SC4_THREADS)), dim3(SC4_THREADS), 0, cp, KC_OTHER, s, prof);
+    else
+        launch_k(short_conv_kernel, dim3(rows, cb), dim3(256), 0, cp, KC_OTHER, s, prof);
     if (cp.taps > 1) launch_k(conv_commit_kernel, dim3(nslot_grid, cb), dim3(256), 0, cp, KC_OTHER, s, prof);
 }
 
@@ -432,10 +437,10 @@ void b200rwkv_engine::kx_short_conv(cudaStream_t s, Profiler* prof, const ShortC
 void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, int H_, int dk, int dv, const float* q, const float* k, const float* v,
                              const float* gate, int ld, float* out, int ldo, int rows, int nslot_grid, bool decode) {
     SeqModel& m = *kx;
-    const ScanShape sh = scan_shape(dk, dv, 3, decode);
+    const ScanShape sh = scan_shape(dk, dv, 3, decode, scan_wide(H_));
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
-    launch_k(decode ? gla_scan_kernel<true> : gla_scan_kernel<false>, dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), sh.smem_floats() * 4, gp, KC_WKV, s, prof);
+    launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), sh.smem_floats() * 4, gp, KC_WKV, s, prof);
     if (sh.ncta > 1) launch_k(head_norm_kernel, dim3(rows, cdiv(H_, 4)), dim3(128), 0, gp.norm, KC_LN, s, prof);
 }
 
@@ -503,6 +508,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 KvWriteParams kw{m.kv, D, l.cache, m.d_table, m.npages, m.page, l.dkv_norm, rk, dr, c.rot.dims, l.freq, l.mag, m.cfg.eps, mv, m.sm};
                 launch_k(kv_write_kernel, dim3(rows), dim3(128), 0, kw, KC_OTHER, s, prof);
             }
+            const bool whole = !m.exact && !decode && nsplit == 1 && D % 4 == 0 && rk <= 64 * LP_MAX_NT && latent_prompt_smem(D) <= LATENT_PROMPT_SMEM;      // latent_prompt.cuh
             LatentAttnParams ap{m.qa, l.cache, m.d_table, m.npages, m.page, m.part, H_, rk, dr, nsplit, c.scale, mv, m.sm};
             if (whole) {
                 LatentPromptParams lp{ap, m.olat, std::min(H_, 16), 0};
@@ -526,7 +532,6 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             {
                 LinParams p = lin(m.olat, H_ * rk, l.uv, m.vout, H_ * dv, dv, rk);
                 p.x_gstride = rk; p.w_gstride = (long long)dv * rk; p.y_gstride = dv;
-            const bool whole = !m.exact && !decode && nsplit == 1 && D % 4 == 0 && rk <= 64 * LP_MAX_NT && latent_prompt_smem(D) <= LATENT_PROMPT_SMEM;      // latent_prompt.cuh
                 kx_lin(s, prof, p, rows, H_);
             }
             LinParams po = lin(m.vout, H_ * dv, l.o, m.x, W, W, H_ * dv, LE_GATED_ADD);
@@ -668,7 +673,11 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     }
     int lg = 0;
     while ((1 << lg) < nsplit) ++lg;
-    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg;
+    int wide = 0;                          // the recurrences' shapes depend on the count of sequences: the smallest head count that runs wide
+    for (const KxLayer& l : kx->layers)
+        for (int h : {l.c.heads, l.c.mm_heads})
+            if (!decode && h > 0 && h < 256 && scan_wide(h) && (wide == 0 || h < wide)) wide = h;
+    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (wide << 22);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

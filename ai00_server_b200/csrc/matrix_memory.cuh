@@ -35,8 +35,9 @@ struct MatrixMemoryParams {
 
 constexpr int MM_MAX_N = SCAN_MAX_DK / SCAN_THREADS_PROMPT;      // normaliser entries per thread
 
-template <bool STEP>
-__global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) matrix_memory_kernel(const MatrixMemoryParams p) {
+// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread
+template <int NCOL>
+__global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT, NCOL == 0 ? 2 : (NCOL == 1 ? 4 : 3)) matrix_memory_kernel(const MatrixMemoryParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const ScanShape& sh = p.s;
@@ -59,8 +60,17 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) matrix_memory_kern
     float* gm = p.m + hs * dv + cb * sh.cols;
     __shared__ float red[SCAN_THREADS / 32];
     const bool mine = part == 0 && col < ncol;     // this thread writes the column's read-outs
-    float s[SCAN_R];
-    scan_load_state(sh, rec, dv, j, part, s);
+    constexpr bool STEP = NCOL == 0;
+    constexpr int NC = STEP ? 1 : NCOL;           // columns of this thread: j, j + cstep
+    const int cstep = blockDim.x >> sh.lks;
+    float s[STEP ? SCAN_R : 1];
+    f32x2 s2[NC][STEP ? 1 : SCAN_R / 2];
+    if constexpr (STEP) {
+        scan_load_state(sh, rec, dv, j, part, s);
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) scan_load_state2(sh, rec, dv, j + c * cstep, part, s2[c]);
+    }
     float g_j = 0.f, w_j = 0.f, o_last = 0.f;      // STEP: gate and weight of the column, asked for early
     if (STEP && mine && sh.ncta == 1) {
         g_j = p.norm.gate[(size_t)t0 * p.norm.ldg + (size_t)h * dv + j];
@@ -125,6 +135,34 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) matrix_memory_kern
             const float* row = buf + (size_t)t * tokf;
             const float* kr = row + part * SCAN_ROW;
             const float4 sc = sscal[t];
+            if constexpr (!STEP) {
+                f32x2 v2[NC], oa[NC], ob[NC];
+                const f32x2 keep2 = pack2(sc.x, sc.x);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) { const float v = row[2 * krow + col + c * cstep] * sc.y; v2[c] = pack2(v, v); oa[c] = ob[c] = 0ull; }
+#pragma unroll
+                for (int r = 0; r < SCAN_R; r += 4) {
+                    const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(kr + r), q2 = *reinterpret_cast<const ulonglong2*>(kr + krow + r);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        s2[c][r / 2] = fmadd2(k2.x, v2[c], prod2(s2[c][r / 2], keep2));
+                        s2[c][r / 2 + 1] = fmadd2(k2.y, v2[c], prod2(s2[c][r / 2 + 1], keep2));
+                        fma2(oa[c], s2[c][r / 2], q2.x); fma2(ob[c], s2[c][r / 2 + 1], q2.y);
+                    }
+                }
+                float o[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float2 a2 = unpack2(oa[c]), b2 = unpack2(ob[c]);
+                    o[c] = (a2.x + a2.y) + (b2.x + b2.y);
+                }
+                for (int o_ = 1; o_ < ks; o_ <<= 1)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) o[c] += __shfl_xor_sync(0xffffffffu, o[c], o_);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (part == 0 && col + c * cstep < ncol) orow[(size_t)t * p.norm.ldx + c * cstep] = o[c];
+            } else {
             const float vj = row[2 * krow + col] * sc.y;
             float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
 #pragma unroll
@@ -135,8 +173,9 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) matrix_memory_kern
                 o0 = fmaf(s[r], q4.x, o0); o1 = fmaf(s[r + 1], q4.y, o1); o2 = fmaf(s[r + 2], q4.z, o2); o3 = fmaf(s[r + 3], q4.w, o3);
             }
             const float o = scan_part_sum((o0 + o1) + (o2 + o3), ks);
-            if (STEP && sh.ncta == 1) o_last = o;
+            if (sh.ncta == 1) o_last = o;
             else if (mine) orow[(size_t)t * p.norm.ldx] = o;
+            }
             if (cb == 0) {                         // the normaliser and its product with the query
                 float nq = 0.f;
 #pragma unroll
@@ -177,7 +216,12 @@ __global__ void __launch_bounds__(SCAN_THREADS, STEP ? 2 : 1) matrix_memory_kern
             }
         }
     }
-    scan_store_state(sh, rec, dv, j, part, s);
+    if constexpr (STEP) {
+        scan_store_state(sh, rec, dv, j, part, s);
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) scan_store_state2(sh, rec, dv, j + c * cstep, part, s2[c]);
+    }
     if (cb == 0)
 #pragma unroll
         for (int e = 0; e < NE; ++e)

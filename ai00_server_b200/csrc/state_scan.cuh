@@ -3,7 +3,9 @@
 //
 // The columns of a state (one per value entry) are independent of one another.  A CTA owns `cols` of them; a column belongs to
 // `ks` neighbouring lanes, each keeping `rt` of its dk entries in registers for all tokens of the step, so a product with the key
-// or query is straight-line FMA on registers followed by log2(ks) exchanges, and no barrier separates the tokens.  Heads whose
+// or query is straight-line FMA on registers followed by log2(ks) exchanges, and no barrier separates the tokens.  Prompt steps of several sequences
+// give a thread TWO columns (`nc`): the loop over tokens is bound by the reads of staged keys and queries (24 of 16 bytes for 128 products a column and
+// token in the delta rule), which two columns share; products run as packed pairs of neighbouring entries.  Heads whose
 // columns do not fit one CTA are split over `ncta` of them (prompt steps always prefer many small CTAs).  Keys, queries and the
 // CTA's value entries of the next `tc` tokens arrive by cp.async while the current ones are worked on.
 //
@@ -17,6 +19,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "linear.cuh"
 
 namespace b200 {
@@ -32,6 +35,7 @@ constexpr int SCAN_SMEM_FIVE = 44 * 1024;          // ... with five CTAs on an S
 struct ScanShape {
     int ks, lks, rt;                               // lanes per column (a power of two and its logarithm), entries per lane (a multiple of 4)
     int threads, cols, ncta;                       // block size, columns per CTA, CTAs per head
+    int nc;                                        // columns per thread (prompt steps)
     int tc, nbuf;                                  // tokens per staged group, staging buffers
     int rows;                                      // staged vectors of the key dimension per token (key, query, ...)
     __host__ __device__ int tok_floats() const { return rows * ks * SCAN_ROW + ((cols + 3) & ~3); }
@@ -51,14 +55,16 @@ __host__ inline size_t scan_state_floats(int dk, int dv) {
     return (size_t)ks * rt * dv;
 }
 
-__host__ inline ScanShape scan_shape(int dk, int dv, int rows, bool decode) {
+// `wide`: the caller's launch fills the chip with two columns a thread
+__host__ inline ScanShape scan_shape(int dk, int dv, int rows, bool decode, bool wide = false) {
     ScanShape s;
     scan_parts(dk, s.ks, s.lks, s.rt);
     s.rows = rows;
     const int need = (dv * s.ks + 31) / 32 * 32;   // threads that hold a whole head
     s.threads = SCAN_THREADS_PROMPT;
     if (decode && need <= SCAN_THREADS) s.threads = need > SCAN_THREADS_PROMPT ? need : SCAN_THREADS_PROMPT;
-    s.cols = s.threads / s.ks;
+    s.nc = !decode && wide && dv > s.threads / s.ks ? 2 : 1;
+    s.cols = s.threads / s.ks * s.nc;
     s.ncta = (dv + s.cols - 1) / s.cols;
     s.nbuf = decode ? 1 : 2;
     s.tc = decode ? 1 : 16;
@@ -117,6 +123,27 @@ __device__ __forceinline__ void scan_store_state(const ScanShape& s, float* rec,
 #pragma unroll
     for (int r = 0; r < SCAN_R / 4; ++r)
         if (j < dv && 4 * r < s.rt) r4[r * plane] = make_float4(st[4 * r], st[4 * r + 1], st[4 * r + 2], st[4 * r + 3]);
+}
+
+// the same with pairs of neighbouring entries
+__device__ __forceinline__ void scan_load_state2(const ScanShape& s, const float* rec, int dv, int j, int part, f32x2 (&st)[SCAN_R / 2]) {
+    const float4* r4 = reinterpret_cast<const float4*>(rec) + (size_t)j * s.ks + part;
+    const size_t plane = (size_t)dv * s.ks;
+#pragma unroll
+    for (int r = 0; r < SCAN_R / 4; ++r) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < dv && 4 * r < s.rt) v = r4[r * plane];
+        st[2 * r] = pack2(v.x, v.y); st[2 * r + 1] = pack2(v.z, v.w);
+    }
+}
+__device__ __forceinline__ void scan_store_state2(const ScanShape& s, float* rec, int dv, int j, int part, const f32x2 (&st)[SCAN_R / 2]) {
+    float4* r4 = reinterpret_cast<float4*>(rec) + (size_t)j * s.ks + part;
+    const size_t plane = (size_t)dv * s.ks;
+#pragma unroll
+    for (int r = 0; r < SCAN_R / 4; ++r) {
+        const float2 a = unpack2(st[2 * r]), b = unpack2(st[2 * r + 1]);
+        if (j < dv && 4 * r < s.rt) r4[r * plane] = make_float4(a.x, a.y, b.x, b.y);
+    }
 }
 
 // x[t, h, :] <- f x / rms(f x) * w * act(gate) * mul   in place, f = fac[t, h] (1 without fac), act = sigmoid or silu
