@@ -1,4 +1,4 @@
-// Projection GEMM of long steps (more than 128 tokens):  Y[T, N] = X[T, K] (f16) * W[N, K]^T (f16), f32 accumulate, on pairs of SMs.
+// Projection GEMM of steps of more than 64 tokens (one GPU, f16 weights):  Y[T, N] = X[T, K] (f16) * W[N, K]^T (f16), f32 accumulate, on pairs of SMs.
 //
 // Same weight blocks, segments and epilogues as gemm.cuh / gemm_wide.cuh; replaces the projection dispatches of `Runtime::infer` (reference
 // crates/ai00-core/src/run.rs:1143) in steps that hold long prompts.
@@ -14,6 +14,7 @@
 //   * eight epilogue warps drain one accumulator while the next unit's MMAs run; f16 operands are transposed warp by warp.
 // Measured (3B widths, 1792 tokens a launch against seven launches of 256 tokens on single SMs, ncu): R/K/V/G 253 -> 83 us (1.13 PFLOP/s), output 132 -> 27,
 // channel mix 307 -> 96 and 171 -> 61, first low-rank stage 225 -> 23; 32 prompts of 512 tokens 53.5 -> 21.5 ms.
+// 100 tokens of 7B widths (weights from HBM): 42 -> 34, 18 -> 18, 45 -> 37 and 32 -> 29 us.
 #pragma once
 #include <cuda.h>
 #include <cudaTypedefs.h>

@@ -1,4 +1,5 @@
-// Projection GEMM of prompt steps (17 .. 128 tokens; longer steps: gemm_pair.cuh, which leaves the one-block tiles to the SHORT form here):  Y[T, N] = X[T, K] (f16) * W[N, K]^T (f16), f32 accumulate.
+// Projection GEMM of prompt steps (17 .. 128 tokens; from 65 on gemm_pair.cuh where that applies, which leaves launches of a few tiles of a long k and the one-block
+// tiles of every length to the forms here):  Y[T, N] = X[T, K] (f16) * W[N, K]^T (f16), f32 accumulate.
 //
 // Same operands, segments, epilogues and stream-K fix-up as gemm.cuh (its decode kernel reads the same weight blocks); replaces
 // the projection dispatches of `Runtime::infer` (reference crates/ai00-core/src/run.rs:1143) in steps that hold a prompt.

