@@ -397,7 +397,7 @@ struct SeqModel {
     float* last_tok = nullptr;                    // [S] last token of every sequence (families with pair embeddings)
     // bf16 operand rows of one projection launch (linear_umma.cuh) per stream, sized by a walk over the largest step; tile counters
     __nv_bfloat16 *lin_x16 = nullptr, *lin_x16_side = nullptr; size_t lin_x16_bytes = 0;
-    __nv_bfloat16 *h16 = nullptr, *ys16 = nullptr;      // sublayer input and gated units as bf16 operands (prompt steps of some families)
+    __nv_bfloat16 *h16 = nullptr, *hs16 = nullptr, *ys16 = nullptr;      // sublayer input and gated units as bf16 operands (prompt steps of some families)
     unsigned *lin_counters = nullptr, *lin_counters_side = nullptr;
     int max_top = 1;                             // experts a token may choose (rows of the routed launches)
     bool side_lin = false; float* lin_ws_side = nullptr;      // projections also run on the side stream: split-k sums of their own

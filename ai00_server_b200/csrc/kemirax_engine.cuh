@@ -259,6 +259,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     m.sel = (int*)dalloc(T_ * z.max_top * 4); m.row_of = (int*)dalloc(T_ * z.max_top * 4); m.list = (int*)dalloc(T_ * z.max_top * 4);
     m.cnt = (int*)dalloc((size_t)z.max_E * 4); m.off = (int*)dalloc((size_t)z.max_E * 4);
     if (!m.exact && W % 8 == 0) m.h16 = (__nv_bfloat16*)dalloc(T_ * W * 2, true);
+    if (!m.exact && W % 8 == 0 && m.cfg.family == KX_FAMILY_KEMIRAX) m.hs16 = (__nv_bfloat16*)dalloc(T_ * W * 2, true);
     if (!m.exact && z.n_ys % 8 == 0 && z.n_ys) m.ys16 = (__nv_bfloat16*)dalloc(T_ * z.n_ys * 2, true);
     d_hidden = fa(T_ * W);
     d_logits = fa((size_t)maxR * V);
@@ -418,6 +419,12 @@ void b200rwkv_engine::kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int ro
     }
 }
 
+// the router's choices -> row lists of the experts
+void b200rwkv_engine::kx_moe_group(cudaStream_t s, Profiler* prof, const MoeGroupParams& gp, int rows) {
+    if (rows > 128 && gp.E <= MOE_GROUP_MAX_E) launch_k(moe_group_wide_kernel, dim3(1), dim3(MOE_GROUP_THREADS), moe_group_wide_smem(std::max(gp.E, 1)), gp, KC_OTHER, s, prof);
+    else launch_k(moe_group_kernel, dim3(1), dim3(256), ((size_t)std::max(gp.E, 1) * 2 + (size_t)rows * gp.top) * 4, gp, KC_OTHER, s, prof);
+}
+
 // the short convolutions of a layer: one launch in steps of one token per sequence, otherwise the convolution and then the new tails
 void b200rwkv_engine::kx_short_conv(cudaStream_t s, Profiler* prof, const ShortConvParams& cp, int rows, int nslot_grid, bool decode) {
     const int cb = cdiv(cp.C, 256);
@@ -486,13 +493,20 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             continue;
         }
         NormShiftParams ns{m.x, m.h, m.hs, l.mu, l.shift_state, l.gain, m.cfg.eps, W, mv};
+        // prompt steps: the norm and the gated units leave their projections' bf16 operands (the f32 h stays for the router, the experts and the sum)
+        const bool x16 = rows > 16 && m.h16 && m.hs16;
+        if (x16) { ns.h16 = m.h16; ns.hs16 = m.hs16; }
+        auto from = [&](LinParams p, const __nv_bfloat16* b) {
+            if (x16) p.X16 = b;
+            return p;
+        };
         launch_k(norm_shift_kernel, dim3(rows), dim3(NORM_THREADS), 0, ns, KC_LN, s, prof);
         launch_k(shift_commit_kernel, dim3(nslot_grid), dim3(NORM_THREADS), 0, ns, KC_LN, s, prof);
         const int GW = c.has_mlp ? 2 * W : W;
-        kx_lin(s, prof, lin(m.h, W, l.rg, m.G, GW, GW, W, LE_SIGMOID, l.rg_b), rows, 1);
+        kx_lin(s, prof, from(lin(m.h, W, l.rg, m.G, GW, GW, W, LE_SIGMOID, l.rg_b), m.h16), rows, 1);
         if (c.mixer == KX_LATENT) {
             const int H_ = c.heads, dn = c.dim, dr = c.rot_dim, dv = c.vdim, rk = c.kv_rank, D = rk + dr, QW = H_ * (dn + dr);
-            kx_lin(s, prof, lin(m.hs, W, l.dq, m.cq, c.q_rank, c.q_rank, W), rows, 1);
+            kx_lin(s, prof, from(lin(m.hs, W, l.dq, m.cq, c.q_rank, c.q_rank, W), m.hs16), rows, 1);
             RmsRowsParams rr{m.cq, c.q_rank, m.cq, c.q_rank, l.dq_norm, c.q_rank, 1, m.cfg.eps, cntT};
             launch_k(rms_rows_kernel, dim3(rows, 1), dim3(128), 0, rr, KC_LN, s, prof);
             kx_lin(s, prof, lin(m.cq, c.q_rank, l.uq, m.q, QW, QW, c.q_rank), rows, 1);
@@ -504,7 +518,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 kx_lin(s, prof, p, rows, H_);
             }
             if (c.kv_from < 0) {
-                kx_lin(s, prof, lin(m.hs, W, l.dkv, m.kv, D, D, W), rows, 1);
+                kx_lin(s, prof, from(lin(m.hs, W, l.dkv, m.kv, D, D, W), m.hs16), rows, 1);
                 KvWriteParams kw{m.kv, D, l.cache, m.d_table, m.npages, m.page, l.dkv_norm, rk, dr, c.rot.dims, l.freq, l.mag, m.cfg.eps, mv, m.sm};
                 launch_k(kv_write_kernel, dim3(rows), dim3(128), 0, kw, KC_OTHER, s, prof);
             }
@@ -539,7 +553,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             kx_lin(s, prof, po, rows, 1);
         } else {
             const int H_ = c.heads, dk = c.dim, dv = c.vdim;
-            kx_lin(s, prof, lin(m.hs, W, l.proj, m.pr, l.proj_n, l.proj_n, W), rows, 1);
+            kx_lin(s, prof, from(lin(m.hs, W, l.proj, m.pr, l.proj_n, l.proj_n, W), m.hs16), rows, 1);
             kx_lin(s, prof, lin(m.pr + 2 * H_ * dk + 2 * H_ * dv, l.proj_n, l.a2, m.z, H_ * dk, H_ * dk, l.a_rank, LE_STORE, l.a2_b), rows, 1);
             kx_gla(s, prof, l, H_, dk, dv, m.pr, m.pr + H_ * dk, m.pr + 2 * H_ * dk, m.pr + 2 * H_ * dk + H_ * dv, l.proj_n, m.vout, H_ * dv, rows, nslot_grid,
                    decode);
@@ -552,7 +566,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             MoeRouteParams rp{m.h, W, l.router, W, l.corr, NE, c.top, m.sel, m.wgt, mv};
             launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, NE), rp, KC_OTHER, s, prof);
             MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
-            launch_k(moe_group_kernel, dim3(1), dim3(rows > 128 ? MOE_GROUP_THREADS : 256), ((size_t)std::max(E, 1) * 2 + (size_t)rows * c.top) * 4, gp, KC_OTHER, s, prof);
+            kx_moe_group(s, prof, gp, rows);
             if (E > 0) {
                 LinParams p1 = lin(m.h, W, l.gu, m.yc, ff, 2 * ff, W, LE_GLU_CLAMP);
                 p1.w_gstride = (long long)2 * ff * W; p1.cnt = m.cnt; p1.cnt_gstride = 1; p1.off = m.off; p1.xlist = m.list; p1.limit = c.limit;
@@ -562,10 +576,11 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 kx_lin(s, prof, p2, rows, E);
             }
             if (c.has_shared) {
-                LinParams p1 = lin(m.h, W, l.sh_gu, m.ys, c.sff, 2 * c.sff, W, LE_GLU_CLAMP);
+                LinParams p1 = from(lin(m.h, W, l.sh_gu, m.ys, c.sff, 2 * c.sff, W, LE_GLU_CLAMP), m.h16), p2 = lin(m.ys, c.sff, l.sh_down, m.ds, W, W, c.sff);
                 p1.limit = c.slimit;
+                if (x16 && m.ys16 && c.sff % 8 == 0) { p1.Y16 = m.ys16; p2.X16 = m.ys16; }
                 kx_lin(s, prof, p1, rows, 1);
-                kx_lin(s, prof, lin(m.ys, c.sff, l.sh_down, m.ds, W, W, c.sff), rows, 1);
+                kx_lin(s, prof, p2, rows, 1);
             }
             MoeCombineParams cp{m.x, m.h, m.G + W, GW, m.dn, m.row_of, m.wgt, c.top, c.has_shared ? m.ds : nullptr, l.sg, W, mv};
             launch_k(moe_combine_kernel, dim3(rows), dim3(256), 0, cp, KC_OTHER, s, prof);

@@ -238,7 +238,7 @@ void b200rwkv_engine::ps_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 MoeRouteParams rp{m.h, W, l.router, W, l.corr, E, c.top, m.sel, m.wgt, mv, MOE_TOP_LOGITS};
                 launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, E), rp, KC_OTHER, s, prof);
                 MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
-                launch_k(moe_group_kernel, dim3(1), dim3(rows > 128 ? MOE_GROUP_THREADS : 256), ((size_t)E * 2 + (size_t)rows * c.top) * 4, gp, KC_OTHER, s, prof);
+                kx_moe_group(s, prof, gp, rows);
                 LinParams p1 = lin(m.h, W, l.gu, m.yc, ff, 2 * ff, W, LE_GLU_SILU);
                 p1.w_gstride = (long long)2 * ff * W; p1.cnt = m.cnt; p1.cnt_gstride = 1; p1.off = m.off; p1.xlist = m.list;
                 kx_lin(s, prof, p1, rows, E);

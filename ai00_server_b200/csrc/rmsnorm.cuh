@@ -92,12 +92,15 @@ __global__ void __launch_bounds__(128) last_token_commit_kernel(const EmbedRowsP
 struct NormShiftParams {
     const float* x;          // [T, W] residual
     float* h;                // [T, W] normed row (feed-forward, gates)
-    float* hs;               // [T, W] token-shifted normed row (mixer); nullptr: no shift
+    float* hs;               // [T, W] token-shifted normed row (mixer); nullptr: no shift, or bf16 only
     const float* mu;         // [W]
     float* shift_state;      // [S, W] of this layer
     float gain, eps;
     int W;
     MetaView meta;
+    // prompt steps: the rows as the projections' bf16 operands (rounded once, here instead of by a packing launch in front of each of them)
+    __nv_bfloat16* h16 = nullptr;
+    __nv_bfloat16* hs16 = nullptr;
 };
 
 __global__ void __launch_bounds__(NORM_THREADS) norm_shift_kernel(const NormShiftParams p) {
@@ -123,9 +126,12 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_shift_kernel(const NormShif
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
         const float hv = xr[c] * r;
         p.h[(size_t)t * W + c] = hv;
-        if (p.hs) {
+        if (p.h16) p.h16[(size_t)t * W + c] = __float2bfloat16(hv);
+        if (p.hs || p.hs16) {
             const float hp = prev >= 0 ? p.x[(size_t)prev * W + c] * rp : p.shift_state[(size_t)slot * W + c];
-            p.hs[(size_t)t * W + c] = hv + (hp - hv) * p.mu[c];
+            const float v = hv + (hp - hv) * p.mu[c];
+            if (p.hs16) p.hs16[(size_t)t * W + c] = __float2bfloat16(v);
+            else p.hs[(size_t)t * W + c] = v;
         }
     }
 }
