@@ -1,0 +1,101 @@
+"""Prompt steps of many sequences: the kernels that take over once a step fills the chip (64 rows to a staged key tile, two state columns a thread,
+convolutions in registers), at the edges of their tiles, against the families' restatements."""
+import json
+
+import numpy as np
+import pytest
+
+from ai00_server_b200 import capi, runtime, synth
+from oracle import degavik_numpy, fufipel_numpy, kemirax_numpy, panupel_numpy
+from oracle import rwkv_numpy as O
+
+pytestmark = pytest.mark.gpu
+
+# f32 engine against float64: the bound the families' own tests hold (2e-4 of the logits' spread in any row); bf16 operands (2^-9 each): a few percent in the
+# median row, a wrong row is off by its own size
+TIGHT, BF16_TOL, ROW_TOL = 2e-4, 5e-2, 0.5
+N_SEQ = 48
+
+
+def _errs(got, want):
+    return np.sqrt(((got - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean())
+
+
+def _check(make, module, layers, precision, kv=16, **kw):
+    """48 sequences of 1 to 97 tokens in one call (steps of several hundred tokens); four of them against the restatement, row by row, then five tokens more
+    of those four (the states and caches the step left)."""
+    cfg, st, w = make(layers, seed=4, **kw)
+    rng = np.random.default_rng(7)
+    lens = [97, 1, 64, 33] + rng.integers(1, 90, N_SEQ - 4).tolist()
+    toks = [rng.integers(1, 90, n + 5).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=N_SEQ, token_chunk_size=512, precision=precision, config=cfg, kv_tokens=sum(lens) + 8 * N_SEQ, kv_page=kv)
+    try:
+        for s in range(N_SEQ):
+            m.state.reset(s)
+        opt = [capi.OPTION_FULL] * 4 + [capi.OPTION_LAST] * (N_SEQ - 4)
+        got = m.infer_raw(list(range(N_SEQ)), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw([0, 1, 2, 3], [5] * 4, sum((toks[s][lens[s]:] for s in range(4)), []), [capi.OPTION_FULL] * 4)
+        for s in range(4):
+            want = module.run(json.loads(cfg), w, toks[s])
+            err = _errs(np.concatenate([got[s], more[s]]), want)
+            if precision == 1:
+                assert err.max() <= TIGHT, (s, int(err.argmax()), float(err.max()))
+            else:
+                assert np.median(err) <= BF16_TOL and err.max() <= ROW_TOL, (s, float(np.median(err)), int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
+P, F, K, D = synth.panupel_layer, synth.fufipel_layer, synth.kemirax_layer, synth.degavik_layer
+
+
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(4, 4, 24, 24), (4, 1, 40, 72), (6, 2, 128, 128), (3, 1, 16, 112)])
+def test_attention_over_the_whole_context(heads, kv_heads, dim, vdim):
+    """64 rows are 64, 16, 21 and 21 tokens of one key head; sizes below, at and between the 64-entry halves of a value row."""
+    _check(synth.make_panupel, panupel_numpy, [P("parallel", heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, mm_heads=2, mm_dim=72)], 1, width=96, loop=None)
+
+
+@pytest.mark.parametrize("window, keep", [(8, 2), (33, 0), (40, 5)])
+def test_attention_in_a_window(window, keep):
+    """Kept first tokens in front of windows that end inside, at and behind a 32-key tile, a bias per distance, a gate per entry; a chunked layer beside it."""
+    _check(synth.make_fufipel, fufipel_numpy, [F("attention", heads=4, kv_heads=2, dim=20, window=window, keep_first=keep), F("parallel", heads=2, dim=24, chunk=11)], 1, width=80)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dim, vdim, conv", [(72, 72, 4), (128, 40, 4), (24, 24, 4), (40, 72, 3)])
+def test_delta_rule(dim, vdim, conv, precision):
+    """One and two columns a thread (vdim above and below the columns a CTA holds), convolutions of four taps in registers and of three as before."""
+    _check(synth.make_panupel, panupel_numpy, [P("delta", heads=2, dim=dim, vdim=vdim, conv=conv)], precision, width=96, loop=None)
+
+
+def test_delta_rule_with_a_decay_per_channel():
+    _check(synth.make_degavik, degavik_numpy, [D("channel_delta", heads=2, dim=72, vdim=72, conv=4)], 1, width=96)
+
+
+@pytest.mark.parametrize("dim, vdim", [(72, 72), (16, 24)])
+def test_gated_linear_attention(dim, vdim):
+    _check(synth.make_kemirax, kemirax_numpy, [K("gla", heads=2, dim=dim, vdim=vdim, mlp=False)], 1, width=96)
+
+
+@pytest.mark.parametrize("heads, kv_rank, rot_dim", [(4, 24, 8), (16, 40, 16), (5, 72, 4), (20, 64, 8)])
+def test_latent_attention(heads, kv_rank, rot_dim):
+    """64 rows of 4, 16, 5 and 20 (two CTAs) heads; latent rows with and without pad columns; channels that do not fill eight warps."""
+    _check(synth.make_kemirax, kemirax_numpy, [K("latent_attention", heads=heads, kv_rank=kv_rank, rot_dim=rot_dim, experts=6, top=3)], 0, width=96)
+
+
+@pytest.mark.parametrize("n", [17, 100, 300])
+@pytest.mark.parametrize("ranks", [(64, 128), (32, 32), (64, 64)])
+def test_low_rank_second_stages(ranks, n):
+    """Both kernels of lora2.cuh at every rank they are built for, one tile of tokens and several."""
+    st = synth.make_st(synth.Shape(6, 2, 256, 896, V=512, Dm=ranks[0], Dd=ranks[1]), 3)
+    orc = O.Oracle(O.parse_st(st), "f16")
+    toks = np.random.default_rng(n).integers(1, 500, n).tolist()
+    m = runtime.Model(st, max_batch=1, token_chunk_size=128)
+    try:
+        m.state.reset(0)
+        got = m.infer_raw([0], [n], toks, [capi.OPTION_LAST])[0]
+        want, state = orc.run(toks, orc.state_init())
+        assert np.abs(got - want).max() <= 1e-3 * np.abs(want).max()
+        assert np.abs(m.state.back(0) - state).max() <= 1e-3 * np.abs(state).max()
+    finally:
+        m.close()
