@@ -540,6 +540,8 @@ struct b200rwkv_engine {
     MetaView meta_view(int* base, int T) const { return MetaView{base, meta_rows(T), S}; }
     SeqMeta seq_meta(int* base, int T) const { return SeqMeta{base + MetaView::ints(meta_rows(T), S), meta_rows(T)}; }
     size_t step_meta_ints(int T) const { return MetaView::ints(meta_rows(T), S) + (kx ? SeqMeta::ints(meta_rows(T)) : 0); }
+    // slots of a benchmarked or profiled decode step, a logits row each (as many as a portion of a prompt step holds, never more than maxR rows)
+    int bench_slots() const { return kx ? kx->portion : std::min(maxT, 256); }
     int step_rows = 0;                 // config.json families: rows of the step being enqueued
     int step_seqs = 0;                 // sequences of the step
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
@@ -2808,7 +2810,7 @@ static int32_t rank_bench_decode(b200rwkv_engine* e, int32_t nslot, const int32_
                               int32_t steps, int32_t flush_l2, float* ms_out, int64_t* launches_out, float* step_ms_out) {
     API_BEGIN(e)
     REQUIRE(e && slot && tokens && ms_out, B200RWKV_ERR_INVALID, "null argument");
-    REQUIRE(nslot >= 1 && nslot <= e->S && nslot <= e->maxT && steps >= 1 && warmup >= 0, B200RWKV_ERR_INVALID, "bad argument");
+    REQUIRE(nslot >= 1 && nslot <= e->S && nslot <= e->bench_slots() && steps >= 1 && warmup >= 0, B200RWKV_ERR_INVALID, "bad argument");
     for (int i = 0; i < nslot; ++i) REQUIRE(slot[i] >= 0 && slot[i] < e->S, B200RWKV_ERR_STATE, "slot out of range");
     std::lock_guard<std::mutex> lk(e->mu);
     CK(cudaSetDevice(e->dev));
@@ -2862,7 +2864,7 @@ static int32_t rank_profile_step(b200rwkv_engine* e, int32_t nslot, const int32_
                               int32_t launches[4], int64_t* gemm_weight_bytes) {
     API_BEGIN(e)
     REQUIRE(e && slot && tokens && ms && launches, B200RWKV_ERR_INVALID, "null argument");
-    REQUIRE(nslot >= 1 && nslot <= e->S && nslot <= e->maxT, B200RWKV_ERR_INVALID, "bad argument");
+    REQUIRE(nslot >= 1 && nslot <= e->S && nslot <= e->bench_slots(), B200RWKV_ERR_INVALID, "bad argument");
     std::lock_guard<std::mutex> lk(e->mu);
     CK(cudaSetDevice(e->dev));
     std::vector<int> all, splits;
@@ -2898,7 +2900,7 @@ static int32_t rank_profile_insitu(b200rwkv_engine* e, int32_t nslot, const int3
     API_BEGIN(e)
     REQUIRE(e && slot && tokens && n_out && types && start_us && end_us && bytes && step_us && reps >= 1 && cap >= 1, B200RWKV_ERR_INVALID,
             "bad argument");
-    REQUIRE(nslot >= 1 && nslot <= e->S && nslot <= e->maxT, B200RWKV_ERR_INVALID, "bad argument");
+    REQUIRE(nslot >= 1 && nslot <= e->S && nslot <= e->bench_slots(), B200RWKV_ERR_INVALID, "bad argument");
     std::lock_guard<std::mutex> lk(e->mu);
     CK(cudaSetDevice(e->dev));
     if (!e->d_step_trace) e->d_step_trace = (unsigned long long*)e->dalloc((size_t)b200rwkv_engine::STEP_TRACE_MAX * b200rwkv_engine::STEP_TRACE_ROW * 8, true);
