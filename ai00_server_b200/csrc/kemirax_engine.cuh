@@ -245,10 +245,9 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     auto fa = [&](size_t n) { return (float*)dalloc(n * 4); };
     m.x = fa(T_ * W * z.n_streams); m.h = fa(T_ * W); m.hs = fa(T_ * W); m.G = fa(T_ * 2 * W); m.hn = fa(T_ * W);
     m.cq = fa(T_ * z.n_cq); m.q = fa(T_ * z.n_q); m.qa = fa(T_ * z.n_qa); m.kv = fa(T_ * z.n_kv);
-    // partial attention results: the context is split over at most max_split CTAs and only while the launch has fewer CTAs than two waves, 4 tokens
-    // to a CTA (kx_fill_step): long steps keep one part a token
-    m.part = fa(std::max(std::min(T_, (size_t)16 * num_sms) * z.n_part, T_ * (z.n_part / std::max(1, m.max_split))));
-
+    // partial attention results: the context is split only while the launch has fewer CTAs than two waves, four tokens to a CTA (kx_fill_step), so that tokens
+    // times parts stay below 16 a SM; long steps keep one part a token
+    m.part = fa(std::max(T_, (size_t)16 * num_sms) * std::max<size_t>(1, z.n_part / std::max(1, m.max_split)));
     m.olat = fa(T_ * z.n_olat); m.vout = fa(T_ * z.n_vout); m.pr = fa(T_ * z.n_pr); m.z = fa(T_ * z.n_z);
     m.rl = fa(T_ * z.n_rl); m.wgt = fa(T_ * z.max_top); m.yc = fa(T_ * z.max_top * z.n_yc); m.dn = fa(T_ * z.max_top * W);
     m.ys = fa(T_ * z.n_ys); m.ds = fa(T_ * W);
