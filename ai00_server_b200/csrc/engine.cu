@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include "kx_rows.cuh"
 #include "gemm.cuh"
 #include "gemm_wide.cuh"
 #include "gemm_pair.cuh"

@@ -204,9 +204,9 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     // Portions of up to 512 tokens when the caller's token_chunk_size asks for them, 128 otherwise.  A serving-precision step holds sixteen
     // chunks, 2048 tokens at most: prompts then stream the weights once per 2048 tokens, fill the experts' row tiles and the two-SM projections.
     // f32-exact steps hold one portion (plain FMA tiles, which a longer step does not fill better)
-    m.portion = chunk > 256 ? 512 : (chunk > 128 ? 256 : 128);
-    maxT = m.exact ? m.portion : std::max(m.portion, rup((int)std::min<long long>(16ll * chunk, 2048), 128));
-    maxR = std::min(maxT, 512);
+    m.portion = kx_portion(chunk);
+    maxT = kx_max_rows(chunk, m.exact);
+    maxR = std::min(maxT, KX_MAX_OUT_ROWS);
     dbg_T = m.portion;
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&sm_stream, cudaStreamNonBlocking));
@@ -299,7 +299,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
         m.lin_counters = (unsigned*)dalloc(LU_MAX_COUNTERS * 4, true);
         if (m.side_lin) m.lin_counters_side = (unsigned*)dalloc(LU_MAX_COUNTERS * 4, true);
         planning = true;
-        for (int r = maxT; r > 16; r = r > 512 ? r - 256 : r / 2) kx_enqueue_step(stream, r, std::min(r, maxR), false, 1, nullptr);
+        for (int r = maxT; r > 16; r = kx_bucket_below(r)) kx_enqueue_step(stream, r, std::min(r, maxR), false, 1, nullptr);
         planning = false;
         if (m.lin_x16_bytes) {
             m.lin_x16 = (__nv_bfloat16*)dalloc(m.lin_x16_bytes, false);
@@ -453,6 +453,7 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
 void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool decode, int nsplit, Profiler* prof) {
     launches_last_step = 0;
     SeqModel& m = *kx;
+    REQUIRE(rows <= maxT && rrows <= maxR, B200RWKV_ERR_INVALID, "internal: a step's launches have more rows than its buffers");
     step_rows = rows;
     m.sm = seq_meta(d_meta, rows);
     const int W = m.W;
@@ -597,13 +598,6 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
         ph.cnt = cntR;
         kx_lin(s, prof, ph, rrows, 1);
     }
-}
-
-// rows of a step's launches: powers of two up to 512 (one graph each), whole tiles of 256 beyond
-static inline int kx_bucket(int n) {
-    for (int b = 8; b <= 512; b *= 2)
-        if (n <= b) return b;
-    return rup(n, 256);
 }
 
 // positions, attention chunks and page-table updates of one step; hands out pages

@@ -1,0 +1,29 @@
+// Rows of a step of the config.json families: what buffers hold and what launches ask for.  Plain arithmetic, the same for every family.
+#pragma once
+#include <algorithm>
+
+namespace b200 {
+
+constexpr int KX_MAX_STEP = 2048;              // tokens of a step
+constexpr int KX_MAX_OUT_ROWS = 512;           // logits rows of a step
+
+// rows of a step's launches: powers of two up to 512 (one graph each), whole tiles of 256 beyond
+inline int kx_bucket(int n) {
+    for (int b = 8; b <= 512; b *= 2)
+        if (n <= b) return b;
+    return (n + 255) / 256 * 256;
+}
+// the next smaller bucket
+inline int kx_bucket_below(int b) { return b > 512 ? b - 256 : b / 2; }
+
+// tokens of a portion
+inline int kx_portion(int chunk) { return chunk > 256 ? 512 : (chunk > 128 ? 256 : 128); }
+
+// rows every buffer of a step holds: sixteen chunks and a portion at least, and a bucket itself, since launches cover the bucket of a step's tokens (operands are
+// packed and tensor maps encoded with that many rows a group).  f32-exact steps hold one portion
+inline int kx_max_rows(int chunk, bool exact) {
+    const int portion = kx_portion(chunk);
+    return exact ? portion : kx_bucket(std::max(portion, (int)std::min<long long>(16ll * chunk, KX_MAX_STEP)));
+}
+
+}  // namespace b200

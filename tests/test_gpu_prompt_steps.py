@@ -110,10 +110,10 @@ BF16_TOL = 5e-2
 ROW_TOL = 0.5
 
 
-def _check_family(make, layers, module, n, **kw):
+def _check_family(make, layers, module, n, chunk=512, **kw):
     cfg, st, w = make(layers, seed=4, **kw)
     toks = np.random.default_rng(n).integers(1, 90, n).tolist()
-    m = runtime.Model(st, max_batch=1, token_chunk_size=512, config=cfg, kv_tokens=n + 64, kv_page=16)
+    m = runtime.Model(st, max_batch=1, token_chunk_size=chunk, config=cfg, kv_tokens=n + 64, kv_page=16)
     try:
         m.state.reset(0)
         got = m.infer_raw([0], [n], toks, [capi.OPTION_FULL])[0]
@@ -165,6 +165,14 @@ def test_routed_projections_of_a_step_of_n_rows(n, experts, top):
     """Row lists of experts: groups of very unequal size, empty ones among them."""
     layer = synth.kemirax_layer("gla", heads=2, dim=16, vdim=24, experts=experts, identity=1, top=top, ff=88, shared_ff=40)
     _check_family(synth.make_kemirax, [layer], kemirax_numpy, n, width=72)
+
+
+@pytest.mark.parametrize("chunk", [20, 33, 40, 100])
+def test_full_steps_of_chunks_between_the_row_counts_of_launches(chunk):
+    """Sixteen chunks that are no row count of a launch (powers of two, multiples of 256): a full step and a little more, grouped projections (a group a head, a group an
+    expert) and their operands' buffers at their last rows."""
+    layer = synth.kemirax_layer("latent_attention", heads=16, kv_rank=40, rot_dim=16, experts=6, top=3)
+    _check_family(synth.make_kemirax, [layer], kemirax_numpy, 16 * chunk + 21, chunk=chunk, width=96)
 
 
 @pytest.mark.parametrize("n", [1, 9, 16])
