@@ -301,6 +301,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pair_kernel(const __grid
             const bool row_ok = n < sg.N;
             const int out_mode = sg.out_mode, ldo = sg.ldo;
             const float bias = (row_ok && live > 0 && sg.bias) ? sg.bias[n] : 0.f;
+            const bool lerp = out_mode == OUT_LERP_A16;
+            const float mu = (lerp && row_ok && live > 0) ? sg.aux2[n] : 0.f;
             mbar_wait_cluster(tfull_bar + acc * 8, use & 1u, 35);
             tc_fence_after();
             const uint32_t tm = tmem_base + lane_base + acc * NTOK + half * (NTOK / 2);
@@ -325,6 +327,15 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_pair_kernel(const __grid
                             }
                         }
                         continue;
+                    }
+                    if (ACT_C == ACT_NONE && lerp) {        // low ranks beyond one k block (one-block ones: lora2.cuh, gemm_wide.cuh)
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const bool ok = row_ok && c + j < live;
+                            const size_t a_ = (size_t)(m0 + c + j) * sg.ld_aux + n;
+                            const float xx = ok ? sg.aux0[a_] : 0.f, sx = ok ? sg.aux1[a_] : 0.f;
+                            v[j] = xx + sx * (mu + v[j]);
+                        }
                     }
                     // 16-byte chunks of eight rows: the rows of a chunk are lanes of this warp
 #pragma unroll

@@ -87,6 +87,17 @@ def test_latent_attention(heads, kv_rank, rot_dim):
 @pytest.mark.parametrize("ranks", [(64, 128), (32, 32), (64, 64)])
 def test_low_rank_second_stages(ranks, n):
     """Both kernels of lora2.cuh at every rank they are built for, one tile of tokens and several."""
+    _check_low_ranks(ranks, n)
+
+
+@pytest.mark.parametrize("n", [17, 70, 128, 300])
+@pytest.mark.parametrize("ranks", [(96, 160), (160, 64), (264, 128)])
+def test_low_ranks_of_other_sizes(ranks, n):
+    """Ranks lora2.cuh is not built for, of one k block (128) and of several: the projections' own epilogue mixes the rows, in every form that can meet it."""
+    _check_low_ranks(ranks, n)
+
+
+def _check_low_ranks(ranks, n):
     st = synth.make_st(synth.Shape(6, 2, 256, 896, V=512, Dm=ranks[0], Dd=ranks[1]), 3)
     orc = O.Oracle(O.parse_st(st), "f16")
     toks = np.random.default_rng(n).integers(1, 500, n).tolist()
