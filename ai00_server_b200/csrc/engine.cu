@@ -1824,6 +1824,7 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
     if (world > 1) launch_k(tp_barrier_kernel, dim3(1), dim3(32), 0, tpbar, KC_OTHER, s, prof);
 }
 
+constexpr int GRAPH_MT = 16;           // steps of up to 256 tokens are captured
 // 16-token tiles of a step's launches: powers of two up to 128 tokens, whole tiles of 128 beyond
 static inline int mt_bucket(int rows) { return rows <= 16 ? 1 : (rows <= 32 ? 2 : (rows <= 64 ? 4 : cdiv(rows, 128) * 8)); }
 
@@ -1840,8 +1841,10 @@ void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MT, int MTR) {
 }
 
 void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
-    // steps of more than 128 tokens go out launch by launch: their kernels outlast their launches, and a graph per length would be built for each
-    if (!use_graph || MT > 8) {
+    // steps of more than 256 tokens go out launch by launch: their kernels outlast their launches, and a graph per length would be built for each.  Up to 256
+    // they do not at narrow widths (eight layers of width 512, 200 tokens: 1021 us captured, 1047 launch by launch; of width 1024: 1241 and 1265; 200 slots decoding
+    // through four layers of width 1024: 520 and 526; 300 tokens and more: the same within 0.2 %)
+    if (!use_graph || MT > GRAPH_MT) {
         enqueue_step(stream, MT, MTR, nullptr, runs);
         enqueue_keep(stream, MT, MTR);
         launch_total += launches_last_step;
