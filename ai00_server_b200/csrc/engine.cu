@@ -548,6 +548,13 @@ struct b200rwkv_engine {
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
     // column a thread, and a chain of tokens takes longer with two)
     bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }
+    // Recurrences of prompt steps that have at most one CTA an SM: each asks for more than half an SM's shared memory, so that no two share one.  They start early
+    // (programmatic launches), when most SMs are full of the projections in front of them, were packed onto the few that were not and took turns there.
+    // Measured (whole prompts, four layers of width 2560): one of 200 tokens 988 -> 856 us; two layers of gated delta rule, matrix memory and attention of width 2048:
+    // one of 300 tokens 1001 -> 801; with two CTAs an SM and more nothing is gained
+    bool scan_alone = false;           // of the step being enqueued
+    size_t scan_launch_smem(size_t need) const { return scan_alone ? std::max<size_t>(need, SCAN_ALONE_SMEM) : need; }
+    int kx_scan_ctas() const;
     int dbg_T = 0;                     // rows a layer has in the debug copy of the residual stream
     double pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const;
     void launch_pair(const GemmLaunch& g, const GemmParams& gp, int rows, int parts, cudaStream_t s, Profiler* prof);
@@ -1146,9 +1153,9 @@ void b200rwkv_engine::build(const StFile& st) {
         CK(cudaFuncSetAttribute(wkv_kernel<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
     }
     allow_smem(ln_mix_rows_kernel, (size_t)(LN_ROWS + 1) * C * 4);
-    allow_smem(wkv_scan_kernel<5>, WksCfg<5>::SMEM_BYTES);
-    allow_smem(wkv_scan_kernel<6>, WksCfg<6>::SMEM_BYTES);
-    allow_smem(wkv_scan_kernel<7>, WksCfg<7>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<5>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<6>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<7>, SCAN_ALONE_SMEM);
     if (precision == 1) split_act = true;         // f32-activation mode (web-rwkv `Bundle::<f32>`): no activation is rounded to f16
     if (const char* v = dbg_env("B200RWKV_PREFETCH_BLOCKS")) prefetch_blocks = std::max(0, atoi(v));
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;
@@ -1787,9 +1794,9 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             const bool sp = split_on && MT == 1;
             if (scan) {
                 const dim3 grid(Hl, wkv_slots), block(WKS_THREADS);
-                if (info.version == 5) launch_k(wkv_scan_kernel<5>, grid, block, WksCfg<5>::SMEM_BYTES, wp, KC_WKV, s, prof);
-                else if (info.version == 6) launch_k(wkv_scan_kernel<6>, grid, block, WksCfg<6>::SMEM_BYTES, wp, KC_WKV, s, prof);
-                else launch_k(wkv_scan_kernel<7>, grid, block, WksCfg<7>::SMEM_BYTES, wp, KC_WKV, s, prof);
+                if (info.version == 5) launch_k(wkv_scan_kernel<5>, grid, block, scan_launch_smem(WksCfg<5>::SMEM_BYTES), wp, KC_WKV, s, prof);
+                else if (info.version == 6) launch_k(wkv_scan_kernel<6>, grid, block, scan_launch_smem(WksCfg<6>::SMEM_BYTES), wp, KC_WKV, s, prof);
+                else launch_k(wkv_scan_kernel<7>, grid, block, scan_launch_smem(WksCfg<7>::SMEM_BYTES), wp, KC_WKV, s, prof);
             } else {
             const size_t sm_b = wkv_smem_bytes(info.version, fold_wd2, info.time_decay_adapter, rows, sp);
             switch (info.version * 2 + (sp ? 1 : 0)) {
@@ -1841,6 +1848,7 @@ void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MT, int MTR) {
 }
 
 void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
+    scan_alone = runs && Hl * step_seqs <= num_sms;
     // steps of more than 256 tokens go out launch by launch: their kernels outlast their launches, and a graph per length would be built for each.  Up to 256
     // they do not at narrow widths (eight layers of width 512, 200 tokens: 1021 us captured, 1047 launch by launch; of width 1024: 1241 and 1265; 200 slots decoding
     // through four layers of width 1024: 520 and 526; 300 tokens and more: the same within 0.2 %)
@@ -1850,7 +1858,7 @@ void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
         launch_total += launches_last_step;
         return;
     }
-    const int key = (MT * 256 + MTR) * 2 + (runs ? 1 : 0);
+    const int key = ((MT * 256 + MTR) * 2 + (runs ? 1 : 0)) * 2 + (scan_alone ? 1 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

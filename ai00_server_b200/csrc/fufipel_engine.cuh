@@ -127,8 +127,8 @@ void b200rwkv_engine::ff_load(const StFile& st, KxSizes& z) {
         z.n_pr = std::max(z.n_pr, (size_t)r.proj); z.n_q = std::max(z.n_q, (size_t)H_ * dk); z.n_vout = std::max(z.n_vout, (size_t)r.out);
     }
     sa_plan_model(m);
-    CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
-    CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
+    CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
+    CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     REQUIRE((size_t)W * 8 <= 200 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the norm kernel");
     CK(cudaFuncSetAttribute(pre_norm_kernel<NORM_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(pre_norm_kernel<PRE_NORM_THREADS_FEW_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

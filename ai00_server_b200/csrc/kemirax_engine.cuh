@@ -283,8 +283,8 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
         allow_smem(latent_attn_tc_kernel<2, 8>, smem_tc);
         allow_smem(latent_prompt_kernel, LATENT_PROMPT_SMEM);
     }
-    CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
-    CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM));
+    CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
+    CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
     CK(cudaFuncSetAttribute(lin_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_TC_SMEM));
@@ -446,7 +446,7 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
     const ScanShape sh = scan_shape(dk, dv, 3, decode, scan_wide(H_));
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
-    launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), sh.smem_floats() * 4, gp, KC_WKV, s, prof);
+    launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
     if (sh.ncta > 1) launch_k(head_norm_kernel, dim3(rows, cdiv(H_, 4)), dim3(128), 0, gp.norm, KC_LN, s, prof);
 }
 
@@ -455,6 +455,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
     SeqModel& m = *kx;
     REQUIRE(rows <= maxT && rrows <= maxR, B200RWKV_ERR_INVALID, "internal: a step's launches have more rows than its buffers");
     step_rows = rows;
+    if (decode) scan_alone = false;
     m.sm = seq_meta(d_meta, rows);
     const int W = m.W;
     const MetaView mv = meta_view(d_meta, step_rows);
@@ -671,8 +672,24 @@ void b200rwkv_engine::kx_fill_step(int* hm, const std::vector<int>& slots, const
     *decode = dec; *nsplit = ns;
 }
 
+// CTAs a sequence has in the largest recurrence launch of a prompt step
+int b200rwkv_engine::kx_scan_ctas() const {
+    int most = 0;
+    auto add = [&](int heads, int dk, int dv) { most = std::max(most, heads * scan_shape(dk, dv, 3, false, scan_wide(heads)).ncta); };
+    for (const KxLayer& l : kx->layers) {
+        if (l.c.mixer == KX_GLA || l.c.mixer == KX_DELTA) add(l.c.heads, l.c.dim, l.c.vdim);
+        if (l.c.mixer == KX_PARALLEL || l.c.mixer == KX_CHUNK_GLA) add(l.c.mm_heads, l.c.mm_dim, l.c.mm_vdim);
+    }
+    return most;
+}
+
 void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     const int rows = kx_bucket(T), rrows = R > 0 ? kx_bucket(R) : 0;
+    scan_alone = false;
+    if (!decode) {
+        const int ctas = kx_scan_ctas() * step_seqs;
+        scan_alone = ctas > 0 && ctas <= num_sms;
+    }
     if (!use_graph || rows > 512) {        // (launch by launch: the kernels of a long step outlast their launches)
         kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
         enqueue_keep(stream, cdiv(rows, 16), rrows / 16 + (rrows % 16 ? 1 : 0));
@@ -685,7 +702,7 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     for (const KxLayer& l : kx->layers)
         for (int h : {l.c.heads, l.c.mm_heads})
             if (!decode && h > 0 && h < 256 && scan_wide(h) && (wide == 0 || h < wide)) wide = h;
-    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (wide << 22);
+    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

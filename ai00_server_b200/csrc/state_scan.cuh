@@ -32,6 +32,7 @@ constexpr int SCAN_THREADS = 512;                  // most threads per CTA (a wh
 constexpr int SCAN_THREADS_PROMPT = 128;
 constexpr int SCAN_SMEM = 64 * 1024;               // most shared memory of a launch
 constexpr int SCAN_SMEM_FIVE = 44 * 1024;          // ... with five CTAs on an SM
+constexpr int SCAN_ALONE_SMEM = 114 * 1024;        // a second CTA with as much does not fit an SM (228 KB, 1 KB of it a CTA's own)
 
 struct ScanShape {
     int ks, lks, rt;                               // lanes per column (a power of two and its logarithm), entries per lane (a multiple of 4)
