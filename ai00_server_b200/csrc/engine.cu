@@ -621,6 +621,7 @@ struct b200rwkv_engine {
     bool kx_umma(cudaStream_t s, Profiler* prof, LinParams& p, int rows, int groups);
     void kx_lin(cudaStream_t s, Profiler* prof, LinParams p, int rows, int groups, bool force_exact = false);
     void kx_moe_group(cudaStream_t s, Profiler* prof, const MoeGroupParams& gp, int rows);
+    void kx_head_norm(cudaStream_t s, Profiler* prof, const HeadNormParams& np, int rows, bool decode);
     void kx_short_conv(cudaStream_t s, Profiler* prof, const ShortConvParams& cp, int rows, int nslot_grid, bool decode);
     void kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, int H_, int dk, int dv, const float* q, const float* k, const float* v,
                 const float* gate, int ld, float* out, int ldo, int rows, int nslot_grid, bool decode);

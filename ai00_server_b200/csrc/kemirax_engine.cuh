@@ -424,6 +424,15 @@ void b200rwkv_engine::kx_moe_group(cudaStream_t s, Profiler* prof, const MoeGrou
     else launch_k(moe_group_kernel, dim3(1), dim3(256), ((size_t)std::max(gp.E, 1) * 2 + (size_t)rows * gp.top) * 4, gp, KC_OTHER, s, prof);
 }
 
+// Norms of the heads of a recurrence that several CTAs share.  In prompt steps they start behind it and not early: their CTAs, waiting for hundreds of microseconds on
+// every SM, kept the attention beside the recurrence (side stream) from starting, since it needs more shared memory than their SMs were set up with.  Measured (two
+// layers of gated delta rule, matrix memory and attention): one prompt of 1000 tokens of width 512 1751 -> 1360 us, of width 1024 1845 -> 1451; 512 tokens of
+// width 2048 1165 -> 930; nothing beside the recurrence: the same within 1 %
+void b200rwkv_engine::kx_head_norm(cudaStream_t s, Profiler* prof, const HeadNormParams& np, int rows, bool decode) {
+    if (!decode) pdl_prev = nullptr;
+    launch_k(head_norm_kernel, dim3(rows, cdiv(np.H, 4)), dim3(128), 0, np, KC_LN, s, prof);
+}
+
 // the short convolutions of a layer: one launch in steps of one token per sequence, otherwise the convolution and then the new tails
 void b200rwkv_engine::kx_short_conv(cudaStream_t s, Profiler* prof, const ShortConvParams& cp, int rows, int nslot_grid, bool decode) {
     const int cb = cdiv(cp.C, 256);
@@ -447,7 +456,7 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
     launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
-    if (sh.ncta > 1) launch_k(head_norm_kernel, dim3(rows, cdiv(H_, 4)), dim3(128), 0, gp.norm, KC_LN, s, prof);
+    if (sh.ncta > 1) kx_head_norm(s, prof, gp.norm, rows, decode);
 }
 
 void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool decode, int nsplit, Profiler* prof) {
