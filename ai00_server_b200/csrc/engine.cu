@@ -535,6 +535,14 @@ struct b200rwkv_engine {
     CUtensorMap ta256, ta128;
     int step_tokens = 128;             // tokens of a full step
     int maxR = 0;                      // logits rows of a step
+    bool step_tiled(int MT) const { return MT >= 8 && maxT > 128; }      // more than 64 tokens: operands in 128-token tiles, projections on pairs of SMs
+    int step_th(int MT) const { return (split_on && MT == 1) ? 32 : (step_tiled(MT) ? 128 : 16 * MT); }      // token rows of a step's A16 operands
+    // partial sums that a row-parallel projection leaves in a step (`split` in steps of up to 64 tokens)
+    int step_parts(const GemmLaunch& g, int MT, int split) const {
+        int ntok, parts = split;
+        if (step_tiled(MT)) pair_plan(g, 16 * MT, &ntok, &parts);
+        return parts;
+    }
     int part_stride(bool tiled) const { return tiled ? maxT : std::min(maxT, 128); }      // token rows between partial sums
     // step metadata: steps of up to 128 tokens use arrays of that length, so that a decode step uploads a few KB
     int meta_rows(int T) const { return T > 128 ? maxT : std::min(maxT, 128); }
@@ -576,7 +584,7 @@ struct b200rwkv_engine {
     std::map<int, long long> graph_launches;   // kernels per captured step graph
     long long launch_total = 0;                // kernels launched by this engine's steps since creation
     long long launches_last_step = 0;
-    int last_T = 0, last_th = 16;      // tokens / A16 token rows of the most recent step
+    int last_T = 0;                    // tokens of the most recent step
 
     // softmax
     float *sm_in = nullptr, *sm_out = nullptr;
@@ -1636,20 +1644,14 @@ void b200rwkv_engine::finalize_tp() {
 void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* prof, bool runs) {
     launches_last_step = 0;
     const int rows = MT * 16;
-    const bool tiled = MT >= 8 && maxT > 128;  // more than 64 tokens: operands in 128-token tiles, projections on pairs of SMs
+    const bool tiled = step_tiled(MT);
     const MetaView mv = meta_view(d_meta, rows);
     // token rows of this step's A16 operands (common.cuh): every producer and consumer of the step uses the same value
-    const int th = (split_on && MT == 1) ? 32 : (tiled ? 128 : 16 * MT);
+    const int th = step_th(MT);
     const int th_rows = (split_on && MT == 1) ? 32 : std::min(128, 16 * MTR);        // the head's operand holds output rows
     auto th_of = [&](int tile_kb) { return tiled ? th | tile_kb << 16 : th; };
-    last_th = th;
     // longer steps choose how many partial sums the row-parallel projections leave
-    int parts_o = 0, parts_v = 0;
-    if (tiled) {
-        int nt;
-        pair_plan(layers[0].o, rows, &nt, &parts_o);
-        pair_plan(layers[0].ffn.back(), rows, &nt, &parts_v);
-    }
+    const int parts_o = step_parts(layers[0].o, MT, split_att), parts_v = step_parts(layers[0].ffn.back(), MT, split_ffn);
     auto take_parts = [&](auto& q, float* base, int n) {
         if (!tiled || q.n_parts == 0) return;
         q.n_parts = n;
@@ -3174,7 +3176,7 @@ int32_t b200rwkv_debug_read(b200rwkv_engine* e, const char* name, float* out, si
         CK(cudaSetDevice(e->dev));
         CK(cudaStreamSynchronize(e->stream));
         const std::string n(name);
-        const int T = std::max(e->last_T, 1);
+        const int T = std::max(e->last_T, 1), MT = mt_bucket(T);
         if (e->kx) {
             // "layers_on": keep the residual stream after every layer of the following steps (un-graphed); "layers": read it,
             // [num_layer][128 token rows][num_emb]
@@ -3198,10 +3200,11 @@ int32_t b200rwkv_debug_read(b200rwkv_engine* e, const char* name, float* out, si
             if (n == f.n) {
                 REQUIRE((size_t)T * f.cols <= cap, B200RWKV_ERR_INVALID, "debug buffer too small");
                 CK(cudaMemcpy(out, f.p, (size_t)T * f.cols * 4, cudaMemcpyDeviceToHost));
-                const int nsum = (n == "part_att") ? e->split_att : (n == "part_ffn" ? e->split_ffn : 1);
+                const int nsum = (n == "part_att") ? e->step_parts(e->layers[0].o, MT, e->split_att)
+                                                   : (n == "part_ffn" ? e->step_parts(e->layers[0].ffn.back(), MT, e->split_ffn) : 1);
                 std::vector<float> tmp((size_t)T * f.cols);
                 for (int sp = 1; sp < nsum; ++sp) {       // split-K partials: sum the slices
-                    CK(cudaMemcpy(tmp.data(), f.p + (size_t)sp * e->part_stride(false) * e->C, tmp.size() * 4, cudaMemcpyDeviceToHost));
+                    CK(cudaMemcpy(tmp.data(), f.p + (size_t)sp * e->part_stride(e->step_tiled(MT)) * e->C, tmp.size() * 4, cudaMemcpyDeviceToHost));
                     for (size_t i = 0; i < tmp.size(); ++i) out[i] += tmp[i];
                 }
                 return f.cols;
@@ -3220,7 +3223,7 @@ int32_t b200rwkv_debug_read(b200rwkv_engine* e, const char* name, float* out, si
                 const size_t at0 = (size_t)a.mat * a.b->halves_per_matrix;
                 std::vector<__half> h((size_t)a.b->tile_kb * A16_KB_HALVES * cdiv(e->maxT, A16_KB_ROWS) - at0);
                 CK(cudaMemcpy(h.data(), a.b->p + at0, h.size() * 2, cudaMemcpyDeviceToHost));
-                const int th = T > 128 ? e->last_th | a.b->tile_kb << 16 : e->last_th;
+                const int th = e->step_tiled(MT) ? e->step_th(MT) | a.b->tile_kb << 16 : e->step_th(MT);
                 for (int t = 0; t < T; ++t)
                     for (int c = 0; c < a.cols; ++c) out[(size_t)t * a.cols + c] = __half2float(h[a16_index(t, c, th)]);
                 return a.cols;

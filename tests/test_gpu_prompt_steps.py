@@ -82,6 +82,23 @@ def test_long_steps_of_small_chunks(chunk):
     _check("tiny6", [700, 31], full=False, chunk=chunk)
 
 
+def test_debug_reads_of_steps_of_every_form():
+    """The residual behind a layer's mixer is the one in front of it plus the partial sums of the output projection, and the f16 operands hold the same rows, whatever form
+    the last step had and whether it was captured or replayed."""
+    st = synth.make_st(synth.Shape(6, 2, 512, 1792, V=512), 3)
+    m = runtime.Model(st, max_batch=1, token_chunk_size=128)
+    try:
+        m.state.reset(0)
+        for n in (100, 5, 300, 100, 40, 5, 200):
+            m.infer_raw([0], [n], list(range(1, n + 1)), [capi.OPTION_NONE])
+            x_a, x_b, parts = (m.debug_read(k, n) for k in ("x_a", "x_b", "part_att"))
+            assert np.abs(x_b - x_a - parts).max() <= 1e-5 * np.abs(x_b).max(), n          # f32 sums of a few parts, in another order
+            d = m.debug_read("a_x1", n).astype(np.float64)                                # the key operand of the last layer: RWKV-6's mix between xx and sx
+            assert np.isfinite(d).all() and (np.abs(d).sum(1) > 0).all(), n
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("lens, rows", [([200], [(0, 128, 200)]), ([130, 140, 5], [(1, 121, 140)])])
 def test_last_hidden_answers_the_last_portion(lens, rows):
     """Without keep_hidden the hidden rows are those of the call's last portion of at most 128 tokens, whatever a step holds."""
