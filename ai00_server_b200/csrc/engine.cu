@@ -1949,8 +1949,8 @@ void b200rwkv_engine::infer(int nslot, const int32_t* slot, const int32_t* ntok,
     const int step_cap = std::min(chunk, split_on ? 16 : (kx ? (kx->dbg_layers ? dbg_T : kx->portion) : std::min(maxT, 128)));
     // RWKV steps hold up to sixteen portions (gemm_pair.cuh: one pass over the weights for all their tokens): the portions, and with them the
     // rows b200rwkv_last_hidden answers, are those of 128-token steps
-    // (config.json families: portions of up to 512, steps as in kx_build)
-    const int substeps = kx ? (kx->dbg_layers ? 1 : std::max(1, maxT / step_cap)) : (maxT > 128 ? std::max(1, (int)std::min<long long>(step_tokens, 16ll * chunk) / step_cap) : 1);
+    // (config.json families: portions of up to 512, steps as in kx_rows.cuh)
+    const int substeps = kx ? (kx->dbg_layers ? 1 : std::max(1, kx_step_tokens(chunk, kx->exact) / step_cap)) : (maxT > 128 ? std::max(1, (int)std::min<long long>(step_tokens, 16ll * chunk) / step_cap) : 1);
     // Step packing: every step shares its token budget evenly over the entries that still have tokens (web-rwkv shares the
     // chunk "fairly across slots"; results do not depend on the cut).  Many slots with one token each keep
     // the WKV kernels wide (one CTA per head and slot) where a single slot with 64 tokens would run them 40 CTAs wide.

@@ -19,11 +19,11 @@ inline int kx_bucket_below(int b) { return b > 512 ? b - 256 : b / 2; }
 // tokens of a portion
 inline int kx_portion(int chunk) { return chunk > 256 ? 512 : (chunk > 128 ? 256 : 128); }
 
-// rows every buffer of a step holds: sixteen chunks and a portion at least, and a bucket itself, since launches cover the bucket of a step's tokens (operands are
-// packed and tensor maps encoded with that many rows a group).  f32-exact steps hold one portion
-inline int kx_max_rows(int chunk, bool exact) {
-    const int portion = kx_portion(chunk);
-    return exact ? portion : kx_bucket(std::max(portion, (int)std::min<long long>(16ll * chunk, KX_MAX_STEP)));
-}
+// tokens of a step: sixteen chunks (f32-exact models: one portion)
+inline int kx_step_tokens(int chunk, bool exact) { return exact ? std::min(chunk, kx_portion(chunk)) : (int)std::min<long long>(16ll * chunk, KX_MAX_STEP); }
+
+// rows every buffer of a step holds: a step's tokens and a whole portion at least, and a bucket itself, since launches cover the bucket of a step's tokens (operands
+// are packed and tensor maps encoded with that many rows a group)
+inline int kx_max_rows(int chunk, bool exact) { return kx_bucket(std::max(kx_portion(chunk), kx_step_tokens(chunk, exact))); }
 
 }  // namespace b200

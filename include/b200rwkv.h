@@ -111,8 +111,10 @@ typedef struct {
      * attention beside gated linear attention, pair embeddings; bf16 weights): the JSON text, borrowed during the call.  NULL: the
      * family is recognised from the tensor names (RWKV v5 / v6 / v7).  Such models keep an attention cache in pages of
      * `kv_page` tokens (0 = 64) drawn from a pool sized for `kv_tokens` tokens over all live sequences (0 = 4096 per slot);
-     * precision 0 = bf16 tensor-core products with f32 accumulation, 1 = every product in plain f32.  Their steps hold up to
-     * 128 tokens, 256 or 512 when token_chunk_size asks for more than 128 / 256. */
+     * precision 0 = bf16 tensor-core products with f32 accumulation, 1 = every product in plain f32.  Tokens are taken in portions of
+     * at most token_chunk_size, never more than 512; a step holds sixteen token_chunk_size tokens (2048 at most) at precision 0 and one portion
+     * at precision 1.  Activations of a step's tokens are reserved when the model is created, the cache pages of all its tokens are taken before it
+     * runs: a step that does not fit the pool is refused as a whole (B200RWKV_ERR_STATE). */
     const uint8_t* config_json;
     size_t config_len;
     int32_t kv_tokens;
@@ -157,8 +159,8 @@ int32_t b200rwkv_get_info(b200rwkv_engine*, b200rwkv_info* out);
  * `RnnInput`: a ragged batch of `nslot` entries; entry i feeds `ntok[i]` tokens
  * (tokens + sum(ntok[0..i])) to state slot `slot[i]` with RnnOption `option[i]`.
  * All tokens are consumed (internally in portions of at most min(token_chunk_size, 128) tokens shared evenly over the
- * entries, two full-sized portions to a step on one GPU, the policy
- * web-rwkv applies across calls at run.rs:1134-1145).  Logits rows (num_vocab f32 each) are
+ * entries, the policy web-rwkv applies across calls at run.rs:1134-1145; unquantised f16 models on one GPU run up to sixteen
+ * token_chunk_size tokens, 2048 at most, as one step, others one portion, of 16 tokens at precision 1; see b200rwkv_options for the config.json families).  Logits rows (num_vocab f32 each) are
  * written contiguously to `logits_out` in entry order: 1 row for LAST (0 if ntok[i]==0),
  * ntok[i] rows for FULL, none for NONE; rows_out[i] receives the row count of entry i
  * (== RnnOutputBatch being empty or not, run.rs:1146-1155).  `logits_cap` is in floats.

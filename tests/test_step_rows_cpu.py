@@ -18,7 +18,8 @@ int main() {
             const int rows = kx_max_rows(chunk, exact), out = std::min(rows, KX_MAX_OUT_ROWS), portion = kx_portion(chunk);
             std::set<int> walked;
             for (int r = rows; r > 16; r = kx_bucket_below(r)) walked.insert(r);
-            bool ok = rows >= portion && out >= std::min(chunk, portion) && (exact || rows >= std::min(16 * chunk, KX_MAX_STEP));
+            const int step = kx_step_tokens(chunk, exact), cap = std::min(chunk, portion);      // tokens of a step, of a portion
+            bool ok = rows >= portion && out >= cap && rows >= step && step >= cap && step == (exact ? cap : std::min(16 * chunk, 2048));
             for (int n = 1; n <= rows; ++n) ok = ok && kx_bucket(n) >= n && kx_bucket(n) <= rows && (kx_bucket(n) <= 16 || walked.count(kx_bucket(n)));
             for (int n = 1; n <= out; ++n) ok = ok && kx_bucket(n) <= out;
             if (!ok && bad++ < 20) printf("chunk %d exact %d: buffers of %d rows, a full step's launches have %d, %d logits rows' %d\n", chunk, exact, rows, kx_bucket(rows), out, kx_bucket(out));
