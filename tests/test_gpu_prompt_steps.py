@@ -184,6 +184,14 @@ def test_routed_projections_of_a_step_of_n_rows(n, experts, top):
     _check_family(synth.make_kemirax, [layer], kemirax_numpy, n, width=72)
 
 
+@pytest.mark.parametrize("n", [130, 300])
+@pytest.mark.parametrize("experts, top", [(40, 3), (256, 8), (300, 2)])
+def test_row_lists_of_many_experts(n, experts, top):
+    """Lists built by matching lanes for more experts than a warp has lanes, for the most that form takes, and one by one for more."""
+    layer = synth.kemirax_layer("gla", heads=2, dim=16, vdim=24, experts=experts, identity=1, top=top, ff=24, shared_ff=40)
+    _check_family(synth.make_kemirax, [layer], kemirax_numpy, n, width=72)
+
+
 @pytest.mark.parametrize("chunk", [20, 33, 40, 100])
 def test_full_steps_of_chunks_between_the_row_counts_of_launches(chunk):
     """Sixteen chunks that are no row count of a launch (powers of two, multiples of 256): a full step and a little more, grouped projections (a group a head, a group an
