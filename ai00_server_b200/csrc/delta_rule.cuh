@@ -156,7 +156,7 @@ struct DeltaScanParams {
     HeadNormParams norm;                          // norm.x: raw read-outs, normed and gated in place
 };
 
-// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread
+// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread (2: packed pairs)
 template <bool CHANNEL, int NCOL>
 __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT, NCOL == 0 ? 2 : (NCOL == 1 ? 5 : 4)) delta_scan_kernel(const DeltaScanParams p) {
     pdl_launch_dependents();
@@ -177,12 +177,12 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
     float* rec = p.state + ((size_t)slot * p.H + h) * ((size_t)ks * sh.rt * dv);
     __shared__ float red[SCAN_THREADS / 32];
     const bool mine = part == 0 && col < ncol;    // this thread writes the column's read-outs
-    constexpr bool STEP = NCOL == 0;
+    constexpr bool STEP = NCOL == 0, PACKED = NCOL == 2;
     constexpr int NC = STEP ? 1 : NCOL;           // columns of this thread: j, j + cstep
     const int cstep = blockDim.x >> sh.lks;
-    float s[STEP ? SCAN_R : 1];
-    f32x2 s2[NC][STEP ? 1 : SCAN_R / 2];
-    if constexpr (STEP) {
+    float s[PACKED ? 1 : SCAN_R];
+    f32x2 s2[NC][PACKED ? SCAN_R / 2 : 1];
+    if constexpr (!PACKED) {
         scan_load_state(sh, rec, dv, j, part, s);
     } else {
 #pragma unroll
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
         for (int t = 0; t < n; ++t) {
             const float* kr = buf + (size_t)t * tokf + part * SCAN_ROW;
             const float4 sc = sscal[t];
-            if constexpr (!STEP) {
+            if constexpr (PACKED) {
                 float v[NC], d[NC];
                 f32x2 oa[NC], ob[NC], u2[NC];
                 const f32x2 g2 = pack2(sc.x, sc.x);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
             }
             const float d = scan_part_sum((d0 + d1) + (d2 + d3), ks);
             const float u = sc.y * (vj - d * sc.z) * sc.z;         // u / |k|: the write is (k / |k|) u^T
-            asm volatile("" ::: "memory");               // read the key again below instead of keeping it: 64 registers, two CTAs per SM
+            if (STEP) asm volatile("" ::: "memory");     // read the key again below instead of keeping it: 64 registers, two CTAs per SM
             float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
 #pragma unroll
             for (int r = 0; r < SCAN_R; r += 4) {
@@ -328,13 +328,13 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
                 o0 = fmaf(s[r], q4.x, o0); o1 = fmaf(s[r + 1], q4.y, o1); o2 = fmaf(s[r + 2], q4.z, o2); o3 = fmaf(s[r + 3], q4.w, o3);
             }
             const float o = scan_part_sum((o0 + o1) + (o2 + o3), ks) * sc.w;
-            if (sh.ncta == 1) o_last = o;
+            if (STEP && sh.ncta == 1) o_last = o;
             else if (mine) orow[(size_t)t * p.norm.ldx] = o;
             }
         }
         if (!STEP) __syncthreads();
     }
-    if constexpr (STEP) {
+    if constexpr (!PACKED) {
         scan_store_state(sh, rec, dv, j, part, s);
     } else {
 #pragma unroll

@@ -23,9 +23,9 @@ struct GlaParams {
     HeadNormParams norm;                          // norm.x: raw read-outs, normed and gated in place
 };
 
-// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread
+// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread (2: packed pairs)
 template <int NCOL>
-__global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT, NCOL == 0 ? 2 : (NCOL == 1 ? 5 : 4)) gla_scan_kernel(const GlaParams p) {
+__global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT, NCOL == 0 ? 2 : 4) gla_scan_kernel(const GlaParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const ScanShape& sh = p.s;
@@ -42,12 +42,12 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
     float* rec = p.state + ((size_t)slot * p.H + h) * ((size_t)ks * sh.rt * dv);
     __shared__ float red[SCAN_THREADS / 32];
     const bool mine = part == 0 && col < ncol;    // this thread writes the column's read-outs
-    constexpr bool STEP = NCOL == 0;
+    constexpr bool STEP = NCOL == 0, PACKED = NCOL == 2;
     constexpr int NC = STEP ? 1 : NCOL;           // columns of this thread: j, j + cstep
     const int cstep = blockDim.x >> sh.lks;
-    float s[STEP ? SCAN_R : 1];
-    f32x2 s2[NC][STEP ? 1 : SCAN_R / 2];
-    if constexpr (STEP) {
+    float s[PACKED ? 1 : SCAN_R];
+    f32x2 s2[NC][PACKED ? SCAN_R / 2 : 1];
+    if constexpr (!PACKED) {
         scan_load_state(sh, rec, dv, j, part, s);
     } else {
 #pragma unroll
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
         float* orow = p.norm.x + (size_t)(t0 + c * sh.tc) * p.norm.ldx + (size_t)h * dv + j;
         for (int t = 0; t < n; ++t) {
             const float* kr = buf + (size_t)t * tokf + part * SCAN_ROW;
-            if constexpr (!STEP) {
+            if constexpr (PACKED) {
                 f32x2 v2[NC], oa[NC], ob[NC];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) { const float v = buf[(size_t)t * tokf + 3 * krow + col + c * cstep]; v2[c] = pack2(v, v); oa[c] = ob[c] = 0ull; }
@@ -131,13 +131,13 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
                 o0 = fmaf(s[r], q4.x, o0); o1 = fmaf(s[r + 1], q4.y, o1); o2 = fmaf(s[r + 2], q4.z, o2); o3 = fmaf(s[r + 3], q4.w, o3);
             }
             const float o = scan_part_sum((o0 + o1) + (o2 + o3), ks) * p.q_scale;
-            if (sh.ncta == 1) o_last = o;
+            if (STEP && sh.ncta == 1) o_last = o;
             else if (mine) orow[(size_t)t * p.norm.ldx] = o;
             }
         }
         if (!STEP) __syncthreads();
     }
-    if constexpr (STEP) {
+    if constexpr (!PACKED) {
         scan_store_state(sh, rec, dv, j, part, s);
     } else {
 #pragma unroll

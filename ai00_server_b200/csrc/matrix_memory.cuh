@@ -35,7 +35,7 @@ struct MatrixMemoryParams {
 
 constexpr int MM_MAX_N = SCAN_MAX_DK / SCAN_THREADS_PROMPT;      // normaliser entries per thread
 
-// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread
+// NCOL = 0: steps of one token per sequence; 1, 2: prompt steps, columns per thread (2: packed pairs)
 template <int NCOL>
 __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT, NCOL == 0 ? 2 : (NCOL == 1 ? 4 : 3)) matrix_memory_kernel(const MatrixMemoryParams p) {
     pdl_launch_dependents();
@@ -60,12 +60,12 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
     float* gm = p.m + hs * dv + cb * sh.cols;
     __shared__ float red[SCAN_THREADS / 32];
     const bool mine = part == 0 && col < ncol;     // this thread writes the column's read-outs
-    constexpr bool STEP = NCOL == 0;
+    constexpr bool STEP = NCOL == 0, PACKED = NCOL == 2;
     constexpr int NC = STEP ? 1 : NCOL;           // columns of this thread: j, j + cstep
     const int cstep = blockDim.x >> sh.lks;
-    float s[STEP ? SCAN_R : 1];
-    f32x2 s2[NC][STEP ? 1 : SCAN_R / 2];
-    if constexpr (STEP) {
+    float s[PACKED ? 1 : SCAN_R];
+    f32x2 s2[NC][PACKED ? SCAN_R / 2 : 1];
+    if constexpr (!PACKED) {
         scan_load_state(sh, rec, dv, j, part, s);
     } else {
 #pragma unroll
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
             const float* row = buf + (size_t)t * tokf;
             const float* kr = row + part * SCAN_ROW;
             const float4 sc = sscal[t];
-            if constexpr (!STEP) {
+            if constexpr (PACKED) {
                 f32x2 v2[NC], oa[NC], ob[NC];
                 const f32x2 keep2 = pack2(sc.x, sc.x);
 #pragma unroll
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
                 o0 = fmaf(s[r], q4.x, o0); o1 = fmaf(s[r + 1], q4.y, o1); o2 = fmaf(s[r + 2], q4.z, o2); o3 = fmaf(s[r + 3], q4.w, o3);
             }
             const float o = scan_part_sum((o0 + o1) + (o2 + o3), ks);
-            if (sh.ncta == 1) o_last = o;
+            if (STEP && sh.ncta == 1) o_last = o;
             else if (mine) orow[(size_t)t * p.norm.ldx] = o;
             }
             if (cb == 0) {                         // the normaliser and its product with the query
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(NCOL == 0 ? SCAN_THREADS : SCAN_THREADS_PROMPT
             }
         }
     }
-    if constexpr (STEP) {
+    if constexpr (!PACKED) {
         scan_store_state(sh, rec, dv, j, part, s);
     } else {
 #pragma unroll

@@ -5,8 +5,10 @@
 // `ks` neighbouring lanes, each keeping `rt` of its dk entries in registers for all tokens of the step, so a product with the key
 // or query is straight-line FMA on registers followed by log2(ks) exchanges, and no barrier separates the tokens.  Prompt steps of several sequences
 // give a thread TWO columns (`nc`): the loop over tokens is bound by the reads of staged keys and queries (24 of 16 bytes for 128 products a column and
-// token in the delta rule), which two columns share; products run as packed pairs of neighbouring entries.
-// Measured (2048 tokens of 16 sequences, 16 heads of 128 x 128, ncu): delta rule 237 -> 211 us, gated linear attention 365 -> 328.  Heads whose
+// token in the delta rule), which two columns share; their products run as packed pairs of neighbouring entries.
+// Measured (2048 tokens of 16 sequences, 16 heads of 128 x 128, ncu): delta rule 237 -> 211 us, gated linear attention 365 -> 328.  With ONE column a thread the chain of a
+// token holds the loop and products are single: as packed pairs they took 2-6 % longer (one sequence of 512 tokens, ncu: delta rule 298 -> 307, matrix memory 292 -> 298;
+// 128 tokens of gated linear attention 83 -> 88; whole prompts 1-2 %).  Heads whose
 // columns do not fit one CTA are split over `ncta` of them (prompt steps always prefer many small CTAs).  Keys, queries and the
 // CTA's value entries of the next `tc` tokens arrive by cp.async while the current ones are worked on.
 //
