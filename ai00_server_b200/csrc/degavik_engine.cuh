@@ -238,7 +238,7 @@ void b200rwkv_engine::dg_enqueue_layer(cudaStream_t s, KxLayer& l, int rows, int
         const ScanShape sh = scan_shape(dk, dv, 3, decode, scan_wide(H_));
         DeltaScanParams dp{m.cv, m.cv + G_ * dk, m.cv + 2 * G_ * dk, C_, m.z, H_ * dk, m.pr + C_, PN, l.a_log, l.rec_state, H_, G_, dk, dv,
                            1.f / sqrtf((float)dk), 1e-6f, sh, {m.vout, H_ * dv, nullptr, m.gl, H_ * dv, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 0, mv}};
-        launch_k(decode ? delta_scan_kernel<true, 0> : (sh.nc == 2 ? delta_scan_kernel<true, 2> : delta_scan_kernel<true, 1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
+        launch_k(decode ? delta_scan_kernel<true, 0> : (sh.nc == 2 ? delta_scan_kernel<true, 2> : delta_scan_kernel<true, 1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
         if (sh.ncta > 1) kx_head_norm(s, prof, dp.norm, rows, decode);
     } else {
         AttnPrepParams ap{m.pr, m.pr + H_ * dk, m.pr + H_ * dk + G_ * dk, PN, m.q, H_ * dk, l.cache, m.d_table, m.npages, m.page, l.qn_w, l.kn_w,

@@ -399,7 +399,7 @@ enum KClass { KC_GEMM = 0, KC_WKV = 1, KC_LN = 2, KC_OTHER = 3 };
 
 struct GemmLaunch {
     GemmParams p;
-    CUtensorMap tw;            // the weight blocks as rows of 1 KB (steps of more than 128 tokens)
+    CUtensorMap tw;            // the weight blocks as rows of 1 KB (gemm_pair.cuh: steps of more than 64 tokens)
     bool chain = false;        // the segments are slices of one k range: longer steps choose their own number of partial sums
     int grid = 0;
     int grid_wide = 0;         // grid of steps with more than 64 tokens (see make_launch)
@@ -529,7 +529,7 @@ struct b200rwkv_engine {
     float *f_r = nullptr, *f_k = nullptr, *f_v = nullptr, *f_g = nullptr, *f_w = nullptr, *f_a = nullptr, *f_nu = nullptr,
           *f_vfirst = nullptr, *f_rr = nullptr, *part_att = nullptr, *part_ffn = nullptr, *d_logits = nullptr, *d_hidden = nullptr;
     A16Buf a_x[6], a_lora[5], a_out, a_kk, a_head;
-    // steps of more than 128 tokens (gemm_pair.cuh): every A16 buffer lies in one arena that two tensor maps cover
+    // steps of more than 64 tokens (gemm_pair.cuh): every A16 buffer lies in one arena that two tensor maps cover
     __half* a16_arena = nullptr;
     size_t a16_arena_halves = 0, a16_used = 0;
     CUtensorMap ta256, ta128;
@@ -561,6 +561,12 @@ struct b200rwkv_engine {
     // Measured (whole prompts, four layers of width 2560): one of 200 tokens 988 -> 856 us; two layers of gated delta rule, matrix memory and attention of width 2048:
     // one of 300 tokens 1001 -> 801; with two CTAs an SM and more nothing is gained
     bool scan_alone = false;           // of the step being enqueued
+    int scan_alone_seqs = 0;           // sequences such a step holds at most: CTAs for slots beyond would wait for an SM's shared memory only to leave
+    void set_scan_alone(bool prompt, int ctas_a_seq) {
+        scan_alone = prompt && ctas_a_seq > 0 && ctas_a_seq * step_seqs <= num_sms;
+        scan_alone_seqs = scan_alone ? num_sms / ctas_a_seq : 0;
+    }
+    int scan_slots(int slots) const { return scan_alone ? std::min(slots, scan_alone_seqs) : slots; }
     size_t scan_launch_smem(size_t need) const { return scan_alone ? std::max<size_t>(need, SCAN_ALONE_SMEM) : need; }
     int kx_scan_ctas() const;
     int dbg_T = 0;                     // rows a layer has in the debug copy of the residual stream
@@ -1056,7 +1062,7 @@ void b200rwkv_engine::launch_gemm(const GemmLaunch& g, int MT, cudaStream_t s, P
     }
 }
 
-// A step of more than 128 tokens: time of a launch in us as the waves of its units take it (a stage of 64 k: 0.30 us of tensor core with 256
+// A step of more than 64 tokens: time of a launch in us as the waves of its units take it (a stage of 64 k: 0.30 us of tensor core with 256
 // tokens, 0.21 us of L2 reads with 128), the narrower token tile or more partial sums where they fill the last wave better.  A partial sum costs
 // a write and a read of its rows.
 double b200rwkv_engine::pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const {
@@ -1796,7 +1802,7 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             wp.meta = mv;
             const bool sp = split_on && MT == 1;
             if (scan) {
-                const dim3 grid(Hl, wkv_slots), block(WKS_THREADS);
+                const dim3 grid(Hl, scan_slots(wkv_slots)), block(WKS_THREADS);
                 if (info.version == 5) launch_k(wkv_scan_kernel<5>, grid, block, scan_launch_smem(WksCfg<5>::SMEM_BYTES), wp, KC_WKV, s, prof);
                 else if (info.version == 6) launch_k(wkv_scan_kernel<6>, grid, block, scan_launch_smem(WksCfg<6>::SMEM_BYTES), wp, KC_WKV, s, prof);
                 else launch_k(wkv_scan_kernel<7>, grid, block, scan_launch_smem(WksCfg<7>::SMEM_BYTES), wp, KC_WKV, s, prof);
@@ -1851,7 +1857,7 @@ void b200rwkv_engine::enqueue_keep(cudaStream_t s, int MT, int MTR) {
 }
 
 void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
-    scan_alone = runs && Hl * step_seqs <= num_sms;
+    set_scan_alone(runs, Hl);
     // steps of more than 256 tokens go out launch by launch: their kernels outlast their launches, and a graph per length would be built for each.  Up to 256
     // they do not at narrow widths (eight layers of width 512, 200 tokens: 1021 us captured, 1047 launch by launch; of width 1024: 1241 and 1265; 200 slots decoding
     // through four layers of width 1024: 520 and 526; 300 tokens and more: the same within 0.2 %)

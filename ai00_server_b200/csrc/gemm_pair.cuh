@@ -10,7 +10,7 @@
 //   * both operands lie in memory in the order the tensor core reads them, so a stage of 64 k is one box of plain 1 KB rows per operand: tiled TMA
 //     (not the untiled copy) because its arrival may be counted on the leader's barrier;
 //   * steps hold up to 2048 tokens, the units of a launch (token tiles fastest, so that neighbours share weights) are dealt to persistent clusters;
-//   * NTOK = 256, or 128 where the launch would leave more of its last wave empty with 256 than the narrower tile costs (pair_units);
+//   * NTOK = 256, or 128 where the launch would leave more of its last wave empty with 256 than the narrower tile costs (pair_plan in engine.cu);
 //   * eight epilogue warps drain one accumulator while the next unit's MMAs run; f16 operands are transposed warp by warp.
 // Measured (3B widths, 1792 tokens a launch against seven launches of 256 tokens on single SMs, ncu): R/K/V/G 253 -> 83 us (1.13 PFLOP/s), output 132 -> 27,
 // channel mix 307 -> 96 and 171 -> 61, first low-rank stage 225 -> 23; 32 prompts of 512 tokens 53.5 -> 21.5 ms.

@@ -455,7 +455,7 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
     const ScanShape sh = scan_shape(dk, dv, 3, decode, scan_wide(H_));
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
-    launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
+    launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
     if (sh.ncta > 1) kx_head_norm(s, prof, gp.norm, rows, decode);
 }
 
@@ -694,11 +694,7 @@ int b200rwkv_engine::kx_scan_ctas() const {
 
 void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     const int rows = kx_bucket(T), rrows = R > 0 ? kx_bucket(R) : 0;
-    scan_alone = false;
-    if (!decode) {
-        const int ctas = kx_scan_ctas() * step_seqs;
-        scan_alone = ctas > 0 && ctas <= num_sms;
-    }
+    set_scan_alone(!decode, kx_scan_ctas());
     if (!use_graph || rows > 512) {        // (launch by launch: the kernels of a long step outlast their launches)
         kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
         enqueue_keep(stream, cdiv(rows, 16), rrows / 16 + (rrows % 16 ? 1 : 0));

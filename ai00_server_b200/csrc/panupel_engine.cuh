@@ -200,7 +200,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 MatrixMemoryParams mp{m.pr + r.mq, m.pr + r.mk, m.pr + r.mv, PN, m.pr + r.mi, m.pr + r.mf, l.mm_state, l.mm_n, l.mm_m, m.z, Hm, mk, mvd,
                                       c.mm_cap, 1.f / sqrtf((float)mk), 1e-6f, sh,
                                       {m.vout + H_ * dv, KO, m.z, m.pr + r.mg, PN, l.mm_norm_w, mvd, Hm, mvd, eps, c.mm_mul, 0, mv}};
-                launch_k(decode ? matrix_memory_kernel<0> : (sh.nc == 2 ? matrix_memory_kernel<2> : matrix_memory_kernel<1>), dim3(Hm * sh.ncta, nslot_grid), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), mp, KC_WKV, s2, prof);
+                launch_k(decode ? matrix_memory_kernel<0> : (sh.nc == 2 ? matrix_memory_kernel<2> : matrix_memory_kernel<1>), dim3(Hm * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), mp, KC_WKV, s2, prof);
                 if (sh.ncta > 1) kx_head_norm(s2, prof, mp.norm, rows, decode);
             }
             RotPrepParams rp{m.pr + r.q, m.pr + r.k, m.pr + r.v, PN, m.q, H_ * dk, l.cache, m.d_table, m.npages, m.page, l.qn_w, l.kn_w, l.freq_d,
@@ -226,7 +226,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             const ScanShape sh = scan_shape(dk, dv, 2, decode, scan_wide(H_));
             DeltaScanParams dp{m.cv, m.cv + G_ * dk, m.cv + 2 * G_ * dk, ldc, m.pr + r.a, PN, m.pr + r.b, PN, l.a_log, l.rec_state, H_, G_, dk, dv,
                                1.f / sqrtf((float)dk), 1e-6f, sh, {m.vout, KO, nullptr, m.pr + r.g, PN, l.norm_w, 0, H_, dv, eps, 1.f, 1, mv}};
-            launch_k(decode ? delta_scan_kernel<false, 0> : (sh.nc == 2 ? delta_scan_kernel<false, 2> : delta_scan_kernel<false, 1>), dim3(H_ * sh.ncta, nslot_grid), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
+            launch_k(decode ? delta_scan_kernel<false, 0> : (sh.nc == 2 ? delta_scan_kernel<false, 2> : delta_scan_kernel<false, 1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
             if (sh.ncta > 1) kx_head_norm(s, prof, dp.norm, rows, decode);
         }
         kx_lin(s, prof, lin(m.vout, KO, l.o, m.y, W, W, KO), rows, 1);

@@ -13,7 +13,7 @@
 //   * the loop over tokens leaves the four read-outs of a thread as they are; the eight lanes' parts are summed with the norms and outputs, per group, a
 //     warp per token (exchanges between lanes in the loop were a chain of four, some 25 cycles each, on every token).  Sums over keys run even and odd
 //     keys apart: results agree with wkv.cuh's to f32 rounding.
-// Decays come from the decay projection's own launch in these steps (17 us beside the scan's own time below).  Where the decode kernel
+// Decays come from the decay projection's own launch in these steps (lora2.cuh: 6 us beside the scan's own time below).  Where the decode kernel
 // evaluates that low-rank stage itself (RWKV-6), its sums run in another order: decays, and with them states, agree to f32 rounding and not to the bit.
 // Measured (one prompt of 100 tokens, 64 heads, ncu): 30 us a layer (33 with single products and exchanges in the loop, 263 in the decode kernel).
 #pragma once
