@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
                     f32x2 acc = 0ull;
 #pragma unroll
                     for (int f = 0; f < 4; ++f) {
-                        m[e][f] = fmadd2(v[e], k[f], fmadd2(s2, ka[f], prod2(m[e][f], w[f])));
+                        m[e][f] = fmadd2(v[e], k[f], fmadd2(m[e][f], w[f], prod2(s2, ka[f])));      // the state, the largest term, is not rounded apart
                         fma2(acc, m[e][f], r[f]);
                     }
                     const float2 a2 = unpack2(acc);
