@@ -694,7 +694,7 @@ int b200rwkv_engine::kx_scan_ctas() const {
 
 void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     const int rows = kx_bucket(T), rrows = R > 0 ? kx_bucket(R) : 0;
-    set_scan_alone(!decode, kx_scan_ctas());
+    set_scan_alone(!decode, decode ? 0 : kx_scan_ctas());
     if (!use_graph || rows > 512) {        // (launch by launch: the kernels of a long step outlast their launches)
         kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
         enqueue_keep(stream, cdiv(rows, 16), rrows / 16 + (rrows % 16 ? 1 : 0));
