@@ -1,5 +1,5 @@
 // Latent attention of prompt steps on the tensor cores (serving precision): the function of latent_attn_tc_kernel (latent_attn.cuh) with the same operands
-// (TF32, rounded once, f32 sums and softmax), for steps that fill the chip without splitting the keys.
+// (TF32, rounded once, f32 sums and softmax), for steps whose keys are not split: many tokens, or contexts of fewer than four key tiles of 32 (kx_fill_step).
 //
 // What bounds it: the TF32 rate of mma.sync (about 125 multiply-adds a cycle and SM), if operands come cheaply.  All heads read the same latent row, so a CTA
 // of eight warps keeps 64 rows -- up to 16 heads x 4 tokens, 8 x 8 and so on -- and reads each key tile once for them, where the 16-row form read it four
@@ -10,6 +10,9 @@
 //   * values   a warp owns all 64 rows of an eighth of the channels;
 //   * the finished rows go out normalised: no partial results, no merging launch.
 // Measured (eight documents of up to 700 tokens, 16 heads, rows of 576 floats, two steps, ncu): 2119 us and 124 of merging -> 1127.
+// Where the line lies: short contexts leave it a quarter of the 16-row form's CTAs, but one launch instead of two.  Whole prompts of two layers with the 16-row form and with
+// this one, width 2048: 1 x 20 tokens 342 and 342 us, 2 x 20 367 and 370, 1 x 64 426 and 422, 8 x 64 668 and 618, 16 x 32 606 and 571; width 1024: 1 x 96 361 and 358,
+// 2 x 64 350 and 346, 16 x 32 377 and 374; width 512: 1 x 64 257 and 261, 2 x 20 212 and 215.
 #pragma once
 #include "latent_attn.cuh"
 

@@ -1,5 +1,6 @@
 // Softmax attention of prompt steps over the paged cache: the function of sink_attn.cuh (windows, chunks of the sequence, kept first tokens, a bias per
-// distance, a sink term, a gate; no block means), in f32 throughout, for steps with enough tokens to fill the chip without splitting the keys.
+// distance, a sink term, a gate; no block means), in f32 throughout, for steps whose keys are not split: enough tokens to fill the chip, or
+// contexts of one key tile of 32 (kx_fill_step).
 //
 // What bounds it: f32 multiply-adds, 2 dk + 2 dv a (query head, key).  The register form reads every key row from L2 for four (token, head) rows at a
 // time and spends as many exchanges between lanes as products; here a CTA of four warps keeps 64 rows -- the query heads of ONE key / value head for 64 / rep
@@ -11,6 +12,8 @@
 //   * products run as packed pairs (fma.rn.f32x2), even and odd entries of a score summed apart;
 //   * the next key tile arrives (cp.async) while the values are multiplied, the next value tile while the scores are.
 // Measured (width 2048, 16 sequences, 2048 tokens a step): 280 -> 126 us at 128 tokens of context (ncu); 16 prompts of 1024 tokens 32.5 -> 23.3 ms.
+// Where the line lies, whole prompts of two layers with the register form and with this one, width 2048: 1 x 20 tokens 270 and 233 us, 16 x 32 501 and 453, 1 x 600 1181 and 1076;
+// width 512: 1 x 20 165 and 159, 2 x 20 167 and 161, 16 x 32 239 and 231.
 #pragma once
 #include "f32x2.cuh"
 #include "sink_attn.cuh"

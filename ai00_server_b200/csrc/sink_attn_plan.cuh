@@ -160,8 +160,8 @@ static void sa_plan_model(SeqModel& m) {
     }
 }
 
-// One attention launch.  Prompt steps whose chunks fill the chip without splitting the keys (kx_fill_step's rule) take the kernel that stages a key tile for 64
-// (token, head) rows, where its 16-byte rows and sizes allow; block means and longer rows stay with the forms above.
+// One attention launch.  Prompt steps whose keys are not split (kx_fill_step: their chunks fill the chip, or the context is one key tile) take the kernel that stages a
+// key tile for 64 (token, head) rows, where its 16-byte rows and sizes allow; block means and longer rows stay with the forms above.
 void b200rwkv_engine::kx_sink_attn(cudaStream_t s, Profiler* prof, const KxLayer& l, const SinkAttnParams& sp, SinkAttnKernel kern, int threads, size_t smem, int rows,
                                    int nslot_grid, int chunks_grid, bool decode, int nsplit) {
     const int rep = sp.H / sp.G;
