@@ -559,7 +559,7 @@ struct b200rwkv_engine {
     // Recurrences of prompt steps that have at most one CTA an SM: each asks for more than half an SM's shared memory, so that no two share one.  They start early
     // (programmatic launches), when most SMs are full of the projections in front of them, were packed onto the few that were not and took turns there.
     // Measured (whole prompts, four layers of width 2560): one of 200 tokens 988 -> 856 us; two layers of gated delta rule, matrix memory and attention of width 2048:
-    // one of 300 tokens 1001 -> 801; with two CTAs an SM and more nothing is gained
+    // one of 300 tokens 1001 -> 801.  Launches of more CTAs share SMs in any case and are left as they are
     bool scan_alone = false;           // of the step being enqueued
     int scan_alone_seqs = 0;           // sequences such a step holds at most: CTAs for slots beyond would wait for an SM's shared memory only to leave
     void set_scan_alone(bool prompt, int ctas_a_seq) {
