@@ -31,10 +31,39 @@ __host__ __device__ inline size_t latent_prompt_smem(int D) {
     return ((size_t)(LP_ROWS + 2 * LP_KT) * la_stride(D) + LP_ROWS * LP_SP + LP_ROWS) * sizeof(float);
 }
 
+// One row (token t at position pos, head h) worked out again by the CTA's warps, key by key, each its channels from `c0` on: see prompt_attn_row.
+__device__ __noinline__ void latent_prompt_row(const LatentPromptParams& pp, const int* tab, int h, int t, int pos, int c0, int cw) {
+    const LatentAttnParams& p = pp.a;
+    const int lane = threadIdx.x & 31, D = p.rk + p.dr;
+    const float* q = p.q + (size_t)t * p.H * D + (size_t)h * D;
+    float m = -CUDART_INF_F, l = 0.f, acc[2] = {0.f, 0.f};
+    for (int kj = 0; kj <= pos; ++kj) {
+        const float* row = p.cache + ((size_t)tab[kj / p.page] * p.page + kj % p.page) * D;
+        float dot = 0.f;
+        for (int d = lane; d < D; d += 32) dot = fmaf(__uint_as_float(to_tf32(q[d])), __uint_as_float(to_tf32(row[d])), dot);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        const float sc = dot * p.scale, mn = fmaxf(m, sc);
+        float pj = 0.f, corr = 1.f;
+        if (mn > -CUDART_INF_F) { pj = expf(sc - mn); corr = expf(m - mn); }
+        l = l * corr + pj;
+        m = mn;
+        pj = __uint_as_float(to_tf32(pj));
+        for (int e = 0; e < 2; ++e) {
+            const int ch = c0 + lane + 32 * e;
+            acc[e] = fmaf(pj, lane + 32 * e < cw && ch < p.rk ? __uint_as_float(to_tf32(row[ch])) : 0.f, acc[e] * corr);
+        }
+    }
+    for (int e = 0; e < 2; ++e) {
+        const int ch = c0 + lane + 32 * e;
+        if (lane + 32 * e < cw && ch < p.rk) pp.out[(size_t)t * p.H * p.rk + (size_t)h * p.rk + ch] = acc[e] / l;
+    }
+}
+
 __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(const __grid_constant__ LatentPromptParams pp) {
     const LatentAttnParams& p = pp.a;
     extern __shared__ __align__(16) float lp_smem[];
-    __shared__ int s_tile[2];
+    __shared__ int s_tile[2], s_again[LP_ROWS];
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
@@ -176,13 +205,24 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(const __gr
 #pragma unroll
     for (int i = 0; i < 4; ++i)
         if ((lane & 15) == 0) scorr[8 * warp + 2 * i + (lane >> 4)] = 1.f / l[i];
+    if (tid < LP_ROWS) s_again[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int rt = 0; rt < 4; ++rt)
+#pragma unroll
+        for (int hrow = 0; hrow < 2; ++hrow) {
+            float sum = 0.f;
+#pragma unroll
+            for (int n = 0; n < LP_MAX_NT; ++n) sum += o[rt][n][hrow * 2] + o[rt][n][hrow * 2 + 1];
+            if (!(fabsf(sum) < CUDART_INF_F)) s_again[rt * 16 + gq + hrow * 8] = 1;
+        }
     __syncthreads();
 #pragma unroll
     for (int rt = 0; rt < 4; ++rt)
 #pragma unroll
         for (int hrow = 0; hrow < 2; ++hrow) {
             const int r = rt * 16 + gq + hrow * 8, qi = r / HG, h = h0 + r % HG;
-            if (qi >= nt || h >= p.H) continue;
+            if (qi >= nt || h >= p.H || s_again[r]) continue;
             const float inv = scorr[r];
             float* const dst = pp.out + (size_t)(t0 + qi) * p.H * rk + (size_t)h * rk;
 #pragma unroll
@@ -194,6 +234,11 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(const __gr
                 if (d + 1 < rk) dst[d + 1] = o[rt][n][hrow * 2 + 1] * inv;
             }
         }
+    unsigned long long left = __ballot_sync(0xffffffffu, s_again[lane]) | (unsigned long long)__ballot_sync(0xffffffffu, s_again[32 + lane]) << 32;
+    for (; left; left &= left - 1) {
+        const int r = __ffsll((long long)left) - 1;
+        if (r / HG < nt && h0 + r % HG < p.H) latent_prompt_row(pp, tab, h0 + r % HG, t0 + r / HG, pos0 + r / HG, warp * cw, cw);
+    }
 }
 
 }  // namespace b200

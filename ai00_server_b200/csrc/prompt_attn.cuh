@@ -31,10 +31,44 @@ __host__ __device__ inline size_t prompt_attn_smem(int dk, int dv) {
     return ((size_t)PA_ROWS * (dk + 4) + (size_t)PA_KT * (dk + 4) + (size_t)PA_KT * (dv + 4) + (size_t)PA_ROWS * (PA_KT + 4) + 2 * PA_ROWS) * sizeof(float);
 }
 
+// One row (token t at position pos, query head h of key head c) worked out again by a warp, key by key.  A key behind a token has weight zero in the tiles above, and zero times a
+// value that is not finite is not a number: a later token of the CTA's 64 rows would reach the earlier ones.  Only rows that came out so get here.
+__device__ __noinline__ void prompt_attn_row(const SinkAttnParams& p, const float* q, const int* tbl, int c, int h, int t, int pos) {
+    const int lane = threadIdx.x & 31, d = 4 * lane, low = sa_low(p, pos);
+    int nkeep, jlo;
+    sa_segments(p, pos, pos, nkeep, jlo);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), qv = d < p.dk ? *reinterpret_cast<const float4*>(q + d) : zero;
+    float4 acc = zero;
+    float m = -CUDART_INF_F, l = 0.f;
+    for (int i = 0; i < nkeep + pos - jlo + 1; ++i) {
+        const int at = i < nkeep ? i : jlo + i - nkeep;
+        if (at > pos || (at < low && at >= p.keep)) continue;
+        const float* row = p.cache + sa_token_row(tbl, p.page, at) * (size_t)p.D;
+        const float4 k = d < p.dk ? *reinterpret_cast<const float4*>(row + p.koff + (size_t)c * p.dk + d) : zero;
+        const float4 v = d < p.dv ? *reinterpret_cast<const float4*>(row + p.voff + (size_t)c * p.dv + d) : zero;
+        float dot = fmaf(qv.x, k.x, fmaf(qv.y, k.y, fmaf(qv.z, k.z, qv.w * k.w)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        const float sc = dot * p.scale + (p.bias ? p.bias[(size_t)h * (p.nb + 1) + min(pos - at, p.nb)] : 0.f);
+        const float mn = fmaxf(m, sc), w = sc > -CUDART_INF_F ? expf(sc - mn) : 0.f, scl = m > -CUDART_INF_F ? expf(m - mn) : 0.f;
+        l = l * scl + w;
+        m = mn;
+        acc.x = fmaf(w, v.x, acc.x * scl); acc.y = fmaf(w, v.y, acc.y * scl); acc.z = fmaf(w, v.z, acc.z * scl); acc.w = fmaf(w, v.w, acc.w * scl);
+    }
+    if (d >= p.dv) return;
+    const float sk = p.sink ? p.sink[h] : -CUDART_INF_F, mx = fmaxf(m, sk), f0 = m > -CUDART_INF_F ? expf(m - mx) : 0.f;
+    const float f = f0 / (l * f0 + (p.sink ? expf(sk - mx) : 0.f));
+    const float o[4] = {acc.x * f, acc.y * f, acc.z * f, acc.w * f};
+    for (int e = 0; e < 4; ++e) {
+        const float g = p.gate ? lin_sigmoid(p.gate[(size_t)t * p.ldg + (p.gate_heads ? (size_t)h : (size_t)h * p.dv + d + e)]) : 1.f;
+        p.out[(size_t)t * p.ldo + (size_t)h * p.dv + d + e] = o[e] * g * p.out_mul;
+    }
+}
+
 __global__ void __launch_bounds__(PA_THREADS, 2) prompt_attn_kernel(const __grid_constant__ PromptAttnParams pp) {
     const SinkAttnParams& p = pp.a;
     extern __shared__ __align__(16) float pa_smem[];
-    __shared__ int s_tile[2];
+    __shared__ int s_tile[2], s_again[PA_ROWS];
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -202,7 +236,12 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prompt_attn_kernel(const __grid
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
         const int r = row_of(u);
-        if (r >= R) continue;
+        float sum = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { const float2 a = unpack2(acc[u][e]); sum += a.x + a.y; }
+        const bool again = (__ballot_sync(0xffffffffu, !(fabsf(sum) < CUDART_INF_F)) >> (16 * half) & 0xFFFFu) != 0;      // the 16 lanes of the row
+        if (vl == 0) s_again[r] = again && r < R;
+        if (r >= R || again) continue;
         const int t = t0 + r / rep, h = c * rep + r % rep;
         const float f = sScl[r];
 #pragma unroll
@@ -220,6 +259,12 @@ __global__ void __launch_bounds__(PA_THREADS, 2) prompt_attn_kernel(const __grid
             float* const dst = p.out + (size_t)t * p.ldo + (size_t)h * dv + d;
             dst[0] = o.x * p.out_mul; dst[1] = o.y * p.out_mul; dst[2] = o.z * p.out_mul; dst[3] = o.w * p.out_mul;
         }
+    }
+    __syncwarp();
+    auto warp_row = [&](int w) { return 16 * (w >> 2) + 4 * warp + (w & 3); };
+    for (unsigned left = __ballot_sync(0xffffffffu, lane < 16 && s_again[warp_row(lane & 15)]); left; left &= left - 1) {
+        const int r = warp_row(__ffs(left) - 1);
+        prompt_attn_row(p, sQ + r * PK, tbl, c, c * rep + r % rep, t0 + r / rep, pos0 + r / rep);
     }
 }
 

@@ -214,6 +214,34 @@ def test_boundaries_of_a_row_of_n_columns(width, n):
     _check_family(synth.make_panupel, [synth.panupel_layer("delta", heads=2, dim=24, ff=48)], panupel_numpy, n, width=width)
 
 
+@pytest.mark.parametrize("family, precision", [("kemirax", 0), ("panupel", 0), ("panupel", 1)])
+def test_a_token_that_is_not_a_number_reaches_no_row_before_it(family, precision):
+    """Attention works on 64 rows of neighbouring tokens at a time: a later token's value has weight zero in the earlier ones, and zero times NaN must not count."""
+    if family == "kemirax":
+        layers, make, module = [synth.kemirax_layer("latent_attention", heads=4, mlp=False)], synth.make_kemirax, kemirax_numpy
+        cfg, st, w = make(layers, seed=4)
+    else:
+        layers, make, module = [synth.panupel_layer("parallel", heads=4, kv_heads=2, dim=24, mm_heads=2, mm_dim=24)], synth.make_panupel, panupel_numpy
+        cfg, st, w = make(layers, seed=4, width=96, loop=None)
+    toks = np.random.default_rng(3).integers(10, 90, 31).tolist()
+    toks[20] = 7
+    st = st.copy()
+    head = int(st[:8].view("<u8")[0])
+    e = json.loads(bytes(st[8:8 + head]))["embed"]
+    rows = st[8 + head + e["data_offsets"][0]:8 + head + e["data_offsets"][1]].reshape(e["shape"][0], -1)
+    rows[7] = np.full(rows.shape[1] // 2, 0x7fc0, "<u2").view(np.uint8)
+    m = runtime.Model(st, max_batch=1, token_chunk_size=64, config=cfg, kv_tokens=64, kv_page=16, precision=precision)
+    try:
+        m.state.reset(0)
+        got = m.infer_raw([0], [31], toks, [capi.OPTION_FULL])[0]
+        assert np.isnan(got[20:]).all() and np.isfinite(got[:20]).all(), np.isfinite(got).all(1).tolist()
+        want = module.run(json.loads(cfg), w, toks[:20])
+        err = np.sqrt(((got[:20] - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean())
+        assert np.median(err) <= (BF16_TOL if precision == 0 else 2e-4) and err.max() <= (ROW_TOL if precision == 0 else 2e-4), err.tolist()
+    finally:
+        m.close()
+
+
 def test_a_nan_stays_one_in_latent_attention():
     """A key that is not a number makes every later row so (rounding to TF32 by integer arithmetic must not turn it into a number)."""
     cfg, st, _ = synth.make_kemirax([synth.kemirax_layer("latent_attention", mlp=False)], seed=4)
