@@ -1,38 +1,88 @@
-// Softmax attention of prompt steps over the paged cache: the function of sink_attn.cuh (windows, chunks of the sequence, kept first tokens, a bias per
-// distance, a sink term, a gate; no block means), in f32 throughout, for steps whose keys are not split: enough tokens to fill the chip, or
-// contexts of one key tile of 32 (kx_fill_step).
+// Softmax attention of prompt steps over the paged cache on the tensor cores: the function of sink_attn.cuh (windows, chunks of the sequence, kept first tokens, a bias per
+// distance, a sink term, a gate; no block means), for steps whose keys are not split: enough tokens to fill the chip, or contexts of one key tile of 32 (kx_fill_step).
 //
-// What bounds it: f32 multiply-adds, 2 dk + 2 dv a (query head, key).  The register form reads every key row from L2 for four (token, head) rows at a
-// time and spends as many exchanges between lanes as products; here a CTA of four warps keeps 64 rows -- the query heads of ONE key / value head for 64 / rep
-// consecutive tokens of one sequence -- and walks the keys in tiles of 32 that it stages once for all of them:
-//   * scores   a thread owns 4 rows x 4 keys (rows and keys interleaved, so that the 16-byte reads of eight lanes fall into different banks): eight
-//              reads for 64 products;
-//   * softmax  running maximum and sum per row in the eight lanes that share it; the weights go through shared memory within the warp;
-//   * values   a thread owns 8 rows x 8 entries of the output: 12 reads for 256 products;
-//   * products run as packed pairs (fma.rn.f32x2), even and odd entries of a score summed apart;
-//   * the next key tile arrives (cp.async) while the values are multiplied, the next value tile while the scores are.
-// Measured (width 2048, 16 sequences, 2048 tokens a step): 280 -> 126 us at 128 tokens of context (ncu); 16 prompts of 1024 tokens 32.5 -> 23.3 ms.
-// Where the line lies, whole prompts of two layers with the register form and with this one, width 2048: 1 x 20 tokens 270 and 233 us, 16 x 32 501 and 453, 1 x 600 1181 and 1076;
-// width 512: 1 x 20 165 and 159, 2 x 20 167 and 161, 16 x 32 239 and 231.
+// Queries, keys, values and weights are f32 and stay it: each number travels as three bf16 parts (the first two rounded to nearest, the third takes what is left: 24 bits),
+// and a product of two numbers is the six products of parts down to 2^-16 of the first; what is left out is 2^-24 of a product.  The small products are summed first, so
+// that eight additions of a score and four of a tile's read-out happen at full size; read-outs of a tile are added to the row in f32 registers.
+//
+// What bounds it: the tensor core, six times the products of a bf16 kernel (f32 multiply-adds, the form before, take 128 a cycle and SM; these 4096 / 6).  A CTA keeps
+// 128 rows -- the query heads of ONE key / value head for 128 / rep consecutive tokens of a sequence -- and walks the keys in tiles of 64:
+//   * queries  live in tensor memory (three parts of 64 columns), so that a score MMA reads only the key tile from shared memory;
+//   * keys and values   are split by four warps each on the way into shared memory, [eight channels][64 keys][16 bytes]: one layout is the K-major operand of the
+//              scores and the MN-major operand of the values;
+//   * scores   S = Q K^T, 64 columns of tensor memory; eight warps take half a row each a thread, exchange maxima, and write the weights back as three parts;
+//   * values   O = P V, a fresh accumulator every tile, added to the rows' registers one tile later;
+//   * one thread issues: the scores of tile t + 1 are multiplied while the softmax of tile t runs, the values of tile t while that of t + 1 does; seven warps split the
+//              tiles ahead of it (16 of eight keys a tile, dealt out), two buffers each for keys and values.
+// Measured (16 sequences of 128 tokens, 16 query heads on 4 key heads of 128 channels, in f32 multiply-adds before and here): 113 -> 36 us at 128 tokens of context, 454 -> 82 at
+// 576, 805 -> 130 at 1024; one prompt of 1000 tokens 376 -> 63, of 20 tokens 25 -> 15; 16 prompts of 1024 tokens, four layers
+// of width 2048, 22.1 -> 15.9 ms.  Distance from 64 bits (2-norm): 6.2e-7 -> 3.0e-7 at 1024 tokens, 1.42e-6 -> 3.5e-7 at 6000, 1.6e-7 -> 1.4e-7 at 20.
+// Slower than before only where most rows are empty and the context is one tile: 64 sequences of 32 tokens, one query head a key head: 87 -> 89 us of 128 channels, 64 -> 80 of 32.
 #pragma once
-#include "f32x2.cuh"
+#include <cuda_bf16.h>
+
+#include "linear_umma.cuh"
 #include "sink_attn.cuh"
 
 namespace b200 {
 
-constexpr int PA_ROWS = 64, PA_KT = 32, PA_THREADS = 128, PA_DMAX = 128;
+constexpr int PT_ROWS = 128, PT_KT = 64, PT_DMAX = 128;
+constexpr int PT_SOFT = 256, PT_CONV_WARPS = 7, PT_THREADS = PT_SOFT + 32 * PT_CONV_WARPS + 32;      // sixteen warps: 128 registers a thread
+// tensor memory: queries (3 x 64 columns), scores, weights (3 x 32), read-outs of a tile
+constexpr uint32_t PT_TQ = 0, PT_TS = 192, PT_TP = 256, PT_TO = 352, PT_TMEM_COLS = 512;
 
 struct PromptAttnParams {
     SinkAttnParams a;
-    int qt;                        // tokens of a CTA: PA_ROWS / (query heads of a key head)
+    int qt;                        // tokens of a CTA: PT_ROWS / (query heads of a key head)
 };
 
+__host__ __device__ inline int pt_up16(int d) { return (d + 15) & ~15; }
+// two key tiles and two value tiles in three parts, later the finished rows
 __host__ __device__ inline size_t prompt_attn_smem(int dk, int dv) {
-    return ((size_t)PA_ROWS * (dk + 4) + (size_t)PA_KT * (dk + 4) + (size_t)PA_KT * (dv + 4) + (size_t)PA_ROWS * (PA_KT + 4) + 2 * PA_ROWS) * sizeof(float);
+    const size_t tiles = (size_t)2 * 3 * PT_KT * 2 * (pt_up16(dk) + pt_up16(dv)), out = (size_t)PT_ROWS * (pt_up16(dv) + 4) * 4;
+    return (tiles > out ? tiles : out) + 128;
 }
 
-// One row (token t at position pos, query head h of key head c) worked out again by a warp, key by key.  A key behind a token has weight zero in the tiles above, and zero times a
-// value that is not finite is not a number: a later token of the CTA's 64 rows would reach the earlier ones.  Only rows that came out so get here.
+// shared memory only: the general form also waits for the global loads in flight (the next keys)
+__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// (a, b) -> packed bf16, and what it leaves of them
+__device__ __forceinline__ uint32_t pt_take(float& a, float& b) {
+    const uint32_t h = pack_bf16x2(make_float2(a, b));
+    a -= __uint_as_float(h << 16);
+    b -= __uint_as_float(h & 0xFFFF0000u);
+    return h;
+}
+
+// eight neighbouring numbers, zeros from `left` on (a multiple of four).  WHOLE: `left` is a multiple of eight and the address one of 32 bytes: one access of a whole sector a
+// lane (two of 16 bytes, each half of 32 sectors, took 150 us where this takes 130: 16 sequences, contexts of 1024)
+template <bool WHOLE>
+__device__ __forceinline__ void pt_load8(float (&v)[8], const float* src, const int left) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0.f;
+    if constexpr (WHOLE) {
+        if (left <= 0) return;
+        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                     : "l"(src));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+            const float4 x = i < left ? *reinterpret_cast<const float4*>(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+        }
+    }
+}
+
+// eight numbers -> the 16 bytes of each part
+__device__ __forceinline__ void pt_split8(float (&v)[8], uint4 (&part)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) part[i] = make_uint4(pt_take(v[0], v[1]), pt_take(v[2], v[3]), pt_take(v[4], v[5]), pt_take(v[6], v[7]));
+}
+
+// One row (token t at position pos, query head h of key head c) worked out again by a warp, key by key.  A key behind a token has weight zero in the tiles below, and zero times a
+// value that is not finite is not a number: a later token of the CTA's rows would reach the earlier ones; and parts of a number that is not finite are not numbers.  Only
+// rows that came out so get here.
 __device__ __noinline__ void prompt_attn_row(const SinkAttnParams& p, const float* q, const int* tbl, int c, int h, int t, int pos) {
     const int lane = threadIdx.x & 31, d = 4 * lane, low = sa_low(p, pos);
     int nkeep, jlo;
@@ -65,207 +115,307 @@ __device__ __noinline__ void prompt_attn_row(const SinkAttnParams& p, const floa
     }
 }
 
-__global__ void __launch_bounds__(PA_THREADS, 2) prompt_attn_kernel(const __grid_constant__ PromptAttnParams pp) {
+// RUNS: runs of eight channels of keys and values (16), 0: any.  WHOLE: sizes, strides and offsets are multiples of eight floats
+template <int RUNS, bool WHOLE>
+__global__ void __launch_bounds__(PT_THREADS, 1) prompt_attn_kernel(const __grid_constant__ PromptAttnParams pp) {
     const SinkAttnParams& p = pp.a;
-    extern __shared__ __align__(16) float pa_smem[];
-    __shared__ int s_tile[2], s_again[PA_ROWS];
-    pdl_launch_dependents();
-    pdl_wait();
+    extern __shared__ __align__(16) uint8_t pt_smem_raw[];
+    __shared__ int s_tile[2], s_again[PT_ROWS], s_hi[PT_ROWS], s_lo[PT_ROWS], s_kept[PT_ROWS];
+    __shared__ float s_max[2][2][PT_ROWS], s_sum[PT_ROWS], s_gate[PT_ROWS];
+    __shared__ int s_off[PT_ROWS];
+    __shared__ __align__(8) unsigned long long s_bar[13];
+    __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == 0) step_token_run(p.meta, pp.qt, blockIdx.x, s_tile);
+    const uint32_t bar = smem_u32(s_bar);
+    // (key and value tiles have two buffers)
+    const uint32_t b_q = bar, b_kfull = bar + 8, b_kfree = bar + 24, b_vfull = bar + 40, b_vfree = bar + 56, b_sfull = bar + 72, b_sfree = bar + 80, b_pfull = bar + 88,
+                   b_ofull = bar + 96;
+    if (tid == 0) {
+        mbar_init(b_q, PT_SOFT / 32);
+        for (int i = 0; i < 16; i += 8) {
+            mbar_init(b_kfull + i, PT_KT / 8); mbar_init(b_kfree + i, 1);
+            mbar_init(b_vfull + i, PT_KT / 8); mbar_init(b_vfree + i, 1);
+        }
+        mbar_init(b_sfull, 1); mbar_init(b_sfree, PT_SOFT / 32);
+        mbar_init(b_pfull, PT_SOFT / 32); mbar_init(b_ofull, 1);
+        mbar_fence_init();
+    }
+    if (warp == PT_THREADS / 32 - 1) tc_alloc(smem_u32(&s_tmem), PT_TMEM_COLS);
+    if (tid < PT_ROWS) s_again[tid] = 0;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&s_tmem);
+    pdl_launch_dependents();                                // behind the allocation: see linear_umma.cuh
+    pdl_wait();
+    // later tokens have more keys: they start first
+    if (warp == 0) step_token_run(p.meta, pp.qt, gridDim.x - 1 - blockIdx.x, s_tile);
     __syncthreads();
     const int si = s_tile[0];
-    if (si < 0) return;
-    const int first = s_tile[1] * pp.qt, nq = min(pp.qt, p.meta.slot_count()[si] - first), t0 = p.meta.slot_start()[si] + first;
-    const int slot = p.meta.slot_id()[si], pos0 = p.sm.tok_pos()[t0], pos1 = pos0 + nq - 1;
-    const int dk = p.dk, dv = p.dv, rep = p.H / p.G, c = blockIdx.y, R = nq * rep, D = p.D;
-    const int PK = dk + 4, PV = dv + 4, PP = PA_KT + 4;
-    float* const sQ = pa_smem;                             // [64][dk + 4]
-    float* const sK = sQ + PA_ROWS * PK;                   // [32][dk + 4]
-    float* const sV = sK + PA_KT * PK;                     // [32][dv + 4]
-    float* const sP = sV + PA_KT * PV;                     // [64][36]
-    float* const sScl = sP + PA_ROWS * PP;                 // [64] rescaling of a row, later 1 / denominator
-    const int* const tbl = p.table + (size_t)slot * p.stride;
-    int nkeep, jlo;
-    sa_segments(p, pos0, pos1, nkeep, jlo);
-    const int nkeys = nkeep + pos1 - jlo + 1, ntiles = (nkeys + PA_KT - 1) / PA_KT;
-    auto position = [&](int i) { return i < nkeep ? i : jlo + i - nkeep; };        // kept tokens first, then the window
-    // a warp loads the rows 8 warp .. 8 warp + 7 of a tile; rows behind the last key hold the last one's values (their weights are zero)
-    auto load = [&](float* dst, const int pitch, const int n4, const size_t off, const int ti) {
-#pragma unroll 1
-        for (int r = warp * (PA_KT / 4); r < (warp + 1) * (PA_KT / 4); ++r) {
-            const float* src = p.cache + sa_token_row(tbl, p.page, position(min(ti * PA_KT + r, nkeys - 1))) * (size_t)D + off;
-            for (int q = lane; q < n4; q += 32) cp_async16(dst + r * pitch + 4 * q, src + 4 * q);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    const size_t koff = (size_t)p.koff + (size_t)c * dk, voff = (size_t)p.voff + (size_t)c * dv;
-    load(sK, PK, dk / 4, koff, 0);
-    load(sV, PV, dv / 4, voff, 0);
-    for (int i = tid; i < PA_ROWS * (dk / 4); i += PA_THREADS) {
-        const int r = i / (dk / 4), q = i - r * (dk / 4);
-        *reinterpret_cast<float4*>(sQ + r * PK + 4 * q) =
-            r < R ? *reinterpret_cast<const float4*>(p.q + (size_t)(t0 + r / rep) * p.ldq + (size_t)(c * rep + r % rep) * dk + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    // scores: rows 16 i + 4 warp + rg (i < 4), keys 8 j + kg (j < 4)
-    const int rg = lane >> 3, kg = lane & 7;
-    float m[4], l[4];
-    int pq[4];
-    const float* bias[4];
+    if (si >= 0) {
+        const int first = s_tile[1] * pp.qt, nq = min(pp.qt, p.meta.slot_count()[si] - first), t0 = p.meta.slot_start()[si] + first;
+        const int slot = p.meta.slot_id()[si], pos0 = p.sm.tok_pos()[t0], pos1 = pos0 + nq - 1;
+        const int dk = RUNS ? 8 * RUNS : p.dk, dv = RUNS ? 8 * RUNS : p.dv, rep = p.H / p.G, c = blockIdx.y, R = nq * rep, D = p.D;
+        const int nck = RUNS ? RUNS : pt_up16(dk) / 8, ncv = RUNS ? RUNS : pt_up16(dv) / 8;      // runs of eight channels
+        const uint32_t raw = smem_u32(pt_smem_raw), tiles = (raw + 127u) & ~127u;
+        uint8_t* const sK = pt_smem_raw + (tiles - raw);                     // [2 tiles][3 parts][runs][64 keys][16 bytes]
+        uint8_t* const sV = sK + (size_t)6 * nck * PT_KT * 16;
+        const int* const tbl = p.table + (size_t)slot * p.stride;
+        int nkeep, jlo;
+        sa_segments(p, pos0, pos1, nkeep, jlo);
+        const int nkeys = nkeep + pos1 - jlo + 1, ntiles = (nkeys + PT_KT - 1) / PT_KT;
+        auto position = [&](int i) { return i < nkeep ? i : jlo + i - nkeep; };      // kept tokens first, then the window
+
+        if (warp == PT_THREADS / 32 - 1) {
+            // ===================== MMA issuer: one lane =====================
+            if (lane == 0) {
+                const uint32_t IDESC_S = umma_idesc_bf16(PT_ROWS, PT_KT), IDESC_O = umma_idesc_bf16(PT_ROWS, 8 * ncv) | (1u << 16);      // values: N contiguous
+                constexpr uint32_t RUN = PT_KT * 16;         // bytes between runs of eight channels
+                // a descriptor's address field counts 16 bytes and sits in its low half: operands further on are sums there
+                const uint64_t dk0 = umma_desc(tiles, RUN, 128), dv0 = umma_desc(tiles + 6 * nck * RUN, 128, RUN);
+                auto at = [](const uint64_t d, const uint32_t off) { return (d & 0xFFFFFFFF00000000ull) | ((uint32_t)d + off); };
+                constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};      // parts of a product, the smallest first
+                const uint32_t kpart = nck * (RUN / 16), vpart = ncv * (RUN / 16);
+                auto values = [&](const int t) {
+                    const int b = t & 1;
+                    mbar_wait(b_vfull + 8 * b, (t >> 1) & 1, 41);
+                    mbar_wait(b_pfull, b, 42);
+                    tc_fence_after();
+                    const uint64_t d0 = at(dv0, 3 * b * vpart), dp[3] = {d0, at(d0, vpart), at(d0, 2 * vpart)};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = 16 * i + 4 * warp + rg;
-        m[i] = -CUDART_INF_F; l[i] = 0.f;
-        pq[i] = r < R ? pos0 + r / rep : -1;               // rows beyond the last see nothing
-        bias[i] = p.bias && r < R ? p.bias + (size_t)(c * rep + r % rep) * (p.nb + 1) : nullptr;
-    }
-    // values: the warp's rows in the same order, eight a half warp (local row 2 u + half of 16), entries 4 vl .. and 64 + 4 vl ..
-    const int half = lane >> 4, vl = lane & 15;
-    f32x2 acc[8][4];
+                    for (int i = 0; i < 6; ++i)
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+                        for (int k = 0; k < PT_KT / 16; ++k)
+                            tc_mma_f16_ts(tmem + PT_TO, tmem + PT_TP + PA[i] * 32 + k * 8, at(dp[PB[i]], k * 16), IDESC_O, i + k > 0);
+                    if (t + 2 < ntiles) tc_commit(b_vfree + 8 * b);
+                    tc_commit(b_ofull);
+                };
+                mbar_wait(b_q, 0, 43);
+                for (int t = 0; t < ntiles; ++t) {
+                    const int b = t & 1;
+                    mbar_wait(b_kfull + 8 * b, (t >> 1) & 1, 44);
+                    if (t > 0) mbar_wait(b_sfree, (t - 1) & 1, 45);
+                    tc_fence_after();
+                    const uint64_t d0 = at(dk0, 3 * b * kpart), dp[3] = {d0, at(d0, kpart), at(d0, 2 * kpart)};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[u][e] = 0ull;
-    auto row_of = [&](int u) { const int w = 2 * u + half; return 16 * (w >> 2) + 4 * warp + (w & 3); };
-    const bool v0 = 4 * vl < dv, v1 = 64 + 4 * vl < dv;
-    for (int ti = 0; ti < ntiles; ++ti) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");        // the key tile
-        __syncthreads();
-        f32x2 s2[4][4];
+                    for (int i = 0; i < 6; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
-        {
-            const float* qp = sQ + (4 * warp + rg) * PK;
-            const float* kp = sK + kg * PK;
-#pragma unroll 4
-            for (int d = 0; d < dk; d += 4) {
-                ulonglong2 q[4], k[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const ulonglong2*>(qp + i * 16 * PK + d);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(kp + j * 8 * PK + d);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        fma2(s2[i][j], q[i].x, k[j].x);
-                        fma2(s2[i][j], q[i].y, k[j].y);
-                    }
+                        for (int k = 0; k < PT_DMAX / 16; ++k)
+                            if (2 * k < nck) tc_mma_f16_ts(tmem + PT_TS, tmem + PT_TQ + PA[i] * 64 + k * 8, at(dp[PB[i]], 2 * k * (RUN / 16)), IDESC_S, i + k > 0);
+                    if (t + 2 < ntiles) tc_commit(b_kfree + 8 * b);
+                    tc_commit(b_sfull);
+                    if (t > 0) values(t - 1);
+                }
+                values(ntiles - 1);
             }
-        }
-        __syncthreads();                                    // every warp is done with the key tile
-        if (ti + 1 < ntiles) load(sK, PK, dk / 4, koff, ti + 1);
-        else asm volatile("cp.async.commit_group;" ::: "memory");
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int low = sa_low(p, pq[i]), r = 16 * i + 4 * warp + rg;
-            float s[4], tmax = -CUDART_INF_F;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int idx = ti * PA_KT + 8 * j + kg, at = position(idx);
-                const float2 h = unpack2(s2[i][j]);
-                const bool vis = idx < nkeys && at <= pq[i] && (at >= low || at < p.keep);
-                s[j] = vis ? (h.x + h.y) * p.scale + (bias[i] ? bias[i][min(pq[i] - at, p.nb)] : 0.f) : -CUDART_INF_F;
-                tmax = fmaxf(tmax, s[j]);
-            }
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 4));
-            const float mn = fmaxf(m[i], tmax);
-            const float scl = m[i] > -CUDART_INF_F ? expf(m[i] - mn) : 0.f;
-            float tsum = 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float w = s[j] > -CUDART_INF_F ? expf(s[j] - mn) : 0.f;
-                sP[r * PP + 8 * j + kg] = w;
-                tsum += w;
-            }
-            tsum += __shfl_xor_sync(0xffffffffu, tsum, 1);
-            tsum += __shfl_xor_sync(0xffffffffu, tsum, 2);
-            tsum += __shfl_xor_sync(0xffffffffu, tsum, 4);
-            l[i] = l[i] * scl + tsum;
-            m[i] = mn;
-            if (kg == 0) sScl[r] = scl;
-        }
-        __syncwarp();                                       // rows of the weights belong to one warp
-        asm volatile("cp.async.wait_group 1;" ::: "memory");        // the value tile
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const float f = sScl[row_of(u)];
-            const f32x2 f2 = pack2(f, f);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) mul2(acc[u][e], f2);
-        }
-#pragma unroll 2
-        for (int k = 0; k < PA_KT; k += 4) {
-            ulonglong2 va[4], vb[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                va[q] = v0 ? *reinterpret_cast<const ulonglong2*>(sV + (k + q) * PV + 4 * vl) : make_ulonglong2(0, 0);
-                vb[q] = v1 ? *reinterpret_cast<const ulonglong2*>(sV + (k + q) * PV + 64 + 4 * vl) : make_ulonglong2(0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float4 w = *reinterpret_cast<const float4*>(sP + row_of(u) * PP + k);
-                const f32x2 w2[4] = {pack2(w.x, w.x), pack2(w.y, w.y), pack2(w.z, w.z), pack2(w.w, w.w)};
+        } else if (warp >= PT_SOFT / 32) {
+            // ===================== f32 rows of the cache -> three bf16 parts: eight keys of a key or value tile at a time, dealt out among the warps =====================
+            const int k8 = lane & 7, cq = lane >> 3;         // a key of the eight, every fourth run of eight channels
+            const float* const base = p.cache + (size_t)c * dk + p.koff;
+            const ptrdiff_t vgap = (ptrdiff_t)p.voff + (size_t)c * dv - ((ptrdiff_t)p.koff + (size_t)c * dk);
+            // rows behind the last key hold the last one's values (their weights are zero)
+            auto locate = [&](const int n) {
+                return base + (n & 8 ? vgap : 0) + sa_token_row(tbl, p.page, position(min((n >> 4) * PT_KT + (n & 7) * 8 + k8, nkeys - 1))) * (size_t)D;
+            };
+            auto fetch = [&](const int n, const float* const src, float (&x)[4][8]) {
+                const int d = n & 8 ? dv : dk;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    fma2(acc[u][0], w2[q], va[q].x); fma2(acc[u][1], w2[q], va[q].y);
-                    fma2(acc[u][2], w2[q], vb[q].x); fma2(acc[u][3], w2[q], vb[q].y);
+                    const int ch = 8 * (4 * q + cq);
+                    pt_load8<WHOLE>(x[q], src + ch, d - ch);
+                }
+            };
+            auto store = [&](const int n, float (&x)[4][8]) {
+                const bool isv = n & 8;
+                const int t = n >> 4, b = t & 1, nc = isv ? ncv : nck;
+                if (t > 1) mbar_wait((isv ? b_vfree : b_kfree) + 8 * b, ((t >> 1) - 1) & 1, 46);
+                uint8_t* const to = (isv ? sV : sK) + (size_t)b * 3 * nc * (PT_KT * 16) + ((n & 7) * 8 + k8) * 16;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int run = 4 * q + cq;
+                    if (run >= nc) continue;
+                    uint4 part[3];
+                    pt_split8(x[q], part);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(to + (size_t)(i * nc + run) * (PT_KT * 16)) = part[i];
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive((isv ? b_vfull : b_kfull) + 8 * b);
+            };
+            const int total = 16 * ntiles;
+            int n = warp - PT_SOFT / 32;
+            float x0[4][8], x1[4][8];
+            fetch(n, locate(n), x0);                         // (there are sixteen at least)
+            const float* src = locate(n + PT_CONV_WARPS);
+            // the next eight keys are on their way while these are split, the page of those behind them is being looked up
+            for (; n < total; n += 2 * PT_CONV_WARPS) {
+                const int n1 = n + PT_CONV_WARPS, n2 = n + 2 * PT_CONV_WARPS;
+                if (n1 < total) fetch(n1, src, x1);
+                src = locate(n2);
+                store(n, x0);
+                if (n2 < total) fetch(n2, src, x0);
+                src = locate(n2 + PT_CONV_WARPS);
+                if (n1 < total) store(n1, x1);
+            }
+        } else {
+            // ===================== softmax: thread = (row, half of the tile's keys, half of the output's channels) =====================
+            const int half = warp >> 2, row = tid & (PT_ROWS - 1);
+            const uint32_t tm = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+            {
+                const bool in = row < R;
+                const int tq = row / rep, h = c * rep + row - tq * rep;
+                // Key idx of the walk is visible if idx <= hi and (idx >= lo or idx < kept): the row's own position and window in the walk's count (rows beyond the last see
+                // nothing; the kept tokens lie before every row's window).  In shared memory: the loop below has no registers to spare; either half writes the same
+                const int pq = in ? pos0 + tq : -1, shift = jlo - nkeep;
+                s_hi[row] = pq - shift; s_lo[row] = sa_low(p, pq) - shift; s_kept[row] = max(p.keep - shift, nkeep);
+                s_off[row] = in ? (t0 + tq) * p.ldo + h * dv : -1;
+                s_gate[row] = in && p.gate && p.gate_heads ? p.gate[(size_t)(t0 + tq) * p.ldg + h] : 0.f;
+                const float* const qrow = p.q + (size_t)(t0 + tq) * p.ldq + (size_t)h * dk;
+                float v[8][8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int d = 64 * half + 8 * i;
+                    pt_load8<WHOLE>(v[i], qrow + d, in ? dk - d : 0);
+                }
+#pragma unroll
+                for (int part = 0; part < 3; ++part)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {            // 32 channels: 16 columns of the part
+                        uint32_t r[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) r[i] = pt_take(v[4 * e + i / 4][2 * (i & 3)], v[4 * e + i / 4][2 * (i & 3) + 1]);
+                        tc_st16(tm + PT_TQ + part * 64 + half * 32 + e * 16, r);
+                    }
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(b_q);
+            }
+            const int low1 = sa_low(p, pos1);
+            float m = -CUDART_INF_F, l = 0.f, scl = 0.f;
+            float o[64];
+#pragma unroll
+            for (int i = 0; i < 64; ++i) o[i] = 0.f;
+            auto add_tile = [&]() {                          // read-outs of a finished tile, whose rescaling of the row is `scl`
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (64 * half + 16 * q >= 8 * ncv) break;
+                    float v[16];
+                    tc_ld16(tm + PT_TO + 64 * half + 16 * q, v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[16 * q + i] = fmaf(o[16 * q + i], scl, v[i]);
+                }
+            };
+            for (int t = 0; t < ntiles; ++t) {
+                mbar_wait(b_sfull, t & 1, 48);
+                tc_fence_after();
+                float s[32];
+                tc_ld32(tm + PT_TS + 32 * half, s);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(b_sfree);
+                // does every row see every key of the tile?
+                const int i0 = t * PT_KT, a0 = position(i0), a1 = position(i0 + PT_KT - 1);
+                float mx = -CUDART_INF_F;
+                if (i0 + PT_KT <= nkeys && i0 >= nkeep && a1 <= pos0 && a0 >= low1 && !p.bias) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) { s[j] *= p.scale; mx = fmaxf(mx, s[j]); }
+                } else {
+                    const int i1 = i0 + 32 * half, hj = s_hi[row] - i1, lj = s_lo[row] - i1, kj = s_kept[row] - i1;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const bool vis = j <= hj && (j >= lj || j < kj);
+                        s[j] = vis ? s[j] * p.scale : -CUDART_INF_F;
+                    }
+                    if (p.bias && row < R) {
+                        const float* const bias = p.bias + (size_t)(c * rep + row % rep) * (p.nb + 1);
+                        const int pq = pos0 + row / rep;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) s[j] += bias[min(max(pq - position(i1 + j), 0), p.nb)];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) mx = fmaxf(mx, s[j]);
+                }
+                s_max[t & 1][half][row] = mx;
+                named_bar_sync(1, PT_SOFT);
+                const float mn = fmaxf(m, fmaxf(mx, s_max[t & 1][half ^ 1][row])), ref = mn > -CUDART_INF_F ? mn : 0.f;
+                const float now = m > -CUDART_INF_F ? expf(m - mn) : 0.f;
+                float sum = 0.f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) { s[j] = expf(s[j] - ref); sum += s[j]; }
+                l = l * now + sum;
+                m = mn;
+                uint32_t r[3][16];
+#pragma unroll
+                for (int part = 0; part < 3; ++part)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) r[part][i] = pt_take(s[2 * i], s[2 * i + 1]);
+                if (t > 0) {                                 // the MMAs of tile t - 1 have read its weights
+                    mbar_wait(b_ofull, (t - 1) & 1, 47);
+                    tc_fence_after();
+                }
+#pragma unroll
+                for (int part = 0; part < 3; ++part) tc_st16(tm + PT_TP + part * 32 + half * 16, r[part]);
+                if (t > 0) add_tile();
+                scl = now;
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(b_pfull);
+            }
+            mbar_wait(b_ofull, (ntiles - 1) & 1, 47);
+            tc_fence_after();
+            add_tile();
+            // both halves' sums; the sink joins the denominator.  Every MMA has completed: the tiles' memory takes the rows
+            if (half == 1) s_sum[row] = l;
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < 64; ++i) sum += o[i];
+            const bool in = row < R;
+            if (in && !(fabsf(sum) < CUDART_INF_F)) s_again[row] = 1;
+            named_bar_sync(1, PT_SOFT);
+            if (half == 0) {
+                l += s_sum[row];
+                const float sk = p.sink && in ? p.sink[c * rep + row % rep] : -CUDART_INF_F, mx = fmaxf(m, sk), f = m > -CUDART_INF_F ? expf(m - mx) : 0.f;
+                s_sum[row] = f / (l * f + (p.sink ? expf(sk - mx) : 0.f)) * (p.gate && p.gate_heads ? lin_sigmoid(s_gate[row]) : 1.f);
+                if (in && !(l < CUDART_INF_F)) s_again[row] = 1;
+            }
+            float* const out = reinterpret_cast<float*>(sK);
+            const int pitch = 8 * ncv + 4;
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+                if (64 * half + 4 * q < 8 * ncv) *reinterpret_cast<float4*>(out + row * pitch + 64 * half + 4 * q) = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+            named_bar_sync(1, PT_SOFT);
+            const float mul = p.out_mul;
+            if (p.gate == nullptr || p.gate_heads) {
+#pragma unroll 4
+                for (int r = warp; r < PT_ROWS; r += 8) {
+                    const int off = s_again[r] ? -1 : s_off[r];
+                    const float f = s_sum[r];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int d = 32 * q + lane;
+                        if (off >= 0 && d < dv) p.out[off + d] = out[r * pitch + d] * f * mul;
+                    }
+                }
+            } else {
+                for (int r = warp; r < R; r += 8) {
+                    if (s_again[r]) continue;
+                    const float* const g = p.gate + (size_t)(t0 + r / rep) * p.ldg + (size_t)(c * rep + r % rep) * dv;
+                    for (int d = lane; d < dv; d += 32) p.out[s_off[r] + d] = out[r * pitch + d] * s_sum[r] * lin_sigmoid(g[d]) * mul;
                 }
             }
-        }
-        __syncthreads();                                    // every warp is done with the value tile
-        if (ti + 1 < ntiles) load(sV, PV, dv / 4, voff, ti + 1);
-        else asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    // the sink joins the denominator
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = 16 * i + 4 * warp + rg;
-        if (kg == 0 && r < R) {
-            const float sk = p.sink ? p.sink[c * rep + r % rep] : -CUDART_INF_F, mx = fmaxf(m[i], sk);
-            const float f = m[i] > -CUDART_INF_F ? expf(m[i] - mx) : 0.f;
-            sScl[r] = f / (l[i] * f + (p.sink ? expf(sk - mx) : 0.f));
-        }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int r = row_of(u);
-        float sum = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { const float2 a = unpack2(acc[u][e]); sum += a.x + a.y; }
-        const bool again = (__ballot_sync(0xffffffffu, !(fabsf(sum) < CUDART_INF_F)) >> (16 * half) & 0xFFFFu) != 0;      // the 16 lanes of the row
-        if (vl == 0) s_again[r] = again && r < R;
-        if (r >= R || again) continue;
-        const int t = t0 + r / rep, h = c * rep + r % rep;
-        const float f = sScl[r];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int d = 64 * e + 4 * vl;
-            if (d >= dv) continue;
-            const float2 a = unpack2(acc[u][2 * e]), b = unpack2(acc[u][2 * e + 1]);
-            float4 o = make_float4(a.x * f, a.y * f, b.x * f, b.y * f);
-            if (p.gate) {
-                const float* g = p.gate + (size_t)t * p.ldg + (p.gate_heads ? (size_t)h : (size_t)h * dv + d);
-                const float g0 = lin_sigmoid(g[0]);
-                o.x *= g0;
-                o.y *= p.gate_heads ? g0 : lin_sigmoid(g[1]); o.z *= p.gate_heads ? g0 : lin_sigmoid(g[2]); o.w *= p.gate_heads ? g0 : lin_sigmoid(g[3]);
+            for (unsigned left = __ballot_sync(0xffffffffu, lane < PT_ROWS / 8 && s_again[warp + 8 * (lane & 15)]); left; left &= left - 1) {
+                const int r = warp + 8 * (__ffs(left) - 1), t = t0 + r / rep, hr = c * rep + r % rep;
+                prompt_attn_row(p, p.q + (size_t)t * p.ldq + (size_t)hr * dk, tbl, c, hr, t, pos0 + r / rep);
             }
-            float* const dst = p.out + (size_t)t * p.ldo + (size_t)h * dv + d;
-            dst[0] = o.x * p.out_mul; dst[1] = o.y * p.out_mul; dst[2] = o.z * p.out_mul; dst[3] = o.w * p.out_mul;
         }
     }
-    __syncwarp();
-    auto warp_row = [&](int w) { return 16 * (w >> 2) + 4 * warp + (w & 3); };
-    for (unsigned left = __ballot_sync(0xffffffffu, lane < 16 && s_again[warp_row(lane & 15)]); left; left &= left - 1) {
-        const int r = warp_row(__ffs(left) - 1);
-        prompt_attn_row(p, sQ + r * PK, tbl, c, c * rep + r % rep, t0 + r / rep, pos0 + r / rep);
-    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == PT_THREADS / 32 - 1) tc_dealloc(tmem, PT_TMEM_COLS);
 }
 
 }  // namespace b200

@@ -61,6 +61,24 @@ def test_attention_in_a_window(window, keep):
     _check(synth.make_fufipel, fufipel_numpy, [F("attention", heads=4, kv_heads=2, dim=20, window=window, keep_first=keep), F("parallel", heads=2, dim=24, chunk=11)], 1, width=80)
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(4, 1, 128, 128), (2, 2, 128, 128), (5, 1, 32, 104), (3, 1, 20, 36)])
+def test_attention_at_the_edges_of_key_tiles(heads, kv_heads, dim, vdim):
+    """Contexts below, at and behind the borders of 64-key tiles, 128 rows of 32, 128, 25 and 42 tokens; heads of 128 channels, of multiples of eight and of four."""
+    cfg, st, w = synth.make_panupel([P("parallel", heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, mm_heads=1, mm_dim=16)], seed=5, width=96, loop=None)
+    lens = [63, 64, 65, 129, 200]
+    toks = [np.random.default_rng(n).integers(1, 90, n).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, precision=1, config=cfg, kv_tokens=sum(lens) + 16 * len(lens), kv_page=16)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        got = m.infer_raw(list(range(len(lens))), lens, sum(toks, []), [capi.OPTION_FULL] * len(lens))
+        for s in range(len(lens)):
+            err = _errs(got[s], panupel_numpy.run(json.loads(cfg), w, toks[s]))
+            assert err.max() <= TIGHT, (s, int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("dim, vdim, conv", [(72, 72, 4), (128, 40, 4), (24, 24, 4), (40, 72, 3)])
 def test_delta_rule(dim, vdim, conv, precision):
