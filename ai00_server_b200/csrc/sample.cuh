@@ -15,14 +15,16 @@
 // valid outcome there; this is one of them, because the probability is a non-decreasing function of the logit.)
 //
 // Shape: one launch, a cluster of eight CTAs per row, an eighth of the row each, in registers (32 elements a thread).  Nothing here is
-// bandwidth (16 rows x 256 KB from L2); sorting every element was the cost (35-65 us for the segments' bitonic sorts, 13 us to merge).
-//   * an element and its place in the total order are one 64-bit key (ordered logit, inverted id);
-//   * the best key of every thread gives two lower bounds of the row's top_k-th key: the smallest over the CTAs of the (top_k / 8)-th best
+// bandwidth (16 rows x 256 KB from L2): instructions and trips through the cluster are the cost.
+//   * the best element of every thread gives two lower bounds of the row's top_k-th: the smallest over the CTAs of the (top_k / 8)-th best
 //     thread, and the largest over the CTAs of the top_k-th best thread.  Elements at or above the larger bound are candidates: about
-//     1.7 top_k of them for a smooth row, at most 32 top_k per CTA for any row (then the CTA keeps its own best top_k);
-//   * every CTA ranks its own candidates against all of the cluster's, read through distributed shared memory: a rank below top_k IS the
-//     output position.  Softmax statistics are combined in CTA order.
-// Results go straight to pinned host memory.  Measured at 16 rows of 65536: see the figures at topk_kernel.
+//     1.7 top_k of them for a smooth row.  All of this compares ordered logits alone, 32 bits an element;
+//   * candidates carry their place in the total order, one 64-bit key (ordered logit, inverted id).  A CTA with more than it may share (many
+//     equal logits, or the row's best in few threads) keeps its own best top_k, found with whole keys;
+//   * what a CTA has to say goes into the others' shared memory before a cluster barrier, so that no remote read is waited for: bounds and softmax
+//     statistics at the first, candidates at the second.  Every CTA ranks its own candidates against all: a rank below top_k IS the output position.
+//     Softmax statistics are combined in CTA order.
+// Results go straight to pinned host memory.  Measured at rows of 65536: see the figures at topk_kernel.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -37,11 +39,13 @@ constexpr int TOPK_SLICE = TOPK_THREADS * TOPK_PER_THREAD;      // elements of a
 constexpr int TOPK_MAX_V = TOPK_CTAS * TOPK_SLICE;              // 65536
 constexpr int TOPK_LIST = 4096;                                 // candidates of a CTA before it cuts them (127 threads x 32 at most)
 constexpr int TOPK_SHARE = 512;                                 // candidates a CTA may share
+constexpr int TOPK_PITCH_PAD = 4;                               // eight CTAs' lists, read side by side, start in different banks
 constexpr int TOPK_INLINE = 64;                                 // rows whose slots travel as kernel parameters
 __host__ __device__ constexpr int topk_slice(int V) { return ((V + TOPK_CTAS - 1) / TOPK_CTAS + 3) & ~3; }      // elements of a CTA
 // entries of its list, and bytes of shared memory (a small vocabulary cannot fill either: more CTAs to an SM)
 __host__ __device__ constexpr int topk_list(int V) { return topk_slice(V) < TOPK_LIST ? topk_slice(V) : TOPK_LIST; }
-__host__ __device__ constexpr size_t topk_smem(int V) { return ((size_t)topk_list(V) + (size_t)TOPK_CTAS * (topk_slice(V) < TOPK_SHARE ? topk_slice(V) : TOPK_SHARE)) * 8; }
+__host__ __device__ constexpr int topk_pitch(int V) { return (topk_slice(V) < TOPK_SHARE ? topk_slice(V) : TOPK_SHARE) + TOPK_PITCH_PAD; }
+__host__ __device__ constexpr size_t topk_smem(int V) { return ((size_t)topk_list(V) + (size_t)TOPK_CTAS * topk_pitch(V)) * 8; }
 
 struct TopkParams {
     const float* keep;          // [S][V] last logits row of every slot
@@ -61,31 +65,38 @@ struct TopkParams {
     float* out_p;               // [nrows][top_k]
 };
 
-// strict total order as one number: larger logit first, then smaller id (-0 and +0 are one value); 0 is below every element
-__device__ __forceinline__ unsigned long long topk_key(float x, unsigned id) {
+// larger logit, larger number (-0 and +0 are one value); 0 is below every logit
+__device__ __forceinline__ unsigned topk_order(float x) {
     const unsigned b = __float_as_uint(x == 0.f ? 0.f : x);
-    const unsigned o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-    return ((unsigned long long)o << 32) | (unsigned)~id;
+    return b ^ (0x80000000u | (unsigned)((int)b >> 31));
 }
+// strict total order as one number: larger logit first, then smaller id; 0 is below every element
+__device__ __forceinline__ unsigned long long topk_key(unsigned order, unsigned id) { return ((unsigned long long)order << 32) | (unsigned)~id; }
 __device__ __forceinline__ float topk_logit(unsigned long long key) {
     const unsigned o = (unsigned)(key >> 32);
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
 }
 
-// 16 rows of 65536 logits, top_k = 128 (ncu, cold caches): 65 + 13 us for two kernels with sorted segments, 26 us here; remote reads of a phase together instead of one
-// after the other took 2.5 us off a call in a running server (46.8 -> 44.3 us with its launch and wait)
+// top_k = 128 of rows of 65536, launches back to back: 20.5 us of one row and 24.7 of sixteen with whole keys throughout and remote reads (of 28.7 thousand cycles of a CTA
+// 8.5 went into ranking the threads' best, 5.0 into picking candidates, 3.0 into each thread's best, 3.5 into remote reads); here 14.0 and 18.5 (15.1 thousand cycles: 2.7 for the
+// ranking, 2.7 for the candidates).  A decode step with its sampling, 3B widths and one sequence: 414 -> 406 us; 7B widths, sixteen: 561 -> 552.
 __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS) topk_kernel(const __grid_constant__ TopkParams p) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char topk_smem[];
-    unsigned long long* const list = reinterpret_cast<unsigned long long*>(topk_smem);      // [topk_list(V)], shared: the first TOPK_SHARE
-    unsigned long long* const all = list + topk_list(p.V);                                  // [TOPK_CTAS * TOPK_SHARE]
+    unsigned long long* const list = reinterpret_cast<unsigned long long*>(topk_smem);      // [topk_list(V)]
+    unsigned long long* const all = list + topk_list(p.V);                                  // [TOPK_CTAS][topk_pitch(V)], written by the CTAs of the cluster
     float* const sx = reinterpret_cast<float*>(topk_smem);                                  // [cnt] while lists are applied
-    __shared__ __align__(16) unsigned long long s_best[TOPK_THREADS];
-    __shared__ unsigned long long s_few, s_full;            // the (top_k / 8)-th and the top_k-th best thread
-    __shared__ float2 s_stat;                               // (max, sum exp(x - max)) of the slice
+    __shared__ __align__(16) unsigned s_best[TOPK_THREADS];
+    __shared__ __align__(16) unsigned long long s_key[TOPK_THREADS];
+    __shared__ unsigned s_few, s_full;                      // the (top_k / 8)-th and the top_k-th best thread
+    __shared__ unsigned long long s_cut;
+    __shared__ __align__(16) uint4 s_stat[TOPK_CTAS];       // every CTA's two bounds, max and sum exp(x - max)
+    __shared__ int s_cnt[TOPK_CTAS];                        // and how many candidates it shares
     __shared__ float red[32];
     __shared__ int s_n;
+    static_assert(TOPK_THREADS / 32 == TOPK_CTAS, "a warp for every CTA of the cluster");
+    cluster.barrier_arrive();                               // (waited for before the first write to another CTA: all have begun)
     const int cta = blockIdx.x, row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int slice = topk_slice(p.V);
     const int lo = min(cta * slice, p.V), cnt = min(lo + slice, p.V) - lo;
@@ -131,76 +142,91 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
         for (int j = 0; j < TOPK_PER_THREAD; ++j)
             if (index(j) < cnt) x[j] = sx[index(j)];
     }
-    // softmax statistics of the slice, best key of the thread
+    // softmax statistics of the slice (places behind the slice hold -inf), best element of the thread
     float mx = -INFINITY;
-    unsigned long long best = 0;
+#pragma unroll
+    for (int j = 0; j < TOPK_PER_THREAD; ++j) mx = fmaxf(mx, x[j]);
+    unsigned o[TOPK_PER_THREAD], best = 0;                  // 0: not an element
 #pragma unroll
     for (int j = 0; j < TOPK_PER_THREAD; ++j) {
-        const int i = index(j);
-        if (i < cnt) {
-            mx = fmaxf(mx, x[j]);
-            best = max(best, topk_key(x[j], (unsigned)(lo + i)));
-        }
+        o[j] = cnt == TOPK_SLICE || index(j) < cnt ? max(topk_order(x[j]), 1u) : 0u;
+        best = max(best, o[j]);
     }
     s_best[tid] = best;
-    if (tid == 0) { s_few = 0; s_full = 0; s_n = 0; }
+    if (tid == 0) { s_few = s_full = ~0u; s_cut = 0; s_n = 0; }
     mx = block_max_any(mx, red);
     float sum = 0.f;
     if (mx > -INFINITY) {
 #pragma unroll
-        for (int j = 0; j < TOPK_PER_THREAD; ++j)
-            if (index(j) < cnt) sum += expf(x[j] - mx);
+        for (int j = 0; j < TOPK_PER_THREAD; ++j) sum += expf(x[j] - mx);
     }
     sum = block_sum_any(sum, red);                          // (its barriers also publish s_best)
-    if (tid == 0) s_stat = make_float2(mx, sum);
     int above = 0;
 #pragma unroll 16
-    for (int i = 0; i < TOPK_THREADS; i += 2) {
-        const ulonglong2 b2 = *reinterpret_cast<const ulonglong2*>(s_best + i);
-        above += (b2.x > best) + (b2.y > best);
+    for (int i = 0; i < TOPK_THREADS; i += 4) {
+        const uint4 b = *reinterpret_cast<const uint4*>(s_best + i);
+        above += (b.x > best) + (b.y > best) + (b.z > best) + (b.w > best);
     }
-    if (best && above == (p.top_k + TOPK_CTAS - 1) / TOPK_CTAS - 1) s_few = best;
-    if (best && above == p.top_k - 1) s_full = best;
-    cluster.sync();
-    // all remote reads of a phase are requested before the first is used: one trip through the cluster instead of eight
-    unsigned long long few = ~0ull, full = 0;
-    float M = -INFINITY;
-    float2 stat[TOPK_CTAS];
-    {
-        unsigned long long fw[TOPK_CTAS], fl[TOPK_CTAS];
-#pragma unroll
-        for (int c = 0; c < TOPK_CTAS; ++c) {
-            fw[c] = *cluster.map_shared_rank(&s_few, c);
-            fl[c] = *cluster.map_shared_rank(&s_full, c);
-            stat[c] = *cluster.map_shared_rank(&s_stat, c);
-        }
-#pragma unroll
-        for (int c = 0; c < TOPK_CTAS; ++c) { few = min(few, fw[c]); full = max(full, fl[c]); M = fmaxf(M, stat[c].x); }
-    }
-    const unsigned long long bound = max(max(few, full), 1ull);
-    // candidates of the slice -> list, in any order
-    int mine = 0;
-#pragma unroll
-    for (int j = 0; j < TOPK_PER_THREAD; ++j) mine += index(j) < cnt && topk_key(x[j], (unsigned)(lo + index(j))) >= bound;
-    int at = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, at, o);
-        if (lane >= o) at += v;
-    }
-    int wbase = 0;
-    if (lane == 31 && at) wbase = atomicAdd(&s_n, at);
-    at += __shfl_sync(0xffffffffu, wbase, 31) - mine;
-    if (mine) {
-#pragma unroll
-        for (int j = 0; j < TOPK_PER_THREAD; ++j) {
-            const unsigned long long key = topk_key(x[j], (unsigned)(lo + index(j)));
-            if (index(j) < cnt && key >= bound) list[at++] = key;
-        }
+    // the k-th best is the least of those with fewer than k above them (0 where fewer than k threads hold elements)
+    const unsigned least_few = __reduce_min_sync(0xffffffffu, above < (p.top_k + TOPK_CTAS - 1) / TOPK_CTAS ? best : ~0u);
+    const unsigned least_full = __reduce_min_sync(0xffffffffu, above < p.top_k ? best : ~0u);
+    if (lane == 0) {
+        atomicMin(&s_few, least_few);
+        atomicMin(&s_full, least_full);
     }
     __syncthreads();
-    int n = s_n;
-    if (n > TOPK_SHARE) {                                   // a row whose best elements sit in few threads: the CTA's own best top_k
+    cluster.barrier_wait();
+    if (tid < TOPK_CTAS) *cluster.map_shared_rank(&s_stat[cta], tid) = make_uint4(s_few, s_full, __float_as_uint(mx), __float_as_uint(sum));
+    cluster.sync();
+    unsigned few = ~0u, full = 0;
+    float M = -INFINITY;
+#pragma unroll
+    for (int c = 0; c < TOPK_CTAS; ++c) { few = min(few, s_stat[c].x); full = max(full, s_stat[c].y); M = fmaxf(M, __uint_as_float(s_stat[c].z)); }
+    const unsigned bound = max(max(few, full), 1u);
+    // elements from `least` on -> list, in any order; how many there are
+    auto collect = [&](const unsigned long long least) {
+        unsigned mask = 0;
+#pragma unroll
+        for (int j = 0; j < TOPK_PER_THREAD; ++j) mask |= (unsigned)(topk_key(o[j], (unsigned)(lo + index(j))) >= least) << j;
+        const int mine = __popc(mask);
+        int at = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, d);
+            if (lane >= d) at += v;
+        }
+        int wbase = 0;
+        if (lane == 31 && at) wbase = atomicAdd(&s_n, at);
+        at += __shfl_sync(0xffffffffu, wbase, 31) - mine;
+        if (mask) {
+#pragma unroll
+            for (int j = 0; j < TOPK_PER_THREAD; ++j)
+                if (mask >> j & 1u) {
+                    if (at < topk_list(p.V)) list[at] = topk_key(o[j], (unsigned)(lo + index(j)));
+                    ++at;
+                }
+        }
+        __syncthreads();
+        return s_n;
+    };
+    int n = collect(topk_key(bound, ~0u));
+    if (n > TOPK_SHARE) {                                   // the CTA's own best top_k: elements from its top_k-th best thread on (at most 32 top_k), ranked
+        unsigned long long bkey = 0;
+#pragma unroll
+        for (int j = 0; j < TOPK_PER_THREAD; ++j)
+            if (o[j] >= bound) bkey = max(bkey, topk_key(o[j], (unsigned)(lo + index(j))));
+        s_key[tid] = bkey;
+        __syncthreads();
+        int over = 0;
+#pragma unroll 16
+        for (int i = 0; i < TOPK_THREADS; i += 2) {
+            const ulonglong2 b2 = *reinterpret_cast<const ulonglong2*>(s_key + i);
+            over += (b2.x > bkey) + (b2.y > bkey);
+        }
+        if (bkey && over == p.top_k - 1) s_cut = bkey;
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        n = collect(max(s_cut, topk_key(bound, ~0u)));
         unsigned long long key[TOPK_LIST / TOPK_THREADS];
         int rank[TOPK_LIST / TOPK_THREADS];
         for (int u = 0; u < TOPK_LIST / TOPK_THREADS; ++u) {
@@ -212,38 +238,28 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
         __syncthreads();
         for (int u = 0; u < TOPK_LIST / TOPK_THREADS; ++u)
             if (tid + u * TOPK_THREADS < n && rank[u] < p.top_k) list[rank[u]] = key[u];
-        n = p.top_k;
+        n = min(n, p.top_k);
         __syncthreads();
-        if (tid == 0) s_n = n;
     }
-    cluster.sync();
-    int total = 0, from[TOPK_CTAS];                         // candidates of the CTAs in front
+    const int pitch = topk_pitch(p.V);
+    {                                                       // warp w: to CTA w
+        unsigned long long* const to = cluster.map_shared_rank(all, warp) + cta * pitch;
+        for (int i = lane; i < n; i += 32) to[i] = list[i];
+        if (lane == 0) *cluster.map_shared_rank(&s_cnt[cta], warp) = n;
+    }
+    cluster.sync();                                         // nothing remote is touched from here on: a CTA may leave when it is done
     float denom = 0.f;
-    {
-        int nc[TOPK_CTAS];
 #pragma unroll
-        for (int c = 0; c < TOPK_CTAS; ++c) nc[c] = *cluster.map_shared_rank(&s_n, c);
-#pragma unroll
-        for (int c = 0; c < TOPK_CTAS; ++c) {
-            from[c] = total;
-            total += nc[c];
-            if (stat[c].x > -INFINITY) denom += stat[c].y * expf(stat[c].x - M);
-        }
+    for (int c = 0; c < TOPK_CTAS; ++c) {
+        const float m = __uint_as_float(s_stat[c].z);
+        if (m > -INFINITY) denom += __uint_as_float(s_stat[c].w) * expf(m - M);
     }
-    for (int i = tid; i < total; i += TOPK_THREADS) {
-        int c = 0, at0 = 0;
-#pragma unroll
-        for (int q = 1; q < TOPK_CTAS; ++q)
-            if (i >= from[q]) { c = q; at0 = from[q]; }
-        all[i] = cluster.map_shared_rank(list, c)[i - at0];
-    }
-    __syncthreads();
-    cluster.barrier_arrive();                               // this CTA has read the others: they may leave (the wait is at the end)
     const float inv = 1.0f / denom;
+    const int seg = lane >> 2, nseg = s_cnt[seg];           // four lanes to a CTA's list
     for (int i = warp; i < n; i += TOPK_THREADS / 32) {
         const unsigned long long key = list[i];
         int rank = 0;
-        for (int k = lane; k < total; k += 32) rank += all[k] > key;
+        for (int k = lane & 3; k < nseg; k += 4) rank += all[seg * pitch + k] > key;
         rank = __reduce_add_sync(0xffffffffu, rank);
         if (lane == 0 && rank < p.top_k) {
             // same expression as softmax_kernel (misc.cuh): exp(x - max) * (1 / sum)
@@ -257,8 +273,6 @@ __global__ void __cluster_dims__(TOPK_CTAS, 1, 1) __launch_bounds__(TOPK_THREADS
             p.out_id[(size_t)row * p.top_k + i] = 0xFFFFFFFFu;
             p.out_p[(size_t)row * p.top_k + i] = 0.f;
         }
-    __syncwarp();
-    cluster.barrier_wait();
 }
 
 // ---------------------------------------------------------------------------------------

@@ -104,3 +104,14 @@ def test_the_best_elements_in_a_small_slice(vocab, cta):
             _check(m, rows, top_k, bias=[{p: 50.0 + 0.01 * int(v) for p, v in zip(place, lift)}])
     finally:
         m.close()
+
+
+@pytest.mark.parametrize("count, top_k", [(512, 128), (513, 128), (4097, 128), (8192, 9), (100, 128)])
+def test_equal_logits_of_one_slice(count, top_k):
+    """Logits that differ in their ids alone, as many as a CTA may share, one more, more than its list holds and a whole slice: the bound they set lets all of them through."""
+    m, rows = _model(65536, 2, zero_head=True)
+    try:
+        bias = [{int(t): 1.0 for t in range(8192, 8192 + count)}, {int(t): 1.0 + (t % 3) for t in range(0, 3 * count, 3)}]
+        _check(m, rows, top_k, bias=bias)
+    finally:
+        m.close()
