@@ -250,6 +250,173 @@ __host__ __device__ inline size_t wkv_smem_bytes(int ver, bool fold, int Dd, int
     return b;
 }
 
+constexpr int WKV_ONE_MAX_D = 256;       // decay ranks of the one-token path
+
+// One token of one slot (every slot of a decode step), the rest of the CTA's work behind the wait.  A chain of latencies, so as few links as the function has: ONE trip for
+// all operands (the general path below asks for them in up to four), the state on its way out before the norm, sums of the norm within warps and one exchange each.
+// Measured (CTA 0 from the wait's release to its end; 3B widths and one sequence / 7B widths and sixteen / RWKV-7 2.9B widths and eight): 7.4 -> 4.4 us, 6.7 -> 3.9, 7.7 -> 4.8, of which
+// the staging of operands had taken 3 to 4.3; the output projection begins 4.5, 2.4 and 5.5 us earlier.
+// `wt`: decay-LoRA slice [Dd][64] in shared memory, `v64`: shared memory for seven rows of 64 floats (staged rows and decays of the general path lie there otherwise).
+template <int VER, bool SPLIT>
+__device__ __forceinline__ void wkv_one_token(const WkvParams& p, const int h, const int t, float (&m)[4][8], float* M, const float* statics, const float bias, const __half* wt,
+                                              const int Dd, float* v64) {
+    constexpr int KC = 8, LANES = WKV_N / KC;
+    __shared__ float s_w[WKV_N], s_part[4][WKV_N], s_d[WKV_ONE_MAX_D], s_red[3][4];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ig = tid / LANES, j4 = tid % LANES, ch = h * WKV_N;
+    const size_t row = (size_t)t * p.ld + ch;
+    const bool fold = VER == 6 && Dd > 0;
+    const int c = tid & (WKV_N - 1), two = tid >> 6;
+    // threads 0 .. 63: r, v (w, a of v7); 64 .. 127: k, g (nu, v_first)
+    float x0 = two ? p.k[row + c] : p.r[row + c], x1 = two ? p.g[row + c] : p.v[row + c], x2 = 0.f, x3 = 0.f, x4 = 0.f, st0 = 0.f, st1 = 0.f;
+    if (VER == 5) { if (!two) x2 = p.w_static[ch + c]; }
+    if (VER == 6 && !fold) { if (!two) x2 = p.w[row + c]; }
+    if (VER == 7) {
+        if (!two) { x2 = p.w[row + c]; x3 = p.a[row + c]; st0 = p.r_k[ch + c]; }
+        else {
+            if (!p.layer0) { x2 = p.nu[row + c]; x3 = p.v_first[row + c]; }
+            x4 = p.a[row + c]; st0 = p.k_k[ch + c]; st1 = p.k_a[ch + c];
+        }
+    }
+    if (fold)
+        for (int k = tid; k < Dd; k += WKV_N * 2) {
+            float d = __half2float(p.d1[a16_index(t, k, p.d1_kq)]);
+            if (SPLIT) d += __half2float(p.d1[a16_index(t + 16, k, p.d1_kq)]);
+            s_d[k] = d;
+        }
+    float* const sr = v64, * const sk = v64 + 64, * const sv = v64 + 128, * const sg = v64 + 192, * const sb = v64 + 256, * const sn = v64 + 320, * const sneg = v64 + 384;
+    if (VER != 7) {
+        (two ? sk : sr)[c] = x0;
+        (two ? sg : sv)[c] = x1;
+        if (!fold && !two) s_w[c] = x2;
+        __syncthreads();
+    } else {
+        float kk = 0.f;
+        if (two) {                                          // keys: unit length over the head (two warps), in-context rate
+            kk = x0 * st0;
+            const float ss = warp_sum(kk * kk);
+            if (lane == 0) s_red[0][warp] = ss;
+            x0 *= 1.f + (x4 - 1.f) * st1;
+            sk[c] = x0;
+            sg[c] = x1;
+            if (!p.layer0) { sb[c] = x2; sn[c] = x3; }      // for the value rows, a barrier later
+        } else {
+            sr[c] = x0;
+            s_w[c] = x2;
+        }
+        __syncthreads();
+        if (two) {
+            kk = kk / fmaxf(sqrtf(s_red[0][2] + s_red[0][3]), 1e-12f);
+            sneg[c] = -kk;
+            s_part[0][c] = kk * x4;
+        } else {
+            float v = x1;
+            if (p.layer0) p.v_first[row + c] = v;
+            else v = v + (sn[c] - v) * sb[c];
+            sv[c] = v;
+            const float bonus = warp_sum(x0 * sk[c] * st0);
+            if (lane == 0) s_red[0][warp] = bonus;
+        }
+        __syncthreads();
+    }
+    if (fold) {
+        // w[c] = exp(-exp(time_decay[c] + sum_k Wd2[c][k] tanh(Wd1 xw)[k])): thread = (two channels, quarter of k)
+        const int c2 = 2 * lane, k0 = warp * (Dd >> 2), k1 = k0 + (Dd >> 2);
+        float a0 = 0.f, a1 = 0.f;
+#pragma unroll 8
+        for (int k = k0; k < k1; ++k) {
+            const float2 w2 = __half22float2(*reinterpret_cast<const __half2*>(wt + k * WKV_N + c2));
+            const float d = s_d[k];
+            a0 = fmaf(w2.x, d, a0); a1 = fmaf(w2.y, d, a1);
+        }
+        *reinterpret_cast<float2*>(&s_part[warp][c2]) = make_float2(a0, a1);
+        __syncthreads();
+        if (tid < WKV_N) s_w[c] = expf(-expf(bias + ((s_part[0][c] + s_part[1][c]) + (s_part[2][c] + s_part[3][c]))));
+        __syncthreads();
+    }
+    float rr[KC], kk_[KC], ww[KC], o[4];
+#pragma unroll
+    for (int f = 0; f < KC; ++f) { rr[f] = sr[j4 * KC + f]; kk_[f] = sk[j4 * KC + f]; ww[f] = s_w[j4 * KC + f]; }
+    if (VER != 7) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float vv = sv[ig * 4 + e];
+            float acc = 0.f;
+#pragma unroll
+            for (int f = 0; f < KC; ++f) {
+                const float kv = kk_[f] * vv;
+                acc += rr[f] * (statics[2 * WKV_N + j4 * KC + f] * kv + m[e][f]);
+                m[e][f] = kv + ww[f] * m[e][f];
+            }
+            o[e] = acc;
+        }
+    } else {
+        float nk[KC], ka[KC], sa[4];
+#pragma unroll
+        for (int f = 0; f < KC; ++f) { nk[f] = sneg[j4 * KC + f]; ka[f] = s_part[0][j4 * KC + f]; }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float s_ = 0.f;
+#pragma unroll
+            for (int f = 0; f < KC; f += 4) s_ += (m[e][f] * nk[f] + m[e][f + 1] * nk[f + 1]) + (m[e][f + 2] * nk[f + 2] + m[e][f + 3] * nk[f + 3]);
+            sa[e] = s_;
+        }
+#pragma unroll
+        for (int off = LANES / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sa[e] += __shfl_xor_sync(0xffffffffu, sa[e], off);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float vv = sv[ig * 4 + e];
+            float acc = 0.f;
+#pragma unroll
+            for (int f = 0; f < KC; ++f) {
+                m[e][f] = m[e][f] * ww[f] + sa[e] * ka[f] + vv * kk_[f];
+                acc += m[e][f] * rr[f];
+            }
+            o[e] = acc;
+        }
+    }
+    // the state is final: it leaves while the norm is worked out
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int q = 0; q < KC / 4; ++q)
+            __stcs(reinterpret_cast<float4*>(M + (ig * 4 + e) * WKV_N + j4 * KC + q * 4), make_float4(m[e][q * 4], m[e][q * 4 + 1], m[e][q * 4 + 2], m[e][q * 4 + 3]));
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] += __shfl_xor_sync(0xffffffffu, o[e], off);
+    // GroupNorm over the head: every lane of a group of eight holds its four rows
+    float s = (o[0] + o[1]) + (o[2] + o[3]);
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    if (lane == 0) s_red[1][warp] = s;
+    __syncthreads();
+    const float mean = ((s_red[1][0] + s_red[1][1]) + (s_red[1][2] + s_red[1][3])) * (1.f / WKV_N);
+    float var = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { o[e] -= mean; var = fmaf(o[e], o[e], var); }
+    var += __shfl_xor_sync(0xffffffffu, var, 8);
+    var += __shfl_xor_sync(0xffffffffu, var, 16);
+    if (lane == 0) s_red[2][warp] = var;
+    __syncthreads();
+    if (j4 >= 4) return;
+    const float rstd = 1.0f / sqrtf(((s_red[2][0] + s_red[2][1]) + (s_red[2][2] + s_red[2][3])) * (1.f / WKV_N) + GN_EPS);
+    const int oc = ig * 4 + j4;                             // a row a lane
+    const float d = j4 < 2 ? (j4 == 0 ? o[0] : o[1]) : (j4 == 2 ? o[2] : o[3]);
+    float y = d * rstd * statics[oc] + statics[WKV_N + oc];
+    if (VER == 7) y += (s_red[0][0] + s_red[0][1]) * sv[oc];
+    y *= sg[oc];
+    if (SPLIT) {                                            // lo halves in the second token tile
+        __half hi, lo;
+        split_h(y, hi, lo);
+        p.out[a16_index(t, ch + oc, p.kq_tile)] = hi;
+        p.out[a16_index(t + 16, ch + oc, p.kq_tile)] = lo;
+    } else {
+        p.out[a16_index(t, ch + oc, p.kq_tile)] = f2h_sat(y);
+    }
+}
+
 // SPLIT (opt-in B200RWKV_SPLIT_ACT=1): the decay-LoRA input and the output are split operands (hi + lo f16 pairs).
 template <int VER, bool SPLIT = false>
 __global__ void __launch_bounds__(WKV_SA_THREADS, 7) wkv_kernel(const __grid_constant__ WkvParams p, const int max_tokens) {
@@ -316,6 +483,11 @@ __global__ void __launch_bounds__(WKV_SA_THREADS, 7) wkv_kernel(const __grid_con
     pdl_wait();
     trace_stamp(p.trace, 1);
     if (!live) return;
+    if (nt == 1 && Dd <= WKV_ONE_MAX_D) {
+        wkv_one_token<VER, SPLIT>(p, h, t0, m, M, statics, bias, wt, Dd, pre_s);
+        trace_stamp(p.trace, 7);
+        return;
+    }
 
     // ---- one batch of loads: staged rows, decay-LoRA inputs ----
     const bool staged = nt <= WKV_STAGE_TOK;

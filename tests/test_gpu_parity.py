@@ -447,3 +447,24 @@ def test_prefill_steps_of_128_tokens(models, preset):
     for s, r in enumerate(runs):
         want, _ = orc.run(r, orc.state_init())
         assert rel_err(rows[s], want) <= REL_TOL and rows[s].argmax() == want.argmax()
+
+
+@pytest.mark.parametrize("over", [{}, {"Dd": 96}, {"Dd": 192}])
+@pytest.mark.parametrize("preset, exact", [("tiny5", False), ("tiny6", False), ("tiny7", False), ("tiny6", True), ("tiny7", True)])
+def test_steps_of_one_token_a_slot_against_steps_of_several(models, preset, exact, over):
+    """The recurrence's path for one token (decay ranks folded in and apart) against the oracle and the path for several: twelve tokens one by one, in a batch whose other slots skip
+    steps, and in steps of three; logits, states and hidden rows in front of the head."""
+    if over and preset != "tiny6":
+        pytest.skip("decay ranks of RWKV-6")
+    m, orc, st = models(preset, exact=exact, **over)
+    if exact:
+        orc = O.Oracle(O.parse_st(st), "f32")
+    toks = [1, 5, 9, 33, 2, 7, 300, 41, 41, 8, 0, 17]
+    for s in range(3):
+        m.state.load(m.state.init(), s)
+    one = [m.infer_raw([0, 2] if i % 2 else [0], [1, 1] if i % 2 else [1], [t, t] if i % 2 else [t], [capi.OPTION_LAST] * (2 if i % 2 else 1))[0].copy() for i, t in enumerate(toks)]
+    three = np.concatenate([m.infer_raw([1], [3], toks[i:i + 3], [capi.OPTION_FULL])[0].copy() for i in range(0, 12, 3)])
+    want, _ = orc.run(toks, orc.state_init(), full=True)
+    tol = 1e-4 if exact else REL_TOL
+    assert rel_err(np.concatenate(one), want) <= REL_TOL and rel_err(np.concatenate(one), three) <= tol
+    assert rel_err(m.state.back(0), m.state.back(1)) <= tol
