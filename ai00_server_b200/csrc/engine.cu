@@ -1833,8 +1833,13 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
         lo.kq_tile = MTR > 8 ? th_rows | a_head.tile_kb << 16 : th_rows;
         lo.meta = mv;
         take_parts(lo, part_ffn, parts_v);
-        if (split_on && MT == 1) launch_k(ln_out_kernel<true>, dim3(rows), dim3(LN_THREADS), 0, lo, KC_LN, s, prof);
-        else launch_k(ln_out_kernel<false>, dim3(rows), dim3(LN_THREADS), 0, lo, KC_LN, s, prof);
+        if (ln_cluster_ok && MT == 1) {
+            launch_cluster = PRE_CLUSTER;
+            if (split_on) launch_k(ln_out_cluster_kernel<true>, dim3(rows * PRE_CLUSTER), dim3(PRE_THREADS), 0, lo, KC_LN, s, prof);
+            else launch_k(ln_out_cluster_kernel<false>, dim3(rows * PRE_CLUSTER), dim3(PRE_THREADS), 0, lo, KC_LN, s, prof);
+        } else {
+            launch_k(ln_out_kernel, dim3(rows), dim3(LN_THREADS), 0, lo, KC_LN, s, prof);
+        }
     }
     if (MTR > 0) launch_gemm_chained(head, MTR);
     if (world > 1) launch_k(tp_barrier_kernel, dim3(1), dim3(32), 0, tpbar, KC_OTHER, s, prof);
