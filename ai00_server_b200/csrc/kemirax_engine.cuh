@@ -281,7 +281,8 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
         allow_smem(latent_attn_tc_kernel<4, 4>, smem_tc);
         allow_smem(latent_attn_tc_kernel<1, 16>, smem_tc);
         allow_smem(latent_attn_tc_kernel<2, 8>, smem_tc);
-        allow_smem(latent_prompt_kernel, LATENT_PROMPT_SMEM);
+        allow_smem(latent_prompt_kernel<true>, latent_prompt_smem(LP_MAX_D, LP_MAX_RK));
+        allow_smem(latent_prompt_kernel<false>, latent_prompt_smem(LP_MAX_D, LP_MAX_RK));
     }
     CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
@@ -532,12 +533,12 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 KvWriteParams kw{m.kv, D, l.cache, m.d_table, m.npages, m.page, l.dkv_norm, rk, dr, c.rot.dims, l.freq, l.mag, m.cfg.eps, mv, m.sm};
                 launch_k(kv_write_kernel, dim3(rows), dim3(128), 0, kw, KC_OTHER, s, prof);
             }
-            const bool whole = !m.exact && !decode && nsplit == 1 && D % 4 == 0 && rk <= 64 * LP_MAX_NT && latent_prompt_smem(D) <= LATENT_PROMPT_SMEM;      // latent_prompt.cuh
+            const bool whole = !m.exact && !decode && nsplit == 1 && D % 4 == 0 && D <= LP_MAX_D && rk <= LP_MAX_RK;      // latent_prompt.cuh
             LatentAttnParams ap{m.qa, l.cache, m.d_table, m.npages, m.page, m.part, H_, rk, dr, nsplit, c.scale, mv, m.sm};
             if (whole) {
                 LatentPromptParams lp{ap, m.olat, std::min(H_, 16), 0};
                 lp.qt = LP_ROWS / lp.hg;
-                launch_k(latent_prompt_kernel, dim3(cdiv(rows, lp.qt) + nslot_grid, cdiv(H_, lp.hg)), dim3(LP_THREADS), latent_prompt_smem(D), lp, KC_WKV, s, prof);
+                launch_k(D % 8 == 0 ? latent_prompt_kernel<true> : latent_prompt_kernel<false>, dim3(cdiv(rows, lp.qt) + nslot_grid, cdiv(H_, lp.hg)), dim3(LP_THREADS), latent_prompt_smem(D, rk), lp, KC_WKV, s, prof);
             } else if (!m.exact) {         // serving precision: both products on the tensor cores (TF32 operands, f32 accumulation and softmax)
                 const size_t sm_b = latent_attn_tc_smem(D);
                 if (!decode) launch_k(latent_attn_tc_kernel<4, 4>, dim3(cdiv(rows, 4) + nslot_grid, cdiv(H_, 4), nsplit), dim3(LA_THREADS), sm_b, ap, KC_WKV, s, prof);

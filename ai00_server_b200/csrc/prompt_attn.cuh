@@ -12,15 +12,14 @@
 //              scores and the MN-major operand of the values;
 //   * scores   S = Q K^T, 64 columns of tensor memory; eight warps take half a row each a thread, exchange maxima, and write the weights back as three parts;
 //   * values   O = P V, a fresh accumulator every tile, added to the rows' registers one tile later;
-//   * one thread issues: the scores of tile t + 1 are multiplied while the softmax of tile t runs, the values of tile t while that of t + 1 does; seven warps split the
+//   * one lane issues: the scores of tile t + 1 are multiplied while the softmax of tile t runs, the values of tile t while that of t + 1 does; seven warps split the
 //              tiles ahead of it (16 of eight keys a tile, dealt out), two buffers each for keys and values.
-// Measured (16 sequences of 128 tokens, 16 query heads on 4 key heads of 128 channels, in f32 multiply-adds before and here): 113 -> 36 us at 128 tokens of context, 454 -> 82 at
-// 576, 805 -> 130 at 1024; one prompt of 1000 tokens 376 -> 63, of 20 tokens 25 -> 15; 16 prompts of 1024 tokens, four layers
-// of width 2048, 22.1 -> 15.9 ms.  Distance from 64 bits (2-norm): 6.2e-7 -> 3.0e-7 at 1024 tokens, 1.42e-6 -> 3.5e-7 at 6000, 1.6e-7 -> 1.4e-7 at 20.
-// Slower than before only where most rows are empty and the context is one tile: 64 sequences of 32 tokens, one query head a key head: 87 -> 89 us of 128 channels, 64 -> 80 of 32.
+// Measured (16 sequences of 128 tokens, 16 query heads on 4 key heads of 128 channels, in f32 multiply-adds before and here): 113 -> 34 us at 128 tokens of context, 454 -> 76 at
+// 576, 805 -> 122 at 1024 (130 with descriptors worked out by the issuing lane alone); one prompt of 1000 tokens 376 -> 59, of 20 tokens 25 -> 15; 16 prompts of 1024 tokens, four
+// layers of width 2048, 22.1 -> 15.7 ms.  Distance from 64 bits (2-norm): 6.2e-7 -> 3.0e-7 at 1024 tokens, 1.42e-6 -> 3.5e-7 at 6000, 1.6e-7 -> 1.4e-7 at 20.
+// Slower than before only where most rows are empty and the context is one tile: 64 sequences of 32 tokens, one query head a key head: 86 -> 82 us of 128 channels, 64 -> 74 of 32.
 #pragma once
-#include <cuda_bf16.h>
-
+#include "bf16_parts.cuh"
 #include "linear_umma.cuh"
 #include "sink_attn.cuh"
 
@@ -41,43 +40,6 @@ __host__ __device__ inline int pt_up16(int d) { return (d + 15) & ~15; }
 __host__ __device__ inline size_t prompt_attn_smem(int dk, int dv) {
     const size_t tiles = (size_t)2 * 3 * PT_KT * 2 * (pt_up16(dk) + pt_up16(dv)), out = (size_t)PT_ROWS * (pt_up16(dv) + 4) * 4;
     return (tiles > out ? tiles : out) + 128;
-}
-
-// shared memory only: the general form also waits for the global loads in flight (the next keys)
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// (a, b) -> packed bf16, and what it leaves of them
-__device__ __forceinline__ uint32_t pt_take(float& a, float& b) {
-    const uint32_t h = pack_bf16x2(make_float2(a, b));
-    a -= __uint_as_float(h << 16);
-    b -= __uint_as_float(h & 0xFFFF0000u);
-    return h;
-}
-
-// eight neighbouring numbers, zeros from `left` on (a multiple of four).  WHOLE: `left` is a multiple of eight and the address one of 32 bytes: one access of a whole sector a
-// lane (two of 16 bytes, each half of 32 sectors, took 150 us where this takes 130: 16 sequences, contexts of 1024)
-template <bool WHOLE>
-__device__ __forceinline__ void pt_load8(float (&v)[8], const float* src, const int left) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = 0.f;
-    if constexpr (WHOLE) {
-        if (left <= 0) return;
-        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                     : "l"(src));
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-            const float4 x = i < left ? *reinterpret_cast<const float4*>(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-            v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
-        }
-    }
-}
-
-// eight numbers -> the 16 bytes of each part
-__device__ __forceinline__ void pt_split8(float (&v)[8], uint4 (&part)[3]) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) part[i] = make_uint4(pt_take(v[0], v[1]), pt_take(v[2], v[3]), pt_take(v[4], v[5]), pt_take(v[6], v[7]));
 }
 
 // One row (token t at position pos, query head h of key head c) worked out again by a warp, key by key.  A key behind a token has weight zero in the tiles below, and zero times a
@@ -167,47 +129,46 @@ __global__ void __launch_bounds__(PT_THREADS, 1) prompt_attn_kernel(const __grid
         auto position = [&](int i) { return i < nkeep ? i : jlo + i - nkeep; };      // kept tokens first, then the window
 
         if (warp == PT_THREADS / 32 - 1) {
-            // ===================== MMA issuer: one lane =====================
-            if (lane == 0) {
-                const uint32_t IDESC_S = umma_idesc_bf16(PT_ROWS, PT_KT), IDESC_O = umma_idesc_bf16(PT_ROWS, 8 * ncv) | (1u << 16);      // values: N contiguous
-                constexpr uint32_t RUN = PT_KT * 16;         // bytes between runs of eight channels
-                // a descriptor's address field counts 16 bytes and sits in its low half: operands further on are sums there
-                const uint64_t dk0 = umma_desc(tiles, RUN, 128), dv0 = umma_desc(tiles + 6 * nck * RUN, 128, RUN);
-                auto at = [](const uint64_t d, const uint32_t off) { return (d & 0xFFFFFFFF00000000ull) | ((uint32_t)d + off); };
-                constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};      // parts of a product, the smallest first
-                const uint32_t kpart = nck * (RUN / 16), vpart = ncv * (RUN / 16);
-                auto values = [&](const int t) {
-                    const int b = t & 1;
-                    mbar_wait(b_vfull + 8 * b, (t >> 1) & 1, 41);
-                    mbar_wait(b_pfull, b, 42);
-                    tc_fence_after();
-                    const uint64_t d0 = at(dv0, 3 * b * vpart), dp[3] = {d0, at(d0, vpart), at(d0, 2 * vpart)};
+            // ===================== MMA issuer: one elected lane; the whole warp walks, so that descriptors are uniform values =====================
+            const bool one = elect_one();
+            const uint32_t IDESC_S = umma_idesc_bf16(PT_ROWS, PT_KT), IDESC_O = umma_idesc_bf16(PT_ROWS, 8 * ncv) | (1u << 16);      // values: N contiguous
+            constexpr uint32_t RUN = PT_KT * 16;             // bytes between runs of eight channels
+            // (the address field counts 16 bytes)
+            const uint64_t dk0 = umma_desc(tiles, RUN, 128), dv0 = umma_desc(tiles + 6 * nck * RUN, 128, RUN);
+            constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};      // parts of a product, the smallest first
+            const uint32_t kpart = nck * (RUN / 16), vpart = ncv * (RUN / 16);
+            auto values = [&](const int t) {
+                const int b = t & 1;
+                mbar_wait(b_vfull + 8 * b, (t >> 1) & 1, 41);
+                mbar_wait(b_pfull, b, 42);
+                tc_fence_after();
+                const uint64_t d0 = dv0 + 3 * b * vpart;
 #pragma unroll
-                    for (int i = 0; i < 6; ++i)
+                for (int i = 0; i < 6; ++i)
 #pragma unroll
-                        for (int k = 0; k < PT_KT / 16; ++k)
-                            tc_mma_f16_ts(tmem + PT_TO, tmem + PT_TP + PA[i] * 32 + k * 8, at(dp[PB[i]], k * 16), IDESC_O, i + k > 0);
-                    if (t + 2 < ntiles) tc_commit(b_vfree + 8 * b);
-                    tc_commit(b_ofull);
-                };
-                mbar_wait(b_q, 0, 43);
-                for (int t = 0; t < ntiles; ++t) {
-                    const int b = t & 1;
-                    mbar_wait(b_kfull + 8 * b, (t >> 1) & 1, 44);
-                    if (t > 0) mbar_wait(b_sfree, (t - 1) & 1, 45);
-                    tc_fence_after();
-                    const uint64_t d0 = at(dk0, 3 * b * kpart), dp[3] = {d0, at(d0, kpart), at(d0, 2 * kpart)};
+                    for (int k = 0; k < PT_KT / 16; ++k)
+                        if (one) tc_mma_f16_ts(tmem + PT_TO, tmem + PT_TP + PA[i] * 32 + k * 8, d0 + PB[i] * vpart + k * 16, IDESC_O, i + k > 0);
+                if (one && t + 2 < ntiles) tc_commit(b_vfree + 8 * b);
+                if (one) tc_commit(b_ofull);
+            };
+            mbar_wait(b_q, 0, 43);
+            for (int t = 0; t < ntiles; ++t) {
+                const int b = t & 1;
+                mbar_wait(b_kfull + 8 * b, (t >> 1) & 1, 44);
+                if (t > 0) mbar_wait(b_sfree, (t - 1) & 1, 45);
+                tc_fence_after();
+                const uint64_t d0 = dk0 + 3 * b * kpart;
 #pragma unroll
-                    for (int i = 0; i < 6; ++i)
+                for (int i = 0; i < 6; ++i)
 #pragma unroll
-                        for (int k = 0; k < PT_DMAX / 16; ++k)
-                            if (2 * k < nck) tc_mma_f16_ts(tmem + PT_TS, tmem + PT_TQ + PA[i] * 64 + k * 8, at(dp[PB[i]], 2 * k * (RUN / 16)), IDESC_S, i + k > 0);
-                    if (t + 2 < ntiles) tc_commit(b_kfree + 8 * b);
-                    tc_commit(b_sfull);
-                    if (t > 0) values(t - 1);
-                }
-                values(ntiles - 1);
+                    for (int k = 0; k < PT_DMAX / 16; ++k)
+                        if (2 * k < nck && one) tc_mma_f16_ts(tmem + PT_TS, tmem + PT_TQ + PA[i] * 64 + k * 8, d0 + PB[i] * kpart + 2 * k * (RUN / 16), IDESC_S, i + k > 0);
+                if (one && t + 2 < ntiles) tc_commit(b_kfree + 8 * b);
+                if (one) tc_commit(b_sfull);
+                if (t > 0) values(t - 1);
             }
+            values(ntiles - 1);
+            __syncwarp();
         } else if (warp >= PT_SOFT / 32) {
             // ===================== f32 rows of the cache -> three bf16 parts: eight keys of a key or value tile at a time, dealt out among the warps =====================
             const int k8 = lane & 7, cq = lane >> 3;         // a key of the eight, every fourth run of eight channels

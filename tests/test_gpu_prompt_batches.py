@@ -102,6 +102,24 @@ def test_latent_attention(heads, kv_rank, rot_dim):
 
 
 @pytest.mark.parametrize("n", [17, 100, 300])
+@pytest.mark.parametrize("heads, kv_rank, rot_dim", [(16, 128, 64), (3, 20, 4), (8, 200, 24)])
+def test_latent_attention_at_the_edges_of_key_tiles(heads, kv_rank, rot_dim):
+    """Contexts below, at and behind the borders of 32-key tiles, latent rows of one, part of one and several pieces of 128 entries, of multiples of eight and of four."""
+    cfg, st, w = synth.make_kemirax([K("latent_attention", heads=heads, kv_rank=kv_rank, rot_dim=rot_dim, mlp=False)], seed=6, width=96)
+    lens = [31, 32, 33, 65, 150]
+    toks = [np.random.default_rng(n).integers(1, 90, n).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, config=cfg, kv_tokens=sum(lens) + 16 * len(lens), kv_page=16)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        got = m.infer_raw(list(range(len(lens))), lens, sum(toks, []), [capi.OPTION_FULL] * len(lens))
+        for s in range(len(lens)):
+            err = _errs(got[s], kemirax_numpy.run(json.loads(cfg), w, toks[s]))
+            assert np.median(err) <= BF16_TOL and err.max() <= ROW_TOL, (s, float(np.median(err)), int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("ranks", [(64, 128), (32, 32), (64, 64)])
 def test_low_rank_second_stages(ranks, n):
     """Both kernels of lora2.cuh at every rank they are built for, one tile of tokens and several."""
