@@ -1168,6 +1168,8 @@ void b200rwkv_engine::build(const StFile& st) {
         CK(cudaFuncSetAttribute(wkv_kernel<7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, wkv_smem_max));
     }
     allow_smem(ln_mix_rows_kernel, (size_t)(LN_ROWS + 1) * C * 4);
+    allow_smem(ln_mix_tall_kernel, std::min<size_t>(ln_tall_smem(C), 200 * 1024));
+    allow_smem(ln_out_tall_kernel, std::min<size_t>(ln_tall_smem(C), 200 * 1024));
     allow_smem(wkv_scan_kernel<5>, SCAN_ALONE_SMEM);
     allow_smem(wkv_scan_kernel<6>, SCAN_ALONE_SMEM);
     allow_smem(wkv_scan_kernel<7>, SCAN_ALONE_SMEM);
@@ -1722,6 +1724,8 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
         ep.meta = mv;
         launch_k(embed_ln0_kernel, dim3(rows), dim3(LN_THREADS), 0, ep, KC_LN, s, prof);
     }
+    // long steps: seven or eight rows to a CTA (mix.cuh) once there are enough for half of the SMs
+    auto ln_tall = [&](int n) { return n >= 512 && ln_tall_smem(C) <= 200 * 1024; };
     auto launch_ln = [&](const LnMixParams& lp0) {
         LnMixParams lp = lp0;
         lp.trace = tr_next(0);
@@ -1731,6 +1735,8 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             launch_cluster = PRE_CLUSTER;
             if (split_on) launch_k(ln_mix_cluster_kernel<true>, dim3(PRE_GRID), dim3(PRE_THREADS), 0, lp, KC_LN, s, prof);
             else launch_k(ln_mix_cluster_kernel<false>, dim3(PRE_GRID), dim3(PRE_THREADS), 0, lp, KC_LN, s, prof);
+        } else if (ln_tall(rows)) {
+            launch_k(ln_mix_tall_kernel, dim3(cdiv(rows, TALL_ROWS)), dim3(TALL_THREADS), ln_tall_smem(C), lp, KC_LN, s, prof);
         } else if (MT >= 2) {
             launch_k(ln_mix_rows_kernel, dim3(rows / LN_ROWS), dim3(LN_ROWS_THREADS), (size_t)(LN_ROWS + 1) * C * 4, lp, KC_LN, s, prof);
         } else {
@@ -1837,6 +1843,8 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             launch_cluster = PRE_CLUSTER;
             if (split_on) launch_k(ln_out_cluster_kernel<true>, dim3(rows * PRE_CLUSTER), dim3(PRE_THREADS), 0, lo, KC_LN, s, prof);
             else launch_k(ln_out_cluster_kernel<false>, dim3(rows * PRE_CLUSTER), dim3(PRE_THREADS), 0, lo, KC_LN, s, prof);
+        } else if (ln_tall(rows)) {
+            launch_k(ln_out_tall_kernel, dim3(cdiv(rows, TALL_ROWS + 1)), dim3(TALL_THREADS), ln_tall_smem(C), lo, KC_LN, s, prof);
         } else {
             launch_k(ln_out_kernel, dim3(rows), dim3(LN_THREADS), 0, lo, KC_LN, s, prof);
         }

@@ -343,6 +343,141 @@ __global__ void __launch_bounds__(LN_ROWS_THREADS) ln_mix_rows_kernel(const __gr
     trace_stamp(p.trace, 7);
 }
 
+// Long prompt steps: TALL_ROWS tokens to a CTA and the one before them, 64 threads a row, rows in shared memory (so that few registers are held and two CTAs of 2560 columns
+// share an SM: sixteen rows' loads in flight).  The row before is read again by one token in seven instead of one in two, and the f16 operands leave eight channels of
+// eight tokens at a time: runs of 112 bytes where a thread of the form above leaves 8.
+// Bytes bound it: 2048 rows of 2560 with one partial sum and a gate, 120 to 140 MB: in place 46 -> 29 us.
+constexpr int TALL_ROWS = 7, TALL_GROUP = 64, TALL_THREADS = (TALL_ROWS + 1) * TALL_GROUP, TALL_PAD = 4;      // pad: eight rows' 16 bytes lie in different banks
+__host__ __device__ inline size_t ln_tall_smem(int C) { return (size_t)(TALL_ROWS + 1) * (C + TALL_PAD) * 4; }
+
+// the updated residual of row t, 64 threads: put(c, four entries) for every four columns
+template <typename F>
+__device__ __forceinline__ void tall_residual(const ResidualSrc& r, const int t, const int l, F&& put) {
+    constexpr int U = 3;
+    const size_t base = (size_t)t * r.C;
+    for (int c0 = 4 * l; c0 < r.C; c0 += 4 * TALL_GROUP * U) {
+        float4 a[U], s[U], v[2][U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + 4 * TALL_GROUP * u;
+            a[u] = c < r.C ? ld4(r.x_in + base + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            s[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (r.n_parts > 0) {
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                if (q >= r.n_parts) break;
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int c = c0 + 4 * TALL_GROUP * u;
+                        v[e][u] = q + e < r.n_parts && c < r.C ? ld4(r.parts[q + e] + base + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                for (int e = 0; e < 2; ++e)        // fixed order, identical on all ranks
+#pragma unroll
+                    for (int u = 0; u < U; ++u) add4(s[u], v[e][u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int c = c0 + 4 * TALL_GROUP * u;
+                if (r.n_gate > 0 && c < r.C) {
+                    const int gb = r.n_gate > 1 ? c / r.gate_cl : 0;
+                    const float* gp = r.gates[0];
+#pragma unroll
+                    for (int i = 1; i < 8; ++i) gp = (gb == i) ? r.gates[i] : gp;
+                    const float4 gt = ld4(gp + (size_t)t * r.gate_cl + (c - gb * r.gate_cl));
+                    s[u].x *= gt.x; s[u].y *= gt.y; s[u].z *= gt.z; s[u].w *= gt.w;
+                }
+                add4(a[u], s[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (c0 + 4 * TALL_GROUP * u < r.C) put(c0 + 4 * TALL_GROUP * u, a[u]);
+    }
+}
+
+// mean and 1 / deviation of a row in shared memory; `bar`: the group's barrier, s1: this thread's sum
+__device__ __forceinline__ void tall_stats(const float* row, const int C, const int l, const int bar, float s1, float* red, float& mean, float& rstd) {
+    auto sum = [&](float v) {
+        v = warp_sum(v);
+        named_bar_sync(bar, TALL_GROUP);
+        if ((l & 31) == 0) red[l >> 5] = v;
+        named_bar_sync(bar, TALL_GROUP);
+        return red[0] + red[1];
+    };
+    mean = sum(s1) / (float)C;
+    float s2 = 0.f;
+    for (int c = 4 * l; c < C; c += 4 * TALL_GROUP) {
+        const float4 a = ld4(row + c);
+        const float dx = a.x - mean, dy = a.y - mean, dz = a.z - mean, dw = a.w - mean;
+        s2 += (dx * dx + dy * dy) + (dz * dz + dw * dw);
+    }
+    rstd = 1.0f / sqrtf(sum(s2) / (float)C + LN_EPS);
+}
+
+__global__ void __launch_bounds__(TALL_THREADS, 2) ln_mix_tall_kernel(const __grid_constant__ LnMixParams p) {
+    extern __shared__ __align__(16) float ln_tall[];
+    __shared__ float red[TALL_ROWS + 1][2];
+    trace_stamp(p.trace, 0);
+    pdl_launch_dependents();
+    const int C = p.C, pitch = C + TALL_PAD, T = p.meta.T(), t0 = blockIdx.x * TALL_ROWS, g = threadIdx.x / TALL_GROUP, l = threadIdx.x % TALL_GROUP;
+    const int t = t0 - 1 + g;                                  // group 0: the row before
+    const bool live = t >= 0 && t < T && (g > 0 || (t0 < T && p.meta.tok_prev()[t0] >= 0));
+    pdl_wait();
+    trace_stamp(p.trace, 1);
+    if (t0 >= T) return;
+    if (live) {
+        const ResidualSrc r = make_residual_src(p);
+        float* const row = ln_tall + (size_t)g * pitch;
+        const bool keep = g > 0 && (p.x_out != p.x_in || p.n_parts > 0);
+        float s1 = 0.f, mean, rstd;
+        tall_residual(r, t, l, [&](const int c, const float4 a) {
+            s1 += (a.x + a.y) + (a.z + a.w);
+            *reinterpret_cast<float4*>(row + c) = a;
+            if (keep) *reinterpret_cast<float4*>(p.x_out + (size_t)t * C + c) = a;
+        });
+        tall_stats(row, C, l, 1 + g, s1, red[g], mean, rstd);
+        for (int c = 4 * l; c < C; c += 4 * TALL_GROUP) *reinterpret_cast<float4*>(row + c) = ln_apply(ld4(row + c), mean, rstd, ld4(p.ln_w + c), ld4(p.ln_b + c));
+    }
+    __syncthreads();
+    // eight channels of a row a thread: rows in neighbouring lanes
+    const int rr = threadIdx.x & 7, to = t0 + rr;
+    if (rr == TALL_ROWS || to >= T) return;
+    const float* const row = ln_tall + (size_t)(rr + 1) * pitch;
+    const bool shared = p.meta.tok_prev()[to] >= 0, commit = p.meta.tok_last()[to] != 0 && p.commit_dst;
+    const int slot = p.meta.tok_slot()[to];
+    const float* const before = shared ? row - pitch : p.shift_state + (size_t)slot * C;
+    for (int c = 8 * (threadIdx.x >> 3); c < C; c += TALL_THREADS) {
+        float4 a[2], sx[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const bool ok = c + 4 * e < C;
+            const float4 pv = ok ? ld4(before + c + 4 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            a[e] = ok ? ld4(row + c + 4 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
+            sx[e] = make_float4(pv.x - a[e].x, pv.y - a[e].y, pv.z - a[e].z, pv.w - a[e].w);
+            if (!ok) continue;
+            *reinterpret_cast<float4*>(p.xx_out + (size_t)to * C + c + 4 * e) = a[e];
+            if (p.sx_out) *reinterpret_cast<float4*>(p.sx_out + (size_t)to * C + c + 4 * e) = sx[e];
+            if (commit) *reinterpret_cast<float4*>(p.commit_dst + (size_t)slot * C + c + 4 * e) = ld4(p.commit_src + (size_t)to * C + c + 4 * e);
+        }
+        for (int m = 0; m < p.n_mix; ++m) {
+            uint2 h[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float4 mu = c + 4 * e < C ? ld4(p.mu[m] + c + 4 * e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                h[e] = make_uint2(pack_h2(a[e].x + sx[e].x * mu.x, a[e].y + sx[e].y * mu.y), pack_h2(a[e].z + sx[e].z * mu.z, a[e].w + sx[e].w * mu.w));
+            }
+            __half* const o = p.mix_out[m] + a16_index(to, c, p.kq_tile);
+            if (c + 4 < C) *reinterpret_cast<uint4*>(o) = make_uint4(h[0].x, h[0].y, h[1].x, h[1].y);
+            else *reinterpret_cast<uint2*>(o) = h[0];
+        }
+    }
+    trace_stamp(p.trace, 7);
+}
+
 // ---------------------------------------------------------------------------------------
 // Embedding gather + LN0 (reference: web-rwkv embeds on the CPU and runs ln0 on the device,
 // here the f16 table lives in HBM and both are one kernel).
@@ -481,6 +616,37 @@ __global__ void __launch_bounds__(LN_THREADS) ln_out_kernel(const __grid_constan
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     ln_out_row(p, t, red);
+}
+
+// Long prompt steps: a row to 64 threads, eight rows a CTA; few rows have logits, and the others stop at their residual.
+// (One row to a CTA whose 256 threads hold eight partial sums each left an SM one row: 54 us for 2048 rows of 2560; now 21.)
+__global__ void __launch_bounds__(TALL_THREADS, 2) ln_out_tall_kernel(const __grid_constant__ LnOutParams p) {
+    extern __shared__ __align__(16) float ln_tall[];
+    __shared__ float red[TALL_ROWS + 1][2];
+    pdl_launch_dependents();
+    const int C = p.C, g = threadIdx.x / TALL_GROUP, l = threadIdx.x % TALL_GROUP, t = blockIdx.x * (TALL_ROWS + 1) + g;
+    const bool live = t < p.meta.T();
+    const int slot = live ? p.meta.tok_slot()[t] : 0, out = live ? p.meta.tok_outrow()[t] : -1;
+    const bool commit = live && p.meta.tok_last()[t] != 0 && p.commit_dst;
+    pdl_wait();
+    if (!live) return;
+    if (commit)
+        for (int c = 4 * l; c < C; c += 4 * TALL_GROUP) *reinterpret_cast<float4*>(p.commit_dst + (size_t)slot * C + c) = ld4(p.commit_src + (size_t)t * C + c);
+    if (out < 0 && !p.hidden_out) return;
+    const ResidualSrc r = make_residual_src(p);
+    float* const row = ln_tall + (size_t)g * (C + TALL_PAD);
+    float s1 = 0.f, mean, rstd;
+    tall_residual(r, t, l, [&](const int c, const float4 a) {
+        s1 += (a.x + a.y) + (a.z + a.w);
+        if (out >= 0) *reinterpret_cast<float4*>(row + c) = a;
+        if (p.hidden_out) *reinterpret_cast<float4*>(p.hidden_out + (size_t)t * C + c) = a;
+    });
+    if (out < 0) return;
+    tall_stats(row, C, l, 1 + g, s1, red[g], mean, rstd);
+    for (int c = 4 * l; c < C; c += 4 * TALL_GROUP) {
+        const float4 y = ln_apply(ld4(row + c), mean, rstd, ld4(p.ln_w + c), ld4(p.ln_b + c));
+        *reinterpret_cast<uint2*>(p.head_in + a16_index(out, c, p.kq_tile)) = make_uint2(pack_h2(y.x, y.y), pack_h2(y.z, y.w));
+    }
 }
 
 }  // namespace b200
