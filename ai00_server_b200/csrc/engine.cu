@@ -41,6 +41,7 @@
 #include "latent_attn.cuh"
 #include "latent_prompt.cuh"
 #include "gla.cuh"
+#include "gla_chunk.cuh"
 #include "moe.cuh"
 #include "retention.cuh"
 #include "state_scan.cuh"
@@ -556,6 +557,7 @@ struct b200rwkv_engine {
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
     // column a thread, and a chain of tokens takes longer with two)
     bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }
+    bool gla_runs(int rows) const { return rows >= GC_RUN * std::max(1, step_seqs); }      // a run of tokens a sequence or more
     // Recurrences of prompt steps that have at most one CTA an SM: each asks for more than half an SM's shared memory, so that no two share one.  They start early
     // (programmatic launches), when most SMs are full of the projections in front of them, were packed onto the few that were not and took turns there.
     // Measured (whole prompts, four layers of width 2560): one of 200 tokens 988 -> 856 us; two layers of gated delta rule, matrix memory and attention of width 2048:

@@ -128,6 +128,7 @@ void b200rwkv_engine::ff_load(const StFile& st, KxSizes& z) {
     }
     sa_plan_model(m);
     CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
+    allow_smem(gla_chunk_kernel, GC_SMEM);
     CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     REQUIRE((size_t)W * 8 <= 200 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the norm kernel");
     CK(cudaFuncSetAttribute(pre_norm_kernel<NORM_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

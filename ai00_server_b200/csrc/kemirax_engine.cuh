@@ -285,6 +285,7 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
         allow_smem(latent_prompt_kernel<false>, latent_prompt_smem(LP_MAX_D, LP_MAX_RK));
     }
     CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
+    allow_smem(gla_chunk_kernel, GC_SMEM);
     CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
@@ -449,15 +450,19 @@ void b200rwkv_engine::kx_short_conv(cudaStream_t s, Profiler* prof, const ShortC
     if (cp.taps > 1) launch_k(conv_commit_kernel, dim3(nslot_grid, cb), dim3(256), 0, cp, KC_OTHER, s, prof);
 }
 
-// gated linear attention of a layer: the recurrence, and the norm over heads that are spread over several CTAs
+// Gated linear attention of a layer: the recurrence, and the norm over heads that are spread over several CTAs.  Sixteen tokens at a time (gla_chunk.cuh) where sequences have
+// as many and heads are not much narrower than its tiles; 16 heads of 128 x 128, eight sequences: 256 tokens 256 us token by token and 69 in runs, 20 tokens of sixteen 38 and
+// 31, 8 tokens of 64 sequences 63 and 76; 64 tokens of sixteen sequences, heads of 64 x 64 49 and 44, of 32 x 32 42 and 43.
 void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, int H_, int dk, int dv, const float* q, const float* k, const float* v,
                              const float* gate, int ld, float* out, int ldo, int rows, int nslot_grid, bool decode) {
     SeqModel& m = *kx;
     const ScanShape sh = scan_shape(dk, dv, 3, decode, scan_wide(H_));
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
-    launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
-    if (sh.ncta > 1) kx_head_norm(s, prof, gp.norm, rows, decode);
+    const bool runs = !decode && gla_runs(rows) && std::max(dk, dv) > 32 && dk <= GC_DMAX && dv <= GC_DMAX;
+    if (runs) launch_k(gla_chunk_kernel, dim3(H_, scan_slots(nslot_grid)), dim3(GC_THREADS), GC_SMEM, gp, KC_WKV, s, prof);
+    else launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
+    if (runs || sh.ncta > 1) kx_head_norm(s, prof, gp.norm, rows, decode);
 }
 
 void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool decode, int nsplit, Profiler* prof) {
@@ -708,7 +713,9 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     for (const KxLayer& l : kx->layers)
         for (int h : {l.c.heads, l.c.mm_heads})
             if (!decode && h > 0 && h < 256 && scan_wide(h) && (wide == 0 || h < wide)) wide = h;
-    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22);
+    bool runs = false;                     // and whether gated linear attention takes them in runs
+    for (const KxLayer& l : kx->layers) runs = runs || (!decode && (l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows));
+    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

@@ -101,7 +101,6 @@ def test_latent_attention(heads, kv_rank, rot_dim):
     _check(synth.make_kemirax, kemirax_numpy, [K("latent_attention", heads=heads, kv_rank=kv_rank, rot_dim=rot_dim, experts=6, top=3)], 0, width=96)
 
 
-@pytest.mark.parametrize("n", [17, 100, 300])
 @pytest.mark.parametrize("heads, kv_rank, rot_dim", [(16, 128, 64), (3, 20, 4), (8, 200, 24)])
 def test_latent_attention_at_the_edges_of_key_tiles(heads, kv_rank, rot_dim):
     """Contexts below, at and behind the borders of 32-key tiles, latent rows of one, part of one and several pieces of 128 entries, of multiples of eight and of four."""
@@ -120,6 +119,7 @@ def test_latent_attention_at_the_edges_of_key_tiles(heads, kv_rank, rot_dim):
         m.close()
 
 
+@pytest.mark.parametrize("n", [17, 100, 300])
 @pytest.mark.parametrize("ranks", [(64, 128), (32, 32), (64, 64)])
 def test_low_rank_second_stages(ranks, n):
     """Both kernels of lora2.cuh at every rank they are built for, one tile of tokens and several."""
