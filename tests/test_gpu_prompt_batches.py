@@ -95,6 +95,31 @@ def test_gated_linear_attention(dim, vdim):
     _check(synth.make_kemirax, kemirax_numpy, [K("gla", heads=2, dim=dim, vdim=vdim, mlp=False)], 1, width=96)
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dim, vdim, tau", [(128, 128, 8.0), (72, 40, 8.0), (34, 33, 8.0), (128, 128, 0.5), (40, 128, 0.02)])
+def test_gated_linear_attention_in_runs(dim, vdim, tau, precision):
+    """Sequences of about a run of sixteen tokens, several and parts of them, continued in a second call; sizes that are no multiples of eight or four; decays that cut runs short,
+    and such that tokens go one by one."""
+    cfg, st, w = synth.make_kemirax([K("gla", heads=3, dim=dim, vdim=vdim, tau=tau, mlp=False)], seed=8, width=96)
+    lens = [15, 16, 17, 33, 120]
+    toks = [np.random.default_rng(n).integers(1, 90, n + 21).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, precision=precision, config=cfg, kv_tokens=512)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        opt = [capi.OPTION_FULL] * len(lens)
+        got = m.infer_raw(list(range(len(lens))), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw(list(range(len(lens))), [21] * len(lens), sum((t[n:] for t, n in zip(toks, lens)), []), opt)
+        for s in range(len(lens)):
+            err = _errs(np.concatenate([got[s], more[s]]), kemirax_numpy.run(json.loads(cfg), w, toks[s]))
+            if precision == 1:
+                assert err.max() <= TIGHT, (s, int(err.argmax()), float(err.max()))
+            else:
+                assert np.median(err) <= BF16_TOL and err.max() <= ROW_TOL, (s, float(np.median(err)), int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("heads, kv_rank, rot_dim", [(4, 24, 8), (16, 40, 16), (5, 72, 4), (20, 64, 8)])
 def test_latent_attention(heads, kv_rank, rot_dim):
     """64 rows of 4, 16, 5 and 20 (two CTAs) heads; latent rows with and without pad columns; channels that do not fill eight warps."""
