@@ -47,6 +47,7 @@
 #include "state_scan.cuh"
 #include "delta_rule.cuh"
 #include "matrix_memory.cuh"
+#include "delta_chunk.cuh"
 #include "window_attn.cuh"
 #include "bias_attn.cuh"
 #include "hyper.cuh"
@@ -558,6 +559,10 @@ struct b200rwkv_engine {
     // column a thread, and a chain of tokens takes longer with two)
     bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }
     bool gla_runs(int rows) const { return rows >= GC_RUN * std::max(1, step_seqs); }      // a run of tokens a sequence or more
+    // Recurrences with one decay a head: three runs a sequence or more, heads wider than half the tiles or a quarter.  Sixteen heads of 128 x 128, token by token and in runs: delta rule,
+    // 128 tokens of sixteen sequences 208 and 103 us, 50 of three (72 x 40) 35 and 29, 33 of two 25 and 27, 20 of sixteen 41 and 41, 8 of 64 62 and 107; 64 of sixteen, heads of 64 x 64
+    // 60 and 57, of 32 x 32 50 and 55.  Matrix memory: 128 of sixteen 213 and 131, 64 of eight (four heads) 42 and 39, 20 of sixteen 44 and 48; heads of 64 x 64 58 and 72.
+    bool run_chunks(int rows, int dk, int dv, int above) const { return rows >= 3 * GC_RUN * std::max(1, step_seqs) && std::max(dk, dv) > above && dk <= GC_DMAX && dv <= GC_DMAX; }
     // Recurrences of prompt steps that have at most one CTA an SM: each asks for more than half an SM's shared memory, so that no two share one.  They start early
     // (programmatic launches), when most SMs are full of the projections in front of them, were packed onto the few that were not and took turns there.
     // Measured (whole prompts, four layers of width 2560): one of 200 tokens 988 -> 856 us; two layers of gated delta rule, matrix memory and attention of width 2048:

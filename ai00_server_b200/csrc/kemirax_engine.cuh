@@ -713,8 +713,9 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     for (const KxLayer& l : kx->layers)
         for (int h : {l.c.heads, l.c.mm_heads})
             if (!decode && h > 0 && h < 256 && scan_wide(h) && (wide == 0 || h < wide)) wide = h;
-    bool runs = false;                     // and whether gated linear attention takes them in runs
-    for (const KxLayer& l : kx->layers) runs = runs || (!decode && (l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows));
+    bool runs = false;                     // and whether they take the tokens in runs
+    for (const KxLayer& l : kx->layers)
+        runs = runs || (!decode && (((l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows)) || ((l.c.mixer == KX_PARALLEL || l.c.mixer == KX_DELTA) && run_chunks(rows, GC_DMAX, GC_DMAX, 0))));
     const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {

@@ -137,6 +137,8 @@ void b200rwkv_engine::pn_load(const StFile& st, KxSizes& z) {
     sa_plan_model(m);
     CK(cudaFuncSetAttribute(delta_scan_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     CK(cudaFuncSetAttribute(delta_scan_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
+    allow_smem(run_chunk_kernel<true>, DC_SMEM);
+    allow_smem(run_chunk_kernel<false>, DC_SMEM);
     CK(cudaFuncSetAttribute(matrix_memory_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     CK(cudaFuncSetAttribute(matrix_memory_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     REQUIRE((size_t)W * 4 <= 200 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the norm kernel");
@@ -200,8 +202,14 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 MatrixMemoryParams mp{m.pr + r.mq, m.pr + r.mk, m.pr + r.mv, PN, m.pr + r.mi, m.pr + r.mf, l.mm_state, l.mm_n, l.mm_m, m.z, Hm, mk, mvd,
                                       c.mm_cap, 1.f / sqrtf((float)mk), 1e-6f, sh,
                                       {m.vout + H_ * dv, KO, m.z, m.pr + r.mg, PN, l.mm_norm_w, mvd, Hm, mvd, eps, c.mm_mul, 0, mv}};
-                launch_k(decode ? matrix_memory_kernel<0> : (sh.nc == 2 ? matrix_memory_kernel<2> : matrix_memory_kernel<1>), dim3(Hm * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), mp, KC_WKV, s2, prof);
-                if (sh.ncta > 1) kx_head_norm(s2, prof, mp.norm, rows, decode);
+                const bool runs = !decode && run_chunks(rows, mk, mvd, 64);
+                if (runs) {
+                    RunChunkParams cp{mp.q, mp.k, mp.v, PN, 1, mp.zf, PN, mp.zi, PN, nullptr, mp.state, mp.n, mp.m, mp.fac, Hm, mk, mvd, mp.q_scale, mp.den_eps, mp.cap, sh, mp.norm};
+                    launch_k(run_chunk_kernel<false>, dim3(Hm, scan_slots(nslot_grid)), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s2, prof);
+                } else {
+                    launch_k(decode ? matrix_memory_kernel<0> : (sh.nc == 2 ? matrix_memory_kernel<2> : matrix_memory_kernel<1>), dim3(Hm * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), mp, KC_WKV, s2, prof);
+                }
+                if (runs || sh.ncta > 1) kx_head_norm(s2, prof, mp.norm, rows, decode);
             }
             RotPrepParams rp{m.pr + r.q, m.pr + r.k, m.pr + r.v, PN, m.q, H_ * dk, l.cache, m.d_table, m.npages, m.page, l.qn_w, l.kn_w, l.freq_d,
                              H_, G_, dk, dv, c.rot.dims, eps, mv, m.sm};
@@ -226,8 +234,14 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             const ScanShape sh = scan_shape(dk, dv, 2, decode, scan_wide(H_));
             DeltaScanParams dp{m.cv, m.cv + G_ * dk, m.cv + 2 * G_ * dk, ldc, m.pr + r.a, PN, m.pr + r.b, PN, l.a_log, l.rec_state, H_, G_, dk, dv,
                                1.f / sqrtf((float)dk), 1e-6f, sh, {m.vout, KO, nullptr, m.pr + r.g, PN, l.norm_w, 0, H_, dv, eps, 1.f, 1, mv}};
-            launch_k(decode ? delta_scan_kernel<false, 0> : (sh.nc == 2 ? delta_scan_kernel<false, 2> : delta_scan_kernel<false, 1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
-            if (sh.ncta > 1) kx_head_norm(s, prof, dp.norm, rows, decode);
+            const bool runs = !decode && run_chunks(rows, dk, dv, 32);
+            if (runs) {
+                RunChunkParams cp{dp.q, dp.k, dp.v, ldc, H_ / G_, dp.z, PN, dp.b, PN, l.a_log, l.rec_state, nullptr, nullptr, nullptr, H_, dk, dv, dp.q_scale, dp.unit_eps, 0.f, sh, dp.norm};
+                launch_k(run_chunk_kernel<true>, dim3(H_, scan_slots(nslot_grid)), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s, prof);
+            } else {
+                launch_k(decode ? delta_scan_kernel<false, 0> : (sh.nc == 2 ? delta_scan_kernel<false, 2> : delta_scan_kernel<false, 1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
+            }
+            if (runs || sh.ncta > 1) kx_head_norm(s, prof, dp.norm, rows, decode);
         }
         kx_lin(s, prof, lin(m.vout, KO, l.o, m.y, W, W, KO), rows, 1);
         post_w = l.norm1b_w;

@@ -120,6 +120,31 @@ def test_gated_linear_attention_in_runs(dim, vdim, tau, precision):
         m.close()
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("layer", [P("delta", heads=2, dim=128, vdim=128, conv=4), P("delta", heads=3, dim=72, vdim=40, conv=4), P("delta", heads=4, kv_heads=2, dim=34, vdim=33, conv=4),
+                                   P("parallel", mm_heads=2, mm_dim=128), P("parallel", mm_heads=3, mm_dim=72, mm_vdim=40), P("parallel", mm_heads=2, mm_dim=33, mm_vdim=66)])
+def test_recurrences_with_one_decay_a_head_in_runs(layer, precision):
+    """Sequences of about a run of sixteen tokens, several and parts of them, continued in a second call; sizes that are no multiples of eight or four; keys of two heads in common."""
+    cfg, st, w = synth.make_panupel([layer], seed=8, width=96, loop=None)
+    lens = [15, 16, 17, 33, 200]
+    toks = [np.random.default_rng(n).integers(1, 90, n + 50).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, precision=precision, config=cfg, kv_tokens=1024)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        opt = [capi.OPTION_FULL] * len(lens)
+        got = m.infer_raw(list(range(len(lens))), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw(list(range(len(lens))), [50] * len(lens), sum((t[n:] for t, n in zip(toks, lens)), []), opt)
+        for s in range(len(lens)):
+            err = _errs(np.concatenate([got[s], more[s]]), panupel_numpy.run(json.loads(cfg), w, toks[s]))
+            if precision == 1:
+                assert err.max() <= TIGHT, (s, int(err.argmax()), float(err.max()))
+            else:
+                assert np.median(err) <= BF16_TOL and err.max() <= ROW_TOL, (s, float(np.median(err)), int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("heads, kv_rank, rot_dim", [(4, 24, 8), (16, 40, 16), (5, 72, 4), (20, 64, 8)])
 def test_latent_attention(heads, kv_rank, rot_dim):
     """64 rows of 4, 16, 5 and 20 (two CTAs) heads; latent rows with and without pad columns; channels that do not fill eight warps."""
