@@ -4,8 +4,8 @@
 // What bounds it: the chain of tokens of one (head, sequence), 64-odd CTAs for one prompt.  The decode kernel spends four barriers, a
 // round trip to memory and the norm of one warp on every token (2.6 us a token at 7B widths, the decay LoRA evaluated in place); here
 // the loop over tokens has NO barrier and no memory latency:
-//   * the vectors of the next TC tokens are requested while TC tokens run, and what does not depend on the state (v7: unit key, removal /
-//     write vectors, value residual, bonus) is worked out per group of tokens, a warp per token;
+//   * the vectors of the next TC tokens are requested while TC tokens run.  RWKV-5 / 6 copy them to their places as they are (cp.async, no registers: 94 instead of 162, so that
+//     five CTAs of an SM run instead of three); RWKV-7 works out what does not depend on the state (unit key, removal / write vectors, value residual, bonus) per group, a warp per token;
 //   * a thread holds 4 values x 8 neighbouring keys of the state; key-indexed vectors lie in shared memory with each run of eight split into
 //     two half rows, so that the eight lanes of a value row read 128 contiguous bytes and the other three rows of the warp share them;
 //   * products run as packed pairs of neighbouring keys (half the instructions of a loop that is bound by them); RWKV-5 / 6: the bonus of the current
@@ -15,7 +15,9 @@
 //     keys apart: results agree with wkv.cuh's to f32 rounding.
 // Decays come from the decay projection's own launch in these steps (lora2.cuh: 6 us beside the scan's own time below).  Where the decode kernel
 // evaluates that low-rank stage itself (RWKV-6), its sums run in another order: decays, and with them states, agree to f32 rounding and not to the bit.
-// Measured (one prompt of 100 tokens, 64 heads, ncu): 30 us a layer (33 with single products and exchanges in the loop, 263 in the decode kernel).
+// Measured, RWKV-6 (vectors through registers and three CTAs an SM before, copied and five now): 64 tokens of 32 sequences, 40 heads, 93 -> 78 us, 128 of sixteen, 64 heads, 141 -> 119, 61 of six
+// 25 -> 25, one prompt of 100, 64 heads, 29 -> 29 (263 in the decode kernel).  At five CTAs the path to shared memory is busy 73 % of the time, issue slots 53 %, multiply-adds 46 %;
+// eight values a thread halve its reads but leave two warps a head (97 us at the first of these).
 #pragma once
 #include "f32x2.cuh"
 #include "wkv.cuh"
@@ -24,7 +26,9 @@ namespace b200 {
 
 constexpr int WKS_THREADS = 128;
 template <int VER> struct WksCfg {
-    static constexpr int TC = VER == 7 ? 8 : 16;            // tokens per group
+    static constexpr int TC = 8;                            // tokens per group
+    static constexpr int CTAS = VER == 7 ? 3 : 5;           // of an SM
+    static constexpr int UNROLL = VER == 7 ? 2 : 1;         // (RWKV-6: two tokens at a time are 80 us instead of 78 in the step below)
     static constexpr int NA = VER == 7 ? 6 : 4;             // staged vectors: r, k, v, w (, -kk, kk a)
     static constexpr int BUF = NA * TC * WKV_N;             // floats of one group
     static constexpr int OUT_ROW = WKV_N + 4, OUT = 8 * OUT_ROW;      // a token's read-outs: eight partial sums of every value (padded: conflict-free)
@@ -34,7 +38,7 @@ template <int VER> struct WksCfg {
 __device__ __forceinline__ int wks_place(int c) { return (c >> 3) * 4 + (c & 3) + ((c >> 2) & 1) * 32; }
 
 template <int VER>
-__global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_constant__ WkvParams p) {
+__global__ void __launch_bounds__(WKS_THREADS, WksCfg<VER>::CTAS) wkv_scan_kernel(const __grid_constant__ WkvParams p) {
     using Cfg = WksCfg<VER>;
     constexpr int TC = Cfg::TC, TW = TC / 4;                // tokens per warp in the per-group phases
     extern __shared__ __align__(16) float wks[];
@@ -57,14 +61,25 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
     const int c2 = ch + lane;                               // the per-group phases give a lane the channels lane and lane + 32
     auto ld2 = [](const float* q) { return make_float2(q[0], q[32]); };
     const float2 lw = ld2(p.lnx_w + c2), lb = ld2(p.lnx_b + c2);
-    float2 kk_ = make_float2(0.f, 0.f), ka_ = kk_, rk_ = kk_, ws = kk_;
+    float2 kk_ = make_float2(0.f, 0.f), ka_ = kk_, rk_ = kk_, u2 = kk_;
     if (VER == 7) { kk_ = ld2(p.k_k + c2); ka_ = ld2(p.k_a + c2); rk_ = ld2(p.r_k + c2); }
-    if (VER == 5) ws = ld2(p.w_static + c2);
-    const float2 u2 = VER != 7 ? ld2(p.u + c2) : make_float2(0.f, 0.f);
+    if (VER != 7) u2 = make_float2(p.u[ch + (lane >> 2) * 8 + (lane & 3)], p.u[ch + (lane >> 2) * 8 + 4 + (lane & 3)]);      // the keys at places lane and lane + 32
     pdl_wait();
 
+    // RWKV-5 / 6: the vectors go to their places as they are, sixteen bytes a copy
+    auto copy = [&](const int g0, const int b) {
+        constexpr int ARR = VER == 6 ? 4 : 3;
+#pragma unroll
+        for (int x = tid; x < ARR * TC * 16; x += WKS_THREADS) {
+            const int arr = x / (TC * 16), tt = x / 16 % TC, c = x & 15;
+            const float* const src = arr == 0 ? p.r : (arr == 1 ? p.k : (arr == 2 ? p.v : p.w));
+            float* const d = wks + b * Cfg::BUF + (arr * TC + tt) * WKV_N + (arr == 2 ? 4 * c : (c >> 1) * 4 + (c & 1) * 32);
+            if (g0 + tt < nt) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_u32(d)), "l"(src + (size_t)(t0 + g0 + tt) * p.ld + ch + 4 * c) : "memory");
+        }
+    };
+    auto landed = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
     struct Row { float2 r, k, v, w, a, nu, vf; };
-    Row row[TW];
+    Row row[VER == 7 ? TW : 1];
     auto request = [&](const int g0) {                      // the group's vectors -> registers
 #pragma unroll
         for (int i = 0; i < TW; ++i) {
@@ -72,11 +87,9 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
             if (t >= nt) continue;
             const size_t at = (size_t)(t0 + t) * p.ld + c2;
             row[i].r = ld2(p.r + at); row[i].k = ld2(p.k + at); row[i].v = ld2(p.v + at);
-            if (VER != 5) row[i].w = ld2(p.w + at);
-            if (VER == 7) {
-                row[i].a = ld2(p.a + at);
-                if (!p.layer0) { row[i].nu = ld2(p.nu + at); row[i].vf = ld2(p.v_first + at); }
-            }
+            row[i].w = ld2(p.w + at);
+            row[i].a = ld2(p.a + at);
+            if (!p.layer0) { row[i].nu = ld2(p.nu + at); row[i].vf = ld2(p.v_first + at); }
         }
     };
     auto prepare = [&](const int g0, const int b) {         // registers -> shared memory, with all that the state does not enter
@@ -93,37 +106,37 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
             if (t >= nt) continue;                          // warp-uniform
             const float2 r = row[i].r;
             float2 k = row[i].k, v = row[i].v;
-            if (VER == 7) {
-                const float2 a = row[i].a;
-                float2 kk = make_float2(k.x * kk_.x, k.y * kk_.y);
-                const float norm = fmaxf(sqrtf(sum2(make_float2(kk.x * kk.x, kk.y * kk.y))), 1e-12f);
-                kk.x /= norm; kk.y /= norm;
-                k.x *= 1.f + (a.x - 1.f) * ka_.x; k.y *= 1.f + (a.y - 1.f) * ka_.y;
-                if (p.layer0) {
-                    float* const d = p.v_first + (size_t)(t0 + t) * p.ld + c2;
-                    d[0] = v.x; d[32] = v.y;
-                } else { v.x += (row[i].vf.x - v.x) * row[i].nu.x; v.y += (row[i].vf.y - v.y) * row[i].nu.y; }
-                const float bonus = sum2(make_float2(r.x * k.x * rk_.x, r.y * k.y * rk_.y));
-                if (lane == 0) sc[b * TC + tt] = bonus;
-                st2(4, tt, make_float2(-kk.x, -kk.y));
-                st2(5, tt, make_float2(kk.x * a.x, kk.y * a.y));
-            }
-            if (VER != 7) {
-                const float bonus = sum2(make_float2(r.x * (u2.x * k.x), r.y * (u2.y * k.y)));
-                if (lane == 0) sc[b * TC + tt] = bonus;
-            }
+            const float2 a = row[i].a;
+            float2 kk = make_float2(k.x * kk_.x, k.y * kk_.y);
+            const float norm = fmaxf(sqrtf(sum2(make_float2(kk.x * kk.x, kk.y * kk.y))), 1e-12f);
+            kk.x /= norm; kk.y /= norm;
+            k.x *= 1.f + (a.x - 1.f) * ka_.x; k.y *= 1.f + (a.y - 1.f) * ka_.y;
+            if (p.layer0) {
+                float* const d = p.v_first + (size_t)(t0 + t) * p.ld + c2;
+                d[0] = v.x; d[32] = v.y;
+            } else { v.x += (row[i].vf.x - v.x) * row[i].nu.x; v.y += (row[i].vf.y - v.y) * row[i].nu.y; }
+            const float bonus = sum2(make_float2(r.x * k.x * rk_.x, r.y * k.y * rk_.y));
+            if (lane == 0) sc[b * TC + tt] = bonus;
+            st2(4, tt, make_float2(-kk.x, -kk.y));
+            st2(5, tt, make_float2(kk.x * a.x, kk.y * a.y));
             st2(0, tt, r); st2(1, tt, k);
             buf[(2 * TC + tt) * WKV_N + lane] = v.x;        // by value
             buf[(2 * TC + tt) * WKV_N + lane + 32] = v.y;
-            st2(3, tt, VER == 5 ? ws : row[i].w);
+            st2(3, tt, row[i].w);
         }
     };
-    request(0);
-    prepare(0, 0);
+    if (VER == 7) { request(0); prepare(0, 0); }
+    else {
+        copy(0, 0);
+        if (VER == 5)
+            for (int x = tid; x < 2 * TC * WKV_N; x += WKS_THREADS) wks[(x / (TC * WKV_N)) * Cfg::BUF + (3 * TC + x / WKV_N % TC) * WKV_N + wks_place(x % WKV_N)] = p.w_static[ch + x % WKV_N];
+        landed();
+    }
     __syncthreads();
     for (int g0 = 0, b = 0; g0 < nt; g0 += TC, b ^= 1) {
         const int n = min(TC, nt - g0);
-        request(g0 + TC);
+        if (VER == 7) request(g0 + TC);
+        else copy(g0 + TC, b ^ 1);
         float2 gate[TW];
 #pragma unroll
         for (int i = 0; i < TW; ++i) {
@@ -131,7 +144,7 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
             gate[i] = t < nt ? ld2(p.g + (size_t)(t0 + t) * p.ld + c2) : make_float2(0.f, 0.f);
         }
         const float* const buf = wks + b * Cfg::BUF;
-#pragma unroll 2
+#pragma unroll (Cfg::UNROLL)
         for (int tt = 0; tt < n; ++tt) {
             auto ld8 = [&](const int arr, f32x2 (&x)[4]) {
                 const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(buf + (arr * TC + tt) * WKV_N + 4 * j);
@@ -186,7 +199,8 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
             }
             *reinterpret_cast<float4*>(so + tt * Cfg::OUT + j * Cfg::OUT_ROW + ig * 4) = make_float4(o[0], o[1], o[2], o[3]);
         }
-        prepare(g0 + TC, b ^ 1);
+        if (VER == 7) prepare(g0 + TC, b ^ 1);
+        else landed();
         __syncthreads();
         // GroupNorm over the head (+ bonus) * gate -> operand of the output projection, a warp per token
 #pragma unroll
@@ -199,7 +213,12 @@ __global__ void __launch_bounds__(WKS_THREADS, 3) wkv_scan_kernel(const __grid_c
                 const float2 y = ld2(so + tt * Cfg::OUT + q * Cfg::OUT_ROW + lane);
                 x.x += y.x; x.y += y.y;
             }
-            const float s = sc[b * TC + tt];
+            float s;
+            if (VER == 7) s = sc[b * TC + tt];
+            else {
+                const float2 r = ld2(buf + tt * WKV_N + lane), k = ld2(buf + (TC + tt) * WKV_N + lane);      // by place
+                s = warp_sum(r.x * (u2.x * k.x)) + warp_sum(r.y * (u2.y * k.y));
+            }
             const float2 v = ld2(buf + (2 * TC + tt) * WKV_N + lane);
             if (VER != 7) { x.x = fmaf(s, v.x, x.x); x.y = fmaf(s, v.y, x.y); }
             const float mean = warp_sum(x.x + x.y) * (1.f / WKV_N);
