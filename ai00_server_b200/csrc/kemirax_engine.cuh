@@ -546,9 +546,9 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 launch_k(D % 8 == 0 ? latent_prompt_kernel<true> : latent_prompt_kernel<false>, dim3(cdiv(rows, lp.qt) + nslot_grid, cdiv(H_, lp.hg)), dim3(LP_THREADS), latent_prompt_smem(D, rk), lp, KC_WKV, s, prof);
             } else if (!m.exact) {         // serving precision: both products on the tensor cores (TF32 operands, f32 accumulation and softmax)
                 const size_t sm_b = latent_attn_tc_smem(D);
-                if (!decode) launch_k(latent_attn_tc_kernel<4, 4>, dim3(cdiv(rows, 4) + nslot_grid, cdiv(H_, 4), nsplit), dim3(LA_THREADS), sm_b, ap, KC_WKV, s, prof);
-                else if (H_ > 8) launch_k(latent_attn_tc_kernel<1, 16>, dim3(rows, cdiv(H_, 16), nsplit), dim3(LA_THREADS), sm_b, ap, KC_WKV, s, prof);
-                else launch_k(latent_attn_tc_kernel<2, 8>, dim3(rows, cdiv(H_, 8), nsplit), dim3(LA_THREADS), sm_b, ap, KC_WKV, s, prof);
+                if (!decode) launch_k(latent_attn_tc_kernel<4, 4>, dim3(cdiv(rows, 4) + nslot_grid, cdiv(H_, 4), nsplit), dim3(LT_THREADS), sm_b, ap, KC_WKV, s, prof);
+                else if (H_ > 8) launch_k(latent_attn_tc_kernel<1, 16>, dim3(rows, cdiv(H_, 16), nsplit), dim3(LT_THREADS), sm_b, ap, KC_WKV, s, prof);
+                else launch_k(latent_attn_tc_kernel<2, 8>, dim3(rows, cdiv(H_, 8), nsplit), dim3(LT_THREADS), sm_b, ap, KC_WKV, s, prof);
             } else if (!decode) {
                 launch_k(latent_attn_kernel<4, 4>, dim3(cdiv(rows, 4) + nslot_grid, cdiv(H_, 4), nsplit), dim3(LA_THREADS), latent_attn_smem<4, 4>(D), ap,
                          KC_WKV, s, prof);

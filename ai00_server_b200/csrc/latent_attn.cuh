@@ -296,10 +296,13 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_kernel(const LatentAtt
 // ------------------------------------------------------------------------------------------------------------------
 // Tensor-core variant for the serving precision: the same CTA shape (16 (token, head) rows, 32-key tiles, online softmax in
 // f32) with both products on mma.sync m16n8k8 TF32 (operands rounded to TF32, f32 accumulation):
-//   scores  S[16 x 32]  = Q[16 x D] . K^T      warp w owns keys 8w .. 8w+7, D / 8 k-steps
-//   output  O[16 x rk] += P[16 x 32] . C       warp w owns a quarter of the latent channels, 4 k-steps per 8 channels
+//   scores  S[16 x 32]  = Q[16 x D] . K^T      warp w owns keys 8 (w % 4) .. + 7 and half of the channels, in two chains of sums
+//   output  O[16 x rk] += P[16 x 32] . C       warp w owns an eighth of the latent channels, 4 k-steps per 8 channels
 // Scores go through shared memory between the two so that the softmax keeps the row-per-warp form of the f32 kernel.
-// Row strides are = 4 (mod 32) floats: fragment loads of the score phase are bank-conflict free.
+// Row strides are = 4 (mod 32) floats: fragment loads are bank-conflict free in the score phase, and in the output phase with keys 2 t and 2 t + 1 of eight in the places t and t + 4.
+// What bounds it: the chain of a CTA that holds two or three tiles (fetch, scores, softmax, output), not bytes.  A row is fetched by a warp (one division by the page size a row; one
+// for every sixteen bytes, and the queries word by word with two more, before).
+// Measured (a decode step of sixteen sequences of 780 keys, 16 heads, rank 512 and 64 rotated, in place): 63 us of the step -> 29.
 // ------------------------------------------------------------------------------------------------------------------
 // nearest TF32 value, ties away from zero (what cvt.rna does), in integer operations: every operand of every product is rounded, and the
 // conversion's issue rate was what the two products waited for.  A NaN stays one (the addition would carry it into another value).
@@ -312,12 +315,12 @@ __device__ __forceinline__ void mma_tf32_1688(float c[4], const uint32_t a[4], c
 __host__ __device__ inline int la_pad8(int n) { return (n + 7) & ~7; }
 __host__ __device__ inline int la_stride(int D) { const int dp = la_pad8(D); return dp + ((4 - dp % 32) + 32) % 32; }
 __host__ __device__ inline size_t latent_attn_tc_smem(int D) {
-    return ((size_t)16 * la_stride(D) + (size_t)LA_KT * la_stride(D) + 16 * 36 + 64) * sizeof(float);
+    return ((size_t)16 * la_stride(D) + (size_t)LA_KT * la_stride(D) + 2 * 16 * 32 + 64) * sizeof(float);      // two CTAs of an SM at 576 channels
 }
-constexpr int LA_TC_MAX_NT = 16;                   // 8-channel tiles per warp: rk <= 512
+constexpr int LT_THREADS = 256, LT_MAX_NT = 8;     // 8-channel tiles per warp: rk <= 512
 
 template <int QB, int HG>
-__global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const LatentAttnParams p) {
+__global__ void __launch_bounds__(LT_THREADS) latent_attn_tc_kernel(const LatentAttnParams p) {
     pdl_launch_dependents();
     pdl_wait();
     static_assert(QB * HG == 16, "one m16 tile of (token, head) rows");
@@ -336,78 +339,94 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
     extern __shared__ __align__(16) float la_tc_smem[];
     float* sq = la_tc_smem;                        // [16][DS]
     float* sk = sq + (size_t)16 * DS;              // [LA_KT][DS]
-    float* ss = sk + (size_t)LA_KT * DS;           // [16][36] scores, then probabilities
-    float* scorr = ss + 16 * 36;                   // [16] rescale of the running output
+    float* ss = sk + (size_t)LA_KT * DS;           // [2][16][32] scores of the two halves of the channels (columns turned: at()); probabilities in the first
+    float* scorr = ss + 2 * 16 * 32;               // [16] rescale of the running output
     float* sml = scorr + 16;                       // [16][2] final (m, l)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
-
-    for (int e = threadIdx.x; e < 16 * DS; e += LA_THREADS) {
-        const int r = e / DS, d = e % DS;
+    const int* tab = p.table + (size_t)slot * p.stride;
+    const bool vec = (D % 4 == 0);
+    auto at = [](const int r, const int c) { return r * 32 + (c ^ ((r & 7) << 2)); };
+    auto fetch = [&](const int kb) {               // a row of the cache per warp and turn
+        for (int j = warp; j < LA_KT; j += LT_THREADS / 32) {
+            const int kj = kb + j;
+            float* const dst = sk + (size_t)j * DS;
+            if (kj < nkeys) {
+                const float* const src = p.cache + ((size_t)tab[kj / p.page] * p.page + kj % p.page) * D;
+                if (vec) {
+                    const uint32_t da = (uint32_t)__cvta_generic_to_shared(dst);
+                    for (int c = lane; c < D / 4; c += 32) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(da + 16 * c), "l"(src + 4 * c) : "memory");
+                } else {
+                    for (int d = lane; d < D; d += 32) dst[d] = src[d];
+                }
+            } else {
+                for (int d = lane; d < D; d += 32) dst[d] = 0.f;
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    if (tile_lo < tile_hi) fetch(tile_lo * LA_KT);
+#pragma unroll
+    for (int r = warp; r < 16; r += LT_THREADS / 32) {
         const int qi = r / HG, h = h0 + r % HG;
-        sq[e] = (d < D && qi < nt && h < p.H) ? __uint_as_float(to_tf32(p.q[(size_t)(t0 + qi) * p.H * D + (size_t)h * D + d])) : 0.f;
+        const bool live = qi < nt && h < p.H;
+        const float* const src = p.q + (live ? (size_t)(t0 + qi) * p.H * D + (size_t)h * D : 0);
+        float* const dst = sq + (size_t)r * DS;
+        if (vec) {
+            for (int c = lane; c < D / 4; c += 32) {
+                const float4 x = live ? *reinterpret_cast<const float4*>(src + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<uint4*>(dst + 4 * c) = make_uint4(to_tf32(x.x), to_tf32(x.y), to_tf32(x.z), to_tf32(x.w));
+            }
+        } else {
+            for (int d = lane; d < D; d += 32) dst[d] = live ? __uint_as_float(to_tf32(src[d])) : 0.f;
+        }
+        for (int d = D + lane; d < DS; d += 32) dst[d] = 0.f;
     }
-    for (int e = threadIdx.x; e < LA_KT * (DS - D); e += LA_THREADS) {       // pad columns of the key tile stay zero
-        const int j = e / (DS - D), d = D + e % (DS - D);
-        sk[(size_t)j * DS + d] = 0.f;
-    }
-    constexpr int RPW = 4;
+    for (int j = warp; j < LA_KT; j += LT_THREADS / 32)       // pad columns of the key tile stay zero
+        for (int d = D + lane; d < DS; d += 32) sk[(size_t)j * DS + d] = 0.f;
+    constexpr int RPW = 16 / (LT_THREADS / 32);
     float m[RPW], l[RPW];
 #pragma unroll
     for (int i = 0; i < RPW; ++i) { m[i] = -CUDART_INF_F; l[i] = 0.f; }
-    const int cw = la_pad8((rk + 3) / 4);          // latent channels per warp, a multiple of 8
-    float o[LA_TC_MAX_NT][4];
+    const int cw = la_pad8((rk + 7) / 8);          // latent channels per warp, a multiple of 8
+    const int steps = Dp / 8, s_lo = (warp >> 2) ? (steps + 1) / 2 : 0, s_hi = (warp >> 2) ? steps : (steps + 1) / 2;      // this warp's channels of the scores
+    float o[LT_MAX_NT][4];
 #pragma unroll
-    for (int n = 0; n < LA_TC_MAX_NT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-    const int* tab = p.table + (size_t)slot * p.stride;
-    const bool vec = (D % 4 == 0);
+    for (int n = 0; n < LT_MAX_NT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
     for (int tile = tile_lo; tile < tile_hi; ++tile) {
         const int kb = tile * LA_KT;
-        __syncthreads();                           // the previous tile is consumed; sq and the pad columns are written
-        if (vec) {
-            const int cpr = D / 4;                 // 16-byte chunks per row
-            for (int e = threadIdx.x; e < LA_KT * cpr; e += LA_THREADS) {
-                const int j = e / cpr, c = e % cpr;
-                const int kj = kb + j;
-                float* dst = sk + (size_t)j * DS + c * 4;
-                if (kj < nkeys) {
-                    const float* src = p.cache + ((size_t)tab[kj / p.page] * p.page + kj % p.page) * D + c * 4;
-                    const uint32_t da = (uint32_t)__cvta_generic_to_shared(dst);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(da), "l"(src) : "memory");
-                } else {
-                    *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-        } else {
-            for (int e = threadIdx.x; e < LA_KT * D; e += LA_THREADS) {
-                const int j = e / D, d = e % D;
-                const int kj = kb + j;
-                sk[(size_t)j * DS + d] = kj < nkeys ? p.cache[((size_t)tab[kj / p.page] * p.page + kj % p.page) * D + d] : 0.f;
-            }
+        if (tile > tile_lo) {
+            __syncthreads();                       // the previous tile is consumed
+            fetch(kb);
         }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
-        {   // scores of keys 8 * warp .. + 7
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        {   // scores of keys 8 * (warp % 4) .. + 7
+            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
             const float* qa0 = sq + (size_t)gq * DS + tq;
             const float* qa1 = sq + (size_t)(gq + 8) * DS + tq;
-            const float* kb0 = sk + (size_t)(warp * 8 + gq) * DS + tq;
-#pragma unroll 4
-            for (int ks = 0; ks < Dp; ks += 8) {
+            const float* kb0 = sk + (size_t)((warp & 3) * 8 + gq) * DS + tq;
+            auto step = [&](const int ks, float (&c)[4]) {
                 uint32_t a[4], b[2];
                 a[0] = __float_as_uint(qa0[ks]); a[1] = __float_as_uint(qa1[ks]); a[2] = __float_as_uint(qa0[ks + 4]); a[3] = __float_as_uint(qa1[ks + 4]);
                 b[0] = to_tf32(kb0[ks]); b[1] = to_tf32(kb0[ks + 4]);
-                mma_tf32_1688(acc, a, b);
-            }
-            ss[gq * 36 + warp * 8 + tq * 2] = acc[0]; ss[gq * 36 + warp * 8 + tq * 2 + 1] = acc[1];
-            ss[(gq + 8) * 36 + warp * 8 + tq * 2] = acc[2]; ss[(gq + 8) * 36 + warp * 8 + tq * 2 + 1] = acc[3];
+                mma_tf32_1688(c, a, b);
+            };
+            int s = s_lo;
+#pragma unroll 4
+            for (; s + 1 < s_hi; s += 2) { step(8 * s, acc[0]); step(8 * s + 8, acc[1]); }
+            if (s < s_hi) step(8 * s, acc[0]);
+            float* const d = ss + (warp >> 2) * 16 * 32;
+            const int c = (warp & 3) * 8 + tq * 2;
+            *reinterpret_cast<float2*>(d + at(gq, c)) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+            *reinterpret_cast<float2*>(d + at(gq + 8, c)) = make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
         }
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < RPW; ++i) {            // softmax rows 4 * warp .. + 3, lane = key
+        for (int i = 0; i < RPW; ++i) {            // softmax rows 2 * warp, + 1, lane = key
             const int r = warp * RPW + i;
             const int qi = r / HG;
             const bool live = qi < nt && (kb + lane) <= pos0 + qi;
-            const float sc = live ? ss[r * 36 + lane] * p.scale : -CUDART_INF_F;
+            const float sc = live ? (ss[at(r, lane)] + ss[16 * 32 + at(r, lane)]) * p.scale : -CUDART_INF_F;
             float mx = sc;
 #pragma unroll
             for (int of = 16; of > 0; of >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, of));
@@ -422,7 +441,7 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
             for (int of = 16; of > 0; of >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, of);
             l[i] = l[i] * corr + ps;
             m[i] = mn;
-            ss[r * 36 + lane] = __uint_as_float(to_tf32(pj));
+            ss[at(r, lane)] = __uint_as_float(to_tf32(pj));
             if (lane == 0) scorr[r] = corr;
         }
         __syncthreads();
@@ -430,20 +449,21 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
             uint32_t a[4][4];
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
-                a[ks][0] = __float_as_uint(ss[gq * 36 + ks * 8 + tq]); a[ks][1] = __float_as_uint(ss[(gq + 8) * 36 + ks * 8 + tq]);
-                a[ks][2] = __float_as_uint(ss[gq * 36 + ks * 8 + tq + 4]); a[ks][3] = __float_as_uint(ss[(gq + 8) * 36 + ks * 8 + tq + 4]);
+                const float2 u = *reinterpret_cast<const float2*>(ss + at(gq, ks * 8 + 2 * tq)), v = *reinterpret_cast<const float2*>(ss + at(gq + 8, ks * 8 + 2 * tq));
+                a[ks][0] = __float_as_uint(u.x); a[ks][1] = __float_as_uint(v.x);
+                a[ks][2] = __float_as_uint(u.y); a[ks][3] = __float_as_uint(v.y);
             }
             const float c0 = scorr[gq], c1 = scorr[gq + 8];
 #pragma unroll
-            for (int n = 0; n < LA_TC_MAX_NT; ++n) {
+            for (int n = 0; n < LT_MAX_NT; ++n) {
                 const int cb = warp * cw + n * 8;
                 if (n * 8 >= cw || cb >= rk) break;
                 o[n][0] *= c0; o[n][1] *= c0; o[n][2] *= c1; o[n][3] *= c1;
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     uint32_t b[2];
-                    b[0] = to_tf32(sk[(size_t)(ks * 8 + tq) * DS + cb + gq]);
-                    b[1] = to_tf32(sk[(size_t)(ks * 8 + tq + 4) * DS + cb + gq]);
+                    b[0] = to_tf32(sk[(size_t)(ks * 8 + 2 * tq) * DS + cb + gq]);
+                    b[1] = to_tf32(sk[(size_t)(ks * 8 + 2 * tq + 1) * DS + cb + gq]);
                     mma_tf32_1688(o[n], a[ks], b);
                 }
             }
@@ -461,7 +481,7 @@ __global__ void __launch_bounds__(LA_THREADS) latent_attn_tc_kernel(const Latent
         if (qi >= nt || h >= p.H) continue;
         float* dst = p.part + (((size_t)(t0 + qi) * p.H + h) * p.nsplit + blockIdx.z) * (rk + 2);
 #pragma unroll
-        for (int n = 0; n < LA_TC_MAX_NT; ++n) {
+        for (int n = 0; n < LT_MAX_NT; ++n) {
             const int cb = warp * cw + n * 8;
             if (n * 8 >= cw || cb >= rk) break;
             const int d = cb + tq * 2;
@@ -479,25 +499,39 @@ struct LatentMergeParams {
     MetaView meta;
 };
 
+constexpr int LM_MAX_SPLIT = 16;                   // KxModel::max_split
+
+// parts of a token's head -> its output.  The parts' factors are worked out once, and a thread requests its channel of eight parts at a time (part after part, with the factor of each
+// behind two dependent reads, before: 9.6 us of the step above, 6.5 now)
 __global__ void __launch_bounds__(128) latent_merge_kernel(const LatentMergeParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x, h = blockIdx.y;
     if (t >= p.meta.T()) return;
+    __shared__ float s_f[LM_MAX_SPLIT];
     const float* src = p.part + ((size_t)t * p.H + h) * p.nsplit * (p.rk + 2);
+    const size_t pitch = p.rk + 2;
     float M = -CUDART_INF_F;
-    for (int z = 0; z < p.nsplit; ++z) M = fmaxf(M, src[(size_t)z * (p.rk + 2) + p.rk]);
+#pragma unroll 8
+    for (int z = 0; z < p.nsplit; ++z) M = fmaxf(M, src[z * pitch + p.rk]);
     float Lsum = 0.f;
+#pragma unroll 8
     for (int z = 0; z < p.nsplit; ++z) {
-        const float mz = src[(size_t)z * (p.rk + 2) + p.rk];
-        if (mz > -CUDART_INF_F) Lsum += src[(size_t)z * (p.rk + 2) + p.rk + 1] * expf(mz - M);
+        const float mz = src[z * pitch + p.rk], lz = src[z * pitch + p.rk + 1];
+        if (mz > -CUDART_INF_F) Lsum += lz * expf(mz - M);
     }
+    for (int z = threadIdx.x; z < p.nsplit; z += blockDim.x) {
+        const float mz = src[z * pitch + p.rk];
+        s_f[z] = mz > -CUDART_INF_F ? expf(mz - M) : -1.f;
+    }
+    __syncthreads();
     const float inv = 1.f / Lsum;
     for (int d = threadIdx.x; d < p.rk; d += blockDim.x) {
         float acc = 0.f;
+#pragma unroll 8
         for (int z = 0; z < p.nsplit; ++z) {
-            const float mz = src[(size_t)z * (p.rk + 2) + p.rk];
-            if (mz > -CUDART_INF_F) acc += src[(size_t)z * (p.rk + 2) + d] * expf(mz - M);
+            const float f = s_f[z], x = src[z * pitch + d];
+            if (f >= 0.f) acc += x * f;
         }
         p.out[(size_t)t * p.H * p.rk + (size_t)h * p.rk + d] = acc * inv;
     }

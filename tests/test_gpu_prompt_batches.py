@@ -169,6 +169,27 @@ def test_latent_attention_at_the_edges_of_key_tiles(heads, kv_rank, rot_dim):
         m.close()
 
 
+@pytest.mark.parametrize("heads, kv_rank, rot_dim", [(16, 42, 8), (20, 512, 64), (5, 30, 4)])
+def test_latent_attention_of_single_tokens(heads, kv_rank, rot_dim):
+    """One token of every sequence behind contexts of one key, parts of a 32-key tile, and several tiles in parts of their own; latent rows that are no whole runs of sixteen bytes, of
+    as many channels as the kernel holds, and of fewer than its warps take."""
+    cfg, st, w = synth.make_kemirax([K("latent_attention", heads=heads, kv_rank=kv_rank, rot_dim=rot_dim, mlp=False)], seed=6, width=96)
+    lens, more = [1, 31, 64, 150, 500], 3
+    toks = [np.random.default_rng(n).integers(1, 90, n + more).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, config=cfg, kv_tokens=sum(lens) + 32 * len(lens), kv_page=16)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        opt = [capi.OPTION_FULL] * len(lens)
+        m.infer_raw(list(range(len(lens))), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
+        rows = [m.infer_raw(list(range(len(lens))), [1] * len(lens), [t[n + i] for t, n in zip(toks, lens)], opt) for i in range(more)]
+        for s, n in enumerate(lens):
+            err = _errs(np.concatenate([r[s] for r in rows]), kemirax_numpy.run(json.loads(cfg), w, toks[s])[n:])
+            assert np.median(err) <= BF16_TOL and err.max() <= ROW_TOL, (s, float(np.median(err)), int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("n", [17, 100, 300])
 @pytest.mark.parametrize("ranks", [(64, 128), (32, 32), (64, 64)])
 def test_low_rank_second_stages(ranks, n):
