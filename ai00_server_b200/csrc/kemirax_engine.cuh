@@ -287,7 +287,8 @@ void b200rwkv_engine::kx_build(const StFile& st, const char* cfg_json, size_t cf
     CK(cudaFuncSetAttribute(gla_scan_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
     allow_smem(gla_chunk_kernel, GC_SMEM);
     CK(cudaFuncSetAttribute(gla_scan_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_ALONE_SMEM));
-    CK(cudaFuncSetAttribute(moe_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+    CK(cudaFuncSetAttribute(moe_route_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+    CK(cudaFuncSetAttribute(moe_route_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     REQUIRE(moe_route_smem(W, 2048) <= 128 * 1024, B200RWKV_ERR_UNSUPPORTED, "width too large for the router kernel");
     CK(cudaFuncSetAttribute(lin_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIN_TC_SMEM));
     CK(cudaFuncSetAttribute(lin_umma_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, LuCfg<32>::SMEM_BYTES));
@@ -580,7 +581,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
         if (c.has_mlp) {
             const int E = c.experts, NE = E + c.identity, ff = c.ff;
             MoeRouteParams rp{m.h, W, l.router, W, l.corr, NE, c.top, m.sel, m.wgt, mv};
-            launch_k(moe_route_kernel, dim3(rows), dim3(MOE_ROUTE_THREADS), moe_route_smem(W, NE), rp, KC_OTHER, s, prof);
+            launch_k(moe_route_threads(rows) == 1024 ? moe_route_kernel<1024> : moe_route_kernel<256>, dim3(rows), dim3(moe_route_threads(rows)), moe_route_smem(W, NE), rp, KC_OTHER, s, prof);
             MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
             kx_moe_group(s, prof, gp, rows);
             if (E > 0) {
@@ -599,7 +600,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
                 kx_lin(s, prof, p2, rows, 1);
             }
             MoeCombineParams cp{m.x, m.h, m.G + W, GW, m.dn, m.row_of, m.wgt, c.top, c.has_shared ? m.ds : nullptr, l.sg, W, mv};
-            launch_k(moe_combine_kernel, dim3(rows), dim3(256), 0, cp, KC_OTHER, s, prof);
+            launch_k(moe_combine_kernel, dim3(rows), dim3(moe_combine_threads(W)), 0, cp, KC_OTHER, s, prof);
         }
         if (m.dbg_layers && !use_graph)
             CK(cudaMemcpyAsync(m.dbg_layers + li * (size_t)dbg_T * W, m.x, (size_t)dbg_T * W * 4, cudaMemcpyDeviceToDevice, s));

@@ -38,8 +38,11 @@ struct MoeRouteParams {
 //                  the chosen scores over their sum.
 enum MoeRouteMode { MOE_SOFTMAX_ALL = 0, MOE_TOP_LOGITS = 1, MOE_SIGMOID_GROUPS = 2 };
 
-constexpr int MOE_ROUTE_THREADS = 256;
-__host__ __device__ inline size_t moe_route_smem(int K, int NE) { return ((size_t)K + 3 * (size_t)NE) * sizeof(float); }
+// Threads of a token's CTA.  Few tokens (decode): 32 warps, so that a warp has its outputs' rows requested in one or two turns (sixteen tokens, width 2048: 12.8 us of the step with
+// eight, 8.5); many: eight, the CTAs of other tokens cover the waits (2000 tokens: 46 us with 32, 38).
+inline int moe_route_threads(int rows) { return rows <= 128 ? 1024 : 256; }
+__host__ __device__ inline int moe_route_row(int K) { return (K + 255) & ~255; }
+__host__ __device__ inline size_t moe_route_smem(int K, int NE) { return ((size_t)moe_route_row(K) + 3 * (size_t)NE) * sizeof(float); }
 
 // warp-wide arg-max over a[0 .. n) in shared memory (ties: lower index); the winner's entry becomes -inf so that the next call
 // finds the runner-up.  Every lane returns the same (index, value).
@@ -63,40 +66,55 @@ __device__ __forceinline__ int moe_warp_take_max(float* a, int n, float& val) {
     return bi;
 }
 
-// One CTA per token: router logits in f32 on the f32 row (every warp takes outputs warp, warp + 8, ...), then warp 0 turns them
+// One CTA per token: router logits in f32 on the f32 row (every warp takes outputs warp, warp + NW, ...), then warp 0 turns them
 // into the choice: softmax, + selection bias, `top` largest, weights = the unbiased probabilities.
-__global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(const MoeRouteParams p) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) moe_route_kernel(const MoeRouteParams p) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float moe_route_sm[];
     float* sh = moe_route_sm;                 // [K]
-    float* z = sh + p.K;                      // [NE]
+    float* z = sh + moe_route_row(p.K);       // [NE]
     const int t = blockIdx.x;
     if (t >= p.meta.T()) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = p.K;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) sh[k] = p.h[(size_t)t * p.ldh + k];
-    __syncthreads();
     const bool vec = (K % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.Wr) & 15) == 0);
-    for (int e = warp; e < p.NE; e += MOE_ROUTE_THREADS / 32) {
-        const __nv_bfloat16* w = p.Wr + (size_t)e * K;
-        float acc = 0.f;
+    // vec: the eight columns of a lane in two halves, so that a warp reads 512 bytes in a row (eight words of a lane side by side: every read of a word met eight lanes in a bank,
+    // 50 us of a prompt step of 2000 tokens, 38 now)
+#pragma unroll 4
+    for (int k = threadIdx.x; k < K; k += blockDim.x) sh[vec ? (k & ~255) + (k & 4) * 32 + ((k >> 3) & 31) * 4 + (k & 3) : k] = p.h[(size_t)t * p.ldh + k];
+    __syncthreads();
+    constexpr int NW = THREADS / 32;
+    for (int e0 = warp; e0 < p.NE; e0 += 2 * NW) {          // two outputs at a time
+        const int e1 = min(e0 + NW, p.NE - 1);
+        const __nv_bfloat16 *w0 = p.Wr + (size_t)e0 * K, *w1 = p.Wr + (size_t)e1 * K;
+        float acc[2] = {0.f, 0.f};
         if (vec) {
+#pragma unroll 4
             for (int k = lane * 8; k < K; k += 256) {
-                const uint4 q = __ldg(reinterpret_cast<const uint4*>(w + k));
-                const __nv_bfloat162* hq = reinterpret_cast<const __nv_bfloat162*>(&q);
+                const uint4 q[2] = {__ldg(reinterpret_cast<const uint4*>(w0 + k)), __ldg(reinterpret_cast<const uint4*>(w1 + k))};
+                const float4 a = *reinterpret_cast<const float4*>(sh + (k & ~255) + 4 * lane), b = *reinterpret_cast<const float4*>(sh + (k & ~255) + 128 + 4 * lane);
+                const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 f = __bfloat1622float2(hq[j]);
-                    acc = fmaf(f.x, sh[k + 2 * j], acc);
-                    acc = fmaf(f.y, sh[k + 2 * j + 1], acc);
+                for (int i = 0; i < 2; ++i) {
+                    const __nv_bfloat162* hq = reinterpret_cast<const __nv_bfloat162*>(&q[i]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 f = __bfloat1622float2(hq[j]);
+                        acc[i] = fmaf(f.x, x[2 * j], acc[i]);
+                        acc[i] = fmaf(f.y, x[2 * j + 1], acc[i]);
+                    }
                 }
             }
         } else {
-            for (int k = lane; k < K; k += 32) acc = fmaf(__bfloat162float(w[k]), sh[k], acc);
+            for (int k = lane; k < K; k += 32) { acc[0] = fmaf(__bfloat162float(w0[k]), sh[k], acc[0]); acc[1] = fmaf(__bfloat162float(w1[k]), sh[k], acc[1]); }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) z[e] = acc + (p.mode == MOE_TOP_LOGITS && p.bias ? p.bias[e] : 0.f);
+        for (int o = 16; o > 0; o >>= 1) { acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o); acc[1] += __shfl_xor_sync(0xffffffffu, acc[1], o); }
+        if (lane < 2 && e0 + lane * NW < p.NE) {
+            const int e = e0 + lane * NW;
+            z[e] = (lane ? acc[1] : acc[0]) + (p.mode == MOE_TOP_LOGITS && p.bias ? p.bias[e] : 0.f);
+        }
     }
     __syncthreads();
     if (warp != 0) return;
@@ -316,7 +334,12 @@ struct MoeCombineParams {
     MetaView meta;
 };
 
-__global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombineParams p) {
+// A thread takes four neighbouring columns and requests all that they need at once, the experts' rows among it (column after column, a round trip to memory each: 20 us of a decode step
+// of sixteen tokens, width 2048, four experts, and 76 of a prompt step of 2000, now 3 and 39).  Widths that are no multiple of four, or wider than the CTA: column after column.
+constexpr int MOE_COMBINE_MAX = 1024;
+inline int moe_combine_threads(int W) { return W % 4 == 0 && W / 4 <= MOE_COMBINE_MAX ? std::max(64, (W / 4 + 31) / 32 * 32) : 256; }
+
+__global__ void __launch_bounds__(MOE_COMBINE_MAX) moe_combine_kernel(const MoeCombineParams p) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[32];
@@ -324,6 +347,34 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombineParams
     if (t >= p.meta.T()) return;
     const int W = p.W;
     float sgate = 0.f;
+    if (W % 4 == 0 && W / 4 <= (int)blockDim.x && p.ldg % 4 == 0 && row_whole(p.x) && row_whole(p.h) && row_whole(p.gate) && row_whole(p.rows) && row_whole(p.shared) && row_whole(p.sg, 8)) {
+        const int c = 4 * threadIdx.x;
+        const bool in = c < W;
+        const size_t at = (size_t)t * W + c;
+        int rows[MOE_MAX_TOP]; float wg[MOE_MAX_TOP];
+#pragma unroll
+        for (int k = 0; k < MOE_MAX_TOP; ++k)
+            if (k < p.top) { rows[k] = p.row_of[(size_t)t * p.top + k]; wg[k] = p.wgt[(size_t)t * p.top + k]; }
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 h = in ? *reinterpret_cast<const float4*>(p.h + at) : none;
+        const float4 g = in ? *reinterpret_cast<const float4*>(p.gate + (size_t)t * p.ldg + c) : none;
+        const float4 sh = in && p.shared ? *reinterpret_cast<const float4*>(p.shared + at) : none;
+        const float4 sg = in && p.shared ? row_bf16(__ldg(reinterpret_cast<const uint2*>(p.sg + c))) : none;
+        float4 x = in ? *reinterpret_cast<const float4*>(p.x + at) : none, e[MOE_MAX_TOP];
+#pragma unroll
+        for (int k = 0; k < MOE_MAX_TOP; ++k)
+            if (k < p.top && in) e[k] = rows[k] >= 0 ? *reinterpret_cast<const float4*>(p.rows + (size_t)rows[k] * W + c) : h;
+        if (p.shared) sgate = 1.f / (1.f + expf(-rms_block_sum(row_dot(sg, h, 0.f), red)));
+        if (!in) return;
+        float4 f = none;
+#pragma unroll
+        for (int k = 0; k < MOE_MAX_TOP; ++k)
+            if (k < p.top) { f.x = fmaf(wg[k], e[k].x, f.x); f.y = fmaf(wg[k], e[k].y, f.y); f.z = fmaf(wg[k], e[k].z, f.z); f.w = fmaf(wg[k], e[k].w, f.w); }
+        if (p.shared) { f.x = fmaf(sgate, sh.x, f.x); f.y = fmaf(sgate, sh.y, f.y); f.z = fmaf(sgate, sh.z, f.z); f.w = fmaf(sgate, sh.w, f.w); }
+        x.x += g.x * f.x; x.y += g.y * f.y; x.z += g.z * f.z; x.w += g.w * f.w;
+        *reinterpret_cast<float4*>(p.x + at) = x;
+        return;
+    }
     if (p.shared) {
         float d = 0.f;
         for (int c = threadIdx.x; c < W; c += blockDim.x) d = fmaf(__bfloat162float(p.sg[c]), p.h[(size_t)t * W + c], d);

@@ -190,6 +190,26 @@ def test_latent_attention_of_single_tokens(heads, kv_rank, rot_dim):
         m.close()
 
 
+@pytest.mark.parametrize("width", [98, 260, 4096, 4104])
+def test_rows_in_pieces_of_sixteen_bytes(width):
+    """Norms, token shift, router and the experts' sum at widths that are no whole pieces, of a part of a CTA's pieces, of all of them, and of more."""
+    cfg, st, w = synth.make_kemirax([K("gla", heads=2, dim=16, vdim=16, experts=11, top=3)], seed=3, width=width)
+    lens = [1, 5, 40]
+    toks = [np.random.default_rng(n).integers(1, 90, n + 1).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, precision=1, config=cfg, kv_tokens=256)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        opt = [capi.OPTION_FULL] * len(lens)
+        got = m.infer_raw(list(range(len(lens))), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw(list(range(len(lens))), [1] * len(lens), [t[n] for t, n in zip(toks, lens)], opt)
+        for s in range(len(lens)):
+            err = _errs(np.concatenate([got[s], more[s]]), kemirax_numpy.run(json.loads(cfg), w, toks[s]))
+            assert err.max() <= TIGHT, (s, int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("n", [17, 100, 300])
 @pytest.mark.parametrize("ranks", [(64, 128), (32, 32), (64, 64)])
 def test_low_rank_second_stages(ranks, n):
