@@ -573,6 +573,8 @@ struct b200rwkv_engine {
         scan_alone = prompt && ctas_a_seq > 0 && ctas_a_seq * step_seqs <= num_sms;
         scan_alone_seqs = scan_alone ? num_sms / ctas_a_seq : 0;
     }
+    // (head, sequence) pairs that the SMs hold three apiece: sixteen tokens a group, see wkv_scan.cuh
+    bool scan_few() const { return Hl * step_seqs <= 3 * num_sms; }
     int scan_slots(int slots) const { return scan_alone ? std::min(slots, scan_alone_seqs) : slots; }
     size_t scan_launch_smem(size_t need) const { return scan_alone ? std::max<size_t>(need, SCAN_ALONE_SMEM) : need; }
     int kx_scan_ctas() const;
@@ -1177,9 +1179,11 @@ void b200rwkv_engine::build(const StFile& st) {
     allow_smem(ln_mix_rows_kernel, (size_t)(LN_ROWS + 1) * C * 4);
     allow_smem(ln_mix_tall_kernel, std::min<size_t>(ln_tall_smem(C), 200 * 1024));
     allow_smem(ln_out_tall_kernel, std::min<size_t>(ln_tall_smem(C), 200 * 1024));
-    allow_smem(wkv_scan_kernel<5>, SCAN_ALONE_SMEM);
-    allow_smem(wkv_scan_kernel<6>, SCAN_ALONE_SMEM);
-    allow_smem(wkv_scan_kernel<7>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<5, 8>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<5, 16>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<6, 8>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<6, 16>, SCAN_ALONE_SMEM);
+    allow_smem(wkv_scan_kernel<7, 8>, SCAN_ALONE_SMEM);
     if (precision == 1) split_act = true;         // f32-activation mode (web-rwkv `Bundle::<f32>`): no activation is rounded to f16
     if (const char* v = dbg_env("B200RWKV_PREFETCH_BLOCKS")) prefetch_blocks = std::max(0, atoi(v));
     if (const char* v = dbg_env("B200RWKV_FUSED_PRE")) fused_pre = atoi(v) != 0;
@@ -1731,8 +1735,9 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
         ep.meta = mv;
         launch_k(embed_ln0_kernel, dim3(rows), dim3(LN_THREADS), 0, ep, KC_LN, s, prof);
     }
-    // long steps: seven or eight rows to a CTA (mix.cuh) once there are enough for half of the SMs
-    auto ln_tall = [&](int n) { return n >= 512 && ln_tall_smem(C) <= 200 * 1024; };
+    // long steps: seven or eight rows to a CTA (mix.cuh) once there are enough for all SMs (steps of four layers of width 2560, rows by themselves and in sevens: 512 rows 1013 and 1154 us,
+    // 640 1547 and 1591, 1024 2250 and 2232)
+    auto ln_tall = [&](int n) { return n >= 1024 && ln_tall_smem(C) <= 200 * 1024; };
     auto launch_ln = [&](const LnMixParams& lp0) {
         LnMixParams lp = lp0;
         lp.trace = tr_next(0);
@@ -1816,9 +1821,10 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
             const bool sp = split_on && MT == 1;
             if (scan) {
                 const dim3 grid(Hl, scan_slots(wkv_slots)), block(WKS_THREADS);
-                if (info.version == 5) launch_k(wkv_scan_kernel<5>, grid, block, scan_launch_smem(WksCfg<5>::SMEM_BYTES), wp, KC_WKV, s, prof);
-                else if (info.version == 6) launch_k(wkv_scan_kernel<6>, grid, block, scan_launch_smem(WksCfg<6>::SMEM_BYTES), wp, KC_WKV, s, prof);
-                else launch_k(wkv_scan_kernel<7>, grid, block, scan_launch_smem(WksCfg<7>::SMEM_BYTES), wp, KC_WKV, s, prof);
+                auto go = [&](auto k, size_t smem) { launch_k(k, grid, block, scan_launch_smem(smem), wp, KC_WKV, s, prof); };
+                if (info.version == 7) go(wkv_scan_kernel<7, 8>, WksCfg<7, 8>::SMEM_BYTES);
+                else if (info.version == 6) scan_few() ? go(wkv_scan_kernel<6, 16>, WksCfg<6, 16>::SMEM_BYTES) : go(wkv_scan_kernel<6, 8>, WksCfg<6, 8>::SMEM_BYTES);
+                else scan_few() ? go(wkv_scan_kernel<5, 16>, WksCfg<5, 16>::SMEM_BYTES) : go(wkv_scan_kernel<5, 8>, WksCfg<5, 8>::SMEM_BYTES);
             } else {
             const size_t sm_b = wkv_smem_bytes(info.version, fold_wd2, info.time_decay_adapter, rows, sp);
             switch (info.version * 2 + (sp ? 1 : 0)) {
@@ -1887,7 +1893,7 @@ void b200rwkv_engine::run_step(int MT, int MTR, bool runs) {
         launch_total += launches_last_step;
         return;
     }
-    const int key = ((MT * 256 + MTR) * 2 + (runs ? 1 : 0)) * 2 + (scan_alone ? 1 : 0);
+    const int key = (((MT * 256 + MTR) * 2 + (runs ? 1 : 0)) * 2 + (scan_alone ? 1 : 0)) * 2 + (runs && scan_few() ? 1 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;
@@ -3118,20 +3124,20 @@ int32_t b200rwkv_op_wkv(int32_t device, int32_t version, int32_t T, int32_t H, c
     p.kq_tile = 64;                       // token rows of the A16 output: any value >= T the reader below agrees on
     CK(cudaMemset(p.out, 0, halves * 2));
     const size_t smem = wkv_smem_bytes(version, false, 0, maxT);
-    allow_smem(wkv_scan_kernel<5>, WksCfg<5>::SMEM_BYTES);
-    allow_smem(wkv_scan_kernel<6>, WksCfg<6>::SMEM_BYTES);
-    allow_smem(wkv_scan_kernel<7>, WksCfg<7>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<5, 16>, WksCfg<5, 16>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<6, 16>, WksCfg<6, 16>::SMEM_BYTES);
+    allow_smem(wkv_scan_kernel<7, 8>, WksCfg<7, 8>::SMEM_BYTES);
     switch (version) {
         case 5:
-            if (T > WKV_STAGE_TOK) wkv_scan_kernel<5><<<dim3(H, 1), WKS_THREADS, WksCfg<5>::SMEM_BYTES>>>(p);
+            if (T > WKV_STAGE_TOK) wkv_scan_kernel<5, 16><<<dim3(H, 1), WKS_THREADS, WksCfg<5, 16>::SMEM_BYTES>>>(p);
             else wkv_kernel<5><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT);
             break;
         case 6:
-            if (T > WKV_STAGE_TOK) wkv_scan_kernel<6><<<dim3(H, 1), WKS_THREADS, WksCfg<6>::SMEM_BYTES>>>(p);
+            if (T > WKV_STAGE_TOK) wkv_scan_kernel<6, 16><<<dim3(H, 1), WKS_THREADS, WksCfg<6, 16>::SMEM_BYTES>>>(p);
             else wkv_kernel<6><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT);
             break;
         default:
-            if (T > WKV_STAGE_TOK) wkv_scan_kernel<7><<<dim3(H, 1), WKS_THREADS, WksCfg<7>::SMEM_BYTES>>>(p);
+            if (T > WKV_STAGE_TOK) wkv_scan_kernel<7, 8><<<dim3(H, 1), WKS_THREADS, WksCfg<7, 8>::SMEM_BYTES>>>(p);
             else wkv_kernel<7><<<dim3(H, 1), WKV_SA_THREADS, smem>>>(p, maxT);
             break;
     }

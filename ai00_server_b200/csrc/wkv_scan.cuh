@@ -16,7 +16,7 @@
 // Decays come from the decay projection's own launch in these steps (lora2.cuh: 6 us beside the scan's own time below).  Where the decode kernel
 // evaluates that low-rank stage itself (RWKV-6), its sums run in another order: decays, and with them states, agree to f32 rounding and not to the bit.
 // Measured, RWKV-6 (vectors through registers and three CTAs an SM before, copied and five now): 64 tokens of 32 sequences, 40 heads, 93 -> 78 us, 128 of sixteen, 64 heads, 141 -> 119, 61 of six
-// 25 -> 25, one prompt of 100, 64 heads, 29 -> 29 (263 in the decode kernel).  At five CTAs the path to shared memory is busy 73 % of the time, issue slots 53 %, multiply-adds 46 %;
+// 25 -> 25, one prompt of 100, 64 heads, 29 -> 27 (263 in the decode kernel).  At five CTAs the path to shared memory is busy 73 % of the time, issue slots 53 %, multiply-adds 46 %;
 // eight values a thread halve its reads but leave two warps a head (97 us at the first of these).
 #pragma once
 #include "f32x2.cuh"
@@ -25,10 +25,12 @@
 namespace b200 {
 
 constexpr int WKS_THREADS = 128;
-template <int VER> struct WksCfg {
-    static constexpr int TC = 8;                            // tokens per group
-    static constexpr int CTAS = VER == 7 ? 3 : 5;           // of an SM
-    static constexpr int UNROLL = VER == 7 ? 2 : 1;         // (RWKV-6: two tokens at a time are 80 us instead of 78 in the step below)
+// TC_: tokens per group.  RWKV-5 / 6: eight, of which an SM holds five CTAs, or sixteen, three CTAs, where three an SM are all there are (one prompt of 100 tokens, 64 heads, 29 and 27 us;
+// 64 tokens of 32 sequences, 40 heads, 78 and 87)
+template <int VER, int TC_> struct WksCfg {
+    static constexpr int TC = TC_;
+    static constexpr int CTAS = VER == 7 || TC_ == 16 ? 3 : 5;      // of an SM
+    static constexpr int UNROLL = CTAS == 3 ? 2 : 1;        // (five CTAs: two tokens at a time are 80 us instead of 78 in the step above)
     static constexpr int NA = VER == 7 ? 6 : 4;             // staged vectors: r, k, v, w (, -kk, kk a)
     static constexpr int BUF = NA * TC * WKV_N;             // floats of one group
     static constexpr int OUT_ROW = WKV_N + 4, OUT = 8 * OUT_ROW;      // a token's read-outs: eight partial sums of every value (padded: conflict-free)
@@ -37,9 +39,9 @@ template <int VER> struct WksCfg {
 // place of key c in a staged vector: keys 8 j .. 8 j + 3 at 4 j, 8 j + 4 .. 8 j + 7 at 32 + 4 j
 __device__ __forceinline__ int wks_place(int c) { return (c >> 3) * 4 + (c & 3) + ((c >> 2) & 1) * 32; }
 
-template <int VER>
-__global__ void __launch_bounds__(WKS_THREADS, WksCfg<VER>::CTAS) wkv_scan_kernel(const __grid_constant__ WkvParams p) {
-    using Cfg = WksCfg<VER>;
+template <int VER, int TC_>
+__global__ void __launch_bounds__(WKS_THREADS, WksCfg<VER, TC_>::CTAS) wkv_scan_kernel(const __grid_constant__ WkvParams p) {
+    using Cfg = WksCfg<VER, TC_>;
     constexpr int TC = Cfg::TC, TW = TC / 4;                // tokens per warp in the per-group phases
     extern __shared__ __align__(16) float wks[];
     float* const sc = wks + 2 * Cfg::BUF;                   // [2][TC] bonus of the token

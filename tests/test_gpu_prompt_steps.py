@@ -59,11 +59,17 @@ def test_steps_of_many_tiles(shape, n):
     _check(st, [n], full=False)
 
 
-@pytest.mark.parametrize("lens", [[505], [511], [519], [7, 1, 8, 6, 500], [14, 490, 7, 7, 3]])
+@pytest.mark.parametrize("lens", [[1017], [1023], [1031], [7, 1, 8, 6, 1012], [14, 1002, 7, 7, 3], [7, 8, 6, 13, 15, 1] * 21])
 @pytest.mark.parametrize("shape", ["tiny5", "tiny7", "odd6"])
 def test_rows_of_steps_in_groups_of_seven(shape, lens):
     """Norm and token shift of long steps take seven rows and the one before them a CTA: sequences that begin and end inside, at and between the groups; rows of 320 columns."""
-    _check(synth.Shape(6, 2, 320, 1160, V=512, Dm=32, Dd=64) if shape == "odd6" else shape, lens, full=True)
+    _check(synth.Shape(6, 2, 320, 1160, V=512, Dm=32, Dd=64) if shape == "odd6" else shape, lens, full=False)
+
+
+@pytest.mark.parametrize("shape, count", [("tiny5", 240), ("odd6", 96)])
+def test_scans_of_many_heads_and_sequences(shape, count):
+    """More (head, sequence) pairs than three an SM: groups of eight tokens, parts of one, one and several."""
+    _check(synth.Shape(6, 2, 320, 1160, V=512, Dm=32, Dd=64) if shape == "odd6" else shape, ([6, 17, 8] * count)[:count], full=False)
 
 
 @pytest.mark.parametrize("lens", [[300, 250, 1, 700], [90] * 9])
