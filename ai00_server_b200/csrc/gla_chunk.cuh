@@ -12,7 +12,7 @@
 //     the second to the state; the products within a run (A v) are f32 multiply-adds;
 //   * eight warps prepare the next run meanwhile: decays, their sums, q', k', A, and the operands' parts.
 // Parts of the queries lie side by side, so that a part of the state meets all it needs in one MMA: S_high [q_high, q_mid, q_low], S_mid [q_high, q_mid], S_low [q_high].
-// Measured (heads of 128 x 128, sixteen a layer): 256 tokens of eight sequences 256 -> 69 us, 128 of sixteen 184 -> 76, 1000 of one 618 -> 232 (6500 cycles a run of a head; the split of
+// Measured (heads of 128 x 128, sixteen a layer): 256 tokens of eight sequences 256 -> 70 us, 128 of sixteen 184 -> 78, 1000 of one 618 -> 240 (6500 cycles a run of a head; the split of
 // the state and its exchange with the tensor core hold it).  Distance from 64 bits (2-norm): read-outs 2.6e-7 -> 1.4e-7, states 2.7e-7 -> 8.8e-8.
 #pragma once
 #include <math_constants.h>
