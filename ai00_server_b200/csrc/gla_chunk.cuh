@@ -3,8 +3,8 @@
 // over a run of n <= 16 tokens, with b_t the sum of the run's log alpha up to t and S' = diag(e^{b_n}) S_0:
 //     q'_t = q_t e^{b_t - b_n},   k'_s = k_s e^{b_n - b_s},   A[t, s] = q'_t . k'_s (s <= t)
 //     o_t = q_scale (S'^T q'_t + sum_{s <= t} A[t, s] v_s),    S_n = S' + sum_s k'_s v_s^T
-// A run ends before a channel's decays come to less than e^-12, so every factor is a number and its exponent's rounding stays small; where that leaves fewer than four tokens (decays
-// of e^-4 a token) the CTA goes token by token instead.
+// A run ends before a channel's decays come to less than e^-12, so every factor is a number and its exponent's rounding stays small, and before a decay that is no number, which
+// would be a factor of the tokens before it; where that leaves fewer than four tokens (decays of e^-4 a token) the CTA goes token by token instead.
 //
 // What bounds the token-by-token form (gla.cuh): a chain of products, exchanges and reads a token, about 1400 cycles of an SM for half a head (39 % of the issue slots, no unit busy).
 // Here the state's products are MMAs of full height, every f32 number in three bf16 parts (24 bits; six products of parts), sums in f32:
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gla_chunk_kernel(const __grid_c
                     add4(sum, g[t]);
                     if (t == 2 * w) own[0] = sum;
                     if (t == 2 * w + 1) own[1] = sum;
-                    most += fminf(fminf(sum.x, sum.y), fminf(sum.z, sum.w)) >= GC_LEAST;
+                    most += sum.x >= GC_LEAST && sum.y >= GC_LEAST && sum.z >= GC_LEAST && sum.w >= GC_LEAST;      // (a sum that is no number counts as too small)
                 }
                 most = __reduce_min_sync(0xffffffffu, most);
                 const bool few = most < min(GC_SHORT, left);
