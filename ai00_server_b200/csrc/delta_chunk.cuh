@@ -4,7 +4,8 @@
 // Over a run of n <= 16 tokens, b_t the sum of the logarithms of the decays up to t (never positive):
 //     u_t = beta_t (v_t - e^{b_t} S_0^T k_t - sum_{s < t} e^{b_t - b_s} (k_s . k_t) u_s)      or  e^(i - m') v_t
 //     o_t = e^{b_t} S_0^T q_t + sum_{s <= t} e^{b_t - b_s} (k_s . q_t) u_s,      S_n = e^{b_n} S_0 + sum_s e^{b_n - b_s} k_s u_s^T
-// Decays are factors of sums here and never of operands, so that no run has to end early.
+// Decays are factors of sums here and never of operands, so that no run has to end early.  A logarithm below DC_LEAST, -inf among them, counts as DC_LEAST: its factor is zero in f32
+// either way (e^-104 is), and sums with the parts they lost need finite terms.
 //
 // What bounds the token-by-token forms: a chain of two reductions and exchanges a token (1.6 us a token of a sequence on an SM).  Here eight warps keep the state in registers, as in
 // gla_chunk.cuh; the triangular system for u is solved by the thread of a column in registers, a row of it a step; eight warps prepare the next run: unit lengths and gates within a
@@ -36,6 +37,7 @@ struct RunChunkParams {
 
 constexpr int DC_KEYS = GC_RUN * GC_DMAX * 4, DC_BUF = GC_OPS + GC_VAL + 2 * GC_A + 512 + DC_KEYS;
 constexpr size_t DC_SMEM = GC_STATE + 2 * DC_BUF + GC_VPARTS + 2 * 8 * GC_RUN * GC_RUN * 4 + 128;
+constexpr float DC_LEAST = -1e4f;
 constexpr uint32_t DC_TD1 = 0, DC_TD2 = 192, DC_TMEM_COLS = 512;      // tensor memory: read-outs [2 halves of the channels][3 parts][16 queries, 16 keys], the run's addition to the state
 
 template <bool DELTA>
@@ -128,6 +130,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) run_chunk_kernel(const __grid_c
                 float bt, write = 0.f, least = 0.f;          // b_t, what a value is written with, e^-m
                 if (DELTA) {
                     bt = in ? -rate * (fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)))) : 0.f;
+                    if (bt < DC_LEAST) bt = DC_LEAST;        // (not fmaxf: what is no number stays so)
                     write = in ? 1.f / (1.f + expf(-g)) : 0.f;
                 } else {
                     const float ig = p.cap * tanhf(g / p.cap), zc = p.cap * tanhf(z / p.cap);

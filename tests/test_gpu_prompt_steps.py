@@ -298,6 +298,17 @@ def test_a_decay_that_is_not_a_number_reaches_no_row_before_it(dim, vdim, precis
         m.close()
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dim, vdim, n", [(72, 40, 60), (128, 128, 200), (24, 24, 60)])
+def test_a_decay_rate_beyond_f32(dim, vdim, n, precision):
+    """A head of the delta rule that keeps nothing from token to token (e^100 a token: its logarithms are -inf in f32) beside one that does."""
+    cfg, st, w = synth.make_panupel([synth.panupel_layer("delta", heads=2, dim=dim, vdim=vdim)], seed=4, width=96, loop=None)
+    st, w = st.copy(), dict(w)
+    _tensor(st, "l0.mix.A_log")[1] = 0x42c8
+    w["l0.mix.A_log"] = np.array([w["l0.mix.A_log"][0], 100.0])
+    _check_image(cfg, st, w, panupel_numpy, n, precision)
+
+
 def test_a_nan_stays_one_in_latent_attention():
     """A key that is not a number makes every later row so (rounding to TF32 by integer arithmetic must not turn it into a number)."""
     cfg, st, _ = synth.make_kemirax([synth.kemirax_layer("latent_attention", mlp=False)], seed=4)
