@@ -42,6 +42,13 @@ __device__ __forceinline__ void gc_mma_bf16(float (&c)[4], const uint32_t (&a)[4
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// the smaller of two numbers, not a number if either is none (fminf leaves those out)
+__device__ __forceinline__ float gc_min(const float a, const float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 __global__ void __launch_bounds__(GC_THREADS, 1) gla_chunk_kernel(const __grid_constant__ GlaParams p) {
     extern __shared__ __align__(16) uint8_t gc_smem_raw[];
     __shared__ __align__(8) unsigned long long s_bar[6];
@@ -132,7 +139,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gla_chunk_kernel(const __grid_c
                     add4(sum, g[t]);
                     if (t == 2 * w) own[0] = sum;
                     if (t == 2 * w + 1) own[1] = sum;
-                    most += sum.x >= GC_LEAST && sum.y >= GC_LEAST && sum.z >= GC_LEAST && sum.w >= GC_LEAST;      // (a sum that is no number counts as too small)
+                    most += gc_min(gc_min(sum.x, sum.y), gc_min(sum.z, sum.w)) >= GC_LEAST;      // (a sum that is no number counts as too small)
                 }
                 most = __reduce_min_sync(0xffffffffu, most);
                 const bool few = most < min(GC_SHORT, left);
