@@ -577,6 +577,17 @@ struct b200rwkv_engine {
     bool scan_few() const { return Hl * step_seqs <= 3 * num_sms; }
     int scan_slots(int slots) const { return scan_alone ? std::min(slots, scan_alone_seqs) : slots; }
     size_t scan_launch_smem(size_t need) const { return scan_alone ? std::max<size_t>(need, SCAN_ALONE_SMEM) : need; }
+    // Sequences that a step's launches have CTAs for.  Prompt steps: as many as there are, or in a captured step, which serves others of its rows too, up to eight or any number: CTAs for
+    // sequences there are not wait for an SM of their own in the kernels on the tensor cores, only to leave (64 slots, four layers of attention, 32 heads of 64 channels: one prompt of 20
+    // tokens 294 us and 260, two of 32 369 and 290, four of 16 383 and 292)
+    static constexpr int FEW_SEQS = 8;
+    bool step_few(bool decode) const { return !decode && step_seqs > 0 && step_seqs <= FEW_SEQS; }
+    bool step_captured(int rows) const { return use_graph && rows <= 512; }
+    int step_slots(int rows, bool decode) const {
+        const int most = std::min(S, rows);
+        if (!decode && step_seqs > 0 && !step_captured(rows)) return std::min(most, step_seqs);
+        return step_few(decode) ? std::min(most, (int)FEW_SEQS) : most;
+    }
     int kx_scan_ctas() const;
     int dbg_T = 0;                     // rows a layer has in the debug copy of the residual stream
     double pair_plan(const GemmLaunch& g, int rows, int* ntok, int* parts) const;
@@ -595,8 +606,8 @@ struct b200rwkv_engine {
     int *d_meta = nullptr, *h_meta = nullptr;
     int* d_meta_all = nullptr;
     size_t meta_ints = 0;
-    std::map<int, cudaGraphExec_t> graphs;
-    std::map<int, long long> graph_launches;   // kernels per captured step graph
+    std::map<int64_t, cudaGraphExec_t> graphs;
+    std::map<int64_t, long long> graph_launches;   // kernels per captured step graph
     long long launch_total = 0;                // kernels launched by this engine's steps since creation
     long long launches_last_step = 0;
     int last_T = 0;                    // tokens of the most recent step

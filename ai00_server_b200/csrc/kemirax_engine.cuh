@@ -492,7 +492,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
         launch_k(embed_rows_kernel, dim3(rows), dim3(NORM_THREADS), 0, ep, KC_LN, s, prof);
         if (m.pairs && !decode) launch_k(last_token_commit_kernel, dim3(cdiv(std::min(S, rows), 128)), dim3(128), 0, ep, KC_LN, s, prof);
     }
-    const int nslot_grid = std::min(S, rows);
+    const int nslot_grid = step_slots(rows, decode);
     // these end with the last norm
     const bool own_stack = m.cfg.family == KX_FAMILY_ZUFULIX || m.cfg.family == KX_FAMILY_PASOPEL || m.cfg.family == KX_FAMILY_PANUPEL ||
                            m.cfg.family == KX_FAMILY_FUFIPEL;
@@ -702,7 +702,7 @@ int b200rwkv_engine::kx_scan_ctas() const {
 void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     const int rows = kx_bucket(T), rrows = R > 0 ? kx_bucket(R) : 0;
     set_scan_alone(!decode, decode ? 0 : kx_scan_ctas());
-    if (!use_graph || rows > 512) {        // (launch by launch: the kernels of a long step outlast their launches)
+    if (!step_captured(rows)) {            // (launch by launch: the kernels of a long step outlast their launches)
         kx_enqueue_step(stream, rows, rrows, decode, nsplit, nullptr);
         enqueue_keep(stream, cdiv(rows, 16), rrows / 16 + (rrows % 16 ? 1 : 0));
         launch_total += launches_last_step;
@@ -717,7 +717,8 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     bool runs = false;                     // and whether they take the tokens in runs
     for (const KxLayer& l : kx->layers)
         runs = runs || (!decode && (((l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows)) || ((l.c.mixer == KX_PARALLEL || l.c.mixer == KX_DELTA) && run_chunks(rows, GC_DMAX, GC_DMAX, 0))));
-    const int key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0);
+    const int64_t key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0) +
+                        (step_few(decode) ? (int64_t)1 << 31 : 0);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

@@ -79,6 +79,27 @@ def test_attention_at_the_edges_of_key_tiles(heads, kv_heads, dim, vdim):
         m.close()
 
 
+@pytest.mark.parametrize("make, module, layers", [
+    (synth.make_kemirax, kemirax_numpy, [K("gla", heads=2, dim=40, vdim=24, mlp=False), K("latent_attention", heads=3, kv_rank=24, rot_dim=8, mlp=False)]),
+    (synth.make_panupel, panupel_numpy, [P("delta", heads=2, dim=24), P("parallel", heads=4, kv_heads=2, dim=24, mm_heads=2, mm_dim=24)]),
+    (synth.make_fufipel, fufipel_numpy, [F("attention", heads=4, kv_heads=2, dim=20, window=8, keep_first=2), F("parallel", heads=2, dim=24, chunk=11)])])
+def test_steps_of_one_row_count_and_several_numbers_of_sequences(make, module, layers):
+    """Steps of 24 tokens in one sequence, eight, nine and twelve (captured ones hold CTAs for eight sequences or for any number), and longer ones of 3 and 20 (as many as there are)."""
+    cfg, st, w = make(layers, seed=4, width=96, **({"loop": None} if make is synth.make_panupel else {}))
+    m = runtime.Model(st, max_batch=24, token_chunk_size=512, precision=1, config=cfg, kv_tokens=2048, kv_page=16)
+    try:
+        for lens in ([24], [3] * 8, [3, 3, 3, 3, 3, 3, 2, 2, 2], [2] * 12, [24], [200, 3, 330], [30] * 20, [2] * 12):
+            toks = [np.random.default_rng([n, i]).integers(1, 90, n).tolist() for i, n in enumerate(lens)]
+            for s in range(len(lens)):
+                m.state.reset(s)
+            got = m.infer_raw(list(range(len(lens))), lens, sum(toks, []), [capi.OPTION_FULL] * len(lens))
+            for s in (0, len(lens) // 2, len(lens) - 1):
+                err = _errs(got[s], module.run(json.loads(cfg), w, toks[s]))
+                assert err.max() <= TIGHT, (lens, s, int(err.argmax()), float(err.max()))
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("dim, vdim, conv", [(72, 72, 4), (128, 40, 4), (24, 24, 4), (40, 72, 3)])
 def test_delta_rule(dim, vdim, conv, precision):
