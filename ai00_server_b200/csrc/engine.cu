@@ -53,6 +53,7 @@
 #include "hyper.cuh"
 #include "sink_attn.cuh"
 #include "prompt_attn.cuh"
+#include "short_attn.cuh"
 
 namespace b200 {
 
@@ -555,6 +556,17 @@ struct b200rwkv_engine {
     int bench_slots() const { return kx ? kx->portion : std::min(maxT, 256); }
     int step_rows = 0;                 // config.json families: rows of the step being enqueued
     int step_seqs = 0;                 // sequences of the step
+    int step_total = 0, step_context = 0;       // config.json families: its tokens, and the most keys a token of it can see
+    // Attention of a prompt step by short_attn.cuh (dk, dv up to 128): sequences of few (token, head) rows of a key head, 32 on average (16 where rows are long and a key head has several
+    // query heads), whose keys are one or two of its tiles (one where rows are long), and enough (sequence, key head) pairs that SMs would take several turns with one each.  Both sides,
+    // steps of four layers on the tensor cores and in f32 multiply-adds (us; sequences x tokens): 16 heads of 32 channels 64x32 716 and 660, 48x40 658 and 707, 16x16 377 and 335,
+    // 8x16 266 and 284; of 128 channels 64x16 818 and 777, 64x32 997 and 1006, 48x40 916 and 1071, 16x32 487 and 463, 4x32 319 and 368; 16 query heads on 8 key heads of 128 channels
+    // 64x8 483 and 473, 64x12 561 and 578; on 4 key heads of 32 channels 64x8 351 and 335, 64x16 416 and 426, 32x8 310 and 330; 32 heads of 64 channels, 32 tokens on 200 keys each, 1191
+    // and 1903.  Steps of more than eight sequences have CTAs for every slot when captured (step_slots): 128 pairs do there, of one or two query heads a key head
+    bool attn_short(int H, int G, int dk, int dv) const {
+        const int rep = H / G, d = std::max(dk, dv);
+        return step_seqs * G >= (step_seqs > FEW_SEQS && rep <= 2 ? 128 : 192) && rep * step_total <= (d > 64 && rep > 1 ? 16 : 32) * step_seqs && step_context <= (d > 64 ? 32 : 64);
+    }
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
     // column a thread, and a chain of tokens takes longer with two)
     bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }

@@ -686,6 +686,7 @@ void b200rwkv_engine::kx_fill_step(int* hm, const std::vector<int>& slots, const
             ns *= 2;                                       // at most one wave of CTAs, and of clusters
     }
     *decode = dec; *nsplit = ns;
+    step_total = T; step_context = ctx_max;
 }
 
 // CTAs a sequence has in the largest recurrence launch of a prompt step
@@ -717,8 +718,11 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     bool runs = false;                     // and whether they take the tokens in runs
     for (const KxLayer& l : kx->layers)
         runs = runs || (!decode && (((l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows)) || ((l.c.mixer == KX_PARALLEL || l.c.mixer == KX_DELTA) && run_chunks(rows, GC_DMAX, GC_DMAX, 0))));
+    int64_t forms = 0;                     // which layers attend in the form for short sequences
+    for (const KxLayer& l : kx->layers)
+        if (!decode && l.sa_reg && l.c.kv_heads > 0) forms = (forms * 31 + (attn_short(l.c.heads, l.c.kv_heads, l.c.dim, l.c.vdim) ? 1 : 0)) % 1000000007;
     const int64_t key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0) +
-                        (step_few(decode) ? (int64_t)1 << 31 : 0);
+                        (step_few(decode) ? (int64_t)1 << 31 : 0) + (forms << 32);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

@@ -17,7 +17,7 @@
 // Measured (16 sequences of 128 tokens, 16 query heads on 4 key heads of 128 channels, in f32 multiply-adds before and here): 113 -> 34 us at 128 tokens of context, 454 -> 76 at
 // 576, 805 -> 122 at 1024 (130 with descriptors worked out by the issuing lane alone); one prompt of 1000 tokens 376 -> 59, of 20 tokens 25 -> 15; 16 prompts of 1024 tokens, four
 // layers of width 2048, 22.1 -> 15.7 ms.  Distance from 64 bits (2-norm): 6.2e-7 -> 3.0e-7 at 1024 tokens, 1.42e-6 -> 3.5e-7 at 6000, 1.6e-7 -> 1.4e-7 at 20.
-// Slower than before only where most rows are empty and the context is one tile: 64 sequences of 32 tokens, one query head a key head: 86 -> 82 us of 128 channels, 64 -> 74 of 32.
+// Where most rows are empty and the context is a tile the multiply-add form is the better one (64 sequences of 32 tokens, one query head a key head, 32 channels: 64 -> 74 us): short_attn.cuh.
 #pragma once
 #include "bf16_parts.cuh"
 #include "linear_umma.cuh"

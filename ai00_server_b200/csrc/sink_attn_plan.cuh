@@ -123,6 +123,7 @@ static void sa_plan_model(SeqModel& m) {
         CK(cudaFuncSetAttribute(sa_tile_kernel(rb), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         for (bool decode : {false, true}) CK(cudaFuncSetAttribute(sa_reg_kernel(rb, decode), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
+    allow_smem(short_attn_kernel, short_attn_smem(SH_DMAX, SH_DMAX));
     for (auto k : {prompt_attn_kernel<16, true>, prompt_attn_kernel<0, true>, prompt_attn_kernel<0, false>}) allow_smem(k, prompt_attn_smem(PT_DMAX, PT_DMAX));
     // the largest cluster the attention launch may ask for: what the device can co-schedule at this layer's shared memory
     for (const KxLayer& l : m.layers) {
@@ -161,11 +162,17 @@ static void sa_plan_model(SeqModel& m) {
 }
 
 // One attention launch.  Prompt steps whose keys are not split (kx_fill_step: their chunks fill the chip, or the context is one key tile) take the kernel that multiplies a
-// key tile with 128 (token, head) rows on the tensor core, where its 16-byte rows and sizes allow; block means and longer rows stay with the forms above.
+// key tile with 128 (token, head) rows on the tensor core, or that of many short sequences (attn_short), where their 16-byte rows and sizes allow; block means and longer rows stay with
+// the forms above.
 void b200rwkv_engine::kx_sink_attn(cudaStream_t s, Profiler* prof, const KxLayer& l, const SinkAttnParams& sp, SinkAttnKernel kern, int threads, size_t smem, int rows,
                                    int nslot_grid, int chunks_grid, bool decode, int nsplit) {
     const int rep = sp.H / sp.G;
     if (!decode && nsplit == 1 && l.sa_reg && sp.pool == 0 && rep <= PT_ROWS && sp.koff % 4 == 0 && sp.voff % 4 == 0 && sp.D % 4 == 0 && sp.ldq % 4 == 0) {
+        if (rep <= SH_ROWS && attn_short(sp.H, sp.G, sp.dk, sp.dv)) {
+            PromptAttnParams pa{sp, SH_ROWS / rep};
+            launch_k(short_attn_kernel, dim3(cdiv(rows, pa.qt) + nslot_grid, sp.G), dim3(SH_THREADS), short_attn_smem(sp.dk, sp.dv), pa, KC_WKV, s, prof);
+            return;
+        }
         PromptAttnParams pa{sp, PT_ROWS / rep};
         const bool whole = (sp.dk | sp.dv | sp.koff | sp.voff | sp.D | sp.ldq) % 8 == 0;
         auto k = whole ? (sp.dk == 128 && sp.dv == 128 ? prompt_attn_kernel<16, true> : prompt_attn_kernel<0, true>) : prompt_attn_kernel<0, false>;

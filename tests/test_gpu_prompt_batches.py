@@ -100,6 +100,37 @@ def test_steps_of_one_row_count_and_several_numbers_of_sequences(make, module, l
         m.close()
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim, longest", [(4, 4, 24, 24, 32), (2, 2, 128, 128, 32), (8, 2, 32, 36, 14), (9, 3, 72, 104, 8), (3, 3, 64, 4, 33)])
+def test_attention_of_many_short_sequences(heads, kv_heads, dim, vdim, longest):
+    """64 sequences of 1 to `longest` tokens, then five more of each: the form for few (token, head) rows a key head, below and behind one of its tiles of 32 keys, rows of one, three
+    and four query heads (whose 64 leave one over); and the other side of its rule.  A token that is not a number reaches no row before it and no other sequence."""
+    cfg, st, w = synth.make_panupel([P("parallel", heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, mm_heads=1, mm_dim=16)], seed=5, width=96, loop=None)
+    st = st.copy()
+    head = int(st[:8].view("<u8")[0])
+    e = json.loads(bytes(st[8:8 + head]))["embed"]
+    st[8 + head + e["data_offsets"][0]:8 + head + e["data_offsets"][1]].view("<u2").reshape(e["shape"])[7] = 0x7fc0
+    rng = np.random.default_rng(longest)
+    B = 64
+    lens = [longest, 1, 2, longest - 1] + rng.integers(1, longest, B - 4).tolist()
+    toks = [rng.integers(10, 90, n + 5).tolist() for n in lens]
+    toks[3][longest // 2] = 7
+    m = runtime.Model(st, max_batch=B, token_chunk_size=512, precision=1, config=cfg, kv_tokens=sum(lens) + 24 * B, kv_page=16)
+    try:
+        for s in range(B):
+            m.state.reset(s)
+        opt = [capi.OPTION_FULL] * B
+        got = m.infer_raw(list(range(B)), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw(list(range(B)), [5] * B, sum((t[n:] for t, n in zip(toks, lens)), []), opt)
+        for s in (0, 1, 2, 3, 4, B - 1):
+            rows, n = np.concatenate([got[s], more[s]]), longest // 2 if s == 3 else lens[s] + 5
+            assert np.isfinite(rows[:n]).all() and np.isnan(rows[n:]).all(), (s, np.isfinite(rows).all(1).tolist())
+            err = _errs(rows[:n], panupel_numpy.run(json.loads(cfg), w, toks[s][:n]))
+            assert err.max() <= TIGHT, (s, int(err.argmax()), float(err.max()))
+        assert all(np.isfinite(got[s]).all() and np.isfinite(more[s]).all() for s in range(B) if s != 3)
+    finally:
+        m.close()
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("dim, vdim, conv", [(72, 72, 4), (128, 40, 4), (24, 24, 4), (40, 72, 3)])
 def test_delta_rule(dim, vdim, conv, precision):
