@@ -1450,7 +1450,7 @@ void b200rwkv_engine::build(const StFile& st) {
                 ly.wd2_index = (int)ly.pre.size();
                 ly.pre.push_back(make_launch(sv));
             }
-            if (Dd <= 128 && Dd % 8 == 0 && !dbg_env("B200RWKV_NOFOLD")) {
+            if (Dd <= WKV_FOLD_MAX_D && Dd % 8 == 0 && !dbg_env("B200RWKV_NOFOLD")) {
                 // k-major copy of this rank's time_decay_w2 rows, one contiguous [Dd][64] slice per head: the WKV
                 // kernels evaluate the decay LoRA stage 2 themselves (one launch / phase less per layer)
                 const StTensor& t = st.get(a + "time_decay_w2");

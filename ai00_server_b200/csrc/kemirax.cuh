@@ -403,7 +403,7 @@ struct SeqModel {
     bool side_lin = false; float* lin_ws_side = nullptr;      // projections also run on the side stream: split-k sums of their own
     int portion = 128;                            // tokens of a portion (a step holds several)
     float* dbg_layers = nullptr;                  // [L][dbg_T][W] residual after every layer (bring-up aid; nullptr: off)
-    int max_split = 16;
+    int max_split = LM_MAX_SPLIT;                 // parts of a step's keys at most (families lower it to the clusters their attention can have)
     int sa_ygroups = 1, sa_ygroups_decode = 1;    // head groups (grid rows) of the smallest windowed-attention launch of the model (prompt / decode shape)
     SeqMeta sm{nullptr, 0};
     SeqModel() = default;

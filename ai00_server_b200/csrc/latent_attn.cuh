@@ -499,7 +499,7 @@ struct LatentMergeParams {
     MetaView meta;
 };
 
-constexpr int LM_MAX_SPLIT = 16;                   // KxModel::max_split
+constexpr int LM_MAX_SPLIT = 16;                   // parts of a step's keys at most: what SeqModel::max_split begins with
 
 // parts of a token's head -> its output.  The parts' factors are worked out once, and a thread requests its channel of eight parts at a time (part after part, with the factor of each
 // behind two dependent reads, before: 9.6 us of the step above, 6.5 now)

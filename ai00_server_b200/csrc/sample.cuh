@@ -37,7 +37,8 @@ constexpr int TOPK_CTAS = 8, TOPK_THREADS = 256;                // CTAs of a row
 constexpr int TOPK_PER_THREAD = 32;                             // elements
 constexpr int TOPK_SLICE = TOPK_THREADS * TOPK_PER_THREAD;      // elements of a CTA: 8192
 constexpr int TOPK_MAX_V = TOPK_CTAS * TOPK_SLICE;              // 65536
-constexpr int TOPK_LIST = 4096;                                 // candidates of a CTA before it cuts them (127 threads x 32 at most)
+constexpr int TOPK_LIST = 4096;                                 // list of a CTA: what is left after a cut (32 elements of top_k threads at most); a first pass may count more and collects again
+static_assert(TOPK_LIST >= TOPK_PER_THREAD * TOPK_MAX, "a CTA's own best top_k come from top_k threads");
 constexpr int TOPK_SHARE = 512;                                 // candidates a CTA may share
 constexpr int TOPK_PITCH_PAD = 4;                               // eight CTAs' lists, read side by side, start in different banks
 constexpr int TOPK_INLINE = 64;                                 // rows whose slots travel as kernel parameters

@@ -250,7 +250,7 @@ __host__ __device__ inline size_t wkv_smem_bytes(int ver, bool fold, int Dd, int
     return b;
 }
 
-constexpr int WKV_ONE_MAX_D = 256;       // decay ranks of the one-token path
+constexpr int WKV_FOLD_MAX_D = 128;      // decay ranks whose second stage the kernel works out itself (a slice of [rank][64] weights in shared memory)
 
 // One token of one slot (every slot of a decode step), the rest of the CTA's work behind the wait.  A chain of latencies, so as few links as the function has: ONE trip for
 // all operands (the general path below asks for them in up to four), the state on its way out before the norm, sums of the norm within warps and one exchange each.
@@ -261,7 +261,7 @@ template <int VER, bool SPLIT>
 __device__ __forceinline__ void wkv_one_token(const WkvParams& p, const int h, const int t, float (&m)[4][8], float* M, const float* statics, const float bias, const __half* wt,
                                               const int Dd, float* v64) {
     constexpr int KC = 8, LANES = WKV_N / KC;
-    __shared__ float s_w[WKV_N], s_part[4][WKV_N], s_d[WKV_ONE_MAX_D], s_red[3][4];
+    __shared__ float s_w[WKV_N], s_part[4][WKV_N], s_d[WKV_FOLD_MAX_D], s_red[3][4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ig = tid / LANES, j4 = tid % LANES, ch = h * WKV_N;
     const size_t row = (size_t)t * p.ld + ch;
     const bool fold = VER == 6 && Dd > 0;
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(WKV_SA_THREADS, 7) wkv_kernel(const __grid_con
     pdl_wait();
     trace_stamp(p.trace, 1);
     if (!live) return;
-    if (nt == 1 && Dd <= WKV_ONE_MAX_D) {
+    if (nt == 1) {
         wkv_one_token<VER, SPLIT>(p, h, t0, m, M, statics, bias, wt, Dd, pre_s);
         trace_stamp(p.trace, 7);
         return;
