@@ -452,8 +452,8 @@ def test_prefill_steps_of_128_tokens(models, preset):
 @pytest.mark.parametrize("over", [{}, {"Dd": 96}, {"Dd": 192}])
 @pytest.mark.parametrize("preset, exact", [("tiny5", False), ("tiny6", False), ("tiny7", False), ("tiny6", True), ("tiny7", True)])
 def test_steps_of_one_token_a_slot_against_steps_of_several(models, preset, exact, over):
-    """The recurrence's path for one token (decay ranks folded in and apart) against the oracle and the path for several: twelve tokens one by one, in a batch whose other slots skip
-    steps, and in steps of three; logits, states and hidden rows in front of the head."""
+    """The recurrence's path for one token (decay ranks folded in and apart) against the oracle and the path for several: twelve tokens one by one, in a batch whose other slot skips
+    steps, and in steps of three; logits, states and hidden rows in front of the head, of both slots."""
     if over and preset != "tiny6":
         pytest.skip("decay ranks of RWKV-6")
     m, orc, st = models(preset, exact=exact, **over)
@@ -462,9 +462,25 @@ def test_steps_of_one_token_a_slot_against_steps_of_several(models, preset, exac
     toks = [1, 5, 9, 33, 2, 7, 300, 41, 41, 8, 0, 17]
     for s in range(3):
         m.state.load(m.state.init(), s)
-    one = [m.infer_raw([0, 2] if i % 2 else [0], [1, 1] if i % 2 else [1], [t, t] if i % 2 else [t], [capi.OPTION_LAST] * (2 if i % 2 else 1))[0].copy() for i, t in enumerate(toks)]
+    one, other, hidden, other_hidden = [], [], [], []
+    m.keep_hidden(True)
+    try:
+        for i, t in enumerate(toks):
+            k = 1 + i % 2                                           # the other slot takes every second token
+            rows = m.infer_raw([0, 2][:k], [1] * k, [t] * k, [capi.OPTION_LAST] * k)
+            h = m.last_hidden(max_rows=4)
+            assert h.shape[0] == k
+            one.append(rows[0].copy()); hidden.append(h[0].copy())
+            if k == 2:
+                other.append(rows[1].copy()); other_hidden.append(h[1].copy())
+    finally:
+        m.keep_hidden(False)
     three = np.concatenate([m.infer_raw([1], [3], toks[i:i + 3], [capi.OPTION_FULL])[0].copy() for i in range(0, 12, 3)])
     want, _ = orc.run(toks, orc.state_init(), full=True)
     tol = 1e-4 if exact else REL_TOL
     assert rel_err(np.concatenate(one), want) <= REL_TOL and rel_err(np.concatenate(one), three) <= tol
     assert rel_err(m.state.back(0), m.state.back(1)) <= tol
+    assert rel_err(np.stack(hidden), orc.hidden(toks, orc.state_init())[0]) <= REL_TOL
+    want, state = orc.run(toks[1::2], orc.state_init(), full=True)
+    assert rel_err(np.concatenate(other), want) <= REL_TOL and rel_err(m.state.back(2), state) <= 2 * REL_TOL
+    assert rel_err(np.stack(other_hidden), orc.hidden(toks[1::2], orc.state_init())[0]) <= REL_TOL

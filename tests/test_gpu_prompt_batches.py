@@ -1,5 +1,5 @@
-"""Prompt steps of many sequences: the kernels that take over once a step fills the chip (64 rows to a staged key tile, two state columns a thread,
-convolutions in registers), at the edges of their tiles, against the families' restatements."""
+"""Prompt steps of many sequences: the kernels that take over once a step fills the chip (attention of 128 rows on the tensor cores, recurrences sixteen tokens at a time or with two
+state columns a thread, convolutions in registers), at the edges of their tiles, against the families' restatements."""
 import json
 
 import numpy as np
@@ -51,13 +51,14 @@ P, F, K, D = synth.panupel_layer, synth.fufipel_layer, synth.kemirax_layer, synt
 
 @pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(4, 4, 24, 24), (4, 1, 40, 72), (6, 2, 128, 128), (3, 1, 16, 112)])
 def test_attention_over_the_whole_context(heads, kv_heads, dim, vdim):
-    """64 rows are 64, 16, 21 and 21 tokens of one key head; sizes below, at and between the 64-entry halves of a value row."""
+    """128 rows are 128, 32, 42 and 42 tokens of one key head; sizes below, at and between the 64-entry halves of a value row."""
     _check(synth.make_panupel, panupel_numpy, [P("parallel", heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, mm_heads=2, mm_dim=72)], 1, width=96, loop=None)
 
 
-@pytest.mark.parametrize("window, keep", [(8, 2), (33, 0), (40, 5)])
+@pytest.mark.parametrize("window, keep", [(8, 2), (33, 0), (40, 5), (63, 0), (64, 3), (65, 0), (65, 2)])
 def test_attention_in_a_window(window, keep):
-    """Kept first tokens in front of windows that end inside, at and behind a 32-key tile, a bias per distance, a gate per entry; a chunked layer beside it."""
+    """Kept first tokens in front of windows that end inside, at and behind a tile of 64 keys, sequences longer than the window, a bias per distance, a gate per entry; a chunked layer
+    beside it."""
     _check(synth.make_fufipel, fufipel_numpy, [F("attention", heads=4, kv_heads=2, dim=20, window=window, keep_first=keep), F("parallel", heads=2, dim=24, chunk=11)], 1, width=80)
 
 

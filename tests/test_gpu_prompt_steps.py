@@ -132,6 +132,32 @@ def test_last_hidden_answers_the_last_portion(lens, rows):
         m.close()
 
 
+@pytest.mark.parametrize("lens", [[1100], [700, 500, 3]])
+@pytest.mark.parametrize("preset", ["tiny6", "tiny7"])
+def test_hidden_rows_of_steps_of_many_rows(preset, lens):
+    """keep_hidden over steps of more than a thousand rows, eight of them to a CTA; the logits of the last tokens beside them."""
+    st = synth.make_st(preset, 3)
+    orc = O.Oracle(O.parse_st(st), "f16")
+    toks = [np.random.default_rng(n).integers(1, 500, n).tolist() for n in lens]
+    m = runtime.Model(st, max_batch=len(lens), token_chunk_size=128)
+    try:
+        for s in range(len(lens)):
+            m.state.reset(s)
+        m.keep_hidden(True)
+        rows = m.infer_raw(list(range(len(lens))), lens, sum(toks, []), [capi.OPTION_LAST] * len(lens))
+        got = m.last_hidden(max_rows=sum(lens))
+        assert got.shape[0] == sum(lens)
+        at = 0
+        for s, n in enumerate(lens):
+            want, _ = orc.hidden(toks[s], orc.state_init())
+            assert np.abs(got[at:at + n] - want).max() <= TOL * np.abs(want).max(), s
+            last, _ = orc.run(toks[s], orc.state_init())
+            assert np.abs(rows[s] - last).max() <= TOL * np.abs(last).max(), s
+            at += n
+    finally:
+        m.close()
+
+
 # serving precision of the config.json families: bf16 operands (2^-9 each), f32 sums.  A row of a few layers is off by a few of those
 # roundings, a few percent where a norm divides by a small read-out; a wrong tile, edge or row list is off by its own size
 BF16_TOL = 5e-2
@@ -232,7 +258,7 @@ def test_boundaries_of_a_row_of_n_columns(width, n):
 
 @pytest.mark.parametrize("family, precision", [("kemirax", 0), ("panupel", 0), ("panupel", 1)])
 def test_a_token_that_is_not_a_number_reaches_no_row_before_it(family, precision):
-    """Attention works on 64 rows of neighbouring tokens at a time: a later token's value has weight zero in the earlier ones, and zero times NaN must not count."""
+    """Attention works on 64 and 128 rows of neighbouring tokens at a time: a later token's value has weight zero in the earlier ones, and zero times NaN must not count."""
     if family == "kemirax":
         layers, make, module = [synth.kemirax_layer("latent_attention", heads=4, mlp=False)], synth.make_kemirax, kemirax_numpy
         cfg, st, w = make(layers, seed=4)
@@ -307,6 +333,33 @@ def test_a_decay_rate_beyond_f32(dim, vdim, n, precision):
     _tensor(st, "l0.mix.A_log")[1] = 0x42c8
     w["l0.mix.A_log"] = np.array([w["l0.mix.A_log"][0], 100.0])
     _check_image(cfg, st, w, panupel_numpy, n, precision)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("family, layer", [("kemirax", dict(kind="gla", heads=2, dim=72, vdim=40, mlp=False)), ("kemirax", dict(kind="gla", heads=2, dim=128, vdim=128, mlp=False)),
+                                           ("panupel", dict(kind="delta", heads=2, dim=72, vdim=40)), ("panupel", dict(kind="delta", heads=2, dim=128, vdim=128)),
+                                           ("panupel", dict(kind="parallel", heads=2, dim=24, mm_heads=2, mm_dim=128, mm_vdim=72))])
+def test_a_token_that_is_not_a_number_in_a_run_of_sixteen(family, layer, precision):
+    """The recurrences that take a prompt's tokens sixteen at a time: a token in the middle of a run leaves the rows before it, in the same run too, as they are."""
+    if family == "kemirax":
+        make, module, kw, at = synth.make_kemirax, kemirax_numpy, {}, synth.kemirax_layer
+    else:
+        make, module, kw, at = synth.make_panupel, panupel_numpy, {"loop": None}, synth.panupel_layer
+    cfg, st, w = make([at(**layer)], seed=4, width=96, **kw)
+    toks = np.random.default_rng(3).integers(10, 90, 60).tolist()
+    toks[40] = 7
+    st = st.copy()
+    _tensor(st, "embed")[7] = 0x7fc0
+    m = runtime.Model(st, max_batch=1, token_chunk_size=64, config=cfg, kv_tokens=64, kv_page=16, precision=precision)
+    try:
+        m.state.reset(0)
+        got = m.infer_raw([0], [60], toks, [capi.OPTION_FULL])[0]
+        assert np.isnan(got[40:]).all() and np.isfinite(got[:40]).all(), np.isfinite(got).all(1).tolist()
+        want = module.run(json.loads(cfg), w, toks[:40])
+        err = np.sqrt(((got[:40] - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean())
+        assert np.median(err) <= (BF16_TOL if precision == 0 else 2e-4) and err.max() <= (ROW_TOL if precision == 0 else 2e-4), err.tolist()
+    finally:
+        m.close()
 
 
 def test_a_nan_stays_one_in_latent_attention():
