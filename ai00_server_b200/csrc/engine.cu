@@ -570,10 +570,14 @@ struct b200rwkv_engine {
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
     // column a thread, and a chain of tokens takes longer with two)
     bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }
-    bool gla_runs(int rows) const { return rows >= GC_RUN * std::max(1, step_seqs); }      // a run of tokens a sequence or more
+    // a run of tokens a sequence or more, on average: steps of long sequences beside single tokens gain as well (two layers of latent and linear attention, width 2048, token by token and in
+    // runs: one of 512 tokens beside twenty single ones 1085 and 728 us, one of 1000 beside 61 1600 and 1102, sixteen of 100 beside sixteen 1038 and 983, four of 100 beside sixty of 12 905
+    // and 849)
+    bool gla_runs(int rows) const { return rows >= GC_RUN * std::max(1, step_seqs); }
     // Recurrences with one decay a head: three runs a sequence or more, heads wider than half the tiles or a quarter.  Sixteen heads of 128 x 128, token by token and in runs: delta rule,
     // 128 tokens of sixteen sequences 208 and 103 us, 50 of three (72 x 40) 35 and 29, 33 of two 25 and 27, 20 of sixteen 41 and 41, 8 of 64 62 and 107; 64 of sixteen, heads of 64 x 64
     // 60 and 57, of 32 x 32 50 and 55.  Matrix memory: 128 of sixteen 213 and 131, 64 of eight (four heads) 42 and 39, 20 of sixteen 44 and 48; heads of 64 x 64 58 and 72.
+    // On average, too: one of 512 tokens beside eleven single ones 1213 and 650 us (two layers of width 1024); beside twenty it goes token by token, 1327 us, as before runs were there.
     bool run_chunks(int rows, int dk, int dv, int above) const { return rows >= 3 * GC_RUN * std::max(1, step_seqs) && std::max(dk, dv) > above && dk <= GC_DMAX && dv <= GC_DMAX; }
     // Recurrences of prompt steps that have at most one CTA an SM: each asks for more than half an SM's shared memory, so that no two share one.  They start early
     // (programmatic launches), when most SMs are full of the projections in front of them, were packed onto the few that were not and took turns there.
@@ -1759,7 +1763,8 @@ void b200rwkv_engine::enqueue_step(cudaStream_t s, int MT, int MTR, Profiler* pr
         launch_k(embed_ln0_kernel, dim3(rows), dim3(LN_THREADS), 0, ep, KC_LN, s, prof);
     }
     // long steps: seven or eight rows to a CTA (mix.cuh) once there are enough for all SMs (steps of four layers of width 2560, rows by themselves and in sevens: 512 rows 1013 and 1154 us,
-    // 640 1547 and 1591, 1024 2250 and 2232)
+    // 640 1547 and 1591, 1024 2250 and 2232; of two layers, 768, 1024 and 2048 rows: width 1024 353 and 356, 408 and 386, 588 and 508; 2048 538 and 555, 611 and 598, 988 and 889; 3072 696 and
+    // 738, 868 and 866, 1730 and 1685; 3584 926 and 964, 1105 and 1108, 2215 and 2208; 4096, one CTA of eight rows an SM, 1057 and 1069, 1347 and 1300, 2536 and 2468)
     auto ln_tall = [&](int n) { return n >= 1024 && ln_tall_smem(C) <= 200 * 1024; };
     auto launch_ln = [&](const LnMixParams& lp0) {
         LnMixParams lp = lp0;
