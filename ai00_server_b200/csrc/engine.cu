@@ -562,10 +562,14 @@ struct b200rwkv_engine {
     // steps of four layers on the tensor cores and in f32 multiply-adds (us; sequences x tokens): 16 heads of 32 channels 64x32 716 and 660, 48x40 658 and 707, 16x16 377 and 335,
     // 8x16 266 and 284; of 128 channels 64x16 818 and 777, 64x32 997 and 1006, 48x40 916 and 1071, 16x32 487 and 463, 4x32 319 and 368; 16 query heads on 8 key heads of 128 channels
     // 64x8 483 and 473, 64x12 561 and 578; on 4 key heads of 32 channels 64x8 351 and 335, 64x16 416 and 426, 32x8 310 and 330; 32 heads of 64 channels, 32 tokens on 200 keys each, 1191
-    // and 1903.  Steps of more than eight sequences have CTAs for every slot when captured (step_slots): 128 pairs do there, of one or two query heads a key head
+    // and 1903.  One (sequence, key head) pair an SM is a turn, in which the former is the better one (sixteen sequences of 20 tokens, 8 heads of 64 channels, 301 and 316; of 128, 318 and
+    // 351; 32 of 8, 4 heads of 128, 307 and 334), unless it leaves the recurrences of a parallel layer, one a sequence at least, no SM (32 of 16, 4 heads of 32, 319 and 302; 32 of 32, 8 query
+    // heads on 4 key heads of 64, 404 and 389; on 16 query heads 32 of 8 310 and 326)
     bool attn_short(int H, int G, int dk, int dv) const {
         const int rep = H / G, d = std::max(dk, dv);
-        return step_seqs * G >= (step_seqs > FEW_SEQS && rep <= 2 ? 128 : 192) && rep * step_total <= (d > 64 && rep > 1 ? 16 : 32) * step_seqs && step_context <= (d > 64 ? 32 : 64);
+        if (step_context > (d > 64 ? 32 : 64)) return false;
+        if (step_seqs * G > num_sms) return rep * step_total <= (d > 64 && rep > 1 ? 16 : 32) * step_seqs;
+        return step_seqs * (G + 1) > num_sms && d <= 64 && rep <= 2 && rep * step_total <= 64 * step_seqs;
     }
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
     // column a thread, and a chain of tokens takes longer with two)
@@ -593,16 +597,14 @@ struct b200rwkv_engine {
     bool scan_few() const { return Hl * step_seqs <= 3 * num_sms; }
     int scan_slots(int slots) const { return scan_alone ? std::min(slots, scan_alone_seqs) : slots; }
     size_t scan_launch_smem(size_t need) const { return scan_alone ? std::max<size_t>(need, SCAN_ALONE_SMEM) : need; }
-    // Sequences that a step's launches have CTAs for.  Prompt steps: as many as there are, or in a captured step, which serves others of its rows too, up to eight or any number: CTAs for
-    // sequences there are not wait for an SM of their own in the kernels on the tensor cores, only to leave (64 slots, four layers of attention, 32 heads of 64 channels: one prompt of 20
-    // tokens 294 us and 260, two of 32 369 and 290, four of 16 383 and 292)
-    static constexpr int FEW_SEQS = 8;
-    bool step_few(bool decode) const { return !decode && step_seqs > 0 && step_seqs <= FEW_SEQS; }
+    // Sequences that the launches of the kernels on the tensor cores have CTAs for: as many as there are, or in a captured step, which serves others of its rows too, the next row count of
+    // launches (and eight at least).  A CTA for a sequence there is not waits for an SM of its own, only to leave (four layers of attention, 32 heads of 64 channels; 64 slots: one
+    // prompt of 20 tokens 294 us and 260, four of 16 383 and 292; 256 slots: nine of 50 784 and 474, twelve of 40 805 and 490)
     bool step_captured(int rows) const { return use_graph && rows <= 512; }
     int step_slots(int rows, bool decode) const {
         const int most = std::min(S, rows);
-        if (!decode && step_seqs > 0 && !step_captured(rows)) return std::min(most, step_seqs);
-        return step_few(decode) ? std::min(most, (int)FEW_SEQS) : most;
+        if (decode || step_seqs == 0) return most;
+        return std::min(most, step_captured(rows) ? std::max(8, kx_bucket(step_seqs)) : step_seqs);
     }
     int kx_scan_ctas() const;
     int dbg_T = 0;                     // rows a layer has in the debug copy of the residual stream

@@ -461,7 +461,7 @@ void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, i
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
     const bool runs = !decode && gla_runs(rows) && std::max(dk, dv) > 32 && dk <= GC_DMAX && dv <= GC_DMAX;
-    if (runs) launch_k(gla_chunk_kernel, dim3(H_, scan_slots(nslot_grid)), dim3(GC_THREADS), GC_SMEM, gp, KC_WKV, s, prof);
+    if (runs) launch_k(gla_chunk_kernel, dim3(H_, scan_slots(step_slots(rows, decode))), dim3(GC_THREADS), GC_SMEM, gp, KC_WKV, s, prof);
     else launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
     if (runs || sh.ncta > 1) kx_head_norm(s, prof, gp.norm, rows, decode);
 }
@@ -492,7 +492,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
         launch_k(embed_rows_kernel, dim3(rows), dim3(NORM_THREADS), 0, ep, KC_LN, s, prof);
         if (m.pairs && !decode) launch_k(last_token_commit_kernel, dim3(cdiv(std::min(S, rows), 128)), dim3(128), 0, ep, KC_LN, s, prof);
     }
-    const int nslot_grid = step_slots(rows, decode);
+    const int nslot_grid = std::min(S, rows);
     // these end with the last norm
     const bool own_stack = m.cfg.family == KX_FAMILY_ZUFULIX || m.cfg.family == KX_FAMILY_PASOPEL || m.cfg.family == KX_FAMILY_PANUPEL ||
                            m.cfg.family == KX_FAMILY_FUFIPEL;
@@ -544,7 +544,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             if (whole) {
                 LatentPromptParams lp{ap, m.olat, std::min(H_, 16), 0};
                 lp.qt = LP_ROWS / lp.hg;
-                launch_k(D % 8 == 0 ? latent_prompt_kernel<true> : latent_prompt_kernel<false>, dim3(cdiv(rows, lp.qt) + nslot_grid, cdiv(H_, lp.hg)), dim3(LP_THREADS), latent_prompt_smem(D, rk), lp, KC_WKV, s, prof);
+                launch_k(D % 8 == 0 ? latent_prompt_kernel<true> : latent_prompt_kernel<false>, dim3(cdiv(rows, lp.qt) + step_slots(rows, decode), cdiv(H_, lp.hg)), dim3(LP_THREADS), latent_prompt_smem(D, rk), lp, KC_WKV, s, prof);
             } else if (!m.exact) {         // serving precision: both products on the tensor cores (TF32 operands, f32 accumulation and softmax)
                 const size_t sm_b = latent_attn_tc_smem(D);
                 if (!decode) launch_k(latent_attn_tc_kernel<4, 4>, dim3(cdiv(rows, 4) + nslot_grid, cdiv(H_, 4), nsplit), dim3(LT_THREADS), sm_b, ap, KC_WKV, s, prof);
@@ -720,9 +720,9 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
         runs = runs || (!decode && (((l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows)) || ((l.c.mixer == KX_PARALLEL || l.c.mixer == KX_DELTA) && run_chunks(rows, GC_DMAX, GC_DMAX, 0))));
     int64_t forms = 0;                     // which layers attend in the form for short sequences
     for (const KxLayer& l : kx->layers)
-        if (!decode && l.sa_reg && l.c.kv_heads > 0) forms = (forms * 31 + (attn_short(l.c.heads, l.c.kv_heads, l.c.dim, l.c.vdim) ? 1 : 0)) % 1000000007;
+        if (!decode && l.sa_reg && l.c.kv_heads > 0) forms = (forms * 31 + (attn_short(l.c.heads, l.c.kv_heads, l.c.dim, l.c.vdim) ? 1 : 0)) % 4194301;
     const int64_t key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0) +
-                        (step_few(decode) ? (int64_t)1 << 31 : 0) + (forms << 32);
+                        ((int64_t)step_slots(rows, decode) << 31) + (forms << 41);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
         cudaGraph_t g = nullptr;

@@ -62,6 +62,16 @@ __device__ __forceinline__ void step_token_run(const MetaView& meta, const int q
     if (lane == 0) { out[0] = found; out[1] = left; }
 }
 
+// the same counted from the last run (later tokens have more keys: they start first); launches have CTAs for more runs than there are, and those come last
+__device__ __forceinline__ void step_token_run_back(const MetaView& meta, const int qt, const int back, int* out) {
+    const int lane = threadIdx.x & 31, nslots = meta.nslots();
+    int total = 0;
+    for (int s = lane; s < nslots; s += 32) total += (meta.slot_count()[s] + qt - 1) / qt;
+    const int run = __reduce_add_sync(0xffffffffu, total) - 1 - back;
+    if (run >= 0) step_token_run(meta, qt, run, out);
+    else if (lane == 0) out[0] = -1;
+}
+
 struct PageUpdateParams { SeqMeta sm; int* table; int stride; };
 
 __global__ void page_update_kernel(const PageUpdateParams p) {

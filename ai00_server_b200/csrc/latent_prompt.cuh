@@ -102,8 +102,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(const __gr
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&s_tmem);
     pdl_launch_dependents();                                // behind the allocation: see linear_umma.cuh
     pdl_wait();
-    // later tokens have more keys: they start first
-    if (warp == 0) step_token_run(p.meta, pp.qt, gridDim.x - 1 - blockIdx.x, s_tile);
+    if (warp == 0) step_token_run_back(p.meta, pp.qt, blockIdx.x, s_tile);
     __syncthreads();
     const int si = s_tile[0];
     if (si >= 0) {

@@ -205,7 +205,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 const bool runs = !decode && run_chunks(rows, mk, mvd, 64);
                 if (runs) {
                     RunChunkParams cp{mp.q, mp.k, mp.v, PN, 1, mp.zf, PN, mp.zi, PN, nullptr, mp.state, mp.n, mp.m, mp.fac, Hm, mk, mvd, mp.q_scale, mp.den_eps, mp.cap, sh, mp.norm};
-                    launch_k(run_chunk_kernel<false>, dim3(Hm, scan_slots(nslot_grid)), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s2, prof);
+                    launch_k(run_chunk_kernel<false>, dim3(Hm, scan_slots(step_slots(rows, decode))), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s2, prof);
                 } else {
                     launch_k(decode ? matrix_memory_kernel<0> : (sh.nc == 2 ? matrix_memory_kernel<2> : matrix_memory_kernel<1>), dim3(Hm * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), mp, KC_WKV, s2, prof);
                 }
@@ -237,7 +237,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             const bool runs = !decode && run_chunks(rows, dk, dv, 32);
             if (runs) {
                 RunChunkParams cp{dp.q, dp.k, dp.v, ldc, H_ / G_, dp.z, PN, dp.b, PN, l.a_log, l.rec_state, nullptr, nullptr, nullptr, H_, dk, dv, dp.q_scale, dp.unit_eps, 0.f, sh, dp.norm};
-                launch_k(run_chunk_kernel<true>, dim3(H_, scan_slots(nslot_grid)), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s, prof);
+                launch_k(run_chunk_kernel<true>, dim3(H_, scan_slots(step_slots(rows, decode))), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s, prof);
             } else {
                 launch_k(decode ? delta_scan_kernel<false, 0> : (sh.nc == 2 ? delta_scan_kernel<false, 2> : delta_scan_kernel<false, 1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), dp, KC_WKV, s, prof);
             }

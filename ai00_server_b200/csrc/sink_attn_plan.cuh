@@ -176,7 +176,7 @@ void b200rwkv_engine::kx_sink_attn(cudaStream_t s, Profiler* prof, const KxLayer
         PromptAttnParams pa{sp, PT_ROWS / rep};
         const bool whole = (sp.dk | sp.dv | sp.koff | sp.voff | sp.D | sp.ldq) % 8 == 0;
         auto k = whole ? (sp.dk == 128 && sp.dv == 128 ? prompt_attn_kernel<16, true> : prompt_attn_kernel<0, true>) : prompt_attn_kernel<0, false>;
-        launch_k(k, dim3(cdiv(rows, pa.qt) + nslot_grid, sp.G), dim3(PT_THREADS), prompt_attn_smem(sp.dk, sp.dv), pa, KC_WKV, s, prof);
+        launch_k(k, dim3(cdiv(rows, pa.qt) + step_slots(rows, decode), sp.G), dim3(PT_THREADS), prompt_attn_smem(sp.dk, sp.dv), pa, KC_WKV, s, prof);
         return;
     }
     launch_cluster = nsplit;

@@ -85,11 +85,12 @@ def test_attention_at_the_edges_of_key_tiles(heads, kv_heads, dim, vdim):
     (synth.make_panupel, panupel_numpy, [P("delta", heads=2, dim=24), P("parallel", heads=4, kv_heads=2, dim=24, mm_heads=2, mm_dim=24)]),
     (synth.make_fufipel, fufipel_numpy, [F("attention", heads=4, kv_heads=2, dim=20, window=8, keep_first=2), F("parallel", heads=2, dim=24, chunk=11)])])
 def test_steps_of_one_row_count_and_several_numbers_of_sequences(make, module, layers):
-    """Steps of 24 tokens in one sequence, eight, nine and twelve (captured ones hold CTAs for eight sequences or for any number), and longer ones of 3 and 20 (as many as there are)."""
+    """Steps of 24 tokens in one sequence, eight, nine, twelve and eighteen (captured ones hold CTAs for the next power of two, eight at least), and longer ones of 3 and 20 (as many as
+    there are)."""
     cfg, st, w = make(layers, seed=4, width=96, **({"loop": None} if make is synth.make_panupel else {}))
     m = runtime.Model(st, max_batch=24, token_chunk_size=512, precision=1, config=cfg, kv_tokens=2048, kv_page=16)
     try:
-        for lens in ([24], [3] * 8, [3, 3, 3, 3, 3, 3, 2, 2, 2], [2] * 12, [24], [200, 3, 330], [30] * 20, [2] * 12):
+        for lens in ([24], [3] * 8, [3, 3, 3, 3, 3, 3, 2, 2, 2], [2] * 12, [24], [2] * 6 + [1] * 12, [200, 3, 330], [30] * 20, [2] * 12):
             toks = [np.random.default_rng([n, i]).integers(1, 90, n).tolist() for i, n in enumerate(lens)]
             for s in range(len(lens)):
                 m.state.reset(s)
@@ -101,7 +102,7 @@ def test_steps_of_one_row_count_and_several_numbers_of_sequences(make, module, l
         m.close()
 
 
-@pytest.mark.parametrize("heads, kv_heads, dim, vdim, longest", [(4, 4, 24, 24, 32), (2, 2, 128, 128, 32), (8, 2, 32, 36, 14), (9, 3, 72, 104, 8), (3, 3, 64, 4, 33)])
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim, longest", [(4, 4, 24, 24, 32), (3, 3, 128, 128, 32), (12, 3, 32, 36, 14), (9, 3, 72, 104, 8), (3, 3, 64, 4, 33), (4, 2, 40, 40, 33)])
 def test_attention_of_many_short_sequences(heads, kv_heads, dim, vdim, longest):
     """64 sequences of 1 to `longest` tokens, then five more of each: the form for few (token, head) rows a key head, below and behind one of its tiles of 32 keys, rows of one, three
     and four query heads (whose 64 leave one over); and the other side of its rule.  A token that is not a number reaches no row before it and no other sequence."""
