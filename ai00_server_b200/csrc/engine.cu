@@ -574,15 +574,33 @@ struct b200rwkv_engine {
     // recurrences of prompt steps: two state columns a thread once the step's sequences fill the chip that way (a head of one sequence is some four CTAs with one
     // column a thread, and a chain of tokens takes longer with two)
     bool scan_wide(int heads) const { return heads * step_seqs >= 64 && step_seqs >= 4; }
-    // a run of tokens a sequence or more, on average: steps of long sequences beside single tokens gain as well (two layers of latent and linear attention, width 2048, token by token and in
-    // runs: one of 512 tokens beside twenty single ones 1085 and 728 us, one of 1000 beside 61 1600 and 1102, sixteen of 100 beside sixteen 1038 and 983, four of 100 beside sixty of 12 905
-    // and 849)
-    bool gla_runs(int rows) const { return rows >= GC_RUN * std::max(1, step_seqs); }
-    // Recurrences with one decay a head: three runs a sequence or more, heads wider than half the tiles or a quarter.  Sixteen heads of 128 x 128, token by token and in runs: delta rule,
-    // 128 tokens of sixteen sequences 208 and 103 us, 50 of three (72 x 40) 35 and 29, 33 of two 25 and 27, 20 of sixteen 41 and 41, 8 of 64 62 and 107; 64 of sixteen, heads of 64 x 64
-    // 60 and 57, of 32 x 32 50 and 55.  Matrix memory: 128 of sixteen 213 and 131, 64 of eight (four heads) 42 and 39, 20 of sixteen 44 and 48; heads of 64 x 64 58 and 72.
+    // Recurrences sixteen tokens at a time (gla_chunk.cuh, delta_chunk.cuh): a CTA has an SM to itself and pads its head to 128 x 128 and its last run to sixteen tokens.  Which (head, sequence)
+    // pairs that is the better form for, both sides as steps in runs over steps token by token (four layers, 16 heads; sequences x tokens):
+    //   * heads of which both sizes are above 64: any number of pairs.  128 x 128, gated linear attention 9x16 0.83, 16x16 0.93, 32x16 0.96, 64x20 0.96, 32x64 0.77; 72 x 72 0.85, 0.95, 0.95, 1.00, 0.73;
+    //     delta rule 72 x 72 9x48 0.65, 16x48 0.80, 40x48 0.83; matrix memory 72 x 72 0.90, 0.86, 0.94
+    //   * smaller ones: where SMs take one turn (40 x 40, linear attention: 9x16 0.98, 9x100 0.75) or two (16x48 0.94; delta rule 16x48 0.84, 18x100 0.82); more turns lose (20x20 1.21, 32x20 1.38,
+    //     32x64 1.13; delta rule 20x48 0.98, 32x48 1.14, 40x48 1.26), and so do two of fewer than 32 tokens where both sizes are small (16x16 1.06; 40 x 128 0.93).
+    bool runs_fit(int heads, int dk, int dv) const {
+        const int pairs = heads * step_seqs, small = std::min(dk, dv), large = std::max(dk, dv);
+        if (large > GC_DMAX || step_seqs == 0) return false;
+        if (pairs <= num_sms || small > 64) return true;
+        return pairs <= 2 * num_sms && (large > 64 || step_total >= 2 * GC_RUN * step_seqs);
+    }
+    // Tokens a sequence, on average: steps of long sequences beside single tokens gain as well (two layers of latent and linear attention, width 2048, token by token and in runs: one of 512 tokens
+    // beside twenty single ones 1085 and 728 us, one of 1000 beside 61 1600 and 1102, sixteen of 100 beside sixteen 1038 and 983, four of 100 beside sixty of 12 905 and 849).  A run of them; two
+    // where few pairs with short keys and long values run many CTAs a head token by token (four layers of 16 heads of 40 x 128, one of 20 tokens 222 and 231 us, of 40 264 and 258)
+    bool gla_runs(int heads, int dk, int dv) const {
+        const int least = heads * step_seqs <= 32 && dk <= 64 && dv > 64 ? 2 : 1;
+        return runs_fit(heads, dk, dv) && std::max(dk, dv) > 32 && step_total >= least * GC_RUN * step_seqs;
+    }
+    // One decay a head: three runs, heads wider than half the tiles (matrix memory) or a quarter.  Sixteen heads of 128 x 128, token by token and in runs: delta rule, 128 tokens of sixteen
+    // sequences 208 and 103 us, 50 of three (72 x 40) 35 and 29, 33 of two 25 and 27, 20 of sixteen 41 and 41, 8 of 64 62 and 107.  Matrix memory: 128 of sixteen 213 and 131, 64 of eight
+    // (four heads) 42 and 39, 20 of sixteen 44 and 48; heads of 64 x 64 58 and 72; few pairs from four runs on (four layers of four heads, one of 48 tokens 301 and 296 us, of 50 311 and 322).
     // On average, too: one of 512 tokens beside eleven single ones 1213 and 650 us (two layers of width 1024); beside twenty it goes token by token, 1327 us, as before runs were there.
-    bool run_chunks(int rows, int dk, int dv, int above) const { return rows >= 3 * GC_RUN * std::max(1, step_seqs) && std::max(dk, dv) > above && dk <= GC_DMAX && dv <= GC_DMAX; }
+    bool run_chunks(int heads, int dk, int dv, bool memory) const {
+        const int least = memory && heads * step_seqs <= 32 ? 4 : 3;
+        return runs_fit(heads, dk, dv) && std::max(dk, dv) > (memory ? 64 : 32) && step_total >= least * GC_RUN * step_seqs;
+    }
     // Recurrences of prompt steps that have at most one CTA an SM: each asks for more than half an SM's shared memory, so that no two share one.  They start early
     // (programmatic launches), when most SMs are full of the projections in front of them, were packed onto the few that were not and took turns there.
     // Measured (whole prompts, four layers of width 2560): one of 200 tokens 988 -> 856 us; two layers of gated delta rule, matrix memory and attention of width 2048:

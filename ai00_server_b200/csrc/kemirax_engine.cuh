@@ -451,16 +451,16 @@ void b200rwkv_engine::kx_short_conv(cudaStream_t s, Profiler* prof, const ShortC
     if (cp.taps > 1) launch_k(conv_commit_kernel, dim3(nslot_grid, cb), dim3(256), 0, cp, KC_OTHER, s, prof);
 }
 
-// Gated linear attention of a layer: the recurrence, and the norm over heads that are spread over several CTAs.  Sixteen tokens at a time (gla_chunk.cuh) where sequences have
-// as many and heads are not much narrower than its tiles; 16 heads of 128 x 128, eight sequences: 256 tokens 256 us token by token and 69 in runs, 20 tokens of sixteen 38 and
-// 31, 8 tokens of 64 sequences 63 and 76; 64 tokens of sixteen sequences, heads of 64 x 64 49 and 44, of 32 x 32 42 and 43.
+// Gated linear attention of a layer: the recurrence, and the norm over heads that are spread over several CTAs.  Sixteen tokens at a time (gla_chunk.cuh) by the rule at gla_runs;
+// the recurrence alone, 16 heads of 128 x 128, eight sequences: 256 tokens 256 us token by token and 69 in runs, 20 tokens of sixteen 38 and 31, 8 tokens of 64 sequences 63 and 76; 64
+// tokens of sixteen sequences, heads of 64 x 64 49 and 44, of 32 x 32 42 and 43.
 void b200rwkv_engine::kx_gla(cudaStream_t s, Profiler* prof, const KxLayer& l, int H_, int dk, int dv, const float* q, const float* k, const float* v,
                              const float* gate, int ld, float* out, int ldo, int rows, int nslot_grid, bool decode) {
     SeqModel& m = *kx;
     const ScanShape sh = scan_shape(dk, dv, 3, decode, scan_wide(H_));
     GlaParams gp{q, k, v, ld, m.z, H_ * dk, l.gla_state, H_, dk, dv, 1.f / l.c.tau, 1.f / sqrtf((float)dk), sh,
                  {out, ldo, nullptr, gate, ld, l.norm_w, 0, H_, dv, m.cfg.eps, 1.f, 1, meta_view(d_meta, step_rows)}};
-    const bool runs = !decode && gla_runs(rows) && std::max(dk, dv) > 32 && dk <= GC_DMAX && dv <= GC_DMAX;
+    const bool runs = !decode && gla_runs(H_, dk, dv);
     if (runs) launch_k(gla_chunk_kernel, dim3(H_, scan_slots(step_slots(rows, decode))), dim3(GC_THREADS), GC_SMEM, gp, KC_WKV, s, prof);
     else launch_k(decode ? gla_scan_kernel<0> : (sh.nc == 2 ? gla_scan_kernel<2> : gla_scan_kernel<1>), dim3(H_ * sh.ncta, scan_slots(nslot_grid)), dim3(sh.threads), scan_launch_smem(sh.smem_floats() * 4), gp, KC_WKV, s, prof);
     if (runs || sh.ncta > 1) kx_head_norm(s, prof, gp.norm, rows, decode);
@@ -715,13 +715,18 @@ void b200rwkv_engine::kx_run_step(int T, int R, bool decode, int nsplit) {
     for (const KxLayer& l : kx->layers)
         for (int h : {l.c.heads, l.c.mm_heads})
             if (!decode && h > 0 && h < 256 && scan_wide(h) && (wide == 0 || h < wide)) wide = h;
-    bool runs = false;                     // and whether they take the tokens in runs
-    for (const KxLayer& l : kx->layers)
-        runs = runs || (!decode && (((l.c.mixer == KX_GLA || l.c.mixer == KX_CHUNK_GLA) && gla_runs(rows)) || ((l.c.mixer == KX_PARALLEL || l.c.mixer == KX_DELTA) && run_chunks(rows, GC_DMAX, GC_DMAX, 0))));
-    int64_t forms = 0;                     // which layers attend in the form for short sequences
-    for (const KxLayer& l : kx->layers)
-        if (!decode && l.sa_reg && l.c.kv_heads > 0) forms = (forms * 31 + (attn_short(l.c.heads, l.c.kv_heads, l.c.dim, l.c.vdim) ? 1 : 0)) % 4194301;
-    const int64_t key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) + (runs ? 1 << 30 : 0) +
+    int64_t forms = 0;                     // what form each layer's kernels have: attention of short sequences, recurrences in runs
+    for (const KxLayer& l : kx->layers) {
+        if (decode) break;
+        const KxLayerCfg& c = l.c;
+        int form = l.sa_reg && c.kv_heads > 0 && attn_short(c.heads, c.kv_heads, c.dim, c.vdim) ? 1 : 0;
+        if (c.mixer == KX_GLA) form += gla_runs(c.heads, c.dim, c.vdim) ? 2 : 0;
+        if (c.mixer == KX_CHUNK_GLA) form += gla_runs(c.mm_heads, c.mm_dim, c.mm_vdim) ? 2 : 0;
+        if (c.mixer == KX_PARALLEL) form += run_chunks(c.mm_heads, c.mm_dim, c.mm_vdim, true) ? 2 : 0;
+        if (c.mixer == KX_DELTA) form += run_chunks(c.heads, c.dim, c.vdim, false) ? 2 : 0;
+        forms = (forms * 31 + form) % 4194301;
+    }
+    const int64_t key = 1000000 + (((rows / 8) * 128 + rrows / 8) * 2 + (decode ? 1 : 0)) * 8 + lg + (scan_alone ? 1 << 21 : 0) + (wide << 22) +
                         ((int64_t)step_slots(rows, decode) << 31) + (forms << 41);
     auto it = graphs.find(key);
     if (it == graphs.end()) {

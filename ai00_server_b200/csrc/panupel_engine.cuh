@@ -202,7 +202,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
                 MatrixMemoryParams mp{m.pr + r.mq, m.pr + r.mk, m.pr + r.mv, PN, m.pr + r.mi, m.pr + r.mf, l.mm_state, l.mm_n, l.mm_m, m.z, Hm, mk, mvd,
                                       c.mm_cap, 1.f / sqrtf((float)mk), 1e-6f, sh,
                                       {m.vout + H_ * dv, KO, m.z, m.pr + r.mg, PN, l.mm_norm_w, mvd, Hm, mvd, eps, c.mm_mul, 0, mv}};
-                const bool runs = !decode && run_chunks(rows, mk, mvd, 64);
+                const bool runs = !decode && run_chunks(Hm, mk, mvd, true);
                 if (runs) {
                     RunChunkParams cp{mp.q, mp.k, mp.v, PN, 1, mp.zf, PN, mp.zi, PN, nullptr, mp.state, mp.n, mp.m, mp.fac, Hm, mk, mvd, mp.q_scale, mp.den_eps, mp.cap, sh, mp.norm};
                     launch_k(run_chunk_kernel<false>, dim3(Hm, scan_slots(step_slots(rows, decode))), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s2, prof);
@@ -234,7 +234,7 @@ void b200rwkv_engine::pn_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             const ScanShape sh = scan_shape(dk, dv, 2, decode, scan_wide(H_));
             DeltaScanParams dp{m.cv, m.cv + G_ * dk, m.cv + 2 * G_ * dk, ldc, m.pr + r.a, PN, m.pr + r.b, PN, l.a_log, l.rec_state, H_, G_, dk, dv,
                                1.f / sqrtf((float)dk), 1e-6f, sh, {m.vout, KO, nullptr, m.pr + r.g, PN, l.norm_w, 0, H_, dv, eps, 1.f, 1, mv}};
-            const bool runs = !decode && run_chunks(rows, dk, dv, 32);
+            const bool runs = !decode && run_chunks(H_, dk, dv, false);
             if (runs) {
                 RunChunkParams cp{dp.q, dp.k, dp.v, ldc, H_ / G_, dp.z, PN, dp.b, PN, l.a_log, l.rec_state, nullptr, nullptr, nullptr, H_, dk, dv, dp.q_scale, dp.unit_eps, 0.f, sh, dp.norm};
                 launch_k(run_chunk_kernel<true>, dim3(H_, scan_slots(step_slots(rows, decode))), dim3(GC_THREADS), DC_SMEM, cp, KC_WKV, s, prof);

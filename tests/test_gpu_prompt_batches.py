@@ -156,14 +156,14 @@ def test_gated_linear_attention_in_runs(dim, vdim, tau, precision):
     and such that tokens go one by one."""
     cfg, st, w = synth.make_kemirax([K("gla", heads=3, dim=dim, vdim=vdim, tau=tau, mlp=False)], seed=8, width=96)
     lens = [15, 16, 17, 33, 120]
-    toks = [np.random.default_rng(n).integers(1, 90, n + 21).tolist() for n in lens]
+    toks = [np.random.default_rng(n).integers(1, 90, n + 37).tolist() for n in lens]
     m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, precision=precision, config=cfg, kv_tokens=512)
     try:
         for s in range(len(lens)):
             m.state.reset(s)
         opt = [capi.OPTION_FULL] * len(lens)
         got = m.infer_raw(list(range(len(lens))), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
-        more = m.infer_raw(list(range(len(lens))), [21] * len(lens), sum((t[n:] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw(list(range(len(lens))), [37] * len(lens), sum((t[n:] for t, n in zip(toks, lens)), []), opt)
         for s in range(len(lens)):
             err = _errs(np.concatenate([got[s], more[s]]), kemirax_numpy.run(json.loads(cfg), w, toks[s]))
             if precision == 1:
@@ -180,15 +180,15 @@ def test_gated_linear_attention_in_runs(dim, vdim, tau, precision):
 def test_recurrences_with_one_decay_a_head_in_runs(layer, precision):
     """Sequences of about a run of sixteen tokens, several and parts of them, continued in a second call; sizes that are no multiples of eight or four; keys of two heads in common."""
     cfg, st, w = synth.make_panupel([layer], seed=8, width=96, loop=None)
-    lens = [15, 16, 17, 33, 200]
-    toks = [np.random.default_rng(n).integers(1, 90, n + 50).tolist() for n in lens]
+    lens, then = [15, 16, 17, 33, 280], 70
+    toks = [np.random.default_rng(n).integers(1, 90, n + then).tolist() for n in lens]
     m = runtime.Model(st, max_batch=len(lens), token_chunk_size=512, precision=precision, config=cfg, kv_tokens=1024)
     try:
         for s in range(len(lens)):
             m.state.reset(s)
         opt = [capi.OPTION_FULL] * len(lens)
         got = m.infer_raw(list(range(len(lens))), lens, sum((t[:n] for t, n in zip(toks, lens)), []), opt)
-        more = m.infer_raw(list(range(len(lens))), [50] * len(lens), sum((t[n:] for t, n in zip(toks, lens)), []), opt)
+        more = m.infer_raw(list(range(len(lens))), [then] * len(lens), sum((t[n:] for t, n in zip(toks, lens)), []), opt)
         for s in range(len(lens)):
             err = _errs(np.concatenate([got[s], more[s]]), panupel_numpy.run(json.loads(cfg), w, toks[s]))
             if precision == 1:

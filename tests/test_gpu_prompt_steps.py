@@ -346,14 +346,14 @@ def test_a_token_that_is_not_a_number_in_a_run_of_sixteen(family, layer, precisi
     else:
         make, module, kw, at = synth.make_panupel, panupel_numpy, {"loop": None}, synth.panupel_layer
     cfg, st, w = make([at(**layer)], seed=4, width=96, **kw)
-    toks = np.random.default_rng(3).integers(10, 90, 60).tolist()
+    toks = np.random.default_rng(3).integers(10, 90, 80).tolist()
     toks[40] = 7
     st = st.copy()
     _tensor(st, "embed")[7] = 0x7fc0
-    m = runtime.Model(st, max_batch=1, token_chunk_size=64, config=cfg, kv_tokens=64, kv_page=16, precision=precision)
+    m = runtime.Model(st, max_batch=1, token_chunk_size=128, config=cfg, kv_tokens=128, kv_page=16, precision=precision)
     try:
         m.state.reset(0)
-        got = m.infer_raw([0], [60], toks, [capi.OPTION_FULL])[0]
+        got = m.infer_raw([0], [80], toks, [capi.OPTION_FULL])[0]
         assert np.isnan(got[40:]).all() and np.isfinite(got[:40]).all(), np.isfinite(got).all(1).tolist()
         want = module.run(json.loads(cfg), w, toks[:40])
         err = np.sqrt(((got[:40] - want) ** 2).mean(1)) / np.sqrt((want ** 2).mean())
