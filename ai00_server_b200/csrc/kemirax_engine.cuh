@@ -517,7 +517,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
             if (x16) p.X16 = b;
             return p;
         };
-        launch_k(norm_shift_kernel, dim3(rows), dim3(NORM_THREADS), 0, ns, KC_LN, s, prof);
+        launch_k(row_pieces(W, rows) ? norm_shift_kernel<true> : norm_shift_kernel<false>, dim3(rows), dim3(NORM_THREADS), 0, ns, KC_LN, s, prof);
         launch_k(shift_commit_kernel, dim3(nslot_grid), dim3(NORM_THREADS), 0, ns, KC_LN, s, prof);
         const int GW = c.has_mlp ? 2 * W : W;
         kx_lin(s, prof, from(lin(m.h, W, l.rg, m.G, GW, GW, W, LE_SIGMOID, l.rg_b), m.h16), rows, 1);
@@ -581,7 +581,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
         if (c.has_mlp) {
             const int E = c.experts, NE = E + c.identity, ff = c.ff;
             MoeRouteParams rp{m.h, W, l.router, W, l.corr, NE, c.top, m.sel, m.wgt, mv};
-            launch_k(moe_route_threads(rows) == 1024 ? moe_route_kernel<1024> : moe_route_kernel<256>, dim3(rows), dim3(moe_route_threads(rows)), moe_route_smem(W, NE), rp, KC_OTHER, s, prof);
+            launch_k(moe_route_threads(rows, W) == 1024 ? moe_route_kernel<1024> : moe_route_kernel<256>, dim3(rows), dim3(moe_route_threads(rows, W)), moe_route_smem(W, NE), rp, KC_OTHER, s, prof);
             MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
             kx_moe_group(s, prof, gp, rows);
             if (E > 0) {
@@ -607,7 +607,7 @@ void b200rwkv_engine::kx_enqueue_step(cudaStream_t s, int rows, int rrows, bool 
     }
     if (!own_stack) {
         FinalNormParams fn{m.x, m.hn, d_hidden, m.final_gain, m.cfg.eps, W, mv, m.final_w};
-        launch_k(final_norm_kernel, dim3(rows), dim3(NORM_THREADS), 0, fn, KC_LN, s, prof);
+        launch_k(row_pieces(W, rows) ? final_norm_kernel<true> : final_norm_kernel<false>, dim3(rows), dim3(NORM_THREADS), 0, fn, KC_LN, s, prof);
     }
     if (rrows > 0) {
         LinParams ph = lin(m.hn, W, m.head, d_logits, V, V, W);

@@ -39,8 +39,8 @@ struct MoeRouteParams {
 enum MoeRouteMode { MOE_SOFTMAX_ALL = 0, MOE_TOP_LOGITS = 1, MOE_SIGMOID_GROUPS = 2 };
 
 // Threads of a token's CTA.  Few tokens (decode): 32 warps, so that a warp has its outputs' rows requested in one or two turns (sixteen tokens, width 2048: 12.8 us of the step with
-// eight, 8.5); many: eight, the CTAs of other tokens cover the waits (2000 tokens: 46 us with 32, 38).
-inline int moe_route_threads(int rows) { return rows <= 128 ? 1024 : 256; }
+// eight, 8.5); many, or narrow rows: eight, the CTAs of other tokens cover the waits (2000 tokens: 46 us with 32, 38; a step of 64 tokens, four layers of width 128, 338 with 32, 321).
+inline int moe_route_threads(int rows, int W) { return rows <= 128 && W >= 384 ? 1024 : 256; }
 __host__ __device__ inline int moe_route_row(int K) { return (K + 255) & ~255; }
 __host__ __device__ inline size_t moe_route_smem(int K, int NE) { return ((size_t)moe_route_row(K) + 3 * (size_t)NE) * sizeof(float); }
 

@@ -39,7 +39,9 @@ __device__ __forceinline__ float rms_block_sum(float v, float* red /* [32] */) {
 // row of 2048 took eight round trips to memory in a row: in a decode step of sixteen tokens norm_shift 8.2 us of the step, embed_rows 10 (now 3.0 and 5.8).
 constexpr int ROW_PIECES = 4;
 __device__ __forceinline__ bool row_whole(const void* p, int bytes = 16) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }      // (true of no pointer)
-__host__ __device__ inline bool row_pieces(int W) { return W % 4 == 0 && W <= 4 * ROW_PIECES * NORM_THREADS; }
+// The norms hold 71 and 58 registers a thread with it and 32 without, three or four CTAs an SM instead of eight, which many narrow rows feel: they have the form or not (`PIECES`), by width and
+// rows.  Both sides in steps of four layers, 2048 rows: width 256 356 us without and 369 with, 512 376 and 382, 768 399 and 398, 1024 423 and 416; one row of 384 100 and 97
+inline bool row_pieces(int W, int rows) { return W % 4 == 0 && W <= 4 * ROW_PIECES * NORM_THREADS && (W >= 768 || rows <= 256); }
 __device__ __forceinline__ float row_dot(const float4 a, const float4 b, float sum) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, sum)))); }
 __device__ __forceinline__ float4 row_bf16(const uint2 q) {
     const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(q.x)), b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(q.y));
@@ -90,7 +92,7 @@ __global__ void __launch_bounds__(NORM_THREADS) embed_rows_kernel(const EmbedRow
         }
     }
     float* dst = p.x + (size_t)t * p.copies * p.W;
-    if (row_pieces(p.W) && row_whole(src, 8) && row_whole(src2, 8) && row_whole(dst)) {
+    if (p.W % 4 == 0 && p.W <= 4 * ROW_PIECES * NORM_THREADS && row_whole(src, 8) && row_whole(src2, 8) && row_whole(dst)) {
         float4 v[ROW_PIECES];
 #pragma unroll
         for (int i = 0; i < ROW_PIECES; ++i) {
@@ -141,6 +143,7 @@ struct NormShiftParams {
     __nv_bfloat16* hs16 = nullptr;
 };
 
+template <bool PIECES>
 __global__ void __launch_bounds__(NORM_THREADS) norm_shift_kernel(const NormShiftParams p) {
     pdl_launch_dependents();
     pdl_wait();
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_shift_kernel(const NormShif
     const int prev = p.meta.tok_prev()[t];
     const int slot = p.meta.tok_slot()[t];
     float ss = 0.f, sp = 0.f;
-    if (row_pieces(W) && row_whole(p.x) && row_whole(p.h) && row_whole(p.hs) && row_whole(p.h16, 8) && row_whole(p.hs16, 8) && row_whole(p.mu) && row_whole(p.shift_state)) {
+    if (PIECES && row_whole(p.x) && row_whole(p.h) && row_whole(p.hs) && row_whole(p.h16, 8) && row_whole(p.hs16, 8) && row_whole(p.mu) && row_whole(p.shift_state)) {
         const bool shifted = p.hs || p.hs16;
         float4 x[ROW_PIECES], u[ROW_PIECES], mu[ROW_PIECES];       // u: the row before, or the state
         const float* const ur = prev >= 0 ? p.x + (size_t)prev * W : p.shift_state + (size_t)slot * W;
@@ -252,6 +255,7 @@ struct FinalNormParams {
     const float* weight = nullptr;   // [W] per-channel weight instead of the scalar gain
 };
 
+template <bool PIECES>
 __global__ void __launch_bounds__(NORM_THREADS) final_norm_kernel(const FinalNormParams p) {
     pdl_launch_dependents();
     pdl_wait();
@@ -261,7 +265,7 @@ __global__ void __launch_bounds__(NORM_THREADS) final_norm_kernel(const FinalNor
     const int W = p.W;
     const float* xr = p.x + (size_t)t * W;
     const int row = p.meta.tok_outrow()[t];
-    if (row_pieces(W) && row_whole(p.x) && row_whole(p.hidden) && row_whole(p.y) && row_whole(p.weight)) {
+    if (PIECES && row_whole(p.x) && row_whole(p.hidden) && row_whole(p.y) && row_whole(p.weight)) {
         float4 x[ROW_PIECES], w[ROW_PIECES];
 #pragma unroll
         for (int i = 0; i < ROW_PIECES; ++i) {

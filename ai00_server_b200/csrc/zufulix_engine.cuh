@@ -245,7 +245,7 @@ void b200rwkv_engine::zf_enqueue_layers(cudaStream_t s, int rows, int nslot_grid
             } else {
                 const int E = c.experts, ff = c.ff;
                 MoeRouteParams rp{m.h, W, l.router, W, nullptr, E, c.top, m.sel, m.wgt, mv, MOE_SIGMOID_GROUPS, c.groups, c.groups_keep};
-                launch_k(moe_route_threads(rows) == 1024 ? moe_route_kernel<1024> : moe_route_kernel<256>, dim3(rows), dim3(moe_route_threads(rows)), moe_route_smem(W, E), rp, KC_OTHER, s, prof);
+                launch_k(moe_route_threads(rows, W) == 1024 ? moe_route_kernel<1024> : moe_route_kernel<256>, dim3(rows), dim3(moe_route_threads(rows, W)), moe_route_smem(W, E), rp, KC_OTHER, s, prof);
                 MoeGroupParams gp{m.sel, c.top, E, m.cnt, m.off, m.list, m.row_of, mv};
                 kx_moe_group(s, prof, gp, rows);
                 LinParams p1 = lin(m.h, W, l.gu, m.yc, ff, ff, W, LE_RELU_SQ);
